@@ -386,6 +386,20 @@ int latent_attn_mma(const float* q, const __nv_bfloat16* kc, const int32_t* bloc
                     int rank, int block_size, float scale, const float* sink, cudaStream_t s, int n_splits, float* part, int window) {
   if (T == 0) return B200_OK;
   B200_REQUIRE(latent_attn_mma_supported(heads, krow, rank), B200_ERR_UNSUPPORTED, "latent_attn_mma: shape %d / %d / %d", heads, krow, rank);
+  if (n_splits < 1 || part == nullptr) n_splits = 1;
+  B200_REQUIRE(n_splits <= kLaMaxSplits, B200_ERR_INVALID, "attention: %d splits (at most %d)", n_splits, kLaMaxSplits);
+  const auto at = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr); };
+  B200_REQUIRE(at(kc) % 16 == 0, B200_ERR_INVALID, "attention: cache not 16-byte aligned");
+  // tcgen05 wherever the shape fits and the rows can be read and written in its wide pieces (what it measured stands there; it is
+  // the faster one from one decode row up); other shapes, blocks that a key tile would straddle and odd addresses stay here
+  if (latent_attn_tc_supported(heads, krow, rank, block_size) && at(q) % 16 == 0 && at(out) % 32 == 0 && ((at(runs) | at(part)) & 7) == 0) {
+    const int rc = latent_attn_tc(q, kc, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, krow, rank, block_size, scale,
+                                  sink, s, n_splits, part, window);
+    if (rc || n_splits == 1) return rc;
+    B200_CUDA(launch(latent_attn_merge_kernel, dim3((T * heads + 3) / 4), dim3(128), (size_t)0, s, (const float*)part, out, T * heads, heads,
+                     rank, n_splits, sink, (const __nv_bfloat16*)nullptr, (int64_t)0));
+    return B200_OK;
+  }
   return attn_mma_launch(q, kc, nullptr, 1, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, krow, rank, block_size,
                          scale, sink, s, n_splits, part, window, AttnExtra());
 }

@@ -1,0 +1,537 @@
+// Paged causal attention over latent cache rows on tcgen05 (bf16 serving mode of B200_MIXER_LATENT).
+//
+// One kv head serves every query head and a key row's leading `rank` entries are its value.  A work item is 128 (row, head)
+// pairs of one run of consecutive rows of a sequence (128 / heads rows) on the MMA's M dimension times one half of the value
+// columns; per tile of 64 keys
+//   S[128][64] = Q[128][krow] . K_tile^T            O[128][<= 256] += P[128][64] . V_tile   (V_tile: columns of K_tile, MN-major)
+// The two halves of the value columns are items of their own because O takes all 512 TMEM columns otherwise: the scores are
+// computed twice (1.5 x the operations), and nothing is exchanged between CTAs.
+//
+// What bounds it: the issue and execution of 36 score MMAs of 64 columns a tile (about 1.9 us per tile, krow 576), then the query
+// staging and the output at an item's ends.  Q is the large operand (krow 576: 147 KB of bf16), so the part that matches the value
+// columns lives in TMEM (columns 384..511, A operand read from there) and only the rest in shared memory, which leaves room for
+// three stages of value columns and a tile of the other columns.  TMEM: O 0..255, two score buffers of 64 columns, the Q part.
+// The weights overwrite the scores in place (bf16 pairs, A operand of the second product) and never touch shared memory.
+// Against the mma.sync kernel of attn_latent.cu with 16 pairs a CTA, which reads every key tile once per row: 2 048 rows of 16
+// heads over 512 + 64 at contexts 1..2048 907 -> 183 us, 64 decode rows at contexts 500..1000 98 -> 47 us; error against 64 bits
+// 2.57e-3 -> 2.60e-3 and 2.65e-3 -> 2.71e-3 (0.98 to 1.03 of the other kernel's over other sizes: both round queries, weights
+// and results to bf16).
+// Warps: TMA producer, MMA issuer, four softmax warps (a thread owns a pair), eight that stage the next item's queries.
+// The running maximum is only followed when it rises by more than 2^8 (the scaling of all terms is the same, so the
+// quotient is exact); a warp then rescales its own 32 rows of O in TMEM.
+// Every wait is bounded (tc.cuh).
+#include <stdlib.h>
+
+#include <algorithm>
+
+#include "tc.cuh"
+
+namespace b200 {
+namespace {
+
+using namespace tc;
+
+constexpr int kLtKeys = 64, kLtPairs = 128, kLtThreads = 448;
+constexpr int kLtChunk = kLtKeys * 128;        // [64 keys][64 columns] bf16: 8 KiB
+constexpr int kLtQChunk = kLtPairs * 128;      // [128 pairs][64 columns] bf16: 16 KiB
+constexpr int kLtMaxStages = 4, kLtMaxRest = 5, kLtMaxSlots = 12;
+constexpr int kLtSmem = 232448, kLtTail = 2048;
+constexpr int kLtTable = 32;                   // items of a CTA whose description is worked out ahead
+constexpr uint32_t kTmS = 256, kTmQ = 384;     // TMEM columns: O at 0, scores (then weights) of even / odd tiles, Q part
+
+struct LtParams {
+  const float* q;
+  const int32_t* block_table;
+  const int32_t* row_to_seq;
+  const int32_t* ctx_lens;
+  const int32_t* runs;      // (first row, rows) pairs: at most 16 rows of one sequence, contexts rising by one
+  const int32_t* n_runs;
+  const float* sink;
+  __nv_bfloat16* out;
+  float* part;
+  int n_rows, bt_stride, heads, krow, rank, block_size, n_splits, window, own_stages, rest_slots, halves, rows_per_item, items_per_run;
+  float scale;
+};
+
+struct LtItem {
+  int t0, nr, half, split, seq, ctx0, ctx_max, tile_lo, tile_hi;   // ctx0: context of the item's first row
+};
+
+// item `it` of the list (run, part of the run, split, half); false: nothing there
+__device__ __forceinline__ bool lt_item(const LtParams& p, int n_runs, int it, LtItem& w) {
+  w.half = it % p.halves;
+  it /= p.halves;
+  w.split = it % p.n_splits;
+  it /= p.n_splits;
+  // mostly whole runs (prefill): a run's parts follow each other, all by falling context.  Mostly short runs (decode rows): the first
+  // parts of all runs lead, so that the parts that do not exist fall to the end of the list and every CTA gets its share of work
+  const bool whole = p.n_rows >= n_runs * p.rows_per_item;
+  const int part = whole ? p.items_per_run - 1 - it % p.items_per_run : it / n_runs;
+  const int run = n_runs - 1 - (whole ? it / p.items_per_run : it % n_runs);
+  const int2 r = __ldg(reinterpret_cast<const int2*>(p.runs) + run);
+  w.t0 = r.x + part * p.rows_per_item;
+  w.nr = min(r.y - part * p.rows_per_item, p.rows_per_item);
+  if (w.nr <= 0) return false;
+  w.seq = p.row_to_seq ? __ldg(p.row_to_seq + w.t0) : w.t0;
+  w.ctx0 = __ldg(p.ctx_lens + w.t0);
+  w.ctx_max = __ldg(p.ctx_lens + w.t0 + w.nr - 1);
+  const int tile0 = p.window > 0 ? max(w.ctx0 - p.window, 0) / kLtKeys : 0;
+  const int tiles = max((w.ctx_max + kLtKeys - 1) / kLtKeys - tile0, 0), per = (tiles + p.n_splits - 1) / p.n_splits;
+  w.tile_lo = tile0 + min(tiles, w.split * per);
+  w.tile_hi = tile0 + min(tiles, (w.split + 1) * per);
+  return true;
+}
+
+__global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __grid_constant__ CUtensorMap map, const LtParams p) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int chunks = (p.krow + 63) >> 6, ksteps = p.krow >> 4;
+  // value columns of a half and the chunks that hold them (the largest half decides the layout of shared memory)
+  const int width0 = min(p.rank, 256), own0 = (width0 + 63) >> 6;
+  const int width1 = p.halves > 1 ? p.rank - 256 : width0, own1 = (width1 + 63) >> 6;
+  const int max_rest = chunks - min(own0, own1), max_own = max(own0, own1);
+  unsigned char* qs = smem;                                  // [max_rest][128][64] queries of the columns outside the half
+  unsigned char* own_ring = qs + max_rest * kLtQChunk;       // [own_stages][max_own][64][64] value columns of a tile
+  unsigned char* rest_ring = own_ring + p.own_stages * max_own * kLtChunk;   // [rest_slots][64][64] the tile's other chunks
+  uint64_t* own_full = reinterpret_cast<uint64_t*>(rest_ring + p.rest_slots * kLtChunk);
+  uint64_t* own_free = own_full + kLtMaxStages;
+  uint64_t* rest_full = own_free + kLtMaxStages;
+  uint64_t* rest_free = rest_full + kLtMaxSlots;
+  uint64_t* s_full = rest_free + kLtMaxSlots;    // [2]
+  uint64_t* p_ready = s_full + 2;                // [2]
+  uint64_t* o_full = p_ready + 2;                // [2]
+  uint64_t* q_ready = o_full + 2;
+  uint64_t* q_free = q_ready + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(q_free + 1);
+  LtItem* table = reinterpret_cast<LtItem*>(tmem_slot + 2);   // nr 0: nothing there
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.own_stages; ++s) {
+      mbar_init(own_full + s, 1);
+      mbar_init(own_free + s, 1);
+    }
+    for (int s = 0; s < p.rest_slots; ++s) {
+      mbar_init(rest_full + s, 1);
+      mbar_init(rest_free + s, 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(s_full + s, 1);
+      mbar_init(p_ready + s, 4);
+      mbar_init(o_full + s, 1);
+    }
+    mbar_init(q_ready, 8);
+    mbar_init(q_free, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  pdl_wait();
+  pdl_launch_dependents();
+  const int n_runs = *p.n_runs, n_items = n_runs * p.items_per_run * p.n_splits * p.halves;
+  // the descriptions hang on a chain of loads (run, contexts, sequence): all of the CTA's first ones at once, for every role
+  if (warp == 6 && (int)(blockIdx.x + lane * gridDim.x) < n_items) {
+    LtItem w;
+    if (!lt_item(p, n_runs, blockIdx.x + lane * gridDim.x, w)) w.nr = 0;
+    table[lane] = w;
+  }
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const uint32_t tmem = *tmem_slot;
+  int turn = 0;   // of the role's walk over the CTA's items
+  auto next_item = [&](int it, LtItem& w) {
+    const int k = turn++;
+    if (k >= kLtTable) return lt_item(p, n_runs, it, w);
+    w = table[k];
+    return w.nr > 0;
+  };
+
+  if (warp == 0) {
+    // ===== TMA: per tile the chunks outside the half first (the scores take them first), then the half's own =====
+    const bool issuer = elect_one();
+    if (issuer) asm volatile("prefetch.tensormap [%0];" ::"l"(&map) : "memory");
+    int st = 0, sl = 0;
+    uint32_t st_ph = 1, sl_ph = 1;   // parity of the release that a slot's next load waits for (the first round finds it free)
+    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
+      LtItem w;
+      if (!next_item(it, w)) continue;
+      const int own = w.half ? own1 : own0, first = w.half * 4, rest = chunks - own;
+      const int32_t* bt = p.block_table + (int64_t)w.seq * p.bt_stride;
+      for (int i = w.tile_lo; i < w.tile_hi; ++i) {
+        const int tok = i * kLtKeys;
+        const int blk = __shfl_sync(0xffffffffu, __ldg(bt + tok / p.block_size), 0);
+        const int row = blk * p.block_size + tok % p.block_size;
+        for (int c = 0; c < rest; ++c) {
+          mbar_wait(rest_free + sl, sl_ph);
+          if (issuer) {
+            mbar_expect_tx(rest_full + sl, kLtChunk);
+            tma_load_2d(rest_ring + sl * kLtChunk, &map, (c < first ? c : c + own) * 64, row, rest_full + sl);
+          }
+          if (++sl == p.rest_slots) sl = 0, sl_ph ^= 1;
+        }
+        mbar_wait(own_free + st, st_ph);
+        if (issuer) {
+          mbar_expect_tx(own_full + st, own * kLtChunk);
+          for (int c = 0; c < own; ++c) tma_load_2d(own_ring + (st * max_own + c) * kLtChunk, &map, (first + c) * 64, row, own_full + st);
+        }
+        __syncwarp();
+        if (++st == p.own_stages) st = 0, st_ph ^= 1;
+      }
+    }
+  } else if (warp == 1) {
+    // ===== MMA: the scores of tile n + 1 are issued before the weights of tile n are waited for =====
+    const bool issuer = elect_one();
+    const uint64_t desc_q = make_desc(smem_u32(qs), 16, 1024), desc_own = make_desc(smem_u32(own_ring), 16, 1024),
+                   desc_rest = make_desc(smem_u32(rest_ring), 16, 1024), desc_v = make_desc(smem_u32(own_ring), kLtChunk, 1024);
+    int st = 0, sl = 0, pv_st = 0;   // own stage and rest slot of the next scores, own stage of the next second product
+    uint32_t st_ph = 0, sl_ph = 0;
+    int n = 0, active = 0;
+    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
+      LtItem w;
+      if (!next_item(it, w)) continue;
+      const int nt = __shfl_sync(0xffffffffu, w.tile_hi - w.tile_lo, 0);
+      if (nt <= 0) continue;
+      const int half = __shfl_sync(0xffffffffu, w.half, 0);
+      const int own = half ? own1 : own0, first = half * 4, rest = chunks - own;
+      const uint32_t id_s = idesc_bf16(kLtKeys, 0), id_o = idesc_bf16(half ? width1 : width0, 1);
+      auto issue_s = [&](int n) {
+        const uint32_t d = tmem + kTmS + (n & 1) * kLtKeys;
+        for (int c = 0; c < rest; ++c) {
+          const int col = c < first ? c : c + own, ks = min(4, ksteps - col * 4);
+          mbar_wait(rest_full + sl, sl_ph);
+          fence_after();
+          const uint64_t da = desc_q + (uint64_t)((c * kLtQChunk) >> 4), db = desc_rest + (uint64_t)((sl * kLtChunk) >> 4);
+          const uint32_t acc = c ? 1u : 0u;
+          if (issuer) {
+            if (ks == 4) {   // unrolled: descriptors stay a uniform base plus a constant
+#pragma unroll
+              for (int j = 0; j < 4; ++j) mma_ss(d, da + j * 2, db + j * 2, id_s, j ? 1u : acc);
+            } else {
+              for (int j = 0; j < ks; ++j) mma_ss(d, da + j * 2, db + j * 2, id_s, j ? 1u : acc);
+            }
+            commit(rest_free + sl);
+          }
+          __syncwarp();
+          if (++sl == p.rest_slots) sl = 0, sl_ph ^= 1;
+        }
+        mbar_wait(own_full + st, st_ph);
+        fence_after();
+        if (issuer) {
+          const uint64_t dk = desc_own + (uint64_t)((st * max_own * kLtChunk) >> 4);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            if (c >= own) break;
+            const int ks = min(4, ksteps - (first + c) * 4);
+            const uint32_t acc = c || rest ? 1u : 0u;
+            if (ks == 4) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) mma_ts(d, tmem + kTmQ + c * 32 + j * 8, dk + ((c * kLtChunk) >> 4) + j * 2, id_s, j ? 1u : acc);
+            } else {
+              for (int j = 0; j < ks; ++j) mma_ts(d, tmem + kTmQ + c * 32 + j * 8, dk + ((c * kLtChunk) >> 4) + j * 2, id_s, j ? 1u : acc);
+            }
+          }
+          commit(s_full + (n & 1));
+        }
+        __syncwarp();
+        if (++st == p.own_stages) st = 0, st_ph ^= 1;
+      };
+      mbar_wait(q_ready, active & 1);
+      fence_after();
+      issue_s(n);
+      if (nt == 1 && issuer) commit(q_free);
+      for (int i = 0; i < nt; ++i, ++n) {
+        if (i + 1 < nt) {
+          issue_s(n + 1);
+          if (i + 2 == nt && issuer) commit(q_free);   // the item's last scores are on their way
+        }
+        mbar_wait(p_ready + (n & 1), (n >> 1) & 1);
+        fence_after();
+        const uint64_t dv = desc_v + (uint64_t)((pv_st * max_own * kLtChunk) >> 4);
+        if (issuer) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)   // 16 keys per step
+            mma_ts(tmem, tmem + kTmS + (n & 1) * kLtKeys + j * 8, dv + (uint64_t)((j * 2048) >> 4), id_o, (i | j) ? 1u : 0u);
+          commit(own_free + pv_st);
+          commit(o_full + (n & 1));
+        }
+        __syncwarp();
+        if (++pv_st == p.own_stages) pv_st = 0;
+      }
+      ++active;
+    }
+  } else if (warp >= 6) {
+    // ===== queries of the next item: fp32 rows -> bf16, the half's own columns to TMEM, the others to shared memory.  Two warps
+    // per quarter of the pairs, the chunks dealt alternately.  The own part travels into registers while the item before is still
+    // computed; the shared-memory part follows once its last scores have been taken. =====
+    const int quad = warp & 3, sub = (warp - 6) >> 2;
+    int active = 0;
+    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
+      LtItem w;
+      if (!next_item(it, w) || w.tile_hi <= w.tile_lo) continue;
+      const int own = w.half ? own1 : own0, first = w.half * 4, rest = chunks - own;
+      const int live = w.nr * p.heads;
+      const float* qbase = p.q + (int64_t)w.t0 * p.heads * p.krow;   // pair m = (row m / heads, head m % heads): row m of this
+      // four lanes take 64 neighbouring bytes of a row, eight rows per load: the fragment layout of the 16-lane store
+      uint32_t r[2][2][16];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int c = sub + 2 * k;
+#pragma unroll
+        for (int hl = 0; hl < 2; ++hl) {
+          float4 v[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {   // piece j / 2 of 16 columns, rows x / 4 (j even) and x / 4 + 8
+            const int col = (first + c) * 64 + (j >> 1) * 16 + (lane & 3) * 4, mm = quad * 32 + hl * 16 + (j & 1) * 8 + (lane >> 2);
+            v[j] = c < own && mm < live && col < p.krow ? __ldg(reinterpret_cast<const float4*>(qbase + (int64_t)mm * p.krow + col))
+                                                        : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            r[k][hl][2 * j] = pack_bf16(v[j].x, v[j].y);
+            r[k][hl][2 * j + 1] = pack_bf16(v[j].z, v[j].w);
+          }
+        }
+      }
+      if (active > 0) mbar_wait(q_free, (active - 1) & 1);
+      fence_after();
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        if (sub + 2 * k < own) {
+          const uint32_t a = tmem + kTmQ + (sub + 2 * k) * 32 + ((uint32_t)(quad * 32) << 16);
+          st_16x256b_x4(a, r[k][0]);
+          st_16x256b_x4(a + (16u << 16), r[k][1]);
+        }
+      // eight lanes per row of a chunk (16-byte pieces), four rows per step
+      for (int c = sub; c < rest; c += 2) {
+        const int col = (c < first ? c : c + own) * 64 + (lane & 7) * 8;
+        float4 v[16];
+#pragma unroll
+        for (int r4 = 0; r4 < 8; ++r4) {
+          const int mm = quad * 32 + r4 * 4 + (lane >> 3);
+          const bool ok = mm < live && col < p.krow;
+          const float4* src = reinterpret_cast<const float4*>(qbase + (int64_t)mm * p.krow + col);
+          v[2 * r4] = ok ? __ldg(src) : make_float4(0.f, 0.f, 0.f, 0.f);
+          v[2 * r4 + 1] = ok ? __ldg(src + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int r4 = 0; r4 < 8; ++r4) {
+          const int mm = quad * 32 + r4 * 4 + (lane >> 3);
+          const float4 a = v[2 * r4], b = v[2 * r4 + 1];
+          *reinterpret_cast<uint4*>(qs + c * kLtQChunk + (mm >> 3) * 1024 + (mm & 7) * 128 + (((lane & 7) ^ (mm & 7)) << 4)) =
+              make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
+        }
+      }
+      st_wait();
+      fence_async_smem();
+      fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(q_ready);
+      ++active;
+    }
+  } else {
+    // ===== softmax and output: a thread owns a pair =====
+    const int quad = warp & 3, m = quad * 32 + lane;
+    const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
+    const int r = m / p.heads, h = m % p.heads;
+    const float sc2 = p.scale * 1.4426950408889634f;   // scores in the log2 domain
+    int n = 0;
+    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
+      LtItem w;
+      if (!next_item(it, w)) continue;
+      const bool alive = r < w.nr;
+      const int ctx = alive ? w.ctx0 + r : 0, lo = p.window > 0 ? max(ctx - p.window, 0) : 0;
+      const int width = w.half ? width1 : width0, own = w.half ? own1 : own0;
+      float mu = -INFINITY, l = 0.f;
+      for (int i = w.tile_lo; i < w.tile_hi; ++i, ++n) {
+        const int base = i * kLtKeys;
+        mbar_wait(s_full + (n & 1), (n >> 1) & 1);
+        fence_after();
+        const uint32_t s_addr = tmem + lane_off + kTmS + (n & 1) * kLtKeys;
+        uint32_t s[64];
+        ld32(s_addr, s);
+        ld32(s_addr + 32, s + 32);
+        ld_wait<64>(s);
+        const int j_lo = lo - base, j_hi = ctx - base;   // live columns [j_lo, j_hi)
+        if (__any_sync(0xffffffffu, j_lo > 0 || j_hi < kLtKeys)) {
+#pragma unroll
+          for (int j = 0; j < 64; ++j)
+            if (j < j_lo || j >= j_hi) s[j] = 0xff800000u;   // -inf
+        }
+        float mx = -INFINITY;
+#pragma unroll
+        for (int j = 0; j < 64; ++j) mx = fmaxf(mx, __uint_as_float(s[j]));
+        mx *= sc2;
+        const bool jump = mx > mu + 8.f;   // also the first live key (mu = -inf)
+        if (__any_sync(0xffffffffu, jump)) {
+          const float mn = jump ? mx : mu, f = jump && mu != -INFINITY ? exp2_fast(mu - mn) : 1.f;
+          if (i > w.tile_lo) {
+            mbar_wait(o_full + ((n - 1) & 1), ((n - 1) >> 1) & 1);
+            fence_after();
+            if (__any_sync(0xffffffffu, f != 1.f))
+              for (int c = 0; c < width; c += 16) {
+                uint32_t o[16];
+                ld16(tmem + lane_off + c, o);
+                ld_wait<16>(o);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
+                st16(tmem + lane_off + c, o);
+              }
+          }
+          l *= f;
+          mu = mn;
+        }
+        const float mref = mu > -INFINITY ? mu : 0.f;
+        float sum = 0.f;
+        uint32_t pk[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const float p0 = exp2_fast(fmaf(__uint_as_float(s[2 * j]), sc2, -mref)), p1 = exp2_fast(fmaf(__uint_as_float(s[2 * j + 1]), sc2, -mref));
+          pk[j] = pack_bf16(p0, p1);
+          sum += bf16lo(pk[j]) + bf16hi(pk[j]);   // the weights as the second product takes them: what rounding adds to all cancels
+        }
+        l += sum;
+        st32(s_addr, pk);
+        const int n_valid = w.ctx_max - base;
+        if (n_valid < kLtKeys) {
+          // value rows past the context may hold anything, and 0 * NaN = NaN: zero them under their zero weights
+          const int st = n % p.own_stages;
+          mbar_wait(own_full + st, (n / p.own_stages) & 1);
+          unsigned char* vb = own_ring + st * max_own * kLtChunk;
+          for (int c = 0; c < own; ++c)
+            for (int e = n_valid * 8 + m; e < kLtKeys * 8; e += 128) *reinterpret_cast<uint4*>(vb + c * kLtChunk + e * 16) = make_uint4(0u, 0u, 0u, 0u);
+          fence_async_smem();
+        }
+        st_wait();
+        fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_ready + (n & 1));
+      }
+      const bool any = w.tile_hi > w.tile_lo;
+      if (any) {
+        mbar_wait(o_full + ((n - 1) & 1), ((n - 1) >> 1) & 1);
+        fence_after();
+      }
+      const int64_t pair = (int64_t)(w.t0 + r) * p.heads + h;
+      if (p.n_splits > 1) {
+        // unnormalised sums [pair][split][rank | maximum | denominator], the maximum in natural units
+        float* dst = p.part + (pair * p.n_splits + w.split) * (p.rank + 2);
+        if (alive && w.half == 0) {
+          dst[p.rank] = mu * 0.6931471805599453f;
+          dst[p.rank + 1] = l;
+        }
+        for (int c = 0; c < width; c += 16) {
+          uint32_t o[16];
+          if (any) {
+            ld16(tmem + lane_off + c, o);
+            ld_wait<16>(o);
+          }
+          if (alive) {
+            float2* d2 = reinterpret_cast<float2*>(dst + w.half * 256 + c);   // rank + 2 is even: 8-byte aligned rows
+#pragma unroll
+            for (int j = 0; j < 8; ++j) d2[j] = any ? make_float2(__uint_as_float(o[2 * j]), __uint_as_float(o[2 * j + 1])) : make_float2(0.f, 0.f);
+          }
+        }
+      } else {
+        float f = 1.f;
+        if (p.sink != nullptr && alive) {   // one more term of the denominator
+          const float sk = __ldg(p.sink + h) * 1.4426950408889634f, mn = fmaxf(mu, sk);
+          f = exp2_fast(mu - mn);
+          l = l * f + exp2_fast(sk - mn);
+        }
+        const float inv = l > 0.f ? f / l : 0.f;
+        __nv_bfloat16* dst = p.out + pair * p.rank + w.half * 256;
+        for (int c = 0; c < width; c += 16) {
+          uint32_t o[16], v[8];
+          if (any) {
+            ld16(tmem + lane_off + c, o);
+            ld_wait<16>(o);
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] = any ? pack_bf16(__uint_as_float(o[2 * j]) * inv, __uint_as_float(o[2 * j + 1]) * inv) : 0u;
+          if (alive) store_sector(dst + c, v);   // rank % 16 == 0: whole sectors
+        }
+      }
+      fence_before();
+      // all four warps have read O before any of them hands over the next item's first weights (whose product restarts O):
+      // the hand-over needs an arrival of every warp
+    }
+  }
+  fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+  }
+}
+
+struct LtShape {
+  int halves, own_stages, rest_slots;
+};
+// false: a shape whose queries or key tiles do not fit beside each other.  Three stages of value columns keep the loads of a tile
+// (freed by its second product) off the chain of the next ones (2 048 rows of 16 heads, 512 + 64: 2.2 us a tile with two stages);
+// the other chunks are freed earlier, a tile and one chunk of them is enough.
+bool lt_shape(int heads, int krow, int rank, LtShape& s) {
+  if (heads < 1 || heads > kLtPairs || krow % 16 || rank % 16 || rank < 16 || rank > 512 || rank > krow) return false;
+  s.halves = rank > 256 ? 2 : 1;
+  const int chunks = (krow + 63) / 64, own0 = (std::min(rank, 256) + 63) / 64, own1 = s.halves > 1 ? (rank - 256 + 63) / 64 : own0;
+  const int max_rest = chunks - std::min(own0, own1), max_own = std::max(own0, own1);
+  if (max_rest > kLtMaxRest) return false;
+  const int slots = (kLtSmem - 1024 - kLtTail - max_rest * kLtQChunk) / kLtChunk;
+  for (s.own_stages = kLtMaxStages; s.own_stages >= 2; --s.own_stages) {
+    s.rest_slots = std::min(slots - s.own_stages * max_own, kLtMaxSlots);
+    if (s.rest_slots >= max_rest + 1) return true;
+  }
+  return false;
+}
+
+}  // namespace
+
+bool latent_attn_tc_supported(int heads, int krow, int rank, int block_size) {
+  LtShape s;
+  return block_size > 0 && block_size % kLtKeys == 0 && lt_shape(heads, krow, rank, s);
+}
+
+// one launch over the step's run list; part given: n_splits CTAs per item leave unnormalised sums (the caller merges)
+int latent_attn_tc(const float* q, const __nv_bfloat16* kc, const int32_t* block_table, int bt_stride, const int32_t* row_to_seq,
+                   const int32_t* ctx_lens, __nv_bfloat16* out, const int32_t* runs, const int32_t* n_runs, int T, int heads, int krow,
+                   int rank, int block_size, float scale, const float* sink, cudaStream_t s, int n_splits, float* part, int window) {
+  LtShape sh;
+  B200_REQUIRE(latent_attn_tc_supported(heads, krow, rank, block_size) && lt_shape(heads, krow, rank, sh), B200_ERR_UNSUPPORTED,
+               "latent_attn_tc: shape %d / %d / %d", heads, krow, rank);
+  CUtensorMap map;
+  const int rc = get_tensor_map_2d(kc, 1ull << 31, krow, krow, kLtKeys, &map);   // rows touched come from the block table
+  if (rc) return rc;
+  LtParams p = {};
+  p.q = q;
+  p.block_table = block_table;
+  p.row_to_seq = row_to_seq;
+  p.ctx_lens = ctx_lens;
+  p.runs = runs;
+  p.n_runs = n_runs;
+  p.sink = sink;
+  p.out = out;
+  p.part = part;
+  p.n_rows = T;
+  p.bt_stride = bt_stride;
+  p.heads = heads;
+  p.krow = krow;
+  p.rank = rank;
+  p.block_size = block_size;
+  p.n_splits = n_splits;
+  p.window = window;
+  p.own_stages = sh.own_stages;
+  p.rest_slots = sh.rest_slots;
+  p.halves = sh.halves;
+  p.rows_per_item = std::min(kLtPairs / heads, 16);   // a run has at most 16 rows
+  p.items_per_run = (16 + p.rows_per_item - 1) / p.rows_per_item;
+  p.scale = scale;
+  static bool done[64] = {};
+  B200_CUDA(ensure_dynamic_smem(latent_attn_tc_kernel, kLtSmem, done));
+  const int64_t most = (int64_t)T * p.items_per_run * n_splits * sh.halves;   // upper bound; the kernel reads the real count
+  B200_CUDA(launch(latent_attn_tc_kernel, dim3((unsigned)std::min<int64_t>(most, kNumSMs)), dim3(kLtThreads), (size_t)kLtSmem, s, map, p));
+  return B200_OK;
+}
+
+}  // namespace b200
