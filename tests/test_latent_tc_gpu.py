@@ -1,0 +1,65 @@
+"""The tcgen05 form of latent attention (cache blocks of whole 64-key tiles) against the same attention in float64."""
+import pytest
+import torch
+
+from conftest import pkg
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _oracle(q, rows, ctx, rank, scale, sink, window):
+    lo = max(ctx - window, 0) if window else 0
+    s = (q @ rows[lo:ctx].T) * scale
+    m = s.max(-1, keepdim=True).values
+    m = torch.maximum(m, sink[:, None]) if sink is not None else m
+    e = torch.exp(s - m)
+    den = e.sum(-1, keepdim=True) + (torch.exp(sink[:, None] - m) if sink is not None else 0.0)
+    return (e / den) @ rows[lo:ctx, :rank]
+
+
+# heads: one, a count that leaves pairs idle (5 x 16 rows = 80 of 128), the tile's own divisor, more rows than a run (1), all pairs one row (128).
+# rank / rotated part: one half with a partial last chunk, two halves, the second half short, everything in TMEM (rank = row), a key row of
+# nine chunks
+@pytest.mark.parametrize("heads,rank,rd,bs,splits,window,with_sink", [
+    (16, 512, 64, 128, 1, 0, True), (16, 512, 64, 64, 3, 0, True), (5, 256, 32, 128, 1, 0, False), (1, 16, 16, 128, 16, 0, False),
+    (128, 64, 0, 128, 1, 0, True), (16, 304, 16, 64, 2, 0, False), (16, 256, 0, 128, 1, 100, True), (7, 80, 48, 192, 1, 64, False)])
+def test_latent_attention_tile_edges(heads, rank, rd, bs, splits, window, with_sink):
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    g = torch.Generator().manual_seed(heads * 1000 + rank)
+    krow, n_tok, scale = rank + rd, 700, 0.6 / (rank + rd) ** 0.5
+    nb = (n_tok + bs - 1) // bs
+    rows = torch.randn(n_tok, krow, generator=g).to(torch.bfloat16)
+    perm = torch.randperm(nb + 3, generator=g)[:nb]
+    # decode rows of sequences of their own around tile and block edges, then two runs that start inside a tile
+    ctxs = [1, 2, 63, 64, 65, 127, 128, 129, 700] + list(range(1, 39)) + list(range(650, 700))
+    seq = list(range(9)) + [9] * 38 + [10] * 50
+    T = len(ctxs)
+    q = (torch.randn(T, heads, krow, generator=g) * 4).to(torch.bfloat16).float()   # large scores: the running maximum jumps
+    sink = torch.randn(heads, generator=g) * 2 if with_sink else None
+    want = torch.stack([_oracle(q[t].double(), rows.double(), ctxs[t], rank, scale, sink.double() if with_sink else None, window) for t in range(T)])
+    # every sequence reads the same first n_tok rows through its own table; what lies past a context is poison where nobody may look
+    kc = torch.full((nb + 3, 1, bs, krow), float("nan"), dtype=torch.bfloat16)
+    for j in range(n_tok):
+        kc[perm[j // bs], 0, j % bs] = rows[j]
+    dev = lambda t: t.to(DEV).contiguous()   # noqa: E731
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)   # noqa: E731
+    bt = dev(perm.to(torch.int32)[None, :].repeat(11, 1))
+    ws = torch.zeros(int(lib.b200_paged_attn_anydim_workspace_bytes(T)), dtype=torch.uint8, device=DEV)
+    out = torch.full((T, heads, rank), float("nan"), dtype=torch.bfloat16, device=DEV)
+    part = torch.full((T * heads * splits * (rank + 2),), float("nan"), device=DEV)
+    qd, kd, sd, sq, cx = dev(q), dev(kc), dev(sink) if with_sink else None, i32(seq), i32(ctxs)
+    sp = sd.data_ptr() if with_sink else None
+    if window:
+        check(lib.b200_latent_attn_window(qd.data_ptr(), kd.data_ptr(), bt.data_ptr(), nb, sq.data_ptr(), cx.data_ptr(), out.data_ptr(), T, heads, krow,
+                                          rank, bs, scale, sp, ws.data_ptr(), window, None))
+    else:
+        check(lib.b200_latent_attn(qd.data_ptr(), kd.data_ptr(), bt.data_ptr(), nb, sq.data_ptr(), cx.data_ptr(), out.data_ptr(), T, heads, krow, rank,
+                                   bs, scale, sp, ws.data_ptr(), splits, part.data_ptr() if splits > 1 else None, None))
+    torch.cuda.synchronize()
+    got = out.double().cpu()
+    assert torch.isfinite(got).all()
+    # queries are exact in bf16; weights and results are rounded once each (2^-9 relative, rms 2^-9 / sqrt 3 apiece), the sum over keys only
+    # averages the weights' part: below 2^-8 in the 2-norm, and no single result further off than the weights' worst case, 2^-8 of the largest value
+    assert (got - want).norm() / want.norm() < 2.0 ** -8
+    assert (got - want).abs().max() < 2.0 ** -8 * rows.float().abs().max() + 2.0 ** -9 * want.abs().max()
