@@ -1,0 +1,89 @@
+"""The recurrences' kernels at the edges of their stages and chunks, against the same recurrence row by row in float64."""
+import pytest
+import torch
+
+from conftest import pkg
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _i32(x):
+    return torch.tensor(x, dtype=torch.int32, device=DEV)
+
+
+def _mlstm(x, gates, state, heads, dim, vdim):
+    """Rows x [n][2 hd + hv], log gates, state (S [heads][vdim][dim], n [heads][dim], m [heads]) -> outputs, what one relative
+    error of all terms of a sum can do to them, new state; float64."""
+    S, nn, m = (t.clone() for t in state)
+    hd, out, span = heads * dim, [], []
+    for t in range(x.shape[0]):
+        q = x[t, :hd].reshape(heads, dim) * dim ** -0.5
+        k, v = x[t, hd:2 * hd].reshape(heads, dim), x[t, 2 * hd:2 * hd + heads * vdim].reshape(heads, vdim)
+        i, f = gates[t, :heads], gates[t, heads:]
+        mn = torch.maximum(f + m, i)
+        a, b, m = torch.exp(f + m - mn), torch.exp(i - mn), mn
+        S = a[:, None, None] * S + v[:, :, None] * (b[:, None] * k)[:, None, :]
+        nn = a[:, None] * nn + b[:, None] * k
+        den = torch.maximum((nn * q).sum(-1).abs(), torch.exp(-m)) + 1e-6
+        o = (S @ q[:, :, None])[..., 0] / den[:, None]
+        out.append(o.reshape(-1))
+        span.append(((S.abs() @ q.abs()[:, :, None])[..., 0] / den[:, None] + o.abs() * ((nn * q).abs().sum(-1) / den)[:, None]).reshape(-1))
+    return torch.stack(out), torch.stack(span), (S, nn, m)
+
+
+# portions of two sequences, several steps: one row, less than a stage of 16, around 64-row chunks, several chunks; the second slot starts dirty
+STEPS = [([3], [70]), ([1], [64]), ([15, 66], [1, 2]), ([130], [16])]
+
+
+@pytest.mark.parametrize("f32,heads,dim,vdim,pad", [(0, 2, 128, 64, 0), (0, 3, 64, 40, 0), (0, 1, 40, 24, 0), (0, 2, 16, 8, 8), (0, 2, 36, 20, 0),
+                                                    (0, 1, 128, 48, 4), (0, 1, 200, 32, 0), (1, 2, 128, 32, 0), (1, 1, 50, 7, 0)])
+def test_mlstm_scan_portions_and_hard_gates(f32, heads, dim, vdim, pad):
+    """pad: columns of other data behind a row (4: rows that do not start at 16-byte addresses)."""
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    g = torch.Generator().manual_seed(dim * 10 + vdim)
+    adt = torch.float32 if f32 else torch.bfloat16
+    hd, hv, nz = heads * dim, heads * vdim, (vdim + 31) // 32
+    floats, ld = int(lib.b200_mlstm_state_floats(heads, dim, vdim)), 2 * hd + hv + pad
+    assert floats == heads * vdim * dim + heads * nz * dim + heads * nz
+    stride = floats + 6
+    state = torch.full((4, stride), 7.5, device=DEV)                      # whatever a slot held: a sequence at position 0 starts from zeros
+    slots, pos = [2, 0], [0, 0]
+    oracle = [tuple(torch.zeros(s, dtype=torch.float64) for s in ((heads, vdim, dim), (heads, dim), (heads,))) for _ in range(2)]
+    for a, b in STEPS:
+        for cuts in (list(zip(a, b)) if len(a) == len(b) else [(a[0], b[0])]):
+            T = sum(cuts)
+            x = torch.randn(T, ld, generator=g).to(adt)
+            gates = torch.randn(T, 2 * heads, generator=g) * 2
+            gates[:, heads:] = torch.nn.functional.logsigmoid(gates[:, heads:] + 3)
+            if T > 20:
+                gates[11, heads:] = -14.9      # all but forgotten
+                gates[17, :heads] = 14.0       # a row that dwarfs what is there
+                gates[18:, :heads] -= 6.0
+            start = [0, cuts[0], T]
+            out = torch.full((T, hv), float("nan"), device=DEV)
+            xd, gd = x.to(DEV), gates.to(DEV)
+            p = list(range(pos[0], pos[0] + cuts[0])) + list(range(pos[1], pos[1] + cuts[1]))
+            ptd, std, sld = _i32(p), _i32(start), _i32(slots)
+            check(lib.b200_mlstm_scan(f32, xd.data_ptr(), ld, 0, hd, 2 * hd, gd.data_ptr(), ptd.data_ptr(), std.data_ptr(), sld.data_ptr(),
+                                      state.data_ptr(), stride, out.data_ptr(), 2, heads, dim, vdim, None))
+            torch.cuda.synchronize()
+            for s in range(2):
+                lo, hi = start[s], start[s + 1]
+                want, span, oracle[s] = _mlstm(x[lo:hi].double(), gates[lo:hi].double(), oracle[s], heads, dim, vdim)
+                got = out[lo:hi].double().cpu()
+                # row by row, f + m - m' is rounded twice in fp32 at |f| + |m| < 32 (2^-20 each): 2e-6 of a weight a row, a few rows' worth lives on;
+                # the chunks take these sums in 64 bits.  The division magnifies what happens to a small |n . q|, so the results are held to what
+                # such an error of every term could do to them
+                tol = 2e-6 if not f32 and dim % 8 == 0 and dim <= 128 and vdim % 8 == 0 and pad % 8 == 0 else 1e-5
+                assert ((got - want).abs() <= tol * span + 1e-7 * want.abs()).all(), (cuts, s, float(((got - want).abs() / span).max()))
+                st = state[slots[s]].double().cpu()
+                S = st[:heads * vdim * dim].reshape(heads, vdim, dim)
+                n = st[heads * vdim * dim:heads * vdim * dim + heads * nz * dim].reshape(heads, nz, dim)
+                m = st[heads * vdim * dim + heads * nz * dim:floats].reshape(heads, nz)
+                for z in range(nz):
+                    assert (n[:, z] - oracle[s][1]).norm() < tol * oracle[s][1].norm() and (m[:, z] - oracle[s][2]).abs().max() < 1e-5
+                assert (S - oracle[s][0]).norm() < tol * oracle[s][0].norm()
+                assert (st[floats:] == 7.5).all()
+                pos[s] += cuts[s]
+    assert (state[[1, 3]] == 7.5).all()
