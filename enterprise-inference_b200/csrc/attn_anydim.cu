@@ -157,18 +157,20 @@ constexpr int kTcThreads = 256;
 // One CTA of 1024 threads.  Row t opens a segment when it is the step's first row, belongs to another sequence than row
 // t - 1, or does not continue its context length by one; inside a segment a run starts every kRunRows rows.  Per chunk of
 // 1024 rows: an inclusive max-scan carries every row's segment start, a prefix sum of the run starts gives each run its place.
+// Lists of runs of at most 16, 32, .. 16 << (kRunLists - 1) rows are made in the same pass (list k at runs + 2 T k, its length at
+// n_runs[k]): the five prefix sums of a chunk travel in one 64-bit word, 12 bits each.
 __global__ void __launch_bounds__(1024)
 attn_runs_plan_kernel(const int32_t* __restrict__ row_to_seq, const int32_t* __restrict__ ctx_lens, int T, int32_t* __restrict__ runs,
                       int32_t* __restrict__ n_runs) {
-  __shared__ int wseg[32], wcnt[32];
-  __shared__ int carry_seg, carry_cnt;
+  __shared__ int wseg[32];
+  __shared__ uint64_t wcnt[32];
+  __shared__ int carry_seg, carry_cnt[kRunLists];
+  static_assert(kRunRows == 16 && kRunLists * 12 <= 64, "run lists");
   pdl_wait();
   pdl_launch_dependents();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) {
-    carry_seg = 0;
-    carry_cnt = 0;
-  }
+  if (tid == 0) carry_seg = 0;
+  if (tid < kRunLists) carry_cnt[tid] = 0;
   __syncthreads();
   for (int c0 = 0; c0 < T; c0 += 1024) {
     const int t = c0 + tid;
@@ -185,29 +187,40 @@ attn_runs_plan_kernel(const int32_t* __restrict__ row_to_seq, const int32_t* __r
     int before = carry_seg;
     for (int w = 0; w < warp; ++w) before = max(before, wseg[w]);
     seg = max(seg, before);
-    const bool starts = live && (t - seg) % kRunRows == 0;
-    int cnt = starts ? 1 : 0;                     // inclusive prefix count of run starts
+    uint64_t mine = 0, cnt;                       // the lists in which a run starts here; inclusive prefix counts
+#pragma unroll
+    for (int k = 0; k < kRunLists; ++k) mine |= (uint64_t)(live && (t - seg) % (kRunRows << k) == 0 ? 1 : 0) << (12 * k);
+    cnt = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, cnt, o);
+      const uint64_t v = __shfl_up_sync(0xffffffffu, cnt, o);
       if (lane >= o) cnt += v;
     }
     if (lane == 31) wcnt[warp] = cnt;
     __syncthreads();
-    int base = carry_cnt;
-    for (int w = 0; w < warp; ++w) base += wcnt[w];
-    if (starts) runs[2 * (base + cnt - 1)] = t;
+    for (int w = 0; w < warp; ++w) cnt += wcnt[w];
+    int total[kRunLists];
+#pragma unroll
+    for (int k = 0; k < kRunLists; ++k) {
+      total[k] = carry_cnt[k] + (int)((cnt >> (12 * k)) & 0xfff);
+      if ((mine >> (12 * k)) & 1) runs[(int64_t)2 * T * k + 2 * (total[k] - 1)] = t;
+    }
     __syncthreads();
     if (tid == 1023) {
       carry_seg = seg;
-      carry_cnt = base + cnt;
+#pragma unroll
+      for (int k = 0; k < kRunLists; ++k) carry_cnt[k] = total[k];
     }
     __syncthreads();
   }
   // lengths: a run ends where the next one starts
-  const int n = carry_cnt;
-  for (int i = tid; i < n; i += 1024) runs[2 * i + 1] = (i + 1 < n ? runs[2 * (i + 1)] : T) - runs[2 * i];
-  if (tid == 0) *n_runs = n;
+#pragma unroll
+  for (int k = 0; k < kRunLists; ++k) {
+    const int n = carry_cnt[k];
+    int32_t* list = runs + (int64_t)2 * T * k;
+    for (int i = tid; i < n; i += 1024) list[2 * i + 1] = (i + 1 < n ? list[2 * (i + 1)] : T) - list[2 * i];
+    if (tid == 0) n_runs[k] = n;
+  }
 }
 
 template <typename CT, typename AT>
@@ -338,9 +351,9 @@ paged_attn_runs_kernel(const float* __restrict__ q, const CT* __restrict__ kc, c
 
 }  // namespace
 
-int64_t paged_attn_anydim_workspace_bytes(int T) { return ((int64_t)2 * T + 8) * 4; }
+int64_t paged_attn_anydim_workspace_bytes(int T) { return ((int64_t)2 * T * kRunLists + 8) * 4; }
 
-// The run list of a step in ws (n_runs at ws[0], (first row, rows) pairs from ws[8]): what plan = 1 builds, as a call of its
+// The run lists of a step in ws (lengths at ws[0..], (first row, rows) pairs from ws[8]): what plan = 1 builds, as a call of its
 // own for the kernels that share it.
 int paged_attn_runs_plan(const int32_t* row_to_seq, const int32_t* ctx_lens, int T, void* ws, cudaStream_t s) {
   int32_t* runs = static_cast<int32_t*>(ws) + 8;

@@ -412,6 +412,19 @@ int paged_attn_mma(const float* q, const __nv_bfloat16* kc, const __nv_bfloat16*
   if (T == 0) return B200_OK;
   B200_REQUIRE(vc && paged_attn_mma_supported(heads, kv_heads, dim, vdim), B200_ERR_UNSUPPORTED, "paged_attn_mma: shape %d / %d / %d / %d", heads,
                kv_heads, dim, vdim);
+  if (n_splits < 1 || part == nullptr) n_splits = 1;
+  B200_REQUIRE(n_splits <= kLaMaxSplits, B200_ERR_INVALID, "attention: %d splits (at most %d)", n_splits, kLaMaxSplits);
+  const auto at = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr); };
+  B200_REQUIRE(at(kc) % 16 == 0 && at(vc) % 16 == 0, B200_ERR_INVALID, "attention: cache not 16-byte aligned");
+  // as for latent rows: tcgen05 wherever the shape fits, wider heads, smaller blocks and odd addresses stay here
+  if (attn_rows_tc_supported(heads, kv_heads, dim, vdim, block_size) && at(q) % 16 == 0 && at(out) % 16 == 0 && at(part) % 8 == 0) {
+    const int rc = attn_rows_tc_runs(q, kc, vc, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, kv_heads, dim, vdim,
+                                     block_size, scale, sink, s, n_splits, part, window, ex);
+    if (rc || n_splits == 1) return rc;
+    B200_CUDA(launch(latent_attn_merge_kernel, dim3((T * heads + 3) / 4), dim3(128), (size_t)0, s, (const float*)part, out, T * heads, heads,
+                     vdim, n_splits, sink, static_cast<const __nv_bfloat16*>(ex.gate), ex.ldg));
+    return B200_OK;
+  }
   return attn_mma_launch(q, kc, vc, kv_heads, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, dim, vdim, block_size,
                          scale, sink, s, n_splits, part, window, ex);
 }

@@ -11,11 +11,12 @@
 // staging and the output at an item's ends.  Q is the large operand (krow 576: 147 KB of bf16), so the part that matches the value
 // columns lives in TMEM (columns 384..511, A operand read from there) and only the rest in shared memory, which leaves room for
 // three stages of value columns and a tile of the other columns.  TMEM: O 0..255, two score buffers of 64 columns, the Q part.
-// The weights overwrite the scores in place (bf16 pairs, A operand of the second product) and never touch shared memory.
+// The weights overwrite the scores in place (A operand of the second product, per 32 scores 16 columns of bf16 pairs and 16 of what
+// rounding took from them) and never touch shared memory.
 // Against the mma.sync kernel of attn_latent.cu with 16 pairs a CTA, which reads every key tile once per row: 2 048 rows of 16
-// heads over 512 + 64 at contexts 1..2048 907 -> 183 us, 64 decode rows at contexts 500..1000 98 -> 47 us; error against 64 bits
-// 2.57e-3 -> 2.60e-3 and 2.65e-3 -> 2.71e-3 (0.98 to 1.03 of the other kernel's over other sizes: both round queries, weights
-// and results to bf16).
+// heads over 512 + 64 at contexts 1..2048 907 -> 201 us, 64 decode rows at contexts 500..1000 98 -> 53 us; error against 64 bits
+// 2.57e-3 -> 2.30e-3 and 2.65e-3 -> 2.37e-3.  (With weights of one bf16 term, as there: 183 and 47 us, but 2.61e-3 and 2.72e-3: the
+// lazily followed maximum costs the exactness of the largest weight.)
 // Warps: TMA producer, MMA issuer, four softmax warps (a thread owns a pair), eight that stage the next item's queries.
 // The running maximum is only followed when it rises by more than 2^8 (the scaling of all terms is the same, so the
 // quotient is exact); a warp then rescales its own 32 rows of O in TMEM.
@@ -251,8 +252,11 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
         const uint64_t dv = desc_v + (uint64_t)((pv_st * max_own * kLtChunk) >> 4);
         if (issuer) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j)   // 16 keys per step
-            mma_ts(tmem, tmem + kTmS + (n & 1) * kLtKeys + j * 8, dv + (uint64_t)((j * 2048) >> 4), id_o, (i | j) ? 1u : 0u);
+          for (int j = 0; j < 4; ++j) {   // 16 keys per step: 8 columns of weights, 16 further those of the second term
+            const uint32_t pa = tmem + kTmS + (n & 1) * kLtKeys + (j >> 1) * 32 + (j & 1) * 8;
+            mma_ts(tmem, pa, dv + (uint64_t)((j * 2048) >> 4), id_o, (i | j) ? 1u : 0u);
+            mma_ts(tmem, pa + 16, dv + (uint64_t)((j * 2048) >> 4), id_o, 1u);
+          }
           commit(own_free + pv_st);
           commit(o_full + (n & 1));
         }
@@ -383,16 +387,21 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
           mu = mn;
         }
         const float mref = mu > -INFINITY ? mu : 0.f;
-        float sum = 0.f;
-        uint32_t pk[32];
+        float sum[2] = {0.f, 0.f};
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const float p0 = exp2_fast(fmaf(__uint_as_float(s[2 * j]), sc2, -mref)), p1 = exp2_fast(fmaf(__uint_as_float(s[2 * j + 1]), sc2, -mref));
-          pk[j] = pack_bf16(p0, p1);
-          sum += bf16lo(pk[j]) + bf16hi(pk[j]);   // the weights as the second product takes them: what rounding adds to all cancels
+        for (int c = 0; c < 2; ++c) {   // per 32 keys 16 columns of bf16 pairs, 16 of what that rounding took
+          uint32_t pk[32];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const float p0 = exp2_fast(fmaf(__uint_as_float(s[c * 32 + 2 * j]), sc2, -mref)), p1 = exp2_fast(fmaf(__uint_as_float(s[c * 32 + 2 * j + 1]), sc2, -mref));
+            sum[j & 1] += p0 + p1;
+            const uint32_t h0 = __float_as_uint(p0) & 0xffff0000u, h1 = __float_as_uint(p1) & 0xffff0000u;
+            pk[j] = __byte_perm(h0, h1, 0x7632);
+            pk[16 + j] = pack_bf16(p0 - __uint_as_float(h0), p1 - __uint_as_float(h1));
+          }
+          st32(s_addr + c * 32, pk);
         }
-        l += sum;
-        st32(s_addr, pk);
+        l += sum[0] + sum[1];
         const int n_valid = w.ctx_max - base;
         if (n_valid < kLtKeys) {
           // value rows past the context may hold anything, and 0 * NaN = NaN: zero them under their zero weights

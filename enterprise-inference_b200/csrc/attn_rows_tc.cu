@@ -1,0 +1,590 @@
+// Paged causal grouped-query attention on tcgen05 for steps with runs of rows, key and value heads of at most 128 entries.
+//
+// The (row, head) pairs of one kv head fill the MMA's M dimension.  A work item is up to two tiles of 128 pairs (consecutive rows of one
+// sequence times the G heads of a kv head) that share every key and value tile of 64 keys:
+//   S_x[128][64] = Q_x . K_tile^T        O_x[128][vdim] += P_x . V_tile           x = the item's first, second tile of pairs
+// The scores of key tile n + 1 are issued before the weights of tile n are waited for (two score buffers per tile of pairs), so the
+// softmax of either tile never waits for the tensor core once the walk is under way: with one tile of pairs and 128 keys (the kernel
+// this one replaces) S -> softmax -> P V was one dependent chain of 1.85 us, and two tiles of pairs with single score buffers of 128
+// keys still took 3.3 us per 128 keys, a tile's softmax (1.7 us) and its own products (1.05 us) one after the other.
+// The weights overwrite the scores in TMEM (A operand of the second product): per 32 scores 16 columns of bf16 pairs and, HILO, 16 more
+// with what rounding took from them (P then has 16 bits, as attn_tc.cu has it).  TMEM per tile of pairs: two score buffers of 64
+// columns, O 128.
+// Scores may be capped, biased by distance, windowed with kept first keys (EX); outputs may have a sink in the denominator and a gate
+// per head.  The running maximum is only followed when it rises by more than 2^8 (exact: all terms are scaled alike); a warp then
+// rescales its 32 rows of O in TMEM.
+// Bound by the tensor core (HILO) or the softmax's issue slots: 2 048 rows at contexts 1001..3048, 32 heads over 8: 123 us (212 us); 1 900
+// rows of three sequences, 16 heads over 4, capped, biased, window 1024: 103 us (279 us on the mma.sync kernel of attn_latent.cu).
+// Warps: four softmax warps per tile (a thread owns a pair), TMA, MMA, two that stage queries.  Every wait is bounded (tc.cuh).
+#include <stdlib.h>
+
+#include <algorithm>
+
+#include "tc.cuh"
+
+namespace b200 {
+namespace {
+
+using namespace tc;
+
+constexpr int kArKeys = 64, kArThreads = 384;
+constexpr int kArQChunk = 128 * 128;           // [128 pairs][64 columns] bf16: 16 KiB
+constexpr int kArChunk = kArKeys * 128;        // [64 keys][64 columns] bf16: 8 KiB
+constexpr int kArTile = 2 * kArChunk;
+constexpr int kArSlots = 9;                    // key and value tiles in turn
+constexpr int kArStage = 8 * 2048;             // output staging: 2 KiB per softmax warp
+constexpr int kArTable = 32;                   // items of a CTA whose description is worked out ahead
+constexpr int kArSmem = 232448;
+static_assert(1024 + 4 * kArQChunk + kArSlots * kArTile + kArStage + 256 + kArTable * 40 <= kArSmem, "shared memory");
+
+struct RowsItem {
+  int row0, nrows, seq, ctx_max;   // attn_prefill.cu's plan
+};
+
+struct RowsParams {
+  const void* q;
+  int64_t ldq;                 // elements between rows of q
+  const int32_t* block_table;
+  const int32_t* row_to_seq;
+  const int32_t* ctx_lens;
+  const int32_t* runs;         // (first row, rows) pairs whose contexts rise by one, or
+  const int32_t* n_runs;
+  const RowsItem* plan;          // runs of one sequence with their longest context; plan[0].row0 of them from plan[1]
+  const float* sink;
+  __nv_bfloat16* out;
+  int64_t ldo;
+  float* part;
+  int bt_stride, heads, kv_heads, dim, vdim, block_size, n_splits, window, tile_rows;
+  float scale;
+  AttnExtra ex;
+};
+
+struct RowsWork {
+  int row0, nrows, seq, kvh, split, lead, tile0, lo, hi, ctx_max;   // walk [lo, hi): key tile w < lead ? w : w - lead + tile0
+};
+
+__device__ __forceinline__ int ar_tile(const RowsWork& w, int i) { return i < w.lead ? i : i - w.lead + w.tile0; }
+
+// item `it`: (run, kv head, split), the longest contexts (the last runs) first
+__device__ __forceinline__ void ar_work(const RowsParams& p, int n_runs, int it, RowsWork& w) {
+  w.split = it % p.n_splits;
+  it /= p.n_splits;
+  w.kvh = it % p.kv_heads;
+  const int run = n_runs - 1 - it / p.kv_heads;
+  w.tile0 = w.lead = 0;
+  if (p.plan) {
+    const RowsItem* r = p.plan + 1 + run;
+    w.row0 = __ldg(&r->row0);
+    w.nrows = __ldg(&r->nrows);
+    w.seq = __ldg(&r->seq);
+    w.ctx_max = __ldg(&r->ctx_max);
+  } else {
+    w.row0 = __ldg(p.runs + 2 * run);
+    w.nrows = __ldg(p.runs + 2 * run + 1);
+    w.seq = p.row_to_seq ? __ldg(p.row_to_seq + w.row0) : w.row0;
+    w.ctx_max = __ldg(p.ctx_lens + w.row0 + w.nrows - 1);
+    if (p.window > 0) {
+      w.tile0 = max(__ldg(p.ctx_lens + w.row0) - p.window, 0) / kArKeys;
+      w.lead = min((p.ex.keep_first + kArKeys - 1) / kArKeys, w.tile0);
+    }
+  }
+  const int tiles = max((w.ctx_max + kArKeys - 1) / kArKeys - w.tile0, 0) + w.lead, per = (tiles + p.n_splits - 1) / p.n_splits;
+  w.lo = min(tiles, w.split * per);
+  w.hi = min(tiles, (w.split + 1) * per);
+}
+
+template <typename QT> __device__ __forceinline__ uint4 ar_q8(const QT* p);   // eight query entries as bf16
+template <> __device__ __forceinline__ uint4 ar_q8<__nv_bfloat16>(const __nv_bfloat16* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
+template <> __device__ __forceinline__ uint4 ar_q8<float>(const float* p) {
+  const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+  return make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
+}
+
+template <typename QT, bool HILO, bool EX>
+__global__ void __launch_bounds__(kArThreads, 1)
+attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const RowsParams p) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  unsigned char* qs = smem;                        // two tiles of [2][128 pairs][64]
+  unsigned char* ring = qs + 4 * kArQChunk;        // [kArSlots][2][64 keys][64]
+  unsigned char* ostage = ring + kArSlots * kArTile;
+  uint64_t* kv_full = reinterpret_cast<uint64_t*>(ostage + kArStage);
+  uint64_t* kv_free = kv_full + kArSlots;
+  uint64_t* s_full = kv_free + kArSlots;           // [tile of pairs][2] scores of an even / odd key tile are there
+  uint64_t* p_ready = s_full + 4;                  // [tile of pairs][2] its weights are
+  uint64_t* o_full = p_ready + 4;                  // [tile of pairs][2] its second product has finished
+  uint64_t* q_ready = o_full + 4;
+  uint64_t* q_free = q_ready + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(q_free + 1);
+  RowsWork* table = reinterpret_cast<RowsWork*>(tmem_slot + 2);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kArSlots; ++s) {
+      mbar_init(kv_full + s, 1);
+      mbar_init(kv_free + s, 1);
+    }
+    for (int s = 0; s < 4; ++s) {
+      mbar_init(s_full + s, 1);
+      mbar_init(p_ready + s, 4);
+      mbar_init(o_full + s, 1);
+    }
+    mbar_init(q_ready, 2);
+    mbar_init(q_free, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 9) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  pdl_wait();
+  pdl_launch_dependents();
+  const int n_runs = p.plan ? p.plan[0].row0 : *p.n_runs, n_items = n_runs * p.kv_heads * p.n_splits;
+  const int G = p.heads / p.kv_heads, R = p.tile_rows;
+  // every other round backwards: the CTA that had the longest item of one gets the shortest of the next
+  const int grid = gridDim.x, cta = blockIdx.x;
+  auto item_of = [&](int round) { return round * grid + ((round & 1) ? grid - 1 - cta : cta); };
+  // the descriptions hang on a chain of loads (run, sequence, contexts): all of the CTA's first ones at once, for every role
+  if (warp == 10 && item_of(lane) < n_items) ar_work(p, n_runs, item_of(lane), table[lane]);
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const uint32_t tmem = *tmem_slot;   // per tile of pairs 256 columns: scores of even, odd key tiles, O
+  auto work_of = [&](int round, RowsWork& w) {
+    if (round < kArTable) w = table[round];
+    else ar_work(p, n_runs, item_of(round), w);
+  };
+
+  if (warp == 8) {
+    // ===== TMA: key tile, value tile, key tile, ... =====
+    const bool issuer = elect_one();
+    if (issuer) {
+      asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
+      asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
+    }
+    const int kc = (p.dim + 63) >> 6, vc = (p.vdim + 63) >> 6;
+    int slot = 0;
+    uint32_t ph = 1;
+    for (int round = 0; round * grid < n_items; ++round) {
+      if (item_of(round) >= n_items) continue;
+      RowsWork w;
+      work_of(round, w);
+      const int32_t* bt = p.block_table + (int64_t)w.seq * p.bt_stride;
+      for (int i = w.lo; i < w.hi; ++i) {
+        const int tok = ar_tile(w, i) * kArKeys;
+        const int blk = __shfl_sync(0xffffffffu, __ldg(bt + tok / p.block_size), 0);
+        const int row = (blk * p.kv_heads + w.kvh) * p.block_size + tok % p.block_size;
+#pragma unroll
+        for (int kv = 0; kv < 2; ++kv) {
+          mbar_wait(kv_free + slot, ph);
+          if (issuer) {
+            unsigned char* dst = ring + slot * kArTile;
+            const int nc = kv ? vc : kc;
+            mbar_expect_tx(kv_full + slot, nc * kArChunk);
+            for (int c = 0; c < nc; ++c) tma_load_2d(dst + c * kArChunk, kv ? &map_v : &map_k, c * 64, row, kv_full + slot);
+          }
+          __syncwarp();
+          if (++slot == kArSlots) slot = 0, ph ^= 1;
+        }
+      }
+    }
+  } else if (warp == 9) {
+    // ===== MMA: per key tile, for either tile of pairs: the next key tile's scores, then this one's second product =====
+    const bool issuer = elect_one();
+    const uint64_t desc_q = make_desc(smem_u32(qs), 16, 1024), desc_k = make_desc(smem_u32(ring), 16, 1024),
+                   desc_v = make_desc(smem_u32(ring), kArChunk, 1024);
+    const uint32_t id_s = idesc_bf16(kArKeys, 0), id_o = idesc_bf16(p.vdim, 1);
+    const int ksteps = p.dim >> 4;
+    int slot = 0, active = 0, n[2] = {0, 0};   // n: key tiles walked by either tile of pairs so far
+    uint32_t ph = 0;
+    for (int round = 0; round * grid < n_items; ++round) {
+      if (item_of(round) >= n_items) continue;
+      RowsWork w;
+      work_of(round, w);
+      const int nt = __shfl_sync(0xffffffffu, w.hi - w.lo, 0), tiles = __shfl_sync(0xffffffffu, w.nrows > R ? 2 : 1, 0);
+      if (nt <= 0) continue;
+      auto scores = [&](int x, int nx, int k_slot) {
+        const uint64_t da = desc_q + (uint64_t)((x * 2 * kArQChunk) >> 4), db = desc_k + (uint64_t)((k_slot * kArTile) >> 4);
+        const uint32_t d = tmem + x * 256 + (nx & 1) * kArKeys;
+        if (issuer) {
+          if (ksteps == 8) {   // unrolled: descriptors stay a uniform base plus a constant
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              mma_ss(d, da + ((j >> 2) * kArQChunk + (j & 3) * 32) / 16, db + ((j >> 2) * kArChunk + (j & 3) * 32) / 16, id_s, j ? 1u : 0u);
+          } else {
+            for (int j = 0; j < ksteps; ++j)
+              mma_ss(d, da + ((j >> 2) * kArQChunk + (j & 3) * 32) / 16, db + ((j >> 2) * kArChunk + (j & 3) * 32) / 16, id_s, j ? 1u : 0u);
+          }
+          commit(s_full + 2 * x + (nx & 1));
+        }
+        __syncwarp();
+      };
+      auto next_slot = [&]() {
+        if (++slot == kArSlots) slot = 0, ph ^= 1;
+      };
+      mbar_wait(q_ready, active & 1);
+      mbar_wait(kv_full + slot, ph);
+      fence_after();
+      int k_slot = slot;
+      next_slot();
+      scores(0, n[0], k_slot);
+      if (tiles == 2) scores(1, n[1], k_slot);
+      if (issuer) {
+        commit(kv_free + k_slot);
+        if (nt == 1) commit(q_free);
+      }
+      __syncwarp();
+      for (int i = 0; i < nt; ++i) {
+        const int v_slot = slot;
+        const uint32_t v_ph = ph;
+        next_slot();
+        const bool more = i + 1 < nt;
+        if (more) {
+          mbar_wait(kv_full + slot, ph);
+          fence_after();
+          k_slot = slot;
+          next_slot();
+        }
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          if (x >= tiles) break;
+          if (more) {
+            scores(x, n[x] + 1, k_slot);
+            if (x == tiles - 1) {
+              if (issuer) {
+                commit(kv_free + k_slot);
+                if (i + 2 == nt) commit(q_free);   // the item's last scores are on their way
+              }
+              __syncwarp();
+            }
+          }
+          if (x == 0) mbar_wait(kv_full + v_slot, v_ph);
+          mbar_wait(p_ready + 2 * x + (n[x] & 1), (n[x] >> 1) & 1);
+          fence_after();
+          const uint64_t dv = desc_v + (uint64_t)((v_slot * kArTile) >> 4);
+          const uint32_t pa = tmem + x * 256 + (n[x] & 1) * kArKeys, d = tmem + x * 256 + 128;
+          if (issuer) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {   // 16 keys per step: 8 columns of weights, 16 further those of the second term
+              mma_ts(d, pa + (j >> 1) * 32 + (j & 1) * 8, dv + (uint64_t)((j * 2048) >> 4), id_o, (i | j) ? 1u : 0u);
+              if (HILO) mma_ts(d, pa + (j >> 1) * 32 + (j & 1) * 8 + 16, dv + (uint64_t)((j * 2048) >> 4), id_o, 1u);
+            }
+            if (x == tiles - 1) commit(kv_free + v_slot);
+            commit(o_full + 2 * x + (n[x] & 1));
+          }
+          __syncwarp();
+          ++n[x];
+        }
+      }
+      ++active;
+    }
+  } else if (warp >= 10) {
+    // ===== queries of the next item -> the two A operands =====
+    const int t64 = threadIdx.x - 320;
+    int active = 0;
+    for (int round = 0; round * grid < n_items; ++round) {
+      if (item_of(round) >= n_items) continue;
+      RowsWork w;
+      work_of(round, w);
+      if (w.hi <= w.lo) continue;
+      if (active > 0) mbar_wait(q_free, (active - 1) & 1);
+      const QT* q0 = static_cast<const QT*>(p.q) + (int64_t)w.row0 * p.ldq + (int64_t)w.kvh * G * p.dim;
+      const int chunk = t64 & 15, tiles = w.nrows > R ? 2 : 1;   // 16-byte piece of a row; four rows a step
+#pragma unroll 1
+      for (int m0 = t64 >> 4; m0 < tiles * 128; m0 += 64) {
+        uint4 v[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+          const int m = m0 + 4 * u, x = m >> 7, r = (m & 127) / G, g = (m & 127) % G, row = x * R + r;
+          v[u] = make_uint4(0u, 0u, 0u, 0u);
+          if (r < R && row < w.nrows && chunk * 8 < p.dim) v[u] = ar_q8<QT>(q0 + (int64_t)row * p.ldq + g * p.dim + chunk * 8);
+        }
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+          const int m = m0 + 4 * u, x = m >> 7, mm = m & 127;
+          *reinterpret_cast<uint4*>(qs + (2 * x + (chunk >> 3)) * kArQChunk + (mm >> 3) * 1024 + (mm & 7) * 128 + (((chunk & 7) ^ (mm & 7)) << 4)) = v[u];
+        }
+      }
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(q_ready);
+      ++active;
+    }
+  } else {
+    // ===== softmax and output: a thread owns a pair of tile x =====
+    const int x = warp >> 2, quad = warp & 3, m = quad * 32 + lane;
+    const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + x * 256;
+    const int r = m / G, g = m % G, row = x * R + r;
+    constexpr float kLog2e = 1.4426950408889634f;
+    const float sc2 = p.scale * kLog2e;   // scores in the log2 domain
+    const float cap2 = EX ? p.ex.softcap * kLog2e : 0.f, cap_in = EX && p.ex.softcap > 0.f ? 2.0f * sc2 / p.ex.softcap : 0.f;
+    int n = 0, slot = 0;
+    uint32_t ph = 0;   // slot, ph: the ring's position (the key tile of the walk), for the value tile that is cleaned
+    for (int round = 0; round * grid < n_items; ++round) {
+      if (item_of(round) >= n_items) continue;
+      RowsWork w;
+      work_of(round, w);
+      if (x == 1 && w.nrows <= R) continue;   // the item has one tile of pairs (only tile 0 cleans value tiles)
+      const bool alive = r < R && row < w.nrows;
+      const int t = w.row0 + row, ctx = alive ? __ldg(p.ctx_lens + t) : 0, lo = p.window > 0 ? max(ctx - p.window, 0) : 0;
+      const int h = w.kvh * G + g, keep = EX ? p.ex.keep_first : 0;
+      const float* brow = EX && p.ex.dist_bias && alive ? p.ex.dist_bias + (int64_t)h * p.ex.bias_dist : nullptr;
+      const float far_bias = EX && brow ? __ldg(brow + p.ex.bias_dist - 1) * kLog2e : 0.f;
+      float mu = -INFINITY, l = 0.f;
+      for (int i = w.lo; i < w.hi; ++i, ++n) {
+        const int k0 = ar_tile(w, i) * kArKeys, j_lo = lo - k0, j_hi = ctx - k0;   // live columns [j_lo, j_hi), and those below keep
+        mbar_wait(s_full + 2 * x + (n & 1), (n >> 1) & 1);
+        fence_after();
+        const uint32_t s_addr = base + (n & 1) * kArKeys;
+        uint32_t s[64];
+        ld32(s_addr, s);
+        ld32(s_addr + 32, s + 32);
+        ld_wait<64>(s);
+        if constexpr (EX) {   // scaled, capped, biased, in the log2 domain
+          if (p.ex.softcap > 0.f) {
+            // cap tanh(v / cap) = cap - 2 cap / (1 + e^(2 v / cap)) on the hardware's exponential and reciprocal
+            const float top = cap2 + far_bias;
+#pragma unroll
+            for (int j = 0; j < 64; ++j) {
+              float rc;
+              asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rc) : "f"(1.0f + exp2_fast(__uint_as_float(s[j]) * cap_in)));
+              s[j] = __float_as_uint(fmaf(-2.0f * cap2, rc, top));
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 64; ++j) s[j] = __float_as_uint(fmaf(__uint_as_float(s[j]), sc2, far_bias));
+          }
+          // the bias of the last distance is in; nearer keys take their own
+          if (__any_sync(0xffffffffu, brow != nullptr && ctx - 1 - (k0 + kArKeys - 1) < p.ex.bias_dist - 1) && brow) {
+            const int d0 = ctx - 1 - k0;
+#pragma unroll
+            for (int j = 0; j < 64; ++j)
+              s[j] = __float_as_uint(__uint_as_float(s[j]) + fmaf(__ldg(brow + min(max(d0 - j, 0), p.ex.bias_dist - 1)), kLog2e, -far_bias));
+          }
+        }
+        if (__any_sync(0xffffffffu, (j_lo > 0 && !(EX && k0 + kArKeys <= keep)) || j_hi < kArKeys)) {
+#pragma unroll
+          for (int j = 0; j < 64; ++j)
+            if (j >= j_hi || (j < j_lo && !(EX && k0 + j < keep))) s[j] = 0xff800000u;   // -inf
+        }
+        float mx = -INFINITY;
+#pragma unroll
+        for (int j = 0; j < 64; ++j) mx = fmaxf(mx, __uint_as_float(s[j]));
+        if (!EX) mx *= sc2;
+        const bool jump = mx > mu + 8.f;   // also the first live key (mu = -inf)
+        if (__any_sync(0xffffffffu, jump)) {
+          const float mn = jump ? mx : mu, f = jump && mu != -INFINITY ? exp2_fast(mu - mn) : 1.f;
+          if (i > w.lo && __any_sync(0xffffffffu, f != 1.f)) {
+            mbar_wait(o_full + 2 * x + ((n - 1) & 1), ((n - 1) >> 1) & 1);
+            fence_after();
+            for (int c = 0; c < p.vdim; c += 16) {
+              uint32_t o[16];
+              ld16(base + 128 + c, o);
+              ld_wait<16>(o);
+#pragma unroll
+              for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
+              st16(base + 128 + c, o);
+            }
+          }
+          l *= f;
+          mu = mn;
+        }
+        const float mref = mu > -INFINITY ? mu : 0.f;
+        float sum[2] = {0.f, 0.f};
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t pk[32];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const float s0 = __uint_as_float(s[c * 32 + 2 * j]), s1 = __uint_as_float(s[c * 32 + 2 * j + 1]);
+            const float p0 = exp2_fast(EX ? s0 - mref : fmaf(s0, sc2, -mref)), p1 = exp2_fast(EX ? s1 - mref : fmaf(s1, sc2, -mref));
+            if constexpr (HILO) {   // the high term truncated, the rest rounded
+              sum[j & 1] += p0 + p1;
+              const uint32_t h0 = __float_as_uint(p0) & 0xffff0000u, h1 = __float_as_uint(p1) & 0xffff0000u;
+              pk[j] = __byte_perm(h0, h1, 0x7632);
+              pk[16 + j] = pack_bf16(p0 - __uint_as_float(h0), p1 - __uint_as_float(h1));
+            } else {
+              pk[j] = pack_bf16(p0, p1);
+              sum[j & 1] += bf16lo(pk[j]) + bf16hi(pk[j]);   // the weights as the second product takes them
+            }
+          }
+          if constexpr (HILO) st32(s_addr + c * 32, pk);
+          else st16(s_addr + c * 32, pk);
+        }
+        l += sum[0] + sum[1];
+        if (x == 0) {
+          const int n_valid = w.ctx_max - k0;
+          if (n_valid < kArKeys) {
+            // value rows past the context may hold anything, and 0 * NaN = NaN: zero them under their zero weights
+            const int vs = slot + 1 == kArSlots ? 0 : slot + 1;
+            mbar_wait(kv_full + vs, ph ^ (vs == 0 ? 1 : 0));
+            unsigned char* vb = ring + vs * kArTile;
+            for (int c = 0; c < (p.vdim + 63) >> 6; ++c)
+              for (int e = n_valid * 8 + m; e < kArKeys * 8; e += 128) *reinterpret_cast<uint4*>(vb + c * kArChunk + e * 16) = make_uint4(0u, 0u, 0u, 0u);
+            fence_async_smem();
+          }
+          slot += 2;
+          if (slot >= kArSlots) slot -= kArSlots, ph ^= 1;
+        }
+        st_wait();
+        fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_ready + 2 * x + (n & 1));
+      }
+      const bool any = w.hi > w.lo;
+      if (any) {
+        mbar_wait(o_full + 2 * x + ((n - 1) & 1), ((n - 1) >> 1) & 1);
+        fence_after();
+      }
+      if (p.n_splits > 1) {
+        // unnormalised sums [pair][split][vdim | maximum | denominator], the maximum in natural units
+        float* dst = p.part + (((int64_t)t * p.heads + h) * p.n_splits + w.split) * (p.vdim + 2);
+        if (alive) {
+          dst[p.vdim] = mu * 0.6931471805599453f;
+          dst[p.vdim + 1] = l;
+        }
+        for (int c = 0; c < p.vdim; c += 16) {
+          uint32_t o[16];
+          if (any) {
+            ld16(base + 128 + c, o);
+            ld_wait<16>(o);
+          }
+          if (alive) {
+            float2* d2 = reinterpret_cast<float2*>(dst + c);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) d2[j] = any ? make_float2(__uint_as_float(o[2 * j]), __uint_as_float(o[2 * j + 1])) : make_float2(0.f, 0.f);
+          }
+        }
+      } else {
+        float f = 1.f;
+        if (p.sink != nullptr && alive) {   // one more term of the denominator
+          const float sk = __ldg(p.sink + h) * kLog2e, mn = fmaxf(mu, sk);
+          f = exp2_fast(mu - mn);
+          l = l * f + exp2_fast(sk - mn);
+        }
+        float inv = l > 0.f ? f / l : 0.f;
+        if (EX && p.ex.gate && alive) inv /= 1.0f + expf(-__bfloat162float(static_cast<const __nv_bfloat16*>(p.ex.gate)[(int64_t)t * p.ex.ldg + h]));
+        // 32 columns at a time through shared memory: a row's 64 bytes leave from four neighbouring lanes (a lane per row touches 32 lines
+        // with every store: 4.6 us an item)
+        unsigned char* st = ostage + warp * 2048;
+        for (int c = 0; c < p.vdim; c += 32) {
+          uint32_t o[32];
+          if (any) {
+            ld32(base + 128 + c, o);
+            ld_wait<32>(o);
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            uint32_t v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = any ? pack_bf16(__uint_as_float(o[8 * k + 2 * j]) * inv, __uint_as_float(o[8 * k + 2 * j + 1]) * inv) : 0u;
+            *reinterpret_cast<uint4*>(st + lane * 64 + ((k ^ ((lane >> 1) & 3)) << 4)) = make_uint4(v[0], v[1], v[2], v[3]);
+          }
+          __syncwarp();
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int rr = k * 8 + (lane >> 2), mm = quad * 32 + rr, row2 = x * R + mm / G, col = c + (lane & 3) * 8;
+            const uint4 v = *reinterpret_cast<const uint4*>(st + rr * 64 + (((lane & 3) ^ ((rr >> 1) & 3)) << 4));
+            if (mm / G < R && row2 < w.nrows && col < p.vdim)
+              *reinterpret_cast<uint4*>(p.out + (int64_t)(w.row0 + row2) * p.ldo + (int64_t)(w.kvh * G + mm % G) * p.vdim + col) = v;
+          }
+          __syncwarp();
+        }
+      }
+      fence_before();
+      // all four warps of a tile have read its O before any of them hands over the next item's first weights (whose product restarts O)
+    }
+  }
+  fence_before();
+  __syncthreads();
+  if (warp == 9) {
+    fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+  }
+}
+
+template <typename QT, bool HILO, bool EX>
+int ar_launch(const CUtensorMap& mk, const CUtensorMap& mv, const RowsParams& p, int T, cudaStream_t s) {
+  static bool done[64] = {};
+  B200_CUDA(ensure_dynamic_smem(attn_rows_tc_kernel<QT, HILO, EX>, kArSmem, done));
+  const int64_t most = (int64_t)T * p.kv_heads * p.n_splits;   // upper bound; the kernel reads the real count
+  B200_CUDA(launch(attn_rows_tc_kernel<QT, HILO, EX>, dim3((unsigned)std::min<int64_t>(most, kNumSMs)), dim3(kArThreads), (size_t)kArSmem, s, mk, mv, p));
+  return B200_OK;
+}
+
+}  // namespace
+
+// rows of an item: twice what 128 pairs hold
+int attn_rows_tc_rows(int heads, int kv_heads) { return 2 * (128 / (heads / kv_heads)); }
+
+bool attn_rows_tc_supported(int heads, int kv_heads, int dim, int vdim, int block_size) {
+  return heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && heads / kv_heads <= 16 && dim % 16 == 0 && dim >= 16 && dim <= 128 && vdim % 16 == 0 &&
+         vdim >= 16 && vdim <= 128 && block_size > 0 && block_size % 64 == 0;
+}
+
+// bf16 queries in rows of ldq, weights of 16 bits; plan: attn_prefill.cu's items of at most attn_rows_tc_rows rows
+int attn_rows_tc_plan(const __nv_bfloat16* q, int64_t ldq, const __nv_bfloat16* kc, const __nv_bfloat16* vc, const int32_t* block_table, int bt_stride,
+                      const int32_t* ctx_lens, __nv_bfloat16* out, int64_t ldo, int T, int heads, int kv_heads, int dim, int block_size, float scale,
+                      const void* plan, cudaStream_t s) {
+  CUtensorMap mk, mv;
+  int rc = get_tensor_map_2d(kc, 1ull << 31, dim, dim, 64, &mk);   // rows touched come from the block table
+  if (rc) return rc;
+  rc = get_tensor_map_2d(vc, 1ull << 31, dim, dim, 64, &mv);
+  if (rc) return rc;
+  RowsParams p = {};
+  p.q = q;
+  p.ldq = ldq;
+  p.block_table = block_table;
+  p.ctx_lens = ctx_lens;
+  p.plan = static_cast<const RowsItem*>(plan);
+  p.out = out;
+  p.ldo = ldo;
+  p.bt_stride = bt_stride;
+  p.heads = heads;
+  p.kv_heads = kv_heads;
+  p.dim = p.vdim = dim;
+  p.block_size = block_size;
+  p.n_splits = 1;
+  p.tile_rows = attn_rows_tc_rows(heads, kv_heads) / 2;
+  p.scale = scale;
+  return ar_launch<__nv_bfloat16, true, false>(mk, mv, p, T, s);
+}
+
+// fp32 queries [T][heads][dim], weights rounded to bf16; runs, n_runs: the first of the lists that paged_attn_runs_plan leaves for T rows
+int attn_rows_tc_runs(const float* q, const __nv_bfloat16* kc, const __nv_bfloat16* vc, const int32_t* block_table, int bt_stride,
+                      const int32_t* row_to_seq, const int32_t* ctx_lens, __nv_bfloat16* out, const int32_t* runs, const int32_t* n_runs, int T,
+                      int heads, int kv_heads, int dim, int vdim, int block_size, float scale, const float* sink, cudaStream_t s, int n_splits,
+                      float* part, int window, const AttnExtra& ex) {
+  CUtensorMap mk, mv;
+  int rc = get_tensor_map_2d(kc, 1ull << 31, dim, dim, 64, &mk);
+  if (rc) return rc;
+  rc = get_tensor_map_2d(vc, 1ull << 31, vdim, vdim, 64, &mv);
+  if (rc) return rc;
+  int list = 0;   // the longest runs whose pairs fit two tiles: 16 << list rows
+  while (list + 1 < kRunLists && (16 << (list + 1)) <= attn_rows_tc_rows(heads, kv_heads)) ++list;
+  RowsParams p = {};
+  p.q = q;
+  p.ldq = (int64_t)heads * dim;
+  p.block_table = block_table;
+  p.row_to_seq = row_to_seq;
+  p.ctx_lens = ctx_lens;
+  p.runs = runs + (int64_t)2 * T * list;
+  p.n_runs = n_runs + list;
+  p.sink = sink;
+  p.out = out;
+  p.ldo = (int64_t)heads * vdim;
+  p.part = part;
+  p.bt_stride = bt_stride;
+  p.heads = heads;
+  p.kv_heads = kv_heads;
+  p.dim = dim;
+  p.vdim = vdim;
+  p.block_size = block_size;
+  p.n_splits = n_splits;
+  p.window = window;
+  p.tile_rows = 8 << list;
+  p.scale = scale;
+  p.ex = ex;
+  return ex.any() ? ar_launch<float, true, true>(mk, mv, p, T, s) : ar_launch<float, true, false>(mk, mv, p, T, s);
+}
+
+}  // namespace b200
