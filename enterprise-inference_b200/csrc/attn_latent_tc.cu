@@ -182,85 +182,78 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
       }
     }
   } else if (warp == 1) {
-    // ===== MMA: the scores of tile n + 1 are issued before the weights of tile n are waited for =====
-    const bool issuer = elect_one();
+    // ===== MMA: the scores of tile n + 1 are issued before the weights of tile n are waited for.  The whole warp walks the loop; bounds
+    // and addresses that come from memory are broadcast, so that they are uniform to the compiler =====
+    const uint32_t one = elect_one() ? 1u : 0u, tm = __shfl_sync(0xffffffffu, tmem, 0);
     const uint64_t desc_q = make_desc(smem_u32(qs), 16, 1024), desc_own = make_desc(smem_u32(own_ring), 16, 1024),
                    desc_rest = make_desc(smem_u32(rest_ring), 16, 1024), desc_v = make_desc(smem_u32(own_ring), kLtChunk, 1024);
+    const int items = __shfl_sync(0xffffffffu, n_items, 0);
     int st = 0, sl = 0, pv_st = 0;   // own stage and rest slot of the next scores, own stage of the next second product
     uint32_t st_ph = 0, sl_ph = 0;
     int n = 0, active = 0;
-    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
+    for (int it = blockIdx.x; it < items; it += gridDim.x) {
       LtItem w;
-      if (!next_item(it, w)) continue;
-      const int nt = __shfl_sync(0xffffffffu, w.tile_hi - w.tile_lo, 0);
+      const bool have = next_item(it, w);
+      const int nt = __shfl_sync(0xffffffffu, have ? w.tile_hi - w.tile_lo : 0, 0);
       if (nt <= 0) continue;
       const int half = __shfl_sync(0xffffffffu, w.half, 0);
       const int own = half ? own1 : own0, first = half * 4, rest = chunks - own;
       const uint32_t id_s = idesc_bf16(kLtKeys, 0), id_o = idesc_bf16(half ? width1 : width0, 1);
       auto issue_s = [&](int n) {
-        const uint32_t d = tmem + kTmS + (n & 1) * kLtKeys;
+        const uint32_t d = tm + kTmS + (n & 1) * kLtKeys;
         for (int c = 0; c < rest; ++c) {
           const int col = c < first ? c : c + own, ks = min(4, ksteps - col * 4);
           mbar_wait(rest_full + sl, sl_ph);
           fence_after();
           const uint64_t da = desc_q + (uint64_t)((c * kLtQChunk) >> 4), db = desc_rest + (uint64_t)((sl * kLtChunk) >> 4);
           const uint32_t acc = c ? 1u : 0u;
-          if (issuer) {
-            if (ks == 4) {   // unrolled: descriptors stay a uniform base plus a constant
+          if (ks == 4) {   // unrolled: descriptors are a uniform base plus a constant
 #pragma unroll
-              for (int j = 0; j < 4; ++j) mma_ss(d, da + j * 2, db + j * 2, id_s, j ? 1u : acc);
-            } else {
-              for (int j = 0; j < ks; ++j) mma_ss(d, da + j * 2, db + j * 2, id_s, j ? 1u : acc);
-            }
-            commit(rest_free + sl);
+            for (int j = 0; j < 4; ++j) mma_ss(one, d, da + j * 2, db + j * 2, id_s, j ? 1u : acc);
+          } else {
+            for (int j = 0; j < ks; ++j) mma_ss(one, d, da + j * 2, db + j * 2, id_s, j ? 1u : acc);
           }
-          __syncwarp();
+          commit(one, rest_free + sl);
           if (++sl == p.rest_slots) sl = 0, sl_ph ^= 1;
         }
         mbar_wait(own_full + st, st_ph);
         fence_after();
-        if (issuer) {
-          const uint64_t dk = desc_own + (uint64_t)((st * max_own * kLtChunk) >> 4);
+        const uint64_t dk = desc_own + (uint64_t)((st * max_own * kLtChunk) >> 4);
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            if (c >= own) break;
-            const int ks = min(4, ksteps - (first + c) * 4);
-            const uint32_t acc = c || rest ? 1u : 0u;
-            if (ks == 4) {
+        for (int c = 0; c < 4; ++c) {
+          if (c >= own) break;
+          const int ks = min(4, ksteps - (first + c) * 4);
+          const uint32_t acc = c || rest ? 1u : 0u;
+          if (ks == 4) {
 #pragma unroll
-              for (int j = 0; j < 4; ++j) mma_ts(d, tmem + kTmQ + c * 32 + j * 8, dk + ((c * kLtChunk) >> 4) + j * 2, id_s, j ? 1u : acc);
-            } else {
-              for (int j = 0; j < ks; ++j) mma_ts(d, tmem + kTmQ + c * 32 + j * 8, dk + ((c * kLtChunk) >> 4) + j * 2, id_s, j ? 1u : acc);
-            }
+            for (int j = 0; j < 4; ++j) mma_ts(one, d, tm + kTmQ + c * 32 + j * 8, dk + ((c * kLtChunk) >> 4) + j * 2, id_s, j ? 1u : acc);
+          } else {
+            for (int j = 0; j < ks; ++j) mma_ts(one, d, tm + kTmQ + c * 32 + j * 8, dk + ((c * kLtChunk) >> 4) + j * 2, id_s, j ? 1u : acc);
           }
-          commit(s_full + (n & 1));
         }
-        __syncwarp();
+        commit(one, s_full + (n & 1));
         if (++st == p.own_stages) st = 0, st_ph ^= 1;
       };
       mbar_wait(q_ready, active & 1);
       fence_after();
       issue_s(n);
-      if (nt == 1 && issuer) commit(q_free);
+      if (nt == 1) commit(one, q_free);
       for (int i = 0; i < nt; ++i, ++n) {
         if (i + 1 < nt) {
           issue_s(n + 1);
-          if (i + 2 == nt && issuer) commit(q_free);   // the item's last scores are on their way
+          if (i + 2 == nt) commit(one, q_free);   // the item's last scores are on their way
         }
         mbar_wait(p_ready + (n & 1), (n >> 1) & 1);
         fence_after();
         const uint64_t dv = desc_v + (uint64_t)((pv_st * max_own * kLtChunk) >> 4);
-        if (issuer) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {   // 16 keys per step: 8 columns of weights, 16 further those of the second term
-            const uint32_t pa = tmem + kTmS + (n & 1) * kLtKeys + (j >> 1) * 32 + (j & 1) * 8;
-            mma_ts(tmem, pa, dv + (uint64_t)((j * 2048) >> 4), id_o, (i | j) ? 1u : 0u);
-            mma_ts(tmem, pa + 16, dv + (uint64_t)((j * 2048) >> 4), id_o, 1u);
-          }
-          commit(own_free + pv_st);
-          commit(o_full + (n & 1));
+        for (int j = 0; j < 4; ++j) {   // 16 keys per step: 8 columns of weights, 16 further those of the second term
+          const uint32_t pa = tm + kTmS + (n & 1) * kLtKeys + (j >> 1) * 32 + (j & 1) * 8;
+          mma_ts(one, tm, pa, dv + (uint64_t)((j * 2048) >> 4), id_o, (i | j) ? 1u : 0u);
+          mma_ts(one, tm, pa + 16, dv + (uint64_t)((j * 2048) >> 4), id_o, 1u);
         }
-        __syncwarp();
+        commit(one, own_free + pv_st);
+        commit(one, o_full + (n & 1));
         if (++pv_st == p.own_stages) pv_st = 0;
       }
       ++active;

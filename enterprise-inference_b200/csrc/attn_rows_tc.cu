@@ -188,35 +188,33 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
       }
     }
   } else if (warp == 9) {
-    // ===== MMA: per key tile, for either tile of pairs: the next key tile's scores, then this one's second product =====
-    const bool issuer = elect_one();
+    // ===== MMA: per key tile, for either tile of pairs: the next key tile's scores, then this one's second product.  The whole warp
+    // walks the loop; bounds and addresses that come from memory are broadcast, so that they are uniform to the compiler =====
+    const uint32_t one = elect_one() ? 1u : 0u, tm = __shfl_sync(0xffffffffu, tmem, 0);
     const uint64_t desc_q = make_desc(smem_u32(qs), 16, 1024), desc_k = make_desc(smem_u32(ring), 16, 1024),
                    desc_v = make_desc(smem_u32(ring), kArChunk, 1024);
     const uint32_t id_s = idesc_bf16(kArKeys, 0), id_o = idesc_bf16(p.vdim, 1);
-    const int ksteps = p.dim >> 4;
+    const int ksteps = p.dim >> 4, items = __shfl_sync(0xffffffffu, n_items, 0);
     int slot = 0, active = 0, n[2] = {0, 0};   // n: key tiles walked by either tile of pairs so far
     uint32_t ph = 0;
-    for (int round = 0; round * grid < n_items; ++round) {
-      if (item_of(round) >= n_items) continue;
+    for (int round = 0; round * grid < items; ++round) {
+      if (item_of(round) >= items) continue;
       RowsWork w;
       work_of(round, w);
       const int nt = __shfl_sync(0xffffffffu, w.hi - w.lo, 0), tiles = __shfl_sync(0xffffffffu, w.nrows > R ? 2 : 1, 0);
       if (nt <= 0) continue;
       auto scores = [&](int x, int nx, int k_slot) {
         const uint64_t da = desc_q + (uint64_t)((x * 2 * kArQChunk) >> 4), db = desc_k + (uint64_t)((k_slot * kArTile) >> 4);
-        const uint32_t d = tmem + x * 256 + (nx & 1) * kArKeys;
-        if (issuer) {
-          if (ksteps == 8) {   // unrolled: descriptors stay a uniform base plus a constant
+        const uint32_t d = tm + x * 256 + (nx & 1) * kArKeys;
+        if (ksteps == 8) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-              mma_ss(d, da + ((j >> 2) * kArQChunk + (j & 3) * 32) / 16, db + ((j >> 2) * kArChunk + (j & 3) * 32) / 16, id_s, j ? 1u : 0u);
-          } else {
-            for (int j = 0; j < ksteps; ++j)
-              mma_ss(d, da + ((j >> 2) * kArQChunk + (j & 3) * 32) / 16, db + ((j >> 2) * kArChunk + (j & 3) * 32) / 16, id_s, j ? 1u : 0u);
-          }
-          commit(s_full + 2 * x + (nx & 1));
+          for (int j = 0; j < 8; ++j)
+            mma_ss(one, d, da + ((j >> 2) * kArQChunk + (j & 3) * 32) / 16, db + ((j >> 2) * kArChunk + (j & 3) * 32) / 16, id_s, j ? 1u : 0u);
+        } else {
+          for (int j = 0; j < ksteps; ++j)
+            mma_ss(one, d, da + ((j >> 2) * kArQChunk + (j & 3) * 32) / 16, db + ((j >> 2) * kArChunk + (j & 3) * 32) / 16, id_s, j ? 1u : 0u);
         }
-        __syncwarp();
+        commit(one, s_full + 2 * x + (nx & 1));
       };
       auto next_slot = [&]() {
         if (++slot == kArSlots) slot = 0, ph ^= 1;
@@ -228,11 +226,8 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
       next_slot();
       scores(0, n[0], k_slot);
       if (tiles == 2) scores(1, n[1], k_slot);
-      if (issuer) {
-        commit(kv_free + k_slot);
-        if (nt == 1) commit(q_free);
-      }
-      __syncwarp();
+      commit(one, kv_free + k_slot);
+      if (nt == 1) commit(one, q_free);
       for (int i = 0; i < nt; ++i) {
         const int v_slot = slot;
         const uint32_t v_ph = ph;
@@ -250,28 +245,22 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
           if (more) {
             scores(x, n[x] + 1, k_slot);
             if (x == tiles - 1) {
-              if (issuer) {
-                commit(kv_free + k_slot);
-                if (i + 2 == nt) commit(q_free);   // the item's last scores are on their way
-              }
-              __syncwarp();
+              commit(one, kv_free + k_slot);
+              if (i + 2 == nt) commit(one, q_free);   // the item's last scores are on their way
             }
           }
           if (x == 0) mbar_wait(kv_full + v_slot, v_ph);
           mbar_wait(p_ready + 2 * x + (n[x] & 1), (n[x] >> 1) & 1);
           fence_after();
           const uint64_t dv = desc_v + (uint64_t)((v_slot * kArTile) >> 4);
-          const uint32_t pa = tmem + x * 256 + (n[x] & 1) * kArKeys, d = tmem + x * 256 + 128;
-          if (issuer) {
+          const uint32_t pa = tm + x * 256 + (n[x] & 1) * kArKeys, d = tm + x * 256 + 128;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {   // 16 keys per step: 8 columns of weights, 16 further those of the second term
-              mma_ts(d, pa + (j >> 1) * 32 + (j & 1) * 8, dv + (uint64_t)((j * 2048) >> 4), id_o, (i | j) ? 1u : 0u);
-              if (HILO) mma_ts(d, pa + (j >> 1) * 32 + (j & 1) * 8 + 16, dv + (uint64_t)((j * 2048) >> 4), id_o, 1u);
-            }
-            if (x == tiles - 1) commit(kv_free + v_slot);
-            commit(o_full + 2 * x + (n[x] & 1));
+          for (int j = 0; j < 4; ++j) {   // 16 keys per step: 8 columns of weights, 16 further those of the second term
+            mma_ts(one, d, pa + (j >> 1) * 32 + (j & 1) * 8, dv + (uint64_t)((j * 2048) >> 4), id_o, (i | j) ? 1u : 0u);
+            if (HILO) mma_ts(one, d, pa + (j >> 1) * 32 + (j & 1) * 8 + 16, dv + (uint64_t)((j * 2048) >> 4), id_o, 1u);
           }
-          __syncwarp();
+          if (x == tiles - 1) commit(one, kv_free + v_slot);
+          commit(one, o_full + 2 * x + (n[x] & 1));
           ++n[x];
         }
       }
