@@ -13,8 +13,8 @@
 // Scores may be capped, biased by distance, windowed with kept first keys (EX); outputs may have a sink in the denominator and a gate
 // per head.  The running maximum is only followed when it rises by more than 2^8 (exact: all terms are scaled alike); a warp then
 // rescales its 32 rows of O in TMEM.
-// Bound by the tensor core (HILO) or the softmax's issue slots: 2 048 rows at contexts 1001..3048, 32 heads over 8: 123 us (212 us); 1 900
-// rows of three sequences, 16 heads over 4, capped, biased, window 1024: 103 us (279 us on the mma.sync kernel of attn_latent.cu).
+// Bound by the tensor core (HILO) or the softmax's issue slots: 2 048 rows at contexts 1001..3048, 32 heads over 8: 118 us (212 us); 1 900
+// rows of three sequences, 16 heads over 4, capped, biased, window 1024: 77 us (279 us on the mma.sync kernel of attn_latent.cu).
 // Warps: four softmax warps per tile (a thread owns a pair), TMA, MMA, two that stage queries.  Every wait is bounded (tc.cuh).
 #include <stdlib.h>
 
@@ -31,11 +31,13 @@ constexpr int kArKeys = 64, kArThreads = 384;
 constexpr int kArQChunk = 128 * 128;           // [128 pairs][64 columns] bf16: 16 KiB
 constexpr int kArChunk = kArKeys * 128;        // [64 keys][64 columns] bf16: 8 KiB
 constexpr int kArTile = 2 * kArChunk;
-constexpr int kArSlots = 9;                    // key and value tiles in turn
+// key and value tiles in turn; EX gives one of them to the table of score biases of an item's heads
+__host__ __device__ constexpr int ar_slots(bool ex) { return ex ? 8 : 9; }
+constexpr int kArBiasFloats = kArTile / 4, kArBiasPad = 96;   // entries in front (masked keys) and behind (far keys) of a head's, see fill_bias
 constexpr int kArStage = 8 * 2048;             // output staging: 2 KiB per softmax warp
 constexpr int kArTable = 32;                   // items of a CTA whose description is worked out ahead
 constexpr int kArSmem = 232448;
-static_assert(1024 + 4 * kArQChunk + kArSlots * kArTile + kArStage + 256 + kArTable * 40 <= kArSmem, "shared memory");
+static_assert(1024 + 4 * kArQChunk + 9 * kArTile + kArStage + 256 + kArTable * 40 <= kArSmem, "shared memory");
 
 struct RowsItem {
   int row0, nrows, seq, ctx_max;   // attn_prefill.cu's plan
@@ -103,19 +105,22 @@ template <> __device__ __forceinline__ uint4 ar_q8<float>(const float* p) {
 template <typename QT, bool HILO, bool EX>
 __global__ void __launch_bounds__(kArThreads, 1)
 attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const RowsParams p) {
+  constexpr int kArSlots = ar_slots(EX);
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   unsigned char* qs = smem;                        // two tiles of [2][128 pairs][64]
   unsigned char* ring = qs + 4 * kArQChunk;        // [kArSlots][2][64 keys][64]
-  unsigned char* ostage = ring + kArSlots * kArTile;
+  float* bias_tab = reinterpret_cast<float*>(ring + kArSlots * kArTile);   // EX only
+  unsigned char* ostage = ring + 9 * kArTile;
   uint64_t* kv_full = reinterpret_cast<uint64_t*>(ostage + kArStage);
   uint64_t* kv_free = kv_full + kArSlots;
   uint64_t* s_full = kv_free + kArSlots;           // [tile of pairs][2] scores of an even / odd key tile are there
   uint64_t* p_ready = s_full + 4;                  // [tile of pairs][2] its weights are
   uint64_t* o_full = p_ready + 4;                  // [tile of pairs][2] its second product has finished
   uint64_t* q_ready = o_full + 4;
-  uint64_t* q_free = q_ready + 1;
+  uint64_t* q_first = q_ready + 1;                 // the CTA's first queries, staged by the softmax warps as well
+  uint64_t* q_free = q_first + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(q_free + 1);
   RowsWork* table = reinterpret_cast<RowsWork*>(tmem_slot + 2);
   if (threadIdx.x == 0) {
@@ -129,6 +134,7 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
       mbar_init(o_full + s, 1);
     }
     mbar_init(q_ready, 2);
+    mbar_init(q_first, 10);
     mbar_init(q_free, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -152,6 +158,30 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
   auto work_of = [&](int round, RowsWork& w) {
     if (round < kArTable) w = table[round];
     else ar_work(p, n_runs, item_of(round), w);
+  };
+  // the two A operands of an item, thread i of `threads`: 16-byte pieces of rows
+  auto stage_q = [&](const RowsWork& w, int i, int threads) {
+    const QT* q0 = static_cast<const QT*>(p.q) + (int64_t)w.row0 * p.ldq + (int64_t)w.kvh * G * p.dim;
+    const int pieces = (w.nrows > R ? 2 : 1) * 128 * 16;
+    constexpr int U = 8;
+#pragma unroll 1
+    for (int e0 = i; e0 < pieces; e0 += U * threads) {
+      uint4 v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int e = e0 + u * threads, m = e >> 4, chunk = e & 15, r = (m & 127) / G, g = (m & 127) % G, row = (m >> 7) * R + r;
+        v[u] = make_uint4(0u, 0u, 0u, 0u);
+        if (e < pieces && r < R && row < w.nrows && chunk * 8 < p.dim) v[u] = ar_q8<QT>(q0 + (int64_t)row * p.ldq + g * p.dim + chunk * 8);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int e = e0 + u * threads, m = e >> 4, chunk = e & 15, mm = m & 127;
+        if (e < pieces)
+          *reinterpret_cast<uint4*>(qs + (2 * (m >> 7) + (chunk >> 3)) * kArQChunk + (mm >> 3) * 1024 + (mm & 7) * 128 + (((chunk & 7) ^ (mm & 7)) << 4)) = v[u];
+      }
+    }
+    fence_async_smem();
+    __syncwarp();
   };
 
   if (warp == 8) {
@@ -219,7 +249,8 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
       auto next_slot = [&]() {
         if (++slot == kArSlots) slot = 0, ph ^= 1;
       };
-      mbar_wait(q_ready, active & 1);
+      if (active == 0) mbar_wait(q_first, 0);
+      else mbar_wait(q_ready, (active - 1) & 1);
       mbar_wait(kv_full + slot, ph);
       fence_after();
       int k_slot = slot;
@@ -268,34 +299,20 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     }
   } else if (warp >= 10) {
     // ===== queries of the next item -> the two A operands =====
-    const int t64 = threadIdx.x - 320;
     int active = 0;
     for (int round = 0; round * grid < n_items; ++round) {
       if (item_of(round) >= n_items) continue;
       RowsWork w;
       work_of(round, w);
       if (w.hi <= w.lo) continue;
-      if (active > 0) mbar_wait(q_free, (active - 1) & 1);
-      const QT* q0 = static_cast<const QT*>(p.q) + (int64_t)w.row0 * p.ldq + (int64_t)w.kvh * G * p.dim;
-      const int chunk = t64 & 15, tiles = w.nrows > R ? 2 : 1;   // 16-byte piece of a row; four rows a step
-#pragma unroll 1
-      for (int m0 = t64 >> 4; m0 < tiles * 128; m0 += 64) {
-        uint4 v[16];
-#pragma unroll
-        for (int u = 0; u < 16; ++u) {
-          const int m = m0 + 4 * u, x = m >> 7, r = (m & 127) / G, g = (m & 127) % G, row = x * R + r;
-          v[u] = make_uint4(0u, 0u, 0u, 0u);
-          if (r < R && row < w.nrows && chunk * 8 < p.dim) v[u] = ar_q8<QT>(q0 + (int64_t)row * p.ldq + g * p.dim + chunk * 8);
-        }
-#pragma unroll
-        for (int u = 0; u < 16; ++u) {
-          const int m = m0 + 4 * u, x = m >> 7, mm = m & 127;
-          *reinterpret_cast<uint4*>(qs + (2 * x + (chunk >> 3)) * kArQChunk + (mm >> 3) * 1024 + (mm & 7) * 128 + (((chunk & 7) ^ (mm & 7)) << 4)) = v[u];
-        }
+      if (active == 0) {
+        stage_q(w, threadIdx.x - 64, 320);   // (beside the softmax warps' threads 0..255)
+        if (lane == 0) mbar_arrive(q_first);
+      } else {
+        mbar_wait(q_free, (active - 1) & 1);
+        stage_q(w, threadIdx.x - 320, 64);
+        if (lane == 0) mbar_arrive(q_ready);
       }
-      fence_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(q_ready);
       ++active;
     }
   } else {
@@ -306,12 +323,32 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     constexpr float kLog2e = 1.4426950408889634f;
     const float sc2 = p.scale * kLog2e;   // scores in the log2 domain
     const float cap2 = EX ? p.ex.softcap * kLog2e : 0.f, cap_in = EX && p.ex.softcap > 0.f ? 2.0f * sc2 / p.ex.softcap : 0.f;
+    // bias of a distance less that of the farthest, log2 domain, for the item's heads; zeros around, so that a tile that holds some near
+    // key indexes it without clamping each distance
+    const int bias_row = p.ex.bias_dist + 2 * kArBiasPad + 8;
+    const bool tab = EX && p.ex.dist_bias != nullptr && G * bias_row <= kArBiasFloats;
+    auto fill_bias = [&](int kvh) {
+      asm volatile("bar.sync 2, 256;" ::: "memory");
+      for (int e = threadIdx.x; e < G * bias_row; e += 256) {
+        const int gg = e / bias_row, d = e % bias_row - kArBiasPad;
+        const float* b = p.ex.dist_bias + (int64_t)(kvh * G + gg) * p.ex.bias_dist;
+        bias_tab[e] = d >= 0 && d < p.ex.bias_dist ? (__ldg(b + d) - __ldg(b + p.ex.bias_dist - 1)) * kLog2e : 0.f;
+      }
+      asm volatile("bar.sync 2, 256;" ::: "memory");
+    };
+    bool first = true;
     int n = 0, slot = 0;
     uint32_t ph = 0;   // slot, ph: the ring's position (the key tile of the walk), for the value tile that is cleaned
     for (int round = 0; round * grid < n_items; ++round) {
       if (item_of(round) >= n_items) continue;
       RowsWork w;
       work_of(round, w);
+      if (first && w.hi > w.lo) {
+        stage_q(w, threadIdx.x, 320);   // (the stagers are threads 256..319 of this)
+        if (lane == 0) mbar_arrive(q_first);
+        first = false;
+      }
+      if (tab) fill_bias(w.kvh);
       if (x == 1 && w.nrows <= R) continue;   // the item has one tile of pairs (only tile 0 cleans value tiles)
       const bool alive = r < R && row < w.nrows;
       const int t = w.row0 + row, ctx = alive ? __ldg(p.ctx_lens + t) : 0, lo = p.window > 0 ? max(ctx - p.window, 0) : 0;
@@ -345,6 +382,12 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
           // the bias of the last distance is in; nearer keys take their own
           if (__any_sync(0xffffffffu, brow != nullptr && ctx - 1 - (k0 + kArKeys - 1) < p.ex.bias_dist - 1) && brow) {
             const int d0 = ctx - 1 - k0;
+            if (tab) {
+              // below -1 every key is masked, from the last distance + 64 on every key is far: the padding covers what lies between
+              const float* b = bias_tab + g * bias_row + kArBiasPad + min(max(d0, -1), p.ex.bias_dist + 95);
+#pragma unroll
+              for (int j = 0; j < 64; ++j) s[j] = __float_as_uint(__uint_as_float(s[j]) + b[-j]);
+            } else
 #pragma unroll
             for (int j = 0; j < 64; ++j)
               s[j] = __float_as_uint(__uint_as_float(s[j]) + fmaf(__ldg(brow + min(max(d0 - j, 0), p.ex.bias_dist - 1)), kLog2e, -far_bias));

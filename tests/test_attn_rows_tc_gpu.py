@@ -1,0 +1,110 @@
+"""Attention of runs of rows on tcgen05 (heads of at most 128, cache blocks of whole 64-key tiles) against the same attention in float64."""
+import pytest
+import torch
+
+from conftest import pkg
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+CTXS = [1, 2, 63, 64, 65, 127, 128, 129, 500] + list(range(1, 71)) + list(range(300, 431)) + list(range(490, 500))
+SEQ = list(range(9)) + [9] * 70 + [10] * 131 + [11] * 10      # decode rows at tile and block edges, then runs of odd lengths that start inside tiles
+
+
+def _case(heads, kv, dim, vdim, bs, seed):
+    g = torch.Generator().manual_seed(seed)
+    n_tok, T = 500, len(CTXS)
+    nb = (n_tok + bs - 1) // bs
+    perm = torch.randperm(nb + 3, generator=g)[:nb]
+    rows = [torch.randn(n_tok, kv, d, generator=g).to(torch.bfloat16) for d in (dim, vdim)]
+    caches = []
+    for r in rows:   # poison behind the contexts, where nobody may look
+        c = torch.full((nb + 3, kv, bs, r.shape[2]), float("nan"), dtype=torch.bfloat16)
+        for j in range(n_tok):
+            c[perm[j // bs], :, j % bs] = r[j]
+        caches.append(c.to(DEV))
+    q = (torch.randn(T, heads, dim, generator=g) * 3).to(torch.bfloat16)   # the running maximum jumps
+    bt = perm.to(torch.int32)[None, :].repeat(12, 1).to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)   # noqa: E731
+    return g, q, rows, caches, bt, i32(SEQ), i32(CTXS), T
+
+
+def _oracle(q, rows, scale, window=0, keep=0, cap=0.0, bias=None, sink=None, gate=None):
+    T, heads, _ = q.shape
+    K, V = (r.double() for r in rows)
+    kv, out = K.shape[1], []
+    for t in range(T):
+        c = CTXS[t]
+        k, v = (x[:c].repeat_interleave(heads // kv, 1) for x in (K, V))
+        s = torch.einsum("hd,chd->hc", q[t].double(), k) * scale
+        if cap:
+            s = cap * torch.tanh(s / cap)
+        dist = c - 1 - torch.arange(c)
+        if bias is not None:
+            s = s + bias.double()[:, dist.clamp(max=bias.shape[1] - 1)]
+        if window:
+            s = s.masked_fill((dist >= window) & (torch.arange(c) >= keep), float("-inf"))
+        m = s.max(-1, keepdim=True).values
+        m = torch.maximum(m, sink.double()[:, None]) if sink is not None else m
+        e = torch.exp(s - m)
+        o = torch.einsum("hc,chd->hd", e, v) / (e.sum(-1, keepdim=True) + (torch.exp(sink.double()[:, None] - m) if sink is not None else 0.0))
+        out.append(o * torch.sigmoid(gate[t].double())[:, None] if gate is not None else o)
+    return torch.stack(out)
+
+
+def _close(out, want):
+    got = out.double().cpu()
+    assert torch.isfinite(got).all()
+    # queries are exact in bf16 and weights carry 16 bits, so a result is rounded once: 2^-9 of itself at most, beside fp32 noise of the sums
+    # (a capped score's exponential and reciprocal: a few 2^-22 of the cap)
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 2e-4).all(), float((got - want).abs().max())
+
+
+# pairs per row: 4, 1 (128 rows a tile), 16, 5 (idle pairs); heads with a partial second chunk of columns; values narrower than keys
+@pytest.mark.parametrize("heads,kv,dim,vdim,bs", [(8, 2, 128, 128, 128), (2, 2, 64, 64, 64), (16, 1, 80, 48, 128), (10, 2, 96, 128, 192)])
+@pytest.mark.parametrize("form", ["plain", "capped, biased, gated", "window", "kept keys, biased, sink", "long bias", "split"])
+def test_runs_of_rows_tile_edges(heads, kv, dim, vdim, bs, form):
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    g, q, rows, (kc, vc), bt, seq, ctx, T = _case(heads, kv, dim, vdim, bs, heads * 100 + dim)
+    scale, ns = dim ** -0.5, 3 if form == "split" else 1
+    ws = torch.zeros(int(lib.b200_paged_attn_anydim_workspace_bytes(T)), dtype=torch.uint8, device=DEV)
+    out = torch.full((T, heads, vdim), float("nan"), dtype=torch.bfloat16, device=DEV)
+    part = torch.full((T * heads * ns * (vdim + 2),), float("nan"), device=DEV)
+    qd, pos = q.float().to(DEV), (ctx - 1).contiguous()
+    lead = [qd.data_ptr(), kc.data_ptr(), vc.data_ptr(), bt.data_ptr(), bt.shape[1], seq.data_ptr(), ctx.data_ptr()]
+    if form in ("plain", "split"):
+        sink = torch.randn(heads, generator=g).to(DEV)
+        check(lib.b200_paged_attn_mma(*lead, out.data_ptr(), T, heads, kv, dim, vdim, bs, scale, sink.data_ptr(), ws.data_ptr(), 0, ns,
+                                      part.data_ptr() if ns > 1 else None, None))
+        want = _oracle(q, rows, scale, sink=sink.cpu())
+    elif form in ("capped, biased, gated", "long bias", "window"):
+        nd = 3000 if form == "long bias" else 40      # 3000: longer than the on-chip table
+        cap, window = (20.0, 0) if form == "capped, biased, gated" else (0.0, 100 if form == "window" else 0)
+        bias = (torch.randn(heads, nd, generator=g) if form != "window" else None)
+        gate = torch.randn(T, heads, generator=g).to(torch.bfloat16)
+        bd, gd = bias.to(DEV) if bias is not None else None, gate.to(DEV)
+        check(lib.b200_paged_attn_biased(0, 2, *lead, pos.data_ptr(), out.data_ptr(), T, heads, kv, dim, vdim, bs, scale, window, cap,
+                                         bd.data_ptr() if bd is not None else None, nd if bd is not None else 0, gd.data_ptr(), heads, ws.data_ptr(), 1,
+                                         None, None))
+        want = _oracle(q, rows, scale, window, 0, cap, bias, gate=gate)
+    else:
+        bias, sink = torch.randn(heads, 200, generator=g), torch.randn(heads, generator=g)
+        bd, sd = bias.to(DEV), sink.to(DEV)
+        check(lib.b200_paged_attn_kept(0, 2, *lead, pos.data_ptr(), out.data_ptr(), T, heads, kv, dim, vdim, bs, scale, 90, 70, sd.data_ptr(),
+                                       bd.data_ptr(), 200, ws.data_ptr(), 1, None, None))
+        want = _oracle(q, rows, scale, 90, 70, 0.0, bias, sink=sink)
+    torch.cuda.synchronize()
+    _close(out, want)
+
+
+@pytest.mark.parametrize("heads,kv", [(8, 2), (4, 4), (8, 1), (10, 2)])
+def test_prefill_rows_of_the_decoder_stack(heads, kv):
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    g, q, rows, (kc, vc), bt, seq, ctx, T = _case(heads, kv, 128, 128, 128, heads * 7 + kv)
+    wsb = int(lib.b200_paged_attn_workspace_bytes(T, heads, 500, 128))
+    ws = torch.zeros(wsb, dtype=torch.uint8, device=DEV)
+    out = torch.full((T, heads, 128), float("nan"), dtype=torch.bfloat16, device=DEV)
+    qd = q.to(DEV)
+    check(lib.b200_paged_attn_prefill(qd.data_ptr(), heads * 128, kc.data_ptr(), vc.data_ptr(), bt.data_ptr(), bt.shape[1], seq.data_ptr(), ctx.data_ptr(),
+                                      out.data_ptr(), heads * 128, T, heads, kv, 128, 500, 128 ** -0.5, ws.data_ptr(), wsb, None))
+    torch.cuda.synchronize()
+    _close(out, _oracle(q, rows, 128 ** -0.5))
