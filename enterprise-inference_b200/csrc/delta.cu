@@ -12,12 +12,8 @@
 //    slot's tail; silu; the unit vectors; beta; the decays.  Everything leaves in fp32.
 //  * delta_tails: CTAs of 256 channels per sequence, after prep: the last taps - 1 raw rows of the portion (or what is left of the old tail
 //    when the portion is shorter) become the slot's tail.
-//  * delta_scan: the recurrence.  The columns of S do not interact, so one CTA takes (sequence, head, 32 value columns); a warp
-//    owns 4 columns, a lane the key channels lane, lane + 32, ...; the state lives in registers during the walk and is
-//    stored [head][vdim][dim] so that a warp's loads are contiguous.  The step's rows are staged 16 at a time in shared memory,
-//    the next stage travelling into registers while this one is walked.  The only reductions on the chain from one row to the
-//    next are the four S^T k sums of a warp (interleaved shuffles); the read-out leaves per-lane partial sums in shared
-//    memory that are added for the whole stage after its walk.
+//  * delta_scan: the recurrence.  The columns of S do not interact, so a CTA takes (sequence, head, 16 value columns) and walks the
+//    sequence's rows of the step with the state in registers (stored [head][vdim][dim]).
 //    A sequence whose first row of the step is at position 0 starts from zeros, whatever the slot held.
 //
 // Two parameters widen the kernels to other recurrences of the same shape.  The decay of (row, head, key channel) is read at
@@ -26,6 +22,7 @@
 // second-step projection.  DELTA false drops the correction: u = beta v, which is the state-space recurrence
 // S = g S + dt B x^T, y = S^T C of ssd.cu with keys B, queries C, values x and beta = dt.
 #include "common.cuh"
+#include "f32x2.cuh"
 
 namespace b200 {
 namespace {
@@ -121,196 +118,342 @@ delta_tails_kernel(const AT* __restrict__ fused, int64_t ld, const int32_t* __re
     }
 }
 
-constexpr int kDsCols = 4, kDsWarps = 8, kDsBlockCols = kDsCols * kDsWarps, kDsStage = 16, kDsThreads = kDsWarps * 32;
+// The walk.  A lane holds a few neighbouring key channels of four value columns (one shared-memory read of k, q and the decays per row
+// serves all four), a warp owns those four columns, a CTA's four warps sixteen; the state lives in registers as pairs for the packed
+// fp32 arithmetic.  The step's rows are staged 16 at a time in shared memory by cp.async, the next stage travelling while this one is
+// walked.
+// What bounds it: one long sequence fills one warp per scheduler, so a row costs its instructions' latency.  Of the chain from row to row
+// only S^T k needs other lanes.  The delta rule takes two rows per turn: with S' = S diag(g1), S'' = S' diag(g2)
+//   u1 = b1 (v1 - S'^T k1)         u2 = b2 (v2 - S''^T k2 - (sum_d k1 g2 k2) u1)
+//   o1 = S'^T q1 + (k1 . q1) u1    S = S'' + (g2 k1) u1 + k2 u2         o2 = S^T q2
+// so the eight sums of two rows and four columns are reduced together (a lane keeps half of what it holds at every step: 9 shuffles
+// instead of 40), and the two dot products of inputs alone are taken once per stage for all columns.  The read-out leaves per-lane sums in
+// shared memory, added for the whole stage after its walk.
+// 1 900 rows of three sequences, 16 heads of 128 x 128, channel decays: @D1900@ (one row per turn, unpacked, eight warps a CTA: 457 us).
+constexpr int kDsWarps = 4, kDsCols = 4 * kDsWarps, kDsStage = 16, kDsThreads = kDsWarps * 32;
+constexpr int kDsPartRow = 136;   // floats of a row of read-out sums: 32 lanes x 4 columns, rows 32 bytes apart in the banks
 
-template <int DPL, bool DELTA>
-__global__ void __launch_bounds__(kDsThreads)
-delta_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ vn, const float* __restrict__ beta,
-                  const float* __restrict__ decay, int64_t g_row, int g_head, int g_chan, const int32_t* __restrict__ positions, const int32_t* __restrict__ seq_start,
-                  const int32_t* __restrict__ seq_slots, float* __restrict__ state, int64_t slot_stride, float* __restrict__ out, int heads,
-                  int kv_heads, int dim, int vd) {
-  extern __shared__ float stage[];
+struct ScanArgs {
+  const float* qn;
+  const float* kn;
+  const float* vn;
+  const float* beta;
+  const float* decay;
+  const int32_t* positions;
+  const int32_t* seq_start;
+  const int32_t* seq_slots;
+  float* state;
+  float* out;
+  int64_t g_row, slot_stride;
+  int g_head, g_chan, heads, kv_heads, dim, vd;
+  int vec;   // rows of q, k (and channel decays) can be copied 16 bytes, state columns moved 8 bytes at a time
+};
+
+// NP: pairs of channels per lane (1, 2, 4: dim up to 64, 128, 256).  A staged row holds 64 NP floats, zero beyond dim.
+__host__ __device__ constexpr int ds_row(int np) { return 64 * np; }
+// floats of one stage buffer: q | k | (g) rows, then per row the CTA's 16 values, beta and (head decays) g
+__host__ __device__ constexpr int ds_buf(int np, bool chan) { return kDsStage * ((chan ? 3 : 2) * ds_row(np) + kDsCols + 2); }
+__host__ __device__ constexpr int ds_floats(int np, bool chan) { return 2 * ds_buf(np, chan) + kDsStage + kDsWarps * kDsStage * kDsPartRow; }
+
+// the lane's pairs of a staged row; pair i starts at channel 2 x (NP 1), 4 x + 2 (i & 1) + 128 (i >> 1) (else) for lane x
+template <int NP>
+__device__ __forceinline__ void ds_pairs(const float* row, int lane, uint64_t (&x)[NP]) {
+  if constexpr (NP == 1) {
+    x[0] = *reinterpret_cast<const uint64_t*>(row + 2 * lane);
+  } else {
+#pragma unroll
+    for (int v = 0; v < NP / 2; ++v) {
+      const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(row + 128 * v + 4 * lane);
+      x[2 * v] = t.x;
+      x[2 * v + 1] = t.y;
+    }
+  }
+}
+template <int NP>
+__device__ __forceinline__ int ds_chan(int lane, int i) {
+  return NP == 1 ? 2 * lane : 4 * lane + 2 * (i & 1) + 128 * (i >> 1);
+}
+// sums over the warp of N (a power of two) values at once, all of them to every lane
+template <int N>
+__device__ __forceinline__ void ds_reduce(float (&v)[N], int lane) {
+  int bit = 16;
+  float x[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) x[i] = v[i];
+#pragma unroll
+  for (int half = N / 2; half >= 1; half >>= 1, bit >>= 1) {   // keep one half of the values, hand over the other
+    const bool up = (lane & bit) != 0;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const float keep = up ? x[i + half] : x[i], give = up ? x[i] : x[i + half];
+      x[i] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+    }
+  }
+#pragma unroll
+  for (; bit >= 1; bit >>= 1) x[0] += __shfl_xor_sync(0xffffffffu, x[0], bit);
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = __shfl_sync(0xffffffffu, x[0], i * (32 / N));   // value i ended with the lanes i * 32 / N ..
+}
+
+// CHAN: a decay per key channel, else one per row and head.
+template <int NP, bool DELTA, bool CHAN>
+__global__ void __launch_bounds__(kDsThreads) delta_scan_kernel(const ScanArgs a) {
+  extern __shared__ __align__(16) float stage[];
+  constexpr int ROW = ds_row(NP), BUF = ds_buf(NP, CHAN);
   pdl_wait();
   pdl_launch_dependents();
-  const int s = blockIdx.x, h = blockIdx.y, zb = blockIdx.z;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int start = seq_start[s], n_rows = seq_start[s + 1] - start;
+  const int s = blockIdx.x, h = blockIdx.y, jb = blockIdx.z * kDsCols;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int start = a.seq_start[s], n_rows = a.seq_start[s + 1] - start;
   if (n_rows <= 0) return;
-  const bool fresh = positions[start] == 0;
-  const int g = h / (heads / kv_heads);
-  float* S_st = state + (int64_t)seq_slots[s] * slot_stride;   // [heads][vd][dim]
-  const int jb = zb * kDsBlockCols, j0 = jb + warp * kDsCols;
-  float Sr[kDsCols][DPL];
+  const bool fresh = a.positions[start] == 0;
+  const int g = h / (a.heads / a.kv_heads), dim = a.dim, vd = a.vd;
+  const int j0 = jb + warp * 4;   // the warp's first value column
+  float* S_st = a.state + (int64_t)a.seq_slots[s] * a.slot_stride + ((int64_t)h * vd + j0) * dim;
+  const int64_t qk = (int64_t)a.kv_heads * dim, hv = (int64_t)a.heads * vd;
+  const float* qsrc = a.qn + (int64_t)start * qk + (int64_t)g * dim;
+  const float* ksrc = a.kn + (int64_t)start * qk + (int64_t)g * dim;
+  const float* gsrc = a.decay + (int64_t)start * a.g_row + (int64_t)h * a.g_head;
+  const float* vsrc = a.vn + (int64_t)start * hv + (int64_t)h * vd + jb;
+  const float* bsrc = a.beta + (int64_t)start * a.heads + h;
+  uint64_t S[4][NP];
 #pragma unroll
-  for (int i = 0; i < DPL; ++i) {
-    const int d = lane + 32 * i;
+  for (int c = 0; c < 4; ++c)
 #pragma unroll
-    for (int c = 0; c < kDsCols; ++c) Sr[c][i] = (!fresh && d < dim && j0 + c < vd) ? S_st[((int64_t)h * vd + j0 + c) * dim + d] : 0.f;
-  }
-  const int qk = kv_heads * dim, hv = heads * vd;
+    for (int i = 0; i < NP; ++i) {
+      const int d = ds_chan<NP>(lane, i);
+      const float* p = S_st + (int64_t)c * dim + d;
+      S[c][i] = 0;
+      if (!fresh && j0 + c < vd && d < dim) S[c][i] = a.vec ? *reinterpret_cast<const uint64_t*>(p) : f2::pack(p[0], d + 1 < dim ? p[1] : 0.f);
+    }
   if (n_rows == 1) {
     // a decode row: nothing to stage; the row's inputs are fetched beside the state
-    const int64_t t = start;
-    const float b = beta[t * heads + h];
-    float dot[kDsCols], acc[kDsCols], v[kDsCols], q[DPL], k[DPL];
+    const float b = bsrc[0], gs = CHAN ? 0.f : gsrc[0];
+    uint64_t k[NP], q[NP];
+    float d4[4] = {0.f, 0.f, 0.f, 0.f}, o4[4];
 #pragma unroll
-    for (int c = 0; c < kDsCols; ++c) {
-      dot[c] = 0.f;
-      acc[c] = 0.f;
-      v[c] = j0 + c < vd ? vn[t * hv + h * vd + j0 + c] : 0.f;
-    }
+    for (int i = 0; i < NP; ++i) {
+      const int d = ds_chan<NP>(lane, i);
+      auto pair = [&](const float* p, int64_t st) { return f2::pack(d < dim ? p[d * st] : 0.f, d + 1 < dim ? p[(d + 1) * st] : 0.f); };
+      k[i] = pair(ksrc, 1);
+      q[i] = pair(qsrc, 1);
+      const uint64_t gg = CHAN ? pair(gsrc, a.g_chan) : f2::both(gs);
 #pragma unroll
-    for (int i = 0; i < DPL; ++i) {
-      const int d = lane + 32 * i;
-      const bool live = d < dim;
-      q[i] = live ? qn[t * qk + g * dim + d] : 0.f;
-      k[i] = live ? kn[t * qk + g * dim + d] : 0.f;
-      const float gd = live ? decay[t * g_row + h * g_head + d * g_chan] : 0.f;
-#pragma unroll
-      for (int c = 0; c < kDsCols; ++c) {
-        Sr[c][i] *= gd;
-        if (DELTA) dot[c] = fmaf(Sr[c][i], k[i], dot[c]);
-      }
+      for (int c = 0; c < 4; ++c) S[c][i] = f2::mul(S[c][i], gg);
     }
     if (DELTA) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1)
+      for (int c = 0; c < 4; ++c) {
+        uint64_t acc = f2::mul(S[c][0], k[0]);
 #pragma unroll
-        for (int c = 0; c < kDsCols; ++c) dot[c] += __shfl_xor_sync(0xffffffffu, dot[c], o);
-    }
-#pragma unroll
-    for (int c = 0; c < kDsCols; ++c) {
-      const float u = b * (v[c] - dot[c]);
-#pragma unroll
-      for (int i = 0; i < DPL; ++i) {
-        Sr[c][i] = fmaf(k[i], u, Sr[c][i]);
-        acc[c] = fmaf(Sr[c][i], q[i], acc[c]);
+        for (int i = 1; i < NP; ++i) acc = f2::fma(S[c][i], k[i], acc);
+        d4[c] = f2::sum(acc);
       }
+      ds_reduce<4>(d4, lane);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
+    for (int c = 0; c < 4; ++c) {
+      const uint64_t u = f2::both(b * ((j0 + c < vd ? vsrc[warp * 4 + c] : 0.f) - d4[c]));
+      uint64_t acc = 0;
 #pragma unroll
-      for (int c = 0; c < kDsCols; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
-    float mine = 0.f;
-#pragma unroll
-    for (int c = 0; c < kDsCols; ++c)
-      if (lane == c) mine = acc[c];
-    if (lane < kDsCols && j0 + lane < vd) out[t * hv + h * vd + j0 + lane] = mine;
-#pragma unroll
-    for (int i = 0; i < DPL; ++i) {
-      const int d = lane + 32 * i;
-      if (d < dim) {
-#pragma unroll
-        for (int c = 0; c < kDsCols; ++c)
-          if (j0 + c < vd) S_st[((int64_t)h * vd + j0 + c) * dim + d] = Sr[c][i];
+      for (int i = 0; i < NP; ++i) {
+        S[c][i] = f2::fma(k[i], u, S[c][i]);
+        acc = f2::fma(S[c][i], q[i], acc);
       }
+      o4[c] = f2::sum(acc);
     }
-    return;
-  }
-  float* sq = stage;                       // [kDsStage][dim]
-  float* sk = sq + kDsStage * dim;
-  float* sg = sk + kDsStage * dim;
-  float* sv = sg + kDsStage * dim;         // [kDsStage][32]
-  float* sb = sv + kDsStage * kDsBlockCols;   // [kDsStage]
-  float* mypart = sb + kDsStage + warp * (kDsStage * kDsCols * 33);   // [kDsStage][kDsCols][32 lanes + 1]
-  constexpr int EQ = 2 * DPL, EV = kDsStage * kDsBlockCols / kDsThreads;   // elements per thread of a [16][dim] / [16][32] tile
-  float rq[EQ], rk[EQ], rg[EQ], rv[EV], rb = 0.f;
-  auto prefetch = [&](int b0) {
-    const int nb = min(kDsStage, n_rows - b0);
-#pragma unroll
-    for (int i = 0; i < EQ; ++i) {
-      const int e = threadIdx.x + kDsThreads * i, r = e / dim, d = e - r * dim;
-      const bool live = e < nb * dim;
-      const int64_t t = start + b0 + (live ? r : 0);
-      rq[i] = live ? qn[t * qk + g * dim + d] : 0.f;
-      rk[i] = live ? kn[t * qk + g * dim + d] : 0.f;
-      rg[i] = live ? decay[t * g_row + h * g_head + d * g_chan] : 0.f;
+    ds_reduce<4>(o4, lane);
+    const float mine = lane == 0 ? o4[0] : lane == 1 ? o4[1] : lane == 2 ? o4[2] : o4[3];
+    if (lane < 4 && j0 + lane < vd) a.out[(int64_t)start * hv + (int64_t)h * vd + j0 + lane] = mine;
+  } else {
+    float* kq = stage + 2 * BUF;                                          // [kDsStage] per pair of rows: k1 g2 k2, k1 . q1
+    float* part = kq + kDsStage + warp * kDsStage * kDsPartRow;
+    if (dim < ROW) {   // zeros beyond dim, once: the copies leave them alone
+      for (int e = tid; e < 2 * BUF; e += kDsThreads) stage[e] = 0.f;
+      __syncthreads();
     }
+    auto fetch = [&](int b0, float* buf) {
+      const int nb = min(kDsStage, n_rows - b0);
+      float* sq = buf;
+      float* sk = sq + kDsStage * ROW;
+      float* sg = sk + kDsStage * ROW;
+      float* sv = sq + kDsStage * (CHAN ? 3 : 2) * ROW;
+      float* sb = sv + kDsStage * kDsCols;
+      if (a.vec) {
 #pragma unroll
-    for (int i = 0; i < EV; ++i) {
-      const int e = threadIdx.x + kDsThreads * i, r = e / kDsBlockCols, j = jb + e % kDsBlockCols;
-      rv[i] = (r < nb && j < vd) ? vn[(int64_t)(start + b0 + r) * hv + h * vd + j] : 0.f;
-    }
-    if (threadIdx.x < nb) rb = beta[(int64_t)(start + b0 + threadIdx.x) * heads + h];
-  };
-  prefetch(0);
-  for (int b0 = 0; b0 < n_rows; b0 += kDsStage) {
-    const int nb = min(kDsStage, n_rows - b0);
-    __syncthreads();   // the stage before has been consumed
-#pragma unroll
-    for (int i = 0; i < EQ; ++i) {
-      const int e = threadIdx.x + kDsThreads * i;
-      if (e < kDsStage * dim) {
-        sq[e] = rq[i];
-        sk[e] = rk[i];
-        sg[e] = rg[i];
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < EV; ++i) sv[threadIdx.x + kDsThreads * i] = rv[i];
-    if (threadIdx.x < kDsStage) sb[threadIdx.x] = rb;
-    __syncthreads();
-    if (b0 + kDsStage < n_rows) prefetch(b0 + kDsStage);
-    // the walk: state update and per-lane partial read-out sums only; the one reduction on the chain from a row to the next is
-    // S^T k.  The read-out sums over lanes follow for the whole stage.
-    for (int r = 0; r < nb; ++r) {
-      float q[DPL], k[DPL], dot[kDsCols], acc[kDsCols], v[kDsCols];
-#pragma unroll
-      for (int c = 0; c < kDsCols; ++c) {
-        dot[c] = 0.f;
-        acc[c] = 0.f;
-        v[c] = sv[r * kDsBlockCols + warp * kDsCols + c];
-      }
-#pragma unroll
-      for (int i = 0; i < DPL; ++i) {
-        const int d = lane + 32 * i;
-        const bool live = d < dim;
-        q[i] = live ? sq[r * dim + d] : 0.f;
-        k[i] = live ? sk[r * dim + d] : 0.f;
-        const float gd = live ? sg[r * dim + d] : 0.f;
-#pragma unroll
-        for (int c = 0; c < kDsCols; ++c) {
-          Sr[c][i] *= gd;
-          if (DELTA) dot[c] = fmaf(Sr[c][i], k[i], dot[c]);
+        for (int e0 = 0; e0 < kDsStage * ROW / 4; e0 += kDsThreads) {
+          const int e = e0 + tid, r = e / (ROW / 4), c = (e % (ROW / 4)) * 4;
+          if (r < nb && c < dim) {
+            f2::cp16(sq + r * ROW + c, qsrc + (b0 + r) * qk + c);
+            f2::cp16(sk + r * ROW + c, ksrc + (b0 + r) * qk + c);
+            if (CHAN) f2::cp16(sg + r * ROW + c, gsrc + (b0 + r) * a.g_row + c);
+          }
+        }
+      } else {
+        for (int e = tid; e < kDsStage * ROW; e += kDsThreads) {
+          const int r = e / ROW, c = e % ROW;
+          if (r < nb && c < dim) {
+            f2::cp4(sq + r * ROW + c, qsrc + (b0 + r) * qk + c);
+            f2::cp4(sk + r * ROW + c, ksrc + (b0 + r) * qk + c);
+            if (CHAN) f2::cp4(sg + r * ROW + c, gsrc + (b0 + r) * a.g_row + (int64_t)c * a.g_chan);
+          }
         }
       }
+#pragma unroll
+      for (int e0 = 0; e0 < kDsStage * kDsCols; e0 += kDsThreads) {
+        const int e = e0 + tid, r = e / kDsCols, c = e % kDsCols;
+        if (r < nb && jb + c < vd) f2::cp4(sv + e, vsrc + (b0 + r) * hv + c);
+      }
+      if (tid < nb) {
+        f2::cp4(sb + tid, bsrc + (int64_t)(b0 + tid) * a.heads);
+        if (!CHAN) f2::cp4(sb + kDsStage + tid, gsrc + (b0 + tid) * a.g_row);
+      }
+    };
+    fetch(0, stage);
+    for (int b0 = 0, it = 0; b0 < n_rows; b0 += kDsStage, ++it) {
+      const int nb = min(kDsStage, n_rows - b0);
+      const float* sq = stage + (it & 1) * BUF;
+      const float* sk = sq + kDsStage * ROW;
+      const float* sg = sk + kDsStage * ROW;
+      const float* sv = sq + kDsStage * (CHAN ? 3 : 2) * ROW + warp * 4;
+      const float* sb = sv - warp * 4 + kDsStage * kDsCols;
+      f2::cp_wait_all();
+      __syncthreads();   // the stage has landed for everybody, and the one before has been consumed
+      if (b0 + kDsStage < n_rows) fetch(b0 + kDsStage, stage + ((it + 1) & 1) * BUF);
       if (DELTA) {
+        for (int r = 2 * warp; r + 1 < nb; r += 2 * kDsWarps) {
+          float xy[2] = {0.f, 0.f};
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-          for (int c = 0; c < kDsCols; ++c) dot[c] += __shfl_xor_sync(0xffffffffu, dot[c], o);
-      }
-      const float b = sb[r];
-#pragma unroll
-      for (int c = 0; c < kDsCols; ++c) {
-        const float u = b * (v[c] - dot[c]);
-#pragma unroll
-        for (int i = 0; i < DPL; ++i) {
-          Sr[c][i] = fmaf(k[i], u, Sr[c][i]);
-          acc[c] = fmaf(Sr[c][i], q[i], acc[c]);
+          for (int d = 0; d < ROW; d += 32) {
+            const float k1 = sk[r * ROW + d + lane], k2 = sk[(r + 1) * ROW + d + lane];
+            xy[0] = fmaf(CHAN ? k1 * sg[(r + 1) * ROW + d + lane] : k1, k2, xy[0]);
+            xy[1] = fmaf(k1, sq[r * ROW + d + lane], xy[1]);
+          }
+          ds_reduce<2>(xy, lane);
+          if (lane == 0) *reinterpret_cast<float2*>(kq + r) = make_float2(CHAN ? xy[0] : xy[0] * sb[kDsStage + r + 1], xy[1]);
         }
-        mypart[(r * kDsCols + c) * 33 + lane] = acc[c];
+        __syncthreads();
+      }
+      auto decay_row = [&](const uint64_t (&gg)[NP]) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int i = 0; i < NP; ++i) S[c][i] = f2::mul(S[c][i], gg[i]);
+      };
+      auto decays = [&](int r, uint64_t (&gg)[NP]) {
+        if (CHAN) {
+          ds_pairs<NP>(sg + r * ROW, lane, gg);
+        } else {
+          const uint64_t x = f2::both(sb[kDsStage + r]);
+#pragma unroll
+          for (int i = 0; i < NP; ++i) gg[i] = x;
+        }
+      };
+      auto dots = [&](const uint64_t (&x)[NP], float* o) {   // the lane's part of S^T x for the four columns
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint64_t acc = f2::mul(S[c][0], x[0]);
+#pragma unroll
+          for (int i = 1; i < NP; ++i) acc = f2::fma(S[c][i], x[i], acc);
+          o[c] = f2::sum(acc);
+        }
+      };
+      int r = 0;
+      if (DELTA) {
+        for (; r + 1 < nb; r += 2) {
+          uint64_t g1[NP], g2[NP], k1[NP], k2[NP], q1[NP], q2[NP];
+          decays(r, g1);
+          ds_pairs<NP>(sk + r * ROW, lane, k1);
+          decays(r + 1, g2);
+          ds_pairs<NP>(sk + (r + 1) * ROW, lane, k2);
+          ds_pairs<NP>(sq + r * ROW, lane, q1);
+          ds_pairs<NP>(sq + (r + 1) * ROW, lane, q2);
+          const float4 v1 = *reinterpret_cast<const float4*>(sv + r * kDsCols), v2 = *reinterpret_cast<const float4*>(sv + (r + 1) * kDsCols);
+          const float2 bb = *reinterpret_cast<const float2*>(sb + r), kk = *reinterpret_cast<const float2*>(kq + r);
+          float d[8], o1[4], o2[4];
+          decay_row(g1);
+          dots(k1, d);
+          dots(q1, o1);
+          decay_row(g2);
+          dots(k2, d + 4);
+          ds_reduce<8>(d, lane);
+          const float va[4] = {v1.x, v1.y, v1.z, v1.w}, vb[4] = {v2.x, v2.y, v2.z, v2.w};
+          uint64_t kg[NP];
+#pragma unroll
+          for (int i = 0; i < NP; ++i) kg[i] = f2::mul(k1[i], g2[i]);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const float u1 = bb.x * (va[c] - d[c]), u2 = bb.y * (vb[c] - fmaf(kk.x, u1, d[4 + c]));
+            if (lane == 0) o1[c] = fmaf(kk.y, u1, o1[c]);
+            const uint64_t w1 = f2::both(u1), w2 = f2::both(u2);
+#pragma unroll
+            for (int i = 0; i < NP; ++i) S[c][i] = f2::fma(k2[i], w2, f2::fma(kg[i], w1, S[c][i]));
+          }
+          dots(q2, o2);
+          *reinterpret_cast<float4*>(part + r * kDsPartRow + 4 * lane) = make_float4(o1[0], o1[1], o1[2], o1[3]);
+          *reinterpret_cast<float4*>(part + (r + 1) * kDsPartRow + 4 * lane) = make_float4(o2[0], o2[1], o2[2], o2[3]);
+        }
+      }
+#pragma unroll 2
+      for (; r < nb; ++r) {
+        uint64_t gg[NP], k[NP], q[NP];
+        decays(r, gg);
+        ds_pairs<NP>(sk + r * ROW, lane, k);
+        ds_pairs<NP>(sq + r * ROW, lane, q);
+        const float4 v4 = *reinterpret_cast<const float4*>(sv + r * kDsCols);
+        const float va[4] = {v4.x, v4.y, v4.z, v4.w}, b = sb[r];
+        float d[4] = {0.f, 0.f, 0.f, 0.f}, o[4];
+        decay_row(gg);
+        if (DELTA) {
+          dots(k, d);
+          ds_reduce<4>(d, lane);
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const uint64_t u = f2::both(b * (va[c] - d[c]));
+#pragma unroll
+          for (int i = 0; i < NP; ++i) S[c][i] = f2::fma(k[i], u, S[c][i]);
+        }
+        dots(q, o);
+        *reinterpret_cast<float4*>(part + r * kDsPartRow + 4 * lane) = make_float4(o[0], o[1], o[2], o[3]);
+      }
+      __syncwarp();
+      {   // two lanes a row, sixteen lanes' sums each
+        const int rr = lane >> 1, half = lane & 1;
+        const float* src = part + rr * kDsPartRow + half * 64;
+        uint64_t x = 0, y = 0;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(src + 4 * (i ^ half));   // (the two lanes' banks apart)
+          x = f2::add(x, t.x);
+          y = f2::add(y, t.y);
+        }
+        float o[4] = {f2::lo(x), f2::hi(x), f2::lo(y), f2::hi(y)};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) o[c] += __shfl_xor_sync(0xffffffffu, o[c], 1);
+        if (rr < nb) {
+          float* dst = a.out + (int64_t)(start + b0 + rr) * hv + (int64_t)h * vd + j0 + 2 * half;
+          if (j0 + 2 * half < vd) dst[0] = half ? o[2] : o[0];
+          if (j0 + 2 * half + 1 < vd) dst[1] = half ? o[3] : o[1];
+        }
+      }
+      __syncwarp();
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      const int d = ds_chan<NP>(lane, i);
+      float* p = S_st + (int64_t)c * dim + d;
+      if (j0 + c >= vd || d >= dim) continue;
+      if (a.vec) {
+        *reinterpret_cast<uint64_t*>(p) = S[c][i];
+      } else {
+        p[0] = f2::lo(S[c][i]);
+        if (d + 1 < dim) p[1] = f2::hi(S[c][i]);
       }
     }
-    __syncwarp();
-    for (int x = lane; x < nb * kDsCols; x += 32) {   // lane x adds the 32 partials of sum x in lane order
-      float sum = 0.f;
-#pragma unroll 8
-      for (int l = 0; l < 32; ++l) sum += mypart[x * 33 + l];
-      const int r = x / kDsCols, c = x % kDsCols;
-      if (j0 + c < vd) out[(int64_t)(start + b0 + r) * hv + h * vd + j0 + c] = sum;
-    }
-    __syncwarp();
-  }
-#pragma unroll
-  for (int i = 0; i < DPL; ++i) {
-    const int d = lane + 32 * i;
-    if (d < dim) {
-#pragma unroll
-      for (int c = 0; c < kDsCols; ++c)
-        if (j0 + c < vd) S_st[((int64_t)h * vd + j0 + c) * dim + d] = Sr[c][i];
-    }
-  }
 }
 
 }  // namespace
@@ -398,27 +541,32 @@ int linear_scan(bool delta_rule, const float* qn, const float* kn, const float* 
   B200_REQUIRE(dim > 0 && dim <= 256 && vd > 0, B200_ERR_UNSUPPORTED, "delta_scan: key size %d outside (0, 256]", dim);
   B200_REQUIRE(heads > 0 && kv_heads > 0 && heads % kv_heads == 0, B200_ERR_INVALID, "delta_scan: %d heads over %d", heads, kv_heads);
   B200_REQUIRE(positions && seq_start && seq_slots && state, B200_ERR_INVALID, "delta_scan: null argument");
-  const dim3 grid(S, heads, (vd + kDsBlockCols - 1) / kDsBlockCols), block(kDsThreads);
-  const int dpl = (dim + 31) / 32;
-  const size_t smem = (size_t)kDsStage * (3 * dim + kDsBlockCols + 1 + kDsWarps * kDsCols * 33) * 4;   // <= 117 KiB
-#define SCAN2(D, R)                                                                                                                   \
-  do {                                                                                                                                \
-    static bool done[64] = {};                                                                                                        \
-    if (smem > 48 * 1024) B200_CUDA(ensure_dynamic_smem(delta_scan_kernel<D, R>, 128 * 1024, done));                                   \
-    B200_CUDA(launch(delta_scan_kernel<D, R>, grid, block, smem, s, qn, kn, vn, beta, decay, g_row, g_head, g_chan, positions,        \
-                     seq_start, seq_slots, state, slot_stride, out, heads, kv_heads, dim, vd));                                       \
+  const bool chan = g_chan != 0;
+  ScanArgs a = {qn, kn, vn, beta, decay, positions, seq_start, seq_slots, state, out, g_row, slot_stride, g_head, g_chan, heads, kv_heads, dim, vd, 0};
+  const auto at = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr); };
+  // wide pieces: every row and state column starts at a multiple of four floats
+  a.vec = dim % 4 == 0 && slot_stride % 4 == 0 && ((at(qn) | at(kn) | at(state)) & 15) == 0 &&
+          (!chan || (g_chan == 1 && g_row % 4 == 0 && g_head % 4 == 0 && at(decay) % 16 == 0));
+  const dim3 grid(S, heads, (vd + kDsCols - 1) / kDsCols), block(kDsThreads);
+#define SCAN3(D, R, CH)                                                                                       \
+  do {                                                                                                        \
+    static bool done[64] = {};                                                                                \
+    const size_t smem = (size_t)ds_floats(D, CH) * 4;                                                         \
+    if (smem > 48 * 1024) B200_CUDA(ensure_dynamic_smem(delta_scan_kernel<D, R, CH>, (int)smem, done));       \
+    B200_CUDA(launch(delta_scan_kernel<D, R, CH>, grid, block, smem, s, a));                                  \
   } while (0)
-#define SCAN(D)              \
-  do {                       \
-    if (delta_rule) SCAN2(D, true); \
-    else SCAN2(D, false);    \
+#define SCAN(D)                                          \
+  do {                                                   \
+    if (delta_rule && chan) SCAN3(D, true, true);        \
+    else if (delta_rule) SCAN3(D, true, false);          \
+    else if (chan) SCAN3(D, false, true);                \
+    else SCAN3(D, false, false);                         \
   } while (0)
-  if (dpl <= 1) SCAN(1);
-  else if (dpl <= 2) SCAN(2);
-  else if (dpl <= 4) SCAN(4);
-  else SCAN(8);
+  if (dim <= 64) SCAN(1);
+  else if (dim <= 128) SCAN(2);
+  else SCAN(4);
 #undef SCAN
-#undef SCAN2
+#undef SCAN3
   return B200_OK;
 }
 

@@ -362,115 +362,112 @@ moe_expert_grouped_kernel(const AT* __restrict__ x, const __nv_bfloat16* __restr
 
 
 // ---- tensor-core form: grouping and gather --------------------------------------------------------------------------------
-// One CTA of 32 warps.  Every expert's run of (token, slot) pairs starts on a tile boundary (tiles of N rows); tile_expert
-// names the owner of each tile (-1 past the last one), row_pair the pair of each row (-1 for the padding of a run).
-// Within a run the pairs keep their order (by token, then slot).  Warp w owns a contiguous stretch of the pair list and
-// walks it 32 pairs at a time; __match_any_sync gives every lane the lanes with the same expert, so a row of 32 pairs
-// costs one step whatever the number of experts.  First walk: counts per (warp, expert).  Then the runs' first rows
-// (a scan over experts) and every warp's first row inside each run (a scan over warps).  Second walk: places.
+// Every expert's run of (token, slot) pairs starts on a tile boundary (tiles of N rows); tile_expert names the owner of each tile (-1
+// past the last one), row_pair the pair of each row (-1 for the padding of a run), xg[row] = x[row_pair[row] / top] (zeros for padding
+// rows; rows of unused tiles are left alone).  Within a run the pairs keep their order (by token, then slot).
+// in_wts given (the mixing weight belongs to the expert's input): the row is scaled by its pair's weight (fp32 product, rounded
+// once), and ones[pair] = 1 so that the closing linear's per-pair factor is neutral.
+//
+// One CTA per (expert, share of its rows).  Each counts all pairs by expert (shared-memory atomics) and, per warp over a stretch of
+// the list, those of its own expert (ballots); a scan gives the expert's first tile, a second walk every pair its row; the rows of the
+// CTA's share are then copied, a warp a row.  The counting is repeated by every CTA, which costs less than a launch of its own: a single
+// grouping CTA over 8 192 pairs and 32 experts took 34 us and the gather 15 us, this @GRP@.  Bound by the latency of two walks over
+// the ids, then by the row copies.
 constexpr int kGroupThreads = 1024;
 constexpr int kGroupWarps = kGroupThreads / 32;
 
 __global__ void __launch_bounds__(kGroupThreads)
-moe_group_kernel(const int32_t* __restrict__ ids, int n_pairs, int experts, int N, int n_tiles, int32_t* __restrict__ tile_expert,
-                 int32_t* __restrict__ row_pair) {
-  extern __shared__ int32_t gsm[];
-  int32_t* start = gsm;                 // [experts] first row of the expert's run
-  int32_t* wcnt = start + experts;      // [32 warps][experts] count, then next free row, of (warp, expert)
+moe_group_gather_kernel(const int32_t* __restrict__ ids, int n_pairs, int experts, int N, int n_tiles, int32_t* __restrict__ tile_expert,
+                        int32_t* __restrict__ row_pair, const __nv_bfloat16* __restrict__ x, int top, int width, __nv_bfloat16* __restrict__ xg,
+                        const float* __restrict__ in_wts, float* __restrict__ ones) {
+  extern __shared__ int32_t hist[];   // [experts] pairs
+  __shared__ int32_t wcnt[kGroupWarps];
+  __shared__ int32_t run_tile, end_tile;   // first tile of this expert's run; tiles of all runs
   pdl_wait();
   pdl_launch_dependents();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < kGroupWarps * experts; i += kGroupThreads) wcnt[i] = 0;
-  for (int i = threadIdx.x; i < n_tiles * N; i += kGroupThreads) row_pair[i] = -1;
-  for (int i = threadIdx.x; i < n_tiles; i += kGroupThreads) tile_expert[i] = -1;
-  const int rows = (n_pairs + 31) / 32, rpw = (rows + kGroupWarps - 1) / kGroupWarps;
-  const int r0 = warp * rpw, r1 = min(r0 + rpw, rows);
-  int32_t* mine = wcnt + warp * experts;
+  const int e = blockIdx.x, part = blockIdx.y, parts = gridDim.y;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int i = tid; i < experts; i += kGroupThreads) hist[i] = 0;
+  if (tid == 0) run_tile = end_tile = 0;
   __syncthreads();
-  for (int pass = 0; pass < 2; ++pass) {
-    for (int rb = r0; rb < r1; rb += 8) {
-      int ev[8];   // eight rows' experts are requested before the first is used: the walk below is a dependent chain
+  const int seg = ((n_pairs + kGroupWarps - 1) / kGroupWarps + 31) / 32 * 32;   // a warp's stretch of the list
+  const int i0 = min(warp * seg, n_pairs), i1 = min(i0 + seg, n_pairs);
+  int mine = 0;
+  for (int i = i0; i < i1; i += 256) {
+    int ev[8];   // eight rows of 32 pairs are requested before the first is used
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int i = (rb + u) * 32 + lane;
-        ev[u] = (rb + u < r1 && i < n_pairs) ? __ldg(ids + i) : -1;
-      }
+    for (int u = 0; u < 8; ++u) ev[u] = i + u * 32 + lane < i1 ? __ldg(ids + i + u * 32 + lane) : -1;
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        if (rb + u >= r1) break;   // warp-uniform
-        const int i = (rb + u) * 32 + lane;
-        const int e = ev[u] < experts ? ev[u] : -1;
-        const unsigned same = __match_any_sync(0xffffffffu, e);
-        if (e >= 0) {
-          const int before = __popc(same & ((1u << lane) - 1u));
-          if (pass == 1) {
-            const int row = mine[e] + before;
-            if (row < n_tiles * N) row_pair[row] = i;
-          }
-          __syncwarp(same);
-          if (before == 0) mine[e] += __popc(same);   // the group's first lane
-        }
-        __syncwarp();
-      }
+    for (int u = 0; u < 8; ++u) {
+      mine += __popc(__ballot_sync(0xffffffffu, ev[u] == e));
+      if (ev[u] >= 0 && ev[u] < experts) atomicAdd(hist + ev[u], 1);
     }
-    if (pass == 1) break;
-    __syncthreads();
-    for (int e = threadIdx.x; e < experts; e += kGroupThreads) {
-      int c = 0;
-      for (int w = 0; w < kGroupWarps; ++w) c += wcnt[w * experts + e];
-      start[e] = c;   // the expert's pairs; turned into its first row below
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int run = 0;
-      for (int e = 0; e < experts; ++e) {
-        const int nt = (start[e] + N - 1) / N;
-        start[e] = run * N;
-        for (int j = 0; j < nt && run + j < n_tiles; ++j) tile_expert[run + j] = e;
-        run += nt;
-      }
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < experts; e += kGroupThreads) {
-      int at = start[e];
-      for (int w = 0; w < kGroupWarps; ++w) {
-        const int c = wcnt[w * experts + e];
-        wcnt[w * experts + e] = at;
-        at += c;
-      }
-    }
-    __syncthreads();
   }
-}
-
-// xg[row] = x[row_pair[row] / top] (zeros for padding rows); rows of unused tiles are left alone.  width % 8 == 0.
-// in_wts given (the mixing weight belongs to the expert's input): the row is scaled by its pair's weight (fp32 product,
-// rounded once), and ones[pair] = 1 so that the closing linear's per-pair factor is neutral.
-__global__ void __launch_bounds__(128)
-moe_gather_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ tile_expert, const int32_t* __restrict__ row_pair,
-                  int N, int top, int width, __nv_bfloat16* __restrict__ xg, const float* __restrict__ in_wts, float* __restrict__ ones) {
-  pdl_wait();
-  pdl_launch_dependents();
-  const int row = blockIdx.x;
-  if (tile_expert[row / N] < 0) return;
-  const int pair = row_pair[row];
+  if (lane == 0) wcnt[warp] = mine;
+  __syncthreads();
+  {   // tiles of the runs before this expert's, and of all runs
+    int before = 0, all = 0;
+    for (int i = tid; i < experts; i += kGroupThreads) {
+      const int nt = (hist[i] + N - 1) / N;
+      all += nt;
+      before += i < e ? nt : 0;
+    }
+    before = __reduce_add_sync(0xffffffffu, before);
+    all = __reduce_add_sync(0xffffffffu, all);
+    if (lane == 0) {
+      atomicAdd(&run_tile, before);
+      atomicAdd(&end_tile, all);
+    }
+  }
+  __syncthreads();
+  const int count = hist[e], tiles = (count + N - 1) / N, row0 = run_tile * N, rows = min((run_tile + tiles), n_tiles) * N - row0;
+  if (part == 0) {
+    for (int i = tid; i < tiles; i += kGroupThreads)
+      if (run_tile + i < n_tiles) tile_expert[run_tile + i] = e;
+    if (e == experts - 1)
+      for (int i = end_tile + tid; i < n_tiles; i += kGroupThreads) tile_expert[i] = -1;
+  }
+  // this CTA's share of the run's rows
+  const int share = (rows + parts - 1) / parts, lo = min(part * share, rows), hi = min(lo + share, rows);
+  int at = 0;
+  for (int w = 0; w < warp; ++w) at += wcnt[w];
+  if (at < hi && at + mine > lo)
+    for (int i = i0; i < i1; i += 256) {
+      int ev[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) ev[u] = i + u * 32 + lane < i1 ? __ldg(ids + i + u * 32 + lane) : -1;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const unsigned m = __ballot_sync(0xffffffffu, ev[u] == e);
+        const int r = at + __popc(m & ((1u << lane) - 1u));
+        if (ev[u] == e && r >= lo && r < hi) row_pair[row0 + r] = i + u * 32 + lane;
+        at += __popc(m);
+      }
+    }
+  for (int r = max(lo, count) + tid; r < hi; r += kGroupThreads) row_pair[row0 + r] = -1;
+  __syncthreads();   // the share's pairs are there for the whole CTA
   const int chunks = width >> 3;
-  uint4* dst = reinterpret_cast<uint4*>(xg + (int64_t)row * width);
-  if (pair < 0) {
-    for (int c = threadIdx.x; c < chunks; c += 128) dst[c] = make_uint4(0u, 0u, 0u, 0u);
-    return;
-  }
-  const uint4* src = reinterpret_cast<const uint4*>(x + (int64_t)(pair / top) * width);
-  if (in_wts == nullptr) {
-    for (int c = threadIdx.x; c < chunks; c += 128) dst[c] = __ldg(src + c);
-    return;
-  }
-  const float wt = in_wts[pair];
-  if (threadIdx.x == 0) ones[pair] = 1.0f;
-  for (int c = threadIdx.x; c < chunks; c += 128) {
-    const uint4 v = __ldg(src + c);
-    dst[c] = make_uint4(pack_bf16(bf16lo(v.x) * wt, bf16hi(v.x) * wt), pack_bf16(bf16lo(v.y) * wt, bf16hi(v.y) * wt),
-                        pack_bf16(bf16lo(v.z) * wt, bf16hi(v.z) * wt), pack_bf16(bf16lo(v.w) * wt, bf16hi(v.w) * wt));
+  for (int r = lo + warp; r < hi; r += kGroupWarps) {
+    const int pair = row_pair[row0 + r];
+    uint4* dst = reinterpret_cast<uint4*>(xg + (int64_t)(row0 + r) * width);
+    if (pair < 0) {
+      for (int c = lane; c < chunks; c += 32) dst[c] = make_uint4(0u, 0u, 0u, 0u);
+      continue;
+    }
+    const uint4* src = reinterpret_cast<const uint4*>(x + (int64_t)(pair / top) * width);
+    if (in_wts == nullptr) {
+#pragma unroll 8
+      for (int c = lane; c < chunks; c += 32) dst[c] = __ldg(src + c);
+      continue;
+    }
+    const float wt = in_wts[pair];
+    if (lane == 0) ones[pair] = 1.0f;
+#pragma unroll 4
+    for (int c = lane; c < chunks; c += 32) {
+      const uint4 v = __ldg(src + c);
+      dst[c] = make_uint4(pack_bf16(bf16lo(v.x) * wt, bf16hi(v.x) * wt), pack_bf16(bf16lo(v.y) * wt, bf16hi(v.y) * wt),
+                          pack_bf16(bf16lo(v.z) * wt, bf16hi(v.z) * wt), pack_bf16(bf16lo(v.w) * wt, bf16hi(v.w) * wt));
+    }
   }
 }
 
@@ -517,14 +514,14 @@ static int moe_experts_tc(const __nv_bfloat16* x, const __nv_bfloat16* w_gu, con
   __nv_bfloat16* act = reinterpret_cast<__nv_bfloat16*>(p);
   p += al256(rows * ff * 2);
   float* ones = reinterpret_cast<float*>(p);
-  const size_t smem_grp = (size_t)experts * (1 + kGroupWarps) * 4;
+  const size_t smem_grp = (size_t)experts * 4;
   B200_REQUIRE(smem_grp <= 200 * 1024, B200_ERR_UNSUPPORTED, "experts: %d experts exceed the grouping kernel", experts);
   static bool done_grp[64] = {};
-  if (smem_grp > 48 * 1024) B200_CUDA(ensure_dynamic_smem(moe_group_kernel, 200 * 1024, done_grp));
-  B200_CUDA(launch(moe_group_kernel, dim3(1), dim3(kGroupThreads), smem_grp, s, ids, T * top, experts, N, n_tiles,
-                   tile_expert, row_pair));
-  B200_CUDA(launch(moe_gather_kernel, dim3((unsigned)rows), dim3(128), (size_t)0, s, x, (const int32_t*)tile_expert,
-                   (const int32_t*)row_pair, N, top, width, xg, form.weight_input ? wts : (const float*)nullptr, ones));
+  if (smem_grp > 40 * 1024) B200_CUDA(ensure_dynamic_smem(moe_group_gather_kernel, 200 * 1024, done_grp));
+  // about 64 rows a CTA, and no more CTAs than four per SM: beyond that the repeated counting outweighs the copies it spreads
+  const int64_t per = std::max<int64_t>(1, std::min<int64_t>((int64_t)T * top / (64 * (int64_t)experts), 4 * kNumSMs / experts));
+  B200_CUDA(launch(moe_group_gather_kernel, dim3(experts, (unsigned)per), dim3(kGroupThreads), smem_grp, s, ids, T * top, experts, N, n_tiles, tile_expert,
+                   row_pair, x, top, width, xg, form.weight_input ? wts : (const float*)nullptr, ones));
   if (form.weight_input) wts = ones;
   int rc;
   static const int fuse_env = getenv("B200_MOE_FUSE_SILU") ? atoi(getenv("B200_MOE_FUSE_SILU")) : 1;

@@ -87,3 +87,51 @@ def test_mlstm_scan_portions_and_hard_gates(f32, heads, dim, vdim, pad):
                 assert (st[floats:] == 7.5).all()
                 pos[s] += cuts[s]
     assert (state[[1, 3]] == 7.5).all()
+
+
+# channel decays / one per head, delta rule / plain, heads sharing keys, sizes that leave lanes and columns idle; strided decays (g_chan 2);
+# zero decays forget everything, as do rows of zeros; rows that are not 16-byte aligned
+@pytest.mark.parametrize("rule", ["channel", "head", "plain", "plain channel", "strided"])
+@pytest.mark.parametrize("heads,kv,dim,vdim", [(2, 2, 128, 128), (4, 1, 64, 40), (3, 3, 50, 7), (2, 1, 160, 33)])
+def test_linear_scans_portions(rule, heads, kv, dim, vdim):
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    g = torch.Generator().manual_seed(dim + vdim)
+    delta, chan = rule in ("channel", "head", "strided"), rule in ("channel", "plain channel", "strided")
+    step = 2 if rule == "strided" else 1
+    floats = heads * vdim * dim
+    stride = floats + (4 if dim % 4 == 0 else 3)
+    state = torch.full((4, stride), 7.5, device=DEV)
+    slots, pos = [2, 0], [0, 0]
+    oracle = [torch.zeros(heads, vdim, dim, dtype=torch.float64) for _ in range(2)]
+    for cuts in [(3, 70), (1, 1), (2, 17), (16, 15), (33, 32)]:
+        T = sum(cuts)
+        q, k = (torch.nn.functional.normalize(torch.randn(T, kv, dim, generator=g), dim=-1) for _ in range(2))
+        v, beta = torch.randn(T, heads, vdim, generator=g), torch.sigmoid(torch.randn(T, heads, generator=g))
+        decay = torch.rand(T, heads, dim if chan else 1, generator=g) ** 0.1
+        if T > 20:
+            decay[7] = 0.0
+            k[9] = 0.0
+        wide = torch.zeros(T, heads, decay.shape[2] * step).reshape(T, heads, -1)
+        wide[:, :, ::step] = decay
+        t = [x.to(DEV).contiguous() for x in (q, k, v, beta, wide)]
+        start = [0, cuts[0], T]
+        p = list(range(pos[0], pos[0] + cuts[0])) + list(range(pos[1], pos[1] + cuts[1]))
+        ptd, std, sld, out = _i32(p), _i32(start), _i32(slots), torch.full((T, heads * vdim), float("nan"), device=DEV)
+        check(lib.b200_linear_scan(int(delta), *[x.data_ptr() for x in t], heads * wide.shape[2], wide.shape[2], step if chan else 0, ptd.data_ptr(),
+                                   std.data_ptr(), sld.data_ptr(), state.data_ptr(), stride, out.data_ptr(), 2, heads, kv, dim, vdim, None))
+        torch.cuda.synchronize()
+        for s in range(2):
+            S = oracle[s]
+            for r in range(start[s], start[s + 1]):
+                kk, qq = (x[r].double().repeat_interleave(heads // kv, 0) for x in (k, q))
+                S = S * decay[r].double()[:, None, :]
+                u = v[r].double() - ((S @ kk[:, :, None])[..., 0] if delta else 0.0)
+                S = S + (beta[r].double()[:, None] * u)[:, :, None] * kk[:, None, :]
+                want = (S @ qq[:, :, None])[..., 0].reshape(-1)
+                # fp32 throughout: sums of up to 160 terms and the roundings of some tens of live rows, 2^-24 each
+                assert (out[r].double().cpu() - want).norm() < 2e-6 * max(float(want.norm()), float(S.norm()) * 0.05), (cuts, s, r)
+            oracle[s] = S
+            st = state[slots[s]].double().cpu()
+            assert (st[:floats].reshape(S.shape) - S).norm() < 2e-6 * S.norm() and (st[floats:] == 7.5).all()
+            pos[s] += cuts[s]
+    assert (state[[1, 3]] == 7.5).all()
