@@ -59,17 +59,18 @@ latent_attn_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __restr
                        int bt_stride, const int32_t* __restrict__ row_to_seq, const int32_t* __restrict__ ctx_lens,
                        __nv_bfloat16* __restrict__ out, const int32_t* __restrict__ runs, const int32_t* __restrict__ n_runs, int heads,
                        int krow, int rank, int block_size, float scale, const float* __restrict__ sink, int n_splits,
-                       float* __restrict__ part, int window, AttnExtra ex) {
+                       float* __restrict__ part, int window, AttnExtra ex, int short_runs) {
   extern __shared__ __align__(16) unsigned char smraw[];
   pdl_wait();
   pdl_launch_dependents();
   // G query heads share kv head g; a pair i of the group is (row t0 + i / G, head g G + i % G).  Latent rows: one kv head, G = heads.
   const int G = heads / kv_heads;
-  const int item = blockIdx.x, chunk = blockIdx.y % G, g = blockIdx.y / G;
-  if (item >= *n_runs) return;
+  const int chunks = gridDim.y / kv_heads, g = blockIdx.y / chunks, n_items = *n_runs;   // CTAs that share a run's chunks of pairs
+  if (short_runs > 0 && short_runs >= 4 * n_items) return;   // rows of the step: mostly longer runs, attn_rows_tc.cu's
+  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
   const int t0 = runs[2 * item], nr = runs[2 * item + 1];
-  const int nq = nr * G, i0 = chunk * kLaPairs;
-  if (i0 >= nq) return;
+  const int nq = nr * G;
+  for (int i0 = blockIdx.y % chunks * kLaPairs; i0 < nq; i0 += chunks * kLaPairs) {
   const int ks = krow + 8;   // bf16 elements per staged row: 16-byte aligned, 4 words off a bank multiple
   // a value cache of its own (vc) is staged beside the keys in rows of rank + 8; else a key row's leading entries are its value
   const int vs = vc ? rank + 8 : ks;
@@ -246,7 +247,8 @@ latent_attn_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __restr
         }
       }
     }
-    return;
+    __syncthreads();   // shared memory is the next item's
+    continue;
   }
   // finish: sink, normalise, store
 #pragma unroll
@@ -276,6 +278,9 @@ latent_attn_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __restr
         }
       }
     }
+  }
+  __syncthreads();   // shared memory is the next item's
+  }
   }
 }
 
@@ -349,20 +354,21 @@ bool paged_attn_mma_supported(int heads, int kv_heads, int dim, int vdim) {
 static int attn_mma_launch(const float* q, const __nv_bfloat16* kc, const __nv_bfloat16* vc, int kv_heads, const int32_t* block_table,
                            int bt_stride, const int32_t* row_to_seq, const int32_t* ctx_lens, __nv_bfloat16* out, const int32_t* runs,
                            const int32_t* n_runs, int T, int heads, int krow, int rank, int block_size, float scale, const float* sink,
-                           cudaStream_t s, int n_splits, float* part, int window, const AttnExtra& ex) {
+                           cudaStream_t s, int n_splits, float* part, int window, const AttnExtra& ex, bool short_runs = false) {
   if (n_splits < 1 || part == nullptr) n_splits = 1;
   B200_REQUIRE(n_splits <= kLaMaxSplits, B200_ERR_INVALID, "attention: %d splits (at most %d)", n_splits, kLaMaxSplits);
   B200_REQUIRE(reinterpret_cast<uintptr_t>(kc) % 16 == 0 && reinterpret_cast<uintptr_t>(vc) % 16 == 0, B200_ERR_INVALID,
                "attention: cache not 16-byte aligned");
   const size_t smem = la_smem(krow, rank, vc != nullptr);
   // a run has at most 16 rows, so a kv head's group has at most 16 G pairs: G chunks of 16
-  const dim3 grid(T, heads, n_splits), block(kLaThreads);
+  // (beside attn_rows_tc.cu: fewer CTAs, one for all chunks of a run and kv head, so that leaving a step of longer runs alone costs little)
+  const dim3 grid(short_runs ? std::min(T, 256) : T, short_runs ? kv_heads : heads, n_splits), block(kLaThreads);
 #define LA2(NGV, EXV)                                                                                                               \
   do {                                                                                                                              \
     static bool done[64] = {};                                                                                                      \
     if (smem > 48 * 1024) B200_CUDA(ensure_dynamic_smem(latent_attn_mma_kernel<NGV, EXV>, 200 * 1024, done));                       \
     B200_CUDA(launch(latent_attn_mma_kernel<NGV, EXV>, grid, block, smem, s, q, kc, vc, kv_heads, block_table, bt_stride, row_to_seq, \
-                     ctx_lens, out, runs, n_runs, heads, krow, rank, block_size, scale, sink, n_splits, part, window, ex));         \
+                     ctx_lens, out, runs, n_runs, heads, krow, rank, block_size, scale, sink, n_splits, part, window, ex, short_runs ? T : 0)); \
   } while (0)
 #define LA(NGV)                 \
   do {                          \
@@ -374,7 +380,7 @@ static int attn_mma_launch(const float* q, const __nv_bfloat16* kc, const __nv_b
   else LA(4);
 #undef LA
 #undef LA2
-  if (n_splits > 1)
+  if (n_splits > 1 && !short_runs)
     B200_CUDA(launch(latent_attn_merge_kernel, dim3((T * heads + 3) / 4), dim3(128), (size_t)0, s, (const float*)part, out, T * heads, heads,
                      rank, n_splits, sink, static_cast<const __nv_bfloat16*>(ex.gate), ex.ldg));
   return B200_OK;
@@ -416,10 +422,17 @@ int paged_attn_mma(const float* q, const __nv_bfloat16* kc, const __nv_bfloat16*
   B200_REQUIRE(n_splits <= kLaMaxSplits, B200_ERR_INVALID, "attention: %d splits (at most %d)", n_splits, kLaMaxSplits);
   const auto at = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr); };
   B200_REQUIRE(at(kc) % 16 == 0 && at(vc) % 16 == 0, B200_ERR_INVALID, "attention: cache not 16-byte aligned");
-  // as for latent rows: tcgen05 wherever the shape fits, wider heads, smaller blocks and odd addresses stay here
-  if (attn_rows_tc_supported(heads, kv_heads, dim, vdim, block_size) && at(q) % 16 == 0 && at(out) % 16 == 0 && at(part) % 8 == 0) {
-    const int rc = attn_rows_tc_runs(q, kc, vc, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, kv_heads, dim, vdim,
-                                     block_size, scale, sink, s, n_splits, part, window, ex);
+  // tcgen05 for longer runs of rows; wider heads, smaller blocks and odd addresses stay here.  So do decode rows, which fill G of an
+  // item's 256 pairs there (256 rows at contexts 300..600, 16 heads over 4: 184 us against 80; 1 900 rows of three sequences 74
+  // against 278).  How the rows fall into runs is known on the device only: short steps stay here altogether, for others both kernels
+  // are launched, and the one whose kind of step it is not (runs of four rows on average) leaves at once
+  if (T > 128 && attn_rows_tc_supported(heads, kv_heads, dim, vdim, block_size) && at(q) % 16 == 0 && at(out) % 16 == 0 && at(part) % 8 == 0) {
+    int rc = attn_rows_tc_runs(q, kc, vc, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, kv_heads, dim, vdim,
+                               block_size, scale, sink, s, n_splits, part, window, ex);
+    if (rc) return rc;
+    const PdlScope after_rows;
+    rc = attn_mma_launch(q, kc, vc, kv_heads, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, dim, vdim, block_size,
+                         scale, sink, s, n_splits, part, window, ex, true);
     if (rc || n_splits == 1) return rc;
     B200_CUDA(launch(latent_attn_merge_kernel, dim3((T * heads + 3) / 4), dim3(128), (size_t)0, s, (const float*)part, out, T * heads, heads,
                      vdim, n_splits, sink, static_cast<const __nv_bfloat16*>(ex.gate), ex.ldg));

@@ -105,7 +105,7 @@ int paged_attn_prefill_plan(const int32_t* row_to_seq, const int32_t* ctx_lens, 
   B200_REQUIRE(ws && ws_bytes >= paged_attn_prefill_plan_bytes(T), B200_ERR_INVALID,
                "attn_prefill: workspace too small (%lld < %lld)", (long long)ws_bytes,
                (long long)paged_attn_prefill_plan_bytes(T));
-  B200_CUDA(launch(attn_prefill_plan_kernel, dim3(1), dim3(1024), (size_t)0, s, row_to_seq, ctx_lens, T, attn_rows_tc_rows(hq, hkv),
+  B200_CUDA(launch(attn_prefill_plan_kernel, dim3(1), dim3(1024), (size_t)0, s, row_to_seq, ctx_lens, T, attn_rows_tc_rows(T, hq, hkv),
                    static_cast<PlanItem*>(ws)));
   return B200_OK;
 }
@@ -126,6 +126,8 @@ int paged_attn_prefill_fa(const __nv_bfloat16* q, int64_t ldq, const __nv_bfloat
   if (!plan_ready) {
     const int rc0 = paged_attn_prefill_plan(row_to_seq, ctx_lens, T, hq, hkv, ws, ws_bytes, s);
     if (rc0) return rc0;
+    const PdlScope after_plan;
+    return attn_rows_tc_plan(q, ldq, kc, vc, block_table, bt_stride, ctx_lens, out, ldo, T, hq, hkv, kHeadDim, block_size, scale, ws, s);
   }
   return attn_rows_tc_plan(q, ldq, kc, vc, block_table, bt_stride, ctx_lens, out, ldo, T, hq, hkv, kHeadDim, block_size, scale, ws, s);
 }

@@ -14,7 +14,7 @@
 // per head.  The running maximum is only followed when it rises by more than 2^8 (exact: all terms are scaled alike); a warp then
 // rescales its 32 rows of O in TMEM.
 // Bound by the tensor core (HILO) or the softmax's issue slots: 2 048 rows at contexts 1001..3048, 32 heads over 8: 118 us (212 us); 1 900
-// rows of three sequences, 16 heads over 4, capped, biased, window 1024: 77 us (279 us on the mma.sync kernel of attn_latent.cu).
+// rows of three sequences, 16 heads over 4, capped, biased, window 1024: 74 us (278 us on the mma.sync kernel of attn_latent.cu).
 // Warps: four softmax warps per tile (a thread owns a pair), TMA, MMA, two that stage queries.  Every wait is bounded (tc.cuh).
 #include <stdlib.h>
 
@@ -51,12 +51,13 @@ struct RowsParams {
   const int32_t* ctx_lens;
   const int32_t* runs;         // (first row, rows) pairs whose contexts rise by one, or
   const int32_t* n_runs;
+  const int32_t* n_short;      // runs of at most 16 rows in the step (null: no other kernel takes the step)
   const RowsItem* plan;          // runs of one sequence with their longest context; plan[0].row0 of them from plan[1]
   const float* sink;
   __nv_bfloat16* out;
   int64_t ldo;
   float* part;
-  int bt_stride, heads, kv_heads, dim, vdim, block_size, n_splits, window, tile_rows;
+  int n_rows, bt_stride, heads, kv_heads, dim, vdim, block_size, n_splits, window, tile_rows;
   float scale;
   AttnExtra ex;
 };
@@ -144,7 +145,9 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
   }
   pdl_wait();
   pdl_launch_dependents();
-  const int n_runs = p.plan ? p.plan[0].row0 : *p.n_runs, n_items = n_runs * p.kv_heads * p.n_splits;
+  // (steps of mostly shorter runs are attn_latent.cu's, whose launch follows this one; run list 0 decides for both)
+  const int n_runs = p.plan ? p.plan[0].row0 : *p.n_runs;
+  const int n_items = p.n_short && p.n_rows < 4 * *p.n_short ? 0 : n_runs * p.kv_heads * p.n_splits;
   const int G = p.heads / p.kv_heads, R = p.tile_rows;
   // every other round backwards: the CTA that had the longest item of one gets the shortest of the next
   const int grid = gridDim.x, cta = blockIdx.x;
@@ -545,8 +548,12 @@ int ar_launch(const CUtensorMap& mk, const CUtensorMap& mv, const RowsParams& p,
 
 }  // namespace
 
-// rows of an item: twice what 128 pairs hold
-int attn_rows_tc_rows(int heads, int kv_heads) { return 2 * (128 / (heads / kv_heads)); }
+// rows of an item: twice what 128 pairs hold; once, where a step of two-tile items would leave half of the SMs without one (64 rows at
+// contexts 1001..1064, 32 heads over 8: 31 us with one tile an item, 38 with two)
+int attn_rows_tc_rows(int T, int heads, int kv_heads) {
+  const int tile = 128 / (heads / kv_heads);
+  return (int64_t)T * kv_heads < (int64_t)tile * kNumSMs ? tile : 2 * tile;
+}
 
 bool attn_rows_tc_supported(int heads, int kv_heads, int dim, int vdim, int block_size) {
   return heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && heads / kv_heads <= 16 && dim % 16 == 0 && dim >= 16 && dim <= 128 && vdim % 16 == 0 &&
@@ -576,7 +583,7 @@ int attn_rows_tc_plan(const __nv_bfloat16* q, int64_t ldq, const __nv_bfloat16* 
   p.dim = p.vdim = dim;
   p.block_size = block_size;
   p.n_splits = 1;
-  p.tile_rows = attn_rows_tc_rows(heads, kv_heads) / 2;
+  p.tile_rows = 128 / (heads / kv_heads);
   p.scale = scale;
   return ar_launch<__nv_bfloat16, true, false>(mk, mv, p, T, s);
 }
@@ -592,7 +599,7 @@ int attn_rows_tc_runs(const float* q, const __nv_bfloat16* kc, const __nv_bfloat
   rc = get_tensor_map_2d(vc, 1ull << 31, vdim, vdim, 64, &mv);
   if (rc) return rc;
   int list = 0;   // the longest runs whose pairs fit two tiles: 16 << list rows
-  while (list + 1 < kRunLists && (16 << (list + 1)) <= attn_rows_tc_rows(heads, kv_heads)) ++list;
+  while (list + 1 < kRunLists && (16 << (list + 1)) <= 2 * (128 / (heads / kv_heads))) ++list;
   RowsParams p = {};
   p.q = q;
   p.ldq = (int64_t)heads * dim;
@@ -601,6 +608,8 @@ int attn_rows_tc_runs(const float* q, const __nv_bfloat16* kc, const __nv_bfloat
   p.ctx_lens = ctx_lens;
   p.runs = runs + (int64_t)2 * T * list;
   p.n_runs = n_runs + list;
+  p.n_short = n_runs;
+  p.n_rows = T;
   p.sink = sink;
   p.out = out;
   p.ldo = (int64_t)heads * vdim;

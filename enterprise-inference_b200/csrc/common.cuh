@@ -152,6 +152,13 @@ struct LaunchOpts {
   bool pdl = false;  // programmatic stream serialization (set by the ctx inside a step)
 };
 LaunchOpts& launch_opts();
+// For the later launches of an entry point that launches several kernels: their prologues overlap the kernel before, which the same call
+// launched (every kernel waits for its predecessor's memory in pdl_wait).
+struct PdlScope {
+  const bool before;
+  PdlScope() : before(launch_opts().pdl) { launch_opts().pdl = true; }
+  ~PdlScope() { launch_opts().pdl = before; }
+};
 int& launch_counter();
 
 template <typename... KArgs, typename... Args>
@@ -373,7 +380,7 @@ int paged_attn_mma(const float* q, const __nv_bfloat16* kc, const __nv_bfloat16*
                    int heads, int kv_heads, int dim, int vdim, int block_size, float scale, const float* sink, cudaStream_t s,
                    int n_splits = 1, float* part = nullptr, int window = 0, const AttnExtra& ex = AttnExtra());
 // grouped-query attention for heads of at most 128 entries on tcgen05, two tiles of 128 (row, head) pairs a CTA (attn_rows_tc.cu)
-int attn_rows_tc_rows(int heads, int kv_heads);
+int attn_rows_tc_rows(int T, int heads, int kv_heads);
 bool attn_rows_tc_supported(int heads, int kv_heads, int dim, int vdim, int block_size);
 int attn_rows_tc_plan(const __nv_bfloat16* q, int64_t ldq, const __nv_bfloat16* kc, const __nv_bfloat16* vc, const int32_t* block_table, int bt_stride,
                       const int32_t* ctx_lens, __nv_bfloat16* out, int64_t ldo, int T, int heads, int kv_heads, int dim, int block_size, float scale,
@@ -444,7 +451,7 @@ int mlstm_scan(bool f32, const void* qkv, int64_t ld, int q_off, int k_off, int 
 bool mlstm_chunk_supported(const void* qkv, int64_t ld, int q_off, int k_off, int v_off, int dim, int vd);
 int mlstm_chunk(const __nv_bfloat16* qkv, int64_t ld, int q_off, int k_off, int v_off, const float* gates, const int32_t* positions,
                 const int32_t* seq_start, const int32_t* seq_slots, float* state, int64_t slot_stride, float* out, int S, int heads, int dim,
-                int vd, cudaStream_t s);
+                int vd, int min_rows, cudaStream_t s);   // sequences of at most min_rows rows are left alone
 int head_norm_gate(bool f32, const float* o, const float* w, const void* gate, int64_t ldg, void* out, int T, int heads, int vd, float eps,
                    cudaStream_t s, bool gate_silu = false);   // gate_silu: times silu(gate) instead of sigmoid(gate)
 // post-norm layer form (postnorm.cu): layer norm with bias after the sum; attention whose values are its raw keys with per-head

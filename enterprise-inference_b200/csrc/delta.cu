@@ -131,7 +131,8 @@ delta_tails_kernel(const AT* __restrict__ fused, int64_t ld, const int32_t* __re
 // shared memory, added for the whole stage after its walk.
 // 1 900 rows of three sequences, 16 heads of 128 x 128, channel decays: @D1900@ (one row per turn, unpacked, eight warps a CTA: 457 us).
 constexpr int kDsWarps = 4, kDsCols = 4 * kDsWarps, kDsStage = 16, kDsThreads = kDsWarps * 32;
-constexpr int kDsPartRow = 136;   // floats of a row of read-out sums: 32 lanes x 4 columns, rows 32 bytes apart in the banks
+constexpr int kDsFlush = 8;       // rows whose read-out sums are kept (with all 16 of a stage only two CTAs fit an SM: 342 us instead)
+constexpr int kDsPartRow = 144;   // floats of a row of read-out sums: 32 lanes x 4 columns, rows 64 bytes apart in the banks
 
 struct ScanArgs {
   const float* qn;
@@ -153,7 +154,7 @@ struct ScanArgs {
 __host__ __device__ constexpr int ds_row(int np) { return 64 * np; }
 // floats of one stage buffer: q | k | (g) rows, then per row the CTA's 16 values, beta and (head decays) g
 __host__ __device__ constexpr int ds_buf(int np, bool chan) { return kDsStage * ((chan ? 3 : 2) * ds_row(np) + kDsCols + 2); }
-__host__ __device__ constexpr int ds_floats(int np, bool chan) { return 2 * ds_buf(np, chan) + kDsStage + kDsWarps * kDsStage * kDsPartRow; }
+__host__ __device__ constexpr int ds_floats(int np, bool chan) { return 2 * ds_buf(np, chan) + kDsStage + kDsWarps * kDsFlush * kDsPartRow; }
 
 // the lane's pairs of a staged row; pair i starts at channel 2 x (NP 1), 4 x + 2 (i & 1) + 128 (i >> 1) (else) for lane x
 template <int NP>
@@ -267,7 +268,7 @@ __global__ void __launch_bounds__(kDsThreads) delta_scan_kernel(const ScanArgs a
     if (lane < 4 && j0 + lane < vd) a.out[(int64_t)start * hv + (int64_t)h * vd + j0 + lane] = mine;
   } else {
     float* kq = stage + 2 * BUF;                                          // [kDsStage] per pair of rows: k1 g2 k2, k1 . q1
-    float* part = kq + kDsStage + warp * kDsStage * kDsPartRow;
+    float* part = kq + kDsStage + warp * kDsFlush * kDsPartRow;
     if (dim < ROW) {   // zeros beyond dim, once: the copies leave them alone
       for (int e = tid; e < 2 * BUF; e += kDsThreads) stage[e] = 0.f;
       __syncthreads();
@@ -359,8 +360,10 @@ __global__ void __launch_bounds__(kDsThreads) delta_scan_kernel(const ScanArgs a
         }
       };
       int r = 0;
+      for (int f0 = 0; f0 < nb; f0 += kDsFlush) {
+      const int f1 = min(f0 + kDsFlush, nb);
       if (DELTA) {
-        for (; r + 1 < nb; r += 2) {
+        for (; r + 1 < f1; r += 2) {
           uint64_t g1[NP], g2[NP], k1[NP], k2[NP], q1[NP], q2[NP];
           decays(r, g1);
           ds_pairs<NP>(sk + r * ROW, lane, k1);
@@ -390,12 +393,12 @@ __global__ void __launch_bounds__(kDsThreads) delta_scan_kernel(const ScanArgs a
             for (int i = 0; i < NP; ++i) S[c][i] = f2::fma(k2[i], w2, f2::fma(kg[i], w1, S[c][i]));
           }
           dots(q2, o2);
-          *reinterpret_cast<float4*>(part + r * kDsPartRow + 4 * lane) = make_float4(o1[0], o1[1], o1[2], o1[3]);
-          *reinterpret_cast<float4*>(part + (r + 1) * kDsPartRow + 4 * lane) = make_float4(o2[0], o2[1], o2[2], o2[3]);
+          *reinterpret_cast<float4*>(part + (r - f0) * kDsPartRow + 4 * lane) = make_float4(o1[0], o1[1], o1[2], o1[3]);
+          *reinterpret_cast<float4*>(part + (r + 1 - f0) * kDsPartRow + 4 * lane) = make_float4(o2[0], o2[1], o2[2], o2[3]);
         }
       }
 #pragma unroll 2
-      for (; r < nb; ++r) {
+      for (; r < f1; ++r) {
         uint64_t gg[NP], k[NP], q[NP];
         decays(r, gg);
         ds_pairs<NP>(sk + r * ROW, lane, k);
@@ -415,29 +418,30 @@ __global__ void __launch_bounds__(kDsThreads) delta_scan_kernel(const ScanArgs a
           for (int i = 0; i < NP; ++i) S[c][i] = f2::fma(k[i], u, S[c][i]);
         }
         dots(q, o);
-        *reinterpret_cast<float4*>(part + r * kDsPartRow + 4 * lane) = make_float4(o[0], o[1], o[2], o[3]);
+        *reinterpret_cast<float4*>(part + (r - f0) * kDsPartRow + 4 * lane) = make_float4(o[0], o[1], o[2], o[3]);
       }
       __syncwarp();
-      {   // two lanes a row, sixteen lanes' sums each
-        const int rr = lane >> 1, half = lane & 1;
-        const float* src = part + rr * kDsPartRow + half * 64;
+      {   // four lanes a row, eight lanes' sums each
+        const int rr = lane >> 2, quarter = lane & 3;
+        const float* src = part + rr * kDsPartRow + quarter * 32;
         uint64_t x = 0, y = 0;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(src + 4 * (i ^ half));   // (the two lanes' banks apart)
+        for (int i = 0; i < 8; ++i) {
+          const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(src + 4 * (i ^ quarter));   // (the four lanes' banks apart)
           x = f2::add(x, t.x);
           y = f2::add(y, t.y);
         }
         float o[4] = {f2::lo(x), f2::hi(x), f2::lo(y), f2::hi(y)};
 #pragma unroll
-        for (int c = 0; c < 4; ++c) o[c] += __shfl_xor_sync(0xffffffffu, o[c], 1);
-        if (rr < nb) {
-          float* dst = a.out + (int64_t)(start + b0 + rr) * hv + (int64_t)h * vd + j0 + 2 * half;
-          if (j0 + 2 * half < vd) dst[0] = half ? o[2] : o[0];
-          if (j0 + 2 * half + 1 < vd) dst[1] = half ? o[3] : o[1];
+        for (int c = 0; c < 4; ++c) {
+          o[c] += __shfl_xor_sync(0xffffffffu, o[c], 1);
+          o[c] += __shfl_xor_sync(0xffffffffu, o[c], 2);
         }
+        const float mine = quarter == 0 ? o[0] : quarter == 1 ? o[1] : quarter == 2 ? o[2] : o[3];
+        if (f0 + rr < f1 && j0 + quarter < vd) a.out[(int64_t)(start + b0 + f0 + rr) * hv + (int64_t)h * vd + j0 + quarter] = mine;
       }
       __syncwarp();
+      }
     }
   }
 #pragma unroll

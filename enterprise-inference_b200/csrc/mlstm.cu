@@ -75,6 +75,7 @@ struct MlstmArgs {
   int64_t ld, slot_stride;
   int q_off, k_off, v_off, heads, dim, vd;
   float qscale;
+  int max_rows;   // sequences that bring more rows are left alone (0: none)
   int vec;        // rows of q and k can be read 16 bytes at a time
   int vec_state;  // state columns 8 bytes at a time
 };
@@ -117,7 +118,7 @@ __global__ void __launch_bounds__(kScanThreads) mlstm_scan_kernel(const MlstmArg
   const bool keeper = (blockIdx.z & 1) == 0;   // stores n and m
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int start = a.seq_start[s], n_rows = a.seq_start[s + 1] - start;
-  if (n_rows <= 0) return;   // the cluster's other CTA leaves too
+  if (n_rows <= 0 || (a.max_rows > 0 && n_rows > a.max_rows)) return;   // the cluster's other CTA leaves too
   const int heads = a.heads, dim = a.dim, vd = a.vd;
   const bool fresh = a.positions[start] == 0;
   const AT* qkv = static_cast<const AT*>(a.qkv);
@@ -508,15 +509,26 @@ int mlstm_scan(bool f32, const void* qkv, int64_t ld, int q_off, int k_off, int 
   if (S == 0) return B200_OK;
   B200_REQUIRE(dim > 0 && dim <= 256 && vd > 0, B200_ERR_UNSUPPORTED, "mlstm_scan: key size %d outside (0, 256]", dim);
   B200_REQUIRE(positions && seq_start && seq_slots && state, B200_ERR_INVALID, "mlstm_scan: null argument");
-  // longer portions of bf16 rows in chunks on the tensor cores (2 048 rows of 8 heads, 128 x 256: 154 us against 332); decode steps, fp32 rows and odd shapes row by row
-  if (!f32 && !single_rows && mlstm_chunk_supported(qkv, ld, q_off, k_off, v_off, dim, vd))
-    return mlstm_chunk((const __nv_bfloat16*)qkv, ld, q_off, k_off, v_off, gates, positions, seq_start, seq_slots, state, slot_stride, out, S, heads,
-                       dim, vd, s);
-  MlstmArgs a = {qkv, gates, positions, seq_start, seq_slots, state, out, ld, slot_stride, q_off, k_off, v_off, heads, dim, vd, 1.0f / sqrtf((float)dim), 0, 0};
+  // longer portions of bf16 rows in chunks on the tensor cores (2 048 rows of 8 heads, 128 x 256: 141 us against 332); decode steps, fp32
+  // rows and odd shapes row by row.  How many rows a sequence brings is known on the device only: both kernels are launched, each
+  // leaves the other's sequences alone.  Steps of many sequences are mostly decode rows, and the walk fills the SMs.  A chunk kernel's first chunk costs about what 96 rows of the walk do (64 rows of four
+  // sequences: 16 us row by row, 22 in chunks)
+  constexpr int kWalkRows = 96;
+  const bool chunks = !f32 && !single_rows && S <= 16 && mlstm_chunk_supported(qkv, ld, q_off, k_off, v_off, dim, vd);
+  if (chunks) {
+    const int rc = mlstm_chunk((const __nv_bfloat16*)qkv, ld, q_off, k_off, v_off, gates, positions, seq_start, seq_slots, state, slot_stride, out, S,
+                               heads, dim, vd, kWalkRows, s);
+    if (rc) return rc;
+  }
+  MlstmArgs a = {qkv, gates, positions, seq_start, seq_slots, state, out, ld, slot_stride, q_off, k_off, v_off, heads, dim, vd, 1.0f / sqrtf((float)dim), chunks ? kWalkRows : 0, 0, 0};
   const auto at = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr); };
   const int per = f32 ? 4 : 8;   // elements of a 16-byte piece
   a.vec = dim % per == 0 && ld % per == 0 && q_off % per == 0 && k_off % per == 0 && at(qkv) % 16 == 0;
   a.vec_state = dim % 2 == 0 && slot_stride % 2 == 0 && at(state) % 8 == 0;
+  if (chunks) {
+    const PdlScope after_chunks;
+    return mlstm_scan_t<__nv_bfloat16>(a, S, false, s);
+  }
   return f32 ? mlstm_scan_t<float>(a, S, single_rows, s) : mlstm_scan_t<__nv_bfloat16>(a, S, single_rows, s);
 }
 

@@ -12,7 +12,7 @@
 // Warps w of 8: rows 16 (w % 4) of P and O, the key blocks (and for Q S_0 the dimensions) dealt to the two warps of a row group, whose
 // sums meet in shared memory; dimensions 16 w of the state, kept in fp32 accumulator fragments.  A ninth warp works out the next
 // chunk's gate scalars.  Rows arrive by cp.async a chunk ahead.
-// Bound by latency (about 800 instructions a warp and chunk, two barriers).  2 048 rows of 8 heads, 128 x 256: 154 us against 723 us
+// Bound by latency (about 800 instructions a warp and chunk, two barriers).  2 048 rows of 8 heads, 128 x 256: 141 us against 723 us
 // of the scalar walk and 332 us of the packed one; error of the results against 64 bits 6.8e-7 (walk 1.2e-6), of the state 7.5e-8 (1.5e-7).
 #include <algorithm>
 
@@ -35,6 +35,7 @@ struct MlstmChunkArgs {
   int64_t ld, slot_stride;
   int q_off, k_off, v_off, heads, dim, vd;
   float qscale;
+  int min_rows;   // sequences that bring no more rows are left alone
 };
 
 __device__ __forceinline__ uint32_t sa(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -76,14 +77,15 @@ struct GateRows {   // of one chunk
 template <int KS>
 struct McSmem {
   static constexpr int QS = KS * 16 + 8;   // bf16 per staged q / k row
-  __nv_bfloat16 q[2][kMcRows][QS], k[2][kMcRows][QS], v[2][kMcRows][kMcW], w[3][kMcRows][kMcW], s[2][3][KS * 16][kMcW];
+  __nv_bfloat16 q[2][kMcRows][QS], k[2][kMcRows][QS], v[2][kMcRows][kMcW], w[3][kMcRows][kMcW], s[3][KS * 16][kMcW];
   float o[kMcRows][kMcW + 2];   // one warp's sums of a row group, for the other
   GateRows gate[2];
 };
 
 // KS: 16-wide steps over the (zero padded) key dimensions
-template <int KS>
-__global__ void __launch_bounds__(kMcThreads) mlstm_chunk_kernel(const MlstmChunkArgs a) {
+// CTAS: CTAs that share an SM (two when there are more than SMs: fewer registers each)
+template <int KS, int CTAS>
+__global__ void __launch_bounds__(kMcThreads, CTAS) mlstm_chunk_kernel(const MlstmChunkArgs a) {
   extern __shared__ __align__(16) unsigned char raw[];
   McSmem<KS>& sm = *reinterpret_cast<McSmem<KS>*>(raw);
 
@@ -93,7 +95,7 @@ __global__ void __launch_bounds__(kMcThreads) mlstm_chunk_kernel(const MlstmChun
   const bool keeper = (blockIdx.z & 1) == 0;   // stores n and m
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
   const int start = a.seq_start[s], n_rows = a.seq_start[s + 1] - start;
-  if (n_rows <= 0) return;   // the cluster's other CTA leaves too
+  if (n_rows <= a.min_rows) return;   // the cluster's other CTA leaves too
   const int heads = a.heads, dim = a.dim, vd = a.vd;
   const bool fresh = a.positions[start] == 0;
   float* slot = a.state + (int64_t)a.seq_slots[s] * a.slot_stride;                                     // S [heads][vd][dim]
@@ -131,7 +133,7 @@ __global__ void __launch_bounds__(kMcThreads) mlstm_chunk_kernel(const MlstmChun
         if (n == 2 && col == kMcCols) S[n][i] = n_st[d];
       }
     }
-  auto publish = [&](int buf) {   // the state as three bf16 terms, for everybody's Q S
+  auto publish = [&]() {   // the state as three bf16 terms, for everybody's Q S (nobody reads it between a chunk's second barrier and the next one's first)
     if (warp < KS) {
 #pragma unroll
       for (int n = 0; n < 3; ++n)
@@ -140,7 +142,7 @@ __global__ void __launch_bounds__(kMcThreads) mlstm_chunk_kernel(const MlstmChun
           uint32_t t[3];
           split3(S[n][2 * hf], S[n][2 * hf + 1], t[0], t[1], t[2]);
 #pragma unroll
-          for (int x = 0; x < 3; ++x) *reinterpret_cast<uint32_t*>(&sm.s[buf][x][warp * 16 + g + hf * 8][n * 8 + 2 * t4]) = t[x];
+          for (int x = 0; x < 3; ++x) *reinterpret_cast<uint32_t*>(&sm.s[x][warp * 16 + g + hf * 8][n * 8 + 2 * t4]) = t[x];
         }
     }
   };
@@ -201,7 +203,7 @@ __global__ void __launch_bounds__(kMcThreads) mlstm_chunk_kernel(const MlstmChun
   for (int e = tid; e < 2 * kMcRows * 8; e += kMcThreads) sm.v[e / (kMcRows * 8)][(e / 8) % kMcRows][kMcCols + e % 8] = __float2bfloat16_rn(e % 8 == 0 ? 1.f : 0.f);
   if (warp < kMcGate) {
     fetch(0);
-    publish(0);
+    publish();
   } else {
     fetch_gates(0);
     gate_chunk(sm.gate[0]);
@@ -275,8 +277,8 @@ __global__ void __launch_bounds__(kMcThreads) mlstm_chunk_kernel(const MlstmChun
 #pragma unroll
       for (int x = 2; x >= 0; --x) {
         uint32_t b4[4], b2[2];
-        ldsm4t(b4, &sm.s[buf][x][k * 16 + (lane & 15)][(lane >> 4) * 8]);
-        ldsm2t(b2, &sm.s[buf][x][k * 16 + (lane & 15)][kMcCols]);
+        ldsm4t(b4, &sm.s[x][k * 16 + (lane & 15)][(lane >> 4) * 8]);
+        ldsm2t(b2, &sm.s[x][k * 16 + (lane & 15)][kMcCols]);
         mma(I[x][0], qk, b4[0], b4[1]);
         mma(I[x][1], qk, b4[2], b4[3]);
         mma(I[x][2], qk, b2[0], b2[1]);
@@ -316,7 +318,7 @@ __global__ void __launch_bounds__(kMcThreads) mlstm_chunk_kernel(const MlstmChun
 #pragma unroll
         for (int i = 0; i < 4; ++i) S[n][i] = fmaf(gamma, S[n][i], (U[2][n][i] + U[1][n][i]) + U[0][n][i]);
     }
-    publish(buf ^ 1);
+    publish();
     if (!hf) {
 #pragma unroll
       for (int x = 0; x < 2; ++x) {
@@ -369,18 +371,24 @@ bool mlstm_chunk_supported(const void* qkv, int64_t ld, int q_off, int k_off, in
 
 int mlstm_chunk(const __nv_bfloat16* qkv, int64_t ld, int q_off, int k_off, int v_off, const float* gates, const int32_t* positions,
                 const int32_t* seq_start, const int32_t* seq_slots, float* state, int64_t slot_stride, float* out, int S, int heads, int dim,
-                int vd, cudaStream_t s) {
+                int vd, int min_rows, cudaStream_t s) {
   const MlstmChunkArgs a = {qkv, gates, positions, seq_start, seq_slots, state, out, ld, slot_stride, q_off, k_off, v_off, heads, dim, vd,
-                            1.0f / sqrtf((float)dim)};
+                            1.0f / sqrtf((float)dim), std::max(min_rows, 0)};
   const dim3 grid(S, heads, 2 * mlstm_col_blocks(vd)), block(kMcThreads), cluster(1, 1, 2);
-#define CHUNK(K)                                                                                          \
+#define CHUNK(K, C)                                                                                       \
   do {                                                                                                    \
     static bool done[64] = {};                                                                            \
-    B200_CUDA(ensure_dynamic_smem(mlstm_chunk_kernel<K>, (int)sizeof(McSmem<K>), done));                  \
-    B200_CUDA(launch_cluster(mlstm_chunk_kernel<K>, grid, block, sizeof(McSmem<K>), s, cluster, a));      \
+    B200_CUDA(ensure_dynamic_smem(mlstm_chunk_kernel<K, C>, (int)sizeof(McSmem<K>), done));               \
+    B200_CUDA(launch_cluster(mlstm_chunk_kernel<K, C>, grid, block, sizeof(McSmem<K>), s, cluster, a));   \
   } while (0)
-  if (dim <= 64) CHUNK(4);
-  else CHUNK(8);
+  const bool many = (int64_t)grid.x * grid.y * grid.z > kNumSMs;
+  if (dim <= 64) {
+    if (many) CHUNK(4, 2);
+    else CHUNK(4, 1);
+  } else {
+    if (many) CHUNK(8, 2);
+    else CHUNK(8, 1);
+  }
 #undef CHUNK
   return B200_OK;
 }

@@ -371,7 +371,7 @@ moe_expert_grouped_kernel(const AT* __restrict__ x, const __nv_bfloat16* __restr
 // One CTA per (expert, share of its rows).  Each counts all pairs by expert (shared-memory atomics) and, per warp over a stretch of
 // the list, those of its own expert (ballots); a scan gives the expert's first tile, a second walk every pair its row; the rows of the
 // CTA's share are then copied, a warp a row.  The counting is repeated by every CTA, which costs less than a launch of its own: a single
-// grouping CTA over 8 192 pairs and 32 experts took 34 us and the gather 15 us, this @GRP@.  Bound by the latency of two walks over
+// grouping CTA over 8 192 pairs and 32 experts took 34 us and the gather 15 us, this 15.  Bound by the latency of two walks over
 // the ids, then by the row copies.
 constexpr int kGroupThreads = 1024;
 constexpr int kGroupWarps = kGroupThreads / 32;
@@ -522,6 +522,7 @@ static int moe_experts_tc(const __nv_bfloat16* x, const __nv_bfloat16* w_gu, con
   const int64_t per = std::max<int64_t>(1, std::min<int64_t>((int64_t)T * top / (64 * (int64_t)experts), 4 * kNumSMs / experts));
   B200_CUDA(launch(moe_group_gather_kernel, dim3(experts, (unsigned)per), dim3(kGroupThreads), smem_grp, s, ids, T * top, experts, N, n_tiles, tile_expert,
                    row_pair, x, top, width, xg, form.weight_input ? wts : (const float*)nullptr, ones));
+  const PdlScope after_grouping;
   if (form.weight_input) wts = ones;
   int rc;
   static const int fuse_env = getenv("B200_MOE_FUSE_SILU") ? atoi(getenv("B200_MOE_FUSE_SILU")) : 1;
@@ -574,6 +575,7 @@ int moe_route(bool f32, const void* x, const __nv_bfloat16* w_router, const floa
     const int rc = linear_tc((const __nv_bfloat16*)x, width, w_router, nullptr, nullptr, n_rows, T, n_rows, width, lin_ws,
                              lin_ws_bytes, &ex, s);
     if (rc) return rc;
+    const PdlScope after_logits;
     B200_CUDA(launch(moe_select_kernel, dim3((T + kSelWarps - 1) / kSelWarps), dim3(kSelWarps * 32), smem_sel, s,
                      (const float*)logits_ws, bias, T, experts, top, groups, keep, out_ids, out_w, sg, rf));
     return B200_OK;

@@ -2048,6 +2048,7 @@ extern "C" int b200_latent_attn(const float* q, const void* cache, const int32_t
   B200_REQUIRE(q && cache && block_table && ctx_lens && out && workspace && block_size > 0, B200_ERR_INVALID, "latent_attn: bad argument");
   int rc = paged_attn_runs_plan(row_to_seq, ctx_lens, T, workspace, (cudaStream_t)stream);
   if (rc) return rc;
+  const PdlScope after_plan;
   return latent_attn_mma(q, (const __nv_bfloat16*)cache, block_table, bt_stride, row_to_seq, ctx_lens, (__nv_bfloat16*)out,
                          static_cast<const int32_t*>(workspace) + 8, static_cast<const int32_t*>(workspace), T, heads, k_row, rank,
                          block_size, scale, sink, (cudaStream_t)stream, n_splits, part);
@@ -2095,6 +2096,7 @@ extern "C" int b200_latent_attn_window(const float* q, const void* cache, const 
                "latent_attn_window: bad argument");
   int rc = paged_attn_runs_plan(row_to_seq, ctx_lens, T, workspace, (cudaStream_t)stream);
   if (rc) return rc;
+  const PdlScope after_plan;
   return latent_attn_mma(q, (const __nv_bfloat16*)cache, block_table, bt_stride, row_to_seq, ctx_lens, (__nv_bfloat16*)out,
                          static_cast<const int32_t*>(workspace) + 8, static_cast<const int32_t*>(workspace), T, heads, k_row, rank,
                          block_size, scale, sink, (cudaStream_t)stream, 1, nullptr, window);
@@ -2150,6 +2152,7 @@ extern "C" int b200_paged_attn_mma(const float* q, const void* kc, const void* v
                "paged_attn_mma: bad argument");
   int rc = paged_attn_runs_plan(row_to_seq, ctx_lens, T, workspace, (cudaStream_t)stream);
   if (rc) return rc;
+  const PdlScope after_plan;
   return paged_attn_mma(q, (const __nv_bfloat16*)kc, (const __nv_bfloat16*)vc, block_table, bt_stride, row_to_seq, ctx_lens, (__nv_bfloat16*)out,
                         static_cast<const int32_t*>(workspace) + 8, static_cast<const int32_t*>(workspace), T, heads, kv_heads, dim, vdim,
                         block_size, scale, sink, (cudaStream_t)stream, n_splits, part, window);
@@ -2315,6 +2318,7 @@ extern "C" int b200_paged_attn_biased(int32_t f32, int32_t form, const float* q,
     B200_REQUIRE(!f32, B200_ERR_UNSUPPORTED, "paged_attn_biased: the tensor-core form takes bf16 caches");
     int rc = paged_attn_runs_plan(row_to_seq, ctx_lens, T, ws, s);
     if (rc) return rc;
+    const PdlScope after_plan;
     return paged_attn_mma(q, (const __nv_bfloat16*)kc, (const __nv_bfloat16*)vc, block_table, bt_stride, row_to_seq, ctx_lens, (__nv_bfloat16*)out,
                           static_cast<const int32_t*>(ws) + 8, static_cast<const int32_t*>(ws), T, heads, kv_heads, dim, vdim, block_size, scale, nullptr, s,
                           n_splits, part, window, ex);
@@ -2403,6 +2407,7 @@ extern "C" int b200_paged_attn_kept(int32_t f32, int32_t form, const float* q, c
     B200_REQUIRE(!f32, B200_ERR_UNSUPPORTED, "paged_attn_kept: the tensor-core form takes bf16 caches");
     int rc = paged_attn_runs_plan(row_to_seq, ctx_lens, T, ws, s);
     if (rc) return rc;
+    const PdlScope after_plan;
     return paged_attn_mma(q, (const __nv_bfloat16*)kc, (const __nv_bfloat16*)vc, block_table, bt_stride, row_to_seq, ctx_lens, (__nv_bfloat16*)out,
                           static_cast<const int32_t*>(ws) + 8, static_cast<const int32_t*>(ws), T, heads, kv_heads, dim, vdim, block_size, scale, sink, s,
                           n_splits, part, window, ex);

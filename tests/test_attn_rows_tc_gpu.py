@@ -96,7 +96,7 @@ def test_runs_of_rows_tile_edges(heads, kv, dim, vdim, bs, form):
     _close(out, want)
 
 
-@pytest.mark.parametrize("heads,kv", [(8, 2), (4, 4), (8, 1), (10, 2)])
+@pytest.mark.parametrize("heads,kv", [(8, 2), (4, 4), (8, 1), (10, 2), (64, 8), (32, 32)])
 def test_prefill_rows_of_the_decoder_stack(heads, kv):
     lib, check = pkg("_abi").lib(), pkg("_abi").check
     g, q, rows, (kc, vc), bt, seq, ctx, T = _case(heads, kv, 128, 128, 128, heads * 7 + kv)
@@ -108,3 +108,31 @@ def test_prefill_rows_of_the_decoder_stack(heads, kv):
                                       out.data_ptr(), heads * 128, T, heads, kv, 128, 500, 128 ** -0.5, ws.data_ptr(), wsb, None))
     torch.cuda.synchronize()
     _close(out, _oracle(q, rows, 128 ** -0.5))
+
+
+@pytest.mark.parametrize("ns", [1, 2])
+def test_long_steps_of_decode_rows_go_to_the_other_kernel(ns):
+    """More than 128 rows, almost all of them runs of one: which kernel works is decided on the device, the other leaves."""
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    heads, kv, dim, bs, T = 8, 2, 64, 64, 150
+    g = torch.Generator().manual_seed(3)
+    K, V = (torch.randn(500, kv, dim, generator=g).to(torch.bfloat16) for _ in range(2))
+    kc, vc = (torch.cat([x, torch.zeros(12, kv, dim, dtype=torch.bfloat16)]).reshape(8, bs, kv, dim).transpose(1, 2).contiguous().to(DEV) for x in (K, V))
+    ctxs = [(37 * i) % 500 + 1 for i in range(T)]
+    q = torch.randn(T, heads, dim, generator=g).to(torch.bfloat16)
+    bt = torch.arange(8, dtype=torch.int32, device=DEV)[None, :].repeat(T, 1).contiguous()
+    seq, ctx = torch.arange(T, dtype=torch.int32, device=DEV), torch.tensor(ctxs, dtype=torch.int32, device=DEV)
+    ws = torch.zeros(int(lib.b200_paged_attn_anydim_workspace_bytes(T)), dtype=torch.uint8, device=DEV)
+    out = torch.full((T, heads, dim), float("nan"), dtype=torch.bfloat16, device=DEV)
+    part = torch.full((T * heads * ns * (dim + 2),), float("nan"), device=DEV)
+    qd = q.float().to(DEV)
+    check(lib.b200_paged_attn_mma(qd.data_ptr(), kc.data_ptr(), vc.data_ptr(), bt.data_ptr(), 8, seq.data_ptr(), ctx.data_ptr(), out.data_ptr(), T, heads,
+                                  kv, dim, dim, bs, dim ** -0.5, None, ws.data_ptr(), 0, ns, part.data_ptr() if ns > 1 else None, None))
+    torch.cuda.synchronize()
+    got = out.double().cpu()
+    for t in range(T):
+        k, v = (x[:ctxs[t]].double().repeat_interleave(heads // kv, 1) for x in (K, V))
+        w = torch.softmax(torch.einsum("hd,chd->hc", q[t].double(), k) * dim ** -0.5, -1)
+        want = torch.einsum("hc,chd->hd", w, v)
+        # weights and results rounded to bf16 once each: 2^-9 of the largest value, 2^-9 of the result
+        assert ((got[t] - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -9 * v.abs().max()).all(), t
