@@ -447,11 +447,6 @@ int64_t mlstm_state_floats(int heads, int dim, int vd);
 int mlstm_scan(bool f32, const void* qkv, int64_t ld, int q_off, int k_off, int v_off, const float* gates, const int32_t* positions,
                const int32_t* seq_start, const int32_t* seq_slots, float* state, int64_t slot_stride, float* out, int S, int heads,
                int dim, int vd, cudaStream_t s, bool single_rows = false);   // single_rows: every sequence of the step has one row
-// the same over bf16 rows in chunks of 64 on the tensor cores (mlstm_chunk.cu); mlstm_scan takes it for steps of longer portions
-bool mlstm_chunk_supported(const void* qkv, int64_t ld, int q_off, int k_off, int v_off, int dim, int vd);
-int mlstm_chunk(const __nv_bfloat16* qkv, int64_t ld, int q_off, int k_off, int v_off, const float* gates, const int32_t* positions,
-                const int32_t* seq_start, const int32_t* seq_slots, float* state, int64_t slot_stride, float* out, int S, int heads, int dim,
-                int vd, int min_rows, cudaStream_t s);   // sequences of at most min_rows rows are left alone
 int head_norm_gate(bool f32, const float* o, const float* w, const void* gate, int64_t ldg, void* out, int T, int heads, int vd, float eps,
                    cudaStream_t s, bool gate_silu = false);   // gate_silu: times silu(gate) instead of sigmoid(gate)
 // post-norm layer form (postnorm.cu): layer norm with bias after the sum; attention whose values are its raw keys with per-head

@@ -8,35 +8,23 @@
 // w V) enters the bf16 MMA as three bf16 terms (24 bits) against rows that are bf16 to begin with, accumulators are fp32.  n is carried
 // as a 17th column with value 1.
 //
-// One CTA per (sequence, head, 16 value columns) walks the chunks: a cluster of two shares one stored copy of n and m, as in mlstm.cu.
+// One CTA per (sequence, head, 16 value columns) walks the chunks; the two of a cluster share one stored copy of n and m, and a barrier keeps either from storing before both have read.
 // Warps w of 8: rows 16 (w % 4) of P and O, the key blocks (and for Q S_0 the dimensions) dealt to the two warps of a row group, whose
 // sums meet in shared memory; dimensions 16 w of the state, kept in fp32 accumulator fragments.  A ninth warp works out the next
 // chunk's gate scalars.  Rows arrive by cp.async a chunk ahead.
-// Bound by latency (about 800 instructions a warp and chunk, two barriers).  2 048 rows of 8 heads, 128 x 256: 141 us against 723 us
-// of the scalar walk and 332 us of the packed one; error of the results against 64 bits 6.8e-7 (walk 1.2e-6), of the state 7.5e-8 (1.5e-7).
+// Bound by latency (about 800 instructions a warp and chunk, two barriers).  2 048 rows of 8 heads, 128 x 256: 140 us against 724 us
+// of the scalar walk; error of the results against 64 bits 6.8e-7 (walk 1.2e-6), of the state 7.5e-8 (1.5e-7).
 #include <algorithm>
 
-#include "common.cuh"
+#include "mlstm_walk.cuh"
+#include <algorithm>
 
 namespace b200 {
 namespace {
 
 constexpr int kMcRows = 64, kMcCols = 16, kMcW = 24;   // rows of a chunk; value columns; columns with n and its padding (bf16 rows of 48 bytes)
 constexpr int kMcThreads = 288, kMcGate = 8;
-
-struct MlstmChunkArgs {
-  const __nv_bfloat16* qkv;
-  const float* gates;
-  const int32_t* positions;
-  const int32_t* seq_start;
-  const int32_t* seq_slots;
-  float* state;
-  float* out;
-  int64_t ld, slot_stride;
-  int q_off, k_off, v_off, heads, dim, vd;
-  float qscale;
-  int min_rows;   // sequences that bring no more rows are left alone
-};
+static_assert(kMcThreads == kScanThreads && 2 * kMcCols == kScanCols, "the walk takes a pair's columns with one CTA's threads");
 
 __device__ __forceinline__ uint32_t sa(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const void* p) {
@@ -85,7 +73,7 @@ struct McSmem {
 // KS: 16-wide steps over the (zero padded) key dimensions
 // CTAS: CTAs that share an SM (two when there are more than SMs: fewer registers each)
 template <int KS, int CTAS>
-__global__ void __launch_bounds__(kMcThreads, CTAS) mlstm_chunk_kernel(const MlstmChunkArgs a) {
+__global__ void __launch_bounds__(kMcThreads, CTAS) mlstm_chunk_kernel(const MlstmArgs a) {
   extern __shared__ __align__(16) unsigned char raw[];
   McSmem<KS>& sm = *reinterpret_cast<McSmem<KS>*>(raw);
 
@@ -95,7 +83,10 @@ __global__ void __launch_bounds__(kMcThreads, CTAS) mlstm_chunk_kernel(const Mls
   const bool keeper = (blockIdx.z & 1) == 0;   // stores n and m
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
   const int start = a.seq_start[s], n_rows = a.seq_start[s + 1] - start;
-  if (n_rows <= a.min_rows) return;   // the cluster's other CTA leaves too
+  if (n_rows < kChunkFrom) {   // (nothing to do at all among them) the pair's first CTA takes both halves' columns
+    if (keeper && !a.both) mlstm_walk<__nv_bfloat16, KS / 4>(a, reinterpret_cast<float*>(raw), zb, nz);
+    return;
+  }
   const int heads = a.heads, dim = a.dim, vd = a.vd;
   const bool fresh = a.positions[start] == 0;
   float* slot = a.state + (int64_t)a.seq_slots[s] * a.slot_stride;                                     // S [heads][vd][dim]
@@ -103,7 +94,7 @@ __global__ void __launch_bounds__(kMcThreads, CTAS) mlstm_chunk_kernel(const Mls
   float* m_st = slot + (int64_t)heads * vd * dim + (int64_t)heads * nz * dim + (int64_t)h * nz + zb;   // m [heads][nz]
   float* S_st = slot + ((int64_t)h * vd + jb) * dim;
   const int n_chunks = (n_rows + kMcRows - 1) / kMcRows;
-  const __nv_bfloat16* src = a.qkv + (int64_t)start * a.ld;
+  const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(a.qkv) + (int64_t)start * a.ld;
 
   auto fetch = [&](int c) {   // warps 0..7
     const int b0 = c * kMcRows, buf = c & 1;
@@ -364,25 +355,22 @@ __global__ void __launch_bounds__(kMcThreads, CTAS) mlstm_chunk_kernel(const Mls
 }  // namespace
 
 // rows of q, k and v in 16-byte pieces, key dimensions within eight 16-wide steps
-bool mlstm_chunk_supported(const void* qkv, int64_t ld, int q_off, int k_off, int v_off, int dim, int vd) {
-  return dim > 0 && dim <= 128 && dim % 8 == 0 && vd % 8 == 0 && ld % 8 == 0 && (q_off | k_off | v_off) % 8 == 0 &&
-         reinterpret_cast<uintptr_t>(qkv) % 16 == 0;
+bool mlstm_chunk_supported(const MlstmArgs& a) {
+  return a.dim > 0 && a.dim <= 128 && a.dim % 8 == 0 && a.vd % 8 == 0 && a.ld % 8 == 0 && (a.q_off | a.k_off | a.v_off) % 8 == 0 &&
+         reinterpret_cast<uintptr_t>(a.qkv) % 16 == 0;
 }
 
-int mlstm_chunk(const __nv_bfloat16* qkv, int64_t ld, int q_off, int k_off, int v_off, const float* gates, const int32_t* positions,
-                const int32_t* seq_start, const int32_t* seq_slots, float* state, int64_t slot_stride, float* out, int S, int heads, int dim,
-                int vd, int min_rows, cudaStream_t s) {
-  const MlstmChunkArgs a = {qkv, gates, positions, seq_start, seq_slots, state, out, ld, slot_stride, q_off, k_off, v_off, heads, dim, vd,
-                            1.0f / sqrtf((float)dim), std::max(min_rows, 0)};
-  const dim3 grid(S, heads, 2 * mlstm_col_blocks(vd)), block(kMcThreads), cluster(1, 1, 2);
+int mlstm_chunk(const MlstmArgs& a, int S, cudaStream_t s) {
+  const dim3 grid(S, a.heads, 2 * mlstm_col_blocks(a.vd)), block(kMcThreads), cluster(1, 1, 2);
 #define CHUNK(K, C)                                                                                       \
   do {                                                                                                    \
     static bool done[64] = {};                                                                            \
-    B200_CUDA(ensure_dynamic_smem(mlstm_chunk_kernel<K, C>, (int)sizeof(McSmem<K>), done));               \
-    B200_CUDA(launch_cluster(mlstm_chunk_kernel<K, C>, grid, block, sizeof(McSmem<K>), s, cluster, a));   \
+    constexpr size_t smem = std::max(sizeof(McSmem<K>), (size_t)ml_floats(K / 4) * 4);   /* chunks; walk */    \
+    B200_CUDA(ensure_dynamic_smem(mlstm_chunk_kernel<K, C>, (int)smem, done));                            \
+    B200_CUDA(launch_cluster(mlstm_chunk_kernel<K, C>, grid, block, smem, s, cluster, a));                \
   } while (0)
   const bool many = (int64_t)grid.x * grid.y * grid.z > kNumSMs;
-  if (dim <= 64) {
+  if (a.dim <= 64) {
     if (many) CHUNK(4, 2);
     else CHUNK(4, 1);
   } else {
