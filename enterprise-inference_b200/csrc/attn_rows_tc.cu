@@ -10,7 +10,8 @@
 // The weights overwrite the scores in TMEM (A operand of the second product): per 32 scores 16 columns of bf16 pairs and, HILO, 16 more
 // with what rounding took from them (P then has 16 bits, as attn_tc.cu has it).  TMEM per tile of pairs: two score buffers of 64
 // columns, O 128.
-// Scores may be capped, biased by distance, windowed with kept first keys (EX); outputs may have a sink in the denominator and a gate
+// Scores may be capped, biased by distance (each score takes its own distance's bias and no other: tables may end in -inf or any sentinel),
+// windowed with kept first keys (EX); outputs may have a sink in the denominator and a gate
 // per head.  The running maximum is only followed when it rises by more than 2^8 (exact: all terms are scaled alike); a warp then
 // rescales its 32 rows of O in TMEM.
 // Bound by the tensor core (HILO) or the softmax's issue slots: 2 048 rows at contexts 1001..3048, 32 heads over 8: 118 us (212 us); 1 900
@@ -326,16 +327,20 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     constexpr float kLog2e = 1.4426950408889634f;
     const float sc2 = p.scale * kLog2e;   // scores in the log2 domain
     const float cap2 = EX ? p.ex.softcap * kLog2e : 0.f, cap_in = EX && p.ex.softcap > 0.f ? 2.0f * sc2 / p.ex.softcap : 0.f;
-    // bias of a distance less that of the farthest, log2 domain, for the item's heads; zeros around, so that a tile that holds some near
-    // key indexes it without clamping each distance
+    // bias in the log2 domain; a finite sentinel stays finite there (a row that sees nothing but sentinels averages, as exp would have it)
+    auto bias2 = [&](float b) {
+      const float v = b * kLog2e;
+      return isinf(v) && !isinf(b) ? copysignf(3.402823466e38f, b) : v;
+    };
+    // the item's heads' biases by distance; in front zeros (masked keys), behind the farthest distance's, so that a tile that holds some
+    // near key indexes it without clamping each distance
     const int bias_row = p.ex.bias_dist + 2 * kArBiasPad + 8;
     const bool tab = EX && p.ex.dist_bias != nullptr && G * bias_row <= kArBiasFloats;
     auto fill_bias = [&](int kvh) {
       asm volatile("bar.sync 2, 256;" ::: "memory");
       for (int e = threadIdx.x; e < G * bias_row; e += 256) {
         const int gg = e / bias_row, d = e % bias_row - kArBiasPad;
-        const float* b = p.ex.dist_bias + (int64_t)(kvh * G + gg) * p.ex.bias_dist;
-        bias_tab[e] = d >= 0 && d < p.ex.bias_dist ? (__ldg(b + d) - __ldg(b + p.ex.bias_dist - 1)) * kLog2e : 0.f;
+        bias_tab[e] = d >= 0 ? bias2(__ldg(p.ex.dist_bias + (int64_t)(kvh * G + gg) * p.ex.bias_dist + min(d, p.ex.bias_dist - 1))) : 0.f;
       }
       asm volatile("bar.sync 2, 256;" ::: "memory");
     };
@@ -357,7 +362,7 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
       const int t = w.row0 + row, ctx = alive ? __ldg(p.ctx_lens + t) : 0, lo = p.window > 0 ? max(ctx - p.window, 0) : 0;
       const int h = w.kvh * G + g, keep = EX ? p.ex.keep_first : 0;
       const float* brow = EX && p.ex.dist_bias && alive ? p.ex.dist_bias + (int64_t)h * p.ex.bias_dist : nullptr;
-      const float far_bias = EX && brow ? __ldg(brow + p.ex.bias_dist - 1) * kLog2e : 0.f;
+      const float far_bias = EX && brow ? bias2(__ldg(brow + p.ex.bias_dist - 1)) : 0.f;
       float mu = -INFINITY, l = 0.f;
       for (int i = w.lo; i < w.hi; ++i, ++n) {
         const int k0 = ar_tile(w, i) * kArKeys, j_lo = lo - k0, j_hi = ctx - k0;   // live columns [j_lo, j_hi), and those below keep
@@ -369,9 +374,12 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         ld32(s_addr + 32, s + 32);
         ld_wait<64>(s);
         if constexpr (EX) {   // scaled, capped, biased, in the log2 domain
+          // a tile of far keys alone takes the last distance's bias with the scaling, one that holds nearer keys each key's own after it
+          const bool near = __any_sync(0xffffffffu, brow != nullptr && ctx - 1 - (k0 + kArKeys - 1) < p.ex.bias_dist - 1);
+          const float add = near ? 0.f : far_bias;
           if (p.ex.softcap > 0.f) {
             // cap tanh(v / cap) = cap - 2 cap / (1 + e^(2 v / cap)) on the hardware's exponential and reciprocal
-            const float top = cap2 + far_bias;
+            const float top = cap2 + add;
 #pragma unroll
             for (int j = 0; j < 64; ++j) {
               float rc;
@@ -380,20 +388,20 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
             }
           } else {
 #pragma unroll
-            for (int j = 0; j < 64; ++j) s[j] = __float_as_uint(fmaf(__uint_as_float(s[j]), sc2, far_bias));
+            for (int j = 0; j < 64; ++j) s[j] = __float_as_uint(fmaf(__uint_as_float(s[j]), sc2, add));
           }
-          // the bias of the last distance is in; nearer keys take their own
-          if (__any_sync(0xffffffffu, brow != nullptr && ctx - 1 - (k0 + kArKeys - 1) < p.ex.bias_dist - 1) && brow) {
+          if (near && brow) {
             const int d0 = ctx - 1 - k0;
             if (tab) {
               // below -1 every key is masked, from the last distance + 64 on every key is far: the padding covers what lies between
               const float* b = bias_tab + g * bias_row + kArBiasPad + min(max(d0, -1), p.ex.bias_dist + 95);
 #pragma unroll
               for (int j = 0; j < 64; ++j) s[j] = __float_as_uint(__uint_as_float(s[j]) + b[-j]);
-            } else
+            } else {
 #pragma unroll
-            for (int j = 0; j < 64; ++j)
-              s[j] = __float_as_uint(__uint_as_float(s[j]) + fmaf(__ldg(brow + min(max(d0 - j, 0), p.ex.bias_dist - 1)), kLog2e, -far_bias));
+              for (int j = 0; j < 64; ++j)
+                s[j] = __float_as_uint(__uint_as_float(s[j]) + bias2(__ldg(brow + min(max(d0 - j, 0), p.ex.bias_dist - 1))));
+            }
           }
         }
         if (__any_sync(0xffffffffu, (j_lo > 0 && !(EX && k0 + kArKeys <= keep)) || j_hi < kArKeys)) {

@@ -136,3 +136,26 @@ def test_long_steps_of_decode_rows_go_to_the_other_kernel(ns):
         want = torch.einsum("hc,chd->hd", w, v)
         # weights and results rounded to bf16 once each: 2^-9 of the largest value, 2^-9 of the result
         assert ((got[t] - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -9 * v.abs().max()).all(), t
+
+
+# The bias of a distance is that distance's alone: what the table holds for the farthest keys, a mask or a sentinel, leaves near keys as they are.
+@pytest.mark.parametrize("last", [float("-inf"), -1e9, -1e4, "lowest everywhere"])
+@pytest.mark.parametrize("nd", [40, 3000])       # on chip and not
+@pytest.mark.parametrize("cap", [0.0, 20.0])
+def test_masks_and_sentinels_in_the_distance_bias(last, nd, cap):
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    heads, kv, dim, bs = 8, 2, 64, 64
+    g, q, rows, (kc, vc), bt, seq, ctx, T = _case(heads, kv, dim, dim, bs, 17)
+    bias = torch.randn(heads, nd, generator=g)
+    if last == "lowest everywhere":
+        bias[:] = torch.finfo(torch.float32).min      # nothing but sentinels: all keys weigh the same
+    else:
+        bias[:, 39:] = last
+    ws = torch.zeros(int(lib.b200_paged_attn_anydim_workspace_bytes(T)), dtype=torch.uint8, device=DEV)
+    out = torch.full((T, heads, dim), float("nan"), dtype=torch.bfloat16, device=DEV)
+    qd, bd, pos = q.float().to(DEV), bias.to(DEV), (ctx - 1).contiguous()
+    check(lib.b200_paged_attn_biased(0, 2, qd.data_ptr(), kc.data_ptr(), vc.data_ptr(), bt.data_ptr(), bt.shape[1], seq.data_ptr(), ctx.data_ptr(),
+                                     pos.data_ptr(), out.data_ptr(), T, heads, kv, dim, dim, bs, dim ** -0.5, 0, cap, bd.data_ptr(), nd, None, 0,
+                                     ws.data_ptr(), 1, None, None))
+    torch.cuda.synchronize()
+    _close(out, _oracle(q, rows, dim ** -0.5, cap=cap, bias=bias))
