@@ -397,8 +397,9 @@ int latent_attn_mma(const float* q, const __nv_bfloat16* kc, const int32_t* bloc
   const auto at = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr); };
   B200_REQUIRE(at(kc) % 16 == 0, B200_ERR_INVALID, "attention: cache not 16-byte aligned");
   // tcgen05 wherever the shape fits and the rows can be read and written in its wide pieces (what it measured stands there; it is
-  // the faster one from one decode row up); other shapes, blocks that a key tile would straddle and odd addresses stay here
-  if (latent_attn_tc_supported(heads, krow, rank, block_size) && at(q) % 16 == 0 && at(out) % 32 == 0 && ((at(runs) | at(part)) & 7) == 0) {
+  // the faster one from one decode row up); other shapes, blocks that a key tile would straddle and odd addresses stay here, and so do
+  // scales that are not positive (masks and maxima there are taken of the unscaled scores)
+  if (scale > 0.f && latent_attn_tc_supported(heads, krow, rank, block_size) && at(q) % 16 == 0 && at(out) % 32 == 0 && ((at(runs) | at(part)) & 7) == 0) {
     const int rc = latent_attn_tc(q, kc, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, krow, rank, block_size, scale,
                                   sink, s, n_splits, part, window);
     if (rc || n_splits == 1) return rc;
@@ -426,7 +427,8 @@ int paged_attn_mma(const float* q, const __nv_bfloat16* kc, const __nv_bfloat16*
   // item's 256 pairs there (256 rows at contexts 300..600, 16 heads over 4: 184 us against 80; 1 900 rows of three sequences 74
   // against 278).  How the rows fall into runs is known on the device only: short steps stay here altogether, for others both kernels
   // are launched, and the one whose kind of step it is not (runs of four rows on average) leaves at once
-  if (T > 128 && attn_rows_tc_supported(heads, kv_heads, dim, vdim, block_size) && at(q) % 16 == 0 && at(out) % 16 == 0 && at(part) % 8 == 0) {
+  // (scales that are not positive stay here too: masks and maxima of the other kernel are those of the unscaled scores)
+  if (T > 128 && scale > 0.f && attn_rows_tc_supported(heads, kv_heads, dim, vdim, block_size) && at(q) % 16 == 0 && at(out) % 16 == 0 && at(part) % 8 == 0) {
     int rc = attn_rows_tc_runs(q, kc, vc, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, kv_heads, dim, vdim,
                                block_size, scale, sink, s, n_splits, part, window, ex);
     if (rc) return rc;

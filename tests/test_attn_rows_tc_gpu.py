@@ -159,3 +159,24 @@ def test_masks_and_sentinels_in_the_distance_bias(last, nd, cap):
                                      ws.data_ptr(), 1, None, None))
     torch.cuda.synchronize()
     _close(out, _oracle(q, rows, dim ** -0.5, cap=cap, bias=bias))
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.1])
+@pytest.mark.parametrize("cap", [0.0, 20.0])
+def test_scales_that_are_not_positive(scale, cap):
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    heads, kv, dim, bs = 8, 2, 64, 64
+    g, q, rows, (kc, vc), bt, seq, ctx, T = _case(heads, kv, dim, dim, bs, 23)
+    ws = torch.zeros(int(lib.b200_paged_attn_anydim_workspace_bytes(T)), dtype=torch.uint8, device=DEV)
+    out = torch.full((T, heads, dim), float("nan"), dtype=torch.bfloat16, device=DEV)
+    qd, pos = q.float().to(DEV), (ctx - 1).contiguous()
+    lead = [qd.data_ptr(), kc.data_ptr(), vc.data_ptr(), bt.data_ptr(), bt.shape[1], seq.data_ptr(), ctx.data_ptr()]
+    if cap:
+        check(lib.b200_paged_attn_biased(0, 2, *lead, pos.data_ptr(), out.data_ptr(), T, heads, kv, dim, dim, bs, scale, 0, cap, None, 0, None, 0,
+                                         ws.data_ptr(), 1, None, None))
+    else:
+        check(lib.b200_paged_attn_mma(*lead, out.data_ptr(), T, heads, kv, dim, dim, bs, scale, None, ws.data_ptr(), 0, 1, None, None))
+    torch.cuda.synchronize()
+    got, want = out.double().cpu(), _oracle(q, rows, scale, cap=cap)
+    # weights and results rounded to bf16 once each: 2^-9 of the largest value, 2^-9 of the result
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -9 * rows[1].float().abs().max()).all()

@@ -63,3 +63,24 @@ def test_latent_attention_tile_edges(heads, rank, rd, bs, splits, window, with_s
     # averages the weights' part: below 2^-8 in the 2-norm, and no single result further off than the weights' worst case, 2^-8 of the largest value
     assert (got - want).norm() / want.norm() < 2.0 ** -8
     assert (got - want).abs().max() < 2.0 ** -8 * rows.float().abs().max() + 2.0 ** -9 * want.abs().max()
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.02])
+def test_latent_scales_that_are_not_positive(scale):
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    heads, rank, rd, bs = 4, 64, 16, 64
+    g = torch.Generator().manual_seed(9)
+    ctxs = [1, 63, 64, 65, 190] + list(range(20, 60))
+    seq, T, krow = list(range(5)) + [5] * 40, 45, rank + rd
+    rows = torch.randn(192, krow, generator=g).to(torch.bfloat16)
+    q = torch.randn(T, heads, krow, generator=g).to(torch.bfloat16).float()
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)   # noqa: E731
+    bt, sq, cx, kd, qd = i32([[0, 1, 2]] * 6), i32(seq), i32(ctxs), rows.reshape(3, 1, bs, krow).to(DEV), q.to(DEV)
+    ws = torch.zeros(int(lib.b200_paged_attn_anydim_workspace_bytes(T)), dtype=torch.uint8, device=DEV)
+    out = torch.full((T, heads, rank), float("nan"), dtype=torch.bfloat16, device=DEV)
+    check(lib.b200_latent_attn(qd.data_ptr(), kd.data_ptr(), bt.data_ptr(), 3, sq.data_ptr(), cx.data_ptr(), out.data_ptr(), T, heads, krow, rank, bs,
+                               scale, None, ws.data_ptr(), 1, None, None))
+    torch.cuda.synchronize()
+    want = torch.stack([_oracle(q[t].double(), rows.double(), ctxs[t], rank, scale, None, 0) for t in range(T)])
+    # weights and results rounded to bf16 once each: 2^-9 of the largest value, 2^-9 of the result
+    assert ((out.double().cpu() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -9 * rows.float().abs().max()).all()
