@@ -17,7 +17,6 @@
 #include <algorithm>
 
 #include "mlstm_walk.cuh"
-#include <algorithm>
 
 namespace b200 {
 namespace {
@@ -52,6 +51,9 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t& t0, uint32_t&
   t1 = pack_bf16(x1, y1);
   t2 = pack_bf16(x1 - bf16lo(t1), y1 - bf16hi(t1));
 }
+
+// either of two packed bf16 an infinity or NaN
+__device__ __forceinline__ bool odd2(uint32_t x) { return (x & 0x7f800000u) == 0x7f800000u || (x & 0x7f80u) == 0x7f80u; }
 
 struct GateRows {   // of one chunk
   double a[kMcRows];       // F_t - m_t
@@ -154,7 +156,7 @@ __global__ void __launch_bounds__(kMcThreads, CTAS) mlstm_chunk_kernel(const Mls
     double F[2], G[2], M[2];
 #pragma unroll
     for (int x = 0; x < 2; ++x) {   // inclusive sums (a gate below -1e5 leaves nothing in fp32 either way)
-      F[x] = fmaxf(fg[x], -1e5f);
+      F[x] = fg[x] < -1e5f ? -1e5f : fg[x];   // (NaN stays)
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
         const double v = __shfl_up_sync(0xffffffffu, F[x], d);
@@ -241,8 +243,8 @@ __global__ void __launch_bounds__(kMcThreads, CTAS) mlstm_chunk_kernel(const Mls
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int t = rg + g + (i >> 1) * 8, j = sb + n * 8 + 2 * t4 + (i & 1);
-          const float e = j <= t ? expf((float)(((i >> 1) ? a_hi : a_lo) + gt.g[j])) : 0.f;
-          p[n][i] = p[n][i] * a.qscale * e;
+          // (selected, not weighted with 0: a later row's key may be anything)
+          p[n][i] = j <= t ? p[n][i] * a.qscale * expf((float)(((i >> 1) ? a_hi : a_lo) + gt.g[j])) : 0.f;
         }
       uint32_t pa[3][4];
       split3(p[0][0], p[0][1], pa[0][0], pa[1][0], pa[2][0]);
@@ -252,11 +254,34 @@ __global__ void __launch_bounds__(kMcThreads, CTAS) mlstm_chunk_kernel(const Mls
       uint32_t v4[4], v2[2];
       ldsm4t(v4, &sm.v[buf][sb + (lane & 15)][(lane >> 4) * 8]);
       ldsm2t(v2, &sm.v[buf][sb + (lane & 15)][kMcCols]);
+      if (sb == rg && __any_sync(0xffffffffu, odd2(v4[0]) || odd2(v4[1]) || odd2(v4[2]) || odd2(v4[3]))) {
+        // a value that is not finite on the diagonal's block: its products with the zeros above the diagonal would reach earlier rows, so each
+        // row adds its own keys one by one
+#pragma unroll 1
+        for (int j = 0; j < 16; ++j) {
+          const int from = (lane & ~3) | ((j & 7) >> 1);
+          float w[2];
 #pragma unroll
-      for (int x = 2; x >= 0; --x) {
-        mma(O[0], pa[x], v4[0], v4[1]);
-        mma(O[1], pa[x], v4[2], v4[3]);
-        mma(O[2], pa[x], v2[0], v2[1]);
+          for (int x = 0; x < 2; ++x)
+            w[x] = __shfl_sync(0xffffffffu, j < 8 ? (j & 1 ? p[0][2 * x + 1] : p[0][2 * x]) : (j & 1 ? p[1][2 * x + 1] : p[1][2 * x]), from);
+#pragma unroll
+          for (int n = 0; n < 3; ++n) {
+            const uint32_t v = *reinterpret_cast<const uint32_t*>(&sm.v[buf][sb + j][n * 8 + 2 * t4]);
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+              if (j <= g + 8 * x) {
+                O[n][2 * x] = fmaf(w[x], bf16lo(v), O[n][2 * x]);
+                O[n][2 * x + 1] = fmaf(w[x], bf16hi(v), O[n][2 * x + 1]);
+              }
+          }
+        }
+      } else {
+#pragma unroll
+        for (int x = 2; x >= 0; --x) {
+          mma(O[0], pa[x], v4[0], v4[1]);
+          mma(O[1], pa[x], v4[2], v4[3]);
+          mma(O[2], pa[x], v2[0], v2[1]);
+        }
       }
     }
 #pragma unroll

@@ -90,6 +90,50 @@ def test_mlstm_scan_portions_and_hard_gates(f32, heads, dim, vdim, pad):
     assert (state[[1, 3]] == 7.5).all()
 
 
+@pytest.mark.parametrize("what", ["value", "key", "forget gate", "input gate"])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("row", [0, 37, 100])
+def test_mlstm_chunks_are_causal_for_what_is_not_finite(what, bad, row):
+    """An infinity or NaN of one row reaches that row and the later ones (a value's its own column, anything else's its head), and no earlier row."""
+    if "gate" in what and bad == float("inf"):
+        bad = float("nan")
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    heads, dim, vdim, T, col = 2, 64, 64, 130, 21
+    g = torch.Generator().manual_seed(5)
+    hd, hv = heads * dim, heads * vdim
+    floats, ld = int(lib.b200_mlstm_state_floats(heads, dim, vdim)), 2 * hd + hv
+    x = torch.randn(T, ld, generator=g).to(torch.bfloat16)
+    gates = torch.randn(T, 2 * heads, generator=g)
+    gates[:, heads:] = torch.nn.functional.logsigmoid(gates[:, heads:] + 3)
+    zero = tuple(torch.zeros(s, dtype=torch.float64) for s in ((heads, vdim, dim), (heads, dim), (heads,)))
+    want, span, (S, _, _) = _mlstm(x.double(), gates.double(), zero, heads, dim, vdim)
+    hit = torch.zeros(T, heads, vdim, dtype=torch.bool)      # everything in head 1
+    if what == "value":
+        x[row, 2 * hd + vdim + col] = bad
+        hit[row:, 1, col] = True
+    else:
+        hit[row:, 1] = True
+        if what == "key":
+            x[row, hd + dim + 9] = bad
+        else:
+            gates[row, (heads if what == "forget gate" else 0) + 1] = bad
+    state, out = torch.zeros(1, floats, device=DEV), torch.full((T, hv), float("nan"), device=DEV)
+    xd, gd, ptd, std, sld = x.to(DEV), gates.to(DEV), _i32(list(range(T))), _i32([0, T]), _i32([0])
+    check(lib.b200_mlstm_scan(0, xd.data_ptr(), ld, 0, hd, 2 * hd, gd.data_ptr(), ptd.data_ptr(), std.data_ptr(), sld.data_ptr(), state.data_ptr(), floats,
+                              out.data_ptr(), 1, heads, dim, vdim, None))
+    torch.cuda.synchronize()
+    got, hit = out.double().cpu(), hit.reshape(T, hv)
+    assert not torch.isfinite(got[hit]).any()
+    near = (got - want).abs() <= 1e-5 * span + 1e-7 * want.abs()   # (as above)
+    assert near[~hit].all()
+    st = state[0, :heads * vdim * dim].double().cpu().reshape(heads, vdim, dim)
+    if what == "value":
+        assert not torch.isfinite(st[1, col]).any() and torch.isfinite(st[1, :col]).all() and torch.isfinite(st[1, col + 1:]).all()
+    else:
+        assert not torch.isfinite(st[1, :, 9]).any()
+    assert (st[0] - S[0]).norm() < 1e-5 * S[0].norm()
+
+
 # channel decays / one per head, delta rule / plain, heads sharing keys, sizes that leave lanes and columns idle; strided decays (g_chan 2);
 # zero decays forget everything, as do rows of zeros; rows that are not 16-byte aligned
 @pytest.mark.parametrize("rule", ["channel", "head", "plain", "plain channel", "strided"])
