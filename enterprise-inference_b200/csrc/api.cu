@@ -31,7 +31,7 @@ int cuda_fail(cudaError_t e, const char* what, const char* file, int line) {
 }
 
 LaunchOpts& launch_opts() {
-  static thread_local LaunchOpts o;
+  static thread_local LaunchOpts o = {false, !getenv("B200_PDL") || atoi(getenv("B200_PDL")) != 0};
   return o;
 }
 int& launch_counter() {
@@ -367,7 +367,7 @@ extern "C" int b200_allreduce_bf16(b200_ctx* c, void* buf, int64_t count, void* 
 }
 
 extern "C" int b200_set_launch_pdl(int32_t enabled) {
-  launch_opts().pdl = enabled != 0;
+  launch_opts() = {enabled != 0, enabled != 0};
   return B200_OK;
 }
 
@@ -834,7 +834,10 @@ static int pow2_bucket(int v) {
 }
 
 static int run_step(b200_ctx* c, const StepArgs& a, cudaStream_t s) {
-  const bool pdl_prev = launch_opts().pdl;   // the caller's per-thread setting is restored on every exit
+  const struct Restore {   // the caller's per-thread setting, on every exit
+    const LaunchOpts before = launch_opts();
+    ~Restore() { launch_opts() = before; }
+  } restore;
   if (c->stack) {
     const int rc0 = stack_ready(c);
     if (rc0) return rc0;
@@ -856,13 +859,12 @@ static int run_step(b200_ctx* c, const StepArgs& a, cudaStream_t s) {
   if (c->cfg.tp_world > 1) B200_REQUIRE(c->comm, B200_ERR_STATE, "decode_step: b200_nccl_init not called");
 
   const bool use_graph = c->graphs && s != nullptr && c->tap_layer < 0;
-  launch_opts().pdl = getenv("B200_PDL") ? atoi(getenv("B200_PDL")) != 0 : c->pdl;
+  launch_opts().pdl = launch_opts().within = getenv("B200_PDL") ? atoi(getenv("B200_PDL")) != 0 : c->pdl;
   int rc = B200_OK;
   if (!use_graph) {
     launch_counter() = 0;
     rc = c->stack ? stack_enqueue_step(c, a, s) : enqueue_step(c, a, s);
     c->last_launches = launch_counter();
-    launch_opts().pdl = pdl_prev;
     return rc;
   }
   const GraphKey key{{(uint64_t)a.ids,        (uint64_t)a.positions,  (uint64_t)a.slots,
@@ -881,7 +883,6 @@ static int run_step(b200_ctx* c, const StepArgs& a, cudaStream_t s) {
     rc = c->stack ? stack_enqueue_step(c, b, s) : enqueue_step(c, b, s);
     const int n = launch_counter();
     cudaError_t e = cudaStreamEndCapture(s, &g);
-    launch_opts().pdl = pdl_prev;
     if (rc) {
       if (g) cudaGraphDestroy(g);
       return rc;
@@ -898,7 +899,6 @@ static int run_step(b200_ctx* c, const StepArgs& a, cudaStream_t s) {
     it = c->graph_cache.emplace(key, ge).first;
     c->last_launches = n;
   }
-  launch_opts().pdl = pdl_prev;
   B200_CUDA(cudaGraphLaunch(it->second, s));
   return B200_OK;
 }

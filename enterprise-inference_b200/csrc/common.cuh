@@ -149,14 +149,15 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 
 // ---- launch helper -----------------------------------------------------------------------
 struct LaunchOpts {
-  bool pdl = false;  // programmatic stream serialization (set by the ctx inside a step)
+  bool pdl = false;    // programmatic stream serialization (set by the ctx inside a step)
+  bool within = true;  // the same between the kernels of one call; off once either is switched off (b200_set_launch_pdl(0), B200_PDL=0)
 };
 LaunchOpts& launch_opts();
 // For the later launches of an entry point that launches several kernels: their prologues overlap the kernel before, which the same call
 // launched (every kernel waits for its predecessor's memory in pdl_wait).
 struct PdlScope {
   const bool before;
-  PdlScope() : before(launch_opts().pdl) { launch_opts().pdl = true; }
+  PdlScope() : before(launch_opts().pdl) { launch_opts().pdl = before || launch_opts().within; }
   ~PdlScope() { launch_opts().pdl = before; }
 };
 int& launch_counter();

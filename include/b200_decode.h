@@ -161,7 +161,8 @@ B200_API int b200_ctx_set_tap(b200_ctx* ctx, int32_t layer, void* out_hidden, vo
 
 /* Launch attribute for the per-kernel entry points called from THIS thread: 1 = programmatic dependent
  * launch (the kernels of b200_decode_step always use it unless B200_PDL=0): a kernel's prologue and first
- * weight tiles overlap the previous kernel's tail.  Default 0. */
+ * weight tiles overlap the previous kernel's tail; 0 = on no launch.  Before the first call no entry point's first launch
+ * has it, and those that launch several kernels give it to the later ones unless B200_PDL=0. */
 B200_API int b200_set_launch_pdl(int32_t enabled);
 
 /* y[T][n_out] = x[T][k] . w[n_out][k]^T (+bias), fp32 accumulate, one rounding to bf16.
