@@ -858,6 +858,7 @@ static int run_step(b200_ctx* c, const StepArgs& a, cudaStream_t s) {
                "decode_step: max_ctx_len=%d outside (0,%d]", a.max_ctx, c->cfg.max_blocks_per_seq * c->cfg.block_size);
   if (c->cfg.tp_world > 1) B200_REQUIRE(c->comm, B200_ERR_STATE, "decode_step: b200_nccl_init not called");
 
+  if (const int e = wait_status()) return e;
   const bool use_graph = c->graphs && s != nullptr && c->tap_layer < 0;
   launch_opts().pdl = launch_opts().within = getenv("B200_PDL") ? atoi(getenv("B200_PDL")) != 0 : c->pdl;
   int rc = B200_OK;

@@ -20,9 +20,7 @@
 // Warps: TMA producer, MMA issuer, four softmax warps (a thread owns a pair), eight that stage the next item's queries.
 // The running maximum is only followed when it rises by more than 2^8 (the scaling of all terms is the same, so the
 // quotient is exact); a warp then rescales its own 32 rows of O in TMEM.
-// Every wait is bounded (tc.cuh).
-#include <stdlib.h>
-
+// Every wait is bounded and reported (tc.cuh).
 #include <algorithm>
 
 #include "tc.cuh"
@@ -50,6 +48,7 @@ struct LtParams {
   const float* sink;
   __nv_bfloat16* out;
   float* part;
+  uint32_t* status;
   int n_rows, bt_stride, heads, krow, rank, block_size, n_splits, window, own_stages, rest_slots, halves, rows_per_item, items_per_run;
   float scale;
 };
@@ -104,7 +103,9 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
   uint64_t* o_full = p_ready + 2;                // [2]
   uint64_t* q_ready = o_full + 2;
   uint64_t* q_free = q_ready + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(q_free + 1);
+  uint64_t* last = q_free + 1;                   // the MMAs in flight when a wait ran out
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(last + 1);   // and, behind it, the mark of a wait that ran out
+  const Waits mbar_wait(tmem_slot + 1, p.status);
   LtItem* table = reinterpret_cast<LtItem*>(tmem_slot + 2);   // nr 0: nothing there
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.own_stages; ++s) {
@@ -122,6 +123,8 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
     }
     mbar_init(q_ready, 8);
     mbar_init(q_free, 1);
+    mbar_init(last, 1);
+    tmem_slot[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -155,12 +158,13 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
     if (issuer) asm volatile("prefetch.tensormap [%0];" ::"l"(&map) : "memory");
     int st = 0, sl = 0;
     uint32_t st_ph = 1, sl_ph = 1;   // parity of the release that a slot's next load waits for (the first round finds it free)
-    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
+    bool stop = false;
+    for (int it = blockIdx.x; it < n_items && !stop; it += gridDim.x) {
       LtItem w;
       if (!next_item(it, w)) continue;
       const int own = w.half ? own1 : own0, first = w.half * 4, rest = chunks - own;
       const int32_t* bt = p.block_table + (int64_t)w.seq * p.bt_stride;
-      for (int i = w.tile_lo; i < w.tile_hi; ++i) {
+      for (int i = w.tile_lo; i < w.tile_hi && !(stop = mbar_wait.stop()); ++i) {
         const int tok = i * kLtKeys;
         const int blk = __shfl_sync(0xffffffffu, __ldg(bt + tok / p.block_size), 0);
         const int row = blk * p.block_size + tok % p.block_size;
@@ -181,6 +185,10 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
         if (++st == p.own_stages) st = 0, st_ph ^= 1;
       }
     }
+    if (mbar_wait.stop()) {   // the loads in flight: a slot's last one filled it in this round of the ring or in the one before
+      for (int s = 0; s < p.own_stages; ++s) mbar_wait.drain(own_full + s, s < st ? st_ph ^ 1 : st_ph);
+      for (int s = 0; s < p.rest_slots; ++s) mbar_wait.drain(rest_full + s, s < sl ? sl_ph ^ 1 : sl_ph);
+    }
   } else if (warp == 1) {
     // ===== MMA: the scores of tile n + 1 are issued before the weights of tile n are waited for.  The whole warp walks the loop; bounds
     // and addresses that come from memory are broadcast, so that they are uniform to the compiler =====
@@ -191,7 +199,8 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
     int st = 0, sl = 0, pv_st = 0;   // own stage and rest slot of the next scores, own stage of the next second product
     uint32_t st_ph = 0, sl_ph = 0;
     int n = 0, active = 0;
-    for (int it = blockIdx.x; it < items; it += gridDim.x) {
+    bool stop = false;
+    for (int it = blockIdx.x; it < items && !stop; it += gridDim.x) {
       LtItem w;
       const bool have = next_item(it, w);
       const int nt = __shfl_sync(0xffffffffu, have ? w.tile_hi - w.tile_lo : 0, 0);
@@ -238,7 +247,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
       fence_after();
       issue_s(n);
       if (nt == 1) commit(one, q_free);
-      for (int i = 0; i < nt; ++i, ++n) {
+      for (int i = 0; i < nt && !(stop = mbar_wait.stop()); ++i, ++n) {
         if (i + 1 < nt) {
           issue_s(n + 1);
           if (i + 2 == nt) commit(one, q_free);   // the item's last scores are on their way
@@ -257,6 +266,10 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
         if (++pv_st == p.own_stages) pv_st = 0;
       }
       ++active;
+    }
+    if (mbar_wait.stop()) {
+      commit(one, last);
+      mbar_wait.drain(last, 0);
     }
   } else if (warp >= 6) {
     // ===== queries of the next item: fp32 rows -> bf16, the half's own columns to TMEM, the others to shared memory.  Two warps
@@ -502,6 +515,7 @@ int latent_attn_tc(const float* q, const __nv_bfloat16* kc, const int32_t* block
   LtShape sh;
   B200_REQUIRE(latent_attn_tc_supported(heads, krow, rank, block_size) && lt_shape(heads, krow, rank, sh), B200_ERR_UNSUPPORTED,
                "latent_attn_tc: shape %d / %d / %d", heads, krow, rank);
+  if (const int e = wait_status()) return e;
   CUtensorMap map;
   const int rc = get_tensor_map_2d(kc, 1ull << 31, krow, krow, kLtKeys, &map);   // rows touched come from the block table
   if (rc) return rc;
@@ -515,6 +529,7 @@ int latent_attn_tc(const float* q, const __nv_bfloat16* kc, const int32_t* block
   p.sink = sink;
   p.out = out;
   p.part = part;
+  p.status = wait_status_word();
   p.n_rows = T;
   p.bt_stride = bt_stride;
   p.heads = heads;

@@ -16,9 +16,8 @@
 // rescales its 32 rows of O in TMEM.
 // Bound by the tensor core (HILO) or the softmax's issue slots: 2 048 rows at contexts 1001..3048, 32 heads over 8: 118 us (212 us); 1 900
 // rows of three sequences, 16 heads over 4, capped, biased, window 1024: 74 us (278 us on the mma.sync kernel of attn_latent.cu).
-// Warps: four softmax warps per tile (a thread owns a pair), TMA, MMA, two that stage queries.  Every wait is bounded (tc.cuh).
-#include <stdlib.h>
-
+// Warps: four softmax warps per tile (a thread owns a pair), TMA, MMA, two that stage queries.  Every wait is bounded and
+// reported (tc.cuh).
 #include <algorithm>
 
 #include "tc.cuh"
@@ -38,7 +37,7 @@ constexpr int kArBiasFloats = kArTile / 4, kArBiasPad = 96;   // entries in fron
 constexpr int kArStage = 8 * 2048;             // output staging: 2 KiB per softmax warp
 constexpr int kArTable = 32;                   // items of a CTA whose description is worked out ahead
 constexpr int kArSmem = 232448;
-static_assert(1024 + 4 * kArQChunk + 9 * kArTile + kArStage + 256 + kArTable * 40 <= kArSmem, "shared memory");
+static_assert(1024 + 4 * kArQChunk + 9 * kArTile + kArStage + (2 * 9 + 16) * 8 + 8 + kArTable * 40 <= kArSmem, "shared memory");
 
 struct RowsItem {
   int row0, nrows, seq, ctx_max;   // attn_prefill.cu's plan
@@ -58,6 +57,7 @@ struct RowsParams {
   __nv_bfloat16* out;
   int64_t ldo;
   float* part;
+  uint32_t* status;
   int n_rows, bt_stride, heads, kv_heads, dim, vdim, block_size, n_splits, window, tile_rows;
   float scale;
   AttnExtra ex;
@@ -123,7 +123,9 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
   uint64_t* q_ready = o_full + 4;
   uint64_t* q_first = q_ready + 1;                 // the CTA's first queries, staged by the softmax warps as well
   uint64_t* q_free = q_first + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(q_free + 1);
+  uint64_t* last = q_free + 1;                     // the MMAs in flight when a wait ran out
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(last + 1);   // and, behind it, the mark of a wait that ran out
+  const Waits mbar_wait(tmem_slot + 1, p.status);
   RowsWork* table = reinterpret_cast<RowsWork*>(tmem_slot + 2);
   if (threadIdx.x == 0) {
     for (int s = 0; s < kArSlots; ++s) {
@@ -138,6 +140,8 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     mbar_init(q_ready, 2);
     mbar_init(q_first, 10);
     mbar_init(q_free, 1);
+    mbar_init(last, 1);
+    tmem_slot[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 9) {
@@ -198,12 +202,13 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     const int kc = (p.dim + 63) >> 6, vc = (p.vdim + 63) >> 6;
     int slot = 0;
     uint32_t ph = 1;
-    for (int round = 0; round * grid < n_items; ++round) {
+    bool stop = false;
+    for (int round = 0; round * grid < n_items && !stop; ++round) {
       if (item_of(round) >= n_items) continue;
       RowsWork w;
       work_of(round, w);
       const int32_t* bt = p.block_table + (int64_t)w.seq * p.bt_stride;
-      for (int i = w.lo; i < w.hi; ++i) {
+      for (int i = w.lo; i < w.hi && !(stop = mbar_wait.stop()); ++i) {
         const int tok = ar_tile(w, i) * kArKeys;
         const int blk = __shfl_sync(0xffffffffu, __ldg(bt + tok / p.block_size), 0);
         const int row = (blk * p.kv_heads + w.kvh) * p.block_size + tok % p.block_size;
@@ -221,6 +226,8 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         }
       }
     }
+    if (mbar_wait.stop())   // the loads in flight: a slot's last one filled it in this round of the ring or in the one before
+      for (int s = 0; s < kArSlots; ++s) mbar_wait.drain(kv_full + s, s < slot ? ph ^ 1 : ph);
   } else if (warp == 9) {
     // ===== MMA: per key tile, for either tile of pairs: the next key tile's scores, then this one's second product.  The whole warp
     // walks the loop; bounds and addresses that come from memory are broadcast, so that they are uniform to the compiler =====
@@ -231,7 +238,8 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     const int ksteps = p.dim >> 4, items = __shfl_sync(0xffffffffu, n_items, 0);
     int slot = 0, active = 0, n[2] = {0, 0};   // n: key tiles walked by either tile of pairs so far
     uint32_t ph = 0;
-    for (int round = 0; round * grid < items; ++round) {
+    bool stop = false;
+    for (int round = 0; round * grid < items && !stop; ++round) {
       if (item_of(round) >= items) continue;
       RowsWork w;
       work_of(round, w);
@@ -263,7 +271,7 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
       if (tiles == 2) scores(1, n[1], k_slot);
       commit(one, kv_free + k_slot);
       if (nt == 1) commit(one, q_free);
-      for (int i = 0; i < nt; ++i) {
+      for (int i = 0; i < nt && !(stop = mbar_wait.stop()); ++i) {
         const int v_slot = slot;
         const uint32_t v_ph = ph;
         next_slot();
@@ -300,6 +308,10 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         }
       }
       ++active;
+    }
+    if (mbar_wait.stop()) {
+      commit(one, last);
+      mbar_wait.drain(last, 0);
     }
   } else if (warp >= 10) {
     // ===== queries of the next item -> the two A operands =====
@@ -547,6 +559,7 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
 
 template <typename QT, bool HILO, bool EX>
 int ar_launch(const CUtensorMap& mk, const CUtensorMap& mv, const RowsParams& p, int T, cudaStream_t s) {
+  if (const int e = wait_status()) return e;
   static bool done[64] = {};
   B200_CUDA(ensure_dynamic_smem(attn_rows_tc_kernel<QT, HILO, EX>, kArSmem, done));
   const int64_t most = (int64_t)T * p.kv_heads * p.n_splits;   // upper bound; the kernel reads the real count
@@ -591,6 +604,7 @@ int attn_rows_tc_plan(const __nv_bfloat16* q, int64_t ldq, const __nv_bfloat16* 
   p.dim = p.vdim = dim;
   p.block_size = block_size;
   p.n_splits = 1;
+  p.status = wait_status_word();
   p.tile_rows = 128 / (heads / kv_heads);
   p.scale = scale;
   return ar_launch<__nv_bfloat16, true, false>(mk, mv, p, T, s);
@@ -622,6 +636,7 @@ int attn_rows_tc_runs(const float* q, const __nv_bfloat16* kc, const __nv_bfloat
   p.out = out;
   p.ldo = (int64_t)heads * vdim;
   p.part = part;
+  p.status = wait_status_word();
   p.bt_stride = bt_stride;
   p.heads = heads;
   p.kv_heads = kv_heads;

@@ -161,6 +161,9 @@ struct PdlScope {
   ~PdlScope() { launch_opts().pdl = before; }
 };
 int& launch_counter();
+// waits of the tcgen05 attention kernels that ran out (waits.cu): the word they set, and the error of the call that finds it set, which clears it
+uint32_t* wait_status_word();
+int wait_status();
 
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,

@@ -1,4 +1,4 @@
-"""Which launches carry the programmatic attribute, read from the edges of a captured call."""
+"""Launches: which carry the programmatic attribute, read from the edges of a captured call; what a wait that ran out leaves behind."""
 import threading
 
 import pytest
@@ -56,3 +56,19 @@ def test_the_launch_switch_reaches_the_kernels_of_one_call(monkeypatch):
     assert _programmatic_edges(0) == (0, 1)
     monkeypatch.setenv("B200_PDL", "0")
     assert _programmatic_edges(None) == (0, 1)
+
+
+def test_a_wait_that_runs_out_is_reported_once_by_the_next_call():
+    """A small kernel waits for a millisecond at a barrier that nothing arrives at and ends: the context stays usable, the next call says so."""
+    lib = pkg("_abi").lib()
+    keep, call = _latent_call()
+    call(None)
+    torch.cuda.synchronize()
+    want = keep[5].clone()
+    assert lib.b200_debug_expired_wait(None) == 0
+    torch.cuda.synchronize()
+    with pytest.raises(Exception, match="ran out"):
+        call(None)
+    call(None)
+    torch.cuda.synchronize()
+    assert torch.equal(keep[5], want)
