@@ -52,7 +52,9 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // NG: 16-column output groups per warp (rank <= 128 NG).  EX: score cap, distance bias, per-head gate and kept first keys of AttnExtra.
-template <int NG, bool EX>
+// MANY: launched beside attn_rows_tc.cu with fewer CTAs than items, each of which takes several; otherwise one item a CTA (with the loops in
+// every launch 128 decode rows took 65.8 us, without 63.5).
+template <int NG, bool EX, bool MANY>
 __global__ void __launch_bounds__(kLaThreads)
 latent_attn_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __restrict__ kc, const __nv_bfloat16* __restrict__ vc,
                        int kv_heads, const int32_t* __restrict__ block_table,
@@ -66,7 +68,7 @@ latent_attn_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __restr
   // G query heads share kv head g; a pair i of the group is (row t0 + i / G, head g G + i % G).  Latent rows: one kv head, G = heads.
   const int G = heads / kv_heads;
   const int chunks = gridDim.y / kv_heads, g = blockIdx.y / chunks, n_items = *n_runs;   // CTAs that share a run's chunks of pairs
-  if (short_runs > 0 && short_runs >= 4 * n_items) return;   // rows of the step: mostly longer runs, attn_rows_tc.cu's
+  if (MANY && short_runs >= 4 * n_items) return;   // rows of the step: mostly longer runs, attn_rows_tc.cu's
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
   const int t0 = runs[2 * item], nr = runs[2 * item + 1];
   const int nq = nr * G;
@@ -247,6 +249,7 @@ latent_attn_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __restr
         }
       }
     }
+    if constexpr (!MANY) return;
     __syncthreads();   // shared memory is the next item's
     continue;
   }
@@ -279,6 +282,7 @@ latent_attn_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __restr
       }
     }
   }
+  if constexpr (!MANY) return;
   __syncthreads();   // shared memory is the next item's
   }
   }
@@ -363,21 +367,22 @@ static int attn_mma_launch(const float* q, const __nv_bfloat16* kc, const __nv_b
   // a run has at most 16 rows, so a kv head's group has at most 16 G pairs: G chunks of 16
   // (beside attn_rows_tc.cu: fewer CTAs, one for all chunks of a run and kv head, so that leaving a step of longer runs alone costs little)
   const dim3 grid(short_runs ? std::min(T, 256) : T, short_runs ? kv_heads : heads, n_splits), block(kLaThreads);
-#define LA2(NGV, EXV)                                                                                                               \
+#define LA2(NGV, EXV, MV)                                                                                                             \
   do {                                                                                                                              \
     static bool done[64] = {};                                                                                                      \
-    if (smem > 48 * 1024) B200_CUDA(ensure_dynamic_smem(latent_attn_mma_kernel<NGV, EXV>, 200 * 1024, done));                       \
-    B200_CUDA(launch(latent_attn_mma_kernel<NGV, EXV>, grid, block, smem, s, q, kc, vc, kv_heads, block_table, bt_stride, row_to_seq, \
+    if (smem > 48 * 1024) B200_CUDA(ensure_dynamic_smem(latent_attn_mma_kernel<NGV, EXV, MV>, 200 * 1024, done));                       \
+    B200_CUDA(launch(latent_attn_mma_kernel<NGV, EXV, MV>, grid, block, smem, s, q, kc, vc, kv_heads, block_table, bt_stride, row_to_seq, \
                      ctx_lens, out, runs, n_runs, heads, krow, rank, block_size, scale, sink, n_splits, part, window, ex, short_runs ? T : 0)); \
   } while (0)
-#define LA(NGV)                 \
-  do {                          \
-    if (ex.any()) LA2(NGV, true); \
-    else LA2(NGV, false);       \
+#define LA(NGV, MV)                 \
+  do {                              \
+    if (ex.any()) LA2(NGV, true, MV); \
+    else LA2(NGV, false, MV);       \
   } while (0)
-  if (rank <= 128) LA(1);
-  else if (rank <= 256) LA(2);
-  else LA(4);
+  if (short_runs) LA(1, true);   // (rank <= 128: attn_rows_tc.cu's shapes)
+  else if (rank <= 128) LA(1, false);
+  else if (rank <= 256) LA(2, false);
+  else LA(4, false);
 #undef LA
 #undef LA2
   if (n_splits > 1 && !short_runs)
