@@ -199,8 +199,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
     int st = 0, sl = 0, pv_st = 0;   // own stage and rest slot of the next scores, own stage of the next second product
     uint32_t st_ph = 0, sl_ph = 0;
     int n = 0, active = 0;
-    bool stop = false;
-    for (int it = blockIdx.x; it < items && !stop; it += gridDim.x) {
+    for (int it = blockIdx.x; it < items; it += gridDim.x) {
       LtItem w;
       const bool have = next_item(it, w);
       const int nt = __shfl_sync(0xffffffffu, have ? w.tile_hi - w.tile_lo : 0, 0);
@@ -247,7 +246,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
       fence_after();
       issue_s(n);
       if (nt == 1) commit(one, q_free);
-      for (int i = 0; i < nt && !(stop = mbar_wait.stop()); ++i, ++n) {
+      for (int i = 0; i < nt; ++i, ++n) {
         if (i + 1 < nt) {
           issue_s(n + 1);
           if (i + 2 == nt) commit(one, q_free);   // the item's last scores are on their way

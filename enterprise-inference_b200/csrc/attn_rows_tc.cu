@@ -238,8 +238,7 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     const int ksteps = p.dim >> 4, items = __shfl_sync(0xffffffffu, n_items, 0);
     int slot = 0, active = 0, n[2] = {0, 0};   // n: key tiles walked by either tile of pairs so far
     uint32_t ph = 0;
-    bool stop = false;
-    for (int round = 0; round * grid < items && !stop; ++round) {
+    for (int round = 0; round * grid < items; ++round) {
       if (item_of(round) >= items) continue;
       RowsWork w;
       work_of(round, w);
@@ -271,7 +270,7 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
       if (tiles == 2) scores(1, n[1], k_slot);
       commit(one, kv_free + k_slot);
       if (nt == 1) commit(one, q_free);
-      for (int i = 0; i < nt && !(stop = mbar_wait.stop()); ++i) {
+      for (int i = 0; i < nt; ++i) {
         const int v_slot = slot;
         const uint32_t v_ph = ph;
         next_slot();

@@ -52,9 +52,6 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t& t0, uint32_t&
   t2 = pack_bf16(x1 - bf16lo(t1), y1 - bf16hi(t1));
 }
 
-// either of two packed bf16 an infinity or NaN
-__device__ __forceinline__ bool odd2(uint32_t x) { return (x & 0x7f800000u) == 0x7f800000u || (x & 0x7f80u) == 0x7f80u; }
-
 struct GateRows {   // of one chunk
   double a[kMcRows];       // F_t - m_t
   double g[kMcRows];       // i_t - F_t
@@ -254,36 +251,18 @@ __global__ void __launch_bounds__(kMcThreads, CTAS) mlstm_chunk_kernel(const Mls
       uint32_t v4[4], v2[2];
       ldsm4t(v4, &sm.v[buf][sb + (lane & 15)][(lane >> 4) * 8]);
       ldsm2t(v2, &sm.v[buf][sb + (lane & 15)][kMcCols]);
-      if (sb == rg && __any_sync(0xffffffffu, odd2(v4[0]) || odd2(v4[1]) || odd2(v4[2]) || odd2(v4[3]))) {
-        // a value that is not finite on the diagonal's block: its products with the zeros above the diagonal would reach earlier rows, so each
-        // row adds its own keys one by one
-#pragma unroll 1
-        for (int j = 0; j < 16; ++j) {
-          const int from = (lane & ~3) | ((j & 7) >> 1);
-          float w[2];
 #pragma unroll
-          for (int x = 0; x < 2; ++x)
-            w[x] = __shfl_sync(0xffffffffu, j < 8 ? (j & 1 ? p[0][2 * x + 1] : p[0][2 * x]) : (j & 1 ? p[1][2 * x + 1] : p[1][2 * x]), from);
-#pragma unroll
-          for (int n = 0; n < 3; ++n) {
-            const uint32_t v = *reinterpret_cast<const uint32_t*>(&sm.v[buf][sb + j][n * 8 + 2 * t4]);
-#pragma unroll
-            for (int x = 0; x < 2; ++x)
-              if (j <= g + 8 * x) {
-                O[n][2 * x] = fmaf(w[x], bf16lo(v), O[n][2 * x]);
-                O[n][2 * x + 1] = fmaf(w[x], bf16hi(v), O[n][2 * x + 1]);
-              }
-          }
-        }
-      } else {
-#pragma unroll
-        for (int x = 2; x >= 0; --x) {
-          mma(O[0], pa[x], v4[0], v4[1]);
-          mma(O[1], pa[x], v4[2], v4[3]);
-          mma(O[2], pa[x], v2[0], v2[1]);
-        }
+      for (int x = 2; x >= 0; --x) {
+        mma(O[0], pa[x], v4[0], v4[1]);
+        mma(O[1], pa[x], v4[2], v4[3]);
+        mma(O[2], pa[x], v2[0], v2[1]);
       }
     }
+    float odd = 0.f;   // NaN if any sum is not finite
+#pragma unroll
+    for (int n = 0; n < 3; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) odd = fmaf(O[n][i], 0.f, odd);
 #pragma unroll
     for (int kk = 0; kk < KS / 2; ++kk) {
       uint32_t qk[4];
@@ -298,6 +277,45 @@ __global__ void __launch_bounds__(kMcThreads, CTAS) mlstm_chunk_kernel(const Mls
         mma(I[x][0], qk, b4[0], b4[1]);
         mma(I[x][1], qk, b4[2], b4[3]);
         mma(I[x][2], qk, b2[0], b2[1]);
+      }
+    }
+    if (__any_sync(0xffffffffu, odd != 0.f)) {
+      // A value that is not finite in the block on the diagonal: its products with the zeros above the diagonal reached earlier rows.  Once more,
+      // every row adding its own keys one by one.
+#pragma unroll
+      for (int n = 0; n < 3; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) O[n][i] = 0.f;
+#pragma unroll 1
+      for (int sb = hf * 16; sb <= rg; sb += 32) {
+        float p[2][4] = {};
+#pragma unroll 1
+        for (int k = 0; k < KS; ++k) {
+          uint32_t qk[4], b[4];
+          ldsm4(qk, &sm.q[buf][rg + (lane & 15)][k * 16 + (lane >> 4) * 8]);
+          ldsm4(b, &sm.k[buf][sb + (lane & 7) + ((lane >> 4) << 3)][k * 16 + ((lane >> 3) & 1) * 8]);
+          mma(p[0], qk, b[0], b[1]);
+          mma(p[1], qk, b[2], b[3]);
+        }
+#pragma unroll 1
+        for (int j = 0; j < 16; ++j) {
+          const int from = (lane & ~3) | ((j & 7) >> 1);
+          const uint32_t v[3] = {*reinterpret_cast<const uint32_t*>(&sm.v[buf][sb + j][2 * t4]), *reinterpret_cast<const uint32_t*>(&sm.v[buf][sb + j][8 + 2 * t4]),
+                                 *reinterpret_cast<const uint32_t*>(&sm.v[buf][sb + j][16 + 2 * t4])};
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const int t = rg + g + 8 * x;
+            const float w = __shfl_sync(0xffffffffu, j < 8 ? (j & 1 ? p[0][2 * x + 1] : p[0][2 * x]) : (j & 1 ? p[1][2 * x + 1] : p[1][2 * x]), from) * a.qscale *
+                            expf((float)(gt.a[t] + gt.g[sb + j]));
+            if (sb + j <= t) {
+#pragma unroll
+              for (int n = 0; n < 3; ++n) {
+                O[n][2 * x] = fmaf(w, bf16lo(v[n]), O[n][2 * x]);
+                O[n][2 * x + 1] = fmaf(w, bf16hi(v[n]), O[n][2 * x + 1]);
+              }
+            }
+          }
+        }
       }
     }
     const float al[2] = {gt.alpha[rg + g] * a.qscale, gt.alpha[rg + g + 8] * a.qscale};

@@ -35,8 +35,8 @@ __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
 }
 // Waits are bounded.  One that a defect keeps from completing runs out after kWaitNs (a stretch that the GPU spent elsewhere counts
 // for 20 ms at most): it marks the CTA, whose other waits then return as soon as they would have to wait, and sets a word in host memory
-// that the next call reports as an error (waits.cu).  TMA and MMA warps stop at the mark and let what is in flight
-// finish (bounded again) before shared and tensor memory are given up; the other roles' loops are finite.
+// that the next call reports as an error (waits.cu).  The TMA warp stops at the mark, the other roles
+// run through their finite loops; what is in flight then finishes (bounded again) before shared and tensor memory are given up.
 constexpr uint64_t kWaitNs = 2000000000ull;
 __device__ __forceinline__ uint64_t timer_ns() {
   uint64_t t;

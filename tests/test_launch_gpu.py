@@ -22,8 +22,8 @@ def _latent_call():
                                                       80, 64, 64, 0.1, None, ws.data_ptr(), 1, None, s))
 
 
-def _programmatic_edges(switch):
-    """Edges of that call captured in a thread of its own (the switch is the thread's): (programmatic, all)."""
+def _overlaps(switch):
+    """That call captured in a thread of its own (the switch is the thread's): is the edge between its kernels a programmatic one?"""
     from cuda.bindings import runtime as rt
     keep, call = _latent_call()
     call(None)
@@ -37,9 +37,8 @@ def _programmatic_edges(switch):
         ok(rt.cudaStreamBeginCapture(stream.cuda_stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal))
         call(stream.cuda_stream)
         g, = ok(rt.cudaStreamEndCapture(stream.cuda_stream))
-        n = ok(rt.cudaGraphGetEdges_v2(g))[-1]
-        edges = ok(rt.cudaGraphGetEdges_v2(g, n))[2]
-        found.append((sum(int(e.type) == 1 for e in edges[:n]), n))
+        err = rt.cudaGraphGetEdges(g, 4)[0]      # (the query without edge data refuses edges that are not plain)
+        found.append({rt.cudaError_t.cudaSuccess: False, rt.cudaError_t.cudaErrorLossyQuery: True}.get(err, err))
         ok(rt.cudaGraphDestroy(g))
 
     t = threading.Thread(target=work)
@@ -51,11 +50,11 @@ def _programmatic_edges(switch):
 
 def test_the_launch_switch_reaches_the_kernels_of_one_call(monkeypatch):
     monkeypatch.delenv("B200_PDL", raising=False)
-    assert _programmatic_edges(None) == (1, 1)     # the attention overlaps its plan
-    assert _programmatic_edges(1) == (1, 1)
-    assert _programmatic_edges(0) == (0, 1)
+    assert _overlaps(None) is True     # the attention overlaps its plan
+    assert _overlaps(1) is True
+    assert _overlaps(0) is False
     monkeypatch.setenv("B200_PDL", "0")
-    assert _programmatic_edges(None) == (0, 1)
+    assert _overlaps(None) is False
 
 
 def test_a_wait_that_runs_out_is_reported_once_by_the_next_call():
