@@ -691,7 +691,10 @@ B200_API int b200_rotate_back_rows(const void* in, int32_t in_row, void* out, co
                                    int32_t n_tokens, int32_t heads, int32_t vdim, int64_t max_pos, void* stream);
 /* Causal paged attention of fp32 queries [T][heads*dim] over caches [block][kv_heads][block_size][dim | vdim]; out
  * [T][heads*vdim].  vrot != NULL: the output of row t is rotated by -positions[t].  shared_tiles 0: one CTA per (row, head);
- * 1: runs of consecutive rows of a sequence share K/V tiles (workspace: b200_paged_attn_anydim_workspace_bytes(T)). */
+ * 1: runs of consecutive rows of a sequence share K/V tiles (workspace: b200_paged_attn_anydim_workspace_bytes(T)).
+ * Ask for the workspace's size with the library that is loaded, in every process, for the largest T of a call: the entry points that take
+ * it (this one, _latent_attn*, _paged_attn_mma, _biased, _kept) have no argument for its size and cannot refuse a smaller one, and the size
+ * is no formula to copy ((2 T + 8) 4 bytes once, (10 T + 8) 4 now). */
 B200_API int64_t b200_paged_attn_anydim_workspace_bytes(int32_t n_tokens);
 B200_API int b200_paged_attn_anydim(int32_t f32, const float* q, const void* k_cache, const void* v_cache, const int32_t* block_table,
                            int32_t bt_stride, const int32_t* row_to_seq, const int32_t* ctx_lens, const int32_t* positions,
