@@ -49,7 +49,7 @@ def _newest_header() -> float:
 
 def build(force: bool = False, verbose: bool = False, trace: bool = False) -> str:
     """trace=True: a second library (lib/libb200decode_trace.so, -DB200_TRACE_BUILD) whose kernels carry
-    %globaltimer stamps for tools/*_trace.py (load it with B200_LIB=...); never the product library."""
+    %globaltimer stamps for phase traces (load it with B200_LIB=...); never the product library."""
     global OBJ, LIB
     flags = list(NVCC_FLAGS)
     if trace:
