@@ -33,43 +33,30 @@ __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Waits are bounded.  One that a defect keeps from completing runs out after kWaitNs (a stretch that the GPU spent elsewhere counts
-// for 20 ms at most): it marks the CTA, whose other waits then return as soon as they would have to wait, and sets a word in host memory
-// that the next call reports as an error (waits.cu).  The TMA warp stops at the mark, the other roles
-// run through their finite loops; what is in flight then finishes (bounded again) before shared and tensor memory are given up.
-constexpr uint64_t kWaitNs = 2000000000ull;
-__device__ __forceinline__ uint64_t timer_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
+// Waits are bounded.  One that a defect keeps from completing runs out after kWaitTries (4 us each: two seconds): it marks the CTA, whose other
+// waits then return as soon as they would have to wait, and sets a word in host memory that the next call reports as an error (waits.cu).  The
+// TMA warp stops at the mark, the other roles run through their finite loops; what is in flight then finishes (bounded again) before shared
+// and tensor memory are given up.  Tries are counted because a clock costs, even one that is only read after 64 of them: 2 048 prefill rows
+// 108 us with either count or no limit at all, 118 with it.
+constexpr int kWaitTries = 1 << 19;
 struct Waits {
   uint32_t* mark;     // shared: a wait of this CTA ran out
   uint32_t* status;   // host memory
-  uint64_t limit;
-  __device__ __forceinline__ Waits(uint32_t* m, uint32_t* st, uint64_t ns = kWaitNs) : mark(m), status(st), limit(ns) {}
+  int limit;
+  __device__ __forceinline__ Waits(uint32_t* m, uint32_t* st, int tries = kWaitTries) : mark(m), status(st), limit(tries) {}
   __device__ __forceinline__ bool marked() const { return *reinterpret_cast<volatile uint32_t*>(mark) != 0; }
   __device__ __forceinline__ bool stop() const { return __any_sync(0xffffffffu, marked()); }   // the whole warp's answer
   __device__ __forceinline__ void operator()(uint64_t* bar, uint32_t parity) const {
-    if (mbar_try(bar, parity)) return;
-    uint64_t t = timer_ns(), waited = 0;
-    while (!mbar_try(bar, parity)) {
-      if (marked()) return;
-      const uint64_t now = timer_ns();
-      waited += now - t < 20000000u ? now - t : 20000000u;
-      t = now;
-      if (waited > limit) {
+    for (int i = 0; !mbar_try(bar, parity); ++i)
+      if ((i & 63) == 63 && (marked() || i > limit)) {
         *reinterpret_cast<volatile uint32_t*>(mark) = 1;
         if (status) *reinterpret_cast<volatile uint32_t*>(status) = 1;
-        __threadfence_system();
         return;
       }
-    }
   }
   // after the mark: for what is still in flight
   __device__ __forceinline__ void drain(uint64_t* bar, uint32_t parity) const {
-    const uint64_t t0 = timer_ns();
-    while (!mbar_try(bar, parity) && timer_ns() - t0 < limit) {}
+    for (int i = 0; !mbar_try(bar, parity) && i < limit; ++i) {}
   }
 };
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {

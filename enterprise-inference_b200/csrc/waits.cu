@@ -25,7 +25,7 @@ int wait_status() {
 namespace {
 
 // a barrier that nothing arrives at: the first wait runs out, the second finds the mark
-__global__ void __launch_bounds__(64) expired_wait_kernel(uint32_t* status, uint64_t limit_ns) {
+__global__ void __launch_bounds__(64) expired_wait_kernel(uint32_t* status, int tries) {
   __shared__ uint64_t bar;
   __shared__ uint32_t mark;
   if (threadIdx.x == 0) {
@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(64) expired_wait_kernel(uint32_t* status, uint
     mark = 0;
   }
   __syncthreads();
-  const tc::Waits wait(&mark, status, limit_ns);
+  const tc::Waits wait(&mark, status, tries);
   wait(&bar, 0);
   wait(&bar, 0);
 }
@@ -41,8 +41,8 @@ __global__ void __launch_bounds__(64) expired_wait_kernel(uint32_t* status, uint
 }  // namespace
 }  // namespace b200
 
-// debug helper (not in the public header): a kernel whose wait runs out after a millisecond
-extern "C" __attribute__((visibility("default"))) int b200_debug_expired_wait(void* stream) {
-  B200_CUDA(b200::launch(b200::expired_wait_kernel, dim3(1), dim3(64), (size_t)0, (cudaStream_t)stream, b200::wait_status_word(), (uint64_t)1000000));
+// debug helper (not in the public header): a kernel whose wait runs out after so many tries
+extern "C" __attribute__((visibility("default"))) int b200_debug_expired_wait(int32_t tries, void* stream) {
+  B200_CUDA(b200::launch(b200::expired_wait_kernel, dim3(1), dim3(64), (size_t)0, (cudaStream_t)stream, b200::wait_status_word(), tries));
   return B200_OK;
 }
