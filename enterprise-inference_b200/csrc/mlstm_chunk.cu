@@ -52,6 +52,9 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t& t0, uint32_t&
   t2 = pack_bf16(x1 - bf16lo(t1), y1 - bf16hi(t1));
 }
 
+// either of two packed bf16 an infinity or NaN
+__device__ __forceinline__ bool odd2(uint32_t x) { return (x & 0x7f800000u) == 0x7f800000u || (x & 0x7f80u) == 0x7f80u; }
+
 struct GateRows {   // of one chunk
   double a[kMcRows];       // F_t - m_t
   double g[kMcRows];       // i_t - F_t
@@ -67,7 +70,65 @@ struct McSmem {
   __nv_bfloat16 q[2][kMcRows][QS], k[2][kMcRows][QS], v[2][kMcRows][kMcW], w[3][kMcRows][kMcW], s[3][KS * 16][kMcW];
   float o[kMcRows][kMcW + 2];   // one warp's sums of a row group, for the other
   GateRows gate[2];
+  int odd[2];   // a value of the chunk is not finite
 };
+
+// One warp's sums of a chunk (three column tiles of its 16 rows) when a value is not finite: every row adds its own keys one by one, so that nothing
+// is multiplied with a later row's value; what comes from the state before is as in the kernel.
+template <int KS>
+__device__ __noinline__ void mc_careful(const McSmem<KS>& sm, int buf, int hf, int rg, int lane, float qscale, float* out) {
+  const GateRows& gt = sm.gate[buf];
+  const int g = lane >> 2, t4 = lane & 3;
+  float O[3][4] = {}, J[3][4] = {};
+#pragma unroll 1
+  for (int sb = hf * 16; sb <= rg; sb += 32) {
+    float p[2][4] = {};
+#pragma unroll 1
+    for (int k = 0; k < KS; ++k) {
+      uint32_t qk[4], b[4];
+      ldsm4(qk, &sm.q[buf][rg + (lane & 15)][k * 16 + (lane >> 4) * 8]);
+      ldsm4(b, &sm.k[buf][sb + (lane & 7) + ((lane >> 4) << 3)][k * 16 + ((lane >> 3) & 1) * 8]);
+      mma(p[0], qk, b[0], b[1]);
+      mma(p[1], qk, b[2], b[3]);
+    }
+#pragma unroll 1
+    for (int j = 0; j < 16; ++j) {
+      const int from = (lane & ~3) | ((j & 7) >> 1);
+      const __nv_bfloat16* v = &sm.v[buf][sb + j][2 * t4];
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        const int t = rg + g + 8 * x;
+        const float w = __shfl_sync(0xffffffffu, j < 8 ? (j & 1 ? p[0][2 * x + 1] : p[0][2 * x]) : (j & 1 ? p[1][2 * x + 1] : p[1][2 * x]), from) * qscale *
+                        expf((float)(gt.a[t] + gt.g[sb + j]));
+        if (sb + j <= t) {
+#pragma unroll
+          for (int n = 0; n < 3; ++n) {
+            O[n][2 * x] = fmaf(w, __bfloat162float(v[n * 8]), O[n][2 * x]);
+            O[n][2 * x + 1] = fmaf(w, __bfloat162float(v[n * 8 + 1]), O[n][2 * x + 1]);
+          }
+        }
+      }
+    }
+  }
+#pragma unroll 1
+  for (int k = hf * (KS / 2); k < (hf + 1) * (KS / 2); ++k) {
+    uint32_t qk[4];
+    ldsm4(qk, &sm.q[buf][rg + (lane & 15)][k * 16 + (lane >> 4) * 8]);
+#pragma unroll
+    for (int x = 2; x >= 0; --x) {
+      uint32_t b4[4], b2[2];
+      ldsm4t(b4, &sm.s[x][k * 16 + (lane & 15)][(lane >> 4) * 8]);
+      ldsm2t(b2, &sm.s[x][k * 16 + (lane & 15)][kMcCols]);
+      mma(J[0], qk, b4[0], b4[1]);
+      mma(J[1], qk, b4[2], b4[3]);
+      mma(J[2], qk, b2[0], b2[1]);
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < 3; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) out[n * 4 + i] = fmaf(gt.alpha[rg + g + 8 * (i >> 1)] * qscale, J[n][i], O[n][i]);
+}
 
 // KS: 16-wide steps over the (zero padded) key dimensions
 // CTAS: CTAs that share an SM (two when there are more than SMs: fewer registers each)
@@ -207,6 +268,17 @@ __global__ void __launch_bounds__(kMcThreads, CTAS) mlstm_chunk_kernel(const Mls
     __syncthreads();   // rows, gates and state of the chunk are there; the chunk before has been finished with
     const GateRows& gt = sm.gate[buf];
     if (warp == kMcGate) {
+      // (beside the other warps' products: inside them the same question cost 4 % of the whole)
+      bool odd = false;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const uint4 v = *reinterpret_cast<const uint4*>(&sm.v[buf][lane + 32 * (x >> 1)][(x & 1) * 8]);
+        odd |= odd2(v.x) || odd2(v.y) || odd2(v.z) || odd2(v.w);
+      }
+      odd = __any_sync(0xffffffffu, odd);
+      if (lane == 0) sm.odd[buf] = odd;
+      __syncwarp();
+      asm volatile("bar.arrive 1, 288;" ::: "memory");
       gate_chunk(sm.gate[buf ^ 1]);
       fetch_gates(c + 2);
       continue;
@@ -258,11 +330,6 @@ __global__ void __launch_bounds__(kMcThreads, CTAS) mlstm_chunk_kernel(const Mls
         mma(O[2], pa[x], v2[0], v2[1]);
       }
     }
-    float odd = 0.f;   // NaN if any sum is not finite
-#pragma unroll
-    for (int n = 0; n < 3; ++n)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) odd = fmaf(O[n][i], 0.f, odd);
 #pragma unroll
     for (int kk = 0; kk < KS / 2; ++kk) {
       uint32_t qk[4];
@@ -279,45 +346,6 @@ __global__ void __launch_bounds__(kMcThreads, CTAS) mlstm_chunk_kernel(const Mls
         mma(I[x][2], qk, b2[0], b2[1]);
       }
     }
-    if (__any_sync(0xffffffffu, odd != 0.f)) {
-      // A value that is not finite in the block on the diagonal: its products with the zeros above the diagonal reached earlier rows.  Once more,
-      // every row adding its own keys one by one.
-#pragma unroll
-      for (int n = 0; n < 3; ++n)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) O[n][i] = 0.f;
-#pragma unroll 1
-      for (int sb = hf * 16; sb <= rg; sb += 32) {
-        float p[2][4] = {};
-#pragma unroll 1
-        for (int k = 0; k < KS; ++k) {
-          uint32_t qk[4], b[4];
-          ldsm4(qk, &sm.q[buf][rg + (lane & 15)][k * 16 + (lane >> 4) * 8]);
-          ldsm4(b, &sm.k[buf][sb + (lane & 7) + ((lane >> 4) << 3)][k * 16 + ((lane >> 3) & 1) * 8]);
-          mma(p[0], qk, b[0], b[1]);
-          mma(p[1], qk, b[2], b[3]);
-        }
-#pragma unroll 1
-        for (int j = 0; j < 16; ++j) {
-          const int from = (lane & ~3) | ((j & 7) >> 1);
-          const uint32_t v[3] = {*reinterpret_cast<const uint32_t*>(&sm.v[buf][sb + j][2 * t4]), *reinterpret_cast<const uint32_t*>(&sm.v[buf][sb + j][8 + 2 * t4]),
-                                 *reinterpret_cast<const uint32_t*>(&sm.v[buf][sb + j][16 + 2 * t4])};
-#pragma unroll
-          for (int x = 0; x < 2; ++x) {
-            const int t = rg + g + 8 * x;
-            const float w = __shfl_sync(0xffffffffu, j < 8 ? (j & 1 ? p[0][2 * x + 1] : p[0][2 * x]) : (j & 1 ? p[1][2 * x + 1] : p[1][2 * x]), from) * a.qscale *
-                            expf((float)(gt.a[t] + gt.g[sb + j]));
-            if (sb + j <= t) {
-#pragma unroll
-              for (int n = 0; n < 3; ++n) {
-                O[n][2 * x] = fmaf(w, bf16lo(v[n]), O[n][2 * x]);
-                O[n][2 * x + 1] = fmaf(w, bf16hi(v[n]), O[n][2 * x + 1]);
-              }
-            }
-          }
-        }
-      }
-    }
     const float al[2] = {gt.alpha[rg + g] * a.qscale, gt.alpha[rg + g + 8] * a.qscale};
 #pragma unroll
     for (int n = 0; n < 3; ++n)
@@ -329,7 +357,8 @@ __global__ void __launch_bounds__(kMcThreads, CTAS) mlstm_chunk_kernel(const Mls
 #pragma unroll
         for (int x = 0; x < 2; ++x) *reinterpret_cast<float2*>(&sm.o[rg + g + 8 * x][n * 8 + 2 * t4]) = make_float2(O[n][2 * x], O[n][2 * x + 1]);
     }
-    asm volatile("bar.sync 1, 256;" ::: "memory");   // w v is complete, and the other warps' sums are there (not the gate warp's business)
+    asm volatile("bar.sync 1, 288;" ::: "memory");   // w v is complete, the other warps' sums and the gate warp's look at the values are there
+    const int odd = sm.odd[buf];
     if (warp < KS) {
       float U[3][3][4] = {};
 #pragma unroll
@@ -351,6 +380,22 @@ __global__ void __launch_bounds__(kMcThreads, CTAS) mlstm_chunk_kernel(const Mls
       for (int n = 0; n < 3; ++n)
 #pragma unroll
         for (int i = 0; i < 4; ++i) S[n][i] = fmaf(gamma, S[n][i], (U[2][n][i] + U[1][n][i]) + U[0][n][i]);
+    }
+    if (odd) {
+      // in the blocks on the diagonal the products of such a value with the zeros above it reached earlier rows: the sums once more, with care
+      float o[12];
+      mc_careful(sm, buf, hf, rg, lane, a.qscale, o);
+#pragma unroll
+      for (int n = 0; n < 3; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) O[n][i] = o[n * 4 + i];
+      if (hf) {
+#pragma unroll
+        for (int n = 0; n < 3; ++n)
+#pragma unroll
+          for (int x = 0; x < 2; ++x) *reinterpret_cast<float2*>(&sm.o[rg + g + 8 * x][n * 8 + 2 * t4]) = make_float2(O[n][2 * x], O[n][2 * x + 1]);
+      }
+      asm volatile("bar.sync 2, 256;" ::: "memory");
     }
     publish();
     if (!hf) {
