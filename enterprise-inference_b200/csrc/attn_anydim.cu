@@ -150,7 +150,6 @@ paged_attn_rows_kernel(const float* __restrict__ q, const CT* __restrict__ kc, c
 // Work item = (run of up to kRunRows rows of one sequence whose context lengths rise by one, kv head).  The item list is
 // built on the device once per step.  Warp w serves query (row r, head hh) pairs round-robin; a tile is 32 keys: lane =
 // key for the scores, lanes stride the value dimensions for the weighted sum.
-constexpr int kRunRows = 16;
 constexpr int kTileKeys = 32;
 constexpr int kTcThreads = 256;
 
@@ -165,7 +164,9 @@ attn_runs_plan_kernel(const int32_t* __restrict__ row_to_seq, const int32_t* __r
   __shared__ int wseg[32];
   __shared__ uint64_t wcnt[32];
   __shared__ int carry_seg, carry_cnt[kRunLists];
+  __shared__ int first[kRunLists][1024];   // steps of one chunk: the runs' first rows, for their lengths
   static_assert(kRunRows == 16 && kRunLists * 12 <= 64, "run lists");
+  constexpr int kOpens = 1 << 30;   // beside a run's first row, until the lengths are there: it opens a segment
   pdl_wait();
   pdl_launch_dependents();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -203,7 +204,10 @@ attn_runs_plan_kernel(const int32_t* __restrict__ row_to_seq, const int32_t* __r
 #pragma unroll
     for (int k = 0; k < kRunLists; ++k) {
       total[k] = carry_cnt[k] + (int)((cnt >> (12 * k)) & 0xfff);
-      if ((mine >> (12 * k)) & 1) runs[(int64_t)2 * T * k + 2 * (total[k] - 1)] = t;
+      if ((mine >> (12 * k)) & 1) {
+        if (T <= 1024) first[k][total[k] - 1] = t | (brk ? kOpens : 0);
+        else runs[(int64_t)2 * T * k + 2 * (total[k] - 1)] = t | (brk ? kOpens : 0);
+      }
     }
     __syncthreads();
     if (tid == 1023) {
@@ -213,14 +217,32 @@ attn_runs_plan_kernel(const int32_t* __restrict__ row_to_seq, const int32_t* __r
     }
     __syncthreads();
   }
-  // lengths: a run ends where the next one starts
+  // lengths: a run ends where the next one starts; it is whole if it and the next one both open a segment
+  const int n0 = carry_cnt[0];
+  for (int i = tid; i < n0; i += 1024) {
+    int at[kRunLists], end[kRunLists];
 #pragma unroll
-  for (int k = 0; k < kRunLists; ++k) {
-    const int n = carry_cnt[k];
-    int32_t* list = runs + (int64_t)2 * T * k;
-    for (int i = tid; i < n; i += 1024) list[2 * i + 1] = (i + 1 < n ? list[2 * (i + 1)] : T) - list[2 * i];
-    if (tid == 0) n_runs[k] = n;
+    for (int k = 0; k < kRunLists; ++k) {
+      const int n = carry_cnt[k];
+      const int32_t* list = runs + (int64_t)2 * T * k;
+      at[k] = i >= n ? 0 : T <= 1024 ? first[k][i] : list[2 * i];
+      end[k] = i + 1 >= n ? T | kOpens : T <= 1024 ? first[k][i + 1] : list[2 * (i + 1)];
+    }
+#pragma unroll
+    for (int k = 0; k < kRunLists; ++k)
+      if (i < carry_cnt[k]) {
+        int32_t* run = runs + (int64_t)2 * T * k + 2 * i;
+        run[1] = ((end[k] & ~kOpens) - (at[k] & ~kOpens)) | (at[k] & end[k] & kOpens ? kRunWhole : 0);
+        if (T <= 1024) run[0] = at[k] & ~kOpens;
+      }
   }
+  if (tid < kRunLists) n_runs[tid] = carry_cnt[tid];
+  if (T <= 1024) return;
+  __syncthreads();
+  for (int i = tid; i < n0; i += 1024)
+#pragma unroll
+    for (int k = 0; k < kRunLists; ++k)
+      if (i < carry_cnt[k]) runs[(int64_t)2 * T * k + 2 * i] &= ~kOpens;
 }
 
 template <typename CT, typename AT>
@@ -237,7 +259,7 @@ paged_attn_runs_kernel(const float* __restrict__ q, const CT* __restrict__ kc, c
   pdl_launch_dependents();
   const int item = blockIdx.x, g = blockIdx.y;
   if (item >= *n_runs) return;
-  const int t0 = runs[2 * item], nr = runs[2 * item + 1];
+  const int t0 = runs[2 * item], nr = runs[2 * item + 1] & kRunLength;
   const int G = heads / kv_heads;          // query heads per kv head
   const int nq = nr * G;                   // queries of this item
   const int kst = dim + 1, vst = vdim;     // K rows padded: lane = key reads stride kst (conflict-free for odd strides)

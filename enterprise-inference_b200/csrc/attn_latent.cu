@@ -22,7 +22,7 @@
 
 #include <algorithm>
 
-#include "common.cuh"
+#include "runs.cuh"
 
 namespace b200 {
 namespace {
@@ -52,27 +52,36 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // NG: 16-column output groups per warp (rank <= 128 NG).  EX: score cap, distance bias, per-head gate and kept first keys of AttnExtra.
-// MANY: launched beside attn_rows_tc.cu with fewer CTAs than items, each of which takes several; otherwise one item a CTA (with the loops in
-// every launch 128 decode rows took 65.8 us, without 63.5).
+// MANY: launched beside a tcgen05 kernel for its share of the runs, as many CTAs as fit the device, each of which walks over items; otherwise one
+// item a CTA (with the loops in every launch 128 decode rows took 65.2 us, without 64.3).
 template <int NG, bool EX, bool MANY>
-__global__ void __launch_bounds__(kLaThreads)
+__global__ void __launch_bounds__(kLaThreads, NG == 1 ? 4 : NG == 2 ? 3 : 2)
 latent_attn_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __restrict__ kc, const __nv_bfloat16* __restrict__ vc,
                        int kv_heads, const int32_t* __restrict__ block_table,
                        int bt_stride, const int32_t* __restrict__ row_to_seq, const int32_t* __restrict__ ctx_lens,
                        __nv_bfloat16* __restrict__ out, const int32_t* __restrict__ runs, const int32_t* __restrict__ n_runs, int heads,
                        int krow, int rank, int block_size, float scale, const float* __restrict__ sink, int n_splits,
-                       float* __restrict__ part, int window, AttnExtra ex, int short_runs) {
+                       float* __restrict__ part, int window, AttnExtra ex, RunShare share) {
   extern __shared__ __align__(16) unsigned char smraw[];
   pdl_wait();
   pdl_launch_dependents();
   // G query heads share kv head g; a pair i of the group is (row t0 + i / G, head g G + i % G).  Latent rows: one kv head, G = heads.
   const int G = heads / kv_heads;
-  const int chunks = gridDim.y / kv_heads, g = blockIdx.y / chunks, n_items = *n_runs;   // CTAs that share a run's chunks of pairs
-  if (MANY && short_runs >= 4 * n_items) return;   // rows of the step: mostly longer runs, attn_rows_tc.cu's
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-  const int t0 = runs[2 * item], nr = runs[2 * item + 1];
-  const int nq = nr * G;
-  for (int i0 = blockIdx.y % chunks * kLaPairs; i0 < nq; i0 += chunks * kLaPairs) {
+  const int n_items = *n_runs, short_pairs = MANY ? run_share(share, G) : 0;
+  if (MANY && short_pairs == 0) return;
+  // the CTAs that share a run's chunks of pairs: as many as the device has places for (all G of them where it does not matter)
+  const int lanes = n_items * kv_heads * n_splits, chunks = MANY ? min(G, max(1, 8 * kNumSMs / max(lanes, 1))) : G;
+  const int total = MANY ? lanes * chunks : 1;
+  for (int v = MANY ? blockIdx.x : 0; v < total;) {
+  int ticket = 0;   // the next item is asked for before this one is worked on
+  if (MANY && threadIdx.x == 0) ticket = gridDim.x + atomicAdd(share.ticket, 1);
+  // a run's first chunks of pairs lead, so that chunks that do not exist come last
+  const int item = MANY ? v % n_items : blockIdx.x, c0 = MANY ? v / lanes : blockIdx.y % G;
+  const int g = MANY ? v / n_items % kv_heads : blockIdx.y / G, split = MANY ? v % lanes / (n_items * kv_heads) : blockIdx.z;
+  if (!MANY && item >= n_items) return;
+  const int t0 = runs[2 * item], run = runs[2 * item + 1], nr = run & kRunLength;
+  const int nq = !MANY || run_is_short(short_pairs, run, G) ? nr * G : 0;
+  for (int i0 = c0 * kLaPairs; i0 < nq; i0 += chunks * kLaPairs) {
   const int ks = krow + 8;   // bf16 elements per staged row: 16-byte aligned, 4 words off a bank multiple
   // a value cache of its own (vc) is staged beside the keys in rows of rank + 8; else a key row's leading entries are its value
   const int vs = vc ? rank + 8 : ks;
@@ -115,7 +124,7 @@ latent_attn_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __restr
   // first keys that the window keeps: their tiles lead the walk, those between them and the window are skipped
   const int keep = EX ? ex.keep_first : 0, lead = EX ? min((keep + kLaKeys - 1) / kLaKeys, tile0) : 0;
   const int tiles = (ctx_max + kLaKeys - 1) / kLaKeys - tile0 + lead, per = (tiles + n_splits - 1) / n_splits;
-  const int walk_lo = blockIdx.z * per, walk_hi = min(tiles, (int)(blockIdx.z + 1) * per);
+  const int walk_lo = split * per, walk_hi = min(tiles, (split + 1) * per);
   for (int w = walk_lo; w < walk_hi; ++w) {
     const int base = (w < lead ? w : w - lead + tile0) * kLaKeys;
     const int n = min(kLaKeys, ctx_max - base);
@@ -227,7 +236,7 @@ latent_attn_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __restr
     const int prow = rank + 2;
     if (tid < kLaPairs && i0 + tid < nq) {
       const int i = i0 + tid;
-      float* dst = part + (((int64_t)(t0 + i / G) * heads + g * G + i % G) * n_splits + blockIdx.z) * prow;
+      float* dst = part + (((int64_t)(t0 + i / G) * heads + g * G + i % G) * n_splits + split) * prow;
       dst[rank] = mrow[tid];
       dst[rank + 1] = lrow[tid];
     }
@@ -235,7 +244,7 @@ latent_attn_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __restr
     for (int half = 0; half < 2; ++half) {
       const int p = (lane >> 2) + half * 8, i = i0 + p;
       if (i >= nq) continue;
-      float* dst = part + (((int64_t)(t0 + i / G) * heads + g * G + i % G) * n_splits + blockIdx.z) * prow;
+      float* dst = part + (((int64_t)(t0 + i / G) * heads + g * G + i % G) * n_splits + split) * prow;
 #pragma unroll
       for (int cg = 0; cg < NG; ++cg) {
         const int col0 = (warp + kLaWarps * cg) * 16;
@@ -250,7 +259,7 @@ latent_attn_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __restr
       }
     }
     if constexpr (!MANY) return;
-    __syncthreads();   // shared memory is the next item's
+    __syncthreads();   // shared memory is the next chunk's
     continue;
   }
   // finish: sink, normalise, store
@@ -283,8 +292,14 @@ latent_attn_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __restr
     }
   }
   if constexpr (!MANY) return;
-  __syncthreads();   // shared memory is the next item's
+  __syncthreads();   // shared memory is the next chunk's
   }
+  if constexpr (!MANY) return;
+  __shared__ int next;
+  if (threadIdx.x == 0) next = ticket;
+  __syncthreads();
+  v = next;
+  __syncthreads();
   }
 }
 
@@ -358,34 +373,35 @@ bool paged_attn_mma_supported(int heads, int kv_heads, int dim, int vdim) {
 static int attn_mma_launch(const float* q, const __nv_bfloat16* kc, const __nv_bfloat16* vc, int kv_heads, const int32_t* block_table,
                            int bt_stride, const int32_t* row_to_seq, const int32_t* ctx_lens, __nv_bfloat16* out, const int32_t* runs,
                            const int32_t* n_runs, int T, int heads, int krow, int rank, int block_size, float scale, const float* sink,
-                           cudaStream_t s, int n_splits, float* part, int window, const AttnExtra& ex, bool short_runs = false) {
+                           cudaStream_t s, int n_splits, float* part, int window, const AttnExtra& ex, const RunShare* share = nullptr) {
   if (n_splits < 1 || part == nullptr) n_splits = 1;
   B200_REQUIRE(n_splits <= kLaMaxSplits, B200_ERR_INVALID, "attention: %d splits (at most %d)", n_splits, kLaMaxSplits);
   B200_REQUIRE(reinterpret_cast<uintptr_t>(kc) % 16 == 0 && reinterpret_cast<uintptr_t>(vc) % 16 == 0, B200_ERR_INVALID,
                "attention: cache not 16-byte aligned");
   const size_t smem = la_smem(krow, rank, vc != nullptr);
   // a run has at most 16 rows, so a kv head's group has at most 16 G pairs: G chunks of 16
-  // (beside attn_rows_tc.cu: fewer CTAs, one for all chunks of a run and kv head, so that leaving a step of longer runs alone costs little)
-  const dim3 grid(short_runs ? std::min(T, 256) : T, short_runs ? kv_heads : heads, n_splits), block(kLaThreads);
+  // (for a share of the runs: one wave of CTAs)
+  const int64_t wave = (int64_t)kNumSMs * std::max(1, std::min(4, (int)(224 * 1024 / (smem + 1024))));
+  const dim3 grid = share ? dim3((unsigned)std::min<int64_t>((int64_t)T * heads * n_splits, wave)) : dim3(T, heads, n_splits), block(kLaThreads);
 #define LA2(NGV, EXV, MV)                                                                                                             \
   do {                                                                                                                              \
     static bool done[64] = {};                                                                                                      \
     if (smem > 48 * 1024) B200_CUDA(ensure_dynamic_smem(latent_attn_mma_kernel<NGV, EXV, MV>, 200 * 1024, done));                       \
     B200_CUDA(launch(latent_attn_mma_kernel<NGV, EXV, MV>, grid, block, smem, s, q, kc, vc, kv_heads, block_table, bt_stride, row_to_seq, \
-                     ctx_lens, out, runs, n_runs, heads, krow, rank, block_size, scale, sink, n_splits, part, window, ex, short_runs ? T : 0)); \
+                     ctx_lens, out, runs, n_runs, heads, krow, rank, block_size, scale, sink, n_splits, part, window, ex, share ? *share : RunShare())); \
   } while (0)
-#define LA(NGV, MV)                 \
-  do {                              \
-    if (ex.any()) LA2(NGV, true, MV); \
-    else LA2(NGV, false, MV);       \
+#define LA(NGV, MV)                     \
+  do {                                  \
+    if (ex.any()) LA2(NGV, true, MV);   \
+    else LA2(NGV, false, MV);           \
   } while (0)
-  if (short_runs) LA(1, true);   // (rank <= 128: attn_rows_tc.cu's shapes)
+  if (share) LA(1, true);   // (rank <= 128: attn_rows_tc.cu's shapes)
   else if (rank <= 128) LA(1, false);
   else if (rank <= 256) LA(2, false);
   else LA(4, false);
 #undef LA
 #undef LA2
-  if (n_splits > 1 && !short_runs)
+  if (n_splits > 1)
     B200_CUDA(launch(latent_attn_merge_kernel, dim3((T * heads + 3) / 4), dim3(128), (size_t)0, s, (const float*)part, out, T * heads, heads,
                      rank, n_splits, sink, static_cast<const __nv_bfloat16*>(ex.gate), ex.ldg));
   return B200_OK;
@@ -394,17 +410,21 @@ static int attn_mma_launch(const float* q, const __nv_bfloat16* kc, const __nv_b
 // runs / n_runs: the run list of the step (attn_anydim.cu builds it: runs of at most 16 consecutive rows of one sequence)
 int latent_attn_mma(const float* q, const __nv_bfloat16* kc, const int32_t* block_table, int bt_stride, const int32_t* row_to_seq,
                     const int32_t* ctx_lens, __nv_bfloat16* out, const int32_t* runs, const int32_t* n_runs, int T, int heads, int krow,
-                    int rank, int block_size, float scale, const float* sink, cudaStream_t s, int n_splits, float* part, int window) {
+                    int rank, int block_size, float scale, const float* sink, cudaStream_t s, int n_splits, float* part, int window,
+                    bool one_row_each) {
   if (T == 0) return B200_OK;
   B200_REQUIRE(latent_attn_mma_supported(heads, krow, rank), B200_ERR_UNSUPPORTED, "latent_attn_mma: shape %d / %d / %d", heads, krow, rank);
   if (n_splits < 1 || part == nullptr) n_splits = 1;
   B200_REQUIRE(n_splits <= kLaMaxSplits, B200_ERR_INVALID, "attention: %d splits (at most %d)", n_splits, kLaMaxSplits);
   const auto at = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr); };
   B200_REQUIRE(at(kc) % 16 == 0, B200_ERR_INVALID, "attention: cache not 16-byte aligned");
-  // tcgen05 wherever the shape fits and the rows can be read and written in its wide pieces (what it measured stands there; it is
-  // the faster one from one decode row up); other shapes, blocks that a key tile would straddle and odd addresses stay here, and so do
-  // scales that are not positive (masks and maxima there are taken of the unscaled scores)
-  if (scale > 0.f && latent_attn_tc_supported(heads, krow, rank, block_size) && at(q) % 16 == 0 && at(out) % 32 == 0 && ((at(runs) | at(part)) & 7) == 0) {
+  // tcgen05 wherever the shape fits and the rows can be read and written in its wide pieces (what it measured stands there); other shapes, blocks
+  // that a key tile would straddle and odd addresses stay here, and so do scales that are not positive (masks and maxima there are taken of
+  // the unscaled scores) and steps whose rows are known to be sequences of their own (or have one head: 16 pairs a run at most) where
+  // they would make more than three rounds of items there: 256 decode rows of 16 heads 102 us there, 88 here, 64 of one head in 5 splits 74 and 45
+  const bool few_pairs = (one_row_each || !row_to_seq || heads == 1) && heads <= 16 && (int64_t)T * latent_attn_tc_halves(rank) * n_splits > 3 * kNumSMs;
+  if (scale > 0.f && !few_pairs && latent_attn_tc_supported(heads, krow, rank, block_size) && at(q) % 16 == 0 && at(out) % 32 == 0 &&
+      ((at(runs) | at(part)) & 7) == 0) {
     const int rc = latent_attn_tc(q, kc, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, krow, rank, block_size, scale,
                                   sink, s, n_splits, part, window);
     if (rc || n_splits == 1) return rc;
@@ -420,7 +440,7 @@ int latent_attn_mma(const float* q, const __nv_bfloat16* kc, const int32_t* bloc
 int paged_attn_mma(const float* q, const __nv_bfloat16* kc, const __nv_bfloat16* vc, const int32_t* block_table, int bt_stride,
                    const int32_t* row_to_seq, const int32_t* ctx_lens, __nv_bfloat16* out, const int32_t* runs, const int32_t* n_runs, int T,
                    int heads, int kv_heads, int dim, int vdim, int block_size, float scale, const float* sink, cudaStream_t s, int n_splits,
-                   float* part, int window, const AttnExtra& ex) {
+                   float* part, int window, const AttnExtra& ex, bool one_row_each) {
   if (T == 0) return B200_OK;
   B200_REQUIRE(vc && paged_attn_mma_supported(heads, kv_heads, dim, vdim), B200_ERR_UNSUPPORTED, "paged_attn_mma: shape %d / %d / %d / %d", heads,
                kv_heads, dim, vdim);
@@ -428,22 +448,19 @@ int paged_attn_mma(const float* q, const __nv_bfloat16* kc, const __nv_bfloat16*
   B200_REQUIRE(n_splits <= kLaMaxSplits, B200_ERR_INVALID, "attention: %d splits (at most %d)", n_splits, kLaMaxSplits);
   const auto at = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr); };
   B200_REQUIRE(at(kc) % 16 == 0 && at(vc) % 16 == 0, B200_ERR_INVALID, "attention: cache not 16-byte aligned");
-  // tcgen05 for longer runs of rows; wider heads, smaller blocks and odd addresses stay here.  So do decode rows, which fill G of an
-  // item's 256 pairs there (256 rows at contexts 300..600, 16 heads over 4: 184 us against 80; 1 900 rows of three sequences 74
-  // against 278).  How the rows fall into runs is known on the device only: short steps stay here altogether, for others both kernels
-  // are launched, and the one whose kind of step it is not (runs of four rows on average) leaves at once
-  // (scales that are not positive stay here too: masks and maxima of the other kernel are those of the unscaled scores)
-  if (T > 128 && scale > 0.f && attn_rows_tc_supported(heads, kv_heads, dim, vdim, block_size) && at(q) % 16 == 0 && at(out) % 16 == 0 && at(part) % 8 == 0) {
-    int rc = attn_rows_tc_runs(q, kc, vc, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, kv_heads, dim, vdim,
-                               block_size, scale, sink, s, n_splits, part, window, ex);
+  // tcgen05 for longer runs of rows (1 900 rows of three sequences 74 us against 278); wider heads, smaller blocks and odd addresses stay here,
+  // and so do scales that are not positive (masks and maxima of the other kernel are those of the unscaled scores) and decode rows, which fill
+  // G of an item's 256 pairs there (256 rows at contexts 300..600, 16 heads over 4: 184 us against 80).  Short steps stay here
+  // altogether; others launch both kernels, which share the step's runs (runs.cuh), unless every row is known to be a sequence of its own
+  if (T > 128 && row_to_seq && !one_row_each && scale > 0.f && attn_rows_tc_supported(heads, kv_heads, dim, vdim, block_size) && at(q) % 16 == 0 &&
+      at(out) % 16 == 0 && at(part) % 8 == 0) {
+    RunShare share;
+    const int rc = attn_rows_tc_runs(q, kc, vc, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, kv_heads, dim, vdim,
+                                     block_size, scale, sink, s, n_splits, part, window, ex, &share);
     if (rc) return rc;
     const PdlScope after_rows;
-    rc = attn_mma_launch(q, kc, vc, kv_heads, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, dim, vdim, block_size,
-                         scale, sink, s, n_splits, part, window, ex, true);
-    if (rc || n_splits == 1) return rc;
-    B200_CUDA(launch(latent_attn_merge_kernel, dim3((T * heads + 3) / 4), dim3(128), (size_t)0, s, (const float*)part, out, T * heads, heads,
-                     vdim, n_splits, sink, static_cast<const __nv_bfloat16*>(ex.gate), ex.ldg));
-    return B200_OK;
+    return attn_mma_launch(q, kc, vc, kv_heads, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, dim, vdim, block_size,
+                           scale, sink, s, n_splits, part, window, ex, &share);
   }
   return attn_mma_launch(q, kc, vc, kv_heads, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, dim, vdim, block_size,
                          scale, sink, s, n_splits, part, window, ex);

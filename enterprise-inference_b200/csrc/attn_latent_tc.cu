@@ -70,7 +70,7 @@ __device__ __forceinline__ bool lt_item(const LtParams& p, int n_runs, int it, L
   const int run = n_runs - 1 - (whole ? it / p.items_per_run : it % n_runs);
   const int2 r = __ldg(reinterpret_cast<const int2*>(p.runs) + run);
   w.t0 = r.x + part * p.rows_per_item;
-  w.nr = min(r.y - part * p.rows_per_item, p.rows_per_item);
+  w.nr = min((r.y & kRunLength) - part * p.rows_per_item, p.rows_per_item);
   if (w.nr <= 0) return false;
   w.seq = p.row_to_seq ? __ldg(p.row_to_seq + w.t0) : w.t0;
   w.ctx0 = __ldg(p.ctx_lens + w.t0);
@@ -488,7 +488,7 @@ struct LtShape {
 // the other chunks are freed earlier, a tile and one chunk of them is enough.
 bool lt_shape(int heads, int krow, int rank, LtShape& s) {
   if (heads < 1 || heads > kLtPairs || krow % 16 || rank % 16 || rank < 16 || rank > 512 || rank > krow) return false;
-  s.halves = rank > 256 ? 2 : 1;
+  s.halves = latent_attn_tc_halves(rank);
   const int chunks = (krow + 63) / 64, own0 = (std::min(rank, 256) + 63) / 64, own1 = s.halves > 1 ? (rank - 256 + 63) / 64 : own0;
   const int max_rest = chunks - std::min(own0, own1), max_own = std::max(own0, own1);
   if (max_rest > kLtMaxRest) return false;
@@ -506,6 +506,8 @@ bool latent_attn_tc_supported(int heads, int krow, int rank, int block_size) {
   LtShape s;
   return block_size > 0 && block_size % kLtKeys == 0 && lt_shape(heads, krow, rank, s);
 }
+
+int latent_attn_tc_halves(int rank) { return rank > 256 ? 2 : 1; }
 
 // one launch over the step's run list; part given: n_splits CTAs per item leave unnormalised sums (the caller merges)
 int latent_attn_tc(const float* q, const __nv_bfloat16* kc, const int32_t* block_table, int bt_stride, const int32_t* row_to_seq,

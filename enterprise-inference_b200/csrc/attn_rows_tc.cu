@@ -20,6 +20,7 @@
 // reported (tc.cuh).
 #include <algorithm>
 
+#include "runs.cuh"
 #include "tc.cuh"
 
 namespace b200 {
@@ -37,7 +38,7 @@ constexpr int kArBiasFloats = kArTile / 4, kArBiasPad = 96;   // entries in fron
 constexpr int kArStage = 8 * 2048;             // output staging: 2 KiB per softmax warp
 constexpr int kArTable = 32;                   // items of a CTA whose description is worked out ahead
 constexpr int kArSmem = 232448;
-static_assert(1024 + 4 * kArQChunk + 9 * kArTile + kArStage + (2 * 9 + 16) * 8 + 8 + kArTable * 40 <= kArSmem, "shared memory");
+static_assert(1024 + 4 * kArQChunk + 9 * kArTile + kArStage + (2 * 9 + 16) * 8 + 16 + kArTable * 40 <= kArSmem, "shared memory");
 
 struct RowsItem {
   int row0, nrows, seq, ctx_max;   // attn_prefill.cu's plan
@@ -51,15 +52,15 @@ struct RowsParams {
   const int32_t* ctx_lens;
   const int32_t* runs;         // (first row, rows) pairs whose contexts rise by one, or
   const int32_t* n_runs;
-  const int32_t* n_short;      // runs of at most 16 rows in the step (null: no other kernel takes the step)
   const RowsItem* plan;          // runs of one sequence with their longest context; plan[0].row0 of them from plan[1]
   const float* sink;
   __nv_bfloat16* out;
   int64_t ldo;
   float* part;
   uint32_t* status;
-  int n_rows, bt_stride, heads, kv_heads, dim, vdim, block_size, n_splits, window, tile_rows;
+  int n_rows, bt_stride, heads, kv_heads, dim, vdim, block_size, n_splits, window, tile_rows, parts;   // parts: items that a run is cut into
   float scale;
+  RunShare share;
   AttnExtra ex;
 };
 
@@ -69,12 +70,13 @@ struct RowsWork {
 
 __device__ __forceinline__ int ar_tile(const RowsWork& w, int i) { return i < w.lead ? i : i - w.lead + w.tile0; }
 
-// item `it`: (run, kv head, split), the longest contexts (the last runs) first
-__device__ __forceinline__ void ar_work(const RowsParams& p, int n_runs, int it, RowsWork& w) {
+// item `it`: (run, part, kv head, split), the longest contexts (the last runs) first; false: nothing there, or not this kernel's (short_pairs)
+__device__ __forceinline__ bool ar_work(const RowsParams& p, int n_runs, int short_pairs, int it, RowsWork& w) {
   w.split = it % p.n_splits;
   it /= p.n_splits;
   w.kvh = it % p.kv_heads;
-  const int run = n_runs - 1 - it / p.kv_heads;
+  it /= p.kv_heads;
+  const int run = n_runs - 1 - it / p.parts, row = (p.parts - 1 - it % p.parts) * p.tile_rows;
   w.tile0 = w.lead = 0;
   if (p.plan) {
     const RowsItem* r = p.plan + 1 + run;
@@ -84,7 +86,12 @@ __device__ __forceinline__ void ar_work(const RowsParams& p, int n_runs, int it,
     w.ctx_max = __ldg(&r->ctx_max);
   } else {
     w.row0 = __ldg(p.runs + 2 * run);
-    w.nrows = __ldg(p.runs + 2 * run + 1);
+    const int length = __ldg(p.runs + 2 * run + 1);
+    if (short_pairs && run_is_short(short_pairs, length, p.heads / p.kv_heads)) return false;
+    w.row0 += row;
+    w.nrows = (length & kRunLength) - row;
+    if (w.nrows <= 0) return false;
+    if (p.parts > 1) w.nrows = min(w.nrows, p.tile_rows);
     w.seq = p.row_to_seq ? __ldg(p.row_to_seq + w.row0) : w.row0;
     w.ctx_max = __ldg(p.ctx_lens + w.row0 + w.nrows - 1);
     if (p.window > 0) {
@@ -95,6 +102,7 @@ __device__ __forceinline__ void ar_work(const RowsParams& p, int n_runs, int it,
   const int tiles = max((w.ctx_max + kArKeys - 1) / kArKeys - w.tile0, 0) + w.lead, per = (tiles + p.n_splits - 1) / p.n_splits;
   w.lo = min(tiles, w.split * per);
   w.hi = min(tiles, (w.split + 1) * per);
+  return true;
 }
 
 template <typename QT> __device__ __forceinline__ uint4 ar_q8(const QT* p);   // eight query entries as bf16
@@ -126,7 +134,8 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
   uint64_t* last = q_free + 1;                     // the MMAs in flight when a wait ran out
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(last + 1);   // and, behind it, the mark of a wait that ran out
   const Waits mbar_wait(tmem_slot + 1, p.status);
-  RowsWork* table = reinterpret_cast<RowsWork*>(tmem_slot + 2);
+  int* n_table = reinterpret_cast<int*>(tmem_slot + 2);   // entries of the table; the first round of items behind it
+  RowsWork* table = reinterpret_cast<RowsWork*>(n_table + 2);
   if (threadIdx.x == 0) {
     for (int s = 0; s < kArSlots; ++s) {
       mbar_init(kv_full + s, 1);
@@ -144,28 +153,53 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     tmem_slot[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  pdl_wait();
+  pdl_launch_dependents();
+  if (p.share.ticket && blockIdx.x == 0 && threadIdx.x == 0) *p.share.ticket = 0;
+  const int n_runs = p.plan ? p.plan[0].row0 : *p.n_runs, short_pairs = p.share.n_runs ? run_share(p.share, p.heads / p.kv_heads) : 0;
+  const int n_items = short_pairs == kRunsAll || (short_pairs && n_runs == p.n_rows) ? 0 : n_runs * p.parts * p.kv_heads * p.n_splits;
+  if (n_items == 0) return;   // a step of runs that are all the other kernel's
   if (warp == 9) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
-  pdl_wait();
-  pdl_launch_dependents();
-  // (steps of mostly shorter runs are attn_latent.cu's, whose launch follows this one; run list 0 decides for both)
-  const int n_runs = p.plan ? p.plan[0].row0 : *p.n_runs;
-  const int n_items = p.n_short && p.n_rows < 4 * *p.n_short ? 0 : n_runs * p.kv_heads * p.n_splits;
   const int G = p.heads / p.kv_heads, R = p.tile_rows;
   // every other round backwards: the CTA that had the longest item of one gets the shortest of the next
   const int grid = gridDim.x, cta = blockIdx.x;
   auto item_of = [&](int round) { return round * grid + ((round & 1) ? grid - 1 - cta : cta); };
-  // the descriptions hang on a chain of loads (run, sequence, contexts): all of the CTA's first ones at once, for every role
-  if (warp == 10 && item_of(lane) < n_items) ar_work(p, n_runs, item_of(lane), table[lane]);
+  // the descriptions hang on a chain of loads (run, sequence, contexts): a round to a lane, until the table is full, for every role
+  if (warp == 10) {
+    int filled = 0, round = 0;
+    while (filled < kArTable && round * grid < n_items) {
+      RowsWork w;
+      const int it = item_of(round + lane);
+      const bool have = it < n_items && ar_work(p, n_runs, short_pairs, it, w);
+      const unsigned all = __ballot_sync(0xffffffffu, have);
+      const int at = filled + __popc(all & ((1u << lane) - 1u));
+      if (have && at < kArTable) table[at] = w;
+      const unsigned late = __ballot_sync(0xffffffffu, have && at >= kArTable);   // beyond the table: their rounds come again
+      filled = min(filled + __popc(all), kArTable);
+      round += late ? __ffs(late) - 1 : 32;
+    }
+    if (lane == 0) n_table[0] = filled, n_table[1] = round;
+  }
   fence_before();
   __syncthreads();
   fence_after();
   const uint32_t tmem = *tmem_slot;   // per tile of pairs 256 columns: scores of even, odd key tiles, O
-  auto work_of = [&](int round, RowsWork& w) {
-    if (round < kArTable) w = table[round];
-    else ar_work(p, n_runs, item_of(round), w);
+  const int n_tab = n_table[0], tab_round = n_table[1];
+  // a role's next item (k: its count of calls so far); false: there is none
+  auto next_work = [&](int& k, RowsWork& w) {
+    if (k < n_tab) {
+      w = table[k++];
+      return true;
+    }
+    for (;;) {
+      const int round = tab_round + k - n_tab;
+      if (round * grid >= n_items) return false;
+      ++k;
+      if (item_of(round) < n_items && ar_work(p, n_runs, short_pairs, item_of(round), w)) return true;
+    }
   };
   // the two A operands of an item, thread i of `threads`: 16-byte pieces of rows
   auto stage_q = [&](const RowsWork& w, int i, int threads) {
@@ -203,10 +237,8 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     int slot = 0;
     uint32_t ph = 1;
     bool stop = false;
-    for (int round = 0; round * grid < n_items && !stop; ++round) {
-      if (item_of(round) >= n_items) continue;
-      RowsWork w;
-      work_of(round, w);
+    RowsWork w;
+    for (int k = 0; !stop && next_work(k, w);) {
       const int32_t* bt = p.block_table + (int64_t)w.seq * p.bt_stride;
       for (int i = w.lo; i < w.hi && !(stop = mbar_wait.stop()); ++i) {
         const int tok = ar_tile(w, i) * kArKeys;
@@ -235,13 +267,11 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     const uint64_t desc_q = make_desc(smem_u32(qs), 16, 1024), desc_k = make_desc(smem_u32(ring), 16, 1024),
                    desc_v = make_desc(smem_u32(ring), kArChunk, 1024);
     const uint32_t id_s = idesc_bf16(kArKeys, 0), id_o = idesc_bf16(p.vdim, 1);
-    const int ksteps = p.dim >> 4, items = __shfl_sync(0xffffffffu, n_items, 0);
+    const int ksteps = p.dim >> 4;
     int slot = 0, active = 0, n[2] = {0, 0};   // n: key tiles walked by either tile of pairs so far
     uint32_t ph = 0;
-    for (int round = 0; round * grid < items; ++round) {
-      if (item_of(round) >= items) continue;
-      RowsWork w;
-      work_of(round, w);
+    RowsWork w;
+    for (int k = 0; __shfl_sync(0xffffffffu, next_work(k, w), 0);) {
       const int nt = __shfl_sync(0xffffffffu, w.hi - w.lo, 0), tiles = __shfl_sync(0xffffffffu, w.nrows > R ? 2 : 1, 0);
       if (nt <= 0) continue;
       auto scores = [&](int x, int nx, int k_slot) {
@@ -315,10 +345,8 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
   } else if (warp >= 10) {
     // ===== queries of the next item -> the two A operands =====
     int active = 0;
-    for (int round = 0; round * grid < n_items; ++round) {
-      if (item_of(round) >= n_items) continue;
-      RowsWork w;
-      work_of(round, w);
+    RowsWork w;
+    for (int k = 0; next_work(k, w);) {
       if (w.hi <= w.lo) continue;
       if (active == 0) {
         stage_q(w, threadIdx.x - 64, 320);   // (beside the softmax warps' threads 0..255)
@@ -338,10 +366,10 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     constexpr float kLog2e = 1.4426950408889634f;
     const float sc2 = p.scale * kLog2e;   // scores in the log2 domain
     const float cap2 = EX ? p.ex.softcap * kLog2e : 0.f, cap_in = EX && p.ex.softcap > 0.f ? 2.0f * sc2 / p.ex.softcap : 0.f;
-    // bias in the log2 domain; a finite sentinel stays finite there (a row that sees nothing but sentinels averages, as exp would have it)
+    // bias in the log2 domain; a finite sentinel stays finite (a row that sees nothing but sentinels averages, as exp would have it)
     auto bias2 = [&](float b) {
       const float v = b * kLog2e;
-      return isinf(v) && !isinf(b) ? copysignf(3.402823466e38f, b) : v;
+      return isinf(v) ? b : v;
     };
     // the item's heads' biases by distance; in front zeros (masked keys), behind the farthest distance's, so that a tile that holds some
     // near key indexes it without clamping each distance
@@ -358,10 +386,8 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     bool first = true;
     int n = 0, slot = 0;
     uint32_t ph = 0;   // slot, ph: the ring's position (the key tile of the walk), for the value tile that is cleaned
-    for (int round = 0; round * grid < n_items; ++round) {
-      if (item_of(round) >= n_items) continue;
-      RowsWork w;
-      work_of(round, w);
+    RowsWork w;
+    for (int k = 0; next_work(k, w);) {
       if (first && w.hi > w.lo) {
         stage_q(w, threadIdx.x, 320);   // (the stagers are threads 256..319 of this)
         if (lane == 0) mbar_arrive(q_first);
@@ -602,25 +628,31 @@ int attn_rows_tc_plan(const __nv_bfloat16* q, int64_t ldq, const __nv_bfloat16* 
   p.kv_heads = kv_heads;
   p.dim = p.vdim = dim;
   p.block_size = block_size;
-  p.n_splits = 1;
+  p.n_splits = p.parts = 1;
   p.status = wait_status_word();
   p.tile_rows = 128 / (heads / kv_heads);
   p.scale = scale;
   return ar_launch<__nv_bfloat16, true, false>(mk, mv, p, T, s);
 }
 
-// fp32 queries [T][heads][dim], weights rounded to bf16; runs, n_runs: the first of the lists that paged_attn_runs_plan leaves for T rows
+// fp32 queries [T][heads][dim], weights of 16 bits; runs, n_runs: the first of the lists that paged_attn_runs_plan leaves for T rows.  Launched
+// beside the mma.sync kernel, which takes share's runs.
 int attn_rows_tc_runs(const float* q, const __nv_bfloat16* kc, const __nv_bfloat16* vc, const int32_t* block_table, int bt_stride,
                       const int32_t* row_to_seq, const int32_t* ctx_lens, __nv_bfloat16* out, const int32_t* runs, const int32_t* n_runs, int T,
                       int heads, int kv_heads, int dim, int vdim, int block_size, float scale, const float* sink, cudaStream_t s, int n_splits,
-                      float* part, int window, const AttnExtra& ex) {
+                      float* part, int window, const AttnExtra& ex, RunShare* share) {
   CUtensorMap mk, mv;
   int rc = get_tensor_map_2d(kc, 1ull << 31, dim, dim, 64, &mk);
   if (rc) return rc;
   rc = get_tensor_map_2d(vc, 1ull << 31, vdim, vdim, 64, &mv);
   if (rc) return rc;
-  int list = 0;   // the longest runs whose pairs fit two tiles: 16 << list rows
+  // the longest runs whose pairs fit an item: two tiles of 8 << list rows, or one, as attn_rows_tc_rows has it (200 rows in runs of 12, 16 heads
+  // over one, contexts 300 to 600: 49.5 us, with two 58; 300 rows of one sequence, 16 over 4: 49 and 60)
+  int list = 0;
   while (list + 1 < kRunLists && (16 << (list + 1)) <= 2 * (128 / (heads / kv_heads))) ++list;
+  const int tile_rows = 8 << list;
+  const bool one = (int64_t)T * kv_heads < (int64_t)tile_rows * kNumSMs;
+  if (one && list > 0) --list;
   RowsParams p = {};
   p.q = q;
   p.ldq = (int64_t)heads * dim;
@@ -629,7 +661,6 @@ int attn_rows_tc_runs(const float* q, const __nv_bfloat16* kc, const __nv_bfloat
   p.ctx_lens = ctx_lens;
   p.runs = runs + (int64_t)2 * T * list;
   p.n_runs = n_runs + list;
-  p.n_short = n_runs;
   p.n_rows = T;
   p.sink = sink;
   p.out = out;
@@ -644,7 +675,9 @@ int attn_rows_tc_runs(const float* q, const __nv_bfloat16* kc, const __nv_bfloat
   p.block_size = block_size;
   p.n_splits = n_splits;
   p.window = window;
-  p.tile_rows = 8 << list;
+  p.tile_rows = tile_rows;
+  p.parts = one && (kRunRows << list) > tile_rows ? 2 : 1;   // (no list of runs of 8 rows)
+  *share = p.share = {p.n_runs, const_cast<int32_t*>(n_runs) + kRunTicket, T, kv_heads * n_splits, p.parts};
   p.scale = scale;
   p.ex = ex;
   return ex.any() ? ar_launch<float, true, true>(mk, mv, p, T, s) : ar_launch<float, true, false>(mk, mv, p, T, s);

@@ -364,26 +364,31 @@ int paged_attn_anydim(bool f32, const float* q, const void* kc, const void* vc, 
                       const AttnExtra& ex = AttnExtra());
 // kstride / vstride: elements per cache row when they exceed dim / vdim (0: dim / vdim; the value cache may then be the key
 // cache itself, a value being the leading vdim entries of the row); sink [heads]: exp(sink[h]) joins the softmax denominator
-constexpr int kRunLists = 5;   // lists of runs of at most 16, 32, 64, 128, 256 rows
+constexpr int kRunRows = 16, kRunLists = 5;   // lists of runs of at most 16, 32, 64, 128, 256 rows: (first row, length | kRunWhole)
+constexpr int kRunLength = 0xffff, kRunWhole = 1 << 16;   // whole: the run is all of its segment of rising contexts
+constexpr int kRunTicket = 5;   // word behind the lists' lengths: runs.cuh
 int paged_attn_runs_plan(const int32_t* row_to_seq, const int32_t* ctx_lens, int T, void* ws, cudaStream_t s);
 // latent cache rows on the tensor cores (attn_latent.cu): bf16 cache, fp32 queries, bf16 output [T][heads][rank]
 bool latent_attn_mma_supported(int heads, int krow, int rank);
 int latent_attn_mma(const float* q, const __nv_bfloat16* kc, const int32_t* block_table, int bt_stride, const int32_t* row_to_seq,
                     const int32_t* ctx_lens, __nv_bfloat16* out, const int32_t* runs, const int32_t* n_runs, int T, int heads, int krow,
                     int rank, int block_size, float scale, const float* sink, cudaStream_t s, int n_splits = 1, float* part = nullptr,
-                    int window = 0);
+                    int window = 0, bool one_row_each = false);
+// (one_row_each: the step's rows are known to be sequences of their own, as decode steps are)
 // the same attention on tcgen05 (attn_latent_tc.cu), which latent_attn_mma takes for the shapes it fits; n_splits > 1: unmerged sums in part
 bool latent_attn_tc_supported(int heads, int krow, int rank, int block_size);
 int latent_attn_tc(const float* q, const __nv_bfloat16* kc, const int32_t* block_table, int bt_stride, const int32_t* row_to_seq,
                    const int32_t* ctx_lens, __nv_bfloat16* out, const int32_t* runs, const int32_t* n_runs, int T, int heads, int krow,
                    int rank, int block_size, float scale, const float* sink, cudaStream_t s, int n_splits, float* part, int window);
+int latent_attn_tc_halves(int rank);   // items that it makes of a run of few rows
 // the same kernel for grouped-query attention over key and value caches [block][kv_heads][block_size][dim | vdim]
 bool paged_attn_mma_supported(int heads, int kv_heads, int dim, int vdim);
 int paged_attn_mma(const float* q, const __nv_bfloat16* kc, const __nv_bfloat16* vc, const int32_t* block_table, int bt_stride,
                    const int32_t* row_to_seq, const int32_t* ctx_lens, __nv_bfloat16* out, const int32_t* runs, const int32_t* n_runs, int T,
                    int heads, int kv_heads, int dim, int vdim, int block_size, float scale, const float* sink, cudaStream_t s,
-                   int n_splits = 1, float* part = nullptr, int window = 0, const AttnExtra& ex = AttnExtra());
+                   int n_splits = 1, float* part = nullptr, int window = 0, const AttnExtra& ex = AttnExtra(), bool one_row_each = false);
 // grouped-query attention for heads of at most 128 entries on tcgen05, two tiles of 128 (row, head) pairs a CTA (attn_rows_tc.cu)
+struct RunShare;   // runs.cuh
 int attn_rows_tc_rows(int T, int heads, int kv_heads);
 bool attn_rows_tc_supported(int heads, int kv_heads, int dim, int vdim, int block_size);
 int attn_rows_tc_plan(const __nv_bfloat16* q, int64_t ldq, const __nv_bfloat16* kc, const __nv_bfloat16* vc, const int32_t* block_table, int bt_stride,
@@ -392,7 +397,7 @@ int attn_rows_tc_plan(const __nv_bfloat16* q, int64_t ldq, const __nv_bfloat16* 
 int attn_rows_tc_runs(const float* q, const __nv_bfloat16* kc, const __nv_bfloat16* vc, const int32_t* block_table, int bt_stride,
                       const int32_t* row_to_seq, const int32_t* ctx_lens, __nv_bfloat16* out, const int32_t* runs, const int32_t* n_runs, int T,
                       int heads, int kv_heads, int dim, int vdim, int block_size, float scale, const float* sink, cudaStream_t s, int n_splits,
-                      float* part, int window, const AttnExtra& ex);
+                      float* part, int window, const AttnExtra& ex, RunShare* share);
 // context splits for a step (1: none); part holds T * heads * n_splits * (rank + 2) floats
 int latent_attn_splits(int T, int heads, int rank, int max_ctx, int64_t ws_bytes);
 // mixture of experts (moe.cu)

@@ -467,6 +467,7 @@ static int stack_enqueue_step_postnorm(b200_ctx* c, const StepArgs& a, cudaStrea
   B200_REQUIRE(!stateful || seq_slots, B200_ERR_STATE, "step: the state slots of the step's sequences were not given");
   B200_REQUIRE(S <= T, B200_ERR_INVALID, "step: %d sequences in %d rows", S, T);
   int attn_plan = (a.row_to_seq && T >= 32 && T >= 2 * S) ? 1 : 0;
+  const bool own_rows = !a.row_to_seq || a.n_seqs == T;   // decode: every row a sequence of its own
   static const int plan_env = getenv("B200_STACK_ATTN_RUNS") ? atoi(getenv("B200_STACK_ATTN_RUNS")) : 1;
   if (!plan_env) attn_plan = 0;
   bool runs_built = false;   // the step's run list is in the attention workspace
@@ -501,7 +502,7 @@ static int stack_enqueue_step_postnorm(b200_ctx* c, const StepArgs& a, cudaStrea
         STEP(paged_attn_mma(M->q, (const __nv_bfloat16*)W.kc, (const __nv_bfloat16*)W.vc, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens,
                             (__nv_bfloat16*)M->attn, static_cast<const int32_t*>(M->attn_ws) + 8, static_cast<const int32_t*>(M->attn_ws), T,
                             L.heads, L.kv_heads, L.dim, L.vdim, m.block_size, L.scale, sink, s,
-                            latent_attn_splits(T, L.heads, L.vdim, seen, M->lat_ws_bytes), M->lat_ws, L.window));
+                            latent_attn_splits(T, L.heads, L.vdim, seen, M->lat_ws_bytes), M->lat_ws, L.window, AttnExtra(), own_rows));
       } else {
       if (attn_plan) STEP(step_runs(runs_built));
       STEP(paged_attn_anydim(f32, M->q, W.kc, W.vc, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens, a.positions, nullptr, max_pos,
@@ -520,7 +521,7 @@ static int stack_enqueue_step_postnorm(b200_ctx* c, const StepArgs& a, cudaStrea
         const int seen = L.window > 0 ? std::min(a.max_ctx, L.window + 64) : a.max_ctx;
         STEP(latent_attn_mma(M->q, (const __nv_bfloat16*)cache, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens, (__nv_bfloat16*)M->lat,
                              static_cast<const int32_t*>(M->attn_ws) + 8, static_cast<const int32_t*>(M->attn_ws), T, L.heads, kr, kr,
-                             m.block_size, L.scale, nullptr, s, latent_attn_splits(T, L.heads, kr, seen, M->lat_ws_bytes), M->lat_ws, L.window));
+                             m.block_size, L.scale, nullptr, s, latent_attn_splits(T, L.heads, kr, seen, M->lat_ws_bytes), M->lat_ws, L.window, own_rows));
       } else {
         if (attn_plan) STEP(step_runs(runs_built));
         STEP(paged_attn_anydim(f32, M->q, cache, cache, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens, a.positions, nullptr, 1ll << 40,
@@ -581,6 +582,7 @@ static int stack_enqueue_step_parallel(b200_ctx* c, const StepArgs& a, cudaStrea
   B200_REQUIRE(!stateful || seq_slots, B200_ERR_STATE, "step: the state slots of the step's sequences were not given");
   B200_REQUIRE(S <= T, B200_ERR_INVALID, "step: %d sequences in %d rows", S, T);
   int attn_plan = (a.row_to_seq && T >= 32 && T >= 2 * S) ? 1 : 0;
+  const bool own_rows = !a.row_to_seq || a.n_seqs == T;   // decode: every row a sequence of its own
   static const int plan_env = getenv("B200_STACK_ATTN_RUNS") ? atoi(getenv("B200_STACK_ATTN_RUNS")) : 1;
   if (!plan_env) attn_plan = 0;
   bool runs_built = false;   // the step's run list is in the attention workspace
@@ -638,7 +640,7 @@ static int stack_enqueue_step_parallel(b200_ctx* c, const StepArgs& a, cudaStrea
         STEP(paged_attn_mma(M->q, (const __nv_bfloat16*)W.kc, (const __nv_bfloat16*)W.vc, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens,
                             (__nv_bfloat16*)M->attn, static_cast<const int32_t*>(M->attn_ws) + 8, static_cast<const int32_t*>(M->attn_ws), T,
                             L.heads, L.kv_heads, L.dim, L.vdim, m.block_size, L.scale, sink, s,
-                            latent_attn_splits(T, L.heads, L.vdim, seen, M->lat_ws_bytes), M->lat_ws, L.window, ex));
+                            latent_attn_splits(T, L.heads, L.vdim, seen, M->lat_ws_bytes), M->lat_ws, L.window, ex, own_rows));
       } else {
         if (attn_plan) STEP(step_runs(runs_built));
         STEP(paged_attn_anydim(f32, M->q, W.kc, W.vc, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens, a.positions, nullptr, 1ll << 40,
@@ -675,7 +677,7 @@ static int stack_enqueue_step_parallel(b200_ctx* c, const StepArgs& a, cudaStrea
         STEP(latent_attn_mma(M->q, (const __nv_bfloat16*)W.kc, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens,
                              (__nv_bfloat16*)M->lat, static_cast<const int32_t*>(M->attn_ws) + 8, static_cast<const int32_t*>(M->attn_ws), T,
                              L.heads, krow, L.kv_rank, m.block_size, L.scale, sink, s,
-                             latent_attn_splits(T, L.heads, L.kv_rank, a.max_ctx, M->lat_ws_bytes), M->lat_ws));
+                             latent_attn_splits(T, L.heads, L.kv_rank, a.max_ctx, M->lat_ws_bytes), M->lat_ws, 0, own_rows));
       } else {
         if (attn_plan) STEP(step_runs(runs_built));
         STEP(paged_attn_anydim(f32, M->q, W.kc, W.kc, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens, a.positions, nullptr, max_pos,
@@ -772,6 +774,7 @@ static int stack_enqueue_step_hyper(b200_ctx* c, const StepArgs& a, cudaStream_t
   B200_REQUIRE(!stateful || seq_slots, B200_ERR_STATE, "step: the state slots of the step's sequences were not given");
   B200_REQUIRE(S <= T, B200_ERR_INVALID, "step: %d sequences in %d rows", S, T);
   int attn_plan = (a.row_to_seq && T >= 32 && T >= 2 * S) ? 1 : 0;
+  const bool own_rows = !a.row_to_seq || a.n_seqs == T;   // decode: every row a sequence of its own
   static const int plan_env = getenv("B200_STACK_ATTN_RUNS") ? atoi(getenv("B200_STACK_ATTN_RUNS")) : 1;
   if (!plan_env) attn_plan = 0;
   bool runs_built = false;   // the step's run list is in the attention workspace
@@ -829,7 +832,7 @@ static int stack_enqueue_step_hyper(b200_ctx* c, const StepArgs& a, cudaStream_t
         STEP(paged_attn_mma(M->q, (const __nv_bfloat16*)W.kc, (const __nv_bfloat16*)W.vc, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens,
                             (__nv_bfloat16*)M->attn, static_cast<const int32_t*>(M->attn_ws) + 8, static_cast<const int32_t*>(M->attn_ws), T,
                             L.heads, L.kv_heads, L.dim, L.vdim, m.block_size, L.scale, sink, s,
-                            latent_attn_splits(T, L.heads, L.vdim, seen, M->lat_ws_bytes), M->lat_ws, L.window));
+                            latent_attn_splits(T, L.heads, L.vdim, seen, M->lat_ws_bytes), M->lat_ws, L.window, AttnExtra(), own_rows));
       } else {
         if (attn_plan) STEP(step_runs(runs_built));
         STEP(paged_attn_anydim(f32, M->q, W.kc, W.vc, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens, a.positions, nullptr, max_pos,
@@ -918,6 +921,7 @@ static int stack_enqueue_step_looped(b200_ctx* c, const StepArgs& a, cudaStream_
   static const int plan_env = getenv("B200_STACK_ATTN_RUNS") ? atoi(getenv("B200_STACK_ATTN_RUNS")) : 1;
   static const int chunk_env = getenv("B200_STACK_RETENTION_CHUNK") ? atoi(getenv("B200_STACK_RETENTION_CHUNK")) : 1;
   const bool attn_plan = plan_env && a.row_to_seq && T >= 32 && T >= 2 * S;
+  const bool own_rows = !a.row_to_seq || a.n_seqs == T;   // decode: every row a sequence of its own
   bool runs_built = false;   // the step's run list is in the attention workspace
   auto step_runs = [&]() -> int {
     if (runs_built) return B200_OK;
@@ -978,7 +982,7 @@ static int stack_enqueue_step_looped(b200_ctx* c, const StepArgs& a, cudaStream_
         STEP(paged_attn_mma(M->q, (const __nv_bfloat16*)W.kc, (const __nv_bfloat16*)W.vc, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens,
                             (__nv_bfloat16*)M->attn, static_cast<const int32_t*>(M->attn_ws) + 8, static_cast<const int32_t*>(M->attn_ws), T,
                             L.heads, L.kv_heads, L.dim, L.vdim, m.block_size, L.scale, nullptr, s,
-                            latent_attn_splits(T, L.heads, L.vdim, seen, M->lat_ws_bytes), M->lat_ws, L.window, ex));
+                            latent_attn_splits(T, L.heads, L.vdim, seen, M->lat_ws_bytes), M->lat_ws, L.window, ex, own_rows));
       } else {
         if (attn_plan) STEP(step_runs());
         STEP(paged_attn_anydim(f32, M->q, W.kc, W.vc, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens, a.positions, nullptr, 1ll << 40,

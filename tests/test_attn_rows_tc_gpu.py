@@ -180,3 +180,53 @@ def test_scales_that_are_not_positive(scale, cap):
     got, want = out.double().cpu(), _oracle(q, rows, scale, cap=cap)
     # weights and results rounded to bf16 once each: 2^-9 of the largest value, 2^-9 of the result
     assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -9 * rows[1].float().abs().max()).all()
+
+
+def _dense(q, rows, ctxs, scale, window=0):
+    """All rows at once over the same cached tokens, float64."""
+    K, V = (r.double() for r in rows)
+    G, c = q.shape[1] // K.shape[1], torch.tensor(ctxs)[:, None]
+    j = torch.arange(K.shape[0])[None, :]
+    seen = (j < c) & ((j >= c - window) if window else (j >= 0))
+    s = torch.einsum("thd,chd->thc", q.double(), K.repeat_interleave(G, 1)) * scale
+    return torch.einsum("thc,chd->thd", torch.softmax(s.masked_fill(~seen[:, None], float("-inf")), -1), V.repeat_interleave(G, 1))
+
+
+def _steps(runs):
+    """(first context, rows) per run of a sequence of its own -> sequence and context of every row."""
+    return [s for s, (_, n) in enumerate(runs) for _ in range(n)], [c + i for c, n in runs for i in range(n)]
+
+
+_MIX = [(7 * i % 180 + 1, 1) for i in range(300)] + [(5, 2), (60, 3), (1, 5), (33, 8), (100, 9), (64, 15), (20, 16), (1, 17), (127, 40), (3, 100)]
+_MIX = _MIX[:150] + _MIX[300:] + _MIX[150:300] + [(50 + i, 2) for i in range(8)]      # long runs between decode rows
+
+
+# Which kernel takes a run, over steps that both share or one has to itself, and walks of several trips in either: a mixed step (300 runs of one
+# row, others of 2 to 100) with 16 heads over 4, 32 over 2, splits, a window; decode rows only; runs at the border of 16 pairs an item; few
+# rows with many heads a group (items of 8 rows); 5 120 items of 40 rows (more than a CTA describes ahead).
+@pytest.mark.parametrize("heads,kv,dim,runs,ns,window", [
+    (16, 4, 64, _MIX, 1, 0), (16, 4, 64, _MIX, 2, 0), (32, 2, 48, _MIX, 1, 0), (32, 2, 64, _MIX, 2, 50), (8, 8, 32, _MIX, 1, 0),
+    (16, 4, 64, [(i % 190 + 1, 1) for i in range(400)], 1, 0), (16, 4, 64, [(3 * i + 1, 4) for i in range(50)], 1, 0),
+    (16, 4, 64, [(3 * i + 1, 5) for i in range(50)], 1, 0), (16, 1, 64, [(9 * i + 1, 12) for i in range(14)], 1, 40), (16, 1, 128, [(30, 150)], 1, 0),
+    (2, 2, 64, [(1, 180)], 1, 0), (32, 32, 16, [(i % 120 + 1, 40) for i in range(160)], 1, 0)])
+def test_runs_shared_between_the_kernels(heads, kv, dim, runs, ns, window):
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    bs, n_tok = 64, 192
+    seq, ctxs = _steps(runs)
+    T, g = len(seq), torch.Generator().manual_seed(heads + dim)
+    rows = [torch.randn(n_tok, kv, dim, generator=g).to(torch.bfloat16) for _ in range(2)]
+    kc, vc = (r.reshape(n_tok // bs, bs, kv, dim).transpose(1, 2).contiguous().to(DEV) for r in rows)
+    q = torch.randn(T, heads, dim, generator=g).to(torch.bfloat16)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)   # noqa: E731
+    bt, sq, cx = i32([[0, 1, 2]]).repeat(len(runs), 1).contiguous(), i32(seq), i32(ctxs)
+    ws = torch.zeros(int(lib.b200_paged_attn_anydim_workspace_bytes(T)), dtype=torch.uint8, device=DEV)
+    out = torch.full((T, heads, dim), float("nan"), dtype=torch.bfloat16, device=DEV)
+    part = torch.full((T * heads * ns * (dim + 2),), float("nan"), device=DEV)
+    qd = q.float().to(DEV)
+    check(lib.b200_paged_attn_mma(qd.data_ptr(), kc.data_ptr(), vc.data_ptr(), bt.data_ptr(), 3, sq.data_ptr(), cx.data_ptr(), out.data_ptr(), T, heads, kv,
+                                  dim, dim, bs, dim ** -0.5, None, ws.data_ptr(), window, ns, part.data_ptr() if ns > 1 else None, None))
+    torch.cuda.synchronize()
+    got, want = out.double().cpu(), _dense(q, rows, ctxs, dim ** -0.5, window)
+    assert torch.isfinite(got).all()
+    # where the mma.sync kernel works, weights and results are rounded to bf16 once each: 2^-9 of the largest value, 2^-9 of the result
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -9 * rows[1].float().abs().max()).all()

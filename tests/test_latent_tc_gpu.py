@@ -84,3 +84,32 @@ def test_latent_scales_that_are_not_positive(scale):
     want = torch.stack([_oracle(q[t].double(), rows.double(), ctxs[t], rank, scale, None, 0) for t in range(T)])
     # weights and results rounded to bf16 once each: 2^-9 of the largest value, 2^-9 of the result
     assert ((out.double().cpu() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -9 * rows.float().abs().max()).all()
+
+
+# Steps of many items: decode rows (the mma.sync kernel's, runs of one), rows in pairs (the tcgen05 kernel's: 32 pairs an item; 4 800 items, more
+# than a CTA describes ahead), both in one step, and splits.
+@pytest.mark.parametrize("heads,rank,rd,runs,splits", [
+    (16, 272, 16, [1] * 400, 1), (16, 272, 16, [2] * 1200, 1), (4, 64, 16, [1] * 300 + [40, 90], 2), (16, 512, 64, [1] * 230, 1), (1, 272, 16, [1] * 64, 5)])
+def test_latent_steps_of_many_items(heads, rank, rd, runs, splits):
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    g = torch.Generator().manual_seed(heads + rank)
+    krow, bs, scale = rank + rd, 64, 1.0 / (rank + rd) ** 0.5
+    seq = [s for s, n in enumerate(runs) for _ in range(n)]
+    ctxs = [(11 * s) % 90 + 1 + i for s, n in enumerate(runs) for i in range(n)]
+    T, rows = len(seq), torch.randn(192, krow, generator=g).to(torch.bfloat16)
+    q = torch.randn(T, heads, krow, generator=g).to(torch.bfloat16)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)   # noqa: E731
+    bt, sq, cx, kd, qd = i32([[0, 1, 2]]).repeat(len(runs), 1).contiguous(), i32(seq), i32(ctxs), rows.reshape(3, 1, bs, krow).to(DEV), q.float().to(DEV)
+    ws = torch.zeros(int(lib.b200_paged_attn_anydim_workspace_bytes(T)), dtype=torch.uint8, device=DEV)
+    out = torch.full((T, heads, rank), float("nan"), dtype=torch.bfloat16, device=DEV)
+    part = torch.full((T * heads * splits * (rank + 2),), float("nan"), device=DEV)
+    check(lib.b200_latent_attn(qd.data_ptr(), kd.data_ptr(), bt.data_ptr(), 3, sq.data_ptr(), cx.data_ptr(), out.data_ptr(), T, heads, krow, rank, bs,
+                               scale, None, ws.data_ptr(), splits, part.data_ptr() if splits > 1 else None, None))
+    torch.cuda.synchronize()
+    K = rows.double()
+    s = torch.einsum("thd,cd->thc", q.double(), K) * scale
+    s = s.masked_fill(torch.arange(192)[None, None, :] >= torch.tensor(ctxs)[:, None, None], float("-inf"))
+    got, want = out.double().cpu(), torch.einsum("thc,cd->thd", torch.softmax(s, -1), K[:, :rank])
+    assert torch.isfinite(got).all()
+    # weights and results rounded to bf16 once each: 2^-9 of the largest value, 2^-9 of the result
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -9 * rows.float().abs().max()).all()
