@@ -129,7 +129,7 @@ delta_tails_kernel(const AT* __restrict__ fused, int64_t ld, const int32_t* __re
 // so the eight sums of two rows and four columns are reduced together (a lane keeps half of what it holds at every step: 9 shuffles
 // instead of 40), and the two dot products of inputs alone are taken once per stage for all columns.  The read-out leaves per-lane sums in
 // shared memory, added for the whole stage after its walk.
-// 1 900 rows of three sequences, 16 heads of 128 x 128, channel decays: @D1900@ (one row per turn, unpacked, eight warps a CTA: 457 us).
+// 1 900 rows of three sequences, 16 heads of 128 x 128, channel decays: 295 us (one row per turn, unpacked, eight warps a CTA: 457 us).
 constexpr int kDsWarps = 4, kDsCols = 4 * kDsWarps, kDsStage = 16, kDsThreads = kDsWarps * 32;
 constexpr int kDsFlush = 8;       // rows whose read-out sums are kept (with all 16 of a stage only two CTAs fit an SM: 342 us instead)
 constexpr int kDsPartRow = 144;   // floats of a row of read-out sums: 32 lanes x 4 columns, rows 64 bytes apart in the banks
@@ -196,6 +196,102 @@ __device__ __forceinline__ void ds_reduce(float (&v)[N], int lane) {
   for (int i = 0; i < N; ++i) v[i] = __shfl_sync(0xffffffffu, x[0], i * (32 / N));   // value i ended with the lanes i * 32 / N ..
 }
 
+// One row by itself: the four columns' state (pairs of channels, as ds_chan has them) is decayed, corrected, added to and read.  The row's q, k and
+// decays (g_chan apart) start at the head, v and out at the warp's first column, `cols` of which exist.
+template <int NP, bool DELTA, bool CHAN>
+__device__ __forceinline__ void ds_row_alone(const float* q, const float* k, const float* g, int g_chan, const float* v, float b, float* out, int dim, int cols,
+                                             int lane, uint64_t (&S)[4][NP]) {
+  uint64_t kk[NP], qq[NP];
+  const float gs = CHAN ? 0.f : g[0];
+  float d4[4] = {0.f, 0.f, 0.f, 0.f}, o4[4], v4[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) v4[c] = c < cols ? v[c] : 0.f;
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const int d = ds_chan<NP>(lane, i);
+    auto pair = [&](const float* p, int64_t st) { return f2::pack(d < dim ? p[d * st] : 0.f, d + 1 < dim ? p[(d + 1) * st] : 0.f); };
+    kk[i] = pair(k, 1);
+    qq[i] = pair(q, 1);
+    const uint64_t gg = CHAN ? pair(g, g_chan) : f2::both(gs);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) S[c][i] = f2::mul(S[c][i], gg);
+  }
+  if (DELTA) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      uint64_t acc = f2::mul(S[c][0], kk[0]);
+#pragma unroll
+      for (int i = 1; i < NP; ++i) acc = f2::fma(S[c][i], kk[i], acc);
+      d4[c] = f2::sum(acc);
+    }
+    ds_reduce<4>(d4, lane);
+  }
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const uint64_t u = f2::both(b * (v4[c] - d4[c]));
+    uint64_t acc = 0;
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      S[c][i] = f2::fma(kk[i], u, S[c][i]);
+      acc = f2::fma(S[c][i], qq[i], acc);
+    }
+    o4[c] = f2::sum(acc);
+  }
+  ds_reduce<4>(o4, lane);
+  const float mine = lane == 0 ? o4[0] : lane == 1 ? o4[1] : lane == 2 ? o4[2] : o4[3];
+  if (lane < cols) out[lane] = mine;   // (cols <= 4)
+}
+template <int NP>
+__device__ __forceinline__ void ds_load(const float* S_st, int dim, int cols, int vec, bool fresh, int lane, uint64_t (&S)[4][NP]) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      const int d = ds_chan<NP>(lane, i);
+      const float* p = S_st + (int64_t)c * dim + d;
+      S[c][i] = 0;
+      if (!fresh && c < cols && d < dim) S[c][i] = vec ? *reinterpret_cast<const uint64_t*>(p) : f2::pack(p[0], d + 1 < dim ? p[1] : 0.f);
+    }
+}
+template <int NP>
+__device__ __forceinline__ void ds_store(float* S_st, int dim, int cols, int vec, int lane, const uint64_t (&S)[4][NP]) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      const int d = ds_chan<NP>(lane, i);
+      float* p = S_st + (int64_t)c * dim + d;
+      if (c >= cols || d >= dim) continue;
+      if (vec) {
+        *reinterpret_cast<uint64_t*>(p) = S[c][i];
+      } else {
+        p[0] = f2::lo(S[c][i]);
+        if (d + 1 < dim) p[1] = f2::hi(S[c][i]);
+      }
+    }
+}
+
+// Steps of decode rows (one row per sequence): the walk without its stages' shared memory, which leaves three or four CTAs to an SM.
+// 64 sequences, 16 heads of 128 x 128, channel decays: 37 us in the walk, 23 here; the uncorrected rule, 64 heads of 128 x 64: 4 sequences 8.4
+// and 6.4 (7.0 at the unpacked walk, whose CTAs were fewer), 200 sequences 180 and 105.
+template <int NP, bool DELTA, bool CHAN>
+__global__ void __launch_bounds__(kDsThreads) delta_rows_kernel(const ScanArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int s = blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int start = a.seq_start[s], end = a.seq_start[s + 1];
+  if (end <= start) return;
+  const int j0 = blockIdx.z * kDsCols + warp * 4, cols = min(a.vd - j0, 4), g = h / (a.heads / a.kv_heads), dim = a.dim;
+  float* S_st = a.state + (int64_t)a.seq_slots[s] * a.slot_stride + ((int64_t)h * a.vd + j0) * dim;
+  const int64_t qk = (int64_t)a.kv_heads * dim, hv = (int64_t)a.heads * a.vd;
+  uint64_t S[4][NP];
+  ds_load<NP>(S_st, dim, cols, a.vec, a.positions[start] == 0, lane, S);
+  for (int64_t t = start; t < end; ++t)
+    ds_row_alone<NP, DELTA, CHAN>(a.qn + t * qk + (int64_t)g * dim, a.kn + t * qk + (int64_t)g * dim, a.decay + t * a.g_row + (int64_t)h * a.g_head, a.g_chan,
+                                  a.vn + t * hv + (int64_t)h * a.vd + j0, a.beta[t * a.heads + h], a.out + t * hv + (int64_t)h * a.vd + j0, dim, cols, lane, S);
+  ds_store<NP>(S_st, dim, cols, a.vec, lane, S);
+}
+
 // CHAN: a decay per key channel, else one per row and head.
 template <int NP, bool DELTA, bool CHAN>
 __global__ void __launch_bounds__(kDsThreads) delta_scan_kernel(const ScanArgs a) {
@@ -218,54 +314,10 @@ __global__ void __launch_bounds__(kDsThreads) delta_scan_kernel(const ScanArgs a
   const float* vsrc = a.vn + (int64_t)start * hv + (int64_t)h * vd + jb;
   const float* bsrc = a.beta + (int64_t)start * a.heads + h;
   uint64_t S[4][NP];
-#pragma unroll
-  for (int c = 0; c < 4; ++c)
-#pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      const int d = ds_chan<NP>(lane, i);
-      const float* p = S_st + (int64_t)c * dim + d;
-      S[c][i] = 0;
-      if (!fresh && j0 + c < vd && d < dim) S[c][i] = a.vec ? *reinterpret_cast<const uint64_t*>(p) : f2::pack(p[0], d + 1 < dim ? p[1] : 0.f);
-    }
-  if (n_rows == 1) {
-    // a decode row: nothing to stage; the row's inputs are fetched beside the state
-    const float b = bsrc[0], gs = CHAN ? 0.f : gsrc[0];
-    uint64_t k[NP], q[NP];
-    float d4[4] = {0.f, 0.f, 0.f, 0.f}, o4[4];
-#pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      const int d = ds_chan<NP>(lane, i);
-      auto pair = [&](const float* p, int64_t st) { return f2::pack(d < dim ? p[d * st] : 0.f, d + 1 < dim ? p[(d + 1) * st] : 0.f); };
-      k[i] = pair(ksrc, 1);
-      q[i] = pair(qsrc, 1);
-      const uint64_t gg = CHAN ? pair(gsrc, a.g_chan) : f2::both(gs);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) S[c][i] = f2::mul(S[c][i], gg);
-    }
-    if (DELTA) {
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint64_t acc = f2::mul(S[c][0], k[0]);
-#pragma unroll
-        for (int i = 1; i < NP; ++i) acc = f2::fma(S[c][i], k[i], acc);
-        d4[c] = f2::sum(acc);
-      }
-      ds_reduce<4>(d4, lane);
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const uint64_t u = f2::both(b * ((j0 + c < vd ? vsrc[warp * 4 + c] : 0.f) - d4[c]));
-      uint64_t acc = 0;
-#pragma unroll
-      for (int i = 0; i < NP; ++i) {
-        S[c][i] = f2::fma(k[i], u, S[c][i]);
-        acc = f2::fma(S[c][i], q[i], acc);
-      }
-      o4[c] = f2::sum(acc);
-    }
-    ds_reduce<4>(o4, lane);
-    const float mine = lane == 0 ? o4[0] : lane == 1 ? o4[1] : lane == 2 ? o4[2] : o4[3];
-    if (lane < 4 && j0 + lane < vd) a.out[(int64_t)start * hv + (int64_t)h * vd + j0 + lane] = mine;
+  ds_load<NP>(S_st, dim, vd - j0, a.vec, fresh, lane, S);
+  if (n_rows == 1) {   // a decode row beside others' portions: nothing to stage, the row's inputs are fetched beside the state
+    ds_row_alone<NP, DELTA, CHAN>(qsrc, ksrc, gsrc, a.g_chan, vsrc + warp * 4, bsrc[0], a.out + (int64_t)start * hv + (int64_t)h * vd + j0, dim, min(vd - j0, 4),
+                                  lane, S);
   } else {
     float* kq = stage + 2 * BUF;                                          // [kDsStage] per pair of rows: k1 g2 k2, k1 . q1
     float* part = kq + kDsStage + warp * kDsFlush * kDsPartRow;
@@ -444,20 +496,7 @@ __global__ void __launch_bounds__(kDsThreads) delta_scan_kernel(const ScanArgs a
       }
     }
   }
-#pragma unroll
-  for (int c = 0; c < 4; ++c)
-#pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      const int d = ds_chan<NP>(lane, i);
-      float* p = S_st + (int64_t)c * dim + d;
-      if (j0 + c >= vd || d >= dim) continue;
-      if (a.vec) {
-        *reinterpret_cast<uint64_t*>(p) = S[c][i];
-      } else {
-        p[0] = f2::lo(S[c][i]);
-        if (d + 1 < dim) p[1] = f2::hi(S[c][i]);
-      }
-    }
+  ds_store<NP>(S_st, dim, vd - j0, a.vec, lane, S);
 }
 
 }  // namespace
@@ -533,14 +572,14 @@ int delta_tails(bool f32, const void* fused, int64_t ld, const int32_t* position
 
 int delta_scan(const float* qn, const float* kn, const float* vn, const float* beta, const float* decay, const int32_t* positions,
                const int32_t* seq_start, const int32_t* seq_slots, float* state, int64_t slot_stride, float* out, int S, int heads,
-               int kv_heads, int dim, int vd, cudaStream_t s) {
+               int kv_heads, int dim, int vd, cudaStream_t s, bool single_rows) {
   return linear_scan(true, qn, kn, vn, beta, decay, (int64_t)heads * dim, dim, 1, positions, seq_start, seq_slots, state, slot_stride, out, S,
-                     heads, kv_heads, dim, vd, s);
+                     heads, kv_heads, dim, vd, s, single_rows);
 }
 
 int linear_scan(bool delta_rule, const float* qn, const float* kn, const float* vn, const float* beta, const float* decay, int64_t g_row,
                 int g_head, int g_chan, const int32_t* positions, const int32_t* seq_start, const int32_t* seq_slots, float* state,
-                int64_t slot_stride, float* out, int S, int heads, int kv_heads, int dim, int vd, cudaStream_t s) {
+                int64_t slot_stride, float* out, int S, int heads, int kv_heads, int dim, int vd, cudaStream_t s, bool single_rows) {
   if (S == 0) return B200_OK;
   B200_REQUIRE(dim > 0 && dim <= 256 && vd > 0, B200_ERR_UNSUPPORTED, "delta_scan: key size %d outside (0, 256]", dim);
   B200_REQUIRE(heads > 0 && kv_heads > 0 && heads % kv_heads == 0, B200_ERR_INVALID, "delta_scan: %d heads over %d", heads, kv_heads);
@@ -556,6 +595,10 @@ int linear_scan(bool delta_rule, const float* qn, const float* kn, const float* 
   do {                                                                                                        \
     static bool done[64] = {};                                                                                \
     const size_t smem = (size_t)ds_floats(D, CH) * 4;                                                         \
+    if (single_rows) {                                                                                        \
+      B200_CUDA(launch(delta_rows_kernel<D, R, CH>, grid, block, (size_t)0, s, a));                           \
+      break;                                                                                                  \
+    }                                                                                                         \
     if (smem > 48 * 1024) B200_CUDA(ensure_dynamic_smem(delta_scan_kernel<D, R, CH>, (int)smem, done));       \
     B200_CUDA(launch(delta_scan_kernel<D, R, CH>, grid, block, smem, s, a));                                  \
   } while (0)
