@@ -134,6 +134,47 @@ def test_mlstm_chunks_are_causal_for_what_is_not_finite(what, bad, row):
     assert (st[0] - S[0]).norm() < 1e-5 * S[0].norm()
 
 
+# Steps whose CTAs outnumber the SMs: two sequences of 8 heads of 256 columns (256 CTAs, two to an SM, short portions walked beside the chunks),
+# four (512 CTAs: chunks and walk in a launch each, whole portions on both sides of 97 rows), five (the walk alone); the second step
+# starts from the state the first one left.
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("steps", [([130, 30], [20, 97]), ([97, 96, 5, 161], [64, 1, 100, 98]), ([30, 1, 17, 100, 2], [1, 1, 1, 1, 1])])
+def test_mlstm_scan_of_many_ctas(dim, steps):
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    heads, vdim, S = 8, 256, len(steps[0])
+    g = torch.Generator().manual_seed(dim + S)
+    hd, hv, nz = heads * dim, heads * vdim, vdim // 32
+    floats, ld = int(lib.b200_mlstm_state_floats(heads, dim, vdim)), 2 * hd + hv
+    state = torch.full((S + 1, floats), 7.5, device=DEV)
+    slots, pos = [S - s for s in range(S)], [0] * S
+    oracle = [tuple(torch.zeros(s, dtype=torch.float64) for s in ((heads, vdim, dim), (heads, dim), (heads,))) for _ in range(S)]
+    for cuts in steps:
+        T = sum(cuts)
+        x, gates = torch.randn(T, ld, generator=g).to(torch.bfloat16), torch.randn(T, 2 * heads, generator=g)
+        gates[:, heads:] = torch.nn.functional.logsigmoid(gates[:, heads:] + 3)
+        start = [0]
+        for n in cuts:
+            start.append(start[-1] + n)
+        out = torch.full((T, hv), float("nan"), device=DEV)
+        xd, gd = x.to(DEV), gates.to(DEV)
+        ptd, std, sld = _i32([pos[s] + i for s in range(S) for i in range(cuts[s])]), _i32(start), _i32(slots)
+        check(lib.b200_mlstm_scan(0, xd.data_ptr(), ld, 0, hd, 2 * hd, gd.data_ptr(), ptd.data_ptr(), std.data_ptr(), sld.data_ptr(), state.data_ptr(), floats,
+                                  out.data_ptr(), S, heads, dim, vdim, None))
+        torch.cuda.synchronize()
+        for s in range(S):
+            lo, hi = start[s], start[s + 1]
+            want, span, oracle[s] = _mlstm(x[lo:hi].double(), gates[lo:hi].double(), oracle[s], heads, dim, vdim)
+            got, tol = out[lo:hi].double().cpu(), 1e-5     # (as above)
+            assert ((got - want).abs() <= tol * span + 1e-7 * want.abs()).all(), (cuts, s, float(((got - want).abs() / span).max()))
+            st = state[slots[s]].double().cpu()
+            assert (st[:hv * dim].reshape(heads, vdim, dim) - oracle[s][0]).norm() < tol * oracle[s][0].norm()
+            n = st[hv * dim:hv * dim + heads * nz * dim].reshape(heads, nz, dim)
+            assert (n - oracle[s][1][:, None]).norm() < tol * nz ** 0.5 * oracle[s][1].norm()
+            assert (st[hv * dim + heads * nz * dim:].reshape(heads, nz) - oracle[s][2][:, None]).abs().max() < 1e-5
+            pos[s] += cuts[s]
+    assert (state[0] == 7.5).all()
+
+
 # channel decays / one per head, delta rule / plain, heads sharing keys, sizes that leave lanes and columns idle; strided decays (g_chan 2);
 # zero decays forget everything, as do rows of zeros; rows that are not 16-byte aligned
 @pytest.mark.parametrize("rule", ["channel", "head", "plain", "plain channel", "strided"])
