@@ -18,8 +18,6 @@
 // Queries come as fp32 rows [T][heads][krow] (rounded to bf16 when staged); output rows are bf16 [T][heads][rank].
 // Shapes: krow and rank multiples of 16, rank <= 512.  Everything else (and the 32-bit mode) takes attn_anydim.cu; both walk
 // the same cache and the same run list, and agree within bf16 rounding of the operands.
-#include <stdlib.h>
-
 #include <algorithm>
 
 #include "runs.cuh"

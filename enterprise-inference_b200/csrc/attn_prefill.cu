@@ -5,13 +5,11 @@
 // softmax instructions per (tile, column).  Rows of a chunk go to attn_rows_tc.cu instead, whose MMA rows are (row, head) pairs of one
 // kv head; weights reach the second product as hi + lo bf16 (the CPU oracle keeps them in fp32).
 //
-// Rows come in any mix (chunked prefill + decode rows in one step): a one-warp plan kernel cuts the step's rows into items (maximal
+// Rows come in any mix (chunked prefill + decode rows in one step): a plan kernel of one CTA cuts the step's rows into items (maximal
 // runs of one sequence, at most as many rows as fill two tiles of 128 pairs); a decode row becomes an item with one live row.
 //
 // Replaces: the prefill half of the vLLM-CPU attention backend ([V22] vllm/v1/attention/backends/
 // cpu_attn.py:377-396); chunked prefill is selected by the chart (xeon-values.yaml:80-83).
-#include <stdlib.h>
-
 #include "common.cuh"
 
 namespace b200 {

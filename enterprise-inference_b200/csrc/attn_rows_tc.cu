@@ -5,17 +5,16 @@
 //   S_x[128][64] = Q_x . K_tile^T        O_x[128][vdim] += P_x . V_tile           x = the item's first, second tile of pairs
 // The scores of key tile n + 1 are issued before the weights of tile n are waited for (two score buffers per tile of pairs), so the
 // softmax of either tile never waits for the tensor core once the walk is under way: with one tile of pairs and 128 keys (the kernel
-// this one replaces) S -> softmax -> P V was one dependent chain of 1.85 us, and two tiles of pairs with single score buffers of 128
-// keys still took 3.3 us per 128 keys, a tile's softmax (1.7 us) and its own products (1.05 us) one after the other.
-// The weights overwrite the scores in TMEM (A operand of the second product): per 32 scores 16 columns of bf16 pairs and, HILO, 16 more
-// with what rounding took from them (P then has 16 bits, as attn_tc.cu has it).  TMEM per tile of pairs: two score buffers of 64
+// this one replaces) S -> softmax -> P V was one dependent chain of 1.85 us (2 048 rows 212 us), and with two tiles of pairs but single score
+// buffers of 128 keys a tile's softmax and its own products still came one after the other (177 us; two buffers of 64 keys 118).
+// The weights overwrite the scores in TMEM (A operand of the second product): per 32 scores 16 columns of bf16 pairs and 16 more with what
+// rounding took from them (P has 16 bits, as attn_tc.cu has it).  TMEM per tile of pairs: two score buffers of 64
 // columns, O 128.
 // Scores may be capped, biased by distance (each score takes its own distance's bias and no other: tables may end in -inf or any sentinel),
-// windowed with kept first keys (EX); outputs may have a sink in the denominator and a gate
-// per head.  The running maximum is only followed when it rises by more than 2^8 (exact: all terms are scaled alike); a warp then
+// windowed with kept first keys (EX); outputs may have a sink in the denominator and a gate per head.  The running maximum is only followed when it rises by more than 2^8 (exact: all terms are scaled alike); a warp then
 // rescales its 32 rows of O in TMEM.
-// Bound by the tensor core (HILO) or the softmax's issue slots: 2 048 rows at contexts 1001..3048, 32 heads over 8: 118 us (212 us); 1 900
-// rows of three sequences, 16 heads over 4, capped, biased, window 1024: 74 us (278 us on the mma.sync kernel of attn_latent.cu).
+// Bound by the tensor core or the softmax's issue slots: 2 048 rows at contexts 1001..3048, 32 heads over 8: 118 us (212 us); 1 900
+// rows of three sequences, 16 heads over 4, capped, biased, window 1024: 76 us (278 us on the mma.sync kernel of attn_latent.cu).
 // Warps: four softmax warps per tile (a thread owns a pair), TMA, MMA, two that stage queries.  Every wait is bounded and
 // reported (tc.cuh).
 #include <algorithm>
@@ -112,7 +111,7 @@ template <> __device__ __forceinline__ uint4 ar_q8<float>(const float* p) {
   return make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
 }
 
-template <typename QT, bool HILO, bool EX>
+template <typename QT, bool EX>
 __global__ void __launch_bounds__(kArThreads, 1)
 attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const RowsParams p) {
   constexpr int kArSlots = ar_slots(EX);
@@ -329,7 +328,7 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
 #pragma unroll
           for (int j = 0; j < 4; ++j) {   // 16 keys per step: 8 columns of weights, 16 further those of the second term
             mma_ts(one, d, pa + (j >> 1) * 32 + (j & 1) * 8, dv + (uint64_t)((j * 2048) >> 4), id_o, (i | j) ? 1u : 0u);
-            if (HILO) mma_ts(one, d, pa + (j >> 1) * 32 + (j & 1) * 8 + 16, dv + (uint64_t)((j * 2048) >> 4), id_o, 1u);
+            mma_ts(one, d, pa + (j >> 1) * 32 + (j & 1) * 8 + 16, dv + (uint64_t)((j * 2048) >> 4), id_o, 1u);
           }
           if (x == tiles - 1) commit(one, kv_free + v_slot);
           commit(one, o_full + 2 * x + (n[x] & 1));
@@ -477,18 +476,13 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
           for (int j = 0; j < 16; ++j) {
             const float s0 = __uint_as_float(s[c * 32 + 2 * j]), s1 = __uint_as_float(s[c * 32 + 2 * j + 1]);
             const float p0 = exp2_fast(EX ? s0 - mref : fmaf(s0, sc2, -mref)), p1 = exp2_fast(EX ? s1 - mref : fmaf(s1, sc2, -mref));
-            if constexpr (HILO) {   // the high term truncated, the rest rounded
-              sum[j & 1] += p0 + p1;
-              const uint32_t h0 = __float_as_uint(p0) & 0xffff0000u, h1 = __float_as_uint(p1) & 0xffff0000u;
-              pk[j] = __byte_perm(h0, h1, 0x7632);
-              pk[16 + j] = pack_bf16(p0 - __uint_as_float(h0), p1 - __uint_as_float(h1));
-            } else {
-              pk[j] = pack_bf16(p0, p1);
-              sum[j & 1] += bf16lo(pk[j]) + bf16hi(pk[j]);   // the weights as the second product takes them
-            }
+            // the high term truncated, the rest rounded
+            sum[j & 1] += p0 + p1;
+            const uint32_t h0 = __float_as_uint(p0) & 0xffff0000u, h1 = __float_as_uint(p1) & 0xffff0000u;
+            pk[j] = __byte_perm(h0, h1, 0x7632);
+            pk[16 + j] = pack_bf16(p0 - __uint_as_float(h0), p1 - __uint_as_float(h1));
           }
-          if constexpr (HILO) st32(s_addr + c * 32, pk);
-          else st16(s_addr + c * 32, pk);
+          st32(s_addr + c * 32, pk);
         }
         l += sum[0] + sum[1];
         if (x == 0) {
@@ -582,13 +576,13 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
   }
 }
 
-template <typename QT, bool HILO, bool EX>
+template <typename QT, bool EX>
 int ar_launch(const CUtensorMap& mk, const CUtensorMap& mv, const RowsParams& p, int T, cudaStream_t s) {
   if (const int e = wait_status()) return e;
   static bool done[64] = {};
-  B200_CUDA(ensure_dynamic_smem(attn_rows_tc_kernel<QT, HILO, EX>, kArSmem, done));
+  B200_CUDA(ensure_dynamic_smem(attn_rows_tc_kernel<QT, EX>, kArSmem, done));
   const int64_t most = (int64_t)T * p.kv_heads * p.n_splits;   // upper bound; the kernel reads the real count
-  B200_CUDA(launch(attn_rows_tc_kernel<QT, HILO, EX>, dim3((unsigned)std::min<int64_t>(most, kNumSMs)), dim3(kArThreads), (size_t)kArSmem, s, mk, mv, p));
+  B200_CUDA(launch(attn_rows_tc_kernel<QT, EX>, dim3((unsigned)std::min<int64_t>(most, kNumSMs)), dim3(kArThreads), (size_t)kArSmem, s, mk, mv, p));
   return B200_OK;
 }
 
@@ -632,7 +626,7 @@ int attn_rows_tc_plan(const __nv_bfloat16* q, int64_t ldq, const __nv_bfloat16* 
   p.status = wait_status_word();
   p.tile_rows = 128 / (heads / kv_heads);
   p.scale = scale;
-  return ar_launch<__nv_bfloat16, true, false>(mk, mv, p, T, s);
+  return ar_launch<__nv_bfloat16, false>(mk, mv, p, T, s);
 }
 
 // fp32 queries [T][heads][dim], weights of 16 bits; runs, n_runs: the first of the lists that paged_attn_runs_plan leaves for T rows.  Launched
@@ -680,7 +674,7 @@ int attn_rows_tc_runs(const float* q, const __nv_bfloat16* kc, const __nv_bfloat
   *share = p.share = {p.n_runs, const_cast<int32_t*>(n_runs) + kRunTicket, T, kv_heads * n_splits, p.parts};
   p.scale = scale;
   p.ex = ex;
-  return ex.any() ? ar_launch<float, true, true>(mk, mv, p, T, s) : ar_launch<float, true, false>(mk, mv, p, T, s);
+  return ex.any() ? ar_launch<float, true>(mk, mv, p, T, s) : ar_launch<float, false>(mk, mv, p, T, s);
 }
 
 }  // namespace b200

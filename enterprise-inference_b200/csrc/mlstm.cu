@@ -214,10 +214,10 @@ int mlstm_scan(bool f32, const void* qkv, int64_t ld, int q_off, int k_off, int 
   B200_REQUIRE(positions && seq_start && seq_slots && state, B200_ERR_INVALID, "mlstm_scan: null argument");
   MlstmArgs a = {qkv, gates, positions, seq_start, seq_slots, state, out, ld, slot_stride, q_off, k_off, v_off, heads, dim, vd, 1.0f / sqrtf((float)dim), 0, 0, 0};
   mlstm_walk_widths(a, f32);
-  // Steps of a few bf16 portions in chunks on the tensor cores where they are long (2 048 rows of 8 heads, 128 x 256: 140 us; the scalar walk
+  // Steps of a few bf16 portions in chunks on the tensor cores where they are long (2 048 rows of 8 heads, 128 x 256: 144 us; the scalar walk
   // before it 724).  While all CTAs fit the device at once (two an SM), the chunk kernel walks the short portions itself; beyond that each
   // kernel takes its portions (64 rows of four sequences: 15.0 us, in one kernel 23.1: the idle half of each cluster holds up the next).
-  // More sequences than four are mostly decode rows, and the walk alone is the faster the more there are.
+  // More sequences than four go to the walk alone (64 of one row 36 us; longer portions of many sequences in chunks have not been measured).
   if (!f32 && !single_rows && S <= 4 && mlstm_chunk_supported(a)) {
     a.both = (int64_t)S * heads * 2 * mlstm_col_blocks(vd) > 2 * kNumSMs;
     if (const int e = mlstm_chunk(a, S, s)) return e;

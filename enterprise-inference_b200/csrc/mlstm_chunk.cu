@@ -12,7 +12,7 @@
 // Warps w of 8: rows 16 (w % 4) of P and O, the key blocks (and for Q S_0 the dimensions) dealt to the two warps of a row group, whose
 // sums meet in shared memory; dimensions 16 w of the state, kept in fp32 accumulator fragments.  A ninth warp works out the next
 // chunk's gate scalars.  Rows arrive by cp.async a chunk ahead.
-// Bound by latency (about 800 instructions a warp and chunk, two barriers).  2 048 rows of 8 heads, 128 x 256: 140 us against 724 us
+// Bound by latency (about 800 instructions a warp and chunk, two barriers).  2 048 rows of 8 heads, 128 x 256: 144 us against 724 us
 // of the scalar walk; error of the results against 64 bits 6.8e-7 (walk 1.2e-6), of the state 7.5e-8 (1.5e-7).
 #include <algorithm>
 
