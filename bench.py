@@ -4,10 +4,10 @@
     python bench.py [--gpus N] [--steps K] [--warmup W] [--workload NAME] [--impl b200|reference]
 
 A "step" is one scheduler iteration of the decode path over one batch of sequences (every
-sequence emits one token).  Default workload = BASELINE.json configs[1]: Llama-3.1-8B-Instruct
+sequence emits one token).  Default workload: Llama-3.1-8B-Instruct
 bf16, continuous batch of 64 requests, 512-token prompts / 256 output tokens, random-init weights,
-synthetic prompt KV (prefill flops are not part of the decode metric, SURVEY.md §8d).  8B fits one
-GPU and does not shard (SURVEY.md §8e "replicas only"), so the headline of --gpus N is N independent
+synthetic prompt KV (prefill flops are not part of the decode metric).  8B fits one
+GPU and does not shard, so the headline of --gpus N is N independent
 replicas (weak scaling, no data-path collective).
 
 Printed line (rank 0): metric/value/unit per the driver contract plus
@@ -15,8 +15,8 @@ Printed line (rank 0): metric/value/unit per the driver contract plus
   cpu_baseline  the oracle (CPU port of the reference image's algorithm) timed on this host
   e2e           same metric through the engine API with pinned HOST buffers (every step: H2D of its metadata, the
                 step, D2H of its tokens; the engine enqueues step n+1 before it reads step n, engine.py)
-  also          (default workload, N = 1) the other single-GPU configs of BASELINE.json, a few dozen steps each:
-                8B batch 1 (configs[0], the north_star target) and 8B batch 8 at 32 k context
+  also          (default workload, N = 1) other single-GPU workloads, a few dozen steps each:
+                8B batch 1 and 8B batch 8 at 32 k context
   tp            (default workload) the tensor-parallel path at TP = N: a parity check of the sharded step against
                 the committed oracle fixture (peer-memory and NCCL all-reduce), then Llama-3.1-70B decode at
                 batch 64 and batch 1 with the all-reduce timed on its own; at N = 1 that is 70B on one GPU

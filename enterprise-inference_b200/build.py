@@ -3,7 +3,7 @@
     python enterprise-inference_b200/build.py [--force] [--verbose]
 
 The .so is written next to this file under lib/ so that it travels to the GPU box with the
-gpurun snapshot (built artefacts are git-ignored, not gpurun-ignored).
+tree (built artefacts are git-ignored).
 """
 from __future__ import annotations
 

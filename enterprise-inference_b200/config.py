@@ -1,6 +1,6 @@
-"""Model shapes (SURVEY.md §8 shape table) and the RoPE cache, product side.
+"""Model shapes and the RoPE cache, product side.
 
-The reference names models only by HF id (/root/reference/core/helm-charts/vllm/xeon-values.yaml:61,124;
+The reference names models only by HF id (core/helm-charts/vllm/xeon-values.yaml:61,124;
 gaudi-values.yaml:165); the shapes are the public HF configs of those ids.
 """
 from __future__ import annotations

@@ -1,10 +1,10 @@
 """Host-side engine: KV block manager + continuous-batching scheduler with chunked prefill.
 
 Mirrors the scheduler of the image the chart deploys, as parameterised by the chart's flags
-(/root/reference/core/helm-charts/vllm/xeon-values.yaml:70-89): --block-size 128,
+(core/helm-charts/vllm/xeon-values.yaml:70-89): --block-size 128,
 --max-num-batched-tokens 2048 (token budget of one step), --max-num-seqs 256,
 --enable_chunked_prefill, --max-model-len 8192.  Greedy only on the device
-(clients send "temperature": 0, /root/reference/docs/accessing-deployed-models.md:176).
+(clients send "temperature": 0, docs/accessing-deployed-models.md:176).
 Pure host logic: unit-tested on CPU with a fake runner.
 """
 from __future__ import annotations

@@ -1,7 +1,7 @@
 """Device state of one TP rank and one scheduler step through the C-ABI.
 
 Mirrors the worker/model-runner of the image the chart deploys (one worker process per TP rank,
-/root/reference/core/helm-charts/vllm/xeon-values.yaml:78-79; [V22] vllm/v1/worker/*model_runner*):
+core/helm-charts/vllm/xeon-values.yaml:78-79; [V22] vllm/v1/worker/*model_runner*):
 it owns the weights, the paged KV cache and the step inputs, and runs `execute_model` — here
 `b200_decode_step_host` — once per scheduler iteration.  torch allocates; CUDA computes.
 """
@@ -22,7 +22,7 @@ from .config import ModelConfig, rope_cos_sin
 
 @dataclass
 class StepBatch:
-    """Step inputs (SURVEY.md §8 a0).  One entry per token row; block_tables one row per sequence."""
+    """Step inputs.  One entry per token row; block_tables one row per sequence."""
     ids: List[int] = field(default_factory=list)
     positions: List[int] = field(default_factory=list)
     slots: List[int] = field(default_factory=list)

@@ -3,8 +3,8 @@
     python -m enterprise-inference_b200.server --model <hf id> --served-model-name <name> --port 2080 \
         --block-size 128 --dtype bfloat16 --max-model-len 8192 --tensor-parallel-size 1 ...
 
-What the chart passes (must accept; may no-op): /root/reference/core/helm-charts/vllm/xeon-values.yaml:70-89
-and templates/deployment.yaml:66-87.  HTTP surface: /root/reference/docs/api-spec.yaml (POST
+What the chart passes (must accept; may no-op): core/helm-charts/vllm/xeon-values.yaml:70-89
+and templates/deployment.yaml:66-87.  HTTP surface: docs/api-spec.yaml (POST
 /v1/completions, /v1/chat/completions; 422 on a bad body, additionalProperties: false), GET /health
 (values.yaml:135-141), GET /metrics with the vllm:* series the Grafana dashboard queries
 (observability/xeon-exporter/grafana-xeon-dashboard.json), GET /v1/models (docs/getting-started-example.md:79-81).

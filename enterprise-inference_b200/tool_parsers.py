@@ -1,5 +1,5 @@
 """Tool-call parsers for /v1/chat/completions, selected by the chart's `--enable-auto-tool-choice
---tool-call-parser llama3_json|hermes` (/root/reference/core/helm-charts/vllm/xeon-values.yaml:87-88,118-119,209-210).
+--tool-call-parser llama3_json|hermes` (core/helm-charts/vllm/xeon-values.yaml:87-88,118-119,209-210).
 
 llama3_json: the assistant turn is a JSON object (or several separated by ';')
              {"name": "<fn>", "parameters": {...}}   (also accepts "arguments")

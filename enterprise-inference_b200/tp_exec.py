@@ -1,5 +1,5 @@
 """Tensor-parallel execution for the server: one process per GPU (the chart's
-`--distributed_executor_backend mp`, /root/reference/core/helm-charts/vllm/xeon-values.yaml:78-79).
+`--distributed_executor_backend mp`, core/helm-charts/vllm/xeon-values.yaml:78-79).
 
 Rank 0 owns the scheduler and the HTTP front end.  Every scheduler iteration it packs the step inputs
 into its pinned buffer and broadcasts them (header + int32 payload, gloo) to the worker ranks, which run

@@ -1,10 +1,10 @@
 """Host-side weight plumbing: HF names -> fused, per-rank shards (pure torch, no CUDA needed).
 
 Packing follows [V22] vllm/model_executor/models/llama.py:437-444 (q|k|v -> qkv_proj, gate|up ->
-gate_up_proj); sharding is Megatron-style as in SURVEY.md §8e: QKV and gate_up column-parallel (by
+gate_up_proj); sharding is Megatron-style: QKV and gate_up column-parallel (by
 head / by intermediate feature), O and down row-parallel, lm_head vocab-parallel, embedding and norms
 replicated.  Weights come from the HF cache the chart mounts at /data
-(/root/reference/core/helm-charts/vllm/templates/configmap.yaml:18-21).
+(core/helm-charts/vllm/templates/configmap.yaml:18-21).
 """
 from __future__ import annotations
 

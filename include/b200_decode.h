@@ -3,10 +3,10 @@
  *
  * The reference (psurabh/Enterprise-Inference v1.3.0) has NO in-process FFI for this path:
  * its boundary is the container contract of core/helm-charts/vllm (image + args + env + HTTP,
- * /root/reference/core/helm-charts/vllm/templates/deployment.yaml:57,66-87 and
- * /root/reference/docs/api-spec.yaml:6-49).  The arithmetic runs inside the third-party
+ * core/helm-charts/vllm/templates/deployment.yaml:57,66-87 and
+ * docs/api-spec.yaml:6-49).  The arithmetic runs inside the third-party
  * image vllm-cpu-release-repo:v0.10.2 (values.yaml:23-28).  Each entry point below therefore
- * cites the step of that image's decode loop it replaces (SURVEY.md §8a rows a0..a12; the
+ * cites the step of that image's decode loop it replaces (the
  * [V22] citations are the vLLM 0.22 wheel used as the readable statement of the math).
  *
  * Conventions
@@ -102,7 +102,7 @@ B200_API int b200_set_kv_cache(b200_ctx* ctx, void* k_cache, void* v_cache, int6
 /* cos|sin cache [max_pos][head_dim] bf16 ([V22] rotary_embedding/base.py:58-63,82-92). */
 B200_API int b200_set_rope_cache(b200_ctx* ctx, const void* cos_sin, int64_t max_pos);
 
-/* NCCL communicator for TP (SURVEY.md §8 a11; replaces the image's shm all-reduce,
+/* NCCL communicator for TP (replaces the image's shm all-reduce,
  * [V22] vllm/distributed/device_communicators/cpu_communicator.py:229-276).
  * b200_nccl_unique_id writes 128 bytes to host_id (rank 0 calls it and shares the bytes);
  * b200_nccl_init is collective over the tp_world ranks of the ctx. */
@@ -116,7 +116,7 @@ B200_API int b200_nccl_init(b200_ctx* ctx, const void* host_id128);
 B200_API int b200_tp_ipc_export(b200_ctx* ctx, void* host_handle64);
 B200_API int b200_tp_ipc_import(b200_ctx* ctx, const void* host_handles, int32_t world);
 
-/* ---- the hot path: one scheduler step (SURVEY.md §8 a0..a10) ----------------------------
+/* ---- the hot path: one scheduler step ----------------------------
  * Replaces ModelRunner.execute_model of the image for one batch of token rows
  * ([V22] vllm/model_executor/models/llama.py:395-434 + sampler.py:235-236).
  * Row t is one new token: ids[t], positions[t], slot_mapping[t] = block_id*block_size+off,

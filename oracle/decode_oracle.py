@@ -6,10 +6,10 @@ sampling_masks.npz, captured from the `vllm` package by tools/make_vllm_op_golde
 No output of the v0.10.2 CPU image itself is available, so whole-model parity stays unpinned.)  The reference (psurabh/Enterprise-Inference v1.3.0) holds no source
 for this path: its chart only names the third-party image
 ``public.ecr.aws/q9t5s3a7/vllm-cpu-release-repo:v0.10.2``
-(/root/reference/core/helm-charts/vllm/values.yaml:23-28,
- /root/reference/core/helm-charts/vllm/xeon-values.yaml:29-32) and its tests/docs pin
+(core/helm-charts/vllm/values.yaml:23-28,
+ core/helm-charts/vllm/xeon-values.yaml:29-32) and its tests/docs pin
 no outputs (only ``temperature: 0`` smoke prompts whose completions are not recorded,
-/root/reference/docs/single-node-deployment.md:80-87).  The algorithm restated here is
+docs/single-node-deployment.md:80-87).  The algorithm restated here is
 the published vLLM "native" forward for Llama / Qwen2 (vLLM v0.10.2 CPU build is the
 pinned dependency; the readable copy consulted is the vLLM 0.22 wheel in this image,
 cited as [V22]).  Because no golden vector exists in the reference, this oracle is
@@ -52,7 +52,7 @@ BF16 = torch.bfloat16
 
 @dataclass
 class ModelConfig:
-    """Shape of one decoder-only Llama/Qwen2 model (SURVEY.md §8 shape table)."""
+    """Shape of one decoder-only Llama/Qwen2 model."""
     name: str = "tiny"
     hidden: int = 512
     n_layers: int = 2
@@ -83,7 +83,7 @@ class ModelConfig:
         return self.n_kv_heads * self.head_dim
 
     def decode_params(self) -> int:
-        """P_dec of SURVEY.md §8: parameters streamed once per decode step."""
+        """P_dec: parameters streamed once per decode step."""
         h, L, I, V = self.hidden, self.n_layers, self.intermediate, self.vocab
         return L * (h * (self.q_size + 2 * self.kv_size) + self.q_size * h + 3 * h * I) + V * h
 
@@ -163,8 +163,8 @@ def weight_shape(cfg: ModelConfig, name: str):
 
 def make_weights(cfg: ModelConfig, seed: int = 1234, norm_jitter: float = 0.0,
                  std: float = 0.02) -> Dict[str, torch.Tensor]:
-    """Seeded N(0, std^2) bf16 weights, one torch.Generator stream in name order
-    (SURVEY.md §8d).  Norm weights are 1 (+ N(0,norm_jitter^2) when asked, so that the
+    """Seeded N(0, std^2) bf16 weights, one torch.Generator stream in name order.
+    Norm weights are 1 (+ N(0,norm_jitter^2) when asked, so that the
     bf16 weight multiply of R1 is exercised)."""
     g = torch.Generator(device="cpu")
     g.manual_seed(seed)
@@ -193,7 +193,7 @@ def weights_digest(w: Dict[str, torch.Tensor]) -> str:
 
 
 def make_prompt(cfg: ModelConfig, request_index: int, length: int) -> List[int]:
-    """Uniform token ids, seed = 1000 + request index (SURVEY.md §8d)."""
+    """Uniform token ids, seed = 1000 + request index."""
     g = torch.Generator(device="cpu")
     g.manual_seed(1000 + request_index)
     return torch.randint(0, cfg.vocab, (length,), generator=g).tolist()
@@ -477,7 +477,7 @@ class OracleModel:
         return logits
 
     def generate(self, prompt: List[int], n_new: int, keep_logits: bool = False):
-        """Greedy, ignore_eos: exactly n_new tokens (SURVEY.md §8d)."""
+        """Greedy, ignore_eos: exactly n_new tokens."""
         st = self.new_seq()
         logits = self.forward(st, prompt)[-1:]
         toks, all_logits = [], []

@@ -1,7 +1,7 @@
 """Generate tests/golden/*.npz: frozen oracle outputs + the HuggingFace cross-check.
 
 Run here (CPU):  python oracle/make_golden.py
-The reference has no golden vectors for this path ("parity unpinned");
+The reference has no golden vectors for this path;
 these fixtures freeze (a) this repo's oracle and (b) HF transformers 5.5.0 on the same
 seeded weights, as the closest executable stand-in for the vLLM-CPU image.
 """
@@ -75,7 +75,7 @@ def main():
         agree = (tf_logits.argmax(-1) == hf_logits.argmax(-1)).float().mean().item()
         print(f"{name}: oracle-vs-HF softmax max abs err {err:.3e}; greedy agreement {agree:.3f}; "
               f"logit max abs diff {(tf_logits - hf_logits).abs().max():.3e}")
-        assert err <= 2e-2, "oracle disagrees with the HF stand-in beyond the north_star tolerance"
+        assert err <= 2e-2, "oracle disagrees with the HF stand-in beyond the tolerance"
         np.savez_compressed(
             os.path.join(OUT, f"{name}.npz"),
             cfg=np.array(repr(cfg.to_dict())), seed=1234, norm_jitter=0.1,

@@ -1,6 +1,6 @@
 """Writes a small HF-style checkpoint into an HF_HOME hub layout: sharded safetensors + index, config.json with a
 llama3 rope_scaling block, a real `tokenizers` tokenizer with a chat template, generation_config.json — what the chart
-mounts at /data (/root/reference/core/helm-charts/vllm/templates/configmap.yaml:18-21) for `--model <hf id>`."""
+mounts at /data (core/helm-charts/vllm/templates/configmap.yaml:18-21) for `--model <hf id>`."""
 import json
 import os
 

@@ -1,5 +1,5 @@
-"""CPU: the real-checkpoint path of the server (SURVEY.md §8 f4) — `--model <hf id>` resolved in the HF_HOME cache the
-chart mounts at /data (/root/reference/core/helm-charts/vllm/templates/configmap.yaml:18-21), sharded safetensors, HF
+"""CPU: the real-checkpoint path of the server — `--model <hf id>` resolved in the HF_HOME cache the
+chart mounts at /data (core/helm-charts/vllm/templates/configmap.yaml:18-21), sharded safetensors, HF
 tokenizer + chat template (xeon-values.yaml:87-88), generation_config.json defaults — booted through build_engine /
 create_app with a fake runner in place of the device."""
 import json

@@ -152,7 +152,7 @@ def test_abort_returns_blocks_and_row_wherever_the_request_is():
 
 
 def test_a_request_that_can_never_be_admitted_fails_alone():
-    """with nothing running and the head of the queue too big for the free blocks the scheduler used to
+    """With nothing running and the head of the queue too big for the free blocks the scheduler used to
     return [] forever (has_work() stayed true: a busy spin).  Now add() rejects what can never fit, and a request that
     stops fitting is failed by itself while the others go on."""
     fr = FakeRunner(n_blocks=5, block_size=4, max_tokens=16, max_model_len=64)

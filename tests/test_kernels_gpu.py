@@ -120,7 +120,7 @@ def test_linear_tcgen05(lib, abi, T, n_out, k, bias):
 
 def test_linear_global_split_k_path_in_a_fresh_process():
     """B200_TC_CLUSTER=0 (read once per process) keeps the split-K partials in the global workspace with a last-CTA
-    ticket instead of reducing through DSMEM inside a cluster: the A/B path of DESIGN.md §4, kept correct by this run of
+    ticket instead of reducing through DSMEM inside a cluster: the A/B path, kept correct by this run of
     the linear test's split shapes in a child process."""
     import subprocess, sys
     env = dict(os.environ, B200_TC_CLUSTER="0")
@@ -652,7 +652,7 @@ def test_paged_attention_vs_oracle(lib, abi, hq, hkv, ctx_lens, bs):
     got = run_attn(lib, abi, q, K, V, ctx_lens, hq, hkv, bs=bs)
     want = torch.stack([O.attend(q[t], K[t], V[t], ctx_lens[t], 128 ** -0.5) for t in range(T)])
     assert torch.isfinite(got.float()).all()
-    ulp_close(got, want, max_ulp=2, max_frac=0.02, atol_small=2 ** -8)   # measured <= 0.004 (gpurun_out/ulp_fractions.txt)
+    ulp_close(got, want, max_ulp=2, max_frac=0.02, atol_small=2 ** -8)   # measured <= 0.004
 
 
 @pytest.mark.parametrize("hq,hkv", [(4, 1), (5, 1), (16, 2), (8, 8), (2, 1)])
@@ -743,7 +743,7 @@ def test_prefill_attention_chunk_with_max_jumps(lib, abi, hq, hkv):
     got = out.cpu().view(T, hq, 128)
     want = torch.stack([O.attend(q[t], K[sq], V[sq], n, 128 ** -0.5) for t, (sq, n) in enumerate(rows)])
     assert torch.isfinite(got.float()).all()
-    ulp_close(got, want, max_ulp=2, max_frac=0.02, atol_small=2 ** -8)   # measured <= 0.004 (gpurun_out/ulp_fractions.txt)
+    ulp_close(got, want, max_ulp=2, max_frac=0.02, atol_small=2 ** -8)   # measured <= 0.004
 
 
 def test_paged_attention_split_invariance_long_context(lib, abi):

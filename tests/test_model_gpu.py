@@ -1,10 +1,10 @@
 """GPU parity of the whole decode path (C-ABI b200_decode_step / b200_decode_step_host through
 the runner and the engine) against the oracle and the frozen golden fixtures.
 
-Bars (north_star): per-step logits within bf16 tolerance — max abs error after softmax <= 2e-2,
+Bars: per-step logits within bf16 tolerance — max abs error after softmax <= 2e-2,
 here held to 2e-3 on the tiny fixtures — and greedy-token agreement, margin-aware: a mismatch is
 allowed only where the oracle's own top-1/top-2 logit margin is below MARGIN (random-init logits
-are nearly flat; SURVEY.md §7 'hard parts')."""
+are nearly flat)."""
 import numpy as np
 import pytest
 import torch
@@ -53,7 +53,7 @@ def teacher_forced_logits(r, ids, chunk=None, block_ids=None):
 def assert_logits_close(got, want, softmax_tol=2e-3):
     err = (torch.softmax(got, -1) - torch.softmax(want, -1)).abs().max().item()
     assert err <= softmax_tol, f"softmax max abs err {err:.3e}"
-    assert err <= 2e-2   # the north_star bar
+    assert err <= 2e-2   # the bar
     dis = got.argmax(-1) != want.argmax(-1)
     margins = O.top2_margin(want)
     assert (margins[dis] < MARGIN).all(), f"greedy disagreement at oracle margin {margins[dis].max():.3f}"
@@ -301,7 +301,7 @@ def test_step_argument_validation():
 
 def test_openai_server_end_to_end_on_the_gpu():
     """The chart-facing surface over the real runner: POST /v1/completions (temperature 0) returns the
-    engine's greedy tokens; /health and /metrics respond (SURVEY.md §4 smoke shapes)."""
+    engine's greedy tokens; /health and /metrics respond."""
     from fastapi.testclient import TestClient
     S, E = pkg("server"), pkg("engine")
     cfg = O.CONFIGS["tiny"]

@@ -43,7 +43,7 @@ def test_oracle_reproduces_golden(name, golden_dir):
 
 def assert_logits_close(a, b, what):
     """<= 2 bf16 ulp of the row's largest logit per element (an ulp of a small logit is far below the noise of its
-    own sum), softmax max-abs error <= 1e-3 (north_star bar: 2e-2)."""
+    own sum), softmax max-abs error <= 1e-3 (bar: 2e-2)."""
     ulp = b.abs().amax(-1, keepdim=True) * 2.0 ** -7
     worst = ((a - b).abs() / ulp).max().item()
     assert worst <= 2.0, f"{what}: logits differ from the fixture by {worst:.2f} bf16 ulp of the row maximum"
@@ -54,7 +54,7 @@ def assert_logits_close(a, b, what):
 @pytest.mark.parametrize("name", ["tiny", "tiny-qwen", "tiny-g8", "tiny-g8x8"])
 def test_golden_within_north_star_tolerance_of_hf(name, golden_dir):
     """The frozen HF (transformers 5.5.0, CPU bf16) logits bound the oracle: softmax max abs
-    error <= 2e-2 (north_star); greedy picks agree wherever the oracle's margin is not tiny."""
+    error <= 2e-2; greedy picks agree wherever the oracle's margin is not tiny."""
     g = np.load(f"{golden_dir}/{name}.npz")
     a, b = torch.from_numpy(g["tf_logits"]), torch.from_numpy(g["hf_logits"])
     assert (torch.softmax(a, -1) - torch.softmax(b, -1)).abs().max() <= 2e-2
@@ -83,7 +83,7 @@ def test_product_config_and_rope_match_oracle():
         o, p = O.CONFIGS[oname].to_dict(), C.get_config(pname).to_dict()
         o.pop("name"), p.pop("name")
         assert o == p
-    # SURVEY §8 shape table
+    # the published shapes
     assert C.get_config("llama-3.1-8b").decode_params() == 7_504_658_432
     assert C.get_config("qwen2-32b").decode_params() == 31_984_189_440
     assert C.get_config("llama-3.1-70b").decode_params() == 69_501_714_432

@@ -1,5 +1,5 @@
-"""GPU parity at the scale the numbers are quoted on (north_star: "greedy-token agreement ...
-over 256 generated tokens"; /root/reference/docs/single-node-deployment.md:80-87 is the shape of the check:
+"""GPU parity at the scale the numbers are quoted on ("greedy-token agreement ...
+over 256 generated tokens"; docs/single-node-deployment.md:80-87 is the shape of the check:
 `temperature: 0` requests).  The oracle runs live on the host cores; every test is sized to finish in a couple of minutes.
 
  (a) full-depth Llama-3.1-8B (32 layers, V 128256): 128-token prompt, 256 greedy tokens through the serving engine; the
@@ -9,7 +9,7 @@ over 256 generated tokens"; /root/reference/docs/single-node-deployment.md:80-87
  (b) ONE decode step of 64 rows at contexts 512..767 on a 2-layer full-width 8B — the BENCH shape (512 attention items,
      four rounds per persistent CTA, cluster split-K at N = 64 on all four linears) — over cache content produced by real
      prefill, against 64 oracle sequences;
- (c) the decode attention kernel alone at 8 rows x 32 k context, G = 4, 8 kv heads (BASELINE configs[2]).
+ (c) the decode attention kernel alone at 8 rows x 32 k context, G = 4, 8 kv heads.
 """
 import os
 
@@ -110,7 +110,7 @@ def test_full_depth_8b_256_greedy_tokens_vs_oracle():
            f"logits vs oracle: softmax max-abs error {float(err.max()):.2e} (mean {float(err.mean()):.2e}), largest logit "
            f"difference {float(ldiff.max()):.3f} = {float((ldiff / ulp_top).max()):.1f} bf16 ulp of the row's top logit (median "
            f"{float((ldiff / ulp_top).median()):.1f}); replay argmax != engine token at {replay_dis} step(s)")
-    assert float(err.max()) <= 2e-2, "north_star logit bar"
+    assert float(err.max()) <= 2e-2, "logit bar"
     assert float(err.max()) <= 2e-3
     # Random-init logits over 128k tokens are nearly flat: after 32 layers of bf16 roundings two correct implementations
     # differ by a few ulp of the top logit, which is also the typical top-1/top-2 margin.  So: the logit noise itself is

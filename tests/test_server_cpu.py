@@ -1,5 +1,5 @@
 """CPU: the OpenAI surface and the chart's container contract, with a fake runner behind the engine.
-Shapes of the reference's smoke checks (SURVEY.md §4): temperature-0 completions return 200 with
+Shapes of the reference's smoke checks: temperature-0 completions return 200 with
 choices[0].text; /health 200; /metrics exposes the vllm:* series; bad bodies give 422."""
 import json
 import types
@@ -201,7 +201,7 @@ def test_penalties_and_logit_bias_reach_the_device_and_are_validated(client):
 
 
 def test_seed_and_top_k_out_of_range_cannot_kill_the_engine(client):
-    """a negative or 65-bit seed / a 2^31 top_k used to raise inside the engine thread and take every
+    """A negative or 65-bit seed / a 2^31 top_k used to raise inside the engine thread and take every
     request down with it.  Negative int64 seeds are accepted (as vLLM does), absurd values get a 400, /health stays 200."""
     base = {"model": MODEL, "prompt": "hello", "max_tokens": 3, "temperature": 1.0}
     assert client.post("/v1/completions", json={**base, "seed": -7}).status_code == 200
