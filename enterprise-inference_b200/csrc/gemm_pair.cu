@@ -1,0 +1,387 @@
+// tcgen05 linear for more than 128 tokens on pairs of SMs: y[T][n_out] = x[T][k] . w[n_out][k]^T with 256 weight rows and up to 256
+// tokens a tile (tcgen05.mma.cta_group::2), and the grouped form of the same for routed experts.
+//
+// What bounds it: the tensor pipe, if the operands arrive.  A CTA by itself (gemm_tc.cu, 128 weight rows x 256 tokens) fetches 48 KiB per 64 of
+// k for 512 cycles of MMAs, 96 bytes a cycle of the 64 that an SM gets from L2.  A pair shares the token rows: each CTA fetches its own 128
+// weight rows and half of the tokens, 32 KiB for the same 512 cycles.
+//
+// A CTA pair per two SMs, persistent.  Per CTA: warp 0 fetches (TMA, six stages of 32 KiB; both CTAs' bytes complete on the leader's barrier), warp 1
+// of the leader issues the MMAs of both, eight warps turn the accumulator into the launch's output.  The 512 columns of tensor memory hold two
+// accumulators, so a tile's epilogue runs beside the next tile's MMAs; it goes through shared memory of its own, 32 tokens at a time per
+// four warps.  Launches with few tiles share a tile's k between up to four pairs of one cluster, which add up through distributed shared memory.
+//
+// Against 128 x 256 tiles of single CTAs with k split over clusters (us, before -> now): 2000 tokens, k 14336, 4096 features 179 -> 162; 2048, 4096,
+// 28672 404 -> 321; 2048, 4096, 6144 107 -> 78; 1000, 4096, 4096 62 -> 38; 300, 2048, 2048 22 -> 12; 200, 14336, 4096 50 -> 32; 130, 2048, 2048 19 -> 11.
+// 128 tokens and fewer stay on gemm_tc.cu's tiles: their launches stream W, and 148 CTAs with two of them to an SM keep more of it in flight
+// (64 tokens, 4096, 28672: 42 there, 49 here; 128, 14336, 4096: 33 and 34).
+#include <algorithm>
+
+#include "gemm_epilogue.cuh"
+#include "tc.cuh"
+
+namespace b200 {
+
+namespace {
+
+constexpr int kPairThreads = 64 + 256;
+constexpr int kPairStages = 6;
+constexpr int kPairABytes = kBlockM * kBlockK * 2;          // this CTA's weight rows of a stage; the token rows (at most 128) take as much
+constexpr int kPairStageBytes = 2 * kPairABytes;
+constexpr int kPairStgTok = 32;                             // tokens of a staged piece of the epilogue
+constexpr int kPairSplits = 4;                              // shares of k at most: clusters of eight CTAs
+constexpr int kPairStgBytes = kPairStgTok * kBlockM * 4;
+constexpr int kPairSmem = 1024 + kPairStages * kPairStageBytes + 2 * kPairStgBytes + 512;
+constexpr uint64_t kKeepNormal = 0x1000000000000000ull, kKeepLast = 0x14F0000000000000ull;
+
+__device__ __forceinline__ uint32_t smem_of(const void* p, int cta) {   // the same shared-memory address in another CTA of the cluster
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(tc::smem_u32(p)), "r"(cta));
+  return r;
+}
+__device__ __forceinline__ void pair_load(void* dst, const CUtensorMap* map, int c0, int c1, uint32_t bar, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;" ::"r"(
+          tc::smem_u32(dst)),
+      "l"(map), "r"(bar), "r"(c0), "r"(c1), "l"(policy)
+      : "memory");
+}
+__device__ __forceinline__ void pair_mma(uint32_t one, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "setp.ne.b32 q, %5, 0;\n"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+      "}\n" ::"r"(tmem_d),
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(acc), "r"(one)
+      : "memory");
+}
+// arrives at this barrier of the CTAs in `ctas` (one bit each) once the MMAs issued so far are done
+__device__ __forceinline__ void pair_commit(uint32_t one, uint64_t* bar, uint16_t ctas) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.b32 q, %1, 0;\n"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %2;\n"
+      "}\n" ::"r"(tc::smem_u32(bar)),
+      "r"(one), "h"(ctas)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,"
+      "%28,%29,%30,%31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]),
+        "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+struct PairTile {
+  int m, row0, n, expert;   // 256-row tile of W, first token row, tokens (a multiple of 32)
+};
+__device__ __forceinline__ PairTile pair_tile(const TcParams& p, int t) {
+  PairTile r;
+  if (p.pair_tile) {   // an expert's slabs follow each other: its tokens stay in L2
+    const int4 e = __ldg(p.pair_tile + 1 + t / p.pair_m);
+    r.m = t % p.pair_m;
+    r.expert = e.x;
+    r.row0 = e.y;
+    r.n = e.z;
+  } else {             // tokens fast: the tiles in flight share a few slabs and pair_group token tiles
+    const int per = p.pair_group * p.pair_m, g = t / per, gs = min(p.pair_group, p.pair_tok - g * p.pair_group), i = t - g * per;
+    r.m = i / gs;
+    r.expert = 0;
+    r.row0 = (g * p.pair_group + i % gs) * p.pair_n;
+    r.n = p.pair_n;
+  }
+  return r;
+}
+
+__device__ __forceinline__ void pair_bias(const TcParams& p, int m_tile, int r4, float (&bb)[4]) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int row = m_tile * kBlockM + r4 + e;
+    bb[e] = p.bias && row < p.n_out ? __bfloat162float(p.bias[row]) : 0.f;
+  }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kPairThreads, 1)
+linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const TcParams p, uint32_t* status) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  float* stg_all = reinterpret_cast<float*>(smem + kPairStages * kPairStageBytes);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kPairStages * kPairStageBytes + 2 * kPairStgBytes);   // the leader's: both CTAs' bytes
+  uint64_t* empty = full + kPairStages;
+  uint64_t* acc_full = empty + kPairStages;    // [2]
+  uint64_t* acc_free = acc_full + 2;           // [2] the leader's: both CTAs' epilogue warps
+  uint64_t* last = acc_free + 2;               // after a wait that ran out: the MMAs issued before
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(last + 1);
+  uint32_t* mark = tmem_slot + 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // a cluster: the CTA pairs of one tile, each with its share of k
+  const int cta = blockIdx.x % (2 * p.splits), rank = cta & 1, split = cta >> 1, lead = cta - rank;
+  const int first = blockIdx.x / (2 * p.splits), step = gridDim.x / (2 * p.splits);
+  const int kb_base = p.n_kblocks / p.splits, kb_rem = p.n_kblocks % p.splits;
+  const int kb0 = split * kb_base + min(split, kb_rem), kb1 = kb0 + kb_base + (split < kb_rem ? 1 : 0);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kPairStages; ++s) {
+      tc::mbar_init(&full[s], 1);
+      tc::mbar_init(&empty[s], 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      tc::mbar_init(&acc_full[s], 1);
+      tc::mbar_init(&acc_free[s], 16);
+    }
+    tc::mbar_init(last, 1);
+    *mark = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(tc::smem_u32(tmem_slot)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+  }
+  tc::fence_before();
+  __syncthreads();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  tc::fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const tc::Waits wait(mark, status);
+  pdl_wait();
+  pdl_launch_dependents();
+  const int tiles = (p.pair_tile ? __ldg(&p.pair_tile[0].x) : p.pair_tok) * p.pair_m;
+
+  if (warp == 0) {
+    // ===== fetch: the whole warp walks the loop, one lane issues =====
+    const bool issuer = elect_one();
+    if (issuer) {
+      asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
+      asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
+    }
+    int it = 0;
+    for (int t = first; t < tiles; t += step) {
+      const PairTile tile = pair_tile(p, t);
+      const int half = tile.n >> 1, x0 = tile.row0 + rank * half, m = 2 * tile.m + rank;
+      const int w0 = p.gu_ff ? tile.expert * 2 * p.gu_ff + m * (kBlockM / 2) : tile.expert * p.n_out + m * kBlockM;
+      const uint32_t bytes = (uint32_t)(2 * kPairABytes + tile.n * kBlockK * 2);
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        const int st = it % kPairStages;
+        if (it >= kPairStages) wait(&empty[st], (it / kPairStages - 1) & 1);
+        if (issuer) {
+          unsigned char* a = smem + st * kPairStageBytes;
+          const uint32_t bar = smem_of(&full[st], lead);
+          if (rank == 0) tc::mbar_expect_tx(&full[st], bytes);
+          if (p.gu_ff) {   // 64 gate rows, then the matching up rows
+            pair_load(a, &map_w, kb * kBlockK, w0, bar, kKeepNormal);
+            pair_load(a + kPairABytes / 2, &map_w, kb * kBlockK, w0 + p.gu_ff, bar, kKeepNormal);
+          } else {
+            pair_load(a, &map_w, kb * kBlockK, w0, bar, kKeepNormal);
+          }
+          if (p.pair_tile) {
+            for (int r = 0; r < half; r += 16) pair_load(a + kPairABytes + r * 128, &map_x, kb * kBlockK, x0 + r, bar, kKeepLast);
+          } else {
+            pair_load(a + kPairABytes, &map_x, kb * kBlockK, x0, bar, kKeepLast);
+          }
+        }
+        __syncwarp();
+        if (wait.stop()) break;
+      }
+      if (wait.stop()) break;
+    }
+    // after a wait that ran out: what has been requested lands before shared memory is given up
+    if (rank == 0 && wait.stop())
+      for (int s = 0; s < min(it, kPairStages); ++s) wait.drain(&full[s], ((it - 1 - s) / kPairStages) & 1);
+  } else if (warp == 1) {
+    // ===== the leader's MMA warp: instructions predicated to one lane in convergent code =====
+    if (rank == 0) {
+      const uint32_t one = elect_one();
+      const uint16_t both = (uint16_t)(3 << lead);
+      const uint64_t desc0 = tc::make_desc(tc::smem_u32(smem), 16, 1024);
+      int it = 0, i = 0;
+      for (int t = first; t < tiles; t += step, ++i) {
+        const PairTile tile = pair_tile(p, t);
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(tile.n >> 3) << 17) | ((uint32_t)(2 * kBlockM >> 4) << 24);
+        const uint32_t acc = tmem + (uint32_t)((i & 1) * 256);
+        if (i >= 2) wait(&acc_free[i & 1], ((i >> 1) - 1) & 1);
+        tc::fence_after();
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+          const int st = it % kPairStages;
+          wait(&full[st], (it / kPairStages) & 1);
+          tc::fence_after();
+          const uint64_t da = desc0 + (uint64_t)((st * kPairStageBytes) >> 4), db = da + (uint64_t)(kPairABytes >> 4);
+#pragma unroll
+          for (int k = 0; k < kBlockK / 16; ++k)   // 16 of k are 32 bytes inside the swizzle's span
+            pair_mma(one, acc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > kb0 || k) ? 1u : 0u);
+          pair_commit(one, &empty[st], both);
+        }
+        pair_commit(one, &acc_full[i & 1], both);
+        if (wait.stop()) break;
+      }
+      if (wait.stop()) {
+        pair_commit(one, last, both);
+        wait.drain(last, 0);
+      }
+    }
+  } else {
+    // ===== epilogue: two groups of four warps take pieces of 32 tokens in turn =====
+    const int quad = warp & 3, grp = (warp - 2) >> 2, wq = (warp - 2) & 3, srow = quad * 32 + lane, r4 = lane * 4;
+    float* stg = stg_all + grp * (kPairStgBytes / 4);
+    float* whole = reinterpret_cast<float*>(smem);   // with k split: the pair's sums of the tile, [token][128]
+    const int barrier = 1 + grp;
+    int i = 0;
+    for (int t = first; t < tiles; t += step, ++i) {
+      const PairTile tile = pair_tile(p, t);
+      const int m_tile = 2 * tile.m + rank;
+      const int n_rows = p.pair_tile ? tile.n : min(tile.n, p.T - tile.row0);
+      const bool live = (p.gu_ff ? m_tile * (kBlockM / 2) < p.gu_ff : m_tile * kBlockM < p.n_out) && !wait.marked();
+      float bb[4];
+      pair_bias(p, m_tile, r4, bb);
+      if (MODE == kRopeKv) {   // a token's cos|sin row is a dependent load: ask for the tile's rows while its MMAs run
+        const int tt = (warp - 2) * 32 + lane;
+        if (tt < n_rows) {
+          const char* row = reinterpret_cast<const char*>(p.cos_sin + (int64_t)p.positions[tile.row0 + tt] * kHeadDim);
+          asm volatile("prefetch.global.L1 [%0];" ::"l"(row));
+          asm volatile("prefetch.global.L1 [%0];" ::"l"(row + 128));
+        }
+      }
+      wait(&acc_full[i & 1], (i >> 1) & 1);
+      tc::fence_after();
+      const uint32_t taddr = tmem + (uint32_t)((i & 1) * 256) + ((uint32_t)(quad * 32) << 16);
+      for (int c = grp * kPairStgTok; c < tile.n; c += 2 * kPairStgTok) {
+        int pair = -1;   // kScatter: lane l holds the destination and weight of the piece's token l
+        float wt = 1.0f;
+        if (MODE == kScatter && c + lane < n_rows) {
+          pair = p.grp_pair ? __ldg(p.grp_pair + tile.row0 + c + lane) : tile.row0 + c + lane;
+          if (pair >= 0 && p.grp_wt) wt = __ldg(p.grp_wt + pair);
+        }
+        uint32_t r[32];
+        tmem_ld32(taddr + c, r);
+        if (p.splits > 1) {   // one tile a pair: its stages are free by now
+#pragma unroll
+          for (int j = 0; j < 32; ++j) whole[(c + j) * kBlockM + srow] = __uint_as_float(r[j]);
+          continue;
+        }
+#pragma unroll
+        for (int j = 0; j < 32; ++j) stg[j * kBlockM + srow] = __uint_as_float(r[j]);
+        asm volatile("bar.sync %0, 128;" ::"r"(barrier) : "memory");
+        if (live) {
+#pragma unroll 4
+          for (int j = wq; j < kPairStgTok; j += 4) {
+            if (c + j >= n_rows) break;   // warp-uniform
+            const float4 a = *reinterpret_cast<const float4*>(stg + j * kBlockM + r4);
+            if constexpr (MODE == kScatter)
+              finalize4<MODE>(p, m_tile, lane, tile.row0 + c + j, a, bb, __shfl_sync(0xffffffffu, pair, j), __shfl_sync(0xffffffffu, wt, j));
+            else
+              finalize4<MODE>(p, m_tile, lane, tile.row0 + c + j, a, bb);
+          }
+        }
+        asm volatile("bar.sync %0, 128;" ::"r"(barrier) : "memory");
+      }
+      tc::fence_before();
+      __syncwarp();
+      if (lane == 0)
+        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(smem_of(&acc_free[i & 1], lead)) : "memory");
+    }
+  }
+  if (p.splits > 1) {
+    // every pair has the tile's sums over its share of k in shared memory: of the tokens, CTA `split` of a slab adds up and finishes
+    // split, split + splits, ..., the shares in their order
+    __syncthreads();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (warp >= 2) {
+      const PairTile tile = pair_tile(p, first);
+      const int m_tile = 2 * tile.m + rank, r4 = lane * 4, n_rows = min(tile.n, p.T - tile.row0);
+      if (m_tile * kBlockM < p.n_out && !wait.marked()) {
+        float bb[4];
+        pair_bias(p, m_tile, r4, bb);
+        constexpr int U = 4;   // tokens whose loads are in flight together
+        for (int t0 = split + p.splits * (warp - 2); t0 < n_rows; t0 += U * 8 * p.splits) {
+          float4 v[U][kPairSplits];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int t = min(t0 + u * 8 * p.splits, n_rows - 1);
+#pragma unroll
+            for (int s = 0; s < kPairSplits; ++s)
+              if (s < p.splits)
+                asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
+                             : "=f"(v[u][s].x), "=f"(v[u][s].y), "=f"(v[u][s].z), "=f"(v[u][s].w)
+                             : "r"(smem_of(smem, 2 * s + rank) + (uint32_t)(t * kBlockM + r4) * 4u)
+                             : "memory");
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int t = t0 + u * 8 * p.splits;
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int s = 0; s < kPairSplits; ++s)
+              if (s < p.splits) a.x += v[u][s].x, a.y += v[u][s].y, a.z += v[u][s].z, a.w += v[u][s].w;
+            if (t < n_rows) finalize4<MODE>(p, m_tile, lane, tile.row0 + t, a, bb, tile.row0 + t);   // warp-uniform
+          }
+        }
+      }
+    }
+  }
+  tc::fence_before();
+  __syncthreads();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // a CTA's shared and tensor memory serve the other's MMAs
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  tc::fence_after();
+  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+}
+
+template <int MODE>
+int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const TcParams& p, int clusters, cudaStream_t s) {
+  static bool attr_set[64] = {};
+  B200_CUDA(ensure_dynamic_smem(linear_pair_kernel<MODE>, kPairSmem, attr_set));
+  B200_CUDA(launch_cluster(linear_pair_kernel<MODE>, dim3(clusters * 2 * p.splits), dim3(kPairThreads), (size_t)kPairSmem, s, dim3(2 * p.splits, 1, 1), mw, mx, p, wait_status_word()));
+  return B200_OK;
+}
+
+}  // namespace
+
+// Tokens a tile and shares of k by an estimate of the launch's cycles: whole waves of tiles over the clusters that fit the GPU at a time, a tile per 64
+// of k its MMAs (2 cycles a token) or its loads (256 + tokens rows of 128 bytes at 64 bytes a cycle and SM, two SMs), the last tile's epilogue and,
+// where k is shared, the exchange.
+PairPlan linear_pair_plan(int T, int n_out, int k) {
+  constexpr int kActive[kPairSplits + 1] = {0, 74, 33, 22, 15};   // clusters of 2, 4, 6, 8 such CTAs that run at a time (cudaOccupancyMaxActiveClusters)
+  const int m = (n_out + 2 * kBlockM - 1) / (2 * kBlockM), kbs = (k + kBlockK - 1) / kBlockK;
+  PairPlan best = {0, 1};
+  int64_t best_cost = 0;
+  for (int n = 256; n >= 32; n -= 32) {
+    const int64_t tiles = (int64_t)m * ((T + n - 1) / n);
+    for (int s = 1; s <= kPairSplits; ++s) {
+      if (s > 1 && (tiles > kActive[s] || kbs / s < 4)) continue;
+      const int64_t c = (tiles + kActive[s] - 1) / kActive[s] * ((kbs + s - 1) / s) * std::max(2 * n, 256 + n) + 20 * std::min(n, T) + (s > 1 ? 800 + 800 * s : 0);
+      if (best.n == 0 || c < best_cost) best = {n, s}, best_cost = c;
+    }
+  }
+  return best;
+}
+
+int linear_pair(int mode, TcParams p, const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, int k, PairPlan pl, cudaStream_t s) {
+  if (const int e = wait_status()) return e;
+  p.pair_n = pl.n;
+  p.splits = pl.splits;
+  p.pair_tok = (p.T + pl.n - 1) / pl.n;
+  p.pair_m = (p.n_out + 2 * kBlockM - 1) / (2 * kBlockM);
+  p.pair_group = (p.pair_tok + (p.pair_tok + 8) / 9 - 1) / ((p.pair_tok + 8) / 9);
+  CUtensorMap mw, mx;
+  int rc = get_tensor_map_2d(w, (uint64_t)p.n_out, (uint64_t)k, (uint64_t)k, kBlockM, &mw);
+  if (rc) return rc;
+  rc = get_tensor_map_2d(x, (uint64_t)p.T, (uint64_t)k, (uint64_t)ldx, (uint32_t)pl.n / 2, &mx);
+  if (rc) return rc;
+  const int clusters = (int)std::min<int64_t>((int64_t)p.pair_tok * p.pair_m, kNumSMs / 2);
+  switch (mode) {
+    case kScatter: return launch_pair<kScatter>(mw, mx, p, clusters, s);
+    case kSiluMul: return launch_pair<kSiluMul>(mw, mx, p, clusters, s);
+    case kRopeKv: return launch_pair<kRopeKv>(mw, mx, p, clusters, s);
+    default: return launch_pair<kPlain>(mw, mx, p, clusters, s);
+  }
+}
+
+}  // namespace b200

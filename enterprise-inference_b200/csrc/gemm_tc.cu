@@ -1,8 +1,8 @@
-// tcgen05 / TMEM weight-streaming linear: y[T][n_out] = x[T][k] . w[n_out][k]^T (+bias), T >= 5.
+// tcgen05 / TMEM weight-streaming linear: y[T][n_out] = x[T][k] . w[n_out][k]^T (+bias), T <= 128 (more: gemm_pair.cu).
 //
-// Decode GEMMs are skinny (T = 8..256 token rows against n_out = 4096..128256 weight rows), so the
+// Decode GEMMs are skinny (T = 8..128 token rows against n_out = 4096..128256 weight rows), so the
 // operands are SWAPPED: a 128-row slab of W is the UMMA "A" operand (M = 128, fills the tensor
-// core's M), the token rows are "B" (N = 16..256), and the fp32 accumulator D[128 features][N
+// core's M), the token rows are "B" (N = 16..128), and the fp32 accumulator D[128 features][N
 // tokens] lives in TMEM (lane = feature, column = token).  Bound: HBM — algorithmic bytes per
 // launch = n_out*k*2, each weight element crosses HBM once; the tensor pipe needs
 // max(128,M)*N/256 cycles per K=16 step = 32 cycles for N = 64 against 4 KiB of W, i.e. it can
@@ -27,14 +27,12 @@
 #include <mutex>
 #include <unordered_map>
 
-#include "common.cuh"
+#include "gemm_epilogue.cuh"
 
 namespace b200 {
 
 namespace {
 
-constexpr int kBlockM = 128;   // weight rows per CTA = UMMA M
-constexpr int kBlockK = 64;    // bf16 elements per stage row = 128 bytes = one swizzle span
 constexpr int kUmmaK = 16;
 constexpr int kTcThreads = 192;
 constexpr int kCounterBytes = 64 * 1024;  // slab tickets at the head of the workspace (16384 slabs x token tiles)
@@ -48,12 +46,7 @@ constexpr uint64_t kEvictNormal = 0x1000000000000000ull;
 #ifndef B200_STAGES64
 #define B200_STAGES64 4
 #endif
-// N = 256 (prefill-sized token tiles): 2 stages of 48 KiB so that TWO CTAs share an SM (2 x 256 TMEM columns):
-// one CTA's epilogue then overlaps the other's main loop; 4 stages are in flight per SM as before.
-#ifndef B200_STAGES256
-#define B200_STAGES256 2
-#endif
-__host__ __device__ constexpr int stages_for(int N) { return N <= 16 ? B200_STAGES16 : (N <= 32 ? 4 : (N <= 64 ? B200_STAGES64 : (N <= 128 ? 3 : B200_STAGES256))); }
+__host__ __device__ constexpr int stages_for(int N) { return N <= 16 ? B200_STAGES16 : (N <= 32 ? 4 : (N <= 64 ? B200_STAGES64 : 3)); }
 __host__ __device__ constexpr int stage_bytes(int N) { return kBlockM * kBlockK * 2 + N * kBlockK * 2; }
 constexpr int kTailBytes = 1024;   // barriers, TMEM slot, ticket | per-token 1/rms [64] (fused-norm consumer)
 // Decode-sized tiles (N <= 32) exchange their cluster split-K partials by PUSH: every CTA stores the tokens owner r
@@ -152,57 +145,10 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-struct TcParams {
-  const __nv_bfloat16* bias;
-  __nv_bfloat16* y;
-  int64_t ldy;
-  int T, n_out, n_kblocks, splits;
-  float* partials;      // [splits][tok_tiles*N][n_out_pad] fp32
-  unsigned int* tickets;  // [m_tiles * tok_tiles], zero on entry, zero on exit
-  int n_out_pad;
-  int cluster;  // 1: the `splits` CTAs of a slab form a thread-block cluster and reduce through DSMEM
-  // MODE_ROPE_KV (slab == one 128-wide head of the fused qkv projection)
-  const int32_t* positions;
-  const int32_t* slots;
-  const __nv_bfloat16* cos_sin;
-  __nv_bfloat16* kc;
-  __nv_bfloat16* vc;
-  int hq, hkv, block_size;
-  unsigned long long* trace;  // debug (B200_TC_TRACE=1): %globaltimer stamps of CTA 0, else null
-  // Residual stream in fp32 (RMSNorm folded into the linears, T <= 64):
-  //   producer (MODE kResidual, O / down projection): s = bf16(acc) + bf16(sres) in fp32 -> sres, and the sum of
-  //     squares of the slab's 128 values of s -> ssq[tok][m_tile]              (n_out = hidden)
-  //   consumer (NI, QKV / gate_up / lm_head): the B operand is bf16(bf16(s * rinv) * norm_w) built in shared memory
-  //     from sres, rinv = 1/sqrt(sum_slabs ssq / hidden + eps)                  (k = hidden)
-  float* sres;
-  float* ssq;
-  const __nv_bfloat16* norm_w;
-  const int32_t* rows;   // consumer: token t of the launch reads stream row rows[t] (lm_head's logit rows), or null
-  int nslab;             // hidden / 128
-  float eps;
-  // Grouped form (routed experts): w holds [experts][n_out][k]; token tile j multiplies the rows of expert grp_tile[j]
-  // (-1: the tile is not in use and its CTAs leave at once).  The token rows are the experts' tokens, gathered so that
-  // no tile holds rows of two experts.
-  const int32_t* grp_tile;
-  // grouped gate|up with the SiLU*mul epilogue: an expert's rows are [gate (gu_ff) | up (gu_ff)]; slab m of the launch is
-  // gate rows m*64.. and the matching up rows, fetched as two 64-row boxes (the layout kSiluMul expects, made by TMA)
-  int gu_ff;
-  int act;   // kSiluMul: b200_act_kind of the gate (0: silu, rounded to bf16 before the product as the fixed stack does)
-  float act_limit;   // B200_ACT_SWIGLU_CLAMP: the clamp of gate and up value
-  // kScatter: row t of the launch goes to grp_out[grp_pair[t]][n_out] (fp32, unrounded) times grp_wt[grp_pair[t]];
-  // grp_pair[t] < 0 marks a padding row
-  // (both null: the identity and weight 1, i.e. a plain fp32 output)
-  const int32_t* grp_pair;
-  const float* grp_wt;
-  float* grp_out;
-  int post_act;          // kPlain: 1 + b200_act_kind applied to the fp32 sum before the rounding (0: none)
-  int tile_n;            // N of the instantiation (kScatter: index of a token inside its tile)
-};
-
 // kScatter: the tile's destination rows and weights, fetched once per CTA before the accumulator is complete (the two
 // dependent global loads per token would otherwise sit between the TMEM drain and every store)
 __device__ __forceinline__ int* scatter_smem() {
-  __shared__ int buf[512];   // [256] destination row | [256] weight (float bits)
+  __shared__ int buf[256];   // [128] destination row | [128] weight (float bits)
   return buf;
 }
 
@@ -219,130 +165,14 @@ __device__ __forceinline__ void tc_trace(const TcParams& p, int slot) {
   }
 }
 
-// Epilogue modes (template parameter):
-//  kPlain    y[t][row] = bf16(acc + bias), or bf16(act(acc + bias)) (TcParams::post_act)
-//  kSiluMul  the slab holds 64 gate rows then the 64 matching up rows (B200_W_GATE_UP_INTERLEAVED):
-//            y[t][m_tile*64 + i] = bf16(bf16(silu(bf16(g_i))) * bf16(u_i))          (R5)
-//            (TcParams::act != 0: bf16(act(bf16(g_i)) * bf16(u_i)) for the other gate activations)
-//  kRopeKv   the slab is one head of the fused qkv projection: NeoX RoPE in bf16 arithmetic (R3) on q
-//            and k heads, q rows to y, k/v rows straight into the paged cache at slots[t]
-//  kResidual the linear's output is added to the fp32 residual stream (see TcParams::sres): no y is written
-//  kScatter  (grouped form) the fp32 row times a per-row weight goes to the row the indirection names; no y
-enum { kPlain = 0, kSiluMul = 1, kRopeKv = 2, kResidual = 3, kScatter = 4 };
-
-
-// One thread finalises 4 consecutive slab rows (r4..r4+3, lane = r4/4) of one token.
 template <int MODE>
-__device__ __forceinline__ void finalize4(const TcParams& p, int m_tile, int lane, int tok, float4 a, const float (&bb)[4]) {
-  const int r4 = lane * 4;
-  float v[4] = {round_bf16(a.x + bb[0]), round_bf16(a.y + bb[1]), round_bf16(a.z + bb[2]), round_bf16(a.w + bb[3])};
-  if constexpr (MODE == kPlain) {
-    if (p.post_act == 1 + B200_ACT_RELU2) {
-      const float r[4] = {fmaxf(a.x + bb[0], 0.f), fmaxf(a.y + bb[1], 0.f), fmaxf(a.z + bb[2], 0.f), fmaxf(a.w + bb[3], 0.f)};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) v[e] = r[e] * r[e];
-    } else if (p.post_act == 1 + B200_ACT_GELU_ERF) {
-      v[0] = gelu_erf_fast(a.x + bb[0]), v[1] = gelu_erf_fast(a.y + bb[1]);
-      v[2] = gelu_erf_fast(a.z + bb[2]), v[3] = gelu_erf_fast(a.w + bb[3]);
-    } else if (p.post_act) {
-      v[0] = act_apply(a.x + bb[0], p.post_act - 1), v[1] = act_apply(a.y + bb[1], p.post_act - 1);
-      v[2] = act_apply(a.z + bb[2], p.post_act - 1), v[3] = act_apply(a.w + bb[3], p.post_act - 1);
-    }
-    const int row = m_tile * kBlockM + r4;
-    __nv_bfloat16* dst = p.y + (int64_t)tok * p.ldy + row;
-    if (row + 3 < p.n_out && (p.ldy % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.y) & 7) == 0)) {
-      *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (row + e < p.n_out) dst[e] = __float2bfloat16_rn(v[e]);
-    }
-  } else if constexpr (MODE == kSiluMul) {
-    // lanes 0..15 hold 4 gate rows, lanes 16..31 the 4 matching up rows: after the exchange every lane has
-    // both, and each half-warp finalises two of the four features (all 32 lanes busy: the accurate
-    // expf + division of R5 is what this epilogue costs at large T)
-    float x[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) x[e] = __shfl_xor_sync(0xffffffffu, v[e], 16);
-    const bool lo = lane < 16;
-    const float g0 = lo ? v[0] : x[2], g1 = lo ? v[1] : x[3];
-    const float u0 = lo ? x[0] : v[2], u1 = lo ? x[1] : v[3];
-    const int f = m_tile * 64 + (lane & 15) * 4 + (lo ? 0 : 2);                  // output feature
-    const float o0 = p.act == 0 ? silu_to_bf16(g0) * u0 : gate_combine(g0, u0, p.act, p.act_limit);
-    const float o1 = p.act == 0 ? silu_to_bf16(g1) * u1 : gate_combine(g1, u1, p.act, p.act_limit);
-    __nv_bfloat16* dst = p.y + (int64_t)tok * p.ldy + f;
-    if ((p.ldy % 2 == 0) && ((reinterpret_cast<uintptr_t>(p.y) & 3) == 0)) {
-      *reinterpret_cast<uint32_t*>(dst) = pack_bf16(o0, o1);
-    } else {
-      dst[0] = __float2bfloat16_rn(o0);
-      dst[1] = __float2bfloat16_rn(o1);
-    }
-  } else if constexpr (MODE == kResidual) {
-    // x = bf16(acc + bias); s = x + bf16(s_old) in fp32 (R1: the residual is kept in bf16, the sum is not rounded
-    // before the variance and the normalisation); sum of squares in a fixed order: lane's 4 rows, then the warp tree
-    const int row = m_tile * kBlockM + r4;
-    float4* sp = reinterpret_cast<float4*>(p.sres + (int64_t)tok * p.n_out + row);
-    const float4 so = *sp;
-    const float4 sn = make_float4(v[0] + round_bf16(so.x), v[1] + round_bf16(so.y), v[2] + round_bf16(so.z),
-                                  v[3] + round_bf16(so.w));
-    *sp = sn;
-    float ss = fmaf(sn.x, sn.x, 0.f);
-    ss = fmaf(sn.y, sn.y, ss);
-    ss = fmaf(sn.z, sn.z, ss);
-    ss = fmaf(sn.w, sn.w, ss);
-    ss = warp_sum(ss);
-    if (lane == 0) p.ssq[(int64_t)tok * p.nslab + m_tile] = ss;
-  } else if constexpr (MODE == kScatter) {
+__device__ __forceinline__ void finalize_token(const TcParams& p, int m_tile, int lane, int tok, float4 a, const float (&bb)[4]) {
+  if constexpr (MODE == kScatter) {
     const int* sc = scatter_smem();
     const int tl = tok % p.tile_n;
-    const int pair = sc[tl];   // warp-uniform
-    if (pair < 0) return;
-    const float wt = __int_as_float(sc[256 + tl]);
-    const int row = m_tile * kBlockM + r4;
-    float* dst = p.grp_out + (int64_t)pair * p.n_out + row;
-    if (row + 3 < p.n_out && (p.n_out % 4 == 0)) {
-      *reinterpret_cast<float4*>(dst) = make_float4(a.x * wt, a.y * wt, a.z * wt, a.w * wt);
-    } else {
-      const float o[4] = {a.x * wt, a.y * wt, a.z * wt, a.w * wt};
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (row + e < p.n_out) dst[e] = o[e];
-    }
-  } else {  // kRopeKv
-    const int head = m_tile;
-    float o[4];
-    if (head < p.hq + p.hkv) {
-      float other[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) other[e] = __shfl_xor_sync(0xffffffffu, v[e], 16);
-      const int i0 = r4 & 63;
-      const __nv_bfloat16* cs = p.cos_sin + (int64_t)p.positions[tok] * kHeadDim;
-      const uint2 cq = *reinterpret_cast<const uint2*>(cs + i0);
-      const uint2 sq = *reinterpret_cast<const uint2*>(cs + 64 + i0);
-      const float c[4] = {bf16lo(cq.x), bf16hi(cq.x), bf16lo(cq.y), bf16hi(cq.y)};
-      const float sn[4] = {bf16lo(sq.x), bf16hi(sq.x), bf16lo(sq.y), bf16hi(sq.y)};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        // lanes 0..15 hold x1 (o1 = x1*c - x2*s), lanes 16..31 hold x2 (o2 = x2*c + x1*s); every op rounds
-        const float a0 = round_bf16(v[e] * c[e]), b0 = round_bf16(other[e] * sn[e]);
-        o[e] = lane < 16 ? round_bf16(a0 - b0) : round_bf16(a0 + b0);
-      }
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) o[e] = v[e];
-    }
-    __nv_bfloat16* dst;
-    if (head < p.hq) {
-      dst = p.y + (int64_t)tok * p.ldy + head * kHeadDim + r4;
-    } else {
-      const int slot = p.slots[tok];
-      if (slot < 0) return;
-      const bool is_k = head < p.hq + p.hkv;
-      const int kvh = is_k ? head - p.hq : head - p.hq - p.hkv;
-      const int64_t blk = slot / p.block_size, off = slot % p.block_size;
-      dst = (is_k ? p.kc : p.vc) + ((blk * p.hkv + kvh) * p.block_size + off) * kHeadDim + r4;
-    }
-    *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]));
+    finalize4<MODE>(p, m_tile, lane, tok, a, bb, sc[tl], __int_as_float(sc[128 + tl]));
+  } else {
+    finalize4<MODE>(p, m_tile, lane, tok, a, bb);
   }
 }
 
@@ -597,7 +427,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
           if (pair >= 0 && p.grp_wt) wt = __ldg(p.grp_wt + pair);
         }
         sc[t] = pair;
-        sc[256 + t] = __float_as_int(wt);
+        sc[128 + t] = __float_as_int(wt);
       }
       asm volatile("bar.sync 1, 128;" ::: "memory");
     }
@@ -612,51 +442,6 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     // All MMAs have completed (tmem_full), so the pipeline stages are free: stage the fp32 tile
     // [token][128 rows] there for the direct case, or spill it to the split-K workspace.
     float* stg = reinterpret_cast<float*>(smem);
-    constexpr bool kChunked = S * kStageBytes < N * kBlockM * 4;   // N = 256 with 2 stages: 128 tokens at a time
-    if constexpr (kChunked) {
-      // (host side: this instantiation is only launched with splits == 1 and no cluster)
-      constexpr int kEpiTok = 128;
-      static_assert(kEpiTok * kBlockM * 4 <= S * kStageBytes, "staging area");
-      const int r4 = lane * 4;
-      float bb[4] = {0.f, 0.f, 0.f, 0.f};
-      if (p.bias) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (m_tile * kBlockM + r4 + e < p.n_out) bb[e] = __bfloat162float(p.bias[m_tile * kBlockM + r4 + e]);
-      }
-      for (int cb = 0; cb < N && tok0 + cb < p.T; cb += kEpiTok) {
-#pragma unroll
-        for (int c = 0; c < kEpiTok; c += 16) {
-          uint32_t r[16];
-          if (nkb > 0) {
-            tmem_ld16(taddr + cb + c, r);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) r[j] = 0u;
-          }
-#pragma unroll
-          for (int j = 0; j < 16; ++j) stg[(c + j) * kBlockM + srow] = __uint_as_float(r[j]);
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        const int tmax = min(kEpiTok, p.T - tok0 - cb);
-        if (MODE == kRopeKv) {
-          for (int t = wq + 4 * lane; t < tmax; t += 128) {
-            const char* row = reinterpret_cast<const char*>(p.cos_sin + (int64_t)p.positions[tok0 + cb + t] * kHeadDim);
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(row));
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(row + 128));
-          }
-        }
-        for (int t = wq; t < tmax; t += 16) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int tt = t + 4 * u;
-            if (tt < tmax)   // warp-uniform: the shuffles inside finalize4 stay convergent
-              finalize4<MODE>(p, m_tile, lane, tok0 + cb + tt, *reinterpret_cast<const float4*>(stg + tt * kBlockM + r4), bb);
-          }
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");   // the staging area is reused by the next 128 tokens
-      }
-    } else {
 #pragma unroll
     for (int c = 0; c < N; c += 16) {
       uint32_t r[16];
@@ -722,7 +507,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
               acc.z += v.z;
               acc.w += v.w;
             }
-            finalize4<MODE>(p, m_tile, lane, tok0 + split + S2 * tl, acc, bb);   // warp-uniform loop
+            finalize_token<MODE>(p, m_tile, lane, tok0 + split + S2 * tl, acc, bb);   // warp-uniform loop
           }
         }
         if (threadIdx.x == 64) tc_trace(p, 11);   // this CTA's share finalized
@@ -789,12 +574,11 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         for (int u = 0; u < 4; ++u) {
           const int tt = t + 4 * u;
           // warp-uniform condition: the shuffles inside finalize4 stay convergent
-          if (tt < tmax) finalize4<MODE>(p, m_tile, lane, tok0 + tt, acc[u], bb);
+          if (tt < tmax) finalize_token<MODE>(p, m_tile, lane, tok0 + tt, acc[u], bb);
         }
       }
       if (p.splits > 1 && warp == 2 && lane == 0) p.tickets[tile_id] = 0u;  // leave the tickets zero for the next launch
     }
-    }   // !kChunked
     tc_fence_before();
   }
   if (push) {
@@ -855,7 +639,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
               acc.w += v[u][pr].w;
             }
           }
-          if (tt < tmax) finalize4<MODE>(p, m_tile, lane, tok0 + tt, acc, bb);   // warp-uniform condition
+          if (tt < tmax) finalize_token<MODE>(p, m_tile, lane, tok0 + tt, acc, bb);   // warp-uniform condition
         }
       }
     }
@@ -952,6 +736,7 @@ struct Plan {
   int N, m_tiles, tok_tiles, n_kblocks, splits, n_out_pad;
 };
 
+// (T > 128: the workspace that is asked for, and what is refused; the launch itself is gemm_pair.cu's)
 Plan make_plan(int T, int n_out, int k) {
   Plan pl;
   pl.N = n_tile_for(T);
@@ -997,11 +782,6 @@ int launch_tc3(const CUtensorMap& mw, const CUtensorMap& mx, const TcParams& p, 
 
 template <int N, int MODE, bool NI>
 int launch_tc2(const CUtensorMap& mw, const CUtensorMap& mx, const TcParams& p, const Plan& pl, cudaStream_t s) {
-  if constexpr (N == 256) {
-    // the 2-stage kernel (two CTAs per SM, chunked epilogue) has no room for a whole fp32 tile: split-K
-    // launches of a single token tile keep 4 stages
-    if (pl.splits > 1 || p.cluster) return launch_tc3<N, MODE, 4, NI>(mw, mx, p, pl, s);
-  }
   return launch_tc3<N, MODE, stages_for(N), NI>(mw, mx, p, pl, s);
 }
 
@@ -1060,7 +840,7 @@ int linear_tc(const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, const
               const LinearExtra* ex, cudaStream_t s) {
   B200_REQUIRE(k % 8 == 0, B200_ERR_UNSUPPORTED, "linear_tc: k must be a multiple of 8");
   B200_REQUIRE(reinterpret_cast<uintptr_t>(w) % 16 == 0, B200_ERR_INVALID, "linear_tc: w must be 16-byte aligned");
-  const Plan pl = make_plan(T, n_out, k);
+  Plan pl = make_plan(T, n_out, k);
   const int64_t need = linear_tc_workspace_bytes(T, n_out, k);
   static const int cluster_env = getenv("B200_TC_CLUSTER") ? atoi(getenv("B200_TC_CLUSTER")) : 1;
   const bool use_cluster = cluster_env != 0 && pl.splits > 1 && pl.splits <= 8;
@@ -1111,15 +891,12 @@ int linear_tc(const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, const
     p.nslab = k / kBlockM;
     p.eps = ex->eps;
   }
-  CUtensorMap mw, mx;
-  int rc = get_map(w, (uint64_t)n_out, (uint64_t)k, (uint64_t)k, kBlockM, &mw);
-  if (rc) return rc;
-  if (ni) {
-    mx = mw;   // unused: the B operand is built in shared memory
-  } else {
-    B200_REQUIRE(x && reinterpret_cast<uintptr_t>(x) % 16 == 0 && ldx % 8 == 0, B200_ERR_INVALID, "linear_tc: bad x");
-    rc = get_map(x, (uint64_t)T, (uint64_t)k, (uint64_t)ldx, (uint32_t)pl.N, &mx);
-    if (rc) return rc;
+  B200_REQUIRE(ni || (x && reinterpret_cast<uintptr_t>(x) % 16 == 0 && ldx % 8 == 0), B200_ERR_INVALID, "linear_tc: bad x");
+  if (T > 128) {
+    // unrounded fp32 sums with k in more shares than gemm_pair.cu would take keep them: each share is a shorter sum (2 048 rows of 2048 into the
+    // logits of 32 experts: relative error 2.4e-7 in eight shares, 6.5e-7 in one; 13 us a call of the router, 17 in tiles of 256 rows)
+    pl.N = 128;
+    pl.tok_tiles = (T + 127) / 128;
   }
   p.bias = bias;
   p.y = y;
@@ -1132,12 +909,17 @@ int linear_tc(const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, const
   p.partials = ws ? reinterpret_cast<float*>(static_cast<char*>(ws) + kCounterBytes) : nullptr;
   p.n_out_pad = pl.n_out_pad;
   p.tile_n = pl.N;
+  if (T > 128 && (mode != kScatter || pl.splits == 1)) return linear_pair(mode, p, x, ldx, w, k, linear_pair_plan(T, n_out, k), s);
+  CUtensorMap mw, mx;
+  int rc = get_map(w, (uint64_t)n_out, (uint64_t)k, (uint64_t)k, kBlockM, &mw);
+  if (rc) return rc;
+  mx = mw;   // norm_in: unused, the B operand is built in shared memory
+  if (!ni && (rc = get_map(x, (uint64_t)T, (uint64_t)k, (uint64_t)ldx, (uint32_t)pl.N, &mx))) return rc;
   switch (pl.N) {
     case 16: return launch_tc<16>(mode, ni, mw, mx, p, pl, s);
     case 32: return launch_tc<32>(mode, ni, mw, mx, p, pl, s);
     case 64: return launch_tc<64>(mode, ni, mw, mx, p, pl, s);
-    case 128: return launch_tc<128>(mode, ni, mw, mx, p, pl, s);
-    default: return launch_tc<256>(mode, ni, mw, mx, p, pl, s);
+    default: return launch_tc<128>(mode, ni, mw, mx, p, pl, s);
   }
 }
 

@@ -1,4 +1,4 @@
-// Waits of the tcgen05 attention kernels that ran out (tc.cuh): the word they set in host memory, and the error that the next call makes of it.
+// Waits of the tcgen05 attention kernels and pair linears that ran out (tc.cuh): the word they set in host memory, and the error that the next call makes of it.
 #include "tc.cuh"
 
 namespace b200 {
@@ -18,7 +18,7 @@ uint32_t* wait_status_word() {
 int wait_status() {
   uint32_t* const w = wait_status_word();
   B200_REQUIRE(!w || __atomic_load_n(w, __ATOMIC_RELAXED) == 0 || __atomic_exchange_n(w, 0u, __ATOMIC_RELAXED) == 0, B200_ERR_CUDA,
-               "a wait in an attention kernel of an earlier call ran out: that call's results are not valid");
+               "a wait in a kernel of an earlier call ran out: that call's results are not valid");
   return B200_OK;
 }
 

@@ -1,0 +1,70 @@
+"""The tcgen05 linear on pairs of SMs (more than 128 tokens): edges of token tiles, slabs, k blocks and shares of k."""
+import importlib
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+
+
+@pytest.fixture(scope="module")
+def abi():
+    return importlib.import_module("enterprise-inference_b200._abi")
+
+
+def _operands(T, n_out, k, ldx):
+    g = torch.Generator(device="cuda").manual_seed(T * 7 + n_out + k)
+    x = torch.randn(T, ldx, generator=g, device="cuda").to(BF)
+    w = (0.05 * torch.randn(n_out, k, generator=g, device="cuda")).to(BF)
+    return g, x, w
+
+
+def _bound(x, w, y):
+    """Half a unit of bf16 (8 bits), and k additions of fp32 products (24 bits; the tensor core may truncate: one unit each)."""
+    return y.abs() * 2.0 ** -8 + x.shape[1] * 2.0 ** -23 * (x.abs() @ w.abs().T)
+
+
+@pytest.mark.parametrize("T,n_out,k,pad", [
+    (129, 8, 8, 0),             # one slab, one k block, both mostly empty
+    (129, 264, 72, 8),          # a slab of 8 rows, the last k block of 8; rows of x and y with a gap
+    (160, 384, 256, 0),         # an odd number of slabs: a pair's second CTA has none
+    (255, 1000, 4096, 0),       # k shared by clusters
+    (257, 256, 4160, 0),        # uneven shares of 65 k blocks
+    (300, 2048, 2048, 0), (200, 4096, 1536, 0), (256, 6144, 1024, 16),
+    (513, 2048, 1000, 0),
+    (2048, 4096, 256, 0),       # two tiles a pair
+    (5000, 1024, 128, 0),       # token tiles in groups of unequal size, several tiles a pair
+])
+def test_linear_pairs_of_sms(abi, T, n_out, k, pad):
+    lib, P = abi.lib(), abi.ptr
+    g, x, w = _operands(T, n_out, k, k + pad)
+    b = torch.randn(n_out, generator=g, device="cuda").to(BF)
+    wsb = int(lib.b200_linear_workspace_bytes(T, n_out, k))
+    ws = torch.zeros(wsb, dtype=torch.uint8, device="cuda")
+    xd, wd = x[:, :k].double(), w.double()
+    want = xd @ wd.T + b.double()
+    for bias in (b, None):
+        y = torch.full((T, n_out + pad), float("nan"), dtype=BF, device="cuda")
+        abi.check(lib.b200_linear_bf16(P(x), k + pad, P(w), P(bias) if bias is not None else None, P(y), n_out + pad, T, n_out, k, 0, P(ws), wsb, None))
+        torch.cuda.synchronize()
+        ref = want if bias is not None else want - b.double()
+        assert (y[:, :n_out].double() - ref).abs().le(_bound(xd, wd, ref)).all()
+        assert torch.isnan(y[:, n_out:].float()).all(), "columns beyond the output were written"
+
+
+@pytest.mark.parametrize("T,I,k", [(129, 192, 512), (300, 64, 4096), (700, 1600, 256)])
+def test_gate_up_epilogue_on_pairs_of_sms(abi, T, I, k):
+    """SiLU * mul over interleaved slabs, odd numbers of them included, equals the plain linear and b200_silu_mul bit for bit."""
+    lib, P = abi.lib(), abi.ptr
+    _, x, w = _operands(T, 2 * I, k, k)
+    il = torch.stack([w[:I].reshape(-1, 64, k), w[I:].reshape(-1, 64, k)], 1).reshape(2 * I, k).contiguous()
+    wsb = int(lib.b200_linear_workspace_bytes(T, 2 * I, k))
+    ws = torch.zeros(wsb, dtype=torch.uint8, device="cuda")
+    gu, ref = torch.empty(T, 2 * I, dtype=BF, device="cuda"), torch.empty(T, I, dtype=BF, device="cuda")
+    got = torch.full((T + 1, I), float("nan"), dtype=BF, device="cuda")
+    abi.check(lib.b200_linear_bf16(P(x), k, P(w), None, P(gu), 2 * I, T, 2 * I, k, 0, P(ws), wsb, None))
+    abi.check(lib.b200_silu_mul(P(gu), P(ref), T, I, None))
+    abi.check(lib.b200_linear_fused_bf16(P(x), k, P(il), None, P(got), I, T, 2 * I, k, 1, None, None, None, None, None, 0, 0, 0, P(ws), wsb, None))
+    torch.cuda.synchronize()
+    assert torch.equal(got[:T], ref) and torch.isnan(got[T].float()).all()
