@@ -187,5 +187,20 @@ struct PairPlan {
 };
 PairPlan linear_pair_plan(int T, int n_out, int k);
 int linear_pair(int mode, TcParams p, const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, int k, PairPlan pl, cudaStream_t s);
+// The same over the gathered rows of every expert: w [experts][n_out][k], an expert's rows a run of x, cut into token tiles by a table on the device
+// (TcParams::pair_tile).  y[row] = act(x . w_e^T) (post_act: 1 + b200_act_kind, 0 none); gate_up: w [experts][2 ff][k], gate rows then up rows, y[row][ff]
+// the activated product; scatter: out[row_pair[row]] = wts[row_pair[row]] * (x . w_e^T) in fp32 (row_pair < 0: a padding row).
+struct GroupedPairs {
+  const int4* tiles;
+  int max_tiles;    // of the table
+  int64_t rows;     // of x, at most
+  int experts;
+};
+int linear_pair_grouped(const GroupedPairs& g, const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, int n_out, int k, __nv_bfloat16* y, int64_t ldy,
+                        cudaStream_t s, int post_act = 0);
+int linear_pair_gate_up(const GroupedPairs& g, const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, int ff, int k, __nv_bfloat16* y, cudaStream_t s,
+                        int act, float act_limit);
+int linear_pair_scatter(const GroupedPairs& g, const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, int n_out, int k, const int32_t* row_pair,
+                        const float* wts, float* out, cudaStream_t s);
 
 }  // namespace b200

@@ -384,4 +384,64 @@ int linear_pair(int mode, TcParams p, const __nv_bfloat16* x, int64_t ldx, const
   }
 }
 
+// ---- grouped form ----------------------------------------------------------------------------------------------------------
+static int launch_grouped_pair(int mode, TcParams p, const GroupedPairs& g, const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, int w_box, int k,
+                               cudaStream_t s) {
+  B200_REQUIRE(x && w && g.tiles && k > 0 && k % 8 == 0 && ldx % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0,
+               B200_ERR_INVALID, "grouped linear: operands in rows of 16-byte pieces");
+  if (const int e = wait_status()) return e;
+  p.T = (int)g.rows;
+  p.n_kblocks = (k + kBlockK - 1) / kBlockK;
+  p.splits = 1;
+  p.pair_tile = g.tiles;
+  CUtensorMap mw, mx;
+  int rc = get_tensor_map_2d(w, (uint64_t)g.experts * p.n_out, (uint64_t)k, (uint64_t)k, (uint32_t)w_box, &mw);
+  if (rc) return rc;
+  rc = get_tensor_map_2d(x, (uint64_t)g.rows, (uint64_t)k, (uint64_t)ldx, 16, &mx);   // tiles of any number of units
+  if (rc) return rc;
+  const int clusters = (int)std::min<int64_t>((int64_t)g.max_tiles * p.pair_m, kNumSMs / 2);
+  switch (mode) {
+    case kScatter: return launch_pair<kScatter>(mw, mx, p, clusters, s);
+    case kSiluMul: return launch_pair<kSiluMul>(mw, mx, p, clusters, s);
+    default: return launch_pair<kPlain>(mw, mx, p, clusters, s);
+  }
+}
+
+int linear_pair_grouped(const GroupedPairs& g, const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, int n_out, int k, __nv_bfloat16* y, int64_t ldy,
+                        cudaStream_t s, int post_act) {
+  TcParams p = {};
+  p.y = y;
+  p.ldy = ldy;
+  p.n_out = n_out;
+  p.post_act = post_act;
+  p.pair_m = (n_out + 2 * kBlockM - 1) / (2 * kBlockM);
+  return launch_grouped_pair(kPlain, p, g, x, ldx, w, kBlockM, k, s);
+}
+
+int linear_pair_gate_up(const GroupedPairs& g, const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, int ff, int k, __nv_bfloat16* y, cudaStream_t s,
+                        int act, float act_limit) {
+  B200_REQUIRE(ff > 0 && ff % (kBlockM / 2) == 0, B200_ERR_UNSUPPORTED, "grouped gate|up: ff=%d must be a multiple of 64", ff);
+  TcParams p = {};
+  p.y = y;
+  p.ldy = ff;
+  p.n_out = 2 * ff;
+  p.gu_ff = ff;
+  p.act = act;
+  p.act_limit = act_limit;
+  p.pair_m = (ff + kBlockM - 1) / kBlockM;
+  return launch_grouped_pair(kSiluMul, p, g, x, ldx, w, kBlockM / 2, k, s);
+}
+
+int linear_pair_scatter(const GroupedPairs& g, const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, int n_out, int k, const int32_t* row_pair,
+                        const float* wts, float* out, cudaStream_t s) {
+  B200_REQUIRE(row_pair && wts && out && reinterpret_cast<uintptr_t>(out) % 16 == 0, B200_ERR_INVALID, "grouped linear: no destination");
+  TcParams p = {};
+  p.n_out = n_out;
+  p.grp_pair = row_pair;
+  p.grp_wt = wts;
+  p.grp_out = out;
+  p.pair_m = (n_out + 2 * kBlockM - 1) / (2 * kBlockM);
+  return launch_grouped_pair(kScatter, p, g, x, ldx, w, kBlockM, k, s);
+}
+
 }  // namespace b200

@@ -26,6 +26,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "gemm_epilogue.cuh"
 
 namespace b200 {
 namespace {
@@ -368,6 +369,9 @@ moe_expert_grouped_kernel(const AT* __restrict__ x, const __nv_bfloat16* __restr
 // in_wts given (the mixing weight belongs to the expert's input): the row is scaled by its pair's weight (fp32 product, rounded
 // once), and ones[pair] = 1 so that the closing linear's per-pair factor is neutral.
 //
+// pair_tile given (long steps, gemm_pair.cu): N is the unit of a run's length (32 rows) and the table is that of the linear on pairs of SMs: a count,
+// then (expert, first row, rows) of each token tile; a run is cut into as few tiles of at most 256 rows as it takes, of equal length up to a unit.
+//
 // One CTA per (expert, share of its rows).  Each counts all pairs by expert (shared-memory atomics) and, per warp over a stretch of
 // the list, those of its own expert (ballots); a scan gives the expert's first tile, a second walk every pair its row; the rows of the
 // CTA's share are then copied, a warp a row.  The counting is repeated by every CTA, which costs less than a launch of its own: a single
@@ -375,20 +379,22 @@ moe_expert_grouped_kernel(const AT* __restrict__ x, const __nv_bfloat16* __restr
 // the ids, then by the row copies.
 constexpr int kGroupThreads = 1024;
 constexpr int kGroupWarps = kGroupThreads / 32;
+constexpr int kPairUnit = 32, kPairUnits = 8;   // rows of a unit of pair_tile's runs; units of a tile at most
 
 __global__ void __launch_bounds__(kGroupThreads)
 moe_group_gather_kernel(const int32_t* __restrict__ ids, int n_pairs, int experts, int N, int n_tiles, int32_t* __restrict__ tile_expert,
-                        int32_t* __restrict__ row_pair, const __nv_bfloat16* __restrict__ x, int top, int width, __nv_bfloat16* __restrict__ xg,
-                        const float* __restrict__ in_wts, float* __restrict__ ones) {
+                        int4* __restrict__ pair_tile, int32_t* __restrict__ row_pair, const __nv_bfloat16* __restrict__ x, int top, int width,
+                        __nv_bfloat16* __restrict__ xg, const float* __restrict__ in_wts, float* __restrict__ ones) {
   extern __shared__ int32_t hist[];   // [experts] pairs
   __shared__ int32_t wcnt[kGroupWarps];
   __shared__ int32_t run_tile, end_tile;   // first tile of this expert's run; tiles of all runs
+  __shared__ int32_t run_pair, end_pair;   // the same in entries of pair_tile
   pdl_wait();
   pdl_launch_dependents();
   const int e = blockIdx.x, part = blockIdx.y, parts = gridDim.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int i = tid; i < experts; i += kGroupThreads) hist[i] = 0;
-  if (tid == 0) run_tile = end_tile = 0;
+  if (tid == 0) run_tile = end_tile = run_pair = end_pair = 0;
   __syncthreads();
   const int seg = ((n_pairs + kGroupWarps - 1) / kGroupWarps + 31) / 32 * 32;   // a warp's stretch of the list
   const int i0 = min(warp * seg, n_pairs), i1 = min(i0 + seg, n_pairs);
@@ -406,22 +412,35 @@ moe_group_gather_kernel(const int32_t* __restrict__ ids, int n_pairs, int expert
   if (lane == 0) wcnt[warp] = mine;
   __syncthreads();
   {   // tiles of the runs before this expert's, and of all runs
-    int before = 0, all = 0;
+    int before = 0, all = 0, pair_before = 0, pair_all = 0;
     for (int i = tid; i < experts; i += kGroupThreads) {
-      const int nt = (hist[i] + N - 1) / N;
+      const int nt = (hist[i] + N - 1) / N, np = (nt + kPairUnits - 1) / kPairUnits;
       all += nt;
       before += i < e ? nt : 0;
+      pair_all += np;
+      pair_before += i < e ? np : 0;
     }
     before = __reduce_add_sync(0xffffffffu, before);
     all = __reduce_add_sync(0xffffffffu, all);
+    pair_before = __reduce_add_sync(0xffffffffu, pair_before);
+    pair_all = __reduce_add_sync(0xffffffffu, pair_all);
     if (lane == 0) {
       atomicAdd(&run_tile, before);
       atomicAdd(&end_tile, all);
+      atomicAdd(&run_pair, pair_before);
+      atomicAdd(&end_pair, pair_all);
     }
   }
   __syncthreads();
   const int count = hist[e], tiles = (count + N - 1) / N, row0 = run_tile * N, rows = min((run_tile + tiles), n_tiles) * N - row0;
-  if (part == 0) {
+  if (part == 0 && pair_tile != nullptr) {
+    const int np = (tiles + kPairUnits - 1) / kPairUnits;
+    for (int i = tid; i < np; i += kGroupThreads) {
+      const int u0 = tiles * i / np, u1 = tiles * (i + 1) / np;
+      pair_tile[1 + run_pair + i] = make_int4(e, row0 + u0 * N, (u1 - u0) * N, 0);
+    }
+    if (e == 0 && tid == 0) pair_tile[0] = make_int4(end_pair, 0, 0, 0);
+  } else if (part == 0) {
     for (int i = tid; i < tiles; i += kGroupThreads)
       if (run_tile + i < n_tiles) tile_expert[run_tile + i] = e;
     if (e == experts - 1)
@@ -475,10 +494,13 @@ moe_group_gather_kernel(const int32_t* __restrict__ ids, int n_pairs, int expert
 
 static int64_t al256(int64_t v) { return (v + 255) / 256 * 256; }
 
-// tensor-core form: rows and tiles of a step of T tokens (every expert's run padded to whole tiles of N rows)
-static void moe_tc_shape(int T, int top, int experts, int* N, int* n_tiles) {
+// tensor-core form: rows and tiles of a step of T tokens (every expert's run padded to whole tiles of N rows).  More than 64 rows an expert in the mean: runs of
+// whole units of 32 rows for the linears on pairs of SMs.
+static void moe_tc_shape(int T, int top, int experts, int* N, int* n_tiles, bool* pairs_of_sms) {
   const int pairs = T * top;
   *N = linear_tc_grouped_tile(pairs, experts);
+  *pairs_of_sms = *N > 64;
+  if (*pairs_of_sms) *N = kPairUnit;
   *n_tiles = pairs / *N + std::min(experts, pairs);
 }
 
@@ -500,11 +522,15 @@ static int moe_experts_tc(const __nv_bfloat16* x, const __nv_bfloat16* w_gu, con
                           const float* wts, int T, int width, int ff, int experts, int top, float* parts, void* ws,
                           cudaStream_t s, ExpertForm form) {
   int N, n_tiles;
-  moe_tc_shape(T, top, experts, &N, &n_tiles);
+  bool on_pairs;
+  moe_tc_shape(T, top, experts, &N, &n_tiles, &on_pairs);
   const int64_t rows = (int64_t)n_tiles * N;
+  // (the table of on_pairs is up to 12 bytes an expert longer than the other one, its rows 96 an expert fewer)
+  const int max_tiles = n_tiles / kPairUnits + std::min(experts, T * top);
   char* p = static_cast<char*>(ws);
   int32_t* tile_expert = reinterpret_cast<int32_t*>(p);
-  p += al256(((int64_t)T * top / 16 + experts + 1) * 4);
+  int4* pair_tile = on_pairs ? reinterpret_cast<int4*>(p) : nullptr;
+  p += al256(on_pairs ? (int64_t)(max_tiles + 1) * 16 : ((int64_t)T * top / 16 + experts + 1) * 4);
   int32_t* row_pair = reinterpret_cast<int32_t*>(p);
   p += al256(rows * 4);
   __nv_bfloat16* xg = reinterpret_cast<__nv_bfloat16*>(p);
@@ -521,16 +547,29 @@ static int moe_experts_tc(const __nv_bfloat16* x, const __nv_bfloat16* w_gu, con
   // about 64 rows a CTA, and no more CTAs than four per SM: beyond that the repeated counting outweighs the copies it spreads
   const int64_t per = std::max<int64_t>(1, std::min<int64_t>((int64_t)T * top / (64 * (int64_t)experts), 4 * kNumSMs / experts));
   B200_CUDA(launch(moe_group_gather_kernel, dim3(experts, (unsigned)per), dim3(kGroupThreads), smem_grp, s, ids, T * top, experts, N, n_tiles, tile_expert,
-                   row_pair, x, top, width, xg, form.weight_input ? wts : (const float*)nullptr, ones));
+                   pair_tile, row_pair, x, top, width, xg, form.weight_input ? wts : (const float*)nullptr, ones));
   const PdlScope after_grouping;
   if (form.weight_input) wts = ones;
   int rc;
   static const int fuse_env = getenv("B200_MOE_FUSE_SILU") ? atoi(getenv("B200_MOE_FUSE_SILU")) : 1;
+  if (on_pairs) {
+    GroupedPairs g = {pair_tile, max_tiles, rows, experts};
+    const bool fused = form.gated && (form.act == B200_ACT_SILU || form.act == B200_ACT_SWIGLU_CLAMP) && fuse_env && ff % 64 == 0;
+    if (!form.gated) rc = linear_pair_grouped(g, xg, width, w_gu, ff, width, act, ff, s, 1 + form.act);
+    else if (fused) rc = linear_pair_gate_up(g, xg, width, w_gu, ff, width, act, s, form.act, form.limit);
+    else rc = linear_pair_grouped(g, xg, width, w_gu, 2 * ff, width, gu, 2 * ff, s);
+    if (rc) return rc;
+    if (form.gated && !fused) {
+      rc = form.act == B200_ACT_SILU ? silu_mul(gu, act, (int)rows, ff, s) : ff_act(false, gu, act, (int)rows, ff, true, form.act, s, form.limit);
+      if (rc) return rc;
+    }
+    return linear_pair_scatter(g, act, ff, w_down, width, ff, row_pair, wts, parts, s);
+  }
   if (!form.gated) {
     // one projection, activated in the epilogue (on the fp32 sums)
     rc = linear_tc_grouped(xg, width, N, n_tiles, w_gu, experts, ff, width, tile_expert, act, ff, nullptr, nullptr, nullptr, s, form.act);
     if (rc) return rc;
-  } else if (form.act == B200_ACT_SWIGLU_CLAMP && fuse_env && ff % 64 == 0 && (N <= 64 || fuse_env > 1)) {
+  } else if (form.act == B200_ACT_SWIGLU_CLAMP && fuse_env && ff % 64 == 0) {
     // the clamped gate in the same epilogue (it sees the bf16-rounded gate and up values the separate kernel would read)
     rc = linear_tc_grouped_gate_up(xg, width, N, n_tiles, w_gu, experts, ff, width, tile_expert, act, s, form.act, form.limit);
     if (rc) return rc;
@@ -539,10 +578,8 @@ static int moe_experts_tc(const __nv_bfloat16* x, const __nv_bfloat16* w_gu, con
     if (rc) return rc;
     rc = ff_act(false, gu, act, (int)rows, ff, true, form.act, s, form.limit);
     if (rc) return rc;
-  } else if (fuse_env && ff % 64 == 0 && (N <= 64 || fuse_env > 1)) {
-    // gate and up rows of a slab come in as two 64-row boxes; the epilogue activates (as the dense gate|up linear does).
-    // Decode-sized tiles only: at 128 tokens per tile the epilogue's exponentials cost more than the pass they save
-    // (measured: 145 us against 119 + 19 us for 8192 rows of width 2048 into ff 1024)
+  } else if (fuse_env && ff % 64 == 0) {
+    // gate and up rows of a slab come in as two 64-row boxes; the epilogue activates (as the dense gate|up linear does)
     rc = linear_tc_grouped_gate_up(xg, width, N, n_tiles, w_gu, experts, ff, width, tile_expert, act, s);
     if (rc) return rc;
   } else {

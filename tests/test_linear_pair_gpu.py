@@ -68,3 +68,45 @@ def test_gate_up_epilogue_on_pairs_of_sms(abi, T, I, k):
     abi.check(lib.b200_linear_fused_bf16(P(x), k, P(il), None, P(got), I, T, 2 * I, k, 1, None, None, None, None, None, 0, 0, 0, P(ws), wsb, None))
     torch.cuda.synchronize()
     assert torch.equal(got[:T], ref) and torch.isnan(got[T].float()).all()
+
+
+@pytest.mark.parametrize("width,ff,experts,top,rows,gated,weight_input", [
+    (64, 64, 2, 1, 130, True, 0),        # one slab of 64 gate and up rows a pair; runs of whole and part units
+    (264, 192, 5, 2, 400, True, 0),      # odd numbers of slabs, the last k block of 8, an expert without rows
+    (512, 96, 3, 3, 300, True, 0),       # ff not a multiple of 64: gate|up, then the activation on its own
+    (256, 320, 4, 2, 515, False, 0),     # one projection, activated in the epilogue
+    (256, 128, 6, 2, 900, False, 1),     # the mixing weight belongs to the input
+    (128, 128, 1, 1, 1025, True, 0),     # one expert, five tiles
+])
+def test_experts_on_pairs_of_sms(abi, width, ff, experts, top, rows, gated, weight_input):
+    """Routed experts with uneven runs (more than 64 rows in the mean): every (token, slot) row against fp64 from the same bf16 operands.
+
+    The bound: bf16 roundings of gate, up, their activations and product (half a unit, 2^-9, each; silu takes up to twice a gate's for
+    |gate| < 3, relu2 twice), i.e. less than 8 of them on every term of the closing sum."""
+    lib, P = abi.lib(), abi.ptr
+    g = torch.Generator(device="cuda").manual_seed(width + ff + rows)
+    x = torch.randn(rows, width, generator=g, device="cuda").to(BF)
+    wu = (0.5 * width ** -0.5 * torch.randn(experts, (2 if gated else 1) * ff, width, generator=g, device="cuda")).to(BF)
+    wd = (0.05 * torch.randn(experts, width, ff, generator=g, device="cuda")).to(BF)
+    p = torch.arange(1, experts + 1, device="cuda", dtype=torch.float32) ** 2   # uneven loads; expert 1 of many is left out
+    if experts > top + 1:
+        p[1] = 0
+    ids = torch.multinomial(p.expand(rows, experts), top, generator=g).to(torch.int32)
+    wts = torch.rand(rows, top, generator=g, device="cuda")
+    parts = torch.full((rows, top, width), float("nan"), device="cuda")
+    ws = torch.zeros(int(lib.b200_moe_workspace_bytes(rows, top, experts, width, ff)), dtype=torch.uint8, device="cuda")
+    if gated:
+        abi.check(lib.b200_moe_experts(0, P(x), P(wu), P(wd), P(ids), P(wts), rows, width, ff, experts, top, P(parts), P(ws), None))
+    else:
+        abi.check(lib.b200_moe_experts_form(0, P(x), P(wu), P(wd), P(ids), P(wts), rows, width, ff, experts, top, P(parts), P(ws), 0, abi.ACT_RELU2,
+                                            weight_input, None))
+    torch.cuda.synchronize()
+    for e in range(experts):
+        t, j = (ids == e).nonzero(as_tuple=True)
+        xe, w = x[t].double(), wts[t, j, None].double()
+        if weight_input:
+            xe, w = (xe.float() * wts[t, j, None]).to(BF).double(), torch.ones_like(w)
+        u = xe @ wu[e].double().T
+        a = torch.nn.functional.silu(u[:, :ff]) * u[:, ff:] if gated else torch.relu(u) ** 2
+        want, room = (a @ wd[e].double().T) * w, (a.abs() @ wd[e].abs().double().T) * w * 2.0 ** -6
+        assert (parts[t, j].double() - want).abs().le(room + 1e-6).all(), e
