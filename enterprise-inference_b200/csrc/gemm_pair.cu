@@ -12,6 +12,9 @@
 //
 // Against 128 x 256 tiles of single CTAs with k split over clusters (us, before -> now): 2000 tokens, k 14336, 4096 features 179 -> 162; 2048, 4096,
 // 28672 404 -> 321; 2048, 4096, 6144 107 -> 78; 1000, 4096, 4096 62 -> 38; 300, 2048, 2048 22 -> 12; 200, 14336, 4096 50 -> 32; 130, 2048, 2048 19 -> 11.
+// Routed experts (the table of token tiles is moe.cu's): 32 experts of 1024, width 2048, 4 of them a row, router and grouping included, tiles of
+// 128 x 128 before: 2048 rows 263 -> 181, 1000 rows 193 -> 141, 600 rows 165 -> 125; 64 of 512, width 4096, 8 a row, 2048 rows 586 -> 375.  Their
+// weights come from HBM (1000 rows: 402 MB), and whole waves of tiles decide the rest (2048 rows: 5.2 waves of gate|up).
 // 128 tokens and fewer stay on gemm_tc.cu's tiles: their launches stream W, and 148 CTAs with two of them to an SM keep more of it in flight
 // (64 tokens, 4096, 28672: 42 there, 49 here; 128, 14336, 4096: 33 and 34).
 #include <algorithm>
@@ -88,7 +91,7 @@ __device__ __forceinline__ PairTile pair_tile(const TcParams& p, int t) {
     r.m = t % p.pair_m;
     r.expert = e.x;
     r.row0 = e.y;
-    r.n = e.z;
+    r.n = min(max(e.z & ~31, 32), 256);   // (whatever has become of the caller's workspace, never an MMA of an undefined shape)
   } else {             // tokens fast: the tiles in flight share a few slabs and pair_group token tiles
     const int per = p.pair_group * p.pair_m, g = t / per, gs = min(p.pair_group, p.pair_tok - g * p.pair_group), i = t - g * per;
     r.m = i / gs;
@@ -109,7 +112,8 @@ __device__ __forceinline__ void pair_bias(const TcParams& p, int m_tile, int r4,
 
 template <int MODE>
 __global__ void __launch_bounds__(kPairThreads, 1)
-linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const TcParams p, uint32_t* status) {
+linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_rest,
+                   const TcParams p, uint32_t* status) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   float* stg_all = reinterpret_cast<float*>(smem + kPairStages * kPairStageBytes);
@@ -182,7 +186,9 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             pair_load(a, &map_w, kb * kBlockK, w0, bar, kKeepNormal);
           }
           if (p.pair_tile) {
-            for (int r = 0; r < half; r += 16) pair_load(a + kPairABytes + r * 128, &map_x, kb * kBlockK, x0 + r, bar, kKeepLast);
+            int r = 0;
+            for (; r + 64 <= half; r += 64) pair_load(a + kPairABytes + r * 128, &map_x, kb * kBlockK, x0 + r, bar, kKeepLast);
+            for (; r < half; r += 16) pair_load(a + kPairABytes + r * 128, &map_rest, kb * kBlockK, x0 + r, bar, kKeepLast);
           } else {
             pair_load(a + kPairABytes, &map_x, kb * kBlockK, x0, bar, kKeepLast);
           }
@@ -335,10 +341,10 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 }
 
 template <int MODE>
-int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const TcParams& p, int clusters, cudaStream_t s) {
+int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mr, const TcParams& p, int clusters, cudaStream_t s) {
   static bool attr_set[64] = {};
   B200_CUDA(ensure_dynamic_smem(linear_pair_kernel<MODE>, kPairSmem, attr_set));
-  B200_CUDA(launch_cluster(linear_pair_kernel<MODE>, dim3(clusters * 2 * p.splits), dim3(kPairThreads), (size_t)kPairSmem, s, dim3(2 * p.splits, 1, 1), mw, mx, p, wait_status_word()));
+  B200_CUDA(launch_cluster(linear_pair_kernel<MODE>, dim3(clusters * 2 * p.splits), dim3(kPairThreads), (size_t)kPairSmem, s, dim3(2 * p.splits, 1, 1), mw, mx, mr, p, wait_status_word()));
   return B200_OK;
 }
 
@@ -377,10 +383,10 @@ int linear_pair(int mode, TcParams p, const __nv_bfloat16* x, int64_t ldx, const
   if (rc) return rc;
   const int clusters = (int)std::min<int64_t>((int64_t)p.pair_tok * p.pair_m, kNumSMs / 2);
   switch (mode) {
-    case kScatter: return launch_pair<kScatter>(mw, mx, p, clusters, s);
-    case kSiluMul: return launch_pair<kSiluMul>(mw, mx, p, clusters, s);
-    case kRopeKv: return launch_pair<kRopeKv>(mw, mx, p, clusters, s);
-    default: return launch_pair<kPlain>(mw, mx, p, clusters, s);
+    case kScatter: return launch_pair<kScatter>(mw, mx, mx, p, clusters, s);
+    case kSiluMul: return launch_pair<kSiluMul>(mw, mx, mx, p, clusters, s);
+    case kRopeKv: return launch_pair<kRopeKv>(mw, mx, mx, p, clusters, s);
+    default: return launch_pair<kPlain>(mw, mx, mx, p, clusters, s);
   }
 }
 
@@ -394,16 +400,18 @@ static int launch_grouped_pair(int mode, TcParams p, const GroupedPairs& g, cons
   p.n_kblocks = (k + kBlockK - 1) / kBlockK;
   p.splits = 1;
   p.pair_tile = g.tiles;
-  CUtensorMap mw, mx;
+  CUtensorMap mw, mx, mr;
   int rc = get_tensor_map_2d(w, (uint64_t)g.experts * p.n_out, (uint64_t)k, (uint64_t)k, (uint32_t)w_box, &mw);
   if (rc) return rc;
-  rc = get_tensor_map_2d(x, (uint64_t)g.rows, (uint64_t)k, (uint64_t)ldx, 16, &mx);   // tiles of any number of units
+  rc = get_tensor_map_2d(x, (uint64_t)g.rows, (uint64_t)k, (uint64_t)ldx, 64, &mx);   // a CTA's rows of a tile: any multiple of 16
+  if (rc) return rc;
+  rc = get_tensor_map_2d(x, (uint64_t)g.rows, (uint64_t)k, (uint64_t)ldx, 16, &mr);
   if (rc) return rc;
   const int clusters = (int)std::min<int64_t>((int64_t)g.max_tiles * p.pair_m, kNumSMs / 2);
   switch (mode) {
-    case kScatter: return launch_pair<kScatter>(mw, mx, p, clusters, s);
-    case kSiluMul: return launch_pair<kSiluMul>(mw, mx, p, clusters, s);
-    default: return launch_pair<kPlain>(mw, mx, p, clusters, s);
+    case kScatter: return launch_pair<kScatter>(mw, mx, mr, p, clusters, s);
+    case kSiluMul: return launch_pair<kSiluMul>(mw, mx, mr, p, clusters, s);
+    default: return launch_pair<kPlain>(mw, mx, mr, p, clusters, s);
   }
 }
 
