@@ -21,6 +21,8 @@
 // delta_prep then takes the decay's pre-activation straight from the fused row (one column per head, decay_dim 1) instead of a
 // second-step projection.  DELTA false drops the correction: u = beta v, which is the state-space recurrence
 // S = g S + dt B x^T, y = S^T C of ssd.cu with keys B, queries C, values x and beta = dt.
+#include <algorithm>
+
 #include "common.cuh"
 #include "f32x2.cuh"
 
@@ -300,261 +302,470 @@ __global__ void __launch_bounds__(kDsThreads) delta_scan_kernel(const ScanArgs a
   constexpr int ROW = ds_row(NP), BUF = ds_buf(NP, CHAN);
   pdl_wait();
   pdl_launch_dependents();
+#define DS_SYNC() __syncthreads()
+#include "delta_walk.cuh"
+#undef DS_SYNC
+}
+// the same by the first kDsThreads threads of a larger CTA
+template <int NP, bool DELTA, bool CHAN>
+__device__ __forceinline__ void ds_walk(const ScanArgs& a, float* stage) {
+  constexpr int ROW = ds_row(NP), BUF = ds_buf(NP, CHAN);
+#define DS_SYNC() asm volatile("bar.sync 1, 128;" ::: "memory")
+#include "delta_walk.cuh"
+#undef DS_SYNC
+}
+
+// Portions of several rows in blocks of eight.  With L_i the product of the decays up to row i of a block, u the corrected values and S the state before it
+//   u_i = b_i (v_i - S^T (L_i k_i) - sum_{j<i} (k_i . (L_i / L_j) k_j) u_j)
+//   o_i = S^T (L_i q_i) + sum_{j<=i} (q_i . (L_i / L_j) k_j) u_j          S' = L_8 S + sum_j (L_8 / L_j) k_j u_j^T
+// so with w_i = b_i (v_i - S^T (L_i k_i)) the rows of a block meet in two 8 x 8 triangles that depend on its inputs alone: u = T w, o = S^T (L q) + B w
+// (the ratios are products of the decays between the rows: nothing is divided, a decay may be 0).
+// A CTA per (sequence, head, 16 value columns), those of a head in clusters.  Its main warps own four columns per LG lanes and reduce a block's sums over
+// these lanes together (a lane keeps half of what it holds at every step); two warps turn the rows of the blocks ahead into L q, L k and
+// (L_8 / L) k; one or two work out the triangles of every C-th block for the C CTAs of the cluster, a round of blocks ahead.
+// LG 32 (four main warps) while one or two CTAs an SM are enough, LG 16 (two warps, a third fewer instructions a column) for three.
+// What bounds them: a block's chain of about 2 300 cycles (dots 840, their reduction 560, triangles and u 500, update 210, waiting for the
+// cluster 230), and issue slots where CTAs share an SM: a shuffle takes four cycles of a scheduler, a packed fma two.
+// Against the walk (us, 16 heads of 128 x 128, channel decays): one sequence of 1 900 rows 406 -> 295, of 950 205 -> 152, two of 1 000 together
+// 182 -> 167, three of 1 900 295 -> 248; one decay per head 228 -> 146; keys of 64 216 -> 125; 150 rows 37 -> 31.  The walk keeps short portions (a
+// block needs its triangles before it starts, about 5 us), the uncorrected rule (in CTAs of 32 columns three sequences of 64 heads 282 -> 251, but
+// four short ones 11 -> 17) and what would fill the device more than once.
+constexpr int kDbRows = 8, kDbScale = 2, kDbSlots = 4, kDbCluster = 4;   // (clusters of eight such CTAs do not fit the device sixteen at a time)
+constexpr int kDbTri = 2 * kDbRows * kDbRows;   // T, B
+constexpr int db_main(int lg) { return lg == 32 ? 4 : 2; }   // warps with columns; warps that work out triangles
+constexpr int db_tri_warps(int lg) { return lg == 32 ? 2 : 1; }
+constexpr int db_threads(int lg) { return (db_main(lg) + kDbScale + db_tri_warps(lg)) * 32; }
+// rows from which a portion goes in blocks: where the two meet for one sequence, and for two to four
+constexpr int db_from(int lg) { return lg == 32 ? 64 : 128; }
+// floats of a slot: L q | L k | (L_8 / L) k, L_8
+__host__ __device__ constexpr int db_slot(int np) { return (3 * kDbRows + 1) * ds_row(np); }
+// slots; three rounds of triangles; per main warp 8 x 8 pairs (u, u)
+constexpr int db_floats(int np, int lg) { return kDbSlots * db_slot(np) + 3 * db_tri_warps(lg) * kDbCluster * kDbTri + db_main(lg) * kDbRows * 16; }
+template <int N>
+__device__ __forceinline__ void db_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(N) : "memory"); }
+template <int N>
+__device__ __forceinline__ void db_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(N) : "memory"); }
+__device__ __forceinline__ void db_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void db_cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }   // (nothing to show)
+__device__ __forceinline__ void db_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// The sum over the warp of value i of 32, to lane i.
+__device__ __forceinline__ float db_reduce(float (&x)[32], int lane) {
+#pragma unroll
+  for (int half = 16; half >= 1; half >>= 1) {
+    const bool up = (lane & half) != 0;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const float keep = up ? x[i + half] : x[i], give = up ? x[i] : x[i + half];
+      x[i] = keep + __shfl_xor_sync(0xffffffffu, give, half);
+    }
+  }
+  return x[0];
+}
+
+// One step of the sums over a group of lanes: 2 H values become H, the lane keeps one half of them and hands over the other.
+template <int H>
+__device__ __forceinline__ void db_halve(float* x, int lane) {
+  const bool up = (lane & H) != 0;
+#pragma unroll
+  for (int i = 0; i < H; ++i) {
+    const float keep = up ? x[i + H] : x[i], give = up ? x[i] : x[i + H];
+    x[i] = keep + __shfl_xor_sync(0xffffffffu, give, H);
+  }
+}
+
+template <int NP, bool CHAN, int LG, int CTAS>
+__global__ void __launch_bounds__(db_threads(LG), CTAS) delta_block_kernel(const ScanArgs a) {
+  extern __shared__ __align__(16) float stage[];
+  constexpr int ROW = ds_row(NP), R = kDbRows, SLOT = db_slot(NP), MAIN = db_main(LG), BAR = 32 * (MAIN + 1);   // BAR: threads of the main warps and one other
+  constexpr int kFull = 1, kEmpty = 1 + kDbSlots;   // named barriers: slot ready; slot read
+  static_assert(NP <= 2, "a preparing lane's channels are one piece of at most 16 bytes");
+  pdl_wait();
+  pdl_launch_dependents();
   const int s = blockIdx.x, h = blockIdx.y, jb = blockIdx.z * kDsCols;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int start = a.seq_start[s], n_rows = a.seq_start[s + 1] - start;
   if (n_rows <= 0) return;
-  const bool fresh = a.positions[start] == 0;
   const int g = h / (a.heads / a.kv_heads), dim = a.dim, vd = a.vd;
-  const int j0 = jb + warp * 4;   // the warp's first value column
-  float* S_st = a.state + (int64_t)a.seq_slots[s] * a.slot_stride + ((int64_t)h * vd + j0) * dim;
+  const bool fresh = a.positions[start] == 0;
   const int64_t qk = (int64_t)a.kv_heads * dim, hv = (int64_t)a.heads * vd;
   const float* qsrc = a.qn + (int64_t)start * qk + (int64_t)g * dim;
   const float* ksrc = a.kn + (int64_t)start * qk + (int64_t)g * dim;
   const float* gsrc = a.decay + (int64_t)start * a.g_row + (int64_t)h * a.g_head;
   const float* vsrc = a.vn + (int64_t)start * hv + (int64_t)h * vd + jb;
   const float* bsrc = a.beta + (int64_t)start * a.heads + h;
-  uint64_t S[4][NP];
+  float* out = a.out + (int64_t)start * hv + (int64_t)h * vd + jb;
+  float* state = a.state + (int64_t)a.seq_slots[s] * a.slot_stride + ((int64_t)h * vd + jb) * dim;
+  if (n_rows < db_from(LG)) {
+    if (warp < kDsWarps) ds_walk<NP, true, CHAN>(a, stage);
+    return;
+  }
+  const int n_blocks = (n_rows + R - 1) / R;
+  uint32_t C, rank;   // CTAs of the cluster, all of one sequence and head
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(C));
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const int per_round = db_tri_warps(LG) * (int)C, rounds = (n_blocks + per_round - 1) / per_round;
+  float* tris = stage + kDbSlots * SLOT;   // [3][blocks of a round][T | B]
+  // cluster barriers: all CTAs run; then, for every round p, its triangles are there and those of round p - 2 have been read (arrived at a round ahead)
+  db_cluster_arrive_relaxed();
+
+  if (warp >= MAIN + kDbScale) {
+    // ===== triangles: lane l takes the sums of the pair (pi, pj), 28 below the diagonal row by row; lanes from 28 on the diagonal's halves =====
+    int pi = 1;
+    while (pi < R - 1 && lane >= (pi + 1) * pi / 2) ++pi;
+    const int d = 2 * NP * lane;
+    db_cluster_wait();
+    for (int p = 0; p < rounds; ++p) {
+      const int mine = (warp - MAIN - kDbScale) * (int)C + (int)rank, b = p * per_round + mine;
+      if (b < n_blocks) {
+        const int nb = min(n_rows - b * R, R);
+        auto pair = [&](const float* src, int64_t st, int r, int i, uint64_t none) {
+          return r < nb && d < dim ? *reinterpret_cast<const uint64_t*>(src + (int64_t)(b * R + r) * st + d + 2 * i) : none;
+        };
+        const float bs = lane < nb ? bsrc[(int64_t)(b * R + lane) * a.heads] : 0.f, gs = !CHAN && lane < nb ? gsrc[(int64_t)(b * R + lane) * a.g_row] : 1.f;
+        float x[2][32];   // k with k and the diagonal's first half; q with k and its second
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {   // channels in NP passes, for the registers
+          uint64_t k[R], g[R], q[R];
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            k[r] = pair(ksrc, qk, r, i, 0);
+            q[r] = pair(qsrc, qk, r, i, 0);
+            g[r] = CHAN ? pair(gsrc, a.g_row, r, i, f2::both(1.f)) : f2::both(__shfl_sync(0xffffffffu, gs, r));
+          }
+          auto add = [&](float& to, uint64_t a, uint64_t b) {
+            const float sum = f2::sum(f2::mul(a, b));
+            to = i ? to + sum : sum;
+          };
+#pragma unroll
+          for (int j = 0; j < R - 1; ++j) {
+            uint64_t z = k[j];
+#pragma unroll
+            for (int r = j + 1; r < R; ++r) {
+              z = f2::mul(z, g[r]);
+              add(x[0][r * (r - 1) / 2 + j], z, k[r]);
+              add(x[1][r * (r - 1) / 2 + j], z, q[r]);
+            }
+          }
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            add(x[0][28 + r], k[r], q[r]);
+            add(x[1][28 + r], k[4 + r], q[4 + r]);
+          }
+        }
+        const float kk = db_reduce(x[0], lane), qq = db_reduce(x[1], lane);
+        // T = (1 + diag(b) (k with k))^-1 and B = (q with k) T, a column a lane
+        float* tri = tris + (p % 3 * per_round + mine) * kDbTri;
+        float t[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) t[i] = lane == i ? 1.f : 0.f;
+        const float bl = __shfl_sync(0xffffffffu, bs, pi) * kk;
+#pragma unroll
+        for (int m = 0; m < R - 1; ++m)
+#pragma unroll
+          for (int i = m + 1; i < R; ++i) {
+            const float c = __shfl_sync(0xffffffffu, bl, i * (i - 1) / 2 + m);
+            if (lane <= m) t[i] = fmaf(-c, t[m], t[i]);   // (not beyond the column's first row: there is nothing to multiply)
+          }
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          const float c = __shfl_sync(0xffffffffu, i < 4 ? kk : qq, 28 + (i & 3));
+          float y = lane <= i ? c * t[i] : 0.f;
+#pragma unroll
+          for (int m = 0; m < i; ++m) {
+            const float e = __shfl_sync(0xffffffffu, qq, i * (i - 1) / 2 + m);
+            if (lane <= m) y = fmaf(e, t[m], y);
+          }
+          if (lane < R) {
+            tri[i * R + lane] = t[i];
+            tri[(R + i) * R + lane] = y;
+          }
+        }
+        __syncwarp();
+        const float4 quad = *reinterpret_cast<const float4*>(tri + 4 * lane);
+        for (uint32_t c = 0; c < C; ++c) {
+          if (c == rank) continue;
+          uint32_t to;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"((uint32_t)__cvta_generic_to_shared(tri + 4 * lane)), "r"(c));
+          asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to), "f"(quad.x), "f"(quad.y), "f"(quad.z), "f"(quad.w) : "memory");
+        }
+      }
+      db_cluster_arrive();
+      db_cluster_wait();
+    }
+    return;
+  }
+
+  if (warp >= MAIN) {
+    // ===== rows times their decays: a warp a block, a lane NP neighbouring pairs of channels =====
+    const int w = warp - MAIN, d = 2 * NP * lane;
+    const bool live = d < dim;
+    auto store = [&](float* row, const uint64_t (&x)[NP]) {
+      if constexpr (NP == 1) *reinterpret_cast<uint64_t*>(row + d) = x[0];
+      else *reinterpret_cast<ulonglong2*>(row + d) = make_ulonglong2(x[0], x[1]);
+    };
+    uint64_t k[R][NP], q[R][NP], gg[R][NP];
+    float gs = 1.f;   // of row `lane`
+    auto fetch = [&](int b) {   // channels beyond dim and rows past the last one: no weight, no decay
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int64_t t = (int64_t)b * R + r;
+        const bool there = live && t < n_rows;
+        auto get = [&](const float* p, uint64_t none, uint64_t (&x)[NP]) {
+#pragma unroll
+          for (int i = 0; i < NP; ++i) x[i] = none;
+          if (!there) return;
+          if constexpr (NP == 1) {
+            x[0] = *reinterpret_cast<const uint64_t*>(p + d);
+          } else {
+            const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(p + d);
+            x[0] = y.x;
+            x[1] = y.y;
+          }
+        };
+        get(qsrc + t * qk, 0, q[r]);
+        get(ksrc + t * qk, 0, k[r]);
+        if (CHAN) get(gsrc + t * a.g_row, f2::both(1.f), gg[r]);
+      }
+      if (!CHAN) gs = lane < R && b * R + lane < n_rows ? gsrc[(int64_t)(b * R + lane) * a.g_row] : 1.f;
+    };
+    if (w < n_blocks) fetch(w);
+    db_cluster_wait();
+    db_cluster_arrive_relaxed();
+    int round = 0;   // whose barrier this warp has arrived at
+    for (int b = w; b < n_blocks; b += kDbScale) {
+      while (b >= (round + 1) * per_round) {
+        db_cluster_wait();
+        db_cluster_arrive_relaxed();
+        ++round;
+      }
+      if (b >= kDbSlots) db_sync<BAR>(kEmpty + b % kDbSlots);   // block b - kDbSlots has been read
+      float* slot = stage + (b % kDbSlots) * SLOT;
+      uint64_t L[NP], rest[NP], x[NP];
+      if (!CHAN) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const uint64_t y = f2::both(__shfl_sync(0xffffffffu, gs, r));
+#pragma unroll
+          for (int i = 0; i < NP; ++i) gg[r][i] = y;
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+#pragma unroll
+        for (int i = 0; i < NP; ++i) L[i] = r ? f2::mul(L[i], gg[r][i]) : gg[0][i];
+#pragma unroll
+        for (int i = 0; i < NP; ++i) x[i] = f2::mul(q[r][i], L[i]);
+        store(slot + r * ROW, x);
+#pragma unroll
+        for (int i = 0; i < NP; ++i) x[i] = f2::mul(k[r][i], L[i]);
+        store(slot + (R + r) * ROW, x);
+      }
+      store(slot + 3 * R * ROW, L);
+#pragma unroll
+      for (int r = R - 1; r >= 0; --r) {
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+          x[i] = r == R - 1 ? k[r][i] : f2::mul(k[r][i], rest[i]);
+          rest[i] = r == R - 1 ? gg[r][i] : f2::mul(rest[i], gg[r][i]);
+        }
+        store(slot + (2 * R + r) * ROW, x);
+      }
+      __syncwarp();
+      db_arrive<BAR>(kFull + b % kDbSlots);
+      if (b + kDbScale < n_blocks) fetch(b + kDbScale);
+    }
+    while (++round < rounds) {
+      db_cluster_wait();
+      db_cluster_arrive_relaxed();
+    }
+    db_cluster_wait();
+    return;
+  }
+
+  // ===== LG lanes four columns, a lane x of them the channels 4 x + 4 LG v =====
+  constexpr int CW = 128 / LG, V = ROW / (4 * LG);   // columns of a warp; pieces of four channels a lane
+  const int xl = lane & (LG - 1), x16 = lane & 15, grp = lane / LG, j0 = warp * CW + grp * 4, cols = min(vd - jb - j0, 4);
+  float* us = tris + 3 * db_tri_warps(LG) * kDbCluster * kDbTri + warp * R * 16;   // [8 rows][CW columns] pairs (u, u)
+  uint64_t S[4][2 * V];
+  float* S_st = state + (int64_t)j0 * dim;
 #pragma unroll
   for (int c = 0; c < 4; ++c)
 #pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      const int d = ds_chan<NP>(lane, i);
-      const float* p = S_st + (int64_t)c * dim + d;
-      S[c][i] = 0;
-      if (!fresh && j0 + c < vd && d < dim) S[c][i] = a.vec ? *reinterpret_cast<const uint64_t*>(p) : f2::pack(p[0], d + 1 < dim ? p[1] : 0.f);
+    for (int i = 0; i < V; ++i) {
+      const int d = 4 * xl + 4 * LG * i;
+      ulonglong2 y = make_ulonglong2(0, 0);
+      if (!fresh && c < cols && d < dim) y = *reinterpret_cast<const ulonglong2*>(S_st + (int64_t)c * dim + d);
+      S[c][2 * i] = y.x;
+      S[c][2 * i + 1] = y.y;
     }
-  if (n_rows == 1) {
-    // a decode row: nothing to stage; the row's inputs are fetched beside the state
-    const float b = bsrc[0], gs = CHAN ? 0.f : gsrc[0];
-    uint64_t k[NP], q[NP];
-    float d4[4] = {0.f, 0.f, 0.f, 0.f}, o4[4];
+  // the lane's two places in a block's small sums: rows rr and rr + 4 of one of its half's columns
+  const int rr = x16 >> 2, col = x16 & 3, from = grp * 16 + col;
+  const bool have = col < cols;
+  float v[2], bt[2];
+  auto fetch_v = [&](int b) {
 #pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      const int d = ds_chan<NP>(lane, i);
-      auto pair = [&](const float* p, int64_t st) { return f2::pack(d < dim ? p[d * st] : 0.f, d + 1 < dim ? p[(d + 1) * st] : 0.f); };
-      k[i] = pair(ksrc, 1);
-      q[i] = pair(qsrc, 1);
-      const uint64_t gg = CHAN ? pair(gsrc, a.g_chan) : f2::both(gs);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) S[c][i] = f2::mul(S[c][i], gg);
+    for (int i = 0; i < 2; ++i) {
+      const int64_t t = (int64_t)b * R + rr + 4 * i;
+      const bool ok = t < n_rows;
+      v[i] = ok && have ? vsrc[t * hv + j0 + col] : 0.f;
+      bt[i] = ok ? bsrc[t * a.heads] : 0.f;
     }
-    if (DELTA) {
+  };
+  auto row_of = [&](const float* row, uint64_t (&y)[2 * V]) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint64_t acc = f2::mul(S[c][0], k[0]);
-#pragma unroll
-        for (int i = 1; i < NP; ++i) acc = f2::fma(S[c][i], k[i], acc);
-        d4[c] = f2::sum(acc);
-      }
-      ds_reduce<4>(d4, lane);
+    for (int i = 0; i < V; ++i) {
+      const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(row + 4 * xl + 4 * LG * i);
+      y[2 * i] = t.x;
+      y[2 * i + 1] = t.y;
     }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const uint64_t u = f2::both(b * ((j0 + c < vd ? vsrc[warp * 4 + c] : 0.f) - d4[c]));
-      uint64_t acc = 0;
-#pragma unroll
-      for (int i = 0; i < NP; ++i) {
-        S[c][i] = f2::fma(k[i], u, S[c][i]);
-        acc = f2::fma(S[c][i], q[i], acc);
-      }
-      o4[c] = f2::sum(acc);
+  };
+  fetch_v(0);
+  db_cluster_wait();
+  db_cluster_arrive_relaxed();
+  int in_round = per_round - 1, round = -1;   // block of the round, the round
+  for (int b = 0; b < n_blocks; ++b) {
+    if (++in_round == per_round) {
+      in_round = 0;
+      db_cluster_wait();
+      if (++round + 1 < rounds) db_cluster_arrive_relaxed();
     }
-    ds_reduce<4>(o4, lane);
-    const float mine = lane == 0 ? o4[0] : lane == 1 ? o4[1] : lane == 2 ? o4[2] : o4[3];
-    if (lane < 4 && j0 + lane < vd) a.out[(int64_t)start * hv + (int64_t)h * vd + j0 + lane] = mine;
-  } else {
-    float* kq = stage + 2 * BUF;                                          // [kDsStage] per pair of rows: k1 g2 k2, k1 . q1
-    float* part = kq + kDsStage + warp * kDsFlush * kDsPartRow;
-    if (dim < ROW) {   // zeros beyond dim, once: the copies leave them alone
-      for (int e = tid; e < 2 * BUF; e += kDsThreads) stage[e] = 0.f;
-      __syncthreads();
-    }
-    auto fetch = [&](int b0, float* buf) {
-      const int nb = min(kDsStage, n_rows - b0);
-      float* sq = buf;
-      float* sk = sq + kDsStage * ROW;
-      float* sg = sk + kDsStage * ROW;
-      float* sv = sq + kDsStage * (CHAN ? 3 : 2) * ROW;
-      float* sb = sv + kDsStage * kDsCols;
-      if (a.vec) {
+    db_sync<BAR>(kFull + b % kDbSlots);
+    const float* in = stage + (b % kDbSlots) * SLOT;
+    const float* tri = tris + (round % 3 * per_round + in_round) * kDbTri + rr * R;
+    float m[2][3][4];   // T and B: row rr up to column 3, row rr + 4
+    auto triangles = [&]() {
 #pragma unroll
-        for (int e0 = 0; e0 < kDsStage * ROW / 4; e0 += kDsThreads) {
-          const int e = e0 + tid, r = e / (ROW / 4), c = (e % (ROW / 4)) * 4;
-          if (r < nb && c < dim) {
-            f2::cp16(sq + r * ROW + c, qsrc + (b0 + r) * qk + c);
-            f2::cp16(sk + r * ROW + c, ksrc + (b0 + r) * qk + c);
-            if (CHAN) f2::cp16(sg + r * ROW + c, gsrc + (b0 + r) * a.g_row + c);
-          }
+      for (int z = 0; z < 2; ++z)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const float4 e = *reinterpret_cast<const float4*>(tri + z * R * R + (i ? 4 * R + 4 * (i - 1) : 0));
+          m[z][i][0] = e.x, m[z][i][1] = e.y, m[z][i][2] = e.z, m[z][i][3] = e.w;
         }
-      } else {
-        for (int e = tid; e < kDsStage * ROW; e += kDsThreads) {
-          const int r = e / ROW, c = e % ROW;
-          if (r < nb && c < dim) {
-            f2::cp4(sq + r * ROW + c, qsrc + (b0 + r) * qk + c);
-            f2::cp4(sk + r * ROW + c, ksrc + (b0 + r) * qk + c);
-            if (CHAN) f2::cp4(sg + r * ROW + c, gsrc + (b0 + r) * a.g_row + (int64_t)c * a.g_chan);
-          }
-        }
-      }
-#pragma unroll
-      for (int e0 = 0; e0 < kDsStage * kDsCols; e0 += kDsThreads) {
-        const int e = e0 + tid, r = e / kDsCols, c = e % kDsCols;
-        if (r < nb && jb + c < vd) f2::cp4(sv + e, vsrc + (b0 + r) * hv + c);
-      }
-      if (tid < nb) {
-        f2::cp4(sb + tid, bsrc + (int64_t)(b0 + tid) * a.heads);
-        if (!CHAN) f2::cp4(sb + kDsStage + tid, gsrc + (b0 + tid) * a.g_row);
-      }
     };
-    fetch(0, stage);
-    for (int b0 = 0, it = 0; b0 < n_rows; b0 += kDsStage, ++it) {
-      const int nb = min(kDsStage, n_rows - b0);
-      const float* sq = stage + (it & 1) * BUF;
-      const float* sk = sq + kDsStage * ROW;
-      const float* sg = sk + kDsStage * ROW;
-      const float* sv = sq + kDsStage * (CHAN ? 3 : 2) * ROW + warp * 4;
-      const float* sb = sv - warp * 4 + kDsStage * kDsCols;
-      f2::cp_wait_all();
-      __syncthreads();   // the stage has landed for everybody, and the one before has been consumed
-      if (b0 + kDsStage < n_rows) fetch(b0 + kDsStage, stage + ((it + 1) & 1) * BUF);
-      if (DELTA) {
-        for (int r = 2 * warp; r + 1 < nb; r += 2 * kDsWarps) {
-          float xy[2] = {0.f, 0.f};
+    // sets of four rows times four columns: of L k (rows 0..3, 4..7), of L q.  JOINT sets are reduced together, a step of one covers the others' latency
+    constexpr int JOINT = LG == 32 ? 4 : 2;
+    float sum[2][2];   // of L k, of L q; of rows rr and rr + 4
 #pragma unroll
-          for (int d = 0; d < ROW; d += 32) {
-            const float k1 = sk[r * ROW + d + lane], k2 = sk[(r + 1) * ROW + d + lane];
-            xy[0] = fmaf(CHAN ? k1 * sg[(r + 1) * ROW + d + lane] : k1, k2, xy[0]);
-            xy[1] = fmaf(k1, sq[r * ROW + d + lane], xy[1]);
-          }
-          ds_reduce<2>(xy, lane);
-          if (lane == 0) *reinterpret_cast<float2*>(kq + r) = make_float2(CHAN ? xy[0] : xy[0] * sb[kDsStage + r + 1], xy[1]);
-        }
-        __syncthreads();
-      }
-      auto decay_row = [&](const uint64_t (&gg)[NP]) {
+    for (int s0 = 0; s0 < 4; s0 += JOINT) {
+      float part[JOINT][16];
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+      for (int s1 = 0; s1 < JOINT; ++s1) {
+        const int set = s0 + s1;
+        uint64_t y[4][2 * V];
 #pragma unroll
-          for (int i = 0; i < NP; ++i) S[c][i] = f2::mul(S[c][i], gg[i]);
-      };
-      auto decays = [&](int r, uint64_t (&gg)[NP]) {
-        if (CHAN) {
-          ds_pairs<NP>(sg + r * ROW, lane, gg);
-        } else {
-          const uint64_t x = f2::both(sb[kDsStage + r]);
+        for (int r = 0; r < 4; ++r) row_of(in + ((set < 2 ? R : 0) + 4 * (set & 1) + r) * ROW, y[r]);
 #pragma unroll
-          for (int i = 0; i < NP; ++i) gg[i] = x;
-        }
-      };
-      auto dots = [&](const uint64_t (&x)[NP], float* o) {   // the lane's part of S^T x for the four columns
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint64_t acc = f2::mul(S[c][0], x[0]);
-#pragma unroll
-          for (int i = 1; i < NP; ++i) acc = f2::fma(S[c][i], x[i], acc);
-          o[c] = f2::sum(acc);
-        }
-      };
-      int r = 0;
-      for (int f0 = 0; f0 < nb; f0 += kDsFlush) {
-      const int f1 = min(f0 + kDsFlush, nb);
-      if (DELTA) {
-        for (; r + 1 < f1; r += 2) {
-          uint64_t g1[NP], g2[NP], k1[NP], k2[NP], q1[NP], q2[NP];
-          decays(r, g1);
-          ds_pairs<NP>(sk + r * ROW, lane, k1);
-          decays(r + 1, g2);
-          ds_pairs<NP>(sk + (r + 1) * ROW, lane, k2);
-          ds_pairs<NP>(sq + r * ROW, lane, q1);
-          ds_pairs<NP>(sq + (r + 1) * ROW, lane, q2);
-          const float4 v1 = *reinterpret_cast<const float4*>(sv + r * kDsCols), v2 = *reinterpret_cast<const float4*>(sv + (r + 1) * kDsCols);
-          const float2 bb = *reinterpret_cast<const float2*>(sb + r), kk = *reinterpret_cast<const float2*>(kq + r);
-          float d[8], o1[4], o2[4];
-          decay_row(g1);
-          dots(k1, d);
-          dots(q1, o1);
-          decay_row(g2);
-          dots(k2, d + 4);
-          ds_reduce<8>(d, lane);
-          const float va[4] = {v1.x, v1.y, v1.z, v1.w}, vb[4] = {v2.x, v2.y, v2.z, v2.w};
-          uint64_t kg[NP];
-#pragma unroll
-          for (int i = 0; i < NP; ++i) kg[i] = f2::mul(k1[i], g2[i]);
+        for (int r = 0; r < 4; ++r)
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            const float u1 = bb.x * (va[c] - d[c]), u2 = bb.y * (vb[c] - fmaf(kk.x, u1, d[4 + c]));
-            if (lane == 0) o1[c] = fmaf(kk.y, u1, o1[c]);
-            const uint64_t w1 = f2::both(u1), w2 = f2::both(u2);
+            uint64_t acc = f2::mul(S[c][0], y[r][0]);
 #pragma unroll
-            for (int i = 0; i < NP; ++i) S[c][i] = f2::fma(k2[i], w2, f2::fma(kg[i], w1, S[c][i]));
+            for (int i = 1; i < 2 * V; ++i) acc = f2::fma(S[c][i], y[r][i], acc);
+            part[s1][4 * r + c] = f2::sum(acc);
           }
-          dots(q2, o2);
-          *reinterpret_cast<float4*>(part + (r - f0) * kDsPartRow + 4 * lane) = make_float4(o1[0], o1[1], o1[2], o1[3]);
-          *reinterpret_cast<float4*>(part + (r + 1 - f0) * kDsPartRow + 4 * lane) = make_float4(o2[0], o2[1], o2[2], o2[3]);
-        }
       }
-#pragma unroll 2
-      for (; r < f1; ++r) {
-        uint64_t gg[NP], k[NP], q[NP];
-        decays(r, gg);
-        ds_pairs<NP>(sk + r * ROW, lane, k);
-        ds_pairs<NP>(sq + r * ROW, lane, q);
-        const float4 v4 = *reinterpret_cast<const float4*>(sv + r * kDsCols);
-        const float va[4] = {v4.x, v4.y, v4.z, v4.w}, b = sb[r];
-        float d[4] = {0.f, 0.f, 0.f, 0.f}, o[4];
-        decay_row(gg);
-        if (DELTA) {
-          dots(k, d);
-          ds_reduce<4>(d, lane);
-        }
+      auto all = [&](auto&& f) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const uint64_t u = f2::both(b * (va[c] - d[c]));
+        for (int s1 = 0; s1 < JOINT; ++s1) f(part[s1]);
+      };
+      all([&](float* x) { db_halve<8>(x, lane); });
+      if (s0 + JOINT == 4) triangles();
+      all([&](float* x) { db_halve<4>(x, lane); });
+      all([&](float* x) { db_halve<2>(x, lane); });
+      all([&](float* x) { db_halve<1>(x, lane); });
 #pragma unroll
-          for (int i = 0; i < NP; ++i) S[c][i] = f2::fma(k[i], u, S[c][i]);
-        }
-        dots(q, o);
-        *reinterpret_cast<float4*>(part + (r - f0) * kDsPartRow + 4 * lane) = make_float4(o[0], o[1], o[2], o[3]);
-      }
-      __syncwarp();
-      {   // four lanes a row, eight lanes' sums each
-        const int rr = lane >> 2, quarter = lane & 3;
-        const float* src = part + rr * kDsPartRow + quarter * 32;
-        uint64_t x = 0, y = 0;
+      for (int s1 = 0; s1 < JOINT; ++s1)
+        sum[(s0 + s1) >> 1][s1 & 1] = part[s1][0] + (LG == 32 ? __shfl_xor_sync(0xffffffffu, part[s1][0], 16) : 0.f);
+    }
+    const float w[2] = {bt[0] * (v[0] - sum[0][0]), bt[1] * (v[1] - sum[0][1])};
+    fetch_v(b + 1);
+    // u = T w, o = S^T (L q) + B w: the rows up to the lane's own
+    float y[2][2] = {{0.f, 0.f}, {sum[1][0], sum[1][1]}};
+    uint64_t G[2 * V], kx[LG == 32 ? R : 1][2 * V];   // (a lane of 32 has room for the rows that the update takes)
+    row_of(in + 3 * R * ROW, G);
+    if (LG == 32) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(src + 4 * (i ^ quarter));   // (the four lanes' banks apart)
-          x = f2::add(x, t.x);
-          y = f2::add(y, t.y);
-        }
-        float o[4] = {f2::lo(x), f2::hi(x), f2::lo(y), f2::hi(y)};
+      for (int r = 0; r < R; ++r) row_of(in + (2 * R + r) * ROW, kx[r]);
+    }
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          o[c] += __shfl_xor_sync(0xffffffffu, o[c], 1);
-          o[c] += __shfl_xor_sync(0xffffffffu, o[c], 2);
+    for (int j = 0; j < R; ++j) {
+      const float wj = __shfl_sync(0xffffffffu, w[j >> 2], from + 4 * (j & 3));
+#pragma unroll
+      for (int z = 0; z < 2; ++z) {
+        if (j < 4) {
+          if (j <= rr) y[z][0] = fmaf(m[z][0][j], wj, y[z][0]);   // (selected: a later row may be anything)
+          y[z][1] = fmaf(m[z][1][j], wj, y[z][1]);
+        } else if (j - 4 <= rr) {
+          y[z][1] = fmaf(m[z][2][j - 4], wj, y[z][1]);
         }
-        const float mine = quarter == 0 ? o[0] : quarter == 1 ? o[1] : quarter == 2 ? o[2] : o[3];
-        if (f0 + rr < f1 && j0 + quarter < vd) a.out[(int64_t)(start + b0 + f0 + rr) * hv + (int64_t)h * vd + j0 + quarter] = mine;
-      }
-      __syncwarp();
       }
     }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int t = b * R + rr + 4 * i;
+      const float u = t < n_rows ? y[0][i] : 0.f;
+      *reinterpret_cast<float2*>(us + (rr + 4 * i) * 2 * CW + grp * 8 + 2 * col) = make_float2(u, u);
+      if (t < n_rows && have && (LG == 16 || lane < 16)) out[(int64_t)t * hv + j0 + col] = y[1][i];
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int i = 0; i < 2 * V; ++i) S[c][i] = f2::mul(S[c][i], G[i]);
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      uint64_t x[2 * V];
+      if (LG == 32) {
+#pragma unroll
+        for (int i = 0; i < 2 * V; ++i) x[i] = kx[r][i];
+      } else {
+        row_of(in + (2 * R + r) * ROW, x);
+      }
+      const ulonglong2* up = reinterpret_cast<const ulonglong2*>(us + r * 2 * CW + grp * 8);
+      const ulonglong2 u01 = up[0], u23 = up[1];
+      const uint64_t uu[4] = {u01.x, u01.y, u23.x, u23.y};
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int i = 0; i < 2 * V; ++i) S[c][i] = f2::fma(x[i], uu[c], S[c][i]);
+    }
+    if (b + kDbSlots < n_blocks) db_arrive<BAR>(kEmpty + b % kDbSlots);
+    __syncwarp();   // u has been read
   }
 #pragma unroll
   for (int c = 0; c < 4; ++c)
 #pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      const int d = ds_chan<NP>(lane, i);
-      float* p = S_st + (int64_t)c * dim + d;
-      if (j0 + c >= vd || d >= dim) continue;
-      if (a.vec) {
-        *reinterpret_cast<uint64_t*>(p) = S[c][i];
-      } else {
-        p[0] = f2::lo(S[c][i]);
-        if (d + 1 < dim) p[1] = f2::hi(S[c][i]);
-      }
+    for (int i = 0; i < V; ++i) {
+      const int d = 4 * xl + 4 * LG * i;
+      if (c < cols && d < dim) *reinterpret_cast<ulonglong2*>(S_st + (int64_t)c * dim + d) = make_ulonglong2(S[c][2 * i], S[c][2 * i + 1]);
     }
+}
+
+// CTAs of a head that share triangles: the largest divisor of its column blocks up to kDbCluster
+int db_cluster(int blocks) {
+  int c = kDbCluster;
+  while (blocks % c) --c;
+  return c;
+}
+template <int NP, bool CHAN, int LG, int CTAS>   // CTAS: that share an SM
+int delta_block(const ScanArgs& a, int S, cudaStream_t s) {
+  static bool done[64] = {};
+  const dim3 grid(S, a.heads, (a.vd + kDsCols - 1) / kDsCols);
+  // shared memory for CTAS an SM, so that no more meet there: the CTAs of a cluster are packed onto as few SMs as hold them
+  constexpr int need = std::max(db_floats(NP, LG), ds_floats(NP, CHAN)) * 4, bytes = CTAS == 1 ? 120 * 1024 : CTAS == 2 ? 80 * 1024 : need;
+  static_assert(need <= bytes && CTAS * (bytes + 1024) <= 228 * 1024, "CTAs an SM");
+  B200_CUDA(ensure_dynamic_smem(delta_block_kernel<NP, CHAN, LG, CTAS>, bytes, done));
+  B200_CUDA(launch_cluster(delta_block_kernel<NP, CHAN, LG, CTAS>, grid, dim3(db_threads(LG)), (size_t)bytes, s, dim3(1, 1, db_cluster((int)grid.z)), a));
+  return B200_OK;
+}
+
+template <int NP, bool CHAN>
+int delta_blocks(const ScanArgs& a, int S, int64_t ctas, cudaStream_t s) {
+  if constexpr (NP == 2) {
+    if (ctas <= kNumSMs) return delta_block<NP, CHAN, 32, 1>(a, S, s);
+    if (ctas <= 2 * kNumSMs) return delta_block<NP, CHAN, 32, 2>(a, S, s);
+  }
+  return delta_block<NP, CHAN, 16, 3>(a, S, s);
 }
 
 }  // namespace
@@ -649,6 +860,7 @@ int linear_scan(bool delta_rule, const float* qn, const float* kn, const float* 
   a.vec = dim % 4 == 0 && slot_stride % 4 == 0 && ((at(qn) | at(kn) | at(state)) & 15) == 0 &&
           (!chan || (g_chan == 1 && g_row % 4 == 0 && g_head % 4 == 0 && at(decay) % 16 == 0));
   const dim3 grid(S, heads, (vd + kDsCols - 1) / kDsCols), block(kDsThreads);
+  const int64_t ctas = (int64_t)S * heads * grid.z;
 #define SCAN3(D, R, CH)                                                                                       \
   do {                                                                                                        \
     static bool done[64] = {};                                                                                \
@@ -657,6 +869,11 @@ int linear_scan(bool delta_rule, const float* qn, const float* kn, const float* 
       B200_CUDA(launch(delta_rows_kernel<D, R, CH>, grid, block, (size_t)0, s, a));                           \
       break;                                                                                                  \
     }                                                                                                         \
+    if constexpr (D <= 2 && R)                                                                                \
+      if (a.vec && ctas <= 3 * kNumSMs) {                                                                     \
+        if (const int e = delta_blocks<D, CH>(a, S, ctas, s)) return e;                                       \
+        break;                                                                                                \
+      }                                                                                                       \
     if (smem > 48 * 1024) B200_CUDA(ensure_dynamic_smem(delta_scan_kernel<D, R, CH>, (int)smem, done));       \
     B200_CUDA(launch(delta_scan_kernel<D, R, CH>, grid, block, smem, s, a));                                  \
   } while (0)

@@ -221,3 +221,83 @@ def test_linear_scans_portions(rule, heads, kv, dim, vdim):
             assert (st[:floats].reshape(S.shape) - S).norm() < 2e-6 * S.norm() and (st[floats:] == 7.5).all()
             pos[s] += cuts[s]
     assert (state[[1, 3]] == 7.5).all()
+
+
+def _delta(q, k, v, beta, decay, S):
+    """Rows one by one in float64: [T][heads][vdim] and the state [heads][vdim][dim] after them."""
+    y = torch.empty(v.shape, dtype=torch.float64, device=v.device)
+    for r in range(len(v)):
+        S = S * decay[r][:, None, :]
+        u = v[r] - (S @ k[r][:, :, None])[..., 0]
+        S = S + (beta[r][:, None] * u)[:, :, None] * k[r][:, None, :]
+        y[r] = (S @ q[r][:, :, None])[..., 0]
+    return y, S
+
+
+# The delta rule in blocks of eight rows: one, two and three CTAs an SM, portions on both sides of the length from which it takes them (64; 128 with three
+# CTAs an SM), blocks and rounds that are not full, clusters of one to four CTAs, half a warp's columns and channels missing; the second step starts from
+# the state that the first one left.
+@pytest.mark.parametrize("chan", [True, False])
+@pytest.mark.parametrize("heads,kv,dim,vdim,steps", [
+    (16, 16, 128, 128, [[300], [65]]), (2, 1, 128, 128, [[63], [64], [66], [72], [97]]), (3, 3, 100, 16, [[129], [80]]), (1, 1, 68, 40, [[200], [71]]),
+    (16, 4, 128, 128, [[64, 90], [130, 7]]), (40, 8, 128, 48, [[70, 1], [67, 256]]),
+    (16, 16, 128, 128, [[128, 127, 20], [1, 140, 161]]), (8, 2, 64, 128, [[128], [145]]), (16, 4, 64, 128, [[160, 200], [5, 129]]), (4, 4, 36, 24, [[131], [250]]),
+])
+def test_delta_blocks(heads, kv, dim, vdim, steps, chan):
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    g = torch.Generator(device=DEV).manual_seed(dim + vdim + heads)
+    S, rnd = len(steps[0]), lambda *s: torch.randn(*s, generator=g, device=DEV)
+    floats = heads * vdim * dim
+    state = torch.full((S + 1, floats), 7.5, device=DEV)
+    slots, pos = [S - s for s in range(S)], [0] * S
+    oracle = [torch.zeros(heads, vdim, dim, dtype=torch.float64, device=DEV) for _ in range(S)]
+    for cuts in steps:
+        T = sum(cuts)
+        q, k = (torch.nn.functional.normalize(rnd(T, kv, dim), dim=-1) for _ in range(2))
+        v, beta = rnd(T, heads, vdim), torch.sigmoid(rnd(T, heads))
+        decay = torch.rand(T, heads, dim if chan else 1, generator=g, device=DEV) ** 0.1
+        decay[T // 2], k[T // 3], decay[T // 4, 0] = 0.0, 0.0, 1e-30
+        start = [0]
+        for n in cuts:
+            start.append(start[-1] + n)
+        out = torch.full((T, heads * vdim), float("nan"), device=DEV)
+        ptd, std, sld = _i32([pos[s] + i for s in range(S) for i in range(cuts[s])]), _i32(start), _i32(slots)
+        check(lib.b200_linear_scan(1, *[x.data_ptr() for x in (q, k, v, beta, decay)], heads * decay.shape[2], decay.shape[2], int(chan), ptd.data_ptr(),
+                                   std.data_ptr(), sld.data_ptr(), state.data_ptr(), floats, out.data_ptr(), S, heads, kv, dim, vdim, None))
+        torch.cuda.synchronize()
+        wide = [x.double().repeat_interleave(heads // kv, 1) for x in (q, k)] + [x.double() for x in (v, beta, decay)]
+        for s in range(S):
+            lo, hi = start[s], start[s + 1]
+            want, oracle[s] = _delta(*[x[lo:hi] for x in wide], oracle[s])
+            # fp32 throughout, as above: 2^-24 for sums of up to 128 terms and the roundings of some tens of live rows
+            err, size = (out[lo:hi].double().reshape(want.shape) - want).flatten(1).norm(dim=1), want.flatten(1).norm(dim=1)
+            assert (err < 2e-6 * torch.maximum(size, 0.05 * oracle[s].norm())).all(), (cuts, s, float((err / size).max()))
+            assert (state[slots[s]].double().reshape(oracle[s].shape) - oracle[s]).norm() < 2e-6 * oracle[s].norm()
+            pos[s] += cuts[s]
+    assert (state[0] == 7.5).all()
+
+
+@pytest.mark.parametrize("what", ["value", "key", "query", "decay", "beta"])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("row", [0, 37, 99])
+def test_delta_blocks_are_causal_for_what_is_not_finite(what, bad, row):
+    """A row's value that is not finite reaches its own column only, everything else the head's later rows only; a query its own row."""
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    g = torch.Generator(device=DEV).manual_seed(row)
+    T, heads, dim, vdim, rnd = 100, 2, 128, 32, lambda *s: torch.randn(*s, generator=g, device=DEV)
+    q, k = (torch.nn.functional.normalize(rnd(T, heads, dim), dim=-1) for _ in range(2))
+    v, beta, decay = rnd(T, heads, vdim), torch.sigmoid(rnd(T, heads)), torch.rand(T, heads, dim, generator=g, device=DEV) ** 0.1
+    outs = []
+    for clean in (True, False):
+        if not clean:
+            {"value": v, "key": k, "query": q, "decay": decay, "beta": beta[:, :, None]}[what][row, 1, -1] = bad
+        state, out = torch.zeros(1, heads * vdim * dim, device=DEV), torch.empty(T, heads, vdim, device=DEV)
+        pos, start, slot = _i32(list(range(T))), _i32([0, T]), _i32([0])
+        check(lib.b200_linear_scan(1, *[x.data_ptr() for x in (q, k, v, beta, decay)], heads * dim, dim, 1, pos.data_ptr(), start.data_ptr(), slot.data_ptr(),
+                                   state.data_ptr(), state.shape[1], out.data_ptr(), 1, heads, heads, dim, vdim, None))
+        torch.cuda.synchronize()
+        outs.append(out.cpu())
+    a, b = outs
+    same = torch.ones(T, heads, vdim, dtype=torch.bool)
+    same[row:row + 1 if what == "query" else T, 1, -1 if what == "value" else 0:] = False
+    assert torch.equal(a[same], b[same]) and not torch.isfinite(b[row, 1, -1])
