@@ -405,6 +405,17 @@ static int attn_mma_launch(const float* q, const __nv_bfloat16* kc, const __nv_b
   return B200_OK;
 }
 
+// Rows by themselves on tcgen05 (attn_latent_rows.cu): steps whose rows' heads, 16 at a time, fit the device's SMs at once (what they measured stands
+// there; a few rows of one sequence gain as much, up to 128 of them behind 3000 tokens a little), and decode rows that say so in any number: 256 rows
+// of 16 heads at contexts 300..600 86 us on the mma.sync kernel, 51 there.  Beyond that a step of unknown rows may be a prefill chunk, whose runs
+// share their keys on attn_latent_tc.cu (2 048 rows 187 us).
+bool latent_attn_by_rows(const float* q, const __nv_bfloat16* kc, const int32_t* row_to_seq, const __nv_bfloat16* out, int T, int heads, int krow, int rank,
+                         int block_size, float scale, bool one_row_each) {
+  const auto at = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr); };
+  return T > 0 && scale > 0.f && latent_attn_mma_supported(heads, krow, rank) && latent_attn_rows_supported(heads, krow, rank, block_size) &&
+         (at(q) | at(kc) | at(out)) % 16 == 0 && (latent_attn_rows_items(T, heads) <= kNumSMs || one_row_each || !row_to_seq);
+}
+
 // runs / n_runs: the run list of the step (attn_anydim.cu builds it: runs of at most 16 consecutive rows of one sequence)
 int latent_attn_mma(const float* q, const __nv_bfloat16* kc, const int32_t* block_table, int bt_stride, const int32_t* row_to_seq,
                     const int32_t* ctx_lens, __nv_bfloat16* out, const int32_t* runs, const int32_t* n_runs, int T, int heads, int krow,
@@ -416,6 +427,18 @@ int latent_attn_mma(const float* q, const __nv_bfloat16* kc, const int32_t* bloc
   B200_REQUIRE(n_splits <= kLaMaxSplits, B200_ERR_INVALID, "attention: %d splits (at most %d)", n_splits, kLaMaxSplits);
   const auto at = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr); };
   B200_REQUIRE(at(kc) % 16 == 0, B200_ERR_INVALID, "attention: cache not 16-byte aligned");
+  const auto merge = [&](int splits) -> int {
+    B200_CUDA(launch(latent_attn_merge_kernel, dim3((T * heads + 3) / 4), dim3(128), (size_t)0, s, (const float*)part, out, T * heads, heads, rank, splits,
+                     sink, (const __nv_bfloat16*)nullptr, (int64_t)0));
+    return B200_OK;
+  };
+  if (latent_attn_by_rows(q, kc, row_to_seq, out, T, heads, krow, rank, block_size, scale, one_row_each)) {
+    const int rc = latent_attn_rows(q, kc, block_table, bt_stride, row_to_seq, ctx_lens, out, T, heads, krow, rank, block_size, scale, sink, s, window,
+                                    at(part) % 8 == 0 ? part : nullptr, &n_splits);
+    if (rc || n_splits == 1) return rc;
+    const PdlScope after_rows;
+    return merge(n_splits);
+  }
   // tcgen05 wherever the shape fits and the rows can be read and written in its wide pieces (what it measured stands there); other shapes, blocks
   // that a key tile would straddle and odd addresses stay here, and so do scales that are not positive (masks and maxima there are taken of
   // the unscaled scores) and steps whose rows are known to be sequences of their own (or have one head: 16 pairs a run at most) where
@@ -425,10 +448,7 @@ int latent_attn_mma(const float* q, const __nv_bfloat16* kc, const int32_t* bloc
       ((at(runs) | at(part)) & 7) == 0) {
     const int rc = latent_attn_tc(q, kc, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, krow, rank, block_size, scale,
                                   sink, s, n_splits, part, window);
-    if (rc || n_splits == 1) return rc;
-    B200_CUDA(launch(latent_attn_merge_kernel, dim3((T * heads + 3) / 4), dim3(128), (size_t)0, s, (const float*)part, out, T * heads, heads,
-                     rank, n_splits, sink, (const __nv_bfloat16*)nullptr, (int64_t)0));
-    return B200_OK;
+    return rc || n_splits == 1 ? rc : merge(n_splits);
   }
   return attn_mma_launch(q, kc, nullptr, 1, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, krow, rank, block_size,
                          scale, sink, s, n_splits, part, window, AttnExtra());

@@ -157,7 +157,7 @@ LaunchOpts& launch_opts();
 // launched (every kernel waits for its predecessor's memory in pdl_wait).
 struct PdlScope {
   const bool before;
-  PdlScope() : before(launch_opts().pdl) { launch_opts().pdl = before || launch_opts().within; }
+  explicit PdlScope(bool later = true) : before(launch_opts().pdl) { launch_opts().pdl = before || (later && launch_opts().within); }   // later false: nothing was launched before
   ~PdlScope() { launch_opts().pdl = before; }
 };
 int& launch_counter();
@@ -370,6 +370,14 @@ constexpr int kRunTicket = 5;   // word behind the lists' lengths: runs.cuh
 int paged_attn_runs_plan(const int32_t* row_to_seq, const int32_t* ctx_lens, int T, void* ws, cudaStream_t s);
 // latent cache rows on the tensor cores (attn_latent.cu): bf16 cache, fp32 queries, bf16 output [T][heads][rank]
 bool latent_attn_mma_supported(int heads, int krow, int rank);
+// rows by themselves (attn_latent_rows.cu): no run list; latent_attn_mma takes it wherever latent_attn_by_rows says so
+bool latent_attn_rows_supported(int heads, int krow, int rank, int block_size);
+int latent_attn_rows_items(int T, int heads);   // rows times groups of 16 heads
+int latent_attn_rows(const float* q, const __nv_bfloat16* kc, const int32_t* block_table, int bt_stride, const int32_t* row_to_seq, const int32_t* ctx_lens,
+                     __nv_bfloat16* out, int T, int heads, int krow, int rank, int block_size, float scale, const float* sink, cudaStream_t s, int window, float* part,
+                     int* n_splits);   // n_splits: at most, and taken
+bool latent_attn_by_rows(const float* q, const __nv_bfloat16* kc, const int32_t* row_to_seq, const __nv_bfloat16* out, int T, int heads, int krow, int rank,
+                         int block_size, float scale, bool one_row_each);
 int latent_attn_mma(const float* q, const __nv_bfloat16* kc, const int32_t* block_table, int bt_stride, const int32_t* row_to_seq,
                     const int32_t* ctx_lens, __nv_bfloat16* out, const int32_t* runs, const int32_t* n_runs, int T, int heads, int krow,
                     int rank, int block_size, float scale, const float* sink, cudaStream_t s, int n_splits = 1, float* part = nullptr,

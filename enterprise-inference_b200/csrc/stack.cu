@@ -2050,9 +2050,10 @@ extern "C" int b200_latent_attn(const float* q, const void* cache, const int32_t
                                 int32_t block_size, float scale, const float* sink, void* workspace, int32_t n_splits, float* part,
                                 void* stream) {
   B200_REQUIRE(q && cache && block_table && ctx_lens && out && workspace && block_size > 0, B200_ERR_INVALID, "latent_attn: bad argument");
-  int rc = paged_attn_runs_plan(row_to_seq, ctx_lens, T, workspace, (cudaStream_t)stream);
-  if (rc) return rc;
-  const PdlScope after_plan;
+  const bool by_rows = latent_attn_by_rows(q, (const __nv_bfloat16*)cache, row_to_seq, (const __nv_bfloat16*)out, T, heads, k_row, rank, block_size, scale, false);
+  if (!by_rows)
+    if (const int rc = paged_attn_runs_plan(row_to_seq, ctx_lens, T, workspace, (cudaStream_t)stream)) return rc;
+  const PdlScope after_plan(!by_rows);
   return latent_attn_mma(q, (const __nv_bfloat16*)cache, block_table, bt_stride, row_to_seq, ctx_lens, (__nv_bfloat16*)out,
                          static_cast<const int32_t*>(workspace) + 8, static_cast<const int32_t*>(workspace), T, heads, k_row, rank,
                          block_size, scale, sink, (cudaStream_t)stream, n_splits, part);
@@ -2098,9 +2099,10 @@ extern "C" int b200_latent_attn_window(const float* q, const void* cache, const 
                                        void* stream) {
   B200_REQUIRE(q && cache && block_table && ctx_lens && out && workspace && block_size > 0 && window >= 0, B200_ERR_INVALID,
                "latent_attn_window: bad argument");
-  int rc = paged_attn_runs_plan(row_to_seq, ctx_lens, T, workspace, (cudaStream_t)stream);
-  if (rc) return rc;
-  const PdlScope after_plan;
+  const bool by_rows = latent_attn_by_rows(q, (const __nv_bfloat16*)cache, row_to_seq, (const __nv_bfloat16*)out, T, heads, k_row, rank, block_size, scale, false);
+  if (!by_rows)
+    if (const int rc = paged_attn_runs_plan(row_to_seq, ctx_lens, T, workspace, (cudaStream_t)stream)) return rc;
+  const PdlScope after_plan(!by_rows);
   return latent_attn_mma(q, (const __nv_bfloat16*)cache, block_table, bt_stride, row_to_seq, ctx_lens, (__nv_bfloat16*)out,
                          static_cast<const int32_t*>(workspace) + 8, static_cast<const int32_t*>(workspace), T, heads, k_row, rank,
                          block_size, scale, sink, (cudaStream_t)stream, 1, nullptr, window);

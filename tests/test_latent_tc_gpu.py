@@ -113,3 +113,51 @@ def test_latent_steps_of_many_items(heads, rank, rd, runs, splits):
     assert torch.isfinite(got).all()
     # weights and results rounded to bf16 once each: 2^-9 of the largest value, 2^-9 of the result
     assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -9 * rows.float().abs().max()).all()
+
+
+# Rows by themselves (attn_latent_rows.cu): clusters of eight, four, two and one CTA, more CTAs than SMs (rows known to be sequences of their own), heads that
+# are no multiple of 16, one to four pairs of value chunks with and without other chunks beside them, contexts around tiles and blocks, windows.
+@pytest.mark.parametrize("T,heads,rank,rd,bs,window,with_sink,with_seq", [
+    (1, 16, 512, 64, 128, 0, True, True), (15, 16, 512, 64, 64, 0, False, True), (16, 16, 256, 32, 128, 0, True, True), (33, 5, 304, 16, 64, 0, False, True),
+    (34, 16, 512, 0, 128, 0, True, True), (74, 16, 128, 64, 128, 300, True, True), (75, 16, 512, 64, 128, 0, False, True), (148, 1, 16, 16, 192, 0, True, True),
+    (9, 40, 512, 64, 128, 0, True, True), (3, 128, 64, 128, 64, 65, False, True), (200, 16, 512, 64, 128, 0, True, False),
+    (1, 16, 512, 64, 128, -16, True, True), (2, 20, 256, 32, 64, -5, False, True), (7, 16, 80, 48, 128, -2, True, True)])   # (a negative window: so many splits)
+def test_latent_rows_by_themselves(T, heads, rank, rd, bs, window, with_sink, with_seq):
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    splits, window = max(-window, 1), max(window, 0)
+    g = torch.Generator().manual_seed(T * 1000 + rank + heads)
+    krow, n_tok, scale = rank + rd, 1200, 0.6 / (rank + rd) ** 0.5
+    nb = (n_tok + bs - 1) // bs
+    rows = torch.randn(n_tok, krow, generator=g).to(torch.bfloat16)
+    perm = torch.randperm(nb + 3, generator=g)[:nb]
+    edges = [1, 2, 15, 16, 17, 63, 64, 65, 127, 128, 129, 143, 255, 257, 640, 1023, 1025, 1200]
+    ctxs = [edges[(i * 7 + T) % len(edges)] for i in range(T)]
+    q = (torch.randn(T, heads, krow, generator=g) * 4).to(torch.bfloat16).float()   # large scores: the running maximum jumps
+    sink = torch.randn(heads, generator=g) * 2 if with_sink else None
+    want = torch.stack([_oracle(q[t].double(), rows.double(), ctxs[t], rank, scale, sink.double() if with_sink else None, window) for t in range(T)])
+    kc = torch.full((nb + 3, 1, bs, krow), float("nan"), dtype=torch.bfloat16)
+    kc[perm] = torch.cat([rows, torch.full((nb * bs - n_tok, krow), float("nan"), dtype=torch.bfloat16)]).reshape(nb, 1, bs, krow)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)   # noqa: E731
+    bt, cx, kd, qd = perm.to(torch.int32)[None, :].repeat(T, 1).to(DEV), i32(ctxs), kc.to(DEV), q.to(DEV)
+    for t, c in enumerate(ctxs):   # what lies past a context's last tile of 64 keys is nobody's block
+        bt[t, ((c + 63) // 64 * 64 + bs - 1) // bs:] = 1 << 29
+    if splits > 1:   # only tables for more than 32 768 tokens have them taken
+        nb = 32768 // bs + 1
+        bt = torch.nn.functional.pad(bt, (0, nb - bt.shape[1])).contiguous()
+    sq = i32(list(range(T))) if with_seq else None
+    sd = sink.to(DEV) if with_sink else None
+    ws = torch.zeros(int(lib.b200_paged_attn_anydim_workspace_bytes(T)), dtype=torch.uint8, device=DEV)
+    out = torch.full((T, heads, rank), float("nan"), dtype=torch.bfloat16, device=DEV)
+    args = (qd.data_ptr(), kd.data_ptr(), bt.data_ptr(), nb, sq.data_ptr() if with_seq else None, cx.data_ptr(), out.data_ptr(), T, heads, krow, rank, bs, scale,
+            sd.data_ptr() if with_sink else None, ws.data_ptr())
+    if splits > 1:
+        part = torch.full((T * heads * splits * (rank + 2),), float("nan"), device=DEV)
+        check(lib.b200_latent_attn(*args, splits, part.data_ptr(), None))
+    else:
+        check(lib.b200_latent_attn_window(*args, window, None))
+    torch.cuda.synchronize()
+    got = out.double().cpu()
+    assert torch.isfinite(got).all()
+    # (as above)
+    assert (got - want).norm() / want.norm() < 2.0 ** -8
+    assert (got - want).abs().max() < 2.0 ** -8 * rows.float().abs().max() + 2.0 ** -9 * want.abs().max()
