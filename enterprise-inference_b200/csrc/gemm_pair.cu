@@ -207,22 +207,26 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       const uint32_t one = elect_one();
       const uint16_t both = (uint16_t)(3 << lead);
       const uint64_t desc0 = tc::make_desc(tc::smem_u32(smem), 16, 1024);
-      int it = 0, i = 0;
-      for (int t = first; t < tiles; t += step, ++i) {
-        const PairTile tile = pair_tile(p, t);
-        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(tile.n >> 3) << 17) | ((uint32_t)(2 * kBlockM >> 4) << 24);
-        const uint32_t acc = tmem + (uint32_t)((i & 1) * 256);
+      const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+      const int n_tiles = __shfl_sync(0xffffffffu, tiles, 0);
+      int i = 0, st = 0;
+      uint32_t st_ph = 0;
+      for (int t = first; t < n_tiles; t += step, ++i) {
+        const int n = __shfl_sync(0xffffffffu, pair_tile(p, t).n, 0);
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(2 * kBlockM >> 4) << 24);
+        const uint32_t acc = tm + (uint32_t)((i & 1) * 256);
         if (i >= 2) wait(&acc_free[i & 1], ((i >> 1) - 1) & 1);
         tc::fence_after();
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int st = it % kPairStages;
-          wait(&full[st], (it / kPairStages) & 1);
+        for (int kb = kb0; kb < kb1; ++kb) {
+          wait(&full[st], st_ph);
           tc::fence_after();
           const uint64_t da = desc0 + (uint64_t)((st * kPairStageBytes) >> 4), db = da + (uint64_t)(kPairABytes >> 4);
+          const uint32_t more = kb > kb0 ? 1u : 0u;
 #pragma unroll
           for (int k = 0; k < kBlockK / 16; ++k)   // 16 of k are 32 bytes inside the swizzle's span
-            pair_mma(one, acc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > kb0 || k) ? 1u : 0u);
+            pair_mma(one, acc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, k ? 1u : more);
           pair_commit(one, &empty[st], both);
+          if (++st == kPairStages) st = 0, st_ph ^= 1;
         }
         pair_commit(one, &acc_full[i & 1], both);
         if (wait.stop()) break;
