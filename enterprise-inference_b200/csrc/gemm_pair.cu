@@ -11,9 +11,9 @@
 // four warps.  Launches with few tiles share a tile's k between up to four pairs of one cluster, which add up through distributed shared memory.
 //
 // Against 128 x 256 tiles of single CTAs with k split over clusters (us, before -> now): 2000 tokens, k 14336, 4096 features 179 -> 162; 2048, 4096,
-// 28672 404 -> 321; 2048, 4096, 6144 107 -> 78; 1000, 4096, 4096 62 -> 38; 300, 2048, 2048 22 -> 12; 200, 14336, 4096 50 -> 32; 130, 2048, 2048 19 -> 11.
+// 28672 404 -> 320; 2048, 4096, 6144 107 -> 78; 1000, 4096, 4096 62 -> 38; 300, 2048, 2048 22 -> 12; 200, 14336, 4096 50 -> 32; 130, 2048, 2048 19 -> 11.
 // Routed experts (the table of token tiles is moe.cu's): 32 experts of 1024, width 2048, 4 of them a row, router and grouping included, tiles of
-// 128 x 128 before: 2048 rows 263 -> 181, 1000 rows 193 -> 141, 600 rows 165 -> 125; 64 of 512, width 4096, 8 a row, 2048 rows 586 -> 375.  Their
+// 128 x 128 before: 2048 rows 263 -> 174, 1000 rows 193 -> 138, 600 rows 165 -> 125; 64 of 512, width 4096, 8 a row, 2048 rows 586 -> 361.  Their
 // weights come from HBM (1000 rows: 402 MB), and whole waves of tiles decide the rest (2048 rows: 5.2 waves of gate|up).
 // 128 tokens and fewer stay on gemm_tc.cu's tiles: their launches stream W, and 148 CTAs with two of them to an SM keep more of it in flight
 // (64 tokens, 4096, 28672: 42 there, 49 here; 128, 14336, 4096: 33 and 34).
@@ -46,6 +46,14 @@ __device__ __forceinline__ void pair_load(void* dst, const CUtensorMap* map, int
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;" ::"r"(
           tc::smem_u32(dst)),
       "l"(map), "r"(bar), "r"(c0), "r"(c1), "l"(policy)
+      : "memory");
+}
+// two boxes of rows, c2 and the slab behind it
+__device__ __forceinline__ void pair_load3(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;" ::"r"(
+          tc::smem_u32(dst)),
+      "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "l"(policy)
       : "memory");
 }
 __device__ __forceinline__ void pair_mma(uint32_t one, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t acc) {
@@ -81,6 +89,12 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// The token rows in boxes of 16, 32, .. 128 rows: a CTA's half of any tile in one load (a load more a stage costs the fetching warp more than the
+// ring can hide: 2 048 rows of 32 experts in boxes of 64 and 16 180 us, so 174)
+struct PairMaps {
+  CUtensorMap x[8];
+};
+
 struct PairTile {
   int m, row0, n, expert;   // 256-row tile of W, first token row, tokens (a multiple of 32)
 };
@@ -112,8 +126,7 @@ __device__ __forceinline__ void pair_bias(const TcParams& p, int m_tile, int r4,
 
 template <int MODE>
 __global__ void __launch_bounds__(kPairThreads, 1)
-linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_rest,
-                   const TcParams p, uint32_t* status) {
+linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ PairMaps maps, const TcParams p, uint32_t* status) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   float* stg_all = reinterpret_cast<float*>(smem + kPairStages * kPairStageBytes);
@@ -164,13 +177,14 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const bool issuer = elect_one();
     if (issuer) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
-      asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
+      if (!p.pair_tile) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.x[(p.pair_n >> 5) - 1]) : "memory");
     }
     int it = 0;
     for (int t = first; t < tiles; t += step) {
       const PairTile tile = pair_tile(p, t);
       const int half = tile.n >> 1, x0 = tile.row0 + rank * half, m = 2 * tile.m + rank;
-      const int w0 = p.gu_ff ? tile.expert * 2 * p.gu_ff + m * (kBlockM / 2) : tile.expert * p.n_out + m * kBlockM;
+      const int w0 = tile.expert * p.n_out + m * kBlockM;
+      const CUtensorMap* map_x = &maps.x[(tile.n >> 5) - 1];
       const uint32_t bytes = (uint32_t)(2 * kPairABytes + tile.n * kBlockK * 2);
       for (int kb = kb0; kb < kb1; ++kb, ++it) {
         const int st = it % kPairStages;
@@ -179,19 +193,9 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
           unsigned char* a = smem + st * kPairStageBytes;
           const uint32_t bar = smem_of(&full[st], lead);
           if (rank == 0) tc::mbar_expect_tx(&full[st], bytes);
-          if (p.gu_ff) {   // 64 gate rows, then the matching up rows
-            pair_load(a, &map_w, kb * kBlockK, w0, bar, kKeepNormal);
-            pair_load(a + kPairABytes / 2, &map_w, kb * kBlockK, w0 + p.gu_ff, bar, kKeepNormal);
-          } else {
-            pair_load(a, &map_w, kb * kBlockK, w0, bar, kKeepNormal);
-          }
-          if (p.pair_tile) {
-            int r = 0;
-            for (; r + 64 <= half; r += 64) pair_load(a + kPairABytes + r * 128, &map_x, kb * kBlockK, x0 + r, bar, kKeepLast);
-            for (; r < half; r += 16) pair_load(a + kPairABytes + r * 128, &map_rest, kb * kBlockK, x0 + r, bar, kKeepLast);
-          } else {
-            pair_load(a + kPairABytes, &map_x, kb * kBlockK, x0, bar, kKeepLast);
-          }
+          if (p.gu_ff) pair_load3(a, &map_w, kb * kBlockK, m * (kBlockM / 2), 2 * tile.expert, bar, kKeepNormal);   // 64 gate rows, then the matching up rows
+          else pair_load(a, &map_w, kb * kBlockK, w0, bar, kKeepNormal);
+          pair_load(a + kPairABytes, map_x, kb * kBlockK, x0, bar, kKeepLast);
         }
         __syncwarp();
         if (wait.stop()) break;
@@ -345,10 +349,10 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 }
 
 template <int MODE>
-int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mr, const TcParams& p, int clusters, cudaStream_t s) {
+int launch_pair(const CUtensorMap& mw, const PairMaps& mx, const TcParams& p, int clusters, cudaStream_t s) {
   static bool attr_set[64] = {};
   B200_CUDA(ensure_dynamic_smem(linear_pair_kernel<MODE>, kPairSmem, attr_set));
-  B200_CUDA(launch_cluster(linear_pair_kernel<MODE>, dim3(clusters * 2 * p.splits), dim3(kPairThreads), (size_t)kPairSmem, s, dim3(2 * p.splits, 1, 1), mw, mx, mr, p, wait_status_word()));
+  B200_CUDA(launch_cluster(linear_pair_kernel<MODE>, dim3(clusters * 2 * p.splits), dim3(kPairThreads), (size_t)kPairSmem, s, dim3(2 * p.splits, 1, 1), mw, mx, p, wait_status_word()));
   return B200_OK;
 }
 
@@ -380,22 +384,23 @@ int linear_pair(int mode, TcParams p, const __nv_bfloat16* x, int64_t ldx, const
   p.pair_tok = (p.T + pl.n - 1) / pl.n;
   p.pair_m = (p.n_out + 2 * kBlockM - 1) / (2 * kBlockM);
   p.pair_group = (p.pair_tok + (p.pair_tok + 8) / 9 - 1) / ((p.pair_tok + 8) / 9);
-  CUtensorMap mw, mx;
+  CUtensorMap mw;
+  PairMaps mx = {};
   int rc = get_tensor_map_2d(w, (uint64_t)p.n_out, (uint64_t)k, (uint64_t)k, kBlockM, &mw);
   if (rc) return rc;
-  rc = get_tensor_map_2d(x, (uint64_t)p.T, (uint64_t)k, (uint64_t)ldx, (uint32_t)pl.n / 2, &mx);
+  rc = get_tensor_map_2d(x, (uint64_t)p.T, (uint64_t)k, (uint64_t)ldx, (uint32_t)pl.n / 2, &mx.x[pl.n / 32 - 1]);
   if (rc) return rc;
   const int clusters = (int)std::min<int64_t>((int64_t)p.pair_tok * p.pair_m, kNumSMs / 2);
   switch (mode) {
-    case kScatter: return launch_pair<kScatter>(mw, mx, mx, p, clusters, s);
-    case kSiluMul: return launch_pair<kSiluMul>(mw, mx, mx, p, clusters, s);
-    case kRopeKv: return launch_pair<kRopeKv>(mw, mx, mx, p, clusters, s);
-    default: return launch_pair<kPlain>(mw, mx, mx, p, clusters, s);
+    case kScatter: return launch_pair<kScatter>(mw, mx, p, clusters, s);
+    case kSiluMul: return launch_pair<kSiluMul>(mw, mx, p, clusters, s);
+    case kRopeKv: return launch_pair<kRopeKv>(mw, mx, p, clusters, s);
+    default: return launch_pair<kPlain>(mw, mx, p, clusters, s);
   }
 }
 
 // ---- grouped form ----------------------------------------------------------------------------------------------------------
-static int launch_grouped_pair(int mode, TcParams p, const GroupedPairs& g, const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, int w_box, int k,
+static int launch_grouped_pair(int mode, TcParams p, const GroupedPairs& g, const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, int k,
                                cudaStream_t s) {
   B200_REQUIRE(x && w && g.tiles && k > 0 && k % 8 == 0 && ldx % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0,
                B200_ERR_INVALID, "grouped linear: operands in rows of 16-byte pieces");
@@ -404,18 +409,17 @@ static int launch_grouped_pair(int mode, TcParams p, const GroupedPairs& g, cons
   p.n_kblocks = (k + kBlockK - 1) / kBlockK;
   p.splits = 1;
   p.pair_tile = g.tiles;
-  CUtensorMap mw, mx, mr;
-  int rc = get_tensor_map_2d(w, (uint64_t)g.experts * p.n_out, (uint64_t)k, (uint64_t)k, (uint32_t)w_box, &mw);
-  if (rc) return rc;
-  rc = get_tensor_map_2d(x, (uint64_t)g.rows, (uint64_t)k, (uint64_t)ldx, 64, &mx);   // a CTA's rows of a tile: any multiple of 16
-  if (rc) return rc;
-  rc = get_tensor_map_2d(x, (uint64_t)g.rows, (uint64_t)k, (uint64_t)ldx, 16, &mr);
+  CUtensorMap mw;
+  PairMaps mx;
+  int rc = p.gu_ff ? get_tensor_map_3d(w, 2u * (uint32_t)g.experts, (uint64_t)p.gu_ff, (uint64_t)k, kBlockM / 2, &mw)
+                   : get_tensor_map_2d(w, (uint64_t)g.experts * p.n_out, (uint64_t)k, (uint64_t)k, kBlockM, &mw);
+  for (int i = 0; i < 8 && !rc; ++i) rc = get_tensor_map_2d(x, (uint64_t)g.rows, (uint64_t)k, (uint64_t)ldx, 16 * (i + 1), &mx.x[i]);
   if (rc) return rc;
   const int clusters = (int)std::min<int64_t>((int64_t)g.max_tiles * p.pair_m, kNumSMs / 2);
   switch (mode) {
-    case kScatter: return launch_pair<kScatter>(mw, mx, mr, p, clusters, s);
-    case kSiluMul: return launch_pair<kSiluMul>(mw, mx, mr, p, clusters, s);
-    default: return launch_pair<kPlain>(mw, mx, mr, p, clusters, s);
+    case kScatter: return launch_pair<kScatter>(mw, mx, p, clusters, s);
+    case kSiluMul: return launch_pair<kSiluMul>(mw, mx, p, clusters, s);
+    default: return launch_pair<kPlain>(mw, mx, p, clusters, s);
   }
 }
 
@@ -427,7 +431,7 @@ int linear_pair_grouped(const GroupedPairs& g, const __nv_bfloat16* x, int64_t l
   p.n_out = n_out;
   p.post_act = post_act;
   p.pair_m = (n_out + 2 * kBlockM - 1) / (2 * kBlockM);
-  return launch_grouped_pair(kPlain, p, g, x, ldx, w, kBlockM, k, s);
+  return launch_grouped_pair(kPlain, p, g, x, ldx, w, k, s);
 }
 
 int linear_pair_gate_up(const GroupedPairs& g, const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, int ff, int k, __nv_bfloat16* y, cudaStream_t s,
@@ -441,7 +445,7 @@ int linear_pair_gate_up(const GroupedPairs& g, const __nv_bfloat16* x, int64_t l
   p.act = act;
   p.act_limit = act_limit;
   p.pair_m = (ff + kBlockM - 1) / kBlockM;
-  return launch_grouped_pair(kSiluMul, p, g, x, ldx, w, kBlockM / 2, k, s);
+  return launch_grouped_pair(kSiluMul, p, g, x, ldx, w, k, s);
 }
 
 int linear_pair_scatter(const GroupedPairs& g, const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, int n_out, int k, const int32_t* row_pair,
@@ -453,7 +457,7 @@ int linear_pair_scatter(const GroupedPairs& g, const __nv_bfloat16* x, int64_t l
   p.grp_wt = wts;
   p.grp_out = out;
   p.pair_m = (n_out + 2 * kBlockM - 1) / (2 * kBlockM);
-  return launch_grouped_pair(kScatter, p, g, x, ldx, w, kBlockM, k, s);
+  return launch_grouped_pair(kScatter, p, g, x, ldx, w, k, s);
 }
 
 }  // namespace b200

@@ -681,22 +681,23 @@ EncodeTiledFn encode_fn() {
 struct MapKey {
   const void* ptr;
   uint64_t rows, cols, ld;
-  uint32_t box_rows;
+  uint32_t box_rows, slabs;
   bool operator==(const MapKey& o) const {
-    return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows;
+    return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && slabs == o.slabs;
   }
 };
 struct MapKeyHash {
   size_t operator()(const MapKey& k) const {
-    return std::hash<const void*>()(k.ptr) ^ (k.rows * 1315423911ull) ^ (k.cols << 7) ^ (k.ld << 17) ^ k.box_rows;
+    return std::hash<const void*>()(k.ptr) ^ (k.rows * 1315423911ull) ^ (k.cols << 7) ^ (k.ld << 17) ^ k.box_rows ^ ((uint64_t)k.slabs << 40);
   }
 };
 
 // 2D bf16 tensor map [rows][cols] (row stride ld elements), box [box_rows][64], SWIZZLE_128B, zero OOB fill.
-int get_map(const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, CUtensorMap* out) {
+// slabs > 0: 3D [slabs][rows][cols], box [2][box_rows][64].
+int get_map(const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, CUtensorMap* out, uint32_t slabs = 0) {
   static std::mutex mu;
   static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
-  MapKey key{ptr, rows, cols, ld, box_rows};
+  MapKey key{ptr, rows, cols, ld, box_rows, slabs};
   std::lock_guard<std::mutex> lk(mu);
   auto it = cache.find(key);
   if (it != cache.end()) {
@@ -705,12 +706,12 @@ int get_map(const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t
   }
   EncodeTiledFn fn = encode_fn();
   B200_REQUIRE(fn != nullptr, B200_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-  cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {ld * 2};
-  cuuint32_t box[2] = {(cuuint32_t)kBlockK, box_rows};
-  cuuint32_t estr[2] = {1, 1};
+  cuuint64_t dims[3] = {cols, rows, slabs};
+  cuuint64_t strides[2] = {ld * 2, rows * ld * 2};
+  cuuint32_t box[3] = {(cuuint32_t)kBlockK, box_rows, 2};
+  cuuint32_t estr[3] = {1, 1, 1};
   CUtensorMap m;
-  CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
+  CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, slabs ? 3 : 2, const_cast<void*>(ptr), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   B200_REQUIRE(r == CUDA_SUCCESS, B200_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for [%llu x %llu] ld %llu", (int)r,
@@ -819,6 +820,11 @@ int linear_tc_read_trace(unsigned long long* host16) {
 // shared with attn_tc.cu: [rows][cols] bf16 (row stride ld), box [box_rows][64], SWIZZLE_128B
 int get_tensor_map_2d(const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, CUtensorMap* out) {
   return get_map(ptr, rows, cols, ld, box_rows, out);
+}
+
+// [slabs][rows][cols] bf16, box [2][box_rows][64]
+int get_tensor_map_3d(const void* ptr, uint32_t slabs, uint64_t rows, uint64_t cols, uint32_t box_rows, CUtensorMap* out) {
+  return get_map(ptr, rows, cols, cols, box_rows, out, slabs);
 }
 
 bool linear_tc_supported(int T, int n_out, int k) {

@@ -7,6 +7,7 @@
 namespace b200 {
 
 int get_tensor_map_2d(const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, CUtensorMap* out);
+int get_tensor_map_3d(const void* ptr, uint32_t slabs, uint64_t rows, uint64_t cols, uint32_t box_rows, CUtensorMap* out);
 
 namespace tc {
 
