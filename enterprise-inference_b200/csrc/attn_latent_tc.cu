@@ -7,20 +7,21 @@
 // The two halves of the value columns are items of their own because O takes all 512 TMEM columns otherwise: the scores are
 // computed twice (1.5 x the operations), and nothing is exchanged between CTAs.
 //
-// What bounds it: the issue and execution of 36 score MMAs of 64 columns a tile (about 1.9 us per tile, krow 576), then the query
+// What bounds it: the issue and execution of 36 score MMAs of 64 columns a tile (about 1.6 us per tile, krow 576), then the query
 // staging and the output at an item's ends.  Q is the large operand (krow 576: 147 KB of bf16), so the part that matches the value
 // columns lives in TMEM (columns 384..511, A operand read from there) and only the rest in shared memory, which leaves room for
-// three stages of value columns and a tile of the other columns.  TMEM: O 0..255, two score buffers of 64 columns, the Q part.
+// two tiles of keys.  TMEM: O 0..255, two score buffers of 64 columns, the Q part.
 // The weights overwrite the scores in place (A operand of the second product, per 32 scores 16 columns of bf16 pairs and 16 of what
 // rounding took from them) and never touch shared memory.
 // Against the mma.sync kernel of attn_latent.cu with 16 pairs a CTA, which reads every key tile once per row: 2 048 rows of 16
-// heads over 512 + 64 at contexts 1..2048 907 -> 187 us; error against 64 bits 2.57e-3 -> 2.30e-3 (decode rows: attn_latent_rows.cu).  (With weights of one bf16 term, as there, about a tenth faster, but 2.61e-3 and 2.72e-3: the
+// heads over 512 + 64 at contexts 1..2048 907 -> 157 us; error against 64 bits 2.57e-3 -> 2.30e-3 (decode rows: attn_latent_rows.cu).  (With weights of one bf16 term, as there, about a tenth faster, but 2.61e-3 and 2.72e-3: the
 // lazily followed maximum costs the exactness of the largest weight.)
 // Warps: TMA producer, MMA issuer, four softmax warps (a thread owns a pair), eight that stage the next item's queries.
 // The running maximum is only followed when it rises by more than 2^8 (the scaling of all terms is the same, so the
 // quotient is exact); a warp then rescales its own 32 rows of O in TMEM.
 // Every wait is bounded and reported (tc.cuh).
 #include <algorithm>
+#include <type_traits>
 
 #include "tc.cuh"
 
@@ -32,10 +33,13 @@ using namespace tc;
 constexpr int kLtKeys = 64, kLtPairs = 128, kLtThreads = 448;
 constexpr int kLtChunk = kLtKeys * 128;        // [64 keys][64 columns] bf16: 8 KiB
 constexpr int kLtQChunk = kLtPairs * 128;      // [128 pairs][64 columns] bf16: 16 KiB
-constexpr int kLtMaxStages = 4, kLtMaxRest = 5, kLtMaxSlots = 12;
+constexpr int kLtMaxStages = 4, kLtMaxRest = 5, kLtMaxRestStages = 4;
 constexpr int kLtSmem = 232448, kLtTail = 2048;
 constexpr int kLtTable = 32;                   // items of a CTA whose description is worked out ahead
 constexpr uint32_t kTmS = 256, kTmQ = 384;     // TMEM columns: O at 0, scores (then weights) of even / odd tiles, Q part
+
+// value columns of the first half: of more than 256, half of the 64-wide chunks
+__host__ __device__ __forceinline__ int lt_width0(int rank) { return rank > 256 ? (rank + 127) / 128 * 64 : rank; }
 
 struct LtParams {
   const float* q;
@@ -48,7 +52,7 @@ struct LtParams {
   __nv_bfloat16* out;
   float* part;
   uint32_t* status;
-  int n_rows, bt_stride, heads, krow, rank, block_size, n_splits, window, own_stages, rest_slots, halves, rows_per_item, items_per_run;
+  int n_rows, bt_stride, heads, krow, rank, block_size, n_splits, window, own_stages, rest_stages, halves, rows_per_item, items_per_run;
   float scale;
 };
 
@@ -87,17 +91,17 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int chunks = (p.krow + 63) >> 6, ksteps = p.krow >> 4;
   // value columns of a half and the chunks that hold them (the largest half decides the layout of shared memory)
-  const int width0 = min(p.rank, 256), own0 = (width0 + 63) >> 6;
-  const int width1 = p.halves > 1 ? p.rank - 256 : width0, own1 = (width1 + 63) >> 6;
+  const int width0 = lt_width0(p.rank), own0 = (width0 + 63) >> 6;
+  const int width1 = p.halves > 1 ? p.rank - width0 : width0, own1 = (width1 + 63) >> 6;
   const int max_rest = chunks - min(own0, own1), max_own = max(own0, own1);
   unsigned char* qs = smem;                                  // [max_rest][128][64] queries of the columns outside the half
   unsigned char* own_ring = qs + max_rest * kLtQChunk;       // [own_stages][max_own][64][64] value columns of a tile
-  unsigned char* rest_ring = own_ring + p.own_stages * max_own * kLtChunk;   // [rest_slots][64][64] the tile's other chunks
-  uint64_t* own_full = reinterpret_cast<uint64_t*>(rest_ring + p.rest_slots * kLtChunk);
+  unsigned char* rest_ring = own_ring + p.own_stages * max_own * kLtChunk;   // [rest_stages][max_rest][64][64] a tile's other chunks
+  uint64_t* own_full = reinterpret_cast<uint64_t*>(rest_ring + p.rest_stages * max_rest * kLtChunk);
   uint64_t* own_free = own_full + kLtMaxStages;
   uint64_t* rest_full = own_free + kLtMaxStages;
-  uint64_t* rest_free = rest_full + kLtMaxSlots;
-  uint64_t* s_full = rest_free + kLtMaxSlots;    // [2]
+  uint64_t* rest_free = rest_full + kLtMaxRestStages;
+  uint64_t* s_full = rest_free + kLtMaxRestStages;    // [2]
   uint64_t* p_ready = s_full + 2;                // [2]
   uint64_t* o_full = p_ready + 2;                // [2]
   uint64_t* q_ready = o_full + 2;
@@ -111,7 +115,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
       mbar_init(own_full + s, 1);
       mbar_init(own_free + s, 1);
     }
-    for (int s = 0; s < p.rest_slots; ++s) {
+    for (int s = 0; s < p.rest_stages; ++s) {
       mbar_init(rest_full + s, 1);
       mbar_init(rest_free + s, 1);
     }
@@ -161,19 +165,19 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
     for (int it = blockIdx.x; it < n_items && !stop; it += gridDim.x) {
       LtItem w;
       if (!next_item(it, w)) continue;
-      const int own = w.half ? own1 : own0, first = w.half * 4, rest = chunks - own;
+      const int own = w.half ? own1 : own0, first = w.half * own0, rest = chunks - own;
       const int32_t* bt = p.block_table + (int64_t)w.seq * p.bt_stride;
       for (int i = w.tile_lo; i < w.tile_hi && !(stop = mbar_wait.stop()); ++i) {
         const int tok = i * kLtKeys;
         const int blk = __shfl_sync(0xffffffffu, __ldg(bt + tok / p.block_size), 0);
         const int row = blk * p.block_size + tok % p.block_size;
-        for (int c = 0; c < rest; ++c) {
+        if (rest > 0) {
           mbar_wait(rest_free + sl, sl_ph);
           if (issuer) {
-            mbar_expect_tx(rest_full + sl, kLtChunk);
-            tma_load_2d(rest_ring + sl * kLtChunk, &map, (c < first ? c : c + own) * 64, row, rest_full + sl);
+            mbar_expect_tx(rest_full + sl, rest * kLtChunk);
+            for (int c = 0; c < rest; ++c) tma_load_2d(rest_ring + (sl * max_rest + c) * kLtChunk, &map, (c < first ? c : c + own) * 64, row, rest_full + sl);
           }
-          if (++sl == p.rest_slots) sl = 0, sl_ph ^= 1;
+          if (++sl == p.rest_stages) sl = 0, sl_ph ^= 1;
         }
         mbar_wait(own_free + st, st_ph);
         if (issuer) {
@@ -186,7 +190,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
     }
     if (mbar_wait.stop()) {   // the loads in flight: a slot's last one filled it in this round of the ring or in the one before
       for (int s = 0; s < p.own_stages; ++s) mbar_wait.drain(own_full + s, s < st ? st_ph ^ 1 : st_ph);
-      for (int s = 0; s < p.rest_slots; ++s) mbar_wait.drain(rest_full + s, s < sl ? sl_ph ^ 1 : sl_ph);
+      for (int s = 0; s < p.rest_stages; ++s) mbar_wait.drain(rest_full + s, s < sl ? sl_ph ^ 1 : sl_ph);
     }
   } else if (warp == 1) {
     // ===== MMA: the scores of tile n + 1 are issued before the weights of tile n are waited for.  The whole warp walks the loop; bounds
@@ -204,42 +208,89 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
       const int nt = __shfl_sync(0xffffffffu, have ? w.tile_hi - w.tile_lo : 0, 0);
       if (nt <= 0) continue;
       const int half = __shfl_sync(0xffffffffu, w.half, 0);
-      const int own = half ? own1 : own0, first = half * 4, rest = chunks - own;
+      const int own = half ? own1 : own0, first = half * own0, rest = chunks - own;
       const uint32_t id_s = idesc_bf16(kLtKeys, 0), id_o = idesc_bf16(half ? width1 : width0, 1);
-      auto issue_s = [&](int n) {
+      // Issuing is what bounds the walk (with MMAs a quarter as wide it took as long), and branches between the MMAs cost it: straight code for
+      // the usual shapes, and straight blocks of chunks and of what is left of the last one for the others (2 048 rows of 16 heads, 512 + 64:
+      // 184 us with a branch and a wait per chunk, 171 with the straight blocks, 157 with straight code)
+      const int own_steps = min(own * 4, ksteps - first * 4), rest_steps = ksteps - own_steps;
+      auto issue_rest = [&](auto steps_c, int c, uint32_t d, uint64_t dr) {   // from chunk c of the others on
+        const uint64_t da = desc_q + (uint64_t)((c * kLtQChunk) >> 4), db = dr + (uint64_t)((c * kLtChunk) >> 4);
+#pragma unroll
+        for (int j = 0; j < decltype(steps_c)::value; ++j)
+          mma_ss(one, d, da + (uint64_t)(((j >> 2) * kLtQChunk >> 4) + (j & 3) * 2), db + (uint64_t)(((j >> 2) * kLtChunk >> 4) + (j & 3) * 2), id_s, c || j ? 1u : 0u);
+      };
+      auto issue_own = [&](auto steps_c, int c, uint32_t d, uint64_t dk) {
+#pragma unroll
+        for (int j = 0; j < decltype(steps_c)::value; ++j)
+          mma_ts(one, d, tm + kTmQ + c * 32 + j * 8, dk + (uint64_t)(((c + (j >> 2)) * kLtChunk >> 4) + (j & 3) * 2), id_s, rest_steps || c || j ? 1u : 0u);
+      };
+      auto issue_whole = [&](auto own_c, auto rest_c, int n) {
         const uint32_t d = tm + kTmS + (n & 1) * kLtKeys;
-        for (int c = 0; c < rest; ++c) {
-          const int col = c < first ? c : c + own, ks = min(4, ksteps - col * 4);
+        if constexpr (decltype(rest_c)::value > 0) {
           mbar_wait(rest_full + sl, sl_ph);
           fence_after();
-          const uint64_t da = desc_q + (uint64_t)((c * kLtQChunk) >> 4), db = desc_rest + (uint64_t)((sl * kLtChunk) >> 4);
-          const uint32_t acc = c ? 1u : 0u;
-          if (ks == 4) {   // unrolled: descriptors are a uniform base plus a constant
-#pragma unroll
-            for (int j = 0; j < 4; ++j) mma_ss(one, d, da + j * 2, db + j * 2, id_s, j ? 1u : acc);
-          } else {
-            for (int j = 0; j < ks; ++j) mma_ss(one, d, da + j * 2, db + j * 2, id_s, j ? 1u : acc);
-          }
+          issue_rest(rest_c, 0, d, desc_rest + (uint64_t)((sl * max_rest * kLtChunk) >> 4));
           commit(one, rest_free + sl);
-          if (++sl == p.rest_slots) sl = 0, sl_ph ^= 1;
+          if (++sl == p.rest_stages) sl = 0, sl_ph ^= 1;
         }
         mbar_wait(own_full + st, st_ph);
         fence_after();
-        const uint64_t dk = desc_own + (uint64_t)((st * max_own * kLtChunk) >> 4);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          if (c >= own) break;
-          const int ks = min(4, ksteps - (first + c) * 4);
-          const uint32_t acc = c || rest ? 1u : 0u;
-          if (ks == 4) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) mma_ts(one, d, tm + kTmQ + c * 32 + j * 8, dk + ((c * kLtChunk) >> 4) + j * 2, id_s, j ? 1u : acc);
-          } else {
-            for (int j = 0; j < ks; ++j) mma_ts(one, d, tm + kTmQ + c * 32 + j * 8, dk + ((c * kLtChunk) >> 4) + j * 2, id_s, j ? 1u : acc);
+        issue_own(own_c, 0, d, desc_own + (uint64_t)((st * max_own * kLtChunk) >> 4));
+        commit(one, s_full + (n & 1));
+        if (++st == p.own_stages) st = 0, st_ph ^= 1;
+      };
+      auto issue_any = [&](int n) {
+        const uint32_t d = tm + kTmS + (n & 1) * kLtKeys;
+        if (rest > 0) {
+          const uint64_t dr = desc_rest + (uint64_t)((sl * max_rest * kLtChunk) >> 4);
+          const int whole = rest_steps >> 2;
+          mbar_wait(rest_full + sl, sl_ph);
+          fence_after();
+          if (whole == 5) issue_rest(std::integral_constant<int, 20>(), 0, d, dr);
+          else if (whole == 4) issue_rest(std::integral_constant<int, 16>(), 0, d, dr);
+          else if (whole == 3) issue_rest(std::integral_constant<int, 12>(), 0, d, dr);
+          else if (whole == 2) issue_rest(std::integral_constant<int, 8>(), 0, d, dr);
+          else if (whole == 1) issue_rest(std::integral_constant<int, 4>(), 0, d, dr);
+          switch (rest_steps & 3) {
+            case 1: issue_rest(std::integral_constant<int, 1>(), whole, d, dr); break;
+            case 2: issue_rest(std::integral_constant<int, 2>(), whole, d, dr); break;
+            case 3: issue_rest(std::integral_constant<int, 3>(), whole, d, dr); break;
           }
+          commit(one, rest_free + sl);
+          if (++sl == p.rest_stages) sl = 0, sl_ph ^= 1;
+        }
+        const uint64_t dk = desc_own + (uint64_t)((st * max_own * kLtChunk) >> 4);
+        const int whole = own_steps >> 2;
+        mbar_wait(own_full + st, st_ph);
+        fence_after();
+        if (whole == 4) issue_own(std::integral_constant<int, 16>(), 0, d, dk);
+        else if (whole == 3) issue_own(std::integral_constant<int, 12>(), 0, d, dk);
+        else if (whole == 2) issue_own(std::integral_constant<int, 8>(), 0, d, dk);
+        else if (whole == 1) issue_own(std::integral_constant<int, 4>(), 0, d, dk);
+        switch (own_steps & 3) {
+          case 1: issue_own(std::integral_constant<int, 1>(), whole, d, dk); break;
+          case 2: issue_own(std::integral_constant<int, 2>(), whole, d, dk); break;
+          case 3: issue_own(std::integral_constant<int, 3>(), whole, d, dk); break;
         }
         commit(one, s_full + (n & 1));
         if (++st == p.own_stages) st = 0, st_ph ^= 1;
+      };
+      auto issue_s = [&](int n) {
+        using std::integral_constant;
+        switch (own_steps * 32 + rest_steps) {
+          case 16 * 32 + 20: issue_whole(integral_constant<int, 16>(), integral_constant<int, 20>(), n); break;   // 512 + 64
+          case 16 * 32 + 18: issue_whole(integral_constant<int, 16>(), integral_constant<int, 18>(), n); break;   // 512 + 32
+          case 16 * 32 + 16: issue_whole(integral_constant<int, 16>(), integral_constant<int, 16>(), n); break;   // 512
+          case 12 * 32 + 16: issue_whole(integral_constant<int, 12>(), integral_constant<int, 16>(), n); break;   // 384 + 64
+          case 12 * 32 + 10: issue_whole(integral_constant<int, 12>(), integral_constant<int, 10>(), n); break;   // 320 + 32, first half
+          case 8 * 32 + 14: issue_whole(integral_constant<int, 8>(), integral_constant<int, 14>(), n); break;     // and second
+          case 16 * 32 + 4: issue_whole(integral_constant<int, 16>(), integral_constant<int, 4>(), n); break;     // 256 + 64
+          case 16 * 32 + 2: issue_whole(integral_constant<int, 16>(), integral_constant<int, 2>(), n); break;     // 256 + 32
+          case 16 * 32: issue_whole(integral_constant<int, 16>(), integral_constant<int, 0>(), n); break;         // 256
+          case 8 * 32 + 4: issue_whole(integral_constant<int, 8>(), integral_constant<int, 4>(), n); break;       // 128 + 64
+          default: issue_any(n);
+        }
       };
       mbar_wait(q_ready, active & 1);
       fence_after();
@@ -278,7 +329,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
     for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
       LtItem w;
       if (!next_item(it, w) || w.tile_hi <= w.tile_lo) continue;
-      const int own = w.half ? own1 : own0, first = w.half * 4, rest = chunks - own;
+      const int own = w.half ? own1 : own0, first = w.half * own0, rest = chunks - own;
       const int live = w.nr * p.heads;
       const float* qbase = p.q + (int64_t)w.t0 * p.heads * p.krow;   // pair m = (row m / heads, head m % heads): row m of this
       // four lanes take 64 neighbouring bytes of a row, eight rows per load: the fragment layout of the 16-lane store
@@ -441,7 +492,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
             ld_wait<16>(o);
           }
           if (alive) {
-            float2* d2 = reinterpret_cast<float2*>(dst + w.half * 256 + c);   // rank + 2 is even: 8-byte aligned rows
+            float2* d2 = reinterpret_cast<float2*>(dst + w.half * width0 + c);   // rank + 2 is even: 8-byte aligned rows
 #pragma unroll
             for (int j = 0; j < 8; ++j) d2[j] = any ? make_float2(__uint_as_float(o[2 * j]), __uint_as_float(o[2 * j + 1])) : make_float2(0.f, 0.f);
           }
@@ -454,7 +505,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
           l = l * f + exp2_fast(sk - mn);
         }
         const float inv = l > 0.f ? f / l : 0.f;
-        __nv_bfloat16* dst = p.out + pair * p.rank + w.half * 256;
+        __nv_bfloat16* dst = p.out + pair * p.rank + w.half * width0;
         for (int c = 0; c < width; c += 16) {
           uint32_t o[16], v[8];
           if (any) {
@@ -480,22 +531,23 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
 }
 
 struct LtShape {
-  int halves, own_stages, rest_slots;
+  int halves, own_stages, rest_stages;
 };
-// false: a shape whose queries or key tiles do not fit beside each other.  Three stages of value columns keep the loads of a tile
-// (freed by its second product) off the chain of the next ones (2 048 rows of 16 heads, 512 + 64: 2.2 us a tile with two stages);
-// the other chunks are freed earlier, a tile and one chunk of them is enough.
+// false: a shape whose queries or key tiles do not fit beside each other.  The other chunks of a tile share a
+// stage: one wait and one commit a tile, so that the MMAs of a shape stand in straight code (2 048 rows of 16 heads: 512 + 64 184 -> 157 us,
+// 512 + 0 169 -> 145, 384 + 64 156 -> 127 with halves of three chunks instead of four and two; 3 x 683 rows at 1 000, 256 + 32 111 -> 99).
 bool lt_shape(int heads, int krow, int rank, LtShape& s) {
   if (heads < 1 || heads > kLtPairs || krow % 16 || rank % 16 || rank < 16 || rank > 512 || rank > krow) return false;
   s.halves = latent_attn_tc_halves(rank);
-  const int chunks = (krow + 63) / 64, own0 = (std::min(rank, 256) + 63) / 64, own1 = s.halves > 1 ? (rank - 256 + 63) / 64 : own0;
+  const int chunks = (krow + 63) / 64, own0 = (lt_width0(rank) + 63) / 64, own1 = s.halves > 1 ? (rank - own0 * 64 + 63) / 64 : own0;
   const int max_rest = chunks - std::min(own0, own1), max_own = std::max(own0, own1);
   if (max_rest > kLtMaxRest) return false;
   const int slots = (kLtSmem - 1024 - kLtTail - max_rest * kLtQChunk) / kLtChunk;
-  for (s.own_stages = kLtMaxStages; s.own_stages >= 2; --s.own_stages) {
-    s.rest_slots = std::min(slots - s.own_stages * max_own, kLtMaxSlots);
-    if (s.rest_slots >= max_rest + 1) return true;
-  }
+  for (s.own_stages = kLtMaxStages; s.own_stages >= 2; --s.own_stages)
+    if (s.own_stages * max_own + 2 * max_rest <= slots) {   // (two of either always fit)
+      s.rest_stages = max_rest ? std::min((slots - s.own_stages * max_own) / max_rest, kLtMaxRestStages) : 1;
+      return true;
+    }
   return false;
 }
 
@@ -539,7 +591,7 @@ int latent_attn_tc(const float* q, const __nv_bfloat16* kc, const int32_t* block
   p.n_splits = n_splits;
   p.window = window;
   p.own_stages = sh.own_stages;
-  p.rest_slots = sh.rest_slots;
+  p.rest_stages = sh.rest_stages;
   p.halves = sh.halves;
   p.rows_per_item = std::min(kLtPairs / heads, 16);   // a run has at most 16 rows
   p.items_per_run = (16 + p.rows_per_item - 1) / p.rows_per_item;
