@@ -13,11 +13,13 @@
 // Scores may be capped, biased by distance (each score takes its own distance's bias and no other: tables may end in -inf or any sentinel),
 // windowed with kept first keys (EX); outputs may have a sink in the denominator and a gate per head.  The running maximum is only followed when it rises by more than 2^8 (exact: all terms are scaled alike); a warp then
 // rescales its 32 rows of O in TMEM.
-// Bound by the tensor core or the softmax's issue slots: 2 048 rows at contexts 1001..3048, 32 heads over 8: 118 us (212 us); 1 900
+// Bound by the tensor core or the softmax's issue slots: 2 048 rows at contexts 1001..3048, 32 heads over 8: 108 us (112 with branches between the
+// issuing warp's MMAs and the maximum of a key tile in one chain, 212 on the kernel before); 1 900
 // rows of three sequences, 16 heads over 4, capped, biased, window 1024: 76 us (278 us on the mma.sync kernel of attn_latent.cu).
 // Warps: four softmax warps per tile (a thread owns a pair), TMA, MMA, two that stage queries.  Every wait is bounded and
 // reported (tc.cuh).
 #include <algorithm>
+#include <type_traits>
 
 #include "runs.cuh"
 #include "tc.cuh"
@@ -269,16 +271,18 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     const int ksteps = p.dim >> 4;
     int slot = 0, active = 0, n[2] = {0, 0};   // n: key tiles walked by either tile of pairs so far
     uint32_t ph = 0;
-    RowsWork w;
-    for (int k = 0; __shfl_sync(0xffffffffu, next_work(k, w), 0);) {
-      const int nt = __shfl_sync(0xffffffffu, w.hi - w.lo, 0), tiles = __shfl_sync(0xffffffffu, w.nrows > R ? 2 : 1, 0);
-      if (nt <= 0) continue;
+    auto next_slot = [&]() {
+      if (++slot == kArSlots) slot = 0, ph ^= 1;
+    };
+    // an item of nt key tiles: straight code for either count of pair tiles and for the widest heads (branches between the MMAs cost the issuing warp)
+    auto walk = [&](auto tiles_c, auto steps_c, int nt) {
+      constexpr int TILES = decltype(tiles_c)::value, STEPS = decltype(steps_c)::value;
       auto scores = [&](int x, int nx, int k_slot) {
         const uint64_t da = desc_q + (uint64_t)((x * 2 * kArQChunk) >> 4), db = desc_k + (uint64_t)((k_slot * kArTile) >> 4);
         const uint32_t d = tm + x * 256 + (nx & 1) * kArKeys;
-        if (ksteps == 8) {
+        if constexpr (STEPS > 0) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
+          for (int j = 0; j < STEPS; ++j)
             mma_ss(one, d, da + ((j >> 2) * kArQChunk + (j & 3) * 32) / 16, db + ((j >> 2) * kArChunk + (j & 3) * 32) / 16, id_s, j ? 1u : 0u);
         } else {
           for (int j = 0; j < ksteps; ++j)
@@ -286,54 +290,62 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         }
         commit(one, s_full + 2 * x + (nx & 1));
       };
-      auto next_slot = [&]() {
-        if (++slot == kArSlots) slot = 0, ph ^= 1;
-      };
-      if (active == 0) mbar_wait(q_first, 0);
-      else mbar_wait(q_ready, (active - 1) & 1);
       mbar_wait(kv_full + slot, ph);
       fence_after();
       int k_slot = slot;
       next_slot();
-      scores(0, n[0], k_slot);
-      if (tiles == 2) scores(1, n[1], k_slot);
+#pragma unroll
+      for (int x = 0; x < TILES; ++x) scores(x, n[x], k_slot);
       commit(one, kv_free + k_slot);
-      if (nt == 1) commit(one, q_free);
-      for (int i = 0; i < nt; ++i) {
+      commit(nt == 1 ? one : 0u, q_free);
+      auto step = [&](auto more_c, int i) {
+        constexpr bool MORE = decltype(more_c)::value;
         const int v_slot = slot;
         const uint32_t v_ph = ph;
         next_slot();
-        const bool more = i + 1 < nt;
-        if (more) {
+        if constexpr (MORE) {
           mbar_wait(kv_full + slot, ph);
           fence_after();
           k_slot = slot;
           next_slot();
         }
+        const uint64_t dv = desc_v + (uint64_t)((v_slot * kArTile) >> 4);
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          if (x >= tiles) break;
-          if (more) {
-            scores(x, n[x] + 1, k_slot);
-            if (x == tiles - 1) {
-              commit(one, kv_free + k_slot);
-              if (i + 2 == nt) commit(one, q_free);   // the item's last scores are on their way
-            }
+        for (int x = 0; x < TILES; ++x) {
+          if constexpr (MORE) scores(x, n[x] + 1, k_slot);
+          if (MORE && x == TILES - 1) {
+            commit(one, kv_free + k_slot);
+            commit(i + 2 == nt ? one : 0u, q_free);   // the item's last scores are on their way
           }
           if (x == 0) mbar_wait(kv_full + v_slot, v_ph);
           mbar_wait(p_ready + 2 * x + (n[x] & 1), (n[x] >> 1) & 1);
           fence_after();
-          const uint64_t dv = desc_v + (uint64_t)((v_slot * kArTile) >> 4);
           const uint32_t pa = tm + x * 256 + (n[x] & 1) * kArKeys, d = tm + x * 256 + 128;
 #pragma unroll
           for (int j = 0; j < 4; ++j) {   // 16 keys per step: 8 columns of weights, 16 further those of the second term
             mma_ts(one, d, pa + (j >> 1) * 32 + (j & 1) * 8, dv + (uint64_t)((j * 2048) >> 4), id_o, (i | j) ? 1u : 0u);
             mma_ts(one, d, pa + (j >> 1) * 32 + (j & 1) * 8 + 16, dv + (uint64_t)((j * 2048) >> 4), id_o, 1u);
           }
-          if (x == tiles - 1) commit(one, kv_free + v_slot);
+          if (x == TILES - 1) commit(one, kv_free + v_slot);
           commit(one, o_full + 2 * x + (n[x] & 1));
           ++n[x];
         }
+      };
+      for (int i = 0; i + 1 < nt; ++i) step(std::true_type(), i);
+      step(std::false_type(), nt - 1);
+    };
+    RowsWork w;
+    for (int k = 0; __shfl_sync(0xffffffffu, next_work(k, w), 0);) {
+      const int nt = __shfl_sync(0xffffffffu, w.hi - w.lo, 0), tiles = __shfl_sync(0xffffffffu, w.nrows > R ? 2 : 1, 0);
+      if (nt <= 0) continue;
+      if (active == 0) mbar_wait(q_first, 0);
+      else mbar_wait(q_ready, (active - 1) & 1);
+      if (tiles == 2) {
+        if (ksteps == 8) walk(std::integral_constant<int, 2>(), std::integral_constant<int, 8>(), nt);
+        else walk(std::integral_constant<int, 2>(), std::integral_constant<int, 0>(), nt);
+      } else {
+        if (ksteps == 8) walk(std::integral_constant<int, 1>(), std::integral_constant<int, 8>(), nt);
+        else walk(std::integral_constant<int, 1>(), std::integral_constant<int, 0>(), nt);
       }
       ++active;
     }
@@ -445,9 +457,7 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
           for (int j = 0; j < 64; ++j)
             if (j >= j_hi || (j < j_lo && !(EX && k0 + j < keep))) s[j] = 0xff800000u;   // -inf
         }
-        float mx = -INFINITY;
-#pragma unroll
-        for (int j = 0; j < 64; ++j) mx = fmaxf(mx, __uint_as_float(s[j]));
+        float mx = max64(s);
         if (!EX) mx *= sc2;
         const bool jump = mx > mu + 8.f;   // also the first live key (mu = -inf)
         if (__any_sync(0xffffffffu, jump)) {
@@ -468,7 +478,7 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
           mu = mn;
         }
         const float mref = mu > -INFINITY ? mu : 0.f;
-        float sum[2] = {0.f, 0.f};
+        float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           uint32_t pk[32];
@@ -477,14 +487,14 @@ attn_rows_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
             const float s0 = __uint_as_float(s[c * 32 + 2 * j]), s1 = __uint_as_float(s[c * 32 + 2 * j + 1]);
             const float p0 = exp2_fast(EX ? s0 - mref : fmaf(s0, sc2, -mref)), p1 = exp2_fast(EX ? s1 - mref : fmaf(s1, sc2, -mref));
             // the high term truncated, the rest rounded
-            sum[j & 1] += p0 + p1;
+            sum[j & 3] += p0 + p1;
             const uint32_t h0 = __float_as_uint(p0) & 0xffff0000u, h1 = __float_as_uint(p1) & 0xffff0000u;
             pk[j] = __byte_perm(h0, h1, 0x7632);
             pk[16 + j] = pack_bf16(p0 - __uint_as_float(h0), p1 - __uint_as_float(h1));
           }
           st32(s_addr + c * 32, pk);
         }
-        l += sum[0] + sum[1];
+        l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
         if (x == 0) {
           const int n_valid = w.ctx_max - k0;
           if (n_valid < kArKeys) {

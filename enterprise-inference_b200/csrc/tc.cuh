@@ -185,6 +185,15 @@ __device__ __forceinline__ void store_sector(void* p, const uint32_t* v) {
                "r"(v[6]), "r"(v[7])
                : "memory");
 }
+// the largest of 64 scores, in eight chains (one would be 64 dependent steps)
+__device__ __forceinline__ float max64(const uint32_t* s) {
+  float m[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) m[j] = __uint_as_float(s[j]);
+#pragma unroll
+  for (int j = 8; j < 64; ++j) m[j & 7] = fmaxf(m[j & 7], __uint_as_float(s[j]));
+  return fmaxf(fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])), fmaxf(fmaxf(m[4], m[5]), fmaxf(m[6], m[7])));
+}
 // 2^x on the hardware's exponential
 __device__ __forceinline__ float exp2_fast(float x) {
   float y;
