@@ -933,6 +933,7 @@ int linear_tc(const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, const
 // x [n_tiles * N][k] holds the gathered token rows, each expert's run padded to whole tiles of N rows; tile j belongs to
 // expert tile_expert[j] (device array; -1: unused).  w is [experts][n_out][k].  y != null: y[row][n_out] = bf16(x . w_e^T);
 // y == null: out[row_pair[row]][n_out] = (x . w_e^T) * wts[row_pair[row]] in fp32 (padding rows carry row_pair < 0).
+// (128: more than 64 rows an expert, gemm_pair.cu's)
 int linear_tc_grouped_tile(int pairs, int experts) {
   const int avg = (pairs + experts - 1) / std::max(experts, 1);
   return avg <= 16 ? 16 : (avg <= 32 ? 32 : (avg <= 64 ? 64 : 128));
@@ -954,7 +955,7 @@ int linear_tc_grouped_gate_up(const __nv_bfloat16* x, int64_t ldx, int N, int n_
   B200_REQUIRE(x && w && y && tile_expert && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 &&
                    ldx % 8 == 0,
                B200_ERR_INVALID, "linear_tc_grouped_gate_up: operands must be 16-byte aligned");
-  B200_REQUIRE(N == 16 || N == 32 || N == 64 || N == 128, B200_ERR_INVALID, "linear_tc_grouped_gate_up: token tile %d", N);
+  B200_REQUIRE(N == 16 || N == 32 || N == 64, B200_ERR_INVALID, "linear_tc_grouped_gate_up: token tile %d", N);
   B200_REQUIRE(n_tiles > 0 && n_tiles <= 65535 && experts > 0, B200_ERR_INVALID, "linear_tc_grouped_gate_up: %d tiles", n_tiles);
   Plan pl;
   pl.N = N;
@@ -984,8 +985,7 @@ int linear_tc_grouped_gate_up(const __nv_bfloat16* x, int64_t ldx, int N, int n_
   switch (N) {
     case 16: return launch_grouped_silu<16>(mw, mx, p, pl, s);
     case 32: return launch_grouped_silu<32>(mw, mx, p, pl, s);
-    case 64: return launch_grouped_silu<64>(mw, mx, p, pl, s);
-    default: return launch_grouped_silu<128>(mw, mx, p, pl, s);
+    default: return launch_grouped_silu<64>(mw, mx, p, pl, s);
   }
 }
 
@@ -1002,7 +1002,7 @@ int linear_tc_grouped(const __nv_bfloat16* x, int64_t ldx, int N, int n_tiles, c
   B200_REQUIRE(x && w && tile_expert && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 &&
                    ldx % 8 == 0,
                B200_ERR_INVALID, "linear_tc_grouped: operands must be 16-byte aligned");
-  B200_REQUIRE(N == 16 || N == 32 || N == 64 || N == 128, B200_ERR_INVALID, "linear_tc_grouped: token tile %d", N);
+  B200_REQUIRE(N == 16 || N == 32 || N == 64, B200_ERR_INVALID, "linear_tc_grouped: token tile %d", N);
   B200_REQUIRE(n_tiles > 0 && n_tiles <= 65535 && experts > 0, B200_ERR_INVALID, "linear_tc_grouped: %d tiles", n_tiles);
   B200_REQUIRE(y || (row_pair && wts && out && reinterpret_cast<uintptr_t>(out) % 16 == 0), B200_ERR_INVALID,
                "linear_tc_grouped: no destination");
@@ -1037,8 +1037,7 @@ int linear_tc_grouped(const __nv_bfloat16* x, int64_t ldx, int N, int n_tiles, c
   switch (N) {
     case 16: return launch_grouped<16>(scatter, mw, mx, p, pl, s);
     case 32: return launch_grouped<32>(scatter, mw, mx, p, pl, s);
-    case 64: return launch_grouped<64>(scatter, mw, mx, p, pl, s);
-    default: return launch_grouped<128>(scatter, mw, mx, p, pl, s);
+    default: return launch_grouped<64>(scatter, mw, mx, p, pl, s);
   }
 }
 

@@ -13,7 +13,7 @@
 //    slot), and one CTA per (expert, tile of 16 of its tokens) streams the expert's weights once for the whole tile.
 //  * tensor-core form (bf16 serving mode, width and ff multiples of 8; every step size): the (token, slot) pairs are
 //    grouped by expert into whole token tiles, the token rows gathered, and two launches of the grouped tcgen05 linear
-//    (gemm_tc.cu) run gate|up and down for all experts at once; the second one scatters the weighted fp32 rows.
+//    (gemm_tc.cu; many rows an expert: gemm_pair.cu, on pairs of SMs) run gate|up and down for all experts at once; the second one scatters the weighted fp32 rows.
 // Score mode 1 scores every expert with the sigmoid of its logit.  RouteForm: a group may count by the sum of its two largest choice
 // scores, the chosen weights may be divided by their sum, and one more router row may gate a shared expert (its sigmoid per token).
 // Score mode 2 (chosen-softmax router): the bias is part of the logits, the `top` largest logits win and the mixing weights are
