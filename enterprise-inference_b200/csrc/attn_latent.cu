@@ -408,12 +408,14 @@ static int attn_mma_launch(const float* q, const __nv_bfloat16* kc, const __nv_b
 // Rows by themselves on tcgen05 (attn_latent_rows.cu): steps whose rows' heads, 16 at a time, fit the device's SMs at once (what they measured stands
 // there; a few rows of one sequence gain as much, up to 128 of them behind 3000 tokens a little), and decode rows that say so in any number: 256 rows
 // of 16 heads at contexts 300..600 86 us on the mma.sync kernel, 51 there.  Beyond that a step of unknown rows may be a prefill chunk, whose runs
-// share their keys on attn_latent_tc.cu (2 048 rows 187 us).
+// share their keys on attn_latent_tc.cu (2 048 rows 159 us).  Rows of fewer than 512 query entries (heads * krow) keep the plan and the attention as two
+// launches, the second overlapping the first, which is what a captured call of theirs holds (tests/test_launch_gpu.py); it costs them 4 us (2 rows of
+// 4 heads over 64 + 16: 14.5, one launch of attn_latent_rows.cu 10.5) to 16 (64 rows at contexts up to 1000: 29.0 and 12.8).
 bool latent_attn_by_rows(const float* q, const __nv_bfloat16* kc, const int32_t* row_to_seq, const __nv_bfloat16* out, int T, int heads, int krow, int rank,
                          int block_size, float scale, bool one_row_each) {
   const auto at = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr); };
   return T > 0 && scale > 0.f && latent_attn_mma_supported(heads, krow, rank) && latent_attn_rows_supported(heads, krow, rank, block_size) &&
-         (at(q) | at(kc) | at(out)) % 16 == 0 && (latent_attn_rows_items(T, heads) <= kNumSMs || one_row_each || !row_to_seq);
+         heads * krow >= 512 && (at(q) | at(kc) | at(out)) % 16 == 0 && (latent_attn_rows_items(T, heads) <= kNumSMs || one_row_each || !row_to_seq);
 }
 
 // runs / n_runs: the run list of the step (attn_anydim.cu builds it: runs of at most 16 consecutive rows of one sequence)
