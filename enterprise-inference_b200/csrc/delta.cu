@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(db_threads(LG), CTAS) delta_block_kernel(const
     if (++in_round == per_round) {
       in_round = 0;
       db_cluster_wait();
-      if (++round + 1 < rounds) db_cluster_arrive_relaxed();
+      if (++round + 1 < rounds) db_cluster_arrive();   // (release: the round before's triangles have been read, another CTA's go there)
     }
     db_sync<BAR>(kFull + b % kDbSlots);
     const float* in = stage + (b % kDbSlots) * SLOT;
