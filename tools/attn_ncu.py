@@ -1,6 +1,6 @@
 """One launch of the tcgen05 paged attention per shape, for `ncu --set full -k regex:paged_attn_tc`.
 
-    ncu --set full --clock-control none --import-source on -k regex:paged_attn_tc -o gpurun_out/attn \
+    ncu --set full --clock-control none --import-source on -k regex:paged_attn_tc -o attn \
         python tools/attn_ncu.py
 """
 import importlib, os, sys

@@ -1,5 +1,5 @@
 """One 2048-row prefill chunk (Llama-3.1-8B shapes, ctx 0..2048) for an ncu launch list:
-   ncu --metrics gpu__time_duration.sum --clock-control none -k regex:b200 --csv --log-file gpurun_out/prefill.csv python tools/prefill_once.py
+   ncu --metrics gpu__time_duration.sum --clock-control none -k regex:b200 --csv --log-file prefill.csv python tools/prefill_once.py
 """
 import importlib, os, sys
 import torch
