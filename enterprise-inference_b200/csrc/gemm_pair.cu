@@ -20,6 +20,7 @@
 #include <algorithm>
 
 #include "gemm_epilogue.cuh"
+#include "pair_drain.h"
 #include "tc.cuh"
 
 namespace b200 {
@@ -41,6 +42,43 @@ __device__ __forceinline__ uint32_t smem_of(const void* p, int cta) {   // the s
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(tc::smem_u32(p)), "r"(cta));
   return r;
 }
+// A wait that runs out marks every CTA of the cluster: each serves another's loads, MMAs or sums.  What follows is out of the loops' way, in
+// functions of its own, and the loops' predicates stay what they were (an MMA predicate that a wait may clear: 187 us instead of 196).
+constexpr uint32_t kPairRunning = 0xffffffffu;   // Waits::mark[1] until the CTA's fetching warp has ended, then the fills it issued
+__device__ __noinline__ void pair_gave_up(uint32_t* mark, uint32_t* status, int ctas) {
+  *reinterpret_cast<volatile uint32_t*>(mark) = 1;
+  for (int c = 0; c < ctas; ++c) asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(smem_of(mark, c)), "r"(1u) : "memory");
+  if (status) *reinterpret_cast<volatile uint32_t*>(status) = 1;
+}
+__device__ __forceinline__ uint32_t pair_issued(uint32_t* mark, int cta) {
+  uint32_t v;
+  asm volatile("ld.relaxed.cluster.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(smem_of(mark + 1, cta)) : "memory");
+  return v;
+}
+// before the MMA warp commits anything for a fill that did not land: both fetching warps have ended (they see the mark), so nothing is issued on it
+__device__ __noinline__ void pair_await_ends(uint32_t* mark, int lead, int limit) {
+  for (int i = 0; i < limit && (pair_issued(mark, lead) == kPairRunning || pair_issued(mark, lead + 1) == kPairRunning); ++i) __nanosleep(1000);
+}
+struct PairWaits : tc::Waits {
+  int ctas;
+  __device__ __forceinline__ PairWaits(uint32_t* m, uint32_t* st, int n) : tc::Waits(m, st), ctas(n) {}
+  template <typename F>
+  __device__ __forceinline__ void operator()(uint64_t* bar, uint32_t parity, F&& gave_up) const {
+    for (int i = 0; !tc::mbar_try(bar, parity); ++i)
+      if ((i & 63) == 63 && (marked() || i > limit)) {
+        if (!marked()) pair_gave_up(mark, status, ctas);
+        gave_up();
+        return;
+      }
+  }
+  __device__ __forceinline__ void operator()(uint64_t* bar, uint32_t parity) const { (*this)(bar, parity, [] {}); }
+  // for the whole warp; false: it ran out
+  __device__ __forceinline__ bool all(uint64_t* bar, uint32_t parity) const {
+    if (__all_sync(0xffffffffu, tc::mbar_try(bar, parity))) return true;
+    (*this)(bar, parity);
+    return !stop();
+  }
+};
 __device__ __forceinline__ void pair_load(void* dst, const CUtensorMap* map, int c0, int c1, uint32_t bar, uint64_t policy) {
   asm volatile(
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;" ::"r"(
@@ -116,6 +154,19 @@ __device__ __forceinline__ PairTile pair_tile(const TcParams& p, int t) {
   return r;
 }
 
+// After a wait that ran out, with both CTAs' roles at their ends: the loads in flight land before either gives its shared memory up.
+__device__ __forceinline__ void pair_land(const PairWaits& wait, uint64_t* full, const TcParams& p, uint32_t* mark, int lead, int kbs, int first, int step) {
+#pragma unroll 1
+  for (int s = 0; s < kPairStages; ++s) {
+    const PairOwed o = pair_owed(s, kPairStages, (int)pair_issued(mark, lead), (int)pair_issued(mark, lead + 1));
+    if (o.parity < 0) continue;
+    const uint32_t half = kPairABytes + (uint32_t)pair_tile(p, first + o.fill / kbs * step).n * kBlockK;   // a CTA's bytes of the fill
+    if (o.announce > 0) tc::mbar_expect_tx(&full[s], half);
+    if (o.announce < 0) asm volatile("mbarrier.complete_tx.relaxed.cluster.shared::cta.b64 [%0], %1;" ::"r"(tc::smem_u32(&full[s])), "r"(half) : "memory");
+    wait.drain(&full[s], (uint32_t)o.parity);
+  }
+}
+
 __device__ __forceinline__ void pair_bias(const TcParams& p, int m_tile, int r4, float (&bb)[4]) {
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
@@ -136,7 +187,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   uint64_t* acc_free = acc_full + 2;           // [2] the leader's: both CTAs' epilogue warps
   uint64_t* last = acc_free + 2;               // after a wait that ran out: the MMAs issued before
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(last + 1);
-  uint32_t* mark = tmem_slot + 1;
+  uint32_t* mark = tmem_slot + 1;              // and, behind it, how many fills the CTA issued
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // a cluster: the CTA pairs of one tile, each with its share of k
   const int cta = blockIdx.x % (2 * p.splits), rank = cta & 1, split = cta >> 1, lead = cta - rank;
@@ -154,7 +205,8 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       tc::mbar_init(&acc_free[s], 16);
     }
     tc::mbar_init(last, 1);
-    *mark = 0;
+    mark[0] = 0;
+    mark[1] = kPairRunning;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -167,7 +219,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   tc::fence_after();
   const uint32_t tmem = *tmem_slot;
-  const tc::Waits wait(mark, status);
+  const PairWaits wait(mark, status, 2 * p.splits);
   pdl_wait();
   pdl_launch_dependents();
   const int tiles = (p.pair_tile ? __ldg(&p.pair_tile[0].x) : p.pair_tok) * p.pair_m;
@@ -188,7 +240,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       const uint32_t bytes = (uint32_t)(2 * kPairABytes + tile.n * kBlockK * 2);
       for (int kb = kb0; kb < kb1; ++kb, ++it) {
         const int st = it % kPairStages;
-        if (it >= kPairStages) wait(&empty[st], (it / kPairStages - 1) & 1);
+        if (it >= kPairStages && !wait.all(&empty[st], (it / kPairStages - 1) & 1)) break;
         if (issuer) {
           unsigned char* a = smem + st * kPairStageBytes;
           const uint32_t bar = smem_of(&full[st], lead);
@@ -198,13 +250,14 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
           pair_load(a + kPairABytes, map_x, kb * kBlockK, x0, bar, kKeepLast);
         }
         __syncwarp();
-        if (wait.stop()) break;
+        if (wait.stop()) {
+          ++it;   // (this fill too)
+          break;
+        }
       }
       if (wait.stop()) break;
     }
-    // after a wait that ran out: what has been requested lands before shared memory is given up
-    if (rank == 0 && wait.stop())
-      for (int s = 0; s < min(it, kPairStages); ++s) wait.drain(&full[s], ((it - 1 - s) / kPairStages) & 1);
+    if (issuer) *reinterpret_cast<volatile uint32_t*>(mark + 1) = (uint32_t)it;
   } else if (warp == 1) {
     // ===== the leader's MMA warp: instructions predicated to one lane in convergent code =====
     if (rank == 0) {
@@ -222,7 +275,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         if (i >= 2) wait(&acc_free[i & 1], ((i >> 1) - 1) & 1);
         tc::fence_after();
         for (int kb = kb0; kb < kb1; ++kb) {
-          wait(&full[st], st_ph);
+          wait(&full[st], st_ph, [&] { pair_await_ends(mark, lead, wait.limit); });
           tc::fence_after();
           const uint64_t da = desc0 + (uint64_t)((st * kPairStageBytes) >> 4), db = da + (uint64_t)(kPairABytes >> 4);
           const uint32_t more = kb > kb0 ? 1u : 0u;
@@ -236,7 +289,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         if (wait.stop()) break;
       }
       if (wait.stop()) {
-        pair_commit(one, last, both);
+        pair_commit(one, last, (uint16_t)(1 << lead));
         wait.drain(last, 0);
       }
     }
@@ -344,6 +397,12 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   __syncthreads();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // a CTA's shared and tensor memory serve the other's MMAs
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (wait.marked()) {   // the same answer in all CTAs of the cluster, whose waits have ended
+    if (rank == 0 && threadIdx.x == 0) pair_land(wait, full, p, mark, lead, kb1 - kb0, first, step);
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
   tc::fence_after();
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem));
 }
