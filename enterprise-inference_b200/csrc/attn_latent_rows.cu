@@ -126,8 +126,9 @@ __global__ void __launch_bounds__(kLrThreads, 1) latent_rows_kernel(const __grid
   const int t = item / p.groups, h0 = item % p.groups * kLrPairs, shares = p.cluster * p.n_splits, share0 = split * p.cluster + part;
   const int n_heads = min(p.heads - h0, kLrPairs);
   const int ctx = p.ctx_lens[t], lo = p.window > 0 ? max(ctx - p.window, 0) : 0;
-  const int tile0 = lo / kLrKeys, tiles = max((ctx + kLrKeys - 1) / kLrKeys - tile0, 0), per = (tiles + shares - 1) / shares;
-  const int tile_lo = tile0 + min(tiles, share0 * per), tile_hi = tile0 + min(tiles, (share0 + 1) * per);
+  // tiles from the 64 keys that hold the oldest visible one: a cache block is whole 64s, so none is read that lies before the window
+  const int first = lo & ~63, tiles = max((ctx - first + kLrKeys - 1) / kLrKeys, 0), per = (tiles + shares - 1) / shares;
+  const int tile_lo = min(tiles, share0 * per), tile_hi = min(tiles, (share0 + 1) * per);
 
   const int fh = threadIdx.x >> 3, fz = threadIdx.x & 7;   // the factor that the thread works out at the end
   const float sk = threadIdx.x < 8 * kLrPairs && fh < n_heads && p.sink && p.n_splits == 1 ? p.sink[h0 + fh] * 1.4426950408889634f : -INFINITY;
@@ -140,7 +141,7 @@ __global__ void __launch_bounds__(kLrThreads, 1) latent_rows_kernel(const __grid
     int st = 0, rs = 0;
     uint32_t st_ph = 1, rs_ph = 1;   // parity of the release that a slot's next load waits for (the first round finds it free)
     for (int i = tile_lo; i < tile_hi && !wait.stop(); ++i) {
-      const int tok = i * kLrKeys, halves = ctx - tok > 64 ? 2 : 1;
+      const int tok = first + i * kLrKeys, halves = ctx - tok > 64 ? 2 : 1;
       int row[2];
 #pragma unroll
       for (int x = 0; x < 2; ++x) {
@@ -181,7 +182,7 @@ __global__ void __launch_bounds__(kLrThreads, 1) latent_rows_kernel(const __grid
                    desc_q = make_desc(smem_u32(qs), 16, 1024), desc_v = make_desc(smem_u32(ring), kLrChunk, 1024), desc_p = make_desc(smem_u32(ps), 16, 1024);
     const uint32_t id_s = lr_idesc(kLrPairs, 0), id_o = lr_idesc(2 * kLrPairs, 1);
     const bool ahead = p.slots >= 2 * p.vpairs && p.rest_slots >= 2 * p.rest;
-    const int nt = __shfl_sync(0xffffffffu, tile_hi - tile_lo, 0), keys = __shfl_sync(0xffffffffu, ctx - tile_lo * kLrKeys, 0);
+    const int nt = __shfl_sync(0xffffffffu, tile_hi - tile_lo, 0), keys = __shfl_sync(0xffffffffu, ctx - first - tile_lo * kLrKeys, 0);
     int st = 0, rs = 0, pv_st = 0;
     uint32_t st_ph = 0, rs_ph = 0;
     auto chunk = [&](uint32_t d, uint64_t da, int c) {
@@ -273,7 +274,7 @@ __global__ void __launch_bounds__(kLrThreads, 1) latent_rows_kernel(const __grid
     for (int i = 0; i < 16; ++i) mus[i] = 0.f, l[i] = 0.f;
     int n = 0;
     for (int i = tile_lo; i < tile_hi; ++i, ++n) {
-      const int key = i * kLrKeys + m;
+      const int key = first + i * kLrKeys + m;
       const bool live = key >= lo && key < ctx;
       wait(s_full + (n & 1), (n >> 1) & 1);
       fence_after();
@@ -326,7 +327,7 @@ __global__ void __launch_bounds__(kLrThreads, 1) latent_rows_kernel(const __grid
         *reinterpret_cast<uint16_t*>(at) = (uint16_t)(hi >> 16);
         *reinterpret_cast<__nv_bfloat16*>(at + 2048) = __float2bfloat16_rn(w - __uint_as_float(hi));
       }
-      const int n_valid = min(ctx - i * kLrKeys, kLrKeys), n_read = (n_valid + 15) & ~15;
+      const int n_valid = min(ctx - first - i * kLrKeys, kLrKeys), n_read = (n_valid + 15) & ~15;
       if (n_valid < n_read) {
         // value rows past the context may hold anything, and 0 * NaN = NaN: zero those that the last step of 16 keys reads
         const int units = (n_read - n_valid) * 8;

@@ -161,3 +161,35 @@ def test_latent_rows_by_themselves(T, heads, rank, rd, bs, window, with_sink, wi
     # (as above)
     assert (got - want).norm() / want.norm() < 2.0 ** -8
     assert (got - want).abs().max() < 2.0 ** -8 * rows.float().abs().max() + 2.0 ** -9 * want.abs().max()
+
+
+# A window's older blocks may be anybody's: what the table names before the block of the oldest visible key is not read.  Rows by themselves, a row of many heads
+# and runs of rows; blocks of one, three and five times 64, windows whose oldest key lies in the first, a middle and the last 64 of one.
+@pytest.mark.parametrize("T,heads,rank,rd,bs,window,with_seq", [
+    (18, 16, 128, 64, 64, 65, True), (40, 16, 512, 64, 64, 300, True), (100, 16, 256, 32, 192, 130, True), (18, 16, 64, 16, 320, 64, True), (5, 48, 512, 0, 64, 1, True),
+    (200, 8, 128, 64, 64, 70, False), (200, 16, 128, 64, 64, 65, True)])
+def test_latent_windows_leave_passed_blocks_alone(T, heads, rank, rd, bs, window, with_seq):
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    g = torch.Generator().manual_seed(T + heads + bs)
+    krow, n_tok, scale = rank + rd, 1280, 0.6 / (rank + rd) ** 0.5
+    nb = (n_tok + bs - 1) // bs
+    rows = torch.randn(nb * bs, krow, generator=g).to(torch.bfloat16)
+    kc = torch.cat([rows.reshape(nb, 1, bs, krow), torch.full((1, 1, bs, krow), float("nan"), dtype=torch.bfloat16)]).to(DEV)   # block nb: another's
+    ctxs = [1 + (i * 61 + window) % n_tok for i in range(T)]
+    q = torch.randn(T, heads, krow, generator=g).to(torch.bfloat16).float()
+    want = torch.stack([_oracle(q[t].double(), rows.double(), ctxs[t], rank, scale, None, window) for t in range(T)])
+    bt = torch.arange(nb, dtype=torch.int32).repeat(T, 1)
+    for t, c in enumerate(ctxs):
+        bt[t, :max(c - window, 0) // bs] = nb
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)   # noqa: E731
+    bt, cx, sq, qd = bt.to(DEV), i32(ctxs), i32(list(range(T))), q.to(DEV)
+    ws = torch.zeros(int(lib.b200_paged_attn_anydim_workspace_bytes(T)), dtype=torch.uint8, device=DEV)
+    out = torch.full((T, heads, rank), float("nan"), dtype=torch.bfloat16, device=DEV)
+    check(lib.b200_latent_attn_window(qd.data_ptr(), kc.data_ptr(), bt.data_ptr(), nb, sq.data_ptr() if with_seq else None, cx.data_ptr(), out.data_ptr(), T, heads,
+                                      krow, rank, bs, scale, None, ws.data_ptr(), window, None))
+    torch.cuda.synchronize()
+    got = out.double().cpu()
+    assert torch.isfinite(got).all()
+    # (as above)
+    assert (got - want).norm() / want.norm() < 2.0 ** -8
+    assert (got - want).abs().max() < 2.0 ** -8 * rows.float().abs().max() + 2.0 ** -9 * want.abs().max()
