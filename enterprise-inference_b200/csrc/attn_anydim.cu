@@ -157,26 +157,29 @@ constexpr int kTcThreads = 256;
 // t - 1, or does not continue its context length by one; inside a segment a run starts every kRunRows rows.  Per chunk of
 // 1024 rows: an inclusive max-scan carries every row's segment start, a prefix sum of the run starts gives each run its place.
 // Lists of runs of at most 16, 32, .. 16 << (kRunLists - 1) rows are made in the same pass (list k at runs + 2 T k, its length at
-// n_runs[k]): the five prefix sums of a chunk travel in one 64-bit word, 12 bits each.
+// n_runs[k]): the five prefix sums of a chunk travel in one 64-bit word, 12 bits each.  Beside the lengths: the step's longest context, and the
+// tiles of 64 tokens that the runs of the first list walk (by their first rows' contexts).
 __global__ void __launch_bounds__(1024)
 attn_runs_plan_kernel(const int32_t* __restrict__ row_to_seq, const int32_t* __restrict__ ctx_lens, int T, int32_t* __restrict__ runs,
                       int32_t* __restrict__ n_runs) {
   __shared__ int wseg[32];
   __shared__ uint64_t wcnt[32];
   __shared__ int carry_seg, carry_cnt[kRunLists];
+  __shared__ int longest, tiles;           // kRunLongest, kRunTiles
   __shared__ int first[kRunLists][1024];   // steps of one chunk: the runs' first rows, for their lengths
   static_assert(kRunRows == 16 && kRunLists * 12 <= 64, "run lists");
   constexpr int kOpens = 1 << 30;   // beside a run's first row, until the lengths are there: it opens a segment
   pdl_wait();
   pdl_launch_dependents();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) carry_seg = 0;
+  if (tid == 0) carry_seg = longest = tiles = 0;
   if (tid < kRunLists) carry_cnt[tid] = 0;
   __syncthreads();
   for (int c0 = 0; c0 < T; c0 += 1024) {
     const int t = c0 + tid;
     const bool live = t < T;
-    const bool brk = live && (t == 0 || row_to_seq == nullptr || row_to_seq[t] != row_to_seq[t - 1] || ctx_lens[t] != ctx_lens[t - 1] + 1);
+    const int ctx = live ? ctx_lens[t] : 0;
+    const bool brk = live && (t == 0 || row_to_seq == nullptr || row_to_seq[t] != row_to_seq[t - 1] || ctx != ctx_lens[t - 1] + 1);
     int seg = brk ? t : -1;                       // latest segment start at or before t (within the warp, then the chunk)
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -198,6 +201,11 @@ attn_runs_plan_kernel(const int32_t* __restrict__ row_to_seq, const int32_t* __r
       if (lane >= o) cnt += v;
     }
     if (lane == 31) wcnt[warp] = cnt;
+    const int most = __reduce_max_sync(0xffffffffu, ctx), walked = __reduce_add_sync(0xffffffffu, (mine & 1) ? min((ctx + 63) >> 6, 1 << 14) : 0);
+    if (lane == 0) {
+      atomicMax(&longest, most);
+      atomicAdd(&tiles, walked);
+    }
     __syncthreads();
     for (int w = 0; w < warp; ++w) cnt += wcnt[w];
     int total[kRunLists];
@@ -237,6 +245,7 @@ attn_runs_plan_kernel(const int32_t* __restrict__ row_to_seq, const int32_t* __r
       }
   }
   if (tid < kRunLists) n_runs[tid] = carry_cnt[tid];
+  if (tid == kRunLists) n_runs[kRunLongest] = longest, n_runs[kRunTiles] = tiles;
   if (T <= 1024) return;
   __syncthreads();
   for (int i = tid; i < n0; i += 1024)

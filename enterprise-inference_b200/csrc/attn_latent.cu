@@ -19,6 +19,7 @@
 // Shapes: krow and rank multiples of 16, rank <= 512.  Everything else (and the 32-bit mode) takes attn_anydim.cu; both walk
 // the same cache and the same run list, and agree within bf16 rounding of the operands.
 #include <algorithm>
+#include <climits>
 
 #include "runs.cuh"
 
@@ -307,9 +308,10 @@ latent_attn_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __restr
 constexpr int kLaMaxSplits = 16;
 __global__ void __launch_bounds__(128)
 latent_attn_merge_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ out, int n_pairs, int heads, int rank, int n_splits,
-                         const float* __restrict__ sink, const __nv_bfloat16* __restrict__ gate, int64_t ldg) {
+                         const float* __restrict__ sink, const __nv_bfloat16* __restrict__ gate, int64_t ldg, const LatentShare share) {
   pdl_wait();
   pdl_launch_dependents();
+  if (share.plan && latent_by_rows(share)) return;   // there is nothing to merge
   const int pair = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (pair >= n_pairs) return;
   const int prow = rank + 2;
@@ -401,45 +403,79 @@ static int attn_mma_launch(const float* q, const __nv_bfloat16* kc, const __nv_b
 #undef LA2
   if (n_splits > 1)
     B200_CUDA(launch(latent_attn_merge_kernel, dim3((T * heads + 3) / 4), dim3(128), (size_t)0, s, (const float*)part, out, T * heads, heads,
-                     rank, n_splits, sink, static_cast<const __nv_bfloat16*>(ex.gate), ex.ldg));
+                     rank, n_splits, sink, static_cast<const __nv_bfloat16*>(ex.gate), ex.ldg, LatentShare()));
   return B200_OK;
 }
 
-// Rows by themselves on tcgen05 (attn_latent_rows.cu): steps whose rows' heads, 16 at a time, fit the device's SMs at once (what they measured stands
-// there; a few rows of one sequence gain as much, up to 128 of them behind 3000 tokens a little), and decode rows that say so in any number: 256 rows
-// of 16 heads at contexts 300..600 86 us on the mma.sync kernel, 51 there.  Beyond that a step of unknown rows may be a prefill chunk, whose runs
-// share their keys on attn_latent_tc.cu (2 048 rows 159 us).  Rows of fewer than 512 query entries (heads * krow) keep the plan and the attention as two
+static LatentShare latent_share(const int32_t* plan, int T, int heads, int krow, int rank, int n_splits, int window) {
+  LatentShare s = {};
+  s.plan = plan;
+  s.rows = T;
+  s.groups = latent_attn_rows_items(1, heads);
+  s.cluster = latent_attn_rows_cluster(T * s.groups);
+  s.splits = n_splits;
+  s.halves = latent_attn_tc_halves(rank);
+  s.rows_per_item = latent_attn_tc_rows(heads);
+  s.seen = window > 0 ? window : INT_MAX;
+  s.rows_ns = 4.2f + 0.035f * krow;
+  s.runs_ns = 1.15f * std::max(16.5f, 0.043f * krow);
+  s.runs_fixed = 10000.f + 54.f * krow;
+  return s;
+}
+
+// Rows by themselves (attn_latent_rows.cu) wherever they fit, but
+//  * more items of 16 heads than SMs: only rows that are known to be sequences of their own (a prefill chunk's runs share their keys), and up to 32 heads (one of
+//    128 fills the other kernel's MMAs: 512 rows at 2 000 tokens 1 543 us here, 931 there; of 32 heads 404 and 432, of 16 256 and 433);
+//  * contexts that may be so long that the caller's splits would pay for a chunk or a long row among short ones (runs.cuh): the device decides.  Up to seven items have
+//    splits of their own.  Without splits neither is much slower than the other anywhere (100 rows of one sequence of 3 100 tokens 86 and 93).
+// Rows of fewer than 512 query entries (heads * krow) keep the plan and the attention as two
 // launches, the second overlapping the first, which is what a captured call of theirs holds (tests/test_launch_gpu.py); it costs them 4 us (2 rows of
 // 4 heads over 64 + 16: 14.5, one launch of attn_latent_rows.cu 10.5) to 16 (64 rows at contexts up to 1000: 29.0 and 12.8).
-bool latent_attn_by_rows(const float* q, const __nv_bfloat16* kc, const int32_t* row_to_seq, const __nv_bfloat16* out, int T, int heads, int krow, int rank,
-                         int block_size, float scale, bool one_row_each) {
+LatentRoute latent_attn_route(const float* q, const __nv_bfloat16* kc, const int32_t* row_to_seq, const __nv_bfloat16* out, const int32_t* runs, int T, int heads,
+                              int krow, int rank, int block_size, float scale, int n_splits, const float* part, int64_t longest, bool one_row_each) {
   const auto at = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr); };
-  return T > 0 && scale > 0.f && latent_attn_mma_supported(heads, krow, rank) && latent_attn_rows_supported(heads, krow, rank, block_size) &&
-         heads * krow >= 512 && (at(q) | at(kc) | at(out)) % 16 == 0 && (latent_attn_rows_items(T, heads) <= kNumSMs || one_row_each || !row_to_seq);
+  if (T <= 0 || !(scale > 0.f) || !latent_attn_mma_supported(heads, krow, rank) || !latent_attn_rows_supported(heads, krow, rank, block_size) ||
+      heads * krow < 512 || (at(q) | at(kc) | at(out)) % 16 != 0)
+    return LatentRoute::kRuns;
+  const bool own = one_row_each || !row_to_seq, tc = latent_attn_tc_supported(heads, krow, rank, block_size) && at(out) % 32 == 0 && ((at(runs) | at(part)) & 7) == 0;
+  const int items = latent_attn_rows_items(T, heads);
+  if (items > kNumSMs && (!own || (heads > 32 && tc))) return LatentRoute::kRuns;
+  if (n_splits <= 1 || !part || !tc || (items <= 7 && longest > 32768)) return LatentRoute::kRows;
+  // the longest row alone: what its CTAs take, and what they would take over runs in splits, with the launches that tell
+  const LatentShare s = latent_share(nullptr, T, heads, krow, rank, n_splits, 0);
+  const float gain = (s.rows_ns / s.cluster - s.runs_ns / 1.15f / s.splits) * (float)longest;
+  return gain > s.runs_fixed + 12000.f ? LatentRoute::kEither : LatentRoute::kRows;
 }
 
 // runs / n_runs: the run list of the step (attn_anydim.cu builds it: runs of at most 16 consecutive rows of one sequence)
 int latent_attn_mma(const float* q, const __nv_bfloat16* kc, const int32_t* block_table, int bt_stride, const int32_t* row_to_seq,
                     const int32_t* ctx_lens, __nv_bfloat16* out, const int32_t* runs, const int32_t* n_runs, int T, int heads, int krow,
                     int rank, int block_size, float scale, const float* sink, cudaStream_t s, int n_splits, float* part, int window,
-                    bool one_row_each) {
+                    bool one_row_each, int64_t longest) {
   if (T == 0) return B200_OK;
   B200_REQUIRE(latent_attn_mma_supported(heads, krow, rank), B200_ERR_UNSUPPORTED, "latent_attn_mma: shape %d / %d / %d", heads, krow, rank);
   if (n_splits < 1 || part == nullptr) n_splits = 1;
   B200_REQUIRE(n_splits <= kLaMaxSplits, B200_ERR_INVALID, "attention: %d splits (at most %d)", n_splits, kLaMaxSplits);
   const auto at = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr); };
   B200_REQUIRE(at(kc) % 16 == 0, B200_ERR_INVALID, "attention: cache not 16-byte aligned");
-  const auto merge = [&](int splits) -> int {
+  const auto merge = [&](int splits, const LatentShare& share) -> int {
     B200_CUDA(launch(latent_attn_merge_kernel, dim3((T * heads + 3) / 4), dim3(128), (size_t)0, s, (const float*)part, out, T * heads, heads, rank, splits,
-                     sink, (const __nv_bfloat16*)nullptr, (int64_t)0));
+                     sink, (const __nv_bfloat16*)nullptr, (int64_t)0, share));
     return B200_OK;
   };
-  if (latent_attn_by_rows(q, kc, row_to_seq, out, T, heads, krow, rank, block_size, scale, one_row_each)) {
+  const LatentRoute route = latent_attn_route(q, kc, row_to_seq, out, runs, T, heads, krow, rank, block_size, scale, n_splits, part, longest, one_row_each);
+  const LatentShare share = route == LatentRoute::kEither ? latent_share(n_runs, T, heads, krow, rank, n_splits, window) : LatentShare();
+  if (route != LatentRoute::kRuns) {
+    int splits = n_splits;
     const int rc = latent_attn_rows(q, kc, block_table, bt_stride, row_to_seq, ctx_lens, out, T, heads, krow, rank, block_size, scale, sink, s, window,
-                                    at(part) % 8 == 0 ? part : nullptr, &n_splits);
-    if (rc || n_splits == 1) return rc;
+                                    at(part) % 8 == 0 ? part : nullptr, longest, share, &splits);
+    if (rc || (route == LatentRoute::kRows && splits == 1)) return rc;
     const PdlScope after_rows;
-    return merge(n_splits);
+    if (route == LatentRoute::kRows) return merge(splits, share);
+    if (const int e = latent_attn_tc(q, kc, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, krow, rank, block_size, scale, sink, s, n_splits,
+                                     part, window, share))
+      return e;
+    return merge(n_splits, share);
   }
   // tcgen05 wherever the shape fits and the rows can be read and written in its wide pieces (what it measured stands there); other shapes, blocks
   // that a key tile would straddle and odd addresses stay here, and so do scales that are not positive (masks and maxima there are taken of
@@ -449,8 +485,8 @@ int latent_attn_mma(const float* q, const __nv_bfloat16* kc, const int32_t* bloc
   if (scale > 0.f && !few_pairs && latent_attn_tc_supported(heads, krow, rank, block_size) && at(q) % 16 == 0 && at(out) % 32 == 0 &&
       ((at(runs) | at(part)) & 7) == 0) {
     const int rc = latent_attn_tc(q, kc, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, krow, rank, block_size, scale,
-                                  sink, s, n_splits, part, window);
-    return rc || n_splits == 1 ? rc : merge(n_splits);
+                                  sink, s, n_splits, part, window, share);
+    return rc || n_splits == 1 ? rc : merge(n_splits, share);
   }
   return attn_mma_launch(q, kc, nullptr, 1, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, krow, rank, block_size,
                          scale, sink, s, n_splits, part, window, AttnExtra());
@@ -487,3 +523,19 @@ int paged_attn_mma(const float* q, const __nv_bfloat16* kc, const __nv_bfloat16*
 }
 
 }  // namespace b200
+
+// debug helpers (not in the public header): which kernel a call of these forms takes, with everything aligned (0 rows by themselves, 1 the device decides, 2 over
+// runs), and what the device decides of a step whose plan has so many runs, that longest context and so many tiles (1 rows by themselves)
+extern "C" __attribute__((visibility("default"))) int b200_debug_latent_route(int32_t T, int32_t heads, int32_t krow, int32_t rank, int32_t block_size,
+                                                                              int32_t n_splits, int64_t longest, int32_t own) {
+  using namespace b200;
+  const auto p = [](uintptr_t a) { return reinterpret_cast<void*>(a); };
+  return (int)latent_attn_route(static_cast<const float*>(p(64)), static_cast<const __nv_bfloat16*>(p(64)), static_cast<const int32_t*>(p(64)),
+                                static_cast<const __nv_bfloat16*>(p(64)), static_cast<const int32_t*>(p(64)), T, heads, krow, rank, block_size, 1.f, n_splits,
+                                n_splits > 1 ? static_cast<const float*>(p(64)) : nullptr, longest, own != 0);
+}
+extern "C" __attribute__((visibility("default"))) int b200_debug_latent_by_rows(int32_t T, int32_t heads, int32_t krow, int32_t rank, int32_t n_splits, int32_t window,
+                                                                                int32_t n_runs, int32_t longest, int32_t tiles) {
+  using namespace b200;
+  return latent_by_rows(latent_share(nullptr, T, heads, krow, rank, n_splits, window), n_runs, longest, tiles) ? 1 : 0;
+}

@@ -18,6 +18,7 @@
 // rises by more than 2^8, as in attn_latent_tc.cu.  Every wait is bounded and reported (tc.cuh).
 #include <algorithm>
 
+#include "runs.cuh"
 #include "tc.cuh"
 
 namespace b200 {
@@ -43,6 +44,7 @@ struct LrParams {
   uint32_t* status;
   int bt_stride, heads, groups, krow, rank, block_size, window, vpairs, rest, slots, rest_slots, cluster, n_splits;   // groups: of up to 16 heads
   float scale;
+  LatentShare share;
 };
 
 __device__ __forceinline__ uint32_t lr_idesc(int n, int a_mn_major) {
@@ -93,6 +95,10 @@ __global__ void __launch_bounds__(kLrThreads, 1) latent_rows_kernel(const __grid
   float* lred = stat + 2 * kLrPairs;                             // [4 warps][16]
   float* fac = lred + 4 * kLrPairs;                              // [16 heads][8 CTAs] what their sums are weighted with
   const Waits wait(tmem_slot + 1, p.status);
+  if (p.share.plan) {
+    pdl_wait();
+    if (!latent_by_rows(p.share)) return;
+  }
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.slots; ++s) {
@@ -483,12 +489,13 @@ bool latent_attn_rows_supported(int heads, int krow, int rank, int block_size) {
   return heads > 0 && block_size > 0 && block_size % 64 == 0 && lr_shape(krow, rank, p);
 }
 int latent_attn_rows_items(int T, int heads) { return T * ((heads + kLrPairs - 1) / kLrPairs); }
+int latent_attn_rows_cluster(int items) { return items <= 15 ? 8 : items <= 33 ? 4 : items <= 74 ? 2 : 1; }   // clusters of whole SMs that the device holds at a time
 
 // every row by itself (row t of sequence row_to_seq[t], or t); scale > 0.  n_splits: at most so many shares of the context beyond the cluster's; how many were
-// taken (more than one: unmerged sums in part)
+// taken (more than one: unmerged sums in part).  share: whether the step is this kernel's
 int latent_attn_rows(const float* q, const __nv_bfloat16* kc, const int32_t* block_table, int bt_stride, const int32_t* row_to_seq, const int32_t* ctx_lens,
                      __nv_bfloat16* out, int T, int heads, int krow, int rank, int block_size, float scale, const float* sink, cudaStream_t s, int window, float* part,
-                     int* n_splits) {
+                     int64_t longest, const LatentShare& share, int* n_splits) {
   LrParams p = {};
   B200_REQUIRE(latent_attn_rows_supported(heads, krow, rank, block_size) && lr_shape(krow, rank, p), B200_ERR_UNSUPPORTED,
                "latent_attn_rows: shape %d / %d / %d", heads, krow, rank);
@@ -512,11 +519,11 @@ int latent_attn_rows(const float* q, const __nv_bfloat16* kc, const int32_t* blo
   p.window = window;
   p.scale = scale;
   const int items = T * p.groups;
-  p.cluster = items <= 15 ? 8 : items <= 33 ? 4 : items <= 74 ? 2 : 1;   // clusters of whole SMs that the device holds at a time
+  p.cluster = latent_attn_rows_cluster(items);
+  p.share = share;
   // One to seven rows leave SMs for more shares, whose merge is a launch of its own and pays at long contexts only (one row of 3 000 tokens 21 us without, 39 with
-  // all of them; of 16 000 58 and 43, of 60 000 about 180 and 53; 50, 77 and 158 on attn_latent_tc.cu).  How long contexts are is not known here,
-  // how long the block table lets them become is.
-  p.n_splits = part && p.cluster == 8 && (int64_t)bt_stride * block_size > 32768 ? std::max(std::min(*n_splits, 15 / items), 1) : 1;
+  // all of them; of 16 000 58 and 43, of 60 000 about 180 and 53; 50, 77 and 158 on attn_latent_tc.cu).
+  p.n_splits = part && !share.plan && p.cluster == 8 && longest > 32768 ? std::max(std::min(*n_splits, 15 / items), 1) : 1;
   p.part = part;
   *n_splits = p.n_splits;
   static bool done[64] = {};

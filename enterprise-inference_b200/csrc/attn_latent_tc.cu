@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "runs.cuh"
 #include "tc.cuh"
 
 namespace b200 {
@@ -54,6 +55,7 @@ struct LtParams {
   uint32_t* status;
   int n_rows, bt_stride, heads, krow, rank, block_size, n_splits, window, own_stages, rest_stages, halves, rows_per_item, items_per_run;
   float scale;
+  LatentShare share;
 };
 
 struct LtItem {
@@ -109,6 +111,10 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
   uint64_t* last = q_free + 1;                   // the MMAs in flight when a wait ran out
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(last + 1);   // and, behind it, the mark of a wait that ran out
   const Waits mbar_wait(tmem_slot + 1, p.status);
+  if (p.share.plan) {
+    pdl_wait();
+    if (latent_by_rows(p.share)) return;
+  }
   LtItem* table = reinterpret_cast<LtItem*>(tmem_slot + 2);   // nr 0: nothing there
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.own_stages; ++s) {
@@ -558,12 +564,14 @@ bool latent_attn_tc_supported(int heads, int krow, int rank, int block_size) {
   return block_size > 0 && block_size % kLtKeys == 0 && lt_shape(heads, krow, rank, s);
 }
 
+int latent_attn_tc_rows(int heads) { return std::min(kLtPairs / heads, kRunRows); }   // of an item
 int latent_attn_tc_halves(int rank) { return rank > 256 ? 2 : 1; }
 
 // one launch over the step's run list; part given: n_splits CTAs per item leave unnormalised sums (the caller merges)
 int latent_attn_tc(const float* q, const __nv_bfloat16* kc, const int32_t* block_table, int bt_stride, const int32_t* row_to_seq,
                    const int32_t* ctx_lens, __nv_bfloat16* out, const int32_t* runs, const int32_t* n_runs, int T, int heads, int krow,
-                   int rank, int block_size, float scale, const float* sink, cudaStream_t s, int n_splits, float* part, int window) {
+                   int rank, int block_size, float scale, const float* sink, cudaStream_t s, int n_splits, float* part, int window,
+                   const LatentShare& share) {
   LtShape sh;
   B200_REQUIRE(latent_attn_tc_supported(heads, krow, rank, block_size) && lt_shape(heads, krow, rank, sh), B200_ERR_UNSUPPORTED,
                "latent_attn_tc: shape %d / %d / %d", heads, krow, rank);
@@ -593,9 +601,10 @@ int latent_attn_tc(const float* q, const __nv_bfloat16* kc, const int32_t* block
   p.own_stages = sh.own_stages;
   p.rest_stages = sh.rest_stages;
   p.halves = sh.halves;
-  p.rows_per_item = std::min(kLtPairs / heads, 16);   // a run has at most 16 rows
+  p.rows_per_item = latent_attn_tc_rows(heads);
   p.items_per_run = (16 + p.rows_per_item - 1) / p.rows_per_item;
   p.scale = scale;
+  p.share = share;
   static bool done[64] = {};
   B200_CUDA(ensure_dynamic_smem(latent_attn_tc_kernel, kLtSmem, done));
   const int64_t most = (int64_t)T * p.items_per_run * n_splits * sh.halves;   // upper bound; the kernel reads the real count

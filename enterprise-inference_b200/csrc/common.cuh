@@ -366,29 +366,37 @@ int paged_attn_anydim(bool f32, const float* q, const void* kc, const void* vc, 
 // cache itself, a value being the leading vdim entries of the row); sink [heads]: exp(sink[h]) joins the softmax denominator
 constexpr int kRunRows = 16, kRunLists = 5;   // lists of runs of at most 16, 32, 64, 128, 256 rows: (first row, length | kRunWhole)
 constexpr int kRunLength = 0xffff, kRunWhole = 1 << 16;   // whole: the run is all of its segment of rising contexts
-constexpr int kRunTicket = 5;   // word behind the lists' lengths: runs.cuh
+constexpr int kRunTicket = 5, kRunLongest = 6, kRunTiles = 7;   // words behind the lists' lengths: runs.cuh; the longest context; tiles of 64 tokens
+                                                                // that the runs of kRunRows rows walk together
 int paged_attn_runs_plan(const int32_t* row_to_seq, const int32_t* ctx_lens, int T, void* ws, cudaStream_t s);
 // latent cache rows on the tensor cores (attn_latent.cu): bf16 cache, fp32 queries, bf16 output [T][heads][rank]
 bool latent_attn_mma_supported(int heads, int krow, int rank);
-// rows by themselves (attn_latent_rows.cu): no run list; latent_attn_mma takes it wherever latent_attn_by_rows says so
+// rows by themselves (attn_latent_rows.cu): no run list
+struct LatentShare;   // runs.cuh
 bool latent_attn_rows_supported(int heads, int krow, int rank, int block_size);
 int latent_attn_rows_items(int T, int heads);   // rows times groups of 16 heads
+int latent_attn_rows_cluster(int items);        // CTAs that share an item's context
 int latent_attn_rows(const float* q, const __nv_bfloat16* kc, const int32_t* block_table, int bt_stride, const int32_t* row_to_seq, const int32_t* ctx_lens,
                      __nv_bfloat16* out, int T, int heads, int krow, int rank, int block_size, float scale, const float* sink, cudaStream_t s, int window, float* part,
-                     int* n_splits);   // n_splits: at most, and taken
-bool latent_attn_by_rows(const float* q, const __nv_bfloat16* kc, const int32_t* row_to_seq, const __nv_bfloat16* out, int T, int heads, int krow, int rank,
-                         int block_size, float scale, bool one_row_each);
+                     int64_t longest, const LatentShare& share, int* n_splits);   // longest: no context is longer; n_splits: at most, and taken
+// Which kernel latent_attn_mma launches: rows by themselves (the run plan is not read), the one over runs, or both, one of which finds by the plan that the step
+// is the other's
+enum class LatentRoute { kRows, kEither, kRuns };
+LatentRoute latent_attn_route(const float* q, const __nv_bfloat16* kc, const int32_t* row_to_seq, const __nv_bfloat16* out, const int32_t* runs, int T, int heads,
+                              int krow, int rank, int block_size, float scale, int n_splits, const float* part, int64_t longest, bool one_row_each);
 int latent_attn_mma(const float* q, const __nv_bfloat16* kc, const int32_t* block_table, int bt_stride, const int32_t* row_to_seq,
                     const int32_t* ctx_lens, __nv_bfloat16* out, const int32_t* runs, const int32_t* n_runs, int T, int heads, int krow,
-                    int rank, int block_size, float scale, const float* sink, cudaStream_t s, int n_splits = 1, float* part = nullptr,
-                    int window = 0, bool one_row_each = false);
-// (one_row_each: the step's rows are known to be sequences of their own, as decode steps are)
+                    int rank, int block_size, float scale, const float* sink, cudaStream_t s, int n_splits, float* part,
+                    int window, bool one_row_each, int64_t longest);
+// (one_row_each: the step's rows are known to be sequences of their own, as decode steps are; longest: no row sees more tokens)
 // the same attention on tcgen05 (attn_latent_tc.cu), which latent_attn_mma takes for the shapes it fits; n_splits > 1: unmerged sums in part
 bool latent_attn_tc_supported(int heads, int krow, int rank, int block_size);
 int latent_attn_tc(const float* q, const __nv_bfloat16* kc, const int32_t* block_table, int bt_stride, const int32_t* row_to_seq,
                    const int32_t* ctx_lens, __nv_bfloat16* out, const int32_t* runs, const int32_t* n_runs, int T, int heads, int krow,
-                   int rank, int block_size, float scale, const float* sink, cudaStream_t s, int n_splits, float* part, int window);
+                   int rank, int block_size, float scale, const float* sink, cudaStream_t s, int n_splits, float* part, int window,
+                   const LatentShare& share);
 int latent_attn_tc_halves(int rank);   // items that it makes of a run of few rows
+int latent_attn_tc_rows(int heads);    // rows of an item
 // the same kernel for grouped-query attention over key and value caches [block][kv_heads][block_size][dim | vdim]
 bool paged_attn_mma_supported(int heads, int kv_heads, int dim, int vdim);
 int paged_attn_mma(const float* q, const __nv_bfloat16* kc, const __nv_bfloat16* vc, const int32_t* block_table, int bt_stride,

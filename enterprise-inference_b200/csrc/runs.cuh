@@ -31,6 +31,32 @@ __device__ __forceinline__ int run_share(const RunShare& s, int G) {
   return s.rows * G > 16 * n ? 0 : kRunsAll;
 }
 
+// Latent attention of a step that either of two kernels may take.  Rows by themselves (attn_latent_rows.cu) put `cluster` CTAs on a row's 16 heads, which
+// walk its context together; over runs (attn_latent_tc.cu) up to 128 (row, head) pairs share a walk, cut into `splits` by CTAs and merged.  Which is faster
+// hangs on how the rows fall into runs and on how uneven their contexts are: known on the device only, so both are launched where it matters
+// (latent_attn_route), and each estimates both from the run plan.  The estimates, in ns, from 1..148 rows of 4..128 heads over 512 + 64, 512, 256 + 32, 128 + 64
+// and 64 + 16 at contexts 300..64 000, of one sequence, of as many as rows, and one long among short ones:
+//   rows: 4.2 + 0.035 krow a key and CTA       runs: 10 us + 54 krow for splits and merge, 1.15 max(16.5, 0.043 krow) a key and CTA, whole rounds of items
+// e.g. 100 rows of 16 heads over 512 + 64, us, rows and runs: one sequence of 16 100 tokens 385, 183; as many of 16 000 403, 732; one of 32 000 among 600s
+// 756, 368.  The launches that a step does not need cost it 8 us.
+struct LatentShare {
+  const int32_t* plan;   // its words; null: the kernel has the step to itself
+  int rows, groups, cluster, splits, halves, rows_per_item, seen;   // groups: of 16 heads; seen: a window's tokens (or INT_MAX)
+  float rows_ns, runs_ns, runs_fixed;
+};
+__host__ __device__ __forceinline__ bool latent_by_rows(const LatentShare& s, int n_runs, int longest, int tiles) {
+  const float most = (float)(longest < s.seen ? longest : s.seen), each = (float)(s.seen >> 6) + 2.f;
+  const float walked = 64.f * fminf((float)tiles, each * (float)n_runs);                    // keys of all runs
+  const int parts = (s.rows + n_runs * s.rows_per_item - 1) / (n_runs * s.rows_per_item);   // items of a run in the mean
+  const float items = (float)n_runs * parts * s.halves * s.splits, rounds = ceilf(items / kNumSMs);
+  const float by_rows = s.rows_ns * fmaxf(most / s.cluster, walked * s.groups / kNumSMs);
+  const float by_runs = s.runs_fixed + s.runs_ns * fmaxf(most / s.splits, walked * parts * s.halves * rounds / items);
+  return by_rows <= by_runs;
+}
+__device__ __forceinline__ bool latent_by_rows(const LatentShare& s) {
+  return latent_by_rows(s, max(__ldg(s.plan), 1), __ldg(s.plan + kRunLongest), __ldg(s.plan + kRunTiles));
+}
+
 // Is a run (its second word) the mma.sync kernel's?  A segment of at most kRunRows rows is one run in every list.
 __device__ __forceinline__ bool run_is_short(int pairs, int run, int G) {
   return pairs == kRunsAll || ((run & kRunWhole) && (run & kRunLength) <= kRunRows && (run & kRunLength) * G <= pairs);

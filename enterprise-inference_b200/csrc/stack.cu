@@ -521,7 +521,7 @@ static int stack_enqueue_step_postnorm(b200_ctx* c, const StepArgs& a, cudaStrea
         const int seen = L.window > 0 ? std::min(a.max_ctx, L.window + 64) : a.max_ctx;
         STEP(latent_attn_mma(M->q, (const __nv_bfloat16*)cache, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens, (__nv_bfloat16*)M->lat,
                              static_cast<const int32_t*>(M->attn_ws) + 8, static_cast<const int32_t*>(M->attn_ws), T, L.heads, kr, kr,
-                             m.block_size, L.scale, nullptr, s, latent_attn_splits(T, L.heads, kr, seen, M->lat_ws_bytes), M->lat_ws, L.window, own_rows));
+                             m.block_size, L.scale, nullptr, s, latent_attn_splits(T, L.heads, kr, seen, M->lat_ws_bytes), M->lat_ws, L.window, own_rows, seen));
       } else {
         if (attn_plan) STEP(step_runs(runs_built));
         STEP(paged_attn_anydim(f32, M->q, cache, cache, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens, a.positions, nullptr, 1ll << 40,
@@ -677,7 +677,7 @@ static int stack_enqueue_step_parallel(b200_ctx* c, const StepArgs& a, cudaStrea
         STEP(latent_attn_mma(M->q, (const __nv_bfloat16*)W.kc, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens,
                              (__nv_bfloat16*)M->lat, static_cast<const int32_t*>(M->attn_ws) + 8, static_cast<const int32_t*>(M->attn_ws), T,
                              L.heads, krow, L.kv_rank, m.block_size, L.scale, sink, s,
-                             latent_attn_splits(T, L.heads, L.kv_rank, a.max_ctx, M->lat_ws_bytes), M->lat_ws, 0, own_rows));
+                             latent_attn_splits(T, L.heads, L.kv_rank, a.max_ctx, M->lat_ws_bytes), M->lat_ws, 0, own_rows, a.max_ctx));
       } else {
         if (attn_plan) STEP(step_runs(runs_built));
         STEP(paged_attn_anydim(f32, M->q, W.kc, W.kc, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens, a.positions, nullptr, max_pos,
@@ -2050,13 +2050,15 @@ extern "C" int b200_latent_attn(const float* q, const void* cache, const int32_t
                                 int32_t block_size, float scale, const float* sink, void* workspace, int32_t n_splits, float* part,
                                 void* stream) {
   B200_REQUIRE(q && cache && block_table && ctx_lens && out && workspace && block_size > 0, B200_ERR_INVALID, "latent_attn: bad argument");
-  const bool by_rows = latent_attn_by_rows(q, (const __nv_bfloat16*)cache, row_to_seq, (const __nv_bfloat16*)out, T, heads, k_row, rank, block_size, scale, false);
-  if (!by_rows)
+  const int32_t* n_runs = static_cast<const int32_t*>(workspace);
+  const int64_t longest = (int64_t)bt_stride * block_size;
+  const bool plan = latent_attn_route(q, (const __nv_bfloat16*)cache, row_to_seq, (const __nv_bfloat16*)out, n_runs + 8, T, heads, k_row, rank, block_size, scale,
+                                      n_splits, part, longest, false) != LatentRoute::kRows;
+  if (plan)
     if (const int rc = paged_attn_runs_plan(row_to_seq, ctx_lens, T, workspace, (cudaStream_t)stream)) return rc;
-  const PdlScope after_plan(!by_rows);
-  return latent_attn_mma(q, (const __nv_bfloat16*)cache, block_table, bt_stride, row_to_seq, ctx_lens, (__nv_bfloat16*)out,
-                         static_cast<const int32_t*>(workspace) + 8, static_cast<const int32_t*>(workspace), T, heads, k_row, rank,
-                         block_size, scale, sink, (cudaStream_t)stream, n_splits, part);
+  const PdlScope after_plan(plan);
+  return latent_attn_mma(q, (const __nv_bfloat16*)cache, block_table, bt_stride, row_to_seq, ctx_lens, (__nv_bfloat16*)out, n_runs + 8, n_runs, T, heads, k_row,
+                         rank, block_size, scale, sink, (cudaStream_t)stream, n_splits, part, 0, false, longest);
 }
 
 // ---- per-kernel entry points of the post-norm form ---------------------------------------------------------------------------
@@ -2099,13 +2101,15 @@ extern "C" int b200_latent_attn_window(const float* q, const void* cache, const 
                                        void* stream) {
   B200_REQUIRE(q && cache && block_table && ctx_lens && out && workspace && block_size > 0 && window >= 0, B200_ERR_INVALID,
                "latent_attn_window: bad argument");
-  const bool by_rows = latent_attn_by_rows(q, (const __nv_bfloat16*)cache, row_to_seq, (const __nv_bfloat16*)out, T, heads, k_row, rank, block_size, scale, false);
-  if (!by_rows)
+  const int32_t* n_runs = static_cast<const int32_t*>(workspace);
+  const int64_t longest = (int64_t)bt_stride * block_size;
+  const bool plan = latent_attn_route(q, (const __nv_bfloat16*)cache, row_to_seq, (const __nv_bfloat16*)out, n_runs + 8, T, heads, k_row, rank, block_size, scale,
+                                      1, nullptr, longest, false) != LatentRoute::kRows;
+  if (plan)
     if (const int rc = paged_attn_runs_plan(row_to_seq, ctx_lens, T, workspace, (cudaStream_t)stream)) return rc;
-  const PdlScope after_plan(!by_rows);
-  return latent_attn_mma(q, (const __nv_bfloat16*)cache, block_table, bt_stride, row_to_seq, ctx_lens, (__nv_bfloat16*)out,
-                         static_cast<const int32_t*>(workspace) + 8, static_cast<const int32_t*>(workspace), T, heads, k_row, rank,
-                         block_size, scale, sink, (cudaStream_t)stream, 1, nullptr, window);
+  const PdlScope after_plan(plan);
+  return latent_attn_mma(q, (const __nv_bfloat16*)cache, block_table, bt_stride, row_to_seq, ctx_lens, (__nv_bfloat16*)out, n_runs + 8, n_runs, T, heads, k_row,
+                         rank, block_size, scale, sink, (cudaStream_t)stream, 1, nullptr, window, false, longest);
 }
 
 extern "C" int b200_latent_norms(int32_t f32, const void* fused, int64_t ld, int32_t q_rank, int32_t kv_rank, const float* qw, const float* kw,
