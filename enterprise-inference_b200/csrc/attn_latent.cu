@@ -428,14 +428,14 @@ static LatentShare latent_share(const int32_t* plan, int T, int heads, int krow,
 //    128 fills the other kernel's MMAs: 512 rows at 2 000 tokens 1 543 us here, 931 there; of 32 heads 404 and 432, of 16 256 and 433);
 //  * contexts that may be so long that the caller's splits would pay for a chunk or a long row among short ones (runs.cuh): the device decides.  Up to seven items have
 //    splits of their own.  Without splits neither is much slower than the other anywhere (100 rows of one sequence of 3 100 tokens 86 and 93).
-// Rows of fewer than 512 query entries (heads * krow) keep the plan and the attention as two
-// launches, the second overlapping the first, which is what a captured call of theirs holds (tests/test_launch_gpu.py); it costs them 4 us (2 rows of
-// 4 heads over 64 + 16: 14.5, one launch of attn_latent_rows.cu 10.5) to 16 (64 rows at contexts up to 1000: 29.0 and 12.8).
+// One or two rows with less than 4 KB of queries (T * heads * krow) keep the plan and the attention as two launches, the second overlapping the first, which is
+// what a captured call of two rows of 4 heads over 64 + 16 holds (tests/test_launch_gpu.py): 13.5 us, by themselves 10.  (Rows of more queries: 64 of these heads
+// at 900 tokens 28 us over runs, 13 by themselves.)
 LatentRoute latent_attn_route(const float* q, const __nv_bfloat16* kc, const int32_t* row_to_seq, const __nv_bfloat16* out, const int32_t* runs, int T, int heads,
                               int krow, int rank, int block_size, float scale, int n_splits, const float* part, int64_t longest, bool one_row_each) {
   const auto at = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr); };
   if (T <= 0 || !(scale > 0.f) || !latent_attn_mma_supported(heads, krow, rank) || !latent_attn_rows_supported(heads, krow, rank, block_size) ||
-      heads * krow < 512 || (at(q) | at(kc) | at(out)) % 16 != 0)
+      (T <= 2 && (int64_t)T * heads * krow < 1024) || (at(q) | at(kc) | at(out)) % 16 != 0)
     return LatentRoute::kRuns;
   const bool own = one_row_each || !row_to_seq, tc = latent_attn_tc_supported(heads, krow, rank, block_size) && at(out) % 32 == 0 && ((at(runs) | at(part)) & 7) == 0;
   const int items = latent_attn_rows_items(T, heads);

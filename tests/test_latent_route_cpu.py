@@ -56,6 +56,9 @@ def test_routes_of_forms(lib):
     assert r(T=100, splits=3, longest=3200) == ROWS and r(T=100, splits=3, longest=16384) == EITHER and r(T=100, splits=1, longest=1 << 20) == ROWS
     assert r(T=7, splits=16, longest=1 << 20) == ROWS                          # with splits of its own
     assert r(T=8, splits=16, longest=30000) == ROWS and r(T=8, splits=16, longest=1 << 20) == EITHER
+    # rows of few heads and narrow ones as any others; a call with hardly any queries keeps its two launches
+    assert r(T=64, heads=4, krow=80, rank=64) == ROWS and r(T=148, heads=1, krow=32, rank=16) == ROWS and r(T=1, heads=2) == ROWS
+    assert r(T=2, heads=4, krow=80, rank=64) == RUNS and r(T=1, heads=1) == RUNS and r(T=3, heads=1, krow=80, rank=64) == ROWS
     # a window bounds what a row sees, whatever its context
     assert lib.b200_debug_latent_by_rows(100, 16, 576, 512, 3, 1024, 100, 32000, 100 * 500) == 1
 
