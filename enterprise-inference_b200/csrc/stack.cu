@@ -517,11 +517,13 @@ static int stack_enqueue_step_postnorm(b200_ctx* c, const StepArgs& a, cudaStrea
       // q' = W_uk^T q: the scores are taken against the cached latent rows
       STEP(head_linear(f32, true, M->qh, hd, L.dim, W.uk_t, M->q, (int64_t)L.heads * kr, kr, nullptr, 0, 0, T, L.heads, kr, L.dim, s));
       if (!f32 && latent_attn_mma_supported(L.heads, kr, kr)) {
-        STEP(step_runs(runs_built));
-        const int seen = L.window > 0 ? std::min(a.max_ctx, L.window + 64) : a.max_ctx;
-        STEP(latent_attn_mma(M->q, (const __nv_bfloat16*)cache, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens, (__nv_bfloat16*)M->lat,
-                             static_cast<const int32_t*>(M->attn_ws) + 8, static_cast<const int32_t*>(M->attn_ws), T, L.heads, kr, kr,
-                             m.block_size, L.scale, nullptr, s, latent_attn_splits(T, L.heads, kr, seen, M->lat_ws_bytes), M->lat_ws, L.window, own_rows, seen));
+        const int seen = L.window > 0 ? std::min(a.max_ctx, L.window + 64) : a.max_ctx, splits = latent_attn_splits(T, L.heads, kr, seen, M->lat_ws_bytes);
+        const int32_t* n_runs = static_cast<const int32_t*>(M->attn_ws);
+        if (latent_attn_route(M->q, (const __nv_bfloat16*)cache, a.row_to_seq, (const __nv_bfloat16*)M->lat, n_runs + 8, T, L.heads, kr, kr, m.block_size,
+                              L.scale, splits, M->lat_ws, seen, own_rows) != LatentRoute::kRows)
+          STEP(step_runs(runs_built));
+        STEP(latent_attn_mma(M->q, (const __nv_bfloat16*)cache, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens, (__nv_bfloat16*)M->lat, n_runs + 8, n_runs,
+                             T, L.heads, kr, kr, m.block_size, L.scale, nullptr, s, splits, M->lat_ws, L.window, own_rows, seen));
       } else {
         if (attn_plan) STEP(step_runs(runs_built));
         STEP(paged_attn_anydim(f32, M->q, cache, cache, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens, a.positions, nullptr, 1ll << 40,
@@ -673,11 +675,13 @@ static int stack_enqueue_step_parallel(b200_ctx* c, const StepArgs& a, cudaStrea
                        L.dim, s));
       const float* sink = (L.mixer_flags & B200_MIXF_SINK) ? W.sink : nullptr;
       if (!f32 && latent_attn_mma_supported(L.heads, krow, L.kv_rank)) {
-        STEP(step_runs(runs_built));
-        STEP(latent_attn_mma(M->q, (const __nv_bfloat16*)W.kc, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens,
-                             (__nv_bfloat16*)M->lat, static_cast<const int32_t*>(M->attn_ws) + 8, static_cast<const int32_t*>(M->attn_ws), T,
-                             L.heads, krow, L.kv_rank, m.block_size, L.scale, sink, s,
-                             latent_attn_splits(T, L.heads, L.kv_rank, a.max_ctx, M->lat_ws_bytes), M->lat_ws, 0, own_rows, a.max_ctx));
+        const int splits = latent_attn_splits(T, L.heads, L.kv_rank, a.max_ctx, M->lat_ws_bytes);
+        const int32_t* n_runs = static_cast<const int32_t*>(M->attn_ws);
+        if (latent_attn_route(M->q, (const __nv_bfloat16*)W.kc, a.row_to_seq, (const __nv_bfloat16*)M->lat, n_runs + 8, T, L.heads, krow, L.kv_rank, m.block_size,
+                              L.scale, splits, M->lat_ws, a.max_ctx, own_rows) != LatentRoute::kRows)
+          STEP(step_runs(runs_built));
+        STEP(latent_attn_mma(M->q, (const __nv_bfloat16*)W.kc, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens, (__nv_bfloat16*)M->lat, n_runs + 8, n_runs,
+                             T, L.heads, krow, L.kv_rank, m.block_size, L.scale, sink, s, splits, M->lat_ws, 0, own_rows, a.max_ctx));
       } else {
         if (attn_plan) STEP(step_runs(runs_built));
         STEP(paged_attn_anydim(f32, M->q, W.kc, W.kc, a.block_table, a.bt_stride, a.row_to_seq, a.ctx_lens, a.positions, nullptr, max_pos,

@@ -57,3 +57,20 @@ def test_steps_that_either_kernel_may_take(heads, rank, rd, seqs, splits, with_s
         # weights of two bf16 terms, results rounded to bf16 once: 2^-9 of a result and of the largest value
         assert (got - want).norm() / want.norm() < 2.0 ** -8
         assert (got - want).abs().max() < 2.0 ** -8 * kc.float().abs().max() + 2.0 ** -9 * want.abs().max()
+
+
+def test_steps_whose_rows_go_by_themselves_build_no_run_plan():
+    """The same step with cache blocks that the kernel of rows by themselves reads, and with blocks that it does not: one launch less, the same logits."""
+    import dupolorn_util as D
+    import stack_util as U
+    cfg = D.make_cfg(width=128, layers=[D.latent(heads=4, dim=16, rot_dim=16, rot_dims=16, vdim=8, kv_rank=32), D.latent(second=True, heads=8, dim=16, rot_dim=16, vdim=8, kv_rank=48)])
+    w, ids = D.make_weights(cfg, 3), torch.randint(0, 150, (45,), generator=torch.Generator().manual_seed(5)).tolist()
+    launches, logits = [], []
+    for bs in (64, 96):
+        r = D.make_runner(cfg, w, "bfloat16", block_size=bs, n_blocks=12)
+        logits.append(U.replay(U.make_engine(r), [[("p", 45)]], {"p": ids})["p"])
+        launches.append(r.last_step_launches())
+        r.close()
+    assert launches[0] == launches[1] - 1
+    e = U.rel_rms(logits[0], logits[1])
+    assert (e < 0.15).mean() > 0.9, float(e.max())   # (two kernels in bf16, as between schedules of the model's own tests)
