@@ -39,8 +39,11 @@ constexpr int kLtSmem = 232448, kLtTail = 2048;
 constexpr int kLtTable = 32;                   // items of a CTA whose description is worked out ahead
 constexpr uint32_t kTmS = 256, kTmQ = 384;     // TMEM columns: O at 0, scores (then weights) of even / odd tiles, Q part
 
-// value columns of the first half: of more than 256, half of the 64-wide chunks
-__host__ __device__ __forceinline__ int lt_width0(int rank) { return rank > 256 ? (rank + 127) / 128 * 64 : rank; }
+// 64-wide chunks of the values, and those that are a half's own: of more than 256 columns half of the chunks, the last ones in the second half.  Of an odd count
+// the middle chunk is in both, and the second half writes it: either half then runs the same code (halves of 4 and 3 chunks, each with straight code of its own: 448 + 64
+// 241 us for 2 048 rows of 16 heads behind 300 tokens, though either half by itself took 166 and 181; 172 so)
+__host__ __device__ __forceinline__ int lt_value_chunks(int rank) { return (rank + 63) >> 6; }
+__host__ __device__ __forceinline__ int lt_own(int rank) { return rank > 256 ? (lt_value_chunks(rank) + 1) >> 1 : lt_value_chunks(rank); }
 
 struct LtParams {
   const float* q;
@@ -92,14 +95,11 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int chunks = (p.krow + 63) >> 6, ksteps = p.krow >> 4;
-  // value columns of a half and the chunks that hold them (the largest half decides the layout of shared memory)
-  const int width0 = lt_width0(p.rank), own0 = (width0 + 63) >> 6;
-  const int width1 = p.halves > 1 ? p.rank - width0 : width0, own1 = (width1 + 63) >> 6;
-  const int max_rest = chunks - min(own0, own1), max_own = max(own0, own1);
-  unsigned char* qs = smem;                                  // [max_rest][128][64] queries of the columns outside the half
-  unsigned char* own_ring = qs + max_rest * kLtQChunk;       // [own_stages][max_own][64][64] value columns of a tile
-  unsigned char* rest_ring = own_ring + p.own_stages * max_own * kLtChunk;   // [rest_stages][max_rest][64][64] a tile's other chunks
-  uint64_t* own_full = reinterpret_cast<uint64_t*>(rest_ring + p.rest_stages * max_rest * kLtChunk);
+  const int own = lt_own(p.rank), rest = chunks - own, second = lt_value_chunks(p.rank) - own;   // second: the second half's first chunk
+  unsigned char* qs = smem;                                  // [rest][128][64] queries of the columns outside the half
+  unsigned char* own_ring = qs + rest * kLtQChunk;       // [own_stages][own][64][64] value columns of a tile
+  unsigned char* rest_ring = own_ring + p.own_stages * own * kLtChunk;   // [rest_stages][rest][64][64] a tile's other chunks
+  uint64_t* own_full = reinterpret_cast<uint64_t*>(rest_ring + p.rest_stages * rest * kLtChunk);
   uint64_t* own_free = own_full + kLtMaxStages;
   uint64_t* rest_full = own_free + kLtMaxStages;
   uint64_t* rest_free = rest_full + kLtMaxRestStages;
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
     for (int it = blockIdx.x; it < n_items && !stop; it += gridDim.x) {
       LtItem w;
       if (!next_item(it, w)) continue;
-      const int own = w.half ? own1 : own0, first = w.half * own0, rest = chunks - own;
+      const int first = w.half * second;
       const int32_t* bt = p.block_table + (int64_t)w.seq * p.bt_stride;
       for (int i = w.tile_lo; i < w.tile_hi && !(stop = mbar_wait.stop()); ++i) {
         const int tok = i * kLtKeys;
@@ -181,14 +181,14 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
           mbar_wait(rest_free + sl, sl_ph);
           if (issuer) {
             mbar_expect_tx(rest_full + sl, rest * kLtChunk);
-            for (int c = 0; c < rest; ++c) tma_load_2d(rest_ring + (sl * max_rest + c) * kLtChunk, &map, (c < first ? c : c + own) * 64, row, rest_full + sl);
+            for (int c = 0; c < rest; ++c) tma_load_2d(rest_ring + (sl * rest + c) * kLtChunk, &map, (c < first ? c : c + own) * 64, row, rest_full + sl);
           }
           if (++sl == p.rest_stages) sl = 0, sl_ph ^= 1;
         }
         mbar_wait(own_free + st, st_ph);
         if (issuer) {
           mbar_expect_tx(own_full + st, own * kLtChunk);
-          for (int c = 0; c < own; ++c) tma_load_2d(own_ring + (st * max_own + c) * kLtChunk, &map, (first + c) * 64, row, own_full + st);
+          for (int c = 0; c < own; ++c) tma_load_2d(own_ring + (st * own + c) * kLtChunk, &map, (first + c) * 64, row, own_full + st);
         }
         __syncwarp();
         if (++st == p.own_stages) st = 0, st_ph ^= 1;
@@ -207,119 +207,92 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
     const int items = __shfl_sync(0xffffffffu, n_items, 0);
     int st = 0, sl = 0, pv_st = 0;   // own stage and rest slot of the next scores, own stage of the next second product
     uint32_t st_ph = 0, sl_ph = 0;
-    int n = 0, active = 0;
+    int n = 0, active = 0;   // n: tiles walked by the items before
+    // An item of nt key tiles whose half has O chunks of its own and R others.  Issuing is what bounds the walk (with MMAs a quarter as wide it took as long) and
+    // branches between the MMAs cost it: straight code for every pair of counts, but for the row's last chunk where it is not whole (`own_tail`, `rest_tail`: its
+    // 16-wide steps, 4 otherwise).  2 048 rows of 16 heads behind 300 tokens, us, with a loop over chunks and a wait for each / so: 512 + 64 219 / 189, 256 + 32
+    // 91 / 83, 448 + 64 201 / 172, 320 + 32 168 / 134, 192 + 64 83 / 74, 64 + 64 67 / 65.
+    auto walk = [&](auto own_c, auto rest_c, int nt, uint32_t id_o, int own_tail, int rest_tail) {
+      constexpr int O = decltype(own_c)::value, R = decltype(rest_c)::value;
+      const uint32_t id_s = idesc_bf16(kLtKeys, 0);
+      auto last_chunk = [&](int tail, auto&& step, auto base_c) {
+        constexpr int base = decltype(base_c)::value;
+        if (tail == 4) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) step(base + j);
+        } else {
+          step(base);
+          if (tail > 1) step(base + 1);
+          if (tail > 2) step(base + 2);
+        }
+      };
+      auto scores = [&](int m) {
+        const uint32_t d = tm + kTmS + (m & 1) * kLtKeys;
+        if constexpr (R > 0) {
+          mbar_wait(rest_full + sl, sl_ph);
+          fence_after();
+          const uint64_t dr = desc_rest + (uint64_t)((sl * rest * kLtChunk) >> 4);
+          auto step = [&](int j) {
+            mma_ss(one, d, desc_q + (uint64_t)(((j >> 2) * kLtQChunk >> 4) + (j & 3) * 2), dr + (uint64_t)(((j >> 2) * kLtChunk >> 4) + (j & 3) * 2), id_s, j ? 1u : 0u);
+          };
+#pragma unroll
+          for (int j = 0; j < 4 * (R - 1); ++j) step(j);
+          last_chunk(rest_tail, step, std::integral_constant<int, 4 * (R - 1)>());
+          commit(one, rest_free + sl);
+          if (++sl == p.rest_stages) sl = 0, sl_ph ^= 1;
+        }
+        mbar_wait(own_full + st, st_ph);
+        fence_after();
+        const uint64_t dk = desc_own + (uint64_t)((st * own * kLtChunk) >> 4);
+        auto step = [&](int j) { mma_ts(one, d, tm + kTmQ + j * 8, dk + (uint64_t)(((j >> 2) * kLtChunk >> 4) + (j & 3) * 2), id_s, R > 0 || j ? 1u : 0u); };
+#pragma unroll
+        for (int j = 0; j < 4 * (O - 1); ++j) step(j);
+        last_chunk(own_tail, step, std::integral_constant<int, 4 * (O - 1)>());
+        commit(one, s_full + (m & 1));
+        if (++st == p.own_stages) st = 0, st_ph ^= 1;
+      };
+      scores(n);
+      if (nt == 1) commit(one, q_free);
+      for (int i = 0; i < nt; ++i) {
+        const int m = n + i;
+        if (i + 1 < nt) {
+          scores(m + 1);
+          if (i + 2 == nt) commit(one, q_free);   // the item's last scores are on their way
+        }
+        mbar_wait(p_ready + (m & 1), (m >> 1) & 1);
+        fence_after();
+        const uint64_t dv = desc_v + (uint64_t)((pv_st * own * kLtChunk) >> 4);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {   // 16 keys per step: 8 columns of weights, 16 further those of the second term
+          const uint32_t pa = tm + kTmS + (m & 1) * kLtKeys + (j >> 1) * 32 + (j & 1) * 8;
+          mma_ts(one, tm, pa, dv + (uint64_t)((j * 2048) >> 4), id_o, (i | j) ? 1u : 0u);
+          mma_ts(one, tm, pa + 16, dv + (uint64_t)((j * 2048) >> 4), id_o, 1u);
+        }
+        commit(one, own_free + pv_st);
+        commit(one, o_full + (m & 1));
+        if (++pv_st == p.own_stages) pv_st = 0;
+      }
+    };
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
       LtItem w;
       const bool have = next_item(it, w);
       const int nt = __shfl_sync(0xffffffffu, have ? w.tile_hi - w.tile_lo : 0, 0);
       if (nt <= 0) continue;
       const int half = __shfl_sync(0xffffffffu, w.half, 0);
-      const int own = half ? own1 : own0, first = half * own0, rest = chunks - own;
-      const uint32_t id_s = idesc_bf16(kLtKeys, 0), id_o = idesc_bf16(half ? width1 : width0, 1);
-      // Issuing is what bounds the walk (with MMAs a quarter as wide it took as long), and branches between the MMAs cost it: straight code for
-      // the usual shapes, and straight blocks of chunks and of what is left of the last one for the others (2 048 rows of 16 heads, 512 + 64:
-      // 184 us with a branch and a wait per chunk, 171 with the straight blocks, 157 with straight code)
-      const int own_steps = min(own * 4, ksteps - first * 4), rest_steps = ksteps - own_steps;
-      auto issue_rest = [&](auto steps_c, int c, uint32_t d, uint64_t dr) {   // from chunk c of the others on
-        const uint64_t da = desc_q + (uint64_t)((c * kLtQChunk) >> 4), db = dr + (uint64_t)((c * kLtChunk) >> 4);
-#pragma unroll
-        for (int j = 0; j < decltype(steps_c)::value; ++j)
-          mma_ss(one, d, da + (uint64_t)(((j >> 2) * kLtQChunk >> 4) + (j & 3) * 2), db + (uint64_t)(((j >> 2) * kLtChunk >> 4) + (j & 3) * 2), id_s, c || j ? 1u : 0u);
-      };
-      auto issue_own = [&](auto steps_c, int c, uint32_t d, uint64_t dk) {
-#pragma unroll
-        for (int j = 0; j < decltype(steps_c)::value; ++j)
-          mma_ts(one, d, tm + kTmQ + c * 32 + j * 8, dk + (uint64_t)(((c + (j >> 2)) * kLtChunk >> 4) + (j & 3) * 2), id_s, rest_steps || c || j ? 1u : 0u);
-      };
-      auto issue_whole = [&](auto own_c, auto rest_c, int n) {
-        const uint32_t d = tm + kTmS + (n & 1) * kLtKeys;
-        if constexpr (decltype(rest_c)::value > 0) {
-          mbar_wait(rest_full + sl, sl_ph);
-          fence_after();
-          issue_rest(rest_c, 0, d, desc_rest + (uint64_t)((sl * max_rest * kLtChunk) >> 4));
-          commit(one, rest_free + sl);
-          if (++sl == p.rest_stages) sl = 0, sl_ph ^= 1;
-        }
-        mbar_wait(own_full + st, st_ph);
-        fence_after();
-        issue_own(own_c, 0, d, desc_own + (uint64_t)((st * max_own * kLtChunk) >> 4));
-        commit(one, s_full + (n & 1));
-        if (++st == p.own_stages) st = 0, st_ph ^= 1;
-      };
-      auto issue_any = [&](int n) {
-        const uint32_t d = tm + kTmS + (n & 1) * kLtKeys;
-        if (rest > 0) {
-          const uint64_t dr = desc_rest + (uint64_t)((sl * max_rest * kLtChunk) >> 4);
-          const int whole = rest_steps >> 2;
-          mbar_wait(rest_full + sl, sl_ph);
-          fence_after();
-          if (whole == 5) issue_rest(std::integral_constant<int, 20>(), 0, d, dr);
-          else if (whole == 4) issue_rest(std::integral_constant<int, 16>(), 0, d, dr);
-          else if (whole == 3) issue_rest(std::integral_constant<int, 12>(), 0, d, dr);
-          else if (whole == 2) issue_rest(std::integral_constant<int, 8>(), 0, d, dr);
-          else if (whole == 1) issue_rest(std::integral_constant<int, 4>(), 0, d, dr);
-          switch (rest_steps & 3) {
-            case 1: issue_rest(std::integral_constant<int, 1>(), whole, d, dr); break;
-            case 2: issue_rest(std::integral_constant<int, 2>(), whole, d, dr); break;
-            case 3: issue_rest(std::integral_constant<int, 3>(), whole, d, dr); break;
-          }
-          commit(one, rest_free + sl);
-          if (++sl == p.rest_stages) sl = 0, sl_ph ^= 1;
-        }
-        const uint64_t dk = desc_own + (uint64_t)((st * max_own * kLtChunk) >> 4);
-        const int whole = own_steps >> 2;
-        mbar_wait(own_full + st, st_ph);
-        fence_after();
-        if (whole == 4) issue_own(std::integral_constant<int, 16>(), 0, d, dk);
-        else if (whole == 3) issue_own(std::integral_constant<int, 12>(), 0, d, dk);
-        else if (whole == 2) issue_own(std::integral_constant<int, 8>(), 0, d, dk);
-        else if (whole == 1) issue_own(std::integral_constant<int, 4>(), 0, d, dk);
-        switch (own_steps & 3) {
-          case 1: issue_own(std::integral_constant<int, 1>(), whole, d, dk); break;
-          case 2: issue_own(std::integral_constant<int, 2>(), whole, d, dk); break;
-          case 3: issue_own(std::integral_constant<int, 3>(), whole, d, dk); break;
-        }
-        commit(one, s_full + (n & 1));
-        if (++st == p.own_stages) st = 0, st_ph ^= 1;
-      };
-      auto issue_s = [&](int n) {
-        using std::integral_constant;
-        switch (own_steps * 32 + rest_steps) {
-          case 16 * 32 + 20: issue_whole(integral_constant<int, 16>(), integral_constant<int, 20>(), n); break;   // 512 + 64
-          case 16 * 32 + 18: issue_whole(integral_constant<int, 16>(), integral_constant<int, 18>(), n); break;   // 512 + 32
-          case 16 * 32 + 16: issue_whole(integral_constant<int, 16>(), integral_constant<int, 16>(), n); break;   // 512
-          case 12 * 32 + 16: issue_whole(integral_constant<int, 12>(), integral_constant<int, 16>(), n); break;   // 384 + 64
-          case 12 * 32 + 10: issue_whole(integral_constant<int, 12>(), integral_constant<int, 10>(), n); break;   // 320 + 32, first half
-          case 8 * 32 + 14: issue_whole(integral_constant<int, 8>(), integral_constant<int, 14>(), n); break;     // and second
-          case 16 * 32 + 4: issue_whole(integral_constant<int, 16>(), integral_constant<int, 4>(), n); break;     // 256 + 64
-          case 16 * 32 + 2: issue_whole(integral_constant<int, 16>(), integral_constant<int, 2>(), n); break;     // 256 + 32
-          case 16 * 32: issue_whole(integral_constant<int, 16>(), integral_constant<int, 0>(), n); break;         // 256
-          case 8 * 32 + 4: issue_whole(integral_constant<int, 8>(), integral_constant<int, 4>(), n); break;       // 128 + 64
-          default: issue_any(n);
-        }
-      };
+      const uint32_t id_o = idesc_bf16(min(own * 64, p.rank - half * second * 64), 1);
+      const int tail = ksteps & 3 ? ksteps & 3 : 4;
+      const bool own_last = half * second + own == chunks;   // the row's last chunk is one of the half's own
       mbar_wait(q_ready, active & 1);
       fence_after();
-      issue_s(n);
-      if (nt == 1) commit(one, q_free);
-      for (int i = 0; i < nt; ++i, ++n) {
-        if (i + 1 < nt) {
-          issue_s(n + 1);
-          if (i + 2 == nt) commit(one, q_free);   // the item's last scores are on their way
-        }
-        mbar_wait(p_ready + (n & 1), (n >> 1) & 1);
-        fence_after();
-        const uint64_t dv = desc_v + (uint64_t)((pv_st * max_own * kLtChunk) >> 4);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {   // 16 keys per step: 8 columns of weights, 16 further those of the second term
-          const uint32_t pa = tm + kTmS + (n & 1) * kLtKeys + (j >> 1) * 32 + (j & 1) * 8;
-          mma_ts(one, tm, pa, dv + (uint64_t)((j * 2048) >> 4), id_o, (i | j) ? 1u : 0u);
-          mma_ts(one, tm, pa + 16, dv + (uint64_t)((j * 2048) >> 4), id_o, 1u);
-        }
-        commit(one, own_free + pv_st);
-        commit(one, o_full + (n & 1));
-        if (++pv_st == p.own_stages) pv_st = 0;
-      }
+      using std::integral_constant;
+#define LT_WALK(O, R) \
+  case O * 8 + R: walk(integral_constant<int, O>(), integral_constant<int, R>(), nt, id_o, own_last ? tail : 4, own_last ? 4 : tail); break;
+#define LT_WALKS(O) LT_WALK(O, 0) LT_WALK(O, 1) LT_WALK(O, 2) LT_WALK(O, 3) LT_WALK(O, 4) LT_WALK(O, 5)
+      static_assert(kLtMaxRest == 5, "counts of the other chunks");
+      switch (own * 8 + rest) { LT_WALKS(1) LT_WALKS(2) LT_WALKS(3) LT_WALKS(4) }
+#undef LT_WALKS
+#undef LT_WALK
+      n += nt;
       ++active;
     }
     if (mbar_wait.stop()) {
@@ -335,7 +308,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
     for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
       LtItem w;
       if (!next_item(it, w) || w.tile_hi <= w.tile_lo) continue;
-      const int own = w.half ? own1 : own0, first = w.half * own0, rest = chunks - own;
+      const int first = w.half * second;
       const int live = w.nr * p.heads;
       const float* qbase = p.q + (int64_t)w.t0 * p.heads * p.krow;   // pair m = (row m / heads, head m % heads): row m of this
       // four lanes take 64 neighbouring bytes of a row, eight rows per load: the fragment layout of the 16-lane store
@@ -407,7 +380,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
       if (!next_item(it, w)) continue;
       const bool alive = r < w.nr;
       const int ctx = alive ? w.ctx0 + r : 0, lo = p.window > 0 ? max(ctx - p.window, 0) : 0;
-      const int width = w.half ? width1 : width0, own = w.half ? own1 : own0;
+      const int col0 = w.half * second * 64, width = min(own * 64, p.rank - col0), written = p.halves > 1 && w.half == 0 ? second * 64 : width;   // the middle chunk: by the second half
       float mu = -INFINITY, l = 0.f;
       for (int i = w.tile_lo; i < w.tile_hi; ++i, ++n) {
         const int base = i * kLtKeys;
@@ -468,7 +441,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
           // value rows past the context may hold anything, and 0 * NaN = NaN: zero them under their zero weights
           const int st = n % p.own_stages;
           mbar_wait(own_full + st, (n / p.own_stages) & 1);
-          unsigned char* vb = own_ring + st * max_own * kLtChunk;
+          unsigned char* vb = own_ring + st * own * kLtChunk;
           for (int c = 0; c < own; ++c)
             for (int e = n_valid * 8 + m; e < kLtKeys * 8; e += 128) *reinterpret_cast<uint4*>(vb + c * kLtChunk + e * 16) = make_uint4(0u, 0u, 0u, 0u);
           fence_async_smem();
@@ -491,14 +464,14 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
           dst[p.rank] = mu * 0.6931471805599453f;
           dst[p.rank + 1] = l;
         }
-        for (int c = 0; c < width; c += 16) {
+        for (int c = 0; c < written; c += 16) {
           uint32_t o[16];
           if (any) {
             ld16(tmem + lane_off + c, o);
             ld_wait<16>(o);
           }
           if (alive) {
-            float2* d2 = reinterpret_cast<float2*>(dst + w.half * width0 + c);   // rank + 2 is even: 8-byte aligned rows
+            float2* d2 = reinterpret_cast<float2*>(dst + col0 + c);   // rank + 2 is even: 8-byte aligned rows
 #pragma unroll
             for (int j = 0; j < 8; ++j) d2[j] = any ? make_float2(__uint_as_float(o[2 * j]), __uint_as_float(o[2 * j + 1])) : make_float2(0.f, 0.f);
           }
@@ -511,8 +484,8 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
           l = l * f + exp2_fast(sk - mn);
         }
         const float inv = l > 0.f ? f / l : 0.f;
-        __nv_bfloat16* dst = p.out + pair * p.rank + w.half * width0;
-        for (int c = 0; c < width; c += 16) {
+        __nv_bfloat16* dst = p.out + pair * p.rank + col0;
+        for (int c = 0; c < written; c += 16) {
           uint32_t o[16], v[8];
           if (any) {
             ld16(tmem + lane_off + c, o);
@@ -540,18 +513,16 @@ struct LtShape {
   int halves, own_stages, rest_stages;
 };
 // false: a shape whose queries or key tiles do not fit beside each other.  The other chunks of a tile share a
-// stage: one wait and one commit a tile, so that the MMAs of a shape stand in straight code (2 048 rows of 16 heads: 512 + 64 184 -> 157 us,
-// 512 + 0 169 -> 145, 384 + 64 156 -> 127 with halves of three chunks instead of four and two; 3 x 683 rows at 1 000, 256 + 32 111 -> 99).
+// stage: one wait and one commit a tile, so that a tile's MMAs stand in straight code.
 bool lt_shape(int heads, int krow, int rank, LtShape& s) {
   if (heads < 1 || heads > kLtPairs || krow % 16 || rank % 16 || rank < 16 || rank > 512 || rank > krow) return false;
   s.halves = latent_attn_tc_halves(rank);
-  const int chunks = (krow + 63) / 64, own0 = (lt_width0(rank) + 63) / 64, own1 = s.halves > 1 ? (rank - own0 * 64 + 63) / 64 : own0;
-  const int max_rest = chunks - std::min(own0, own1), max_own = std::max(own0, own1);
-  if (max_rest > kLtMaxRest) return false;
-  const int slots = (kLtSmem - 1024 - kLtTail - max_rest * kLtQChunk) / kLtChunk;
+  const int chunks = (krow + 63) / 64, own = lt_own(rank), rest = chunks - own;
+  if (rest > kLtMaxRest) return false;
+  const int slots = (kLtSmem - 1024 - kLtTail - rest * kLtQChunk) / kLtChunk;
   for (s.own_stages = kLtMaxStages; s.own_stages >= 2; --s.own_stages)
-    if (s.own_stages * max_own + 2 * max_rest <= slots) {   // (two of either always fit)
-      s.rest_stages = max_rest ? std::min((slots - s.own_stages * max_own) / max_rest, kLtMaxRestStages) : 1;
+    if (s.own_stages * own + 2 * rest <= slots) {   // (two of either always fit)
+      s.rest_stages = rest ? std::min((slots - s.own_stages * own) / rest, kLtMaxRestStages) : 1;
       return true;
     }
   return false;

@@ -193,3 +193,31 @@ def test_latent_windows_leave_passed_blocks_alone(T, heads, rank, rd, bs, window
     # (as above)
     assert (got - want).norm() / want.norm() < 2.0 ** -8
     assert (got - want).abs().max() < 2.0 ** -8 * rows.float().abs().max() + 2.0 ** -9 * want.abs().max()
+
+
+# Runs of rows whose key rows have every count of chunks that are a half's own (1..4) and that are not (0..5), the last one whole or of one to three 16-wide steps;
+# then two halves of an odd number of chunks (the middle one is in both), with and without splits.
+@pytest.mark.parametrize("rank,rd,splits", [(64 * o - 16 * (r % 3), 64 * r + 16 * (r % 3) - (16 * ((o + r) % 4) if r else 0), 1) for o in range(1, 5) for r in range(6)] + [
+    (80, 0, 1), (272, 0, 1), (272, 16, 2), (288, 16, 1), (320, 32, 2), (336, 0, 1), (400, 48, 2), (448, 64, 3), (448, 0, 1), (464, 0, 2)])
+def test_latent_runs_of_every_count_of_chunks(rank, rd, splits):
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    heads, bs, seqs, krow = 4, 128, [(150, 1), (33, 300), (17, 64)], rank + rd
+    g = torch.Generator(device=DEV).manual_seed(krow * 7 + rank)
+    seq, ctx = [s for s, (n, _) in enumerate(seqs) for _ in range(n)], [c + i for n, c in seqs for i in range(n)]
+    T, scale = len(seq), 0.6 / krow ** 0.5
+    kc = torch.randn(9, 1, bs, krow, generator=g, device=DEV).to(torch.bfloat16)
+    bt = torch.randperm(9, generator=g, device=DEV).to(torch.int32).reshape(3, 3).contiguous()
+    q = (torch.randn(T, heads, krow, generator=g, device=DEV) * 3).to(torch.bfloat16).float()
+    want = torch.stack([_oracle(q[t].double(), kc[bt[seq[t]].long()].reshape(-1, krow).double(), ctx[t], rank, scale, None, 0) for t in range(T)])
+    sq, cx = torch.tensor(seq, dtype=torch.int32, device=DEV), torch.tensor(ctx, dtype=torch.int32, device=DEV)
+    ws = torch.zeros(int(lib.b200_paged_attn_anydim_workspace_bytes(T)), dtype=torch.uint8, device=DEV)
+    part = torch.full((T * heads * splits * (rank + 2),), float("nan"), device=DEV)
+    out = torch.full((T, heads, rank), float("nan"), dtype=torch.bfloat16, device=DEV)
+    check(lib.b200_latent_attn(q.data_ptr(), kc.data_ptr(), bt.data_ptr(), 3, sq.data_ptr(), cx.data_ptr(), out.data_ptr(), T, heads, krow, rank, bs, scale, None,
+                               ws.data_ptr(), splits, part.data_ptr() if splits > 1 else None, None))
+    torch.cuda.synchronize()
+    got = out.double()
+    assert torch.isfinite(got).all()
+    # (as above)
+    assert (got - want).norm() / want.norm() < 2.0 ** -8
+    assert (got - want).abs().max() < 2.0 ** -8 * kc.float().abs().max() + 2.0 ** -9 * want.abs().max()
