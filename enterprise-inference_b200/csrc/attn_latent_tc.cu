@@ -458,11 +458,14 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
       }
       const int64_t pair = (int64_t)(w.t0 + r) * p.heads + h;
       if (p.n_splits > 1) {
-        // unnormalised sums [pair][split][rank | maximum | denominator], the maximum in natural units
+        // sums [pair][split][rank | maximum | denominator], the maximum in natural units.  Two halves add a score's terms in different orders and may follow
+        // the maximum at different tiles: theirs are normalised, with the logarithm of the denominator in the maximum
         float* dst = p.part + (pair * p.n_splits + w.split) * (p.rank + 2);
+        const bool whole = p.halves == 1;
+        const float norm = whole || l <= 0.f ? 1.f : 1.f / l;
         if (alive && w.half == 0) {
-          dst[p.rank] = mu * 0.6931471805599453f;
-          dst[p.rank + 1] = l;
+          dst[p.rank] = (whole || l <= 0.f ? mu : mu + log2f(l)) * 0.6931471805599453f;
+          dst[p.rank + 1] = whole || l <= 0.f ? l : 1.f;
         }
         for (int c = 0; c < written; c += 16) {
           uint32_t o[16];
@@ -473,7 +476,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
           if (alive) {
             float2* d2 = reinterpret_cast<float2*>(dst + col0 + c);   // rank + 2 is even: 8-byte aligned rows
 #pragma unroll
-            for (int j = 0; j < 8; ++j) d2[j] = any ? make_float2(__uint_as_float(o[2 * j]), __uint_as_float(o[2 * j + 1])) : make_float2(0.f, 0.f);
+            for (int j = 0; j < 8; ++j) d2[j] = any ? make_float2(__uint_as_float(o[2 * j]) * norm, __uint_as_float(o[2 * j + 1]) * norm) : make_float2(0.f, 0.f);
           }
         }
       } else {

@@ -221,3 +221,28 @@ def test_latent_runs_of_every_count_of_chunks(rank, rd, splits):
     # (as above)
     assert (got - want).norm() / want.norm() < 2.0 ** -8
     assert (got - want).abs().max() < 2.0 ** -8 * kc.float().abs().max() + 2.0 ** -9 * want.abs().max()
+
+
+def test_latent_splits_of_halves_whose_maxima_part():
+    """The halves of the value columns add a score's terms in different orders.  Here one of them follows the running maximum (17 units, just over the limit of
+    2^8) and the other does not (16, what fp32 leaves of 2^24 + 17 - 2^24): the split's sums have to mean the same in both.  All values are 1."""
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    rank, krow, bs, T, heads, splits = 512, 576, 128, 160, 2, 2
+    kc = torch.ones(3, 1, bs, krow)
+    kc[..., rank:] = 0.0
+    kc[..., 0] = kc[..., 256] = 0.0
+    kc[0, 0, 70, 0], kc[0, 0, 70, 256], kc[0, 0, 70, 512] = 4096.0, -4096.0, 17.0
+    q = torch.zeros(T, heads, krow)
+    q[..., 0] = q[..., 256] = 4096.0
+    q[..., 512] = 1.0
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)   # noqa: E731
+    kd, qd, bt, sq, cx = kc.to(torch.bfloat16).to(DEV), q.to(DEV), i32([[0, 1, 2]]), i32([0] * T), i32(list(range(200, 200 + T)))
+    ws = torch.zeros(int(lib.b200_paged_attn_anydim_workspace_bytes(T)), dtype=torch.uint8, device=DEV)
+    part = torch.full((T * heads * splits * (rank + 2),), float("nan"), device=DEV)
+    out = torch.full((T, heads, rank), float("nan"), dtype=torch.bfloat16, device=DEV)
+    check(lib.b200_latent_attn(qd.data_ptr(), kd.data_ptr(), bt.data_ptr(), 3, sq.data_ptr(), cx.data_ptr(), out.data_ptr(), T, heads, krow, rank, bs, 0.336, None,
+                               ws.data_ptr(), splits, part.data_ptr(), None))
+    torch.cuda.synchronize()
+    got = out.float().cpu()
+    got[..., 0] = got[..., 256] = 1.0
+    assert (got - 1.0).abs().max() < 2.0 ** -7, got.amax()
