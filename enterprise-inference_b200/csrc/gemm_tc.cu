@@ -904,6 +904,10 @@ int linear_tc(const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, const
     pl.N = 128;
     pl.tok_tiles = (T + 127) / 128;
   }
+  // Narrow outputs over deep rows keep these tiles too, while the SMs hold eight shares of k of each at once; pairs share k between four at most, in tiles of 256.
+  // us, in pairs and so: 129 rows, k 14336, 200 features 21.0 and 15.3, 1024 features 22.8 and 18.5; 1024 rows, k 7168, 128 features 16.7 and 13.0; 300 rows,
+  // k 2048, 512 features 12 and 12.  With 24 tiles and more, or fewer shares, it is pairs (300 rows, k 14336, 1024 features 22.8 and 22.5; 512 of k 9.5 and 12.8).
+  const bool narrow = use_cluster && pl.splits == 8 && pl.m_tiles * pl.tok_tiles * 8 <= kNumSMs;
   p.bias = bias;
   p.y = y;
   p.ldy = ldy;
@@ -915,7 +919,7 @@ int linear_tc(const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, const
   p.partials = ws ? reinterpret_cast<float*>(static_cast<char*>(ws) + kCounterBytes) : nullptr;
   p.n_out_pad = pl.n_out_pad;
   p.tile_n = pl.N;
-  if (T > 128 && (mode != kScatter || pl.splits == 1)) return linear_pair(mode, p, x, ldx, w, k, linear_pair_plan(T, n_out, k), s);
+  if (T > 128 && !narrow && (mode != kScatter || pl.splits == 1)) return linear_pair(mode, p, x, ldx, w, k, linear_pair_plan(T, n_out, k), s);
   CUtensorMap mw, mx;
   int rc = get_map(w, (uint64_t)n_out, (uint64_t)k, (uint64_t)k, kBlockM, &mw);
   if (rc) return rc;
