@@ -299,7 +299,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     float* stg = stg_all + grp * (kPairStgBytes / 4);
     float* whole = reinterpret_cast<float*>(smem);   // with k split: the pair's sums of the tile, [token][128]
     const int barrier = 1 + grp;
-    int i = 0;
+    int i = 0, turn = 0;   // turn: the half of the staging area that the next straight piece takes
     for (int t = first; t < tiles; t += step, ++i) {
       const PairTile tile = pair_tile(p, t);
       const int m_tile = 2 * tile.m + rank;
@@ -307,6 +307,13 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       const bool live = (p.gu_ff ? m_tile * (kBlockM / 2) < p.gu_ff : m_tile * kBlockM < p.n_out) && !wait.marked();
       float bb[4];
       pair_bias(p, m_tile, r4, bb);
+      // A whole slab of plain outputs in rows of 16-byte pieces: rounded by the thread that reads them from tensor memory and staged as they are written, 32 tokens in
+      // either half of the staging area in turn (one barrier a piece).  A quarter of the instructions that four features at a time take, which is what launches over
+      // short k are bound by: 2048 tokens, 4096 features, k 512 24.9 us, so 16.9 (20.8 in tiles of 128 x 256, two CTAs to an SM); k 64 24.9, 18.7 (16.7); 1000 tokens
+      // of 8192 features, k 256 23.9, 16.9 (18.7); and 2048 tokens, 28672 features, k 4096 349, 340.
+      const bool straight = MODE == kPlain && p.splits == 1 && p.post_act == 0 && (m_tile + 1) * kBlockM <= p.n_out && p.ldy % 8 == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0;
+      const float bias = straight && p.bias ? __bfloat162float(p.bias[m_tile * kBlockM + srow]) : 0.f;
+      __nv_bfloat16* const y0 = straight ? p.y + (int64_t)tile.row0 * p.ldy + m_tile * kBlockM + (lane & 15) * 8 : nullptr;
       if (MODE == kRopeKv) {   // a token's cos|sin row is a dependent load: ask for the tile's rows while its MMAs run
         const int tt = (warp - 2) * 32 + lane;
         if (tt < n_rows) {
@@ -318,6 +325,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       wait(&acc_full[i & 1], (i >> 1) & 1);
       tc::fence_after();
       const uint32_t taddr = tmem + (uint32_t)((i & 1) * 256) + ((uint32_t)(quad * 32) << 16);
+      if (MODE == kPlain && p.splits == 1 && !straight) asm volatile("bar.sync %0, 128;" ::"r"(barrier) : "memory");   // (the tile before may have been)
       for (int c = grp * kPairStgTok; c < tile.n; c += 2 * kPairStgTok) {
         int pair = -1;   // kScatter: lane l holds the destination and weight of the piece's token l
         float wt = 1.0f;
@@ -330,6 +338,17 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         if (p.splits > 1) {   // one tile a pair: its stages are free by now
 #pragma unroll
           for (int j = 0; j < 32; ++j) whole[(c + j) * kBlockM + srow] = __uint_as_float(r[j]);
+          continue;
+        }
+        if (MODE == kPlain && straight) {
+          __nv_bfloat16* half = reinterpret_cast<__nv_bfloat16*>(stg) + turn * kPairStgTok * kBlockM;
+          turn ^= 1;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) half[j * kBlockM + srow] = __float2bfloat16_rn(__uint_as_float(r[j]) + bias);
+          asm volatile("bar.sync %0, 128;" ::"r"(barrier) : "memory");
+#pragma unroll
+          for (int j = wq * 8 + (lane >> 4); j < wq * 8 + 8; j += 2)   // two tokens a warp and step
+            if (live && c + j < n_rows) *reinterpret_cast<uint4*>(y0 + (int64_t)(c + j) * p.ldy) = *reinterpret_cast<const uint4*>(half + j * kBlockM + (lane & 15) * 8);
           continue;
         }
 #pragma unroll

@@ -128,3 +128,23 @@ def test_gate_up_epilogue_of_narrow_outputs(abi, T, I, k):
 @pytest.mark.parametrize("T,hq,hkv,k,bias", [(200, 2, 1, 2048, True), (700, 1, 1, 4096, False)])
 def test_rope_kv_epilogue_of_narrow_outputs(abi, T, hq, hkv, k, bias):
     importlib.import_module("test_kernels_gpu").test_linear_fused_rope_kv_is_bit_identical_to_unfused(abi.lib(), abi, T, hq, hkv, k, bias)
+
+
+# Plain outputs written in rows of 16-byte pieces, several tiles a pair: slabs that are whole and one that is not, tiles of an odd number of 32-token pieces, short k;
+# and the same where the rows of y are no such pieces (four features at a time), bit for bit.
+@pytest.mark.parametrize("T,n_out,k", [(6000, 1160, 128), (4097, 2048, 64), (2000, 4104, 64), (1300, 8192, 72), (161, 9000, 256), (700, 520, 512)])
+def test_whole_slabs_and_odd_rows_of_outputs(abi, T, n_out, k):
+    lib, P = abi.lib(), abi.ptr
+    g, x, w = _operands(T, n_out, k, k)
+    b = torch.randn(n_out, generator=g, device="cuda").to(BF)
+    wsb = int(lib.b200_linear_workspace_bytes(T, n_out, k))
+    ws, want, ys = torch.zeros(wsb, dtype=torch.uint8, device="cuda"), x.double() @ w.double().T + b.double(), []
+    for ldy, off in ((n_out + 8, 0), (n_out + 3, 0), (n_out + 8, 4)):
+        y = torch.full((T * ldy + 8,), float("nan"), dtype=BF, device="cuda")
+        abi.check(lib.b200_linear_bf16(P(x), k, P(w), P(b), P(y[off:]), ldy, T, n_out, k, 0, P(ws), wsb, None))
+        torch.cuda.synchronize()
+        rows = y[off:off + T * ldy].reshape(T, ldy)
+        assert torch.isnan(rows[:, n_out:].float()).all()
+        ys.append(rows[:, :n_out])
+    assert (ys[0].double() - want).abs().le(_bound(x.double(), w.double(), want)).all()
+    assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
