@@ -810,7 +810,7 @@ int launch_tc(int mode, bool ni, const CUtensorMap& mw, const CUtensorMap& mx, c
 
 }  // namespace
 
-// debug: copy the 16 %globaltimer stamps of the last traced launch (B200_TC_TRACE=1) to the host
+// debug: copy the 16 %globaltimer stamps of the last traced launch (B200_TC_TRACE=1) to the host; launches on pairs of SMs (gemm_pair.cu) carry none and leave the ones before
 int linear_tc_read_trace(unsigned long long* host16) {
   if (!g_trace) return B200_ERR_STATE;
   B200_CUDA(cudaMemcpy(host16, g_trace, 16 * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
@@ -906,8 +906,9 @@ int linear_tc(const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, const
   }
   // Narrow outputs over deep rows keep these tiles too, while the SMs hold eight shares of k of each at once; pairs share k between four at most, in tiles of 256.
   // us, in pairs and so: 129 rows, k 14336, 200 features 21.0 and 15.3, 1024 features 22.8 and 18.5; 1024 rows, k 7168, 128 features 16.7 and 13.0; 300 rows,
-  // k 2048, 512 features 12 and 12.  With 24 tiles and more, or fewer shares, it is pairs (300 rows, k 14336, 1024 features 22.8 and 22.5; 512 of k 9.5 and 12.8).
-  const bool narrow = use_cluster && pl.splits == 8 && pl.m_tiles * pl.tok_tiles * 8 <= kNumSMs;
+  // k 4096, 512 features 14.4 and 11.6.  With 24 tiles and more, or less of k, it is pairs (300 rows, k 14336, 1024 features 22.8 and 22.5; 512 rows, k 2048, 512
+  // features of a fused q|k|v 13.0 and 15.0).
+  const bool narrow = use_cluster && pl.splits == 8 && pl.n_kblocks >= 64 && pl.m_tiles * pl.tok_tiles * 8 <= kNumSMs;
   p.bias = bias;
   p.y = y;
   p.ldy = ldy;

@@ -743,7 +743,8 @@ B200_API int b200_paged_attn_anydim_ex(int32_t f32, const float* q, const void* 
 /* The same attention over bf16 latent cache rows [block][block_size][k_row] on the tensor cores: one kv head, the value of a key
  * is the row's leading `rank` entries, fp32 queries [T][heads][k_row], bf16 output [T][heads][rank].  k_row and rank multiples
  * of 16, rank <= 512 (b200_latent_attn_supported).  workspace: b200_paged_attn_anydim_workspace_bytes(T).  n_splits > 1 with
- * part (n_tokens * heads * n_splits * (rank + 2) floats): the context is walked by n_splits CTAs per group of pairs and merged. */
+ * part (n_tokens * heads * n_splits * (rank + 2) floats): the context is walked by up to n_splits CTAs (or clusters) per group of pairs and
+ * merged.  What is left in the workspace and in part depends on which kernel takes the call. */
 B200_API int b200_latent_attn_supported(int32_t heads, int32_t k_row, int32_t rank);
 B200_API int b200_latent_attn(const float* q, const void* cache, const int32_t* block_table, int32_t bt_stride, const int32_t* row_to_seq,
                               const int32_t* ctx_lens, void* out, int32_t n_tokens, int32_t heads, int32_t k_row, int32_t rank,

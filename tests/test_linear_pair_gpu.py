@@ -113,19 +113,19 @@ def test_experts_on_pairs_of_sms(abi, width, ff, experts, top, rows, gated, weig
 
 
 # Narrow outputs over deep rows of more than 128 tokens (eight shares of k in tiles of 128 x 128) and their neighbours on pairs of SMs: up to 18 tiles and more,
-# 32 k blocks and fewer, uneven shares, part tiles of either side.
-@pytest.mark.parametrize("T,n_out,k", [(129, 8, 2048), (300, 200, 4160), (1024, 264, 2056), (2304, 128, 2048), (2305, 128, 2048), (129, 1152, 4096), (129, 1153, 4096),
-                                       (200, 512, 1984), (257, 1280, 4160), (255, 2312, 4096), (160, 1024, 14336)])
+# 64 k blocks and fewer, uneven shares, part tiles of either side.
+@pytest.mark.parametrize("T,n_out,k", [(129, 8, 4096), (300, 200, 4160), (1024, 264, 4104), (2304, 128, 4096), (2305, 128, 4096), (129, 1152, 4096), (129, 1153, 4096),
+                                       (200, 512, 4032), (257, 1280, 4160), (255, 2312, 4096), (160, 1024, 14336)])
 def test_narrow_outputs_over_deep_rows(abi, T, n_out, k):
     test_linear_pairs_of_sms(abi, T, n_out, k, 8)
 
 
-@pytest.mark.parametrize("T,I,k", [(160, 128, 2048), (700, 64, 4096)])
+@pytest.mark.parametrize("T,I,k", [(160, 128, 4096), (700, 64, 4096)])
 def test_gate_up_epilogue_of_narrow_outputs(abi, T, I, k):
     test_gate_up_epilogue_on_pairs_of_sms(abi, T, I, k)
 
 
-@pytest.mark.parametrize("T,hq,hkv,k,bias", [(200, 2, 1, 2048, True), (700, 1, 1, 4096, False)])
+@pytest.mark.parametrize("T,hq,hkv,k,bias", [(200, 2, 1, 4096, True), (700, 1, 1, 4160, False)])
 def test_rope_kv_epilogue_of_narrow_outputs(abi, T, hq, hkv, k, bias):
     importlib.import_module("test_kernels_gpu").test_linear_fused_rope_kv_is_bit_identical_to_unfused(abi.lib(), abi, T, hq, hkv, k, bias)
 
