@@ -12,8 +12,9 @@
 // before gives its columns back, and 68 MMAs of 40 to 50 cycles; 3.5 us per 128 keys.  (Tiles of 64 keys, whose next one would fit: the scores' MMAs cost
 // as much, 119 us for 100 rows at contexts 1500..3000 against 86.  Rows asked into L2 ahead, 104 against 101: memory is not it.)
 // MMAs of a whole chunk are straight code: in a loop of as many as the chunk has 16-wide steps each took 110 cycles (101 us against 86).
-// 16 heads over 512 + 64 (256 + 32), us, attn_latent_tc.cu -> here: 64 rows at contexts 500..1000 49 -> 28 (35 -> 18), 100 at 1500..3000 184 -> 86
-// (97 -> 54), one at 3000 51 -> 21, 33 at 1000..2000 96 -> 27, 128 of one sequence behind 3000 tokens 87 -> 83, error against 64 bits as there.
+// 16 heads over 512 + 64, us, on attn_latent_tc.cu (with the splits that the caller asks for) and here: 64 rows at contexts 500..1000 49, 27 (among other calls), 100 of
+// 3000 208, 96, one of 3000 54, 25, 33 of 3000 122, 43; of one sequence 33 behind 3000 73, 33, 100 behind 3000 87, 86 and behind 16 000 183, 385: what is whose is
+// latent_attn_route's and runs.cuh's.  Error against 64 bits as there.
 // Warps: TMA producer, MMA issuer, four softmax warps (a thread owns a key, then a value column).  The running maximum is only followed when it
 // rises by more than 2^8, as in attn_latent_tc.cu.  Every wait is bounded and reported (tc.cuh).
 #include <algorithm>

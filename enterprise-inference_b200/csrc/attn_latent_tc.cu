@@ -14,7 +14,7 @@
 // The weights overwrite the scores in place (A operand of the second product, per 32 scores 16 columns of bf16 pairs and 16 of what
 // rounding took from them) and never touch shared memory.
 // Against the mma.sync kernel of attn_latent.cu with 16 pairs a CTA, which reads every key tile once per row: 2 048 rows of 16
-// heads over 512 + 64 at contexts 1..2048 907 -> 157 us; error against 64 bits 2.57e-3 -> 2.30e-3 (decode rows: attn_latent_rows.cu).  (With weights of one bf16 term, as there, about a tenth faster, but 2.61e-3 and 2.72e-3: the
+// heads over 512 + 64 at contexts 1..2048 907 -> 170 us among other calls; error against 64 bits 2.57e-3 -> 2.30e-3 (decode rows: attn_latent_rows.cu).  (With weights of one bf16 term, as there, about a tenth faster, but 2.61e-3 and 2.72e-3: the
 // lazily followed maximum costs the exactness of the largest weight.)
 // Warps: TMA producer, MMA issuer, four softmax warps (a thread owns a pair), eight that stage the next item's queries.
 // The running maximum is only followed when it rises by more than 2^8 (the scaling of all terms is the same, so the

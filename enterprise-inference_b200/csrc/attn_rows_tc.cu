@@ -13,9 +13,9 @@
 // Scores may be capped, biased by distance (each score takes its own distance's bias and no other: tables may end in -inf or any sentinel),
 // windowed with kept first keys (EX); outputs may have a sink in the denominator and a gate per head.  The running maximum is only followed when it rises by more than 2^8 (exact: all terms are scaled alike); a warp then
 // rescales its 32 rows of O in TMEM.
-// Bound by the tensor core or the softmax's issue slots: 2 048 rows at contexts 1001..3048, 32 heads over 8: 108 us (112 with branches between the
-// issuing warp's MMAs and the maximum of a key tile in one chain, 212 on the kernel before); 1 900
-// rows of three sequences, 16 heads over 4, capped, biased, window 1024: 76 us (278 us on the mma.sync kernel of attn_latent.cu).
+// Bound by the tensor core or the softmax's issue slots: 2 048 rows at contexts 1001..3048, 32 heads over 8: 117 us among other calls (119 with branches between
+// the issuing warp's MMAs and the maximum of a key tile in one chain, 211 on the kernel before); 1 900
+// rows of three sequences, 16 heads over 4, capped, biased, window 1024: 74 us (278 us on the mma.sync kernel of attn_latent.cu).
 // Warps: four softmax warps per tile (a thread owns a pair), TMA, MMA, two that stage queries.  Every wait is bounded and
 // reported (tc.cuh).
 #include <algorithm>

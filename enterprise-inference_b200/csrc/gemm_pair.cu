@@ -10,11 +10,12 @@
 // accumulators, so a tile's epilogue runs beside the next tile's MMAs; it goes through shared memory of its own, 32 tokens at a time per
 // four warps.  Launches with few tiles share a tile's k between up to four pairs of one cluster, which add up through distributed shared memory.
 //
-// Against 128 x 256 tiles of single CTAs with k split over clusters (us, before -> now): 2000 tokens, k 14336, 4096 features 179 -> 162; 2048, 4096,
-// 28672 404 -> 320; 2048, 4096, 6144 107 -> 78; 1000, 4096, 4096 62 -> 38; 300, 2048, 2048 22 -> 12; 200, 14336, 4096 50 -> 32; 130, 2048, 2048 19 -> 11.
+// Against 128 x 256 tiles of single CTAs with k split over clusters (us, before -> now; five calls in a row after the L2 was overwritten): 2000 tokens, k 14336,
+// 4096 features 177 -> 158 (among other calls, under the power cap, 208 -> 194); 2048, 4096, 28672 472 -> 337; 2048, 4096, 6144 142 -> 94; 1000, 4096, 4096 72 -> 41;
+// 300, 2048, 2048 32 -> 18; 200, 14336, 4096 67 -> 45; 130, 2048, 2048 29 -> 17.
 // Routed experts (the table of token tiles is moe.cu's): 32 experts of 1024, width 2048, 4 of them a row, router and grouping included, tiles of
-// 128 x 128 before: 2048 rows 263 -> 174, 1000 rows 193 -> 138, 600 rows 165 -> 125; 64 of 512, width 4096, 8 a row, 2048 rows 586 -> 361.  Their
-// weights come from HBM (1000 rows: 402 MB), and whole waves of tiles decide the rest (2048 rows: 5.2 waves of gate|up).
+// 128 x 128 before: 2048 rows 264 -> 175 (among other calls 280 -> 192), 1200 rows 222 -> 135, 700 rows 164 -> 124; 64 of 512, width 4096, 8 a row, 2048 rows
+// 582 -> 363.  Their weights come from HBM (1000 rows: 402 MB), and whole waves of tiles decide the rest (2048 rows: 5.2 waves of gate|up).
 // 128 tokens and fewer stay on gemm_tc.cu's tiles: their launches stream W, and 148 CTAs with two of them to an SM keep more of it in flight
 // (64 tokens, 4096, 28672: 42 there, 49 here; 128, 14336, 4096: 33 and 34).
 #include <algorithm>
