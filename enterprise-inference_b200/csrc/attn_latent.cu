@@ -411,15 +411,17 @@ static LatentShare latent_share(const int32_t* plan, int T, int heads, int krow,
   LatentShare s = {};
   s.plan = plan;
   s.rows = T;
-  s.groups = latent_attn_rows_items(1, heads);
-  s.cluster = latent_attn_rows_cluster(T * s.groups);
   s.splits = n_splits;
   s.halves = latent_attn_tc_halves(rank);
   s.rows_per_item = latent_attn_tc_rows(heads);
   s.seen = window > 0 ? window : INT_MAX;
-  s.rows_ns = 4.2f + 0.035f * krow;
-  s.runs_ns = 1.15f * std::max(16.5f, 0.043f * krow);
-  s.runs_fixed = 10000.f + 54.f * krow;
+  const int groups = latent_attn_rows_items(1, heads);
+  const float by_row = 4.2f + 0.035f * krow, by_run = 1.15f * std::max(16.5f, 0.043f * krow);
+  s.row_key = by_row / latent_attn_rows_cluster(T * groups);
+  s.row_tile = by_row * 64 * groups / kNumSMs;
+  s.run_fixed = 10000.f + 54.f * krow;
+  s.run_key = by_run / n_splits;
+  s.run_item = by_run * 64 / n_splits;
   return s;
 }
 
@@ -443,8 +445,8 @@ LatentRoute latent_attn_route(const float* q, const __nv_bfloat16* kc, const int
   if (n_splits <= 1 || !part || !tc || (items <= 7 && longest > 32768)) return LatentRoute::kRows;
   // the longest row alone: what its CTAs take, and what they would take over runs in splits, with the launches that tell
   const LatentShare s = latent_share(nullptr, T, heads, krow, rank, n_splits, 0);
-  const float gain = (s.rows_ns / s.cluster - s.runs_ns / 1.15f / s.splits) * (float)longest;
-  return gain > s.runs_fixed + 12000.f ? LatentRoute::kEither : LatentRoute::kRows;
+  const float gain = (s.row_key - s.run_key / 1.15f) * (float)longest;
+  return gain > s.run_fixed + 12000.f ? LatentRoute::kEither : LatentRoute::kRows;
 }
 
 // runs / n_runs: the run list of the step (attn_anydim.cu builds it: runs of at most 16 consecutive rows of one sequence)

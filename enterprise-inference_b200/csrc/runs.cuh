@@ -41,20 +41,34 @@ __device__ __forceinline__ int run_share(const RunShare& s, int G) {
 // 756, 368.  The launches that a step does not need cost it 8 us.
 struct LatentShare {
   const int32_t* plan;   // its words; null: the kernel has the step to itself
-  int rows, groups, cluster, splits, halves, rows_per_item, seen;   // groups: of 16 heads; seen: a window's tokens (or INT_MAX)
-  float rows_ns, runs_ns, runs_fixed;
+  int rows, splits, halves, rows_per_item, seen;   // seen: a window's tokens (or INT_MAX)
+  // ns of a key of the longest row and of a 64-token tile of all runs, by rows; the fixed part, a key of the longest row and a key of an item over runs
+  float row_key, row_tile, run_fixed, run_key, run_item;
 };
+// Every kernel of the step has to come to the same answer: products and sums are rounded one by one, not as a compiler joins them.
+__host__ __device__ __forceinline__ float ls_mul(float a, float b) {
+#ifdef __CUDA_ARCH__
+  return __fmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
 __host__ __device__ __forceinline__ bool latent_by_rows(const LatentShare& s, int n_runs, int longest, int tiles) {
-  const float most = (float)(longest < s.seen ? longest : s.seen), each = (float)(s.seen >> 6) + 2.f;
-  const float walked = 64.f * fminf((float)tiles, each * (float)n_runs);                    // keys of all runs
-  const int parts = (s.rows + n_runs * s.rows_per_item - 1) / (n_runs * s.rows_per_item);   // items of a run in the mean
-  const float items = (float)n_runs * parts * s.halves * s.splits, rounds = ceilf(items / kNumSMs);
-  const float by_rows = s.rows_ns * fmaxf(most / s.cluster, walked * s.groups / kNumSMs);
-  const float by_runs = s.runs_fixed + s.runs_ns * fmaxf(most / s.splits, walked * parts * s.halves * rounds / items);
-  return by_rows <= by_runs;
+  const float most = (float)(longest < s.seen ? longest : s.seen), each = ls_mul((float)((s.seen >> 6) + 2), (float)n_runs);
+  const float walked = fminf((float)tiles, each);                                            // tiles of all runs
+  const int parts = (s.rows + n_runs * s.rows_per_item - 1) / (n_runs * s.rows_per_item);    // items of a run in the mean
+  const int rounds = (n_runs * parts * s.halves * s.splits + kNumSMs - 1) / kNumSMs;
+  const float by_rows = fmaxf(ls_mul(s.row_key, most), ls_mul(s.row_tile, walked));
+  const float per_item = ls_mul(walked, (float)rounds), run = fmaxf(ls_mul(ls_mul(s.run_key, most), (float)n_runs), ls_mul(s.run_item, per_item));
+  // (both sides times n_runs: no division)
+#ifdef __CUDA_ARCH__
+  return ls_mul(by_rows, (float)n_runs) <= __fadd_rn(ls_mul(s.run_fixed, (float)n_runs), run);
+#else
+  return ls_mul(by_rows, (float)n_runs) <= s.run_fixed * (float)n_runs + run;
+#endif
 }
 __device__ __forceinline__ bool latent_by_rows(const LatentShare& s) {
-  return latent_by_rows(s, max(__ldg(s.plan), 1), __ldg(s.plan + kRunLongest), __ldg(s.plan + kRunTiles));
+  return latent_by_rows(s, max(__ldcg(s.plan), 1), __ldcg(s.plan + kRunLongest), __ldcg(s.plan + kRunTiles));
 }
 
 // Is a run (its second word) the mma.sync kernel's?  A segment of at most kRunRows rows is one run in every list.

@@ -1,6 +1,8 @@
 """Which kernel latent attention takes: the rule against what both took on a B200."""
 import ctypes
+import random
 
+import numpy as np
 import pytest
 
 from conftest import pkg
@@ -64,6 +66,29 @@ def test_routes_of_forms(lib):
 
 
 def test_nothing_overflows(lib):
-    for T, longest in ((1, 1 << 30), (148, 1 << 30), (1 << 16, 1 << 20)):
+    for T, longest in ((1, 1 << 30), (148, 1 << 30), (148, 1 << 60), (1 << 16, 1 << 20)):
         assert lib.b200_debug_latent_route(T, 16, 576, 512, 128, 16, longest, 1) in (ROWS, EITHER, RUNS)
         assert lib.b200_debug_latent_by_rows(T, 16, 576, 512, 16, 0, T, min(longest, (1 << 31) - 1), (1 << 31) - 1) in (0, 1)
+
+
+def test_the_devices_answer_is_rounded_step_by_step(lib):
+    """Several kernels answer the same question apart: the rule over a grid of plans is what fp32 products and sums give, rounded one by one."""
+    rng, f = random.Random(1), np.float32
+    for _ in range(2000):
+        T, heads, krow, splits = rng.randint(1, 148), rng.choice([1, 4, 16, 17, 40, 128]), rng.choice([80, 192, 288, 512, 576]), rng.randint(2, 16)
+        rank, window, n_runs = min(krow, 512), rng.choice([0, 0, 512, 4096]), rng.randint(1, T)
+        longest = rng.randint(1, 1 << rng.randint(1, 20))
+        tiles = rng.randint(-(-longest // 64), n_runs * -(-longest // 64))
+        groups, per = -(-heads // 16), min(128 // heads, 16)
+        cluster = next(c for n, c in ((15, 8), (33, 4), (74, 2), (1 << 30, 1)) if T * groups <= n)
+        by_row, by_run = f(4.2) + f(0.035) * f(krow), f(1.15) * max(f(16.5), f(0.043) * f(krow))
+        row_key, row_tile = by_row / f(cluster), by_row * f(64) * f(groups) / f(148)
+        fixed, run_key, run_item = f(10000) + f(54) * f(krow), by_run / f(splits), by_run * f(64) / f(splits)
+        seen = window or (1 << 31) - 1
+        most, walked = f(min(longest, seen)), min(f(tiles), f(seen // 64 + 2) * f(n_runs))
+        parts, halves = -(-T // (n_runs * per)), 2 if rank > 256 else 1
+        rounds = -(-(n_runs * parts * halves * splits) // 148)
+        by_rows = max(row_key * most, row_tile * walked)
+        run = max(run_key * most * f(n_runs), run_item * (walked * f(rounds)))
+        want = by_rows * f(n_runs) <= fixed * f(n_runs) + run
+        assert lib.b200_debug_latent_by_rows(T, heads, krow, rank, splits, window, n_runs, longest, tiles) == int(want)
