@@ -494,7 +494,7 @@ int delta_prep(bool f32, const void* fused, int64_t ld, const void* a2, const fl
 // the scan with the decay of (row, head, channel) at decay[t * g_row + h * g_head + d * g_chan]; delta_rule false: u = beta v
 int linear_scan(bool delta_rule, const float* qn, const float* kn, const float* vn, const float* beta, const float* decay, int64_t g_row,
                 int g_head, int g_chan, const int32_t* positions, const int32_t* seq_start, const int32_t* seq_slots, float* state,
-                int64_t slot_stride, float* out, int S, int heads, int kv_heads, int dim, int vd, cudaStream_t s, bool single_rows = false);
+                int64_t slot_stride, float* out, int S, int heads, int kv_heads, int dim, int vd, cudaStream_t s, int rows = 0);   // rows: of the S sequences together (0: not known)
 // state-space mixer (ssd.cu)
 int64_t ssd_tail_floats(int heads, int groups, int state, int vdim, int taps);
 int ssd_prep(bool f32, const void* fused, int64_t ld, const float* conv_w, const float* conv_b, const float* dt_bias, const float* a_log,
@@ -519,7 +519,7 @@ int delta_tails(bool f32, const void* fused, int64_t ld, const int32_t* position
                 float* tails, int64_t slot_stride, int S, int channels, int taps, cudaStream_t s);
 int delta_scan(const float* qn, const float* kn, const float* vn, const float* beta, const float* decay, const int32_t* positions,
                const int32_t* seq_start, const int32_t* seq_slots, float* state, int64_t slot_stride, float* out, int S, int heads,
-               int kv_heads, int dim, int vd, cudaStream_t s, bool single_rows = false);
+               int kv_heads, int dim, int vd, cudaStream_t s, int rows = 0);
 // true-fp32 CUDA-core linear (linear_simt.cu)
 int linear_simt(bool x_f32, bool y_f32, const void* x, int64_t ldx, const __nv_bfloat16* w, void* y, int64_t ldy, int T, int n_out,
                 int k, cudaStream_t s, const __nv_bfloat16* bias = nullptr, int act = -1);

@@ -846,14 +846,14 @@ int delta_tails(bool f32, const void* fused, int64_t ld, const int32_t* position
 
 int delta_scan(const float* qn, const float* kn, const float* vn, const float* beta, const float* decay, const int32_t* positions,
                const int32_t* seq_start, const int32_t* seq_slots, float* state, int64_t slot_stride, float* out, int S, int heads,
-               int kv_heads, int dim, int vd, cudaStream_t s, bool single_rows) {
+               int kv_heads, int dim, int vd, cudaStream_t s, int rows) {
   return linear_scan(true, qn, kn, vn, beta, decay, (int64_t)heads * dim, dim, 1, positions, seq_start, seq_slots, state, slot_stride, out, S,
-                     heads, kv_heads, dim, vd, s, single_rows);
+                     heads, kv_heads, dim, vd, s, rows);
 }
 
 int linear_scan(bool delta_rule, const float* qn, const float* kn, const float* vn, const float* beta, const float* decay, int64_t g_row,
                 int g_head, int g_chan, const int32_t* positions, const int32_t* seq_start, const int32_t* seq_slots, float* state,
-                int64_t slot_stride, float* out, int S, int heads, int kv_heads, int dim, int vd, cudaStream_t s, bool single_rows) {
+                int64_t slot_stride, float* out, int S, int heads, int kv_heads, int dim, int vd, cudaStream_t s, int rows) {
   if (S == 0) return B200_OK;
   B200_REQUIRE(dim > 0 && dim <= 256 && vd > 0, B200_ERR_UNSUPPORTED, "delta_scan: key size %d outside (0, 256]", dim);
   B200_REQUIRE(heads > 0 && kv_heads > 0 && heads % kv_heads == 0, B200_ERR_INVALID, "delta_scan: %d heads over %d", heads, kv_heads);
@@ -866,6 +866,10 @@ int linear_scan(bool delta_rule, const float* qn, const float* kn, const float* 
           (!chan || (g_chan == 1 && g_row % 4 == 0 && g_head % 4 == 0 && at(decay) % 16 == 0));
   const dim3 grid(S, heads, (vd + kDsCols - 1) / kDsCols), block(kDsThreads);
   const int64_t ctas = (int64_t)S * heads * grid.z;
+  const bool single_rows = rows == S;
+  // Blocks where a portion may be long enough for them; where the rows of the step are known to be too few its walk is launched by itself (one portion of 63 rows, 16
+  // heads of 128 x 128: 19.0 us from the block kernel, 18.2; of two rows 5.5 and 5.1)
+  const bool blocks = a.vec && ctas <= 3 * kNumSMs && (rows <= 0 || rows - S + 1 >= db_from(dim > 64 && ctas <= 2 * kNumSMs ? 32 : 16));
 #define SCAN3(D, R, CH)                                                                                       \
   do {                                                                                                        \
     static bool done[64] = {};                                                                                \
@@ -875,7 +879,7 @@ int linear_scan(bool delta_rule, const float* qn, const float* kn, const float* 
       break;                                                                                                  \
     }                                                                                                         \
     if constexpr (D <= 2 && R)                                                                                \
-      if (a.vec && ctas <= 3 * kNumSMs) {                                                                     \
+      if (blocks) {                                                                                           \
         if (const int e = delta_blocks<D, CH>(a, S, ctas, s)) return e;                                       \
         break;                                                                                                \
       }                                                                                                       \

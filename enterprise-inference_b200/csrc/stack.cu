@@ -546,7 +546,7 @@ static int stack_enqueue_step_postnorm(b200_ctx* c, const StepArgs& a, cudaStrea
                       L.decay_rank, L.gate_rank, s));
       STEP(delta_tails(f32, M->qkv, qr, a.positions, M->seq_start, seq_slots, tails, M->slot_floats, S, C, L.conv_taps, s));
       STEP(delta_scan(M->dq, M->dk, M->dv, M->dbeta, M->ddecay, a.positions, M->seq_start, seq_slots, M->state + W.rec_off, M->slot_floats,
-                      M->oraw, S, L.heads, L.kv_heads, L.dim, L.vdim, s, S == T));
+                      M->oraw, S, L.heads, L.kv_heads, L.dim, L.vdim, s, T));
       STEP(head_norm_gate(f32, M->oraw, W.head_norm, M->g2, av, M->attn, T, L.heads, L.vdim, m.norm_eps, s));
     }
     STEP(stack_linear(c, M->attn, av, W.o, M->y, Wd, T, Wd, av, s));
@@ -850,7 +850,7 @@ static int stack_enqueue_step_hyper(b200_ctx* c, const StepArgs& a, cudaStream_t
                       M->slot_floats, M->dq, M->dk, M->dv, M->dbeta, M->ddecay, T, L.heads, L.kv_heads, L.dim, L.vdim, L.conv_taps, 0, 0, s, true));
       STEP(delta_tails(f32, M->qkv, qr, a.positions, M->seq_start, seq_slots, tails, M->slot_floats, S, C, L.conv_taps, s));
       STEP(linear_scan(true, M->dq, M->dk, M->dv, M->dbeta, M->ddecay, L.heads, 1, 0, a.positions, M->seq_start, seq_slots, M->state + W.rec_off,
-                       M->slot_floats, M->oraw, S, L.heads, L.kv_heads, L.dim, L.vdim, s, S == T));
+                       M->slot_floats, M->oraw, S, L.heads, L.kv_heads, L.dim, L.vdim, s, T));
       const char* gptr = static_cast<const char*>(M->qkv) + (int64_t)C * es;
       STEP(head_norm_gate(f32, M->oraw, W.head_norm, gptr, qr, M->attn, T, L.heads, L.vdim, m.norm_eps, s, true));
     } else {
@@ -861,7 +861,7 @@ static int stack_enqueue_step_hyper(b200_ctx* c, const StepArgs& a, cudaStream_t
       const char* xbc = static_cast<const char*>(M->qkv) + (int64_t)av * es;
       STEP(delta_tails(f32, xbc, qr, a.positions, M->seq_start, seq_slots, tails, M->slot_floats, S, C, L.conv_taps, s));
       STEP(linear_scan(false, M->dq, M->dk, M->dv, M->dbeta, M->ddecay, L.heads, 1, 0, a.positions, M->seq_start, seq_slots, M->state + W.rec_off,
-                       M->slot_floats, M->oraw, S, L.heads, L.kv_heads, L.dim, L.vdim, s, S == T));
+                       M->slot_floats, M->oraw, S, L.heads, L.kv_heads, L.dim, L.vdim, s, T));
       STEP(ssd_gate_norm(f32, M->oraw, M->dv, W.skip, M->qkv, qr, W.head_norm, M->attn, T, L.heads, L.vdim, L.norm_groups, m.norm_eps, s));
     }
     STEP(stack_linear(c, M->attn, av, W.o, M->y, Wd, T, Wd, av, s));
