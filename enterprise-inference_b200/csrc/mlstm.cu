@@ -11,7 +11,7 @@
 //    sequence's rows of the step in order (mlstm_walk.cuh; a decode row is a walk of one) with the state in registers; it is stored as
 //    [head][vdim][dim].  n and m are kept once per 32 columns (every CTA of a head needs them from the step before, so they cannot
 //    all share one copy that one of them overwrites).  A sequence whose first row is at position 0 starts from zeros.  Longer portions
-//    go through the tensor cores in chunks (mlstm_chunk.cu).
+//    go through the tensor cores in chunks (mlstm_chunk.cuh) and segments (mlstm_chunk.cu).
 //  * head_norm_gate: unit RMS per head, weight, sigmoid gate (or the gate's silu).
 #include "mlstm_walk.cuh"
 
@@ -212,14 +212,15 @@ int mlstm_scan(bool f32, const void* qkv, int64_t ld, int q_off, int k_off, int 
   if (S == 0) return B200_OK;
   B200_REQUIRE(dim > 0 && dim <= 256 && vd > 0, B200_ERR_UNSUPPORTED, "mlstm_scan: key size %d outside (0, 256]", dim);
   B200_REQUIRE(positions && seq_start && seq_slots && state, B200_ERR_INVALID, "mlstm_scan: null argument");
-  MlstmArgs a = {qkv, gates, positions, seq_start, seq_slots, state, out, ld, slot_stride, q_off, k_off, v_off, heads, dim, vd, 1.0f / sqrtf((float)dim), 0, 0, 0};
+  MlstmArgs a = {qkv, gates, positions, seq_start, seq_slots, state, out, ld, slot_stride, q_off, k_off, v_off, heads, dim, vd, 1.0f / sqrtf((float)dim), -0.5 * log2((double)dim), 0, 0, 0, 0};
   mlstm_walk_widths(a, f32);
-  // Steps of a few bf16 portions in chunks on the tensor cores where they are long (2 048 rows of 8 heads, 128 x 256: 144 us; the scalar walk
-  // before it 724).  While all CTAs fit the device at once (two an SM), the chunk kernel walks the short portions itself; beyond that each
-  // kernel takes its portions (64 rows of four sequences: 15.0 us, in one kernel 23.1: the idle half of each cluster holds up the next).
-  // More sequences than four go to the walk alone (64 of one row 36 us; longer portions of many sequences in chunks have not been measured).
+  // Steps of a few bf16 portions on the tensor cores where they are long, in segments from 193 rows on and in chunks from 97.  While all CTAs fit the device
+  // at once, the segments' kernel takes the short portions itself; beyond that each kind of portion has its kernel (two sequences of 50 rows, 8 heads of
+  // 128 x 256: 20 us, in one kernel 24).  One launch for all costs portions of 97 to 192 rows, whose length is known on the device only, 0.8 us of 12 to 1.3 of 16.6;
+  // a launch more would cost every call 2 us of host time.
+  // More sequences than four go to the walk alone (64 of one row 36 us; longer portions of many sequences in segments have not been measured).
   if (!f32 && !single_rows && S <= 4 && mlstm_chunk_supported(a)) {
-    a.both = (int64_t)S * heads * 2 * mlstm_col_blocks(vd) > 2 * kNumSMs;
+    a.both = mlstm_chunk_ctas(a, S) > kNumSMs;
     if (const int e = mlstm_chunk(a, S, s)) return e;
     if (!a.both) return B200_OK;
     const PdlScope after_chunks;

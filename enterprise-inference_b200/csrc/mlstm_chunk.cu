@@ -1,443 +1,715 @@
-// The matrix-memory recurrence of mlstm.cu over longer portions in chunks of 64 rows on the tensor cores (bf16 rows).
+// The matrix-memory recurrence of mlstm.cu over longer portions on tcgen05 (bf16 rows), cut in time over the CTAs of a cluster.
 //
-// With F_t the sum of the log forget gates of the chunk up to row t, m_t = F_t + max(m_0, max_{s<=t} (i_s - F_s)) is the running maximum
-// of the row-by-row walk, and
-//   S_t = exp(F_t + m_0 - m_t) S_0 + sum_{s<=t} exp(F_t - F_s + i_s - m_t) k_s v_s^T          (n_t likewise with v = 1)
-// so a chunk is four products: P = Q K^T, weighted by the exponentials under the diagonal; P V; Q S_0; K^T (w V) for the next state.
-// Everything that was fp32 in the walk stays so in effect: sums F are taken in 64 bits (differences of large sums), an fp32 operand (P, S_0,
-// w V) enters the bf16 MMA as three bf16 terms (24 bits) against rows that are bf16 to begin with, accumulators are fp32.  n is carried
-// as a 17th column with value 1.
+// With F_t the sum of the log forget gates up to row t of a segment, M_t = max_{s<=t} (i_s - F_s) and m_t = F_t + max(m_0, M_t), which is the running maximum
+// of the row-by-row walk,
+//   S_t = exp(F_t + m_0 - m_t) S_0 + exp(F_t + M_t - m_t) sum_{s<=t} exp(i_s - F_s - M_t) k_s v_s^T          (n_t likewise with v = 1)
+// so a segment needs S_0, n_0 and m_0 of the rows before it, and neither what it adds to them nor its own sums depend on them.
 //
-// One CTA per (sequence, head, 16 value columns) walks the chunks; the two of a cluster share one stored copy of n and m, and a barrier keeps either from storing before both have read.
-// Warps w of 8: rows 16 (w % 4) of P and O, the key blocks (and for Q S_0 the dimensions) dealt to the two warps of a row group, whose
-// sums meet in shared memory; dimensions 16 w of the state, kept in fp32 accumulator fragments.  A ninth warp works out the next
-// chunk's gate scalars.  Rows arrive by cp.async a chunk ahead.
-// Bound by latency (about 800 instructions a warp and chunk, two barriers).  2 048 rows of 8 heads, 128 x 256: 144 us against 724 us
-// of the scalar walk; error of the results against 64 bits 6.8e-7 (walk 1.2e-6), of the state 7.5e-8 (1.5e-7).
+// A cluster of four CTAs takes (sequence, head, 64 value columns), up to 1 024 rows at a time, each CTA a segment of up to 256:
+//   1. sums F and maxima M of its gates; D = K^T (w V) with w_s = exp(i_s - F_s - M_L), the segment's own part of the state (M: dimensions, N: columns);
+//   2. outputs as attention within the segment: scores Q K^T in blocks of 128 rows x 128 keys, weighted by the exponentials under the diagonal, times V;
+//   3. every CTA reads the earlier segments' D over the cluster's shared memory and adds up its S_0 (the last one the state after all): Q S_0.
+// Nothing walks from chunk to chunk.  Everything that was fp32 in the walk stays so in effect: sums F are taken in 64 bits (differences of large
+// sums), an fp32 operand (weights, w V, S_0) enters the bf16 MMA as three bf16 terms (24 bits) against rows that are bf16 to begin with, the small
+// terms first, accumulators are fp32 and given up for a new one every 64 rows of D and 128 keys.
+// Weights of a row on 32 keys that all lie before it are the product of two exponentials around the keys' maximum, one a row and one a key; only blocks on the diagonal take
+// one a pair (there a later row's key may be the maximum, and the product overflow).
+// A value that is not finite is taken out of V before the products (0 times it would reach earlier rows); its column is NaN from its row on.
+//
+// Why tcgen05, and segments: in chunks of 64 rows on mma.sync (mlstm_chunk.cuh) 2 048 rows of 8 heads, 128 x 256, are 32 dependent chunks of 4.4 us; the same
+// segments on mma.sync took 103 us, because m16n8k16 takes 16 cycles of a scheduler here (three terms of everything: 92 000 cycles).
+// What bounds it now: the instructions of a round (45 000 issue slots a scheduler for two rounds, a third of the stalls are instruction fetches,
+// hence loops that stay loops, one copy of each phase), and the phases' latency, one CTA an SM.  2 048 rows of 8 heads, 128 x 256: 142 -> 57 us; 1 024: 73 -> 31;
+// 512: 38 -> 21; two sequences together 2 048: 146 -> 102; 8 000 rows 545 -> 220; 64 x 128: 114 -> 54.
+// Error of the results against 64 bits, over 32 cases: 5.1e-7 (chunks 5.6e-7), of the state 6.8e-8 (7.8e-8); scores in one accumulator would
+// make it 6.0e-7 (eight truncated sums of 16 dimensions), weights by expf 6.4e-7.
+// Tried: eight warps instead of sixteen 68 us; D over the cluster's shared memory 12 000 cycles a round instead of 4 000; the MMAs issued by a warp with rows 65 us.
 #include <algorithm>
 
-#include "mlstm_walk.cuh"
+#include "mlstm_chunk.cuh"
+#include "tc.cuh"
 
 namespace b200 {
+
+uint32_t* wait_status_word();
+int wait_status();
+
 namespace {
 
-constexpr int kMcRows = 64, kMcCols = 16, kMcW = 24;   // rows of a chunk; value columns; columns with n and its padding (bf16 rows of 48 bytes)
-constexpr int kMcThreads = 288, kMcGate = 8;
-static_assert(kMcThreads == kScanThreads && 2 * kMcCols == kScanCols, "the walk takes a pair's columns with one CTA's threads");
+using namespace tc;
 
-__device__ __forceinline__ uint32_t sa(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const void* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(sa(p)) : "memory");
-}
-__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], const void* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(sa(p)) : "memory");
-}
-__device__ __forceinline__ void ldsm2t(uint32_t (&r)[2], const void* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(sa(p)) : "memory");
-}
-__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// 16 bytes, or zeros (live false)
-__device__ __forceinline__ void cp16z(void* dst, const void* src, bool live) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sa(dst)), "l"(src), "r"(live ? 16 : 0) : "memory");
-}
-// two fp32 values as three packed bf16 terms each: x = t0 + t1 + t2 up to 2^-24 of x (each rest is exact)
-__device__ __forceinline__ void split3(float x, float y, uint32_t& t0, uint32_t& t1, uint32_t& t2) {
-  t0 = pack_bf16(x, y);
-  const float x1 = x - bf16lo(t0), y1 = y - bf16hi(t0);
-  t1 = pack_bf16(x1, y1);
-  t2 = pack_bf16(x1 - bf16lo(t1), y1 - bf16hi(t1));
+constexpr int kSgCluster = 4, kSgRows = 256, kSgCols = 64;   // CTAs of a cluster; rows of a segment; value columns
+constexpr int kSgThreads = 512, kSgAll = kSgThreads + 128;   // sixteen warps, and a group of four of which one issues the MMAs
+// registers a thread: 640 threads are launched with 96 each; four warps give what the sixteen others take (16 x 104 + 4 x 64 = 20 x 96)
+constexpr int kSgRegs = 104, kSgRegsMma = 64;
+static_assert(16 * kSgRegs + 4 * kSgRegsMma <= 20 * 96, "registers of the launch");
+constexpr int kSgRegsChunks = 184, kSgRegsGate = 64, kSgRegsRest = 24;   // portions in chunks: eight warps with rows, four of which one has the gates, eight others
+static_assert(8 * kSgRegsChunks + 4 * kSgRegsGate + 8 * kSgRegsRest <= 20 * 96, "registers of the launch");
+static_assert(kSgThreads >= kScanThreads && 2 * kScanCols == kSgCols, "the walk takes a cluster's columns with two of its CTAs");
+constexpr int kSgPanel = kSgRows * 128, kSgTile = 128 * 128;   // bytes of 64 dimensions (columns) of a segment's rows; of 128 rows of them
+// Tensor memory columns: a block's scores on either half of the dimensions; in the first one's place its weights (32 keys: 16 columns of first
+// terms, 16 of second ones) and later Q S_0 of either row tile; third terms; O of the first row tile and of the second one's two key blocks, in the
+// latter's place D's two accumulators before.
+constexpr int kTmHalf = 128, kTmE = 256, kTmO = 320, kTmD = 384;
+
+// 2^x for x <= 0, but for its last rounding to about 2^-26: n = x rounded, 2^f = 1 + f q(f) on |f| <= 1/2 by its Taylor series (terms ln2^k / k!, the
+// first left out 5e-9).  (The argument of an expf would be rounded first: half an ulp of the weight for each unit of it.)
+__device__ __forceinline__ float sg_exp2(double x) {
+  if (x < -120.0) return 0.f;                     // (-inf too; NaN goes on)
+  const double u = x + 6755399441055744.0;        // 1.5 * 2^52: n in the low bits
+  const float f = (float)(x - (u - 6755399441055744.0));
+  float q = 1.52527338e-5f;
+  q = fmaf(q, f, 1.54035304e-4f);
+  q = fmaf(q, f, 1.33335581e-3f);
+  q = fmaf(q, f, 9.61812911e-3f);
+  q = fmaf(q, f, 5.55041087e-2f);
+  q = fmaf(q, f, 2.40226507e-1f);
+  q = fmaf(q, f, 6.93147181e-1f);
+  return fmaf(f, q, 1.0f) * __int_as_float((127 + __double2loint(u)) << 23);
 }
 
-// either of two packed bf16 an infinity or NaN
-__device__ __forceinline__ bool odd2(uint32_t x) { return (x & 0x7f800000u) == 0x7f800000u || (x & 0x7f80u) == 0x7f80u; }
-
-struct GateRows {   // of one chunk
-  double a[kMcRows];       // F_t - m_t
-  double g[kMcRows];       // i_t - F_t
-  float alpha[kMcRows];    // exp(F_t + m_0 - m_t)
-  float em[kMcRows];       // exp(-m_t)
-  float w[kMcRows];        // exp(F_L - F_t + i_t - m_L)
-  float gamma, pad;     // exp(F_L + m_0 - m_L)
+// Staged rows as SWIZZLE_128B has them: panels of 64 dimensions (columns), rows of 128 bytes whose 16-byte pieces are swapped by the row's number.
+__device__ __forceinline__ unsigned char* sg_at(unsigned char* x, int row, int piece) {
+  return x + (piece >> 3) * kSgPanel + row * 128 + (((piece ^ row) & 7) << 4);
+}
+// barriers.  By the MMA warp: scores of a block, D of a half's rows, weights of a block multiplied, the last ones, Q S_0
+// (sixteen warps wait); by those: a half of w V is there, weights of a block are, S_0 is there
+enum { kScores, kD, kPv, kPvLast, kQs, kWeighed, kWeights, kTerms, kBars };
+constexpr double kLog2e = 1.4426950408889634;
+struct SgSmall {
+  double F[kSgRows], M[kSgRows], G[kSgRows];   // sums, running maxima of G, i - F (M and G times log2 e)
+  double gm[8];                                // the largest G of 32 rows
+  double part[2][8], fl[kSgCluster], ml[kSgCluster];   // F and M of the segments' last rows
+  float w[kSgRows], c[kSgRows];                // exp(G - ml), exp(G - gm)
+  float psum[4][kSgRows], qn[2][kSgRows];      // of the weights; q . n_0 on either half of the dimensions
+  float dn[kSgCluster][128], n[128];           // the segments' parts of n; n_0
+  int odd_from[kSgCols], odd;                  // first row whose value in the column is not finite; any
+  uint64_t bar[kBars];
+  uint32_t tmem, mark;
 };
-
 template <int KS>
-struct McSmem {
-  static constexpr int QS = KS * 16 + 8;   // bf16 per staged q / k row
-  __nv_bfloat16 q[2][kMcRows][QS], k[2][kMcRows][QS], v[2][kMcRows][kMcW], w[3][kMcRows][kMcW], s[3][KS * 16][kMcW];
-  float o[kMcRows][kMcW + 2];   // one warp's sums of a row group, for the other
-  GateRows gate[2];
-  int odd[2];   // a value of the chunk is not finite
+struct SgSmem {   // offsets from a 1 024-byte boundary
+  static constexpr int k = 0, q = k + (KS / 4) * kSgPanel, v = q + (KS / 4) * kSgPanel, r = v + kSgPanel;
+  static constexpr int small = r + 3 * kSgTile, bytes = small + (int)sizeof(SgSmall) + 1024;
 };
+static_assert(SgSmem<8>::bytes <= 232448, "shared memory");
 
-// One warp's sums of a chunk (three column tiles of its 16 rows) when a value is not finite: every row adds its own keys one by one, so that nothing
-// is multiplied with a later row's value; what comes from the state before is as in the kernel.
-template <int KS>
-__device__ __noinline__ void mc_careful(const McSmem<KS>& sm, int buf, int hf, int rg, int lane, float qscale, float* out) {
-  const GateRows& gt = sm.gate[buf];
-  const int g = lane >> 2, t4 = lane & 3;
-  float O[3][4] = {}, J[3][4] = {};
-#pragma unroll 1
-  for (int sb = hf * 16; sb <= rg; sb += 32) {
-    float p[2][4] = {};
-#pragma unroll 1
-    for (int k = 0; k < KS; ++k) {
-      uint32_t qk[4], b[4];
-      ldsm4(qk, &sm.q[buf][rg + (lane & 15)][k * 16 + (lane >> 4) * 8]);
-      ldsm4(b, &sm.k[buf][sb + (lane & 7) + ((lane >> 4) << 3)][k * 16 + ((lane >> 3) & 1) * 8]);
-      mma(p[0], qk, b[0], b[1]);
-      mma(p[1], qk, b[2], b[3]);
-    }
-#pragma unroll 1
-    for (int j = 0; j < 16; ++j) {
-      const int from = (lane & ~3) | ((j & 7) >> 1);
-      const __nv_bfloat16* v = &sm.v[buf][sb + j][2 * t4];
-#pragma unroll
-      for (int x = 0; x < 2; ++x) {
-        const int t = rg + g + 8 * x;
-        const float w = __shfl_sync(0xffffffffu, j < 8 ? (j & 1 ? p[0][2 * x + 1] : p[0][2 * x]) : (j & 1 ? p[1][2 * x + 1] : p[1][2 * x]), from) * qscale *
-                        expf((float)(gt.a[t] + gt.g[sb + j]));
-        if (sb + j <= t) {
-#pragma unroll
-          for (int n = 0; n < 3; ++n) {
-            O[n][2 * x] = fmaf(w, __bfloat162float(v[n * 8]), O[n][2 * x]);
-            O[n][2 * x + 1] = fmaf(w, __bfloat162float(v[n * 8 + 1]), O[n][2 * x + 1]);
-          }
-        }
-      }
-    }
-  }
-#pragma unroll 1
-  for (int k = hf * (KS / 2); k < (hf + 1) * (KS / 2); ++k) {
-    uint32_t qk[4];
-    ldsm4(qk, &sm.q[buf][rg + (lane & 15)][k * 16 + (lane >> 4) * 8]);
-#pragma unroll
-    for (int x = 2; x >= 0; --x) {
-      uint32_t b4[4], b2[2];
-      ldsm4t(b4, &sm.s[x][k * 16 + (lane & 15)][(lane >> 4) * 8]);
-      ldsm2t(b2, &sm.s[x][k * 16 + (lane & 15)][kMcCols]);
-      mma(J[0], qk, b4[0], b4[1]);
-      mma(J[1], qk, b4[2], b4[3]);
-      mma(J[2], qk, b2[0], b2[1]);
-    }
-  }
-#pragma unroll
-  for (int n = 0; n < 3; ++n)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) out[n * 4 + i] = fmaf(gt.alpha[rg + g + 8 * (i >> 1)] * qscale, J[n][i], O[n][i]);
+__device__ __forceinline__ void sg_st4(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
 }
+__device__ __forceinline__ void sg_ld8(uint32_t taddr, float* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7])
+               : "r"(taddr));
+}
+__device__ __forceinline__ uint32_t sg_remote(const void* p, uint32_t rank) {
+  uint32_t to;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(smem_u32(p)), "r"(rank));
+  return to;
+}
+__device__ __forceinline__ void sg_put(uint32_t at, float x) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(x) : "memory"); }
+__device__ __forceinline__ void sg_put(uint32_t at, double x) { asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(at), "d"(x) : "memory"); }
+__device__ __forceinline__ void sg_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void sg_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
 // KS: 16-wide steps over the (zero padded) key dimensions
-// CTAS: CTAs that share an SM (two when there are more than SMs: fewer registers each)
-template <int KS, int CTAS>
-__global__ void __launch_bounds__(kMcThreads, CTAS) mlstm_chunk_kernel(const MlstmArgs a) {
+template <int KS>
+__global__ void __launch_bounds__(kSgAll, 1) mlstm_segment_kernel(const MlstmArgs a, uint32_t* status) {
   extern __shared__ __align__(16) unsigned char raw[];
-  McSmem<KS>& sm = *reinterpret_cast<McSmem<KS>*>(raw);
+  using L = SgSmem<KS>;
+  constexpr int PIECES = KS * 2;   // 16-byte pieces of a q or k row
+  unsigned char* smem = raw + (-smem_u32(raw) & 1023);   // (an offset: rounded as an address it would be a generic one, 64 bits and a slower load each time)
+  SgSmall& sm = *reinterpret_cast<SgSmall*>(smem + L::small);
 
   pdl_wait();
   pdl_launch_dependents();
-  const int s = blockIdx.x, h = blockIdx.y, zb = blockIdx.z >> 1, nz = gridDim.z >> 1, jb = blockIdx.z * kMcCols;
-  const bool keeper = (blockIdx.z & 1) == 0;   // stores n and m
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+  const int s = blockIdx.x, h = blockIdx.y, rank = blockIdx.z % kSgCluster, cb = blockIdx.z / kSgCluster, jb = cb * kSgCols;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int heads = a.heads, dim = a.dim, vd = a.vd, nz = (vd + kScanCols - 1) / kScanCols;
   const int start = a.seq_start[s], n_rows = a.seq_start[s + 1] - start;
-  if (n_rows < kChunkFrom) {   // (nothing to do at all among them) the pair's first CTA takes both halves' columns
-    if (keeper && !a.both) mlstm_walk<__nv_bfloat16, KS / 4>(a, reinterpret_cast<float*>(raw), zb, nz);
+  if (n_rows < kChunkFrom) {   // (nothing to do at all among them) two CTAs take the cluster's columns
+    if (rank < 2 && 2 * cb + rank < nz && !a.both && tid < kScanThreads)
+      mlstm_walk<__nv_bfloat16, KS / 4>(a, reinterpret_cast<float*>(raw), 2 * cb + rank, nz);
     return;
   }
-  const int heads = a.heads, dim = a.dim, vd = a.vd;
-  const bool fresh = a.positions[start] == 0;
-  float* slot = a.state + (int64_t)a.seq_slots[s] * a.slot_stride;                                     // S [heads][vd][dim]
-  float* n_st = slot + (int64_t)heads * vd * dim + ((int64_t)h * nz + zb) * dim;                       // n [heads][nz][dim]
-  float* m_st = slot + (int64_t)heads * vd * dim + (int64_t)heads * nz * dim + (int64_t)h * nz + zb;   // m [heads][nz]
-  float* S_st = slot + ((int64_t)h * vd + jb) * dim;
-  const int n_chunks = (n_rows + kMcRows - 1) / kMcRows;
-  const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(a.qkv) + (int64_t)start * a.ld;
-
-  auto fetch = [&](int c) {   // warps 0..7
-    const int b0 = c * kMcRows, buf = c & 1;
-    for (int e = tid; e < kMcRows * KS * 2; e += 256) {
-      const int r = e / (KS * 2), d = (e % (KS * 2)) * 8;
-      const bool live = b0 + r < n_rows && d < dim;
-      const __nv_bfloat16* row = src + (live ? (int64_t)(b0 + r) * a.ld + h * dim + d : 0);
-      cp16z(&sm.q[buf][r][d], row + (live ? a.q_off : 0), live);
-      cp16z(&sm.k[buf][r][d], row + (live ? a.k_off : 0), live);
+  if (n_rows < kSegmentFrom) {   // every CTA sixteen columns
+    if (a.both) return;
+    if (warp < kMcGate) {
+      asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSgRegsChunks));
+      mlstm_chunks<KS, 1>(a, raw, blockIdx.z);
+    } else if (warp < kMcGate + 4) {
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kSgRegsGate));
+      if (warp == kMcGate) mlstm_chunks<KS, 2>(a, raw, blockIdx.z);
+    } else {
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kSgRegsRest));
     }
-    if (tid < kMcRows * 2) {
-      const int r = tid >> 1, c8 = (tid & 1) * 8;
-      const bool live = b0 + r < n_rows && jb + c8 < vd;
-      cp16z(&sm.v[buf][r][c8], src + (live ? (int64_t)(b0 + r) * a.ld + a.v_off + h * vd + jb + c8 : 0), live);
-    }
-  };
-  // state of this warp's 16 dimensions: accumulator fragments of two column tiles and of n (column 16)
-  float S[3][4];
-#pragma unroll
-  for (int n = 0; n < 3; ++n)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int d = warp * 16 + g + (i >> 1) * 8, col = n * 8 + 2 * t4 + (i & 1);
-      S[n][i] = 0.f;
-      if (!fresh && warp < KS && d < dim) {
-        if (n < 2 && jb + col < vd) S[n][i] = S_st[(int64_t)col * dim + d];
-        if (n == 2 && col == kMcCols) S[n][i] = n_st[d];
-      }
-    }
-  auto publish = [&]() {   // the state as three bf16 terms, for everybody's Q S (nobody reads it between a chunk's second barrier and the next one's first)
-    if (warp < KS) {
-#pragma unroll
-      for (int n = 0; n < 3; ++n)
-#pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          uint32_t t[3];
-          split3(S[n][2 * hf], S[n][2 * hf + 1], t[0], t[1], t[2]);
-#pragma unroll
-          for (int x = 0; x < 3; ++x) *reinterpret_cast<uint32_t*>(&sm.s[x][warp * 16 + g + hf * 8][n * 8 + 2 * t4]) = t[x];
-        }
-    }
-  };
-  double m0 = fresh ? 0.0 : (double)*m_st;   // (the gate warp's)
-  asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");   // n and m have been read
-  float ig[2], fg[2];
-  auto fetch_gates = [&](int c) {
-#pragma unroll
-    for (int x = 0; x < 2; ++x) {
-      const int t = c * kMcRows + lane + 32 * x;
-      const bool ok = t < n_rows;
-      const float* p = a.gates + (int64_t)(start + (ok ? t : 0)) * 2 * heads + h;
-      ig[x] = ok ? p[0] : -INFINITY;   // rows past the end: no weight, no decay
-      fg[x] = ok ? p[heads] : 0.f;
-    }
-  };
-  auto gate_chunk = [&](GateRows& o) {
-    double F[2], G[2], M[2];
-#pragma unroll
-    for (int x = 0; x < 2; ++x) {   // inclusive sums (a gate below -1e5 leaves nothing in fp32 either way)
-      F[x] = fg[x] < -1e5f ? -1e5f : fg[x];   // (NaN stays)
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const double v = __shfl_up_sync(0xffffffffu, F[x], d);
-        if (lane >= d) F[x] += v;
-      }
-    }
-    F[1] += __shfl_sync(0xffffffffu, F[0], 31);
-#pragma unroll
-    for (int x = 0; x < 2; ++x) {   // inclusive maxima of i - F
-      G[x] = (double)ig[x] - F[x];
-      M[x] = G[x];
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const double v = __shfl_up_sync(0xffffffffu, M[x], d);
-        if (lane >= d) M[x] = fmax(M[x], v);
-      }
-    }
-    M[1] = fmax(M[1], __shfl_sync(0xffffffffu, M[0], 31));
-    float m[2];
-#pragma unroll
-    for (int x = 0; x < 2; ++x) m[x] = (float)(F[x] + fmax(m0, M[x]));
-    const double FL = __shfl_sync(0xffffffffu, F[1], 31);
-    const double mL = (double)__shfl_sync(0xffffffffu, m[1], 31);
-#pragma unroll
-    for (int x = 0; x < 2; ++x) {
-      const int t = lane + 32 * x;
-      o.a[t] = F[x] - (double)m[x];
-      o.g[t] = G[x];
-      o.alpha[t] = expf((float)(F[x] + m0 - (double)m[x]));
-      o.em[t] = expf(-m[x]);
-      o.w[t] = expf((float)(G[x] + (FL - mL)));
-    }
-    if (lane == 0) o.gamma = expf((float)(FL + m0 - mL));
-    m0 = mL;
-  };
-  // the ones column of v (and zeros beside it), once: the copies leave it alone
-  for (int e = tid; e < 2 * kMcRows * 8; e += kMcThreads) sm.v[e / (kMcRows * 8)][(e / 8) % kMcRows][kMcCols + e % 8] = __float2bfloat16_rn(e % 8 == 0 ? 1.f : 0.f);
-  if (warp < kMcGate) {
-    fetch(0);
-    publish();
-  } else {
-    fetch_gates(0);
-    gate_chunk(sm.gate[0]);
-    fetch_gates(1);
+    return;
   }
-  // the row groups of a scheduler's two warps add up to about the same number of key blocks
-  const int hf = warp >> 2, rg = (hf ? 3 - (warp & 3) : warp & 3) * 16;
-  for (int c = 0; c < n_chunks; ++c) {
-    const int buf = c & 1;
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();   // rows, gates and state of the chunk are there; the chunk before has been finished with
-    const GateRows& gt = sm.gate[buf];
-    if (warp == kMcGate) {
-      // (beside the other warps' products: inside them the same question cost 4 % of the whole)
-      bool odd = false;
+  const Waits mbar_wait(&sm.mark, status);
+  if (tid == 0) {
+    for (int i = 0; i < kBars; ++i) mbar_init(sm.bar + i, i < kWeighed ? 1 : kSgThreads / 32);
+    sm.mark = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == kSgThreads / 32) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem)), "r"(512u));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  fence_before();
+  sg_arrive();   // (the others' shared memory is written to from here on)
+  sg_wait();
+  fence_after();
+  const uint32_t tm = __shfl_sync(0xffffffffu, sm.tmem, 0);
+  uint32_t phases = 0;
+  auto wait = [&](int b) {
+    mbar_wait(sm.bar + b, (phases >> b) & 1);
+    phases ^= 1u << b;
+    fence_after();
+  };
+  // segments of equal length (128 rows at least: a row tile's time does not depend on its rows), rounds of four of them
+  const int rounds = (n_rows - 1) / (kSgCluster * kSgRows) + 1, per_round = (n_rows + rounds - 1) / rounds;
+  const int SL = max(128, (per_round + kSgCluster * 16 - 1) / (kSgCluster * 16) * 16);
+
+  if (warp >= kSgThreads / 32) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kSgRegsMma));
+    if (warp > kSgThreads / 32) return;
+    // ===== MMAs =====
+    const uint32_t one = elect_one() ? 1u : 0u;
+    // descriptors (groups of eight rows 1 024 bytes apart; the next 64 of M or N, where they run along the rows, a panel away) of what starts at an
+    // offset; the address's higher bits, which have the CTA of the cluster, are not theirs
+    const uint32_t desc0 = ((smem_u32(smem) & 0x3ffff) >> 4) + ((kSgPanel >> 4) << 16);
+    auto desc = [&](uint32_t at) { return (uint64_t)(desc0 + (at >> 4)) | ((uint64_t)((1024 >> 4) | (1u << 14) | (2u << 29)) << 32); };
+    constexpr uint32_t kIdS = idesc_bf16(128, 0), kIdO = idesc_bf16(kSgCols, 1), kIdD = kIdO | (1u << 15);   // (K^T: M runs along the rows)
+    auto scores = [&](int tile, int block) {
 #pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        const uint4 v = *reinterpret_cast<const uint4*>(&sm.v[buf][lane + 32 * (x >> 1)][(x & 1) * 8]);
-        odd |= odd2(v.x) || odd2(v.y) || odd2(v.z) || odd2(v.w);
+      for (int j = 0; j < KS; ++j)
+        mma_ss(one, tm + (j < KS / 2 ? 0 : kTmHalf), desc(L::q + (j >> 2) * kSgPanel + tile * kSgTile + (j & 3) * 32),
+               desc(L::k + (j >> 2) * kSgPanel + block * kSgTile + (j & 3) * 32), kIdS, j % (KS / 2) ? 1u : 0u);
+      commit(one, sm.bar + kScores);
+    };
+    const int first = a.positions[start];
+    for (int base = 0; base < n_rows; base += kSgCluster * SL) {
+      const int n16 = (max(0, min(SL, n_rows - base - rank * SL)) + 15) & ~15;
+      const bool two = n16 > 128;
+      sg_arrive();   // (nothing to show: the others do not wait for the last products' issue)
+#pragma unroll 1
+      for (int step = 0; step < (n16 ? two ? 3 : 1 : 0); ++step) {   // the first tile, the second on the first block of keys, on its own
+        if (step < 2) {
+          wait(kWeighed);
+          if (step == 0) scores(0, 0);
+          // D of up to 128 rows, an accumulator for every other 64
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const int steps = (n16 - step * 128 - x * 64) >> 4;
+#pragma unroll
+            for (int i = 2; i >= 0; --i)
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                mma_ss(j < steps ? one : 0u, tm + kTmD + x * 64, desc(L::k + (step * 128 + x * 64 + j * 16) * 128),
+                       desc(L::r + i * kSgTile + (x * 64 + j * 16) * 128), kIdD, step || i < 2 || j ? 1u : 0u);
+          }
+          commit(one, sm.bar + kD);
+        }
+        wait(kWeights);
+        const int steps = (n16 - (step >> 1) * 128) >> 4;
+#pragma unroll
+        for (int i = 2; i >= 0; --i) {
+          const uint32_t weights = tm + (i == 2 ? kTmE : i * 16), next = i == 2 ? 16 : 32;   // 32 keys of a term
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            mma_ts(j < steps ? one : 0u, tm + kTmO + step * 64, weights + (j >> 1) * next + (j & 1) * 8, desc(L::v + ((step >> 1) * 128 + j * 16) * 128), kIdO,
+                   i < 2 || j ? 1u : 0u);
+        }
+        commit(one, sm.bar + (step == (two ? 2 : 0) ? kPvLast : kPv));
+        if (two && step < 2) scores(1, step);
       }
-      odd = __any_sync(0xffffffffu, odd);
-      if (lane == 0) sm.odd[buf] = odd;
-      __syncwarp();
-      asm volatile("bar.arrive 1, 288;" ::: "memory");
-      gate_chunk(sm.gate[buf ^ 1]);
-      fetch_gates(c + 2);
+      sg_wait();
+      sg_arrive();
+      sg_wait();
+      if (n16 && !(first == 0 && base == 0 && rank == 0)) {
+        wait(kTerms);
+#pragma unroll 1
+        for (int tile = 0; tile <= (two ? 1 : 0); ++tile)
+#pragma unroll
+          for (int i = 2; i >= 0; --i)
+#pragma unroll
+            for (int j = 0; j < KS; ++j)
+              mma_ss(one, tm + tile * 64, desc(L::q + (j >> 2) * kSgPanel + tile * kSgTile + (j & 3) * 32), desc(L::r + i * kSgTile + j * 2048), kIdO,
+                     i < 2 || j ? 1u : 0u);
+        commit(one, sm.bar + kQs);
+      }
+    }
+    __syncthreads();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm), "r"(512u));
+    return;
+  }
+
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSgRegs));
+  // ===== sixteen warps: rows, gates, weights, state, outputs =====
+  auto sync = [] { asm volatile("bar.sync 1, 512;" ::: "memory"); };
+  auto arrive = [&](int b) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(sm.bar + b);
+  };
+  const int first = a.positions[start], slot = a.seq_slots[s];
+  // a thread's place in tensor memory: lane 32 quad + lane (a row of a tile, a dimension of the state), sixteen columns from 16 part on
+  const int quad = warp & 3, part = warp >> 2, ml = quad * 32 + lane;
+  const uint32_t tl = tm + ((uint32_t)(quad * 32) << 16);
+  const int width = min(vd - jb, kSgCols), cols = min(width - part * 16, 16);   // columns that exist, of the CTA and the thread (multiples of 8, or none)
+  const bool wide = a.vec_out && width == kSgCols;
+
+  for (int base = 0; base < n_rows; base += kSgCluster * SL) {
+    const int r0 = base + rank * SL, nl = max(0, min(SL, n_rows - r0)), n16 = (nl + 15) & ~15;   // this CTA's rows
+    const int last = (min(kSgCluster * SL, n_rows - base) - 1) / SL;                              // the last CTA with rows
+    const bool two = n16 > 128;
+    if (nl == 0) {
+      sg_arrive();
+      sg_wait();
+      sg_arrive();
+      sg_wait();
       continue;
     }
-    if (c + 1 < n_chunks) fetch(c + 1);
-    for (int e = tid; e < kMcRows * kMcW / 2; e += 256) {   // w v as three terms
-      const int r = e / (kMcW / 2), col = (e % (kMcW / 2)) * 2;
-      const uint32_t v2 = *reinterpret_cast<const uint32_t*>(&sm.v[buf][r][col]);
-      const float w = gt.w[r];
-      uint32_t x[3];
-      split3(w * bf16lo(v2), w * bf16hi(v2), x[0], x[1], x[2]);
-#pragma unroll
-      for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(&sm.w[i][r][col]) = x[i];
+    // ---- rows: k and v of the first 128, of the others, q ----
+    float ig = -INFINITY, fg = 0.f;   // rows past the end: no weight, no decay
+    if (tid < nl) {
+      const float* p = a.gates + (int64_t)(start + r0 + tid) * 2 * heads + h;
+      ig = p[0];
+      fg = p[heads];
     }
-    uint32_t qf[KS][4];
+    if (tid < kSgCols) sm.odd_from[tid] = kSgRows;
+    if (tid == 0) sm.odd = 0;
+    {
+      const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(a.qkv) + (int64_t)(start + r0) * a.ld;
+      const int p = tid % PIECES, r_of = tid / PIECES, pv = tid & 7, rv_of = tid >> 3;
+      const bool live = p * 8 < dim, live_v = jb + pv * 8 < vd;
+      const __nv_bfloat16* row = src + h * dim + (live ? p * 8 : 0);
+      auto fetch = [&](int at, int off, int from, int to) {
+#pragma unroll 4
+        for (int r = from + r_of; r < to; r += kSgThreads / PIECES) {
+          const bool ok = live && r < nl;
+          cp16z(sg_at(smem + at, r, p), row + (ok ? (int64_t)r * a.ld : 0) + off, ok);
+        }
+      };
+      const __nv_bfloat16* row_v = src + a.v_off + h * vd + (live_v ? jb + pv * 8 : 0);
+      auto fetch_v = [&](int from, int to) {
+#pragma unroll 2
+        for (int r = from + rv_of; r < to; r += kSgThreads / 8) {
+          const bool ok = live_v && r < nl;
+          cp16z(sg_at(smem + L::v, r, pv), row_v + (ok ? (int64_t)r * a.ld : 0), ok);
+        }
+      };
+#pragma unroll 1
+      for (int from = 0; from < 256; from += 128) {   // (groups without rows among them)
+        const int to = min(n16, from + 128);
+        fetch_v(from, to);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll 1
+        for (int x = 0; x < 2; ++x) fetch(x ? L::q : L::k, x ? a.q_off : a.k_off, from, to);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      }
+    }
+    // ---- gates: a thread a row ----
+    if (warp < 8) {
+      double F = fg < -1e5f ? -1e5f : fg;   // (a gate below -1e5 leaves nothing in fp32 either way; NaN stays)
 #pragma unroll
-    for (int k = 0; k < KS; ++k) ldsm4(qf[k], &sm.q[buf][rg + (lane & 15)][k * 16 + (lane >> 4) * 8]);
-    float O[3][4] = {}, I[3][3][4] = {};   // within the chunk; from the state before it, one sum per term (short chains)
-    const double a_lo = gt.a[rg + g], a_hi = gt.a[rg + g + 8];
-    for (int sb = hf * 16; sb <= rg; sb += 32) {   // key blocks up to the diagonal
-      float p[2][4] = {};
+      for (int d = 1; d < 32; d <<= 1) {
+        const double v = __shfl_up_sync(0xffffffffu, F, d);
+        if (lane >= d) F += v;
+      }
+      if (lane == 31) sm.part[0][warp] = F;
+      asm volatile("bar.sync 2, 256;" ::: "memory");
+      double before = 0.0;
 #pragma unroll
-      for (int k = 0; k < KS; ++k) {
-        uint32_t b[4];
-        ldsm4(b, &sm.k[buf][sb + (lane & 7) + ((lane >> 4) << 3)][k * 16 + ((lane >> 3) & 1) * 8]);
-        mma(p[0], qf[k], b[0], b[1]);
-        mma(p[1], qf[k], b[2], b[3]);
+      for (int i = 0; i < 7; ++i)
+        if (i < warp) before += sm.part[0][i];
+      F += before;
+      const double G = (double)ig - F;
+      double M = G;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const double v = __shfl_up_sync(0xffffffffu, M, d);
+        if (lane >= d) M = fmax(M, v);
+      }
+      const double own = __shfl_sync(0xffffffffu, M, 31);
+      if (lane == 31) sm.part[1][warp] = M;
+      asm volatile("bar.sync 2, 256;" ::: "memory");
+      double all = sm.part[1][0];
+#pragma unroll
+      for (int i = 1; i < 8; ++i) {
+        if (i <= warp) M = fmax(M, sm.part[1][i - 1]);
+        all = fmax(all, sm.part[1][i]);
+      }
+      sm.F[tid] = F;
+      const double g2 = G * kLog2e, own2 = own * kLog2e;
+      sm.M[tid] = M * kLog2e;
+      sm.G[tid] = g2;
+      sm.w[tid] = all == -INFINITY ? 0.f : sg_exp2(g2 - all * kLog2e);
+      sm.c[tid] = own == -INFINITY ? 0.f : sg_exp2(g2 - own2);
+      if (lane == 31) sm.gm[warp] = own2;
+      if (tid == 255) {
+#pragma unroll
+        for (int i = 0; i < kSgCluster; ++i) {   // (nobody reads them before the cluster has met)
+          sg_put(sg_remote(sm.fl + rank, i), F);
+          sg_put(sg_remote(sm.ml + rank, i), all);
+        }
+      }
+    }
+    // ---- w V in three terms, 128 rows at a time ----
+    auto weigh = [&](int from, int to) {
+      const int p = tid & 7;
+#pragma unroll 2
+      for (int r = from + (tid >> 3); r < to; r += kSgThreads / 8) {
+        uint4* at = reinterpret_cast<uint4*>(sg_at(smem + L::v, r, p));
+        uint4 v = *at;
+        if (odd2(v.x) || odd2(v.y) || odd2(v.z) || odd2(v.w)) {
+          auto clean = [&](uint32_t& x, int col) {
+            if ((x & 0x7f80u) == 0x7f80u) x &= 0xffff0000u, atomicMin(&sm.odd_from[col], r);
+            if ((x & 0x7f800000u) == 0x7f800000u) x &= 0xffffu, atomicMin(&sm.odd_from[col + 1], r);
+          };
+          sm.odd = 1;
+          clean(v.x, p * 8);
+          clean(v.y, p * 8 + 2);
+          clean(v.z, p * 8 + 4);
+          clean(v.w, p * 8 + 6);
+          *at = v;
+        }
+        const float w = sm.w[r];
+        uint4 t[3];
+        split3(w * bf16lo(v.x), w * bf16hi(v.x), t[0].x, t[1].x, t[2].x);
+        split3(w * bf16lo(v.y), w * bf16hi(v.y), t[0].y, t[1].y, t[2].y);
+        split3(w * bf16lo(v.z), w * bf16hi(v.z), t[0].z, t[1].z, t[2].z);
+        split3(w * bf16lo(v.w), w * bf16hi(v.w), t[0].w, t[1].w, t[2].w);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) *reinterpret_cast<uint4*>(sg_at(smem + L::r + i * kSgTile, r - from, p)) = t[i];
+      }
+      fence_async_smem();
+      arrive(kWeighed);
+    };
+    asm volatile("cp.async.wait_group 3;" ::: "memory");
+    sync();   // the first rows' values, and the gates
+    asm volatile("cp.async.wait_group 2;" ::: "memory");   // (k and q too, which the products wait for)
+    // ---- outputs within the segment: a warp the weights of 32 rows (quad) on a quarter (part) of each 32 keys of a block ----
+    // (the sum of the weights decides how large an output becomes, and may be far below its terms: 64 bits)
+    auto weights = [&](int tile, int block, bool wait_e) {
+      const double M = sm.M[tile * 128 + ml], mt = (M == -INFINITY ? 0.0 : M) - a.log2_qscale;   // weights times q's scale
+      float s[4][8];
+      double sum = 0.0;
+#pragma unroll
+      for (int x = 0; x < 4; x += 2) {
+        float s2[2][8];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          sg_ld8(tl + (x + i) * 32 + part * 8, s[x + i]);
+          sg_ld8(tl + kTmHalf + (x + i) * 32 + part * 8, s2[i]);
+        }
+        ld_wait<16>(reinterpret_cast<uint32_t*>(s[x]));
+        ld_wait<16>(reinterpret_cast<uint32_t*>(s2[0]));
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) s[x + i][j] += s2[i][j];
       }
 #pragma unroll
-      for (int n = 0; n < 2; ++n)
+      for (int x = 0; x < 4; ++x) {
+        const int sb = block * 4 + x;   // the keys' group of 32
+        if (tile == block && x >= quad) continue;
+        const double gm = sm.gm[sb];
+        const float w = gm == -INFINITY ? 0.f : sg_exp2(gm - mt);
+#pragma unroll
+        for (int j = 0; j < 8; j += 4) {
+          const float4 c = *reinterpret_cast<const float4*>(sm.c + sb * 32 + part * 8 + j);
+          float* y = s[x] + j;
+          y[0] *= w * c.x, y[1] *= w * c.y, y[2] *= w * c.z, y[3] *= w * c.w;
+          sum += (double)((y[0] + y[1]) + (y[2] + y[3]));
+        }
+      }
+      if (tile == block) {   // (selected, above the diagonal and on it: a later row's key may be anything)
+        float y[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float z = quad == 0 ? s[0][j] : quad == 1 ? s[1][j] : quad == 2 ? s[2][j] : s[3][j];
+          const float w = sg_exp2(sm.G[(block * 4 + quad) * 32 + part * 8 + j] - mt);
+          y[j] = part * 8 + j <= lane ? z * w : 0.f;
+        }
+        sum += (double)((y[0] + y[1]) + (y[2] + y[3])) + (double)((y[4] + y[5]) + (y[6] + y[7]));
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) s[x][j] = x == quad ? y[j] : x > quad ? 0.f : s[x][j];
+      }
+      asm volatile("bar.sync %0, 128;" ::"r"(3 + quad) : "memory");   // the four warps of these rows have their scores: weights take their place
+      if (wait_e) wait(kPv);   // the block before has been multiplied: its third terms' place is free
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        uint32_t t[3][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) split3(s[x][2 * j], s[x][2 * j + 1], t[0][j], t[1][j], t[2][j]);
+        sg_st4(tl + x * 32 + part * 4, t[0]);
+        sg_st4(tl + x * 32 + 16 + part * 4, t[1]);
+        sg_st4(tl + kTmE + x * 16 + part * 4, t[2]);
+      }
+      if (tile == 1 && block == 1) sum += (double)sm.psum[part][128 + ml];
+      sm.psum[part][tile * 128 + ml] = (float)sum;
+      st_wait();
+      fence_before();
+    };
+    // the segment's part of n: a warp eight dimensions, a lane every 32nd row
+    auto part_of_n = [&]() {
+      if (warp >= PIECES) return;
+      float x[8] = {};
+#pragma unroll 2
+      for (int r = lane; r < nl; r += 32) {
+        const uint4 k = *reinterpret_cast<const uint4*>(sg_at(smem + L::k, r, warp));
+        const float w = sm.w[r];
+        const uint32_t y[4] = {k.x, k.y, k.z, k.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const int t = rg + g + (i >> 1) * 8, j = sb + n * 8 + 2 * t4 + (i & 1);
-          // (selected, not weighted with 0: a later row's key may be anything)
-          p[n][i] = j <= t ? p[n][i] * a.qscale * expf((float)(((i >> 1) ? a_hi : a_lo) + gt.g[j])) : 0.f;
-        }
-      uint32_t pa[3][4];
-      split3(p[0][0], p[0][1], pa[0][0], pa[1][0], pa[2][0]);
-      split3(p[0][2], p[0][3], pa[0][1], pa[1][1], pa[2][1]);
-      split3(p[1][0], p[1][1], pa[0][2], pa[1][2], pa[2][2]);
-      split3(p[1][2], p[1][3], pa[0][3], pa[1][3], pa[2][3]);
-      uint32_t v4[4], v2[2];
-      ldsm4t(v4, &sm.v[buf][sb + (lane & 15)][(lane >> 4) * 8]);
-      ldsm2t(v2, &sm.v[buf][sb + (lane & 15)][kMcCols]);
-#pragma unroll
-      for (int x = 2; x >= 0; --x) {
-        mma(O[0], pa[x], v4[0], v4[1]);
-        mma(O[1], pa[x], v4[2], v4[3]);
-        mma(O[2], pa[x], v2[0], v2[1]);
-      }
-    }
-#pragma unroll
-    for (int kk = 0; kk < KS / 2; ++kk) {
-      uint32_t qk[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) qk[i] = hf ? qf[KS / 2 + kk][i] : qf[kk][i];
-      const int k = hf * (KS / 2) + kk;
-#pragma unroll
-      for (int x = 2; x >= 0; --x) {
-        uint32_t b4[4], b2[2];
-        ldsm4t(b4, &sm.s[x][k * 16 + (lane & 15)][(lane >> 4) * 8]);
-        ldsm2t(b2, &sm.s[x][k * 16 + (lane & 15)][kMcCols]);
-        mma(I[x][0], qk, b4[0], b4[1]);
-        mma(I[x][1], qk, b4[2], b4[3]);
-        mma(I[x][2], qk, b2[0], b2[1]);
-      }
-    }
-    const float al[2] = {gt.alpha[rg + g] * a.qscale, gt.alpha[rg + g + 8] * a.qscale};
-#pragma unroll
-    for (int n = 0; n < 3; ++n)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) O[n][i] = fmaf(al[i >> 1], (I[2][n][i] + I[1][n][i]) + I[0][n][i], O[n][i]);
-    if (hf) {
-#pragma unroll
-      for (int n = 0; n < 3; ++n)
-#pragma unroll
-        for (int x = 0; x < 2; ++x) *reinterpret_cast<float2*>(&sm.o[rg + g + 8 * x][n * 8 + 2 * t4]) = make_float2(O[n][2 * x], O[n][2 * x + 1]);
-    }
-    asm volatile("bar.sync 1, 288;" ::: "memory");   // w v is complete, the other warps' sums and the gate warp's look at the values are there
-    const int odd = sm.odd[buf];
-    if (warp < KS) {
-      float U[3][3][4] = {};
-#pragma unroll
-      for (int k = 0; k < kMcRows / 16; ++k) {
-        uint32_t ka[4];
-        ldsm4t(ka, &sm.k[buf][k * 16 + (lane & 7) + ((lane >> 4) << 3)][warp * 16 + ((lane >> 3) & 1) * 8]);
-#pragma unroll
-        for (int x = 2; x >= 0; --x) {
-          uint32_t b4[4], b2[2];
-          ldsm4t(b4, &sm.w[x][k * 16 + (lane & 15)][(lane >> 4) * 8]);
-          ldsm2t(b2, &sm.w[x][k * 16 + (lane & 15)][kMcCols]);
-          mma(U[x][0], ka, b4[0], b4[1]);
-          mma(U[x][1], ka, b4[2], b4[3]);
-          mma(U[x][2], ka, b2[0], b2[1]);
+          x[2 * i] = fmaf(w, bf16lo(y[i]), x[2 * i]);
+          x[2 * i + 1] = fmaf(w, bf16hi(y[i]), x[2 * i + 1]);
         }
       }
-      const float gamma = gt.gamma;
 #pragma unroll
-      for (int n = 0; n < 3; ++n)
+      for (int half = 4; half >= 1; half >>= 1) {   // the lane keeps one half of what it holds
+        const bool up = (lane & half) != 0;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) S[n][i] = fmaf(gamma, S[n][i], (U[2][n][i] + U[1][n][i]) + U[0][n][i]);
-    }
-    if (odd) {
-      // in the blocks on the diagonal the products of such a value with the zeros above it reached earlier rows: the sums once more, with care
-      float o[12];
-      mc_careful(sm, buf, hf, rg, lane, a.qscale, o);
-#pragma unroll
-      for (int n = 0; n < 3; ++n)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) O[n][i] = o[n * 4 + i];
-      if (hf) {
-#pragma unroll
-        for (int n = 0; n < 3; ++n)
-#pragma unroll
-          for (int x = 0; x < 2; ++x) *reinterpret_cast<float2*>(&sm.o[rg + g + 8 * x][n * 8 + 2 * t4]) = make_float2(O[n][2 * x], O[n][2 * x + 1]);
-      }
-      asm volatile("bar.sync 2, 256;" ::: "memory");
-    }
-    publish();
-    if (!hf) {
-#pragma unroll
-      for (int x = 0; x < 2; ++x) {
-        const int t = rg + g + 8 * x, row = c * kMcRows + t;
-        float o[3][2];
-#pragma unroll
-        for (int n = 0; n < 3; ++n) {
-          const float2 y = *reinterpret_cast<const float2*>(&sm.o[t][n * 8 + 2 * t4]);
-          o[n][0] = O[n][2 * x] + y.x;
-          o[n][1] = O[n][2 * x + 1] + y.y;
-        }
-        const float nq = __shfl_sync(0xffffffffu, o[2][0], lane & ~3);   // column 16 sits with the first lane of four
-        const float den = fmaxf(fabsf(nq), gt.em[t]) + 1e-6f;
-        if (row < n_rows) {
-          float* dst = a.out + ((int64_t)(start + row) * heads + h) * vd + jb;
-#pragma unroll
-          for (int n = 0; n < 2; ++n)
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-              const int col = n * 8 + 2 * t4 + i;
-              if (jb + col < vd) dst[col] = o[n][i] / den;
-            }
+        for (int i = 0; i < half; ++i) {
+          const float keep = up ? x[i + half] : x[i], give = up ? x[i] : x[i + half];
+          x[i] = keep + __shfl_xor_sync(0xffffffffu, give, half);
         }
       }
+      x[0] += __shfl_xor_sync(0xffffffffu, x[0], 8);
+      x[0] += __shfl_xor_sync(0xffffffffu, x[0], 16);
+      if (lane < 8) {
+#pragma unroll
+        for (int i = 0; i < kSgCluster; ++i) sg_put(sg_remote(&sm.dn[rank][warp * 8 + lane], i), x[0]);
+      }
+    };
+    float4* X = reinterpret_cast<float4*>(smem + L::r);
+    float* scratch = a.out + ((int64_t)(start + base) * heads + h) * vd + jb;   // of the round's first segment
+    const int64_t segment = (int64_t)SL * heads * vd;
+    auto place = [&](int j) { return (int64_t)(j * 32 + (tid >> 4)) * heads * vd + (tid & 15) * 4; };
+#pragma unroll 1
+    for (int step = 0; step < (two ? 3 : 1); ++step) {
+      if (step < 2) {
+        if (step) wait(kD);
+        weigh(step * 128, min(n16, step * 128 + 128));
+      }
+      wait(kScores);
+      weights(step ? 1 : 0, step >> 1, step > 0);
+      if (step != 1) arrive(kWeights);
+      if (step == 0) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        sync();   // all rows
+        part_of_n();
+      }
+      if (step == (two ? 1 : 0)) {
+        wait(kD);
+        float D[16];
+        {
+          uint32_t y[2][16];
+          ld16(tl + kTmD + part * 16, y[0]);
+          ld16(tl + kTmD + 64 + part * 16, y[1]);
+          ld_wait<32>(y[0]);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) D[j] = n16 > 64 ? __uint_as_float(y[0][j]) + __uint_as_float(y[1][j]) : __uint_as_float(y[0][j]);
+        }
+        fence_before();
+        if (step == 1) arrive(kWeights);   // (the products go where D was)
+        if (sm.odd) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (sm.odd_from[part * 16 + j] < kSgRows) D[j] = NAN;
+        }
+        // D: kept in shared memory and, for the segments behind, where this segment's first outputs will be (all 128 rows are there then; a cluster's
+        // shared memory is read at 8 bytes a cycle, L2 at 30).  A thread's four values side by side, or (fewer columns) where they would be as outputs
+        if (rank == last) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) X[j * kSgThreads + tid] = make_float4(D[4 * j], D[4 * j + 1], D[4 * j + 2], D[4 * j + 3]);
+        } else if (wide) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            *reinterpret_cast<float4*>(scratch + rank * segment + place(j)) = make_float4(D[4 * j], D[4 * j + 1], D[4 * j + 2], D[4 * j + 3]);
+        } else if (ml < dim) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (j < cols) scratch[rank * segment + (int64_t)ml * heads * vd + part * 16 + j] = D[j];
+        }
+        sg_arrive();   // D is there, and (from the second round on) the state that the round before left in the slot
+      }
     }
+    sg_wait();
+    const auto S_at = [&] { return a.state + (int64_t)slot * a.slot_stride; };                                    // S [heads][vd][dim]
+    const auto n_st = [&] { return S_at() + (int64_t)heads * vd * dim + ((int64_t)h * nz + 2 * cb) * dim; };      // n [heads][nz][dim]
+    const auto m_st = [&] { return S_at() + (int64_t)heads * (vd + nz) * dim + (int64_t)h * nz + 2 * cb; };       // m [heads][nz]
+    const auto S_st = [&] { return S_at() + ((int64_t)h * vd + jb + part * 16) * dim + ml; };
+    const bool empty = first == 0 && base == 0, zero = empty && rank == 0;   // S_0 is zeros
+    // ---- S_0, n_0, m_0: the state before the round, then segment after segment ----
+    double m0 = empty ? 0.0 : (double)__ldcg(m_st());
+    float S[16], n0 = 0.f;
+    if (empty) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) S[j] = 0.f;
+    } else {
+      if (tid < dim) n0 = __ldcg(n_st() + tid);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) S[j] = ml < dim && j < cols ? __ldcg(S_st() + (int64_t)j * dim) : 0.f;
+    }
+    {
+      float4 x[4];
+      auto get = [&](int i, float4 (&x)[4]) {
+        if (wide) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) x[j] = __ldcg(reinterpret_cast<const float4*>(scratch + i * segment + place(j)));
+        } else {
+          float y[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) y[j] = ml < dim && j < cols ? __ldcg(scratch + i * segment + (int64_t)ml * heads * vd + part * 16 + j) : 0.f;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) x[j] = make_float4(y[4 * j], y[4 * j + 1], y[4 * j + 2], y[4 * j + 3]);
+        }
+      };
+#pragma unroll 1
+      for (int i = 0; i < rank; ++i) {
+        get(i, x);
+        const double fl = sm.fl[i], gl = sm.ml[i], m1 = (double)(float)(fl + fmax(m0, gl));
+        const float gamma = expf((float)(fl + m0 - m1)), beta = expf((float)(fl + gl - m1));
+        m0 = m1;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          S[4 * j] = fmaf(gamma, S[4 * j], beta * x[j].x);
+          S[4 * j + 1] = fmaf(gamma, S[4 * j + 1], beta * x[j].y);
+          S[4 * j + 2] = fmaf(gamma, S[4 * j + 2], beta * x[j].z);
+          S[4 * j + 3] = fmaf(gamma, S[4 * j + 3], beta * x[j].w);
+        }
+        if (tid < dim) n0 = fmaf(gamma, n0, beta * sm.dn[i][tid]);
+      }
+    }
+    if (tid < KS * 16) sm.n[tid] = n0;
+    sg_arrive();
+    float D[16];
+    if (rank == last) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float4 x = X[j * kSgThreads + tid];
+        D[4 * j] = x.x, D[4 * j + 1] = x.y, D[4 * j + 2] = x.z, D[4 * j + 3] = x.w;
+      }
+      sync();   // X has been read
+    }
+    if (!zero) {   // S_0 in three terms, rows of dimensions
+      if (ml < KS * 16) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          uint4 t[3];
+          split3(S[8 * j], S[8 * j + 1], t[0].x, t[1].x, t[2].x);
+          split3(S[8 * j + 2], S[8 * j + 3], t[0].y, t[1].y, t[2].y);
+          split3(S[8 * j + 4], S[8 * j + 5], t[0].z, t[1].z, t[2].z);
+          split3(S[8 * j + 6], S[8 * j + 7], t[0].w, t[1].w, t[2].w);
+#pragma unroll
+          for (int i = 0; i < 3; ++i) *reinterpret_cast<uint4*>(sg_at(smem + L::r + i * kSgTile, ml, part * 2 + j)) = t[i];
+        }
+      }
+      fence_async_smem();
+      arrive(kTerms);
+    }
+    sg_wait();   // everybody has read the slot and the others' parts
+    if (rank == last) {
+      const double m1 = (double)(float)(sm.fl[rank] + fmax(m0, sm.ml[rank]));
+      const float gamma = expf((float)(sm.fl[rank] + m0 - m1)), beta = expf((float)(sm.fl[rank] + sm.ml[rank] - m1));
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (ml < dim && j < cols) S_st()[(int64_t)j * dim] = fmaf(gamma, S[j], beta * D[j]);
+      for (int i = 0; i < min(2, nz - 2 * cb); ++i) {   // the copies of n and m beside these columns
+        if (tid < dim) n_st()[(int64_t)i * dim + tid] = fmaf(gamma, n0, beta * sm.dn[rank][tid]);
+        if (tid == 0) m_st()[i] = (float)m1;
+      }
+    }
+    if (!zero) {   // q . n_0: two threads a row
+      sync();      // (n_0)
+      const int r = tid & 255, half = tid >> 8;
+      if (r < nl) {
+        float x[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int i = 0; i < KS; ++i) {
+          const int p = half * KS + i;
+          const uint4 q = *reinterpret_cast<const uint4*>(sg_at(smem + L::q, r, p));
+          const float4 n_lo = *reinterpret_cast<const float4*>(sm.n + p * 8), n_hi = *reinterpret_cast<const float4*>(sm.n + p * 8 + 4);
+          x[0] = fmaf(bf16lo(q.x), n_lo.x, x[0]);
+          x[1] = fmaf(bf16hi(q.x), n_lo.y, x[1]);
+          x[2] = fmaf(bf16lo(q.y), n_lo.z, x[2]);
+          x[3] = fmaf(bf16hi(q.y), n_lo.w, x[3]);
+          x[0] = fmaf(bf16lo(q.z), n_hi.x, x[0]);
+          x[1] = fmaf(bf16hi(q.z), n_hi.y, x[1]);
+          x[2] = fmaf(bf16lo(q.w), n_hi.z, x[2]);
+          x[3] = fmaf(bf16hi(q.w), n_hi.w, x[3]);
+        }
+        sm.qn[half][r] = (x[0] + x[1]) + (x[2] + x[3]);
+      }
+    }
+    wait(kPvLast);
+    if (!zero) wait(kQs);
+    sync();   // sums of the weights, q . n_0
+    // ---- outputs, by way of shared memory (k and q are done with): a row's 256 bytes leave together ----
+    float4* stage = reinterpret_cast<float4*>(smem + L::k);
+#pragma unroll 1
+    for (int tile = 0; tile <= (two ? 1 : 0); ++tile) {
+      const int t = tile * 128 + ml;
+      uint32_t o[16], o1[16], qs[16];
+      ld16(tl + kTmO + tile * 64 + part * 16, o);
+      ld16(tl + kTmO + 128 + part * 16, o1);
+      ld16(tl + tile * 64 + part * 16, qs);
+      const double F = sm.F[t], M = sm.M[t] * 0.6931471805599453, m = (double)(float)(F + fmax(m0, M));
+      const float in = M == -INFINITY ? 0.f : expf((float)(F + M - m)), ahead = zero ? 0.f : expf((float)(F + m0 - m)) * a.qscale;
+      float nq = in * ((sm.psum[0][t] + sm.psum[1][t]) + (sm.psum[2][t] + sm.psum[3][t]));
+      if (!zero) nq = fmaf(ahead, sm.qn[0][t] + sm.qn[1][t], nq);
+      const float den = fmaxf(fabsf(nq), expf(-(float)m)) + 1e-6f;
+      ld_wait<16>(o);
+      ld_wait<16>(o1);
+      ld_wait<16>(qs);
+      // x / den by the reciprocal and one step of Newton's (rounded as the division is, but for its last bit at most)
+      const float inv = 1.0f / den;
+      float y[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        float x = tile ? __uint_as_float(o[j]) + __uint_as_float(o1[j]) : __uint_as_float(o[j]);
+        x = zero ? in * x : fmaf(in, x, ahead * __uint_as_float(qs[j]));
+        const float z = x * inv, rest = fmaf(-z, den, x);
+        y[j] = rest == rest ? fmaf(rest, inv, z) : z;
+      }
+      if (sm.odd) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (t >= sm.odd_from[part * 16 + j]) y[j] = NAN;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) stage[t * 16 + ((part * 4 + j) ^ (t & 7))] = make_float4(y[4 * j], y[4 * j + 1], y[4 * j + 2], y[4 * j + 3]);
+    }
+    fence_before();
+    sync();
+    float* dst = a.out + ((int64_t)(start + r0) * heads + h) * vd + jb;
+#pragma unroll 1
+    for (int e = tid; e < nl * 16; e += kSgThreads) {
+      const int r = e >> 4, c = e & 15;
+      const float4 y = stage[r * 16 + (c ^ (r & 7))];
+      float* to = dst + (int64_t)r * heads * vd + c * 4;
+      if (wide) {
+        *reinterpret_cast<float4*>(to) = y;
+      } else if (c * 4 < width) {   // (a multiple of 8)
+        to[0] = y.x, to[1] = y.y, to[2] = y.z, to[3] = y.w;
+      }
+    }
+    sync();   // rows, tensor memory and sums have been read
   }
-  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
-  if (warp < KS) {
-#pragma unroll
-    for (int n = 0; n < 3; ++n)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int d = warp * 16 + g + (i >> 1) * 8, col = n * 8 + 2 * t4 + (i & 1);
-        if (d >= dim) continue;
-        if (n < 2 && jb + col < vd) S_st[(int64_t)col * dim + d] = S[n][i];
-        if (n == 2 && col == kMcCols && keeper) n_st[d] = S[n][i];
-      }
-  } else if (warp == kMcGate && keeper && lane == 0) {
-    *m_st = (float)m0;   // (chunks past the last row leave it alone)
-  }
+  __syncthreads();
+}
+
+// Chunks on their own, for steps whose portions take a kernel each: two CTAs share an SM where there are more of them than SMs.
+template <int KS, int CTAS>
+__global__ void __launch_bounds__(kMcThreads, CTAS) mlstm_chunk_kernel(const MlstmArgs a) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  pdl_wait();
+  pdl_launch_dependents();
+  const int n_rows = a.seq_start[blockIdx.x + 1] - a.seq_start[blockIdx.x];
+  if (n_rows >= kChunkFrom && n_rows < kSegmentFrom) mlstm_chunks<KS, 0>(a, raw, blockIdx.z);
 }
 
 }  // namespace
@@ -447,25 +719,28 @@ bool mlstm_chunk_supported(const MlstmArgs& a) {
   return a.dim > 0 && a.dim <= 128 && a.dim % 8 == 0 && a.vd % 8 == 0 && a.ld % 8 == 0 && (a.q_off | a.k_off | a.v_off) % 8 == 0 &&
          reinterpret_cast<uintptr_t>(a.qkv) % 16 == 0;
 }
+// CTAs of a launch
+int64_t mlstm_chunk_ctas(const MlstmArgs& a, int S) { return (int64_t)S * a.heads * kSgCluster * ((a.vd + kSgCols - 1) / kSgCols); }
 
-int mlstm_chunk(const MlstmArgs& a, int S, cudaStream_t s) {
-  const dim3 grid(S, a.heads, 2 * mlstm_col_blocks(a.vd)), block(kMcThreads), cluster(1, 1, 2);
-#define CHUNK(K, C)                                                                                       \
-  do {                                                                                                    \
-    static bool done[64] = {};                                                                            \
-    constexpr size_t smem = std::max(sizeof(McSmem<K>), (size_t)ml_floats(K / 4) * 4);   /* chunks; walk */    \
-    B200_CUDA(ensure_dynamic_smem(mlstm_chunk_kernel<K, C>, (int)smem, done));                            \
-    B200_CUDA(launch_cluster(mlstm_chunk_kernel<K, C>, grid, block, smem, s, cluster, a));                \
+int mlstm_chunk(MlstmArgs a, int S, cudaStream_t s) {
+  if (const int e = wait_status()) return e;
+  a.vec_out = reinterpret_cast<uintptr_t>(a.out) % 16 == 0;
+  const dim3 grid(S, a.heads, kSgCluster * ((a.vd + kSgCols - 1) / kSgCols)), block(kSgAll), cluster(1, 1, kSgCluster);
+#define SEGMENTS(K)                                                                                            \
+  do {                                                                                                         \
+    static bool done[2][64] = {};                                                                              \
+    constexpr size_t smem = std::max({(size_t)SgSmem<K>::bytes, sizeof(McSmem<K>), (size_t)ml_floats(K / 4) * 4});   \
+    if (a.both) {                                                                                              \
+      B200_CUDA(ensure_dynamic_smem(mlstm_chunk_kernel<K, 2>, (int)sizeof(McSmem<K>), done[1]));               \
+      B200_CUDA(launch_cluster(mlstm_chunk_kernel<K, 2>, dim3(S, a.heads, 2 * mlstm_col_blocks(a.vd)), dim3(kMcThreads), sizeof(McSmem<K>), s, dim3(1, 1, 2), a));   \
+    }                                                                                                          \
+    const PdlScope after_chunks(a.both);                                                                       \
+    B200_CUDA(ensure_dynamic_smem(mlstm_segment_kernel<K>, (int)smem, done[0]));                               \
+    B200_CUDA(launch_cluster(mlstm_segment_kernel<K>, grid, block, smem, s, cluster, a, wait_status_word()));  \
   } while (0)
-  const bool many = (int64_t)grid.x * grid.y * grid.z > kNumSMs;
-  if (a.dim <= 64) {
-    if (many) CHUNK(4, 2);
-    else CHUNK(4, 1);
-  } else {
-    if (many) CHUNK(8, 2);
-    else CHUNK(8, 1);
-  }
-#undef CHUNK
+  if (a.dim <= 64) SEGMENTS(4);
+  else SEGMENTS(8);
+#undef SEGMENTS
   return B200_OK;
 }
 

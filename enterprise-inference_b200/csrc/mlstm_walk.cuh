@@ -1,4 +1,4 @@
-// The row-by-row walk of the matrix-memory recurrence (mlstm.cu), which the chunk kernel (mlstm_chunk.cu) can take for short portions too.
+// The row-by-row walk of the matrix-memory recurrence (mlstm.cu), which the segments' kernel (mlstm_chunk.cu) can take for short portions too.
 #pragma once
 #include "common.cuh"
 #include "f32x2.cuh"
@@ -16,14 +16,17 @@ struct MlstmArgs {
   int64_t ld, slot_stride;
   int q_off, k_off, v_off, heads, dim, vd;
   float qscale;
+  double log2_qscale;
   int vec;        // rows of q and k can be read 16 bytes at a time
   int vec_state;  // state columns 8 bytes at a time
-  int both;       // the walk's and the chunks' kernel are both launched, each for its portions
+  int vec_out;    // outputs 16 bytes at a time
+  int both;       // the walk's, the chunks' and the segments' kernel are all launched, each for its portions
 };
 
-// bf16 rows in chunks of 64 on the tensor cores (mlstm_chunk.cu)
+// bf16 rows on the tensor cores (mlstm_chunk.cu)
 bool mlstm_chunk_supported(const MlstmArgs& a);
-int mlstm_chunk(const MlstmArgs& a, int S, cudaStream_t s);
+int64_t mlstm_chunk_ctas(const MlstmArgs& a, int S);
+int mlstm_chunk(MlstmArgs a, int S, cudaStream_t s);
 
 namespace {
 
@@ -44,6 +47,7 @@ constexpr int kScanCols = 32;                    // value columns of a CTA, whic
 constexpr int kScanStage = 16;                   // rows staged in shared memory at a time
 constexpr int kScanThreads = 288, kNWarp = 8;
 constexpr int kChunkFrom = 97;                   // rows of a portion from which chunks pay (97 rows of one sequence: 15 us, walked 23)
+constexpr int kSegmentFrom = 193;                // rows of a portion from which segments pay (256 rows of one sequence 20.0 us, in chunks 22.3; 192 in chunks 17.9)
 constexpr int kPartRow = 132;                    // floats of a row of read-out sums: 32 lanes x 4 columns, rows 16 bytes apart in the banks
 
 // which of its accesses the walk can make wide

@@ -93,12 +93,12 @@ def test_mlstm_scan_portions_and_hard_gates(f32, heads, dim, vdim, pad):
 @pytest.mark.parametrize("what", ["value", "key", "forget gate", "input gate"])
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
 @pytest.mark.parametrize("row", [0, 37, 100])
-def test_mlstm_chunks_are_causal_for_what_is_not_finite(what, bad, row):
+def test_mlstm_chunks_are_causal_for_what_is_not_finite(what, bad, row, T=130):
     """An infinity or NaN of one row reaches that row and the later ones (a value's its own column, anything else's its head), and no earlier row."""
     if "gate" in what and bad == float("inf"):
         bad = float("nan")
     lib, check = pkg("_abi").lib(), pkg("_abi").check
-    heads, dim, vdim, T, col = 2, 64, 64, 130, 21
+    heads, dim, vdim, col = 2, 64, 64, 21
     g = torch.Generator().manual_seed(5)
     hd, hv = heads * dim, heads * vdim
     floats, ld = int(lib.b200_mlstm_state_floats(heads, dim, vdim)), 2 * hd + hv
@@ -132,6 +132,51 @@ def test_mlstm_chunks_are_causal_for_what_is_not_finite(what, bad, row):
     else:
         assert not torch.isfinite(st[1, :, 9]).any()
     assert (st[0] - S[0]).norm() < 1e-5 * S[0].norm()
+
+
+# Segments of a cluster: the border to the chunks (192 rows), two segments with one row in the second's last tile, both tiles of a segment (513 rows), whole
+# rounds and one row more; then a step that starts from what the first one left.  vdim 96: a column block of 32, 40: of 40; `off` floats: outputs that
+# do not start at 16-byte addresses.
+@pytest.mark.parametrize("rows", [192, 193, 257, 513, 1024, 1025])
+@pytest.mark.parametrize("heads,dim,vdim,off", [(2, 128, 64, 0), (1, 128, 96, 0), (1, 40, 40, 1), (2, 64, 64, 0)])
+def test_mlstm_segments(rows, heads, dim, vdim, off):
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    g = torch.Generator().manual_seed(rows + dim + vdim)
+    hd, hv, nz = heads * dim, heads * vdim, (vdim + 31) // 32
+    floats, ld = int(lib.b200_mlstm_state_floats(heads, dim, vdim)), 2 * hd + hv
+    state = torch.full((2, floats), 7.5, device=DEV)
+    oracle = tuple(torch.zeros(s, dtype=torch.float64) for s in ((heads, vdim, dim), (heads, dim), (heads,)))
+    at = 0
+    for T in (rows, 260):
+        x = torch.randn(T, ld, generator=g).to(torch.bfloat16)
+        gates = torch.randn(T, 2 * heads, generator=g) * 1.5
+        gates[:, heads:] = torch.nn.functional.logsigmoid(gates[:, heads:] + 3)
+        gates[T // 2, heads:] = -14.9      # all but forgotten
+        gates[T // 2 + 9, :heads] = 9.0    # a row that dwarfs what is there
+        buf = torch.full((T * hv + off,), float("nan"), device=DEV)
+        out = buf[off:].view(T, hv)
+        xd, gd, ptd, std, sld = x.to(DEV), gates.to(DEV), _i32(list(range(at, at + T))), _i32([0, T]), _i32([1])
+        check(lib.b200_mlstm_scan(0, xd.data_ptr(), ld, 0, hd, 2 * hd, gd.data_ptr(), ptd.data_ptr(), std.data_ptr(), sld.data_ptr(), state.data_ptr(),
+                                  floats, out.data_ptr(), 1, heads, dim, vdim, None))
+        torch.cuda.synchronize()
+        want, span, oracle = _mlstm(x.double(), gates.double(), oracle, heads, dim, vdim)
+        got, tol = out.double().cpu(), 1e-5     # (as above)
+        assert ((got - want).abs() <= tol * span + 1e-7 * want.abs()).all(), (T, float(((got - want).abs() / span).max()))
+        st = state[1].double().cpu()
+        assert (st[:hv * dim].reshape(heads, vdim, dim) - oracle[0]).norm() < tol * oracle[0].norm()
+        n = st[hv * dim:hv * dim + heads * nz * dim].reshape(heads, nz, dim)
+        assert (n - oracle[1][:, None]).norm() < tol * nz ** 0.5 * oracle[1].norm()
+        assert (st[hv * dim + heads * nz * dim:].reshape(heads, nz) - oracle[2][:, None]).abs().max() < 1e-5
+        at += T
+    assert (state[0] == 7.5).all()
+
+
+@pytest.mark.parametrize("what", ["value", "key", "forget gate", "input gate"])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("row", [0, 127, 200, 540])
+def test_mlstm_segments_are_causal_for_what_is_not_finite(what, bad, row):
+    """600 rows: segments of 160, with a second row tile; otherwise as the chunks' test."""
+    test_mlstm_chunks_are_causal_for_what_is_not_finite(what, bad, row, T=600)
 
 
 # Steps whose CTAs outnumber the SMs: two sequences of 8 heads of 256 columns (256 CTAs, two to an SM, short portions walked beside the chunks),
