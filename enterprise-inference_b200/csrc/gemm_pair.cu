@@ -19,6 +19,7 @@
 // 128 tokens and fewer stay on gemm_tc.cu's tiles: their launches stream W, and 148 CTAs with two of them to an SM keep more of it in flight
 // (64 tokens, 4096, 28672: 42 there, 49 here; 128, 14336, 4096: 33 and 34).
 #include <algorithm>
+#include <type_traits>
 
 #include "gemm_epilogue.cuh"
 #include "pair_drain.h"
@@ -306,13 +307,19 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       const int m_tile = 2 * tile.m + rank;
       const int n_rows = p.pair_tile ? tile.n : min(tile.n, p.T - tile.row0);
       const bool live = (p.gu_ff ? m_tile * (kBlockM / 2) < p.gu_ff : m_tile * kBlockM < p.n_out) && !wait.marked();
-      float bb[4];
+      float bb[4], gate_bias[4], up_bias[4];
       pair_bias(p, m_tile, r4, bb);
+      if constexpr (MODE == kSiluMul) {   // of the features that the lane finishes
+        pair_bias(p, m_tile, (quad & 1) * 32 + (lane & 7) * 4, gate_bias);
+        pair_bias(p, m_tile, 64 + (quad & 1) * 32 + (lane & 7) * 4, up_bias);
+      }
       // A whole slab of plain outputs in rows of 16-byte pieces: rounded by the thread that reads them from tensor memory and staged as they are written, 32 tokens in
       // either half of the staging area in turn (one barrier a piece).  A quarter of the instructions that four features at a time take, which is what launches over
       // short k are bound by: 2048 tokens, 4096 features, k 512 24.9 us, so 16.9 (20.8 in tiles of 128 x 256, two CTAs to an SM); k 64 24.9, 18.7 (16.7); 1000 tokens
       // of 8192 features, k 256 23.9, 16.9 (18.7); and 2048 tokens, 28672 features, k 4096 349, 340.
-      const bool straight = MODE == kPlain && p.splits == 1 && p.post_act == 0 && (m_tile + 1) * kBlockM <= p.n_out && p.ldy % 8 == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0;
+      // (squared: the activation of two-matrix experts)
+      const bool squared = MODE == kPlain && p.post_act == 1 + B200_ACT_RELU2;
+      const bool straight = MODE == kPlain && p.splits == 1 && (p.post_act == 0 || squared) && (m_tile + 1) * kBlockM <= p.n_out && p.ldy % 8 == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0;
       const float bias = straight && p.bias ? __bfloat162float(p.bias[m_tile * kBlockM + srow]) : 0.f;
       __nv_bfloat16* const y0 = straight ? p.y + (int64_t)tile.row0 * p.ldy + m_tile * kBlockM + (lane & 15) * 8 : nullptr;
       if (MODE == kRopeKv) {   // a token's cos|sin row is a dependent load: ask for the tile's rows while its MMAs run
@@ -345,11 +352,87 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
           __nv_bfloat16* half = reinterpret_cast<__nv_bfloat16*>(stg) + turn * kPairStgTok * kBlockM;
           turn ^= 1;
 #pragma unroll
-          for (int j = 0; j < 32; ++j) half[j * kBlockM + srow] = __float2bfloat16_rn(__uint_as_float(r[j]) + bias);
+          for (int j = 0; j < 32; ++j) {
+            const float v = __uint_as_float(r[j]) + bias, o = squared ? fmaxf(v, 0.f) * fmaxf(v, 0.f) : v;
+            half[j * kBlockM + srow] = __float2bfloat16_rn(o);
+          }
           asm volatile("bar.sync %0, 128;" ::"r"(barrier) : "memory");
 #pragma unroll
           for (int j = wq * 8 + (lane >> 4); j < wq * 8 + 8; j += 2)   // two tokens a warp and step
             if (live && c + j < n_rows) *reinterpret_cast<uint4*>(y0 + (int64_t)(c + j) * p.ldy) = *reinterpret_cast<const uint4*>(half + j * kBlockM + (lane & 15) * 8);
+          continue;
+        }
+        // Products with an activation and scattered rows: a warp turns its 32 features x 32 tokens in 4 KiB of its own (a token's 16-byte pieces swapped by its number),
+        // eight lanes a token, and every lane's values are worked out side by side, with the stores alone depending on the token.  (Four warps' features together behind two
+        // barriers, token after token with a branch each: 21 000 cycles a tile of gate|up and 12 000 of scattered rows, more than the tile's MMAs take;
+        // 2 048 rows of 32 experts, router and
+        // grouping included, 167 us, so 154; 1 527 rows of 64 without a gate 229, 218.)
+        float4* const own = reinterpret_cast<float4*>(stg_all) + (grp * 4 + quad) * (kPairStgTok * 8);
+        const int tok_of = lane >> 3, piece = lane & 7;
+        if constexpr (MODE == kScatter || MODE == kSiluMul) {
+          float* const cell = reinterpret_cast<float*>(own) + (lane & 3);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) cell[(j * 8 + ((lane >> 2) ^ (j & 7))) * 4] = __uint_as_float(r[j]);
+        }
+        if constexpr (MODE == kScatter) {
+          __syncwarp();
+          const int row = m_tile * kBlockM + quad * 32 + piece * 4;
+          const bool wide = row + 3 < p.n_out && p.n_out % 4 == 0;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int j = 4 * i + tok_of, to = __shfl_sync(0xffffffffu, pair, j);
+            const float w = __shfl_sync(0xffffffffu, wt, j);
+            const float4 a = own[j * 8 + (piece ^ (j & 7))];
+            const float o[4] = {a.x * w, a.y * w, a.z * w, a.w * w};
+            float* dst = p.grp_out + (int64_t)to * p.n_out + row;
+            if (!live || to < 0) continue;   // (rows past the run's end have no destination)
+            if (wide) {
+              *reinterpret_cast<float4*>(dst) = make_float4(o[0], o[1], o[2], o[3]);
+            } else {
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                if (row + e < p.n_out) dst[e] = o[e];
+            }
+          }
+          __syncwarp();
+          continue;
+        }
+        if constexpr (MODE == kSiluMul) {
+          // gate rows with one warp, the matching up rows with another: each finishes half of the tokens
+          const int feat = quad & 1, shared_by = 1 + 2 * grp + feat;
+          asm volatile("bar.sync %0, 64;" ::"r"(shared_by) : "memory");
+          const float4 *gates = reinterpret_cast<const float4*>(stg_all) + (grp * 4 + feat) * (kPairStgTok * 8), *ups = gates + 2 * kPairStgTok * 8;
+          const int f = m_tile * 64 + feat * 32 + piece * 4;
+          const bool wide = p.ldy % 4 == 0 && (reinterpret_cast<uintptr_t>(p.y) & 7) == 0;
+          float o[4][4];
+          auto finish = [&](auto kind) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int j = (quad >> 1) * 16 + 4 * i + tok_of;
+              const float4 ga = gates[j * 8 + (piece ^ (j & 7))], ua = ups[j * 8 + (piece ^ (j & 7))];
+              const float gv[4] = {ga.x, ga.y, ga.z, ga.w}, uv[4] = {ua.x, ua.y, ua.z, ua.w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float g = round_bf16(gv[e] + gate_bias[e]), u = round_bf16(uv[e] + up_bias[e]);
+                o[i][e] = kind == 0 ? silu_to_bf16(g) * u : gate_combine(g, u, kind, p.act_limit);
+              }
+            }
+          };
+          if (p.act == 0) finish(std::integral_constant<int, 0>());   // (the choice outside the loops)
+          else finish(p.act);
+          asm volatile("bar.sync %0, 64;" ::"r"(shared_by) : "memory");
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int t = c + (quad >> 1) * 16 + 4 * i + tok_of;
+            if (!live || t >= n_rows) continue;
+            __nv_bfloat16* dst = p.y + (int64_t)(tile.row0 + t) * p.ldy + f;
+            if (wide) {
+              *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(o[i][0], o[i][1]), pack_bf16(o[i][2], o[i][3]));
+            } else {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) dst[e] = __float2bfloat16_rn(o[i][e]);
+            }
+          }
           continue;
         }
 #pragma unroll
@@ -360,10 +443,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
           for (int j = wq; j < kPairStgTok; j += 4) {
             if (c + j >= n_rows) break;   // warp-uniform
             const float4 a = *reinterpret_cast<const float4*>(stg + j * kBlockM + r4);
-            if constexpr (MODE == kScatter)
-              finalize4<MODE>(p, m_tile, lane, tile.row0 + c + j, a, bb, __shfl_sync(0xffffffffu, pair, j), __shfl_sync(0xffffffffu, wt, j));
-            else
-              finalize4<MODE>(p, m_tile, lane, tile.row0 + c + j, a, bb);
+            finalize4<MODE>(p, m_tile, lane, tile.row0 + c + j, a, bb);
           }
         }
         asm volatile("bar.sync %0, 128;" ::"r"(barrier) : "memory");
