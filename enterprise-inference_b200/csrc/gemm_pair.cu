@@ -5,8 +5,8 @@
 // k for 512 cycles of MMAs, 96 bytes a cycle of the 64 that an SM gets from L2.  A pair shares the token rows: each CTA fetches its own 128
 // weight rows and half of the tokens, 32 KiB for the same 512 cycles.
 //
-// A CTA pair per two SMs, persistent.  Per CTA: warp 0 fetches (TMA, six stages of 32 KiB; both CTAs' bytes complete on the leader's barrier), warp 1
-// of the leader issues the MMAs of both, eight warps turn the accumulator into the launch's output.  The 512 columns of tensor memory hold two
+// A CTA pair per two SMs, persistent.  Per CTA: a warp fetches weights and one token rows (TMA, rings of seven and five times 16 KiB; both CTAs' bytes
+// complete on the leader's barriers), warp 1 of the leader issues the MMAs of both, eight warps turn the accumulator into the launch's output.  The 512 columns of tensor memory hold two
 // accumulators, so a tile's epilogue runs beside the next tile's MMAs; it goes through shared memory of its own, 32 tokens at a time per
 // four warps.  Launches with few tiles share a tile's k between up to four pairs of one cluster, which add up through distributed shared memory.
 //
@@ -29,14 +29,18 @@ namespace b200 {
 
 namespace {
 
-constexpr int kPairThreads = 64 + 256;
-constexpr int kPairStages = 6;
+constexpr int kPairWarps = 11, kPairThreads = kPairWarps * 32;
+// Weights come from HBM, token rows (which other pairs read too) mostly from L2: a ring and a fetching warp for each, the one that waits longer deeper.  Against six
+// stages of both and one warp (us, graph): 383 x 5120 x 7168 34.3 -> 25.1, 700 rows 59.6 -> 47.2, 1500 x 2048 x 8192 43 -> 37.6, 1000 x 4096 x 4096 31 -> 27; 16
+// experts of 1024, width 1024, 2048 rows 93 -> 77.  Rings of 8 and 4 gain as much there, but lose where tokens come late (2000 x 14336 x 4096 157 -> 165, 32
+// experts 155 -> 167); 6 and 6 leave the first group at 30, 56, 43 and 31.
+constexpr int kPairWStages = 7, kPairXStages = 5;
 constexpr int kPairABytes = kBlockM * kBlockK * 2;          // this CTA's weight rows of a stage; the token rows (at most 128) take as much
-constexpr int kPairStageBytes = 2 * kPairABytes;
+constexpr int kPairRings = (kPairWStages + kPairXStages) * kPairABytes;
 constexpr int kPairStgTok = 32;                             // tokens of a staged piece of the epilogue
 constexpr int kPairSplits = 4;                              // shares of k at most: clusters of eight CTAs
 constexpr int kPairStgBytes = kPairStgTok * kBlockM * 4;
-constexpr int kPairSmem = 1024 + kPairStages * kPairStageBytes + 2 * kPairStgBytes + 512;
+constexpr int kPairSmem = 1024 + kPairRings + 2 * kPairStgBytes + 512;
 constexpr uint64_t kKeepNormal = 0x1000000000000000ull, kKeepLast = 0x14F0000000000000ull;
 
 __device__ __forceinline__ uint32_t smem_of(const void* p, int cta) {   // the same shared-memory address in another CTA of the cluster
@@ -46,20 +50,22 @@ __device__ __forceinline__ uint32_t smem_of(const void* p, int cta) {   // the s
 }
 // A wait that runs out marks every CTA of the cluster: each serves another's loads, MMAs or sums.  What follows is out of the loops' way, in
 // functions of its own, and the loops' predicates stay what they were (an MMA predicate that a wait may clear: 187 us instead of 196).
-constexpr uint32_t kPairRunning = 0xffffffffu;   // Waits::mark[1] until the CTA's fetching warp has ended, then the fills it issued
+constexpr uint32_t kPairRunning = 0xffffffffu;   // Waits::mark[1] (weights), [2] (tokens) until the CTA's fetching warp has ended, then the fills it issued
 __device__ __noinline__ void pair_gave_up(uint32_t* mark, uint32_t* status, int ctas) {
   *reinterpret_cast<volatile uint32_t*>(mark) = 1;
   for (int c = 0; c < ctas; ++c) asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(smem_of(mark, c)), "r"(1u) : "memory");
   if (status) *reinterpret_cast<volatile uint32_t*>(status) = 1;
 }
-__device__ __forceinline__ uint32_t pair_issued(uint32_t* mark, int cta) {
+__device__ __forceinline__ uint32_t pair_issued(uint32_t* mark, int ring, int cta) {
   uint32_t v;
-  asm volatile("ld.relaxed.cluster.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(smem_of(mark + 1, cta)) : "memory");
+  asm volatile("ld.relaxed.cluster.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(smem_of(mark + 1 + ring, cta)) : "memory");
   return v;
 }
-// before the MMA warp commits anything for a fill that did not land: both fetching warps have ended (they see the mark), so nothing is issued on it
+// before the MMA warp commits anything for a fill that did not land: all fetching warps have ended (they see the mark), so nothing is issued on it
 __device__ __noinline__ void pair_await_ends(uint32_t* mark, int lead, int limit) {
-  for (int i = 0; i < limit && (pair_issued(mark, lead) == kPairRunning || pair_issued(mark, lead + 1) == kPairRunning); ++i) __nanosleep(1000);
+  for (int i = 0; i < limit && (pair_issued(mark, 0, lead) == kPairRunning || pair_issued(mark, 0, lead + 1) == kPairRunning ||
+                                pair_issued(mark, 1, lead) == kPairRunning || pair_issued(mark, 1, lead + 1) == kPairRunning); ++i)
+    __nanosleep(1000);
 }
 struct PairWaits : tc::Waits {
   int ctas;
@@ -156,16 +162,19 @@ __device__ __forceinline__ PairTile pair_tile(const TcParams& p, int t) {
   return r;
 }
 
-// After a wait that ran out, with both CTAs' roles at their ends: the loads in flight land before either gives its shared memory up.
-__device__ __forceinline__ void pair_land(const PairWaits& wait, uint64_t* full, const TcParams& p, uint32_t* mark, int lead, int kbs, int first, int step) {
+// After a wait that ran out, with both CTAs' roles at their ends: the loads in flight (of either ring) land before either gives its shared memory up.
+__device__ __forceinline__ void pair_land(const PairWaits& wait, uint64_t* full_w, uint64_t* full_x, const TcParams& p, uint32_t* mark, int lead, int kbs, int first,
+                                          int step) {
 #pragma unroll 1
-  for (int s = 0; s < kPairStages; ++s) {
-    const PairOwed o = pair_owed(s, kPairStages, (int)pair_issued(mark, lead), (int)pair_issued(mark, lead + 1));
+  for (int i = 0; i < kPairWStages + kPairXStages; ++i) {
+    const int ring = i >= kPairWStages, s = ring ? i - kPairWStages : i;
+    uint64_t* full = ring ? full_x + s : full_w + s;
+    const PairOwed o = pair_owed(s, ring ? kPairXStages : kPairWStages, (int)pair_issued(mark, ring, lead), (int)pair_issued(mark, ring, lead + 1));
     if (o.parity < 0) continue;
-    const uint32_t half = kPairABytes + (uint32_t)pair_tile(p, first + o.fill / kbs * step).n * kBlockK;   // a CTA's bytes of the fill
-    if (o.announce > 0) tc::mbar_expect_tx(&full[s], half);
-    if (o.announce < 0) asm volatile("mbarrier.complete_tx.relaxed.cluster.shared::cta.b64 [%0], %1;" ::"r"(tc::smem_u32(&full[s])), "r"(half) : "memory");
-    wait.drain(&full[s], (uint32_t)o.parity);
+    const uint32_t half = ring ? (uint32_t)pair_tile(p, first + o.fill / kbs * step).n * kBlockK : kPairABytes;   // a CTA's bytes of the fill
+    if (o.announce > 0) tc::mbar_expect_tx(full, half);
+    if (o.announce < 0) asm volatile("mbarrier.complete_tx.relaxed.cluster.shared::cta.b64 [%0], %1;" ::"r"(tc::smem_u32(full)), "r"(half) : "memory");
+    wait.drain(full, (uint32_t)o.parity);
   }
 }
 
@@ -182,14 +191,16 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ PairMaps maps, const TcParams p, uint32_t* status) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  float* stg_all = reinterpret_cast<float*>(smem + kPairStages * kPairStageBytes);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kPairStages * kPairStageBytes + 2 * kPairStgBytes);   // the leader's: both CTAs' bytes
-  uint64_t* empty = full + kPairStages;
-  uint64_t* acc_full = empty + kPairStages;    // [2]
+  float* stg_all = reinterpret_cast<float*>(smem + kPairRings);
+  uint64_t* full_w = reinterpret_cast<uint64_t*>(smem + kPairRings + 2 * kPairStgBytes);   // the leader's: both CTAs' bytes
+  uint64_t* full_x = full_w + kPairWStages;
+  uint64_t* empty_w = full_x + kPairXStages;
+  uint64_t* empty_x = empty_w + kPairWStages;
+  uint64_t* acc_full = empty_x + kPairXStages;   // [2]
   uint64_t* acc_free = acc_full + 2;           // [2] the leader's: both CTAs' epilogue warps
   uint64_t* last = acc_free + 2;               // after a wait that ran out: the MMAs issued before
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(last + 1);
-  uint32_t* mark = tmem_slot + 1;              // and, behind it, how many fills the CTA issued
+  uint32_t* mark = tmem_slot + 1;              // and, behind it, how many fills of either ring the CTA issued
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // a cluster: the CTA pairs of one tile, each with its share of k
   const int cta = blockIdx.x % (2 * p.splits), rank = cta & 1, split = cta >> 1, lead = cta - rank;
@@ -198,17 +209,14 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   const int kb0 = split * kb_base + min(split, kb_rem), kb1 = kb0 + kb_base + (split < kb_rem ? 1 : 0);
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kPairStages; ++s) {
-      tc::mbar_init(&full[s], 1);
-      tc::mbar_init(&empty[s], 1);
-    }
+    for (int s = 0; s < 2 * (kPairWStages + kPairXStages); ++s) tc::mbar_init(&full_w[s], 1);   // full and empty of both rings
     for (int s = 0; s < 2; ++s) {
       tc::mbar_init(&acc_full[s], 1);
       tc::mbar_init(&acc_free[s], 16);
     }
     tc::mbar_init(last, 1);
     mark[0] = 0;
-    mark[1] = kPairRunning;
+    mark[1] = mark[2] = kPairRunning;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -226,40 +234,47 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   pdl_launch_dependents();
   const int tiles = (p.pair_tile ? __ldg(&p.pair_tile[0].x) : p.pair_tok) * p.pair_m;
 
-  if (warp == 0) {
-    // ===== fetch: the whole warp walks the loop, one lane issues =====
+  if (warp == 0 || warp == kPairWarps - 1) {
+    // ===== fetch weights (warp 0), tokens (the last one): the whole warp walks the loop, one lane issues =====
     const bool issuer = elect_one();
-    if (issuer) {
-      asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
-      if (!p.pair_tile) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.x[(p.pair_n >> 5) - 1]) : "memory");
-    }
-    int it = 0;
-    for (int t = first; t < tiles; t += step) {
-      const PairTile tile = pair_tile(p, t);
-      const int half = tile.n >> 1, x0 = tile.row0 + rank * half, m = 2 * tile.m + rank;
-      const int w0 = tile.expert * p.n_out + m * kBlockM;
-      const CUtensorMap* map_x = &maps.x[(tile.n >> 5) - 1];
-      const uint32_t bytes = (uint32_t)(2 * kPairABytes + tile.n * kBlockK * 2);
-      for (int kb = kb0; kb < kb1; ++kb, ++it) {
-        const int st = it % kPairStages;
-        if (it >= kPairStages && !wait.all(&empty[st], (it / kPairStages - 1) & 1)) break;
-        if (issuer) {
-          unsigned char* a = smem + st * kPairStageBytes;
-          const uint32_t bar = smem_of(&full[st], lead);
-          if (rank == 0) tc::mbar_expect_tx(&full[st], bytes);
-          if (p.gu_ff) pair_load3(a, &map_w, kb * kBlockK, m * (kBlockM / 2), 2 * tile.expert, bar, kKeepNormal);   // 64 gate rows, then the matching up rows
-          else pair_load(a, &map_w, kb * kBlockK, w0, bar, kKeepNormal);
-          pair_load(a + kPairABytes, map_x, kb * kBlockK, x0, bar, kKeepLast);
-        }
-        __syncwarp();
-        if (wait.stop()) {
-          ++it;   // (this fill too)
-          break;
-        }
+    auto fetch = [&](auto ring) {
+      constexpr int RING = decltype(ring)::value, STAGES = RING ? kPairXStages : kPairWStages;
+      uint64_t *full = RING ? full_x : full_w, *empty = RING ? empty_x : empty_w;
+      unsigned char* slots = smem + RING * kPairWStages * kPairABytes;
+      if (issuer) {
+        if (RING == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
+        else if (!p.pair_tile) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.x[(p.pair_n >> 5) - 1]) : "memory");
       }
-      if (wait.stop()) break;
-    }
-    if (issuer) *reinterpret_cast<volatile uint32_t*>(mark + 1) = (uint32_t)it;
+      int it = 0;
+      for (int t = first; t < tiles; t += step) {
+        const PairTile tile = pair_tile(p, t);
+        const int half = tile.n >> 1, x0 = tile.row0 + rank * half, m = 2 * tile.m + rank;
+        const int w0 = tile.expert * p.n_out + m * kBlockM;
+        const CUtensorMap* map_x = &maps.x[(tile.n >> 5) - 1];
+        const uint32_t bytes = RING ? (uint32_t)(tile.n * kBlockK * 2) : (uint32_t)(2 * kPairABytes);
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+          const int st = it % STAGES;
+          if (it >= STAGES && !wait.all(&empty[st], (it / STAGES - 1) & 1)) break;
+          if (issuer) {
+            unsigned char* dst = slots + st * kPairABytes;
+            const uint32_t bar = smem_of(&full[st], lead);
+            if (rank == 0) tc::mbar_expect_tx(&full[st], bytes);
+            if (RING) pair_load(dst, map_x, kb * kBlockK, x0, bar, kKeepLast);
+            else if (p.gu_ff) pair_load3(dst, &map_w, kb * kBlockK, m * (kBlockM / 2), 2 * tile.expert, bar, kKeepNormal);   // 64 gate rows, then the matching up rows
+            else pair_load(dst, &map_w, kb * kBlockK, w0, bar, kKeepNormal);
+          }
+          __syncwarp();
+          if (wait.stop()) {
+            ++it;   // (this fill too)
+            break;
+          }
+        }
+        if (wait.stop()) break;
+      }
+      if (issuer) *reinterpret_cast<volatile uint32_t*>(mark + 1 + RING) = (uint32_t)it;
+    };
+    if (warp == 0) fetch(std::integral_constant<int, 0>());
+    else fetch(std::integral_constant<int, 1>());
   } else if (warp == 1) {
     // ===== the leader's MMA warp: instructions predicated to one lane in convergent code =====
     if (rank == 0) {
@@ -268,8 +283,8 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       const uint64_t desc0 = tc::make_desc(tc::smem_u32(smem), 16, 1024);
       const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
       const int n_tiles = __shfl_sync(0xffffffffu, tiles, 0);
-      int i = 0, st = 0;
-      uint32_t st_ph = 0;
+      int i = 0, sw = 0, sx = 0;
+      uint32_t ph_w = 0, ph_x = 0;
       for (int t = first; t < n_tiles; t += step, ++i) {
         const int n = __shfl_sync(0xffffffffu, pair_tile(p, t).n, 0);
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(2 * kBlockM >> 4) << 24);
@@ -277,15 +292,18 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         if (i >= 2) wait(&acc_free[i & 1], ((i >> 1) - 1) & 1);
         tc::fence_after();
         for (int kb = kb0; kb < kb1; ++kb) {
-          wait(&full[st], st_ph, [&] { pair_await_ends(mark, lead, wait.limit); });
+          wait(&full_x[sx], ph_x, [&] { pair_await_ends(mark, lead, wait.limit); });
+          wait(&full_w[sw], ph_w, [&] { pair_await_ends(mark, lead, wait.limit); });
           tc::fence_after();
-          const uint64_t da = desc0 + (uint64_t)((st * kPairStageBytes) >> 4), db = da + (uint64_t)(kPairABytes >> 4);
+          const uint64_t da = desc0 + (uint64_t)((sw * kPairABytes) >> 4), db = desc0 + (uint64_t)(((kPairWStages + sx) * kPairABytes) >> 4);
           const uint32_t more = kb > kb0 ? 1u : 0u;
 #pragma unroll
           for (int k = 0; k < kBlockK / 16; ++k)   // 16 of k are 32 bytes inside the swizzle's span
             pair_mma(one, acc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, k ? 1u : more);
-          pair_commit(one, &empty[st], both);
-          if (++st == kPairStages) st = 0, st_ph ^= 1;
+          pair_commit(one, &empty_w[sw], both);
+          pair_commit(one, &empty_x[sx], both);
+          if (++sw == kPairWStages) sw = 0, ph_w ^= 1;
+          if (++sx == kPairXStages) sx = 0, ph_x ^= 1;
         }
         pair_commit(one, &acc_full[i & 1], both);
         if (wait.stop()) break;
@@ -460,7 +478,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     __syncthreads();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    if (warp >= 2) {
+    if (warp >= 2 && warp < kPairWarps - 1) {
       const PairTile tile = pair_tile(p, first);
       const int m_tile = 2 * tile.m + rank, r4 = lane * 4, n_rows = min(tile.n, p.T - tile.row0);
       if (m_tile * kBlockM < p.n_out && !wait.marked()) {
@@ -498,7 +516,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // a CTA's shared and tensor memory serve the other's MMAs
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (wait.marked()) {   // the same answer in all CTAs of the cluster, whose waits have ended
-    if (rank == 0 && threadIdx.x == 0) pair_land(wait, full, p, mark, lead, kb1 - kb0, first, step);
+    if (rank == 0 && threadIdx.x == 0) pair_land(wait, full_w, full_x, p, mark, lead, kb1 - kb0, first, step);
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");

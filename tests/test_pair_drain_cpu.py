@@ -96,3 +96,10 @@ def test_everything_that_was_issued_has_landed_before_the_end(owed, seed):
             assert bars[s].phase == max(n) - 1, "the wait would end before the last bytes are there"
             bars[s].land(b)
         assert bars[s].phase == max(n) and (max(n) - 1) & 1 == o.parity and bars[s].tx == 0
+
+
+@pytest.mark.parametrize("stages", [5, 7])
+@pytest.mark.parametrize("seed", range(60))
+def test_rings_of_other_depths(owed, seed, stages, monkeypatch):
+    monkeypatch.setitem(globals(), "STAGES", stages)
+    test_everything_that_was_issued_has_landed_before_the_end(owed, seed)
