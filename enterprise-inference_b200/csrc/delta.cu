@@ -324,10 +324,13 @@ __device__ __forceinline__ void ds_walk(const ScanArgs& a, float* stage) {
 // these lanes together (a lane keeps half of what it holds at every step); two warps turn the rows of the blocks ahead into L q, L k and
 // (L_8 / L) k; one or two work out the triangles of every C-th block for the C CTAs of the cluster, a round of blocks ahead.
 // LG 32 (four main warps) while one or two CTAs an SM are enough, LG 16 (two warps, a third fewer instructions a column) for three.
-// What bounds them: a block's chain of about 2 300 cycles (dots 840, their reduction 560, triangles and u 500, update 210, waiting for the
+// What bounds them: a block's chain of about 2 100 cycles (dots 840, their reduction 400, triangles and u 500, update 210, waiting for the
 // cluster 230), and issue slots where CTAs share an SM: a shuffle takes four cycles of a scheduler, a packed fma two.
-// Against the walk (us, 16 heads of 128 x 128, channel decays): one sequence of 1 900 rows 406 -> 295, of 950 205 -> 152, two of 1 000 together
-// 182 -> 167, three of 1 900 295 -> 248; one decay per head 228 -> 146; keys of 64 216 -> 125; 150 rows 37 -> 31.  The walk keeps short portions (a
+// A reduction's first two steps go over the rows: a lane takes the rows of a set in an order of its own, so that every lane keeps the same registers and
+// hands over the same others.  Choosing them by lane was two selections a shuffle: without, one sequence of 2 000 rows 310 -> 274 us, two of 1 000
+// together 163 -> 147, three of 1 900 244 -> 228, keys of 64 239 -> 205 (same sums, same bits).
+// Against the walk before that (us, 16 heads of 128 x 128, channel decays): one sequence of 1 900 rows 406 -> 295, of 950 205 -> 152, two of 1 000
+// together 182 -> 167, three of 1 900 295 -> 248; one decay per head 228 -> 146; keys of 64 216 -> 125; 150 rows 37 -> 31.  The walk keeps short portions (a
 // block needs its triangles before it starts, about 5 us), the uncorrected rule (in CTAs of 32 columns three sequences of 64 heads 282 -> 251, but
 // four short ones 11 -> 17) and what would fill the device more than once.
 constexpr int kDbRows = 8, kDbScale = 2, kDbSlots = 4, kDbCluster = 4;   // (clusters of eight such CTAs do not fit the device sixteen at a time)
@@ -371,6 +374,13 @@ __device__ __forceinline__ void db_halve(float* x, int lane) {
     const float keep = up ? x[i + H] : x[i], give = up ? x[i] : x[i + H];
     x[i] = keep + __shfl_xor_sync(0xffffffffu, give, H);
   }
+}
+
+// The same where every lane has laid its values out so that the first half is the one it keeps.
+template <int H>
+__device__ __forceinline__ void db_fold(float* x) {
+#pragma unroll
+  for (int i = 0; i < H; ++i) x[i] += __shfl_xor_sync(0xffffffffu, x[i + H], H);
 }
 
 template <int NP, bool CHAN, int LG, int CTAS>
@@ -623,6 +633,10 @@ __global__ void __launch_bounds__(db_threads(LG), CTAS) delta_block_kernel(const
       y[2 * i + 1] = t.y;
     }
   };
+  // a lane takes the rows of a set in the order that leaves its own row of the four first: what it hands over is then the same half in every lane
+  int own[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) own[r] = (r ^ rr) * ROW;
   fetch_v(0);
   db_cluster_wait();
   db_cluster_arrive_relaxed();
@@ -658,7 +672,7 @@ __global__ void __launch_bounds__(db_threads(LG), CTAS) delta_block_kernel(const
         const int set = s0 + s1;
         uint64_t y[4][2 * V];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) row_of(in + ((set < 2 ? R : 0) + 4 * (set & 1) + r) * ROW, y[r]);
+        for (int r = 0; r < 4; ++r) row_of(in + ((set < 2 ? R : 0) + 4 * (set & 1)) * ROW + own[r], y[r]);
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -673,9 +687,9 @@ __global__ void __launch_bounds__(db_threads(LG), CTAS) delta_block_kernel(const
 #pragma unroll
         for (int s1 = 0; s1 < JOINT; ++s1) f(part[s1]);
       };
-      all([&](float* x) { db_halve<8>(x, lane); });
+      all([&](float* x) { db_fold<8>(x); });
       if (s0 + JOINT == 4) triangles();
-      all([&](float* x) { db_halve<4>(x, lane); });
+      all([&](float* x) { db_fold<4>(x); });
       all([&](float* x) { db_halve<2>(x, lane); });
       all([&](float* x) { db_halve<1>(x, lane); });
 #pragma unroll
