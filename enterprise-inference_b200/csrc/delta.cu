@@ -302,13 +302,14 @@ __global__ void __launch_bounds__(kDsThreads) delta_scan_kernel(const ScanArgs a
   constexpr int ROW = ds_row(NP), BUF = ds_buf(NP, CHAN);
   pdl_wait();
   pdl_launch_dependents();
+  const int s = blockIdx.x, h = blockIdx.y, jb = blockIdx.z * kDsCols;
 #define DS_SYNC() __syncthreads()
 #include "delta_walk.cuh"
 #undef DS_SYNC
 }
 // the same by the first kDsThreads threads of a larger CTA
 template <int NP, bool DELTA, bool CHAN>
-__device__ __forceinline__ void ds_walk(const ScanArgs& a, float* stage) {
+__device__ __forceinline__ void ds_walk(const ScanArgs& a, float* stage, int s, int h, int jb) {
   constexpr int ROW = ds_row(NP), BUF = ds_buf(NP, CHAN);
 #define DS_SYNC() asm volatile("bar.sync 1, 128;" ::: "memory")
 #include "delta_walk.cuh"
@@ -323,27 +324,36 @@ __device__ __forceinline__ void ds_walk(const ScanArgs& a, float* stage) {
 // A CTA per (sequence, head, 16 value columns), those of a head in clusters.  Its main warps own four columns per LG lanes and reduce a block's sums over
 // these lanes together (a lane keeps half of what it holds at every step); two warps turn the rows of the blocks ahead into L q, L k and
 // (L_8 / L) k; one or two work out the triangles of every C-th block for the C CTAs of the cluster, a round of blocks ahead.
-// LG 32 (four main warps) while one or two CTAs an SM are enough, LG 16 (two warps, a third fewer instructions a column) for three.
+// LG 32 (four main warps) where one or two CTAs share an SM, LG 16 (two warps, a third fewer instructions a column) for three and for keys of at most 64.
 // What bounds them: a block's chain of about 2 100 cycles (dots 840, their reduction 400, triangles and u 500, update 210, waiting for the
 // cluster 230), and issue slots where CTAs share an SM: a shuffle takes four cycles of a scheduler, a packed fma two.
 // A reduction's first two steps go over the rows: a lane takes the rows of a set in an order of its own, so that every lane keeps the same registers and
 // hands over the same others.  Choosing them by lane was two selections a shuffle: without, one sequence of 2 000 rows 310 -> 274 us, two of 1 000
 // together 163 -> 147, three of 1 900 244 -> 228, keys of 64 239 -> 205 (same sums, same bits).
-// Against the walk before that (us, 16 heads of 128 x 128, channel decays): one sequence of 1 900 rows 406 -> 295, of 950 205 -> 152, two of 1 000
-// together 182 -> 167, three of 1 900 295 -> 248; one decay per head 228 -> 146; keys of 64 216 -> 125; 150 rows 37 -> 31.  The walk keeps short portions (a
-// block needs its triangles before it starts, about 5 us), the uncorrected rule (in CTAs of 32 columns three sequences of 64 heads 282 -> 251, but
-// four short ones 11 -> 17) and what would fill the device more than once.
+// Against the walk (us, 16 heads of 128 x 128, channel decays): one sequence of 1 900 rows 406 -> 260, two of 1 000 together 182 -> 114, three of 1 900
+// 295 -> 186, four of 1 200 315 -> 145; one decay per head, four of 2 048 554 -> 210; keys of 64, four of 2 000 349 -> 129; 150 rows 37 -> 26.  The walk keeps
+// short portions (a block needs its triangles before it starts, about 5 us) and the uncorrected rule (in CTAs of 32 columns three sequences of 64 heads
+// 282 -> 251, but four short ones 11 -> 17).
 constexpr int kDbRows = 8, kDbScale = 2, kDbSlots = 4, kDbCluster = 4;   // (clusters of eight such CTAs do not fit the device sixteen at a time)
 constexpr int kDbTri = 2 * kDbRows * kDbRows;   // T, B
 constexpr int db_main(int lg) { return lg == 32 ? 4 : 2; }   // warps with columns; warps that work out triangles
-constexpr int db_tri_warps(int lg) { return lg == 32 ? 2 : 1; }
-constexpr int db_threads(int lg) { return (db_main(lg) + kDbScale + db_tri_warps(lg)) * 32; }
+constexpr int db_tri_warps(int ctas) { return ctas <= 2 ? 2 : 1; }   // (ctas: that share an SM)
+constexpr int db_threads(int lg, int ctas) { return (db_main(lg) + kDbScale + db_tri_warps(ctas)) * 32; }
 // rows from which a portion goes in blocks: where the two meet for one sequence, and for two to four
 constexpr int db_from(int lg) { return lg == 32 ? 64 : 128; }
+// CTAs that share an SM.  Two where the launch then fills its places twice over (four sequences, 16 heads of 128 x 128: 1 200 rows 145 us, at three 173),
+// three where that leaves a third of a wave alone (three sequences of 1 900 rows 186, at two 247) and from four launches' worth on (eight of 2 048 206, at two 213).
+constexpr int db_share(int64_t ctas) { return ctas <= kNumSMs ? 1 : ctas <= 2 * kNumSMs || (ctas > 3 * kNumSMs && ctas <= 4 * kNumSMs) ? 2 : 3; }
+// lanes of four columns
+constexpr int db_lanes(int np, int share) { return np == 2 && share <= 2 ? 32 : 16; }
+// Sequences of a launch in blocks whose rows the host does not know: with more of them most are likely short, and these are walked faster by the walk's own CTAs
+// (eight sequences of three rows 9.2 us, from the block kernel 10.2; six 9.2 and 8.5).  Where it knows them, up to as many as db_sequence orders, of at
+// least kDbMean rows on average (eight of 125 rows 146 us, in blocks 111; 32 of 25 rows 122 and 111, of three 28 and 36).
+constexpr int kDbSeqs = 6, kDbOrdered = 32, kDbMean = 32;
 // floats of a slot: L q | L k | (L_8 / L) k, L_8
 __host__ __device__ constexpr int db_slot(int np) { return (3 * kDbRows + 1) * ds_row(np); }
 // slots; three rounds of triangles; per main warp 8 x 8 pairs (u, u)
-constexpr int db_floats(int np, int lg) { return kDbSlots * db_slot(np) + 3 * db_tri_warps(lg) * kDbCluster * kDbTri + db_main(lg) * kDbRows * 16; }
+constexpr int db_floats(int np, int lg, int ctas) { return kDbSlots * db_slot(np) + 3 * db_tri_warps(ctas) * kDbCluster * kDbTri + db_main(lg) * kDbRows * 16; }
 template <int N>
 __device__ __forceinline__ void db_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(N) : "memory"); }
 template <int N>
@@ -383,16 +393,30 @@ __device__ __forceinline__ void db_fold(float* x) {
   for (int i = 0; i < H; ++i) x[i] += __shfl_xor_sync(0xffffffffu, x[i + H], H);
 }
 
+// The k-th longest of n portions: the grid goes over the sequences last and the longest first.  The CTAs of an SM are then of several sequences, and
+// what waits for a place is short.  With the sequences first in the grid those of an SM were mostly of one, and the longest one's SMs the last: three of 1 900 rows
+// together 228 us, 186 now, two of 1 000 147 and 114, one decay per head 372 and 254.
+__device__ __forceinline__ int db_sequence(const ScanArgs& a, int n, int k) {
+  static_assert(kDbOrdered == 32, "a lane a sequence");
+  const int lane = threadIdx.x & 31, rows = lane < n ? a.seq_start[lane + 1] - a.seq_start[lane] : -1;
+  int rank = 0;
+  for (int i = 0; i < n; ++i) {
+    const int other = __shfl_sync(0xffffffffu, rows, i);
+    rank += other > rows || (other == rows && i < lane);
+  }
+  return __ffs(__ballot_sync(0xffffffffu, lane < n && rank == k)) - 1;
+}
+
 template <int NP, bool CHAN, int LG, int CTAS>
-__global__ void __launch_bounds__(db_threads(LG), CTAS) delta_block_kernel(const ScanArgs a) {
+__global__ void __launch_bounds__(db_threads(LG, CTAS), CTAS) delta_block_kernel(const ScanArgs a) {
   extern __shared__ __align__(16) float stage[];
   constexpr int ROW = ds_row(NP), R = kDbRows, SLOT = db_slot(NP), MAIN = db_main(LG), BAR = 32 * (MAIN + 1);   // BAR: threads of the main warps and one other
   // named barriers: slot ready; slot read; triangles of an even (odd) round read, from the main warps to those that work triangles out
-  constexpr int kFull = 1, kEmpty = 1 + kDbSlots, kRead = 1 + 2 * kDbSlots, READ = 32 * (MAIN + db_tri_warps(LG));
+  constexpr int kFull = 1, kEmpty = 1 + kDbSlots, kRead = 1 + 2 * kDbSlots, READ = 32 * (MAIN + db_tri_warps(CTAS));
   static_assert(NP <= 2, "a preparing lane's channels are one piece of at most 16 bytes");
   pdl_wait();
   pdl_launch_dependents();
-  const int s = blockIdx.x, h = blockIdx.y, jb = blockIdx.z * kDsCols;
+  const int h = blockIdx.y, jb = blockIdx.x * kDsCols, s = db_sequence(a, gridDim.z, blockIdx.z);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int start = a.seq_start[s], n_rows = a.seq_start[s + 1] - start;
   if (n_rows <= 0) return;
@@ -407,14 +431,14 @@ __global__ void __launch_bounds__(db_threads(LG), CTAS) delta_block_kernel(const
   float* out = a.out + (int64_t)start * hv + (int64_t)h * vd + jb;
   float* state = a.state + (int64_t)a.seq_slots[s] * a.slot_stride + ((int64_t)h * vd + jb) * dim;
   if (n_rows < db_from(LG)) {
-    if (warp < kDsWarps) ds_walk<NP, true, CHAN>(a, stage);
+    if (warp < kDsWarps) ds_walk<NP, true, CHAN>(a, stage, s, h, jb);
     return;
   }
   const int n_blocks = (n_rows + R - 1) / R;
   uint32_t C, rank;   // CTAs of the cluster, all of one sequence and head
   asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(C));
   asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-  const int per_round = db_tri_warps(LG) * (int)C, rounds = (n_blocks + per_round - 1) / per_round;
+  const int per_round = db_tri_warps(CTAS) * (int)C, rounds = (n_blocks + per_round - 1) / per_round;
   float* tris = stage + kDbSlots * SLOT;   // [3][blocks of a round][T | B]
   // cluster barriers: all CTAs run; then, for every round p, its triangles are there and those of round p - 3 have been read
   db_cluster_arrive_relaxed();
@@ -599,7 +623,7 @@ __global__ void __launch_bounds__(db_threads(LG), CTAS) delta_block_kernel(const
   // ===== LG lanes four columns, a lane x of them the channels 4 x + 4 LG v =====
   constexpr int CW = 128 / LG, V = ROW / (4 * LG);   // columns of a warp; pieces of four channels a lane
   const int xl = lane & (LG - 1), x16 = lane & 15, grp = lane / LG, j0 = warp * CW + grp * 4, cols = min(vd - jb - j0, 4);
-  float* us = tris + 3 * db_tri_warps(LG) * kDbCluster * kDbTri + warp * R * 16;   // [8 rows][CW columns] pairs (u, u)
+  float* us = tris + 3 * db_tri_warps(CTAS) * kDbCluster * kDbTri + warp * R * 16;   // [8 rows][CW columns] pairs (u, u)
   uint64_t S[4][2 * V];
   float* S_st = state + (int64_t)j0 * dim;
 #pragma unroll
@@ -769,22 +793,22 @@ int db_cluster(int blocks) {
 template <int NP, bool CHAN, int LG, int CTAS>   // CTAS: that share an SM
 int delta_block(const ScanArgs& a, int S, cudaStream_t s) {
   static bool done[64] = {};
-  const dim3 grid(S, a.heads, (a.vd + kDsCols - 1) / kDsCols);
+  const dim3 grid((a.vd + kDsCols - 1) / kDsCols, a.heads, S);
   // shared memory for CTAS an SM, so that no more meet there: the CTAs of a cluster are packed onto as few SMs as hold them
-  constexpr int need = std::max(db_floats(NP, LG), ds_floats(NP, CHAN)) * 4, bytes = CTAS == 1 ? 120 * 1024 : CTAS == 2 ? 80 * 1024 : need;
+  constexpr int need = std::max(db_floats(NP, LG, CTAS), ds_floats(NP, CHAN)) * 4, bytes = CTAS == 1 ? 120 * 1024 : CTAS == 2 ? 80 * 1024 : need;
   static_assert(need <= bytes && CTAS * (bytes + 1024) <= 228 * 1024, "CTAs an SM");
   B200_CUDA(ensure_dynamic_smem(delta_block_kernel<NP, CHAN, LG, CTAS>, bytes, done));
-  B200_CUDA(launch_cluster(delta_block_kernel<NP, CHAN, LG, CTAS>, grid, dim3(db_threads(LG)), (size_t)bytes, s, dim3(1, 1, db_cluster((int)grid.z)), a));
+  B200_CUDA(launch_cluster(delta_block_kernel<NP, CHAN, LG, CTAS>, grid, dim3(db_threads(LG, CTAS)), (size_t)bytes, s, dim3(db_cluster((int)grid.x), 1, 1), a));
   return B200_OK;
 }
 
 template <int NP, bool CHAN>
 int delta_blocks(const ScanArgs& a, int S, int64_t ctas, cudaStream_t s) {
-  if constexpr (NP == 2) {
-    if (ctas <= kNumSMs) return delta_block<NP, CHAN, 32, 1>(a, S, s);
-    if (ctas <= 2 * kNumSMs) return delta_block<NP, CHAN, 32, 2>(a, S, s);
+  switch (db_share(ctas)) {
+    case 1: return delta_block<NP, CHAN, db_lanes(NP, 1), 1>(a, S, s);
+    case 2: return delta_block<NP, CHAN, db_lanes(NP, 2), 2>(a, S, s);
+    default: return delta_block<NP, CHAN, db_lanes(NP, 3), 3>(a, S, s);
   }
-  return delta_block<NP, CHAN, 16, 3>(a, S, s);
 }
 
 }  // namespace
@@ -883,7 +907,8 @@ int linear_scan(bool delta_rule, const float* qn, const float* kn, const float* 
   const bool single_rows = rows == S;
   // Blocks where a portion may be long enough for them; where the rows of the step are known to be too few its walk is launched by itself (one portion of 63 rows, 16
   // heads of 128 x 128: 19.0 us from the block kernel, 18.2; of two rows 5.5 and 5.1)
-  const bool blocks = a.vec && ctas <= 3 * kNumSMs && (rows <= 0 || rows - S + 1 >= db_from(dim > 64 && ctas <= 2 * kNumSMs ? 32 : 16));
+  const bool few = S <= kDbSeqs && ctas <= kDbSeqs * kNumSMs, many = S <= kDbOrdered && ctas <= kDbOrdered * kNumSMs && rows >= kDbMean * S;
+  const bool blocks = a.vec && (few || many) && (rows <= 0 || rows - S + 1 >= db_from(db_lanes(dim > 64 ? 2 : 1, db_share(ctas))));
 #define SCAN3(D, R, CH)                                                                                       \
   do {                                                                                                        \
     static bool done[64] = {};                                                                                \

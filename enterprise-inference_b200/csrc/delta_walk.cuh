@@ -1,6 +1,6 @@
 // The body of the walk (delta.cu), which its kernel and the block kernel's short portions share as text: as a function in both the kernel's registers
-// fell differently (64 decode rows 40 -> 45 us).  From its surroundings: NP, DELTA, CHAN, the arguments a, shared memory `stage`, DS_SYNC().
-  const int s = blockIdx.x, h = blockIdx.y, jb = blockIdx.z * kDsCols;
+// fell differently (64 decode rows 40 -> 45 us).  From its surroundings: NP, DELTA, CHAN, the arguments a, sequence s, head h,
+// first value column jb, shared memory `stage`, DS_SYNC().
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int start = a.seq_start[s], n_rows = a.seq_start[s + 1] - start;
   if (n_rows <= 0) return;

@@ -322,6 +322,16 @@ def test_delta_blocks(heads, kv, dim, vdim, steps, chan):
     assert (state[0] == 7.5).all()
 
 
+# Portions in the order of their length (equal ones, empty ones, the longest first and last), more CTAs than the device has places for, two and three of them
+# an SM, keys of 64 on CTAs of one and two an SM; the bound is that of the test above.
+@pytest.mark.parametrize("heads,kv,dim,vdim,steps", [
+    (16, 16, 128, 128, [[70, 300, 1, 129], [129, 129, 64, 0]]), (16, 8, 128, 128, [[2, 200, 130, 128, 5, 31], [0, 64, 0, 90, 160, 64]]), (40, 40, 64, 128, [[5, 140, 131]]),
+    (8, 2, 64, 128, [[129, 260]]), (16, 16, 100, 48, [[128, 7, 300, 300, 66]]),
+])
+def test_delta_blocks_of_ordered_portions(heads, kv, dim, vdim, steps):
+    test_delta_blocks(heads, kv, dim, vdim, steps, True)
+
+
 @pytest.mark.parametrize("what", ["value", "key", "query", "decay", "beta"])
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
 @pytest.mark.parametrize("row", [0, 37, 99])
