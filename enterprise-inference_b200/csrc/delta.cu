@@ -330,8 +330,8 @@ __device__ __forceinline__ void ds_walk(const ScanArgs& a, float* stage, int s, 
 // A reduction's first two steps go over the rows: a lane takes the rows of a set in an order of its own, so that every lane keeps the same registers and
 // hands over the same others.  Choosing them by lane was two selections a shuffle: without, one sequence of 2 000 rows 310 -> 274 us, two of 1 000
 // together 163 -> 147, three of 1 900 244 -> 228, keys of 64 239 -> 205 (same sums, same bits).
-// Against the walk (us, 16 heads of 128 x 128, channel decays): one sequence of 1 900 rows 406 -> 260, two of 1 000 together 182 -> 114, three of 1 900
-// 295 -> 186, four of 1 200 315 -> 145; one decay per head, four of 2 048 554 -> 210; keys of 64, four of 2 000 349 -> 129; 150 rows 37 -> 26.  The walk keeps
+// Against the walk (us, 16 heads of 128 x 128, channel decays): one sequence of 1 900 rows 406 -> 245, two of 1 000 together 182 -> 114, three of 1 900
+// 295 -> 186, four of 1 200 315 -> 145; one decay per head, four of 2 048 554 -> 211; keys of 64, four of 2 000 349 -> 129; 150 rows 37 -> 26.  The walk keeps
 // short portions (a block needs its triangles before it starts, about 5 us) and the uncorrected rule (in CTAs of 32 columns three sequences of 64 heads
 // 282 -> 251, but four short ones 11 -> 17).
 constexpr int kDbRows = 8, kDbScale = 2, kDbSlots = 4, kDbCluster = 4;   // (clusters of eight such CTAs do not fit the device sixteen at a time)
@@ -448,24 +448,51 @@ __global__ void __launch_bounds__(db_threads(LG, CTAS), CTAS) delta_block_kernel
     int pi = 1;
     while (pi < R - 1 && lane >= (pi + 1) * pi / 2) ++pi;
     const int d = 2 * NP * lane;
+    using Rows = uint64_t[R];
+    Rows k0, g0, q0;
+    auto pieces = [&](int b, int i, Rows& k, Rows& g, Rows& q, float gs = 0.f) {   // the lane's i-th pairs of the block's rows
+      const int nb = min(n_rows - b * R, R);
+      auto pair = [&](const float* src, int64_t st, int r, uint64_t none) {
+        return r < nb && d < dim ? *reinterpret_cast<const uint64_t*>(src + (int64_t)(b * R + r) * st + d + 2 * i) : none;
+      };
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        k[r] = pair(ksrc, qk, r, 0);
+        q[r] = pair(qsrc, qk, r, 0);
+        g[r] = CHAN ? pair(gsrc, a.g_row, r, f2::both(1.f)) : f2::both(__shfl_sync(0xffffffffu, gs, r));
+      }
+    };
+    // what a block starts with; where a CTA has an SM's registers to itself it is asked for before the wait for the round before (2 000 rows alone 275 -> 258 us; at the
+    // 128 registers of two or three CTAs an SM warps spill for it, three sequences of 1 900 rows 184 -> 232)
+    constexpr bool AHEAD = CTAS == 1 && NP == 2;
+    float bs0, gs0;   // of row `lane`
+    auto scalars = [&](int b, float& bs, float& gs) {
+      const int nb = min(n_rows - b * R, R);
+      bs = lane < nb ? bsrc[(int64_t)(b * R + lane) * a.heads] : 0.f;
+      gs = !CHAN && lane < nb ? gsrc[(int64_t)(b * R + lane) * a.g_row] : 1.f;
+    };
+    auto fetch = [&](int b) {
+      if (b >= n_blocks) return;
+      scalars(b, bs0, gs0);
+      pieces(b, 0, k0, g0, q0);
+    };
+    if (AHEAD) fetch((warp - MAIN - kDbScale) * (int)C + (int)rank);
     db_cluster_wait();
     for (int p = 0; p < rounds; ++p) {
-      const int mine = (warp - MAIN - kDbScale) * (int)C + (int)rank, b = p * per_round + mine;
+      const int own = (warp - MAIN - kDbScale) * (int)C + (int)rank, b = p * per_round + own;
       if (b < n_blocks) {
-        const int nb = min(n_rows - b * R, R);
-        auto pair = [&](const float* src, int64_t st, int r, int i, uint64_t none) {
-          return r < nb && d < dim ? *reinterpret_cast<const uint64_t*>(src + (int64_t)(b * R + r) * st + d + 2 * i) : none;
-        };
-        const float bs = lane < nb ? bsrc[(int64_t)(b * R + lane) * a.heads] : 0.f, gs = !CHAN && lane < nb ? gsrc[(int64_t)(b * R + lane) * a.g_row] : 1.f;
+        float bs, gs;
+        if (AHEAD) bs = bs0, gs = gs0;
+        else scalars(b, bs, gs);
         float x[2][32];   // k with k and the diagonal's first half; q with k and its second
 #pragma unroll
         for (int i = 0; i < NP; ++i) {   // channels in NP passes, for the registers
-          uint64_t k[R], g[R], q[R];
+          Rows k, g, q;
+          if (AHEAD && !i) {
 #pragma unroll
-          for (int r = 0; r < R; ++r) {
-            k[r] = pair(ksrc, qk, r, i, 0);
-            q[r] = pair(qsrc, qk, r, i, 0);
-            g[r] = CHAN ? pair(gsrc, a.g_row, r, i, f2::both(1.f)) : f2::both(__shfl_sync(0xffffffffu, gs, r));
+            for (int r = 0; r < R; ++r) k[r] = k0[r], q[r] = q0[r], g[r] = CHAN ? g0[r] : f2::both(__shfl_sync(0xffffffffu, gs, r));
+          } else {
+            pieces(b, i, k, g, q, gs);
           }
           auto add = [&](float& to, uint64_t a, uint64_t b) {
             const float sum = f2::sum(f2::mul(a, b));
@@ -489,7 +516,7 @@ __global__ void __launch_bounds__(db_threads(LG, CTAS), CTAS) delta_block_kernel
         }
         const float kk = db_reduce(x[0], lane), qq = db_reduce(x[1], lane);
         // T = (1 + diag(b) (k with k))^-1 and B = (q with k) T, a column a lane
-        float* tri = tris + (p % 3 * per_round + mine) * kDbTri;
+        float* tri = tris + (p % 3 * per_round + own) * kDbTri;
         float t[R];
 #pragma unroll
         for (int i = 0; i < R; ++i) t[i] = lane == i ? 1.f : 0.f;
@@ -528,6 +555,7 @@ __global__ void __launch_bounds__(db_threads(LG, CTAS), CTAS) delta_block_kernel
       // write there.  (A release of the main warps' own waits for their outputs' stores: one sequence of 2 000 rows, keys of 64, 280 us instead of 254.)
       if (p >= 2 && p + 1 < rounds) db_sync<READ>(kRead + (p & 1));
       db_cluster_arrive();
+      if (AHEAD) fetch(b + per_round);
       db_cluster_wait();
     }
     return;
