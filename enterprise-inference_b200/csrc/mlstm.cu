@@ -214,13 +214,17 @@ int mlstm_scan(bool f32, const void* qkv, int64_t ld, int q_off, int k_off, int 
   B200_REQUIRE(positions && seq_start && seq_slots && state, B200_ERR_INVALID, "mlstm_scan: null argument");
   MlstmArgs a = {qkv, gates, positions, seq_start, seq_slots, state, out, ld, slot_stride, q_off, k_off, v_off, heads, dim, vd, 1.0f / sqrtf((float)dim), -0.5 * log2((double)dim), 0, 0, 0, 0};
   mlstm_walk_widths(a, f32);
-  // Steps of a few bf16 portions on the tensor cores where they are long, in segments from 193 rows on and in chunks from 97.  While all CTAs fit the device
-  // at once, the segments' kernel takes the short portions itself; beyond that each kind of portion has its kernel (two sequences of 50 rows, 8 heads of
-  // 128 x 256: 20 us, in one kernel 24).  One launch for all costs portions of 97 to 192 rows, whose length is known on the device only, 0.8 us of 12 to 1.3 of 16.6;
-  // a launch more would cost every call 2 us of host time.
-  // More sequences than four go to the walk alone (64 of one row 36 us; longer portions of many sequences in segments have not been measured).
+  // Steps of a few bf16 portions on the tensor cores where they are long.  While a launch in segments has no more CTAs than there are SMs, one launch takes all:
+  // segments from 193 rows on, chunks from 97, the walk below.  (Portions of 97 to 192 rows, whose length is known on the device only, 18.5 -> 19.7 us for it, of 69
+  // rows with keys of 64 15.3 -> 16.5; 2 048 rows of 8 heads, 128 x 256, 144 -> 59.)
+  // Beyond that chunks for all long portions, two CTAs an SM, and while these fit at once the chunk kernel walks the short portions itself; else each kernel
+  // takes its portions (64 rows of four sequences: 15.0 us, in one kernel 23.1: the idle half of each cluster holds up the next).  Segments there too were a
+  // third launch, 5 us of host time for a call of 20 rows, and slower for portions of some hundred rows (three of 400 together, 4 heads, 29 -> 50 us); they won
+  // from about 200 rows a portion on (four of 1 000, 8 heads, 111 -> 97), which the host does not know.
+  // More sequences than four go to the walk alone (64 of one row 36 us; longer portions of many sequences on the tensor cores have not been measured).
   if (!f32 && !single_rows && S <= 4 && mlstm_chunk_supported(a)) {
-    a.both = mlstm_chunk_ctas(a, S) > kNumSMs;
+    if (mlstm_segment_ctas(a, S) <= kNumSMs) return mlstm_segments(a, S, s);
+    a.both = mlstm_chunk_ctas(a, S) > 2 * kNumSMs;
     if (const int e = mlstm_chunk(a, S, s)) return e;
     if (!a.both) return B200_OK;
     const PdlScope after_chunks;

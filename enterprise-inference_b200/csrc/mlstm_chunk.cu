@@ -128,12 +128,11 @@ __global__ void __launch_bounds__(kSgAll, 1) mlstm_segment_kernel(const MlstmArg
   const int heads = a.heads, dim = a.dim, vd = a.vd, nz = (vd + kScanCols - 1) / kScanCols;
   const int start = a.seq_start[s], n_rows = a.seq_start[s + 1] - start;
   if (n_rows < kChunkFrom) {   // (nothing to do at all among them) two CTAs take the cluster's columns
-    if (rank < 2 && 2 * cb + rank < nz && !a.both && tid < kScanThreads)
+    if (rank < 2 && 2 * cb + rank < nz && tid < kScanThreads)
       mlstm_walk<__nv_bfloat16, KS / 4>(a, reinterpret_cast<float*>(raw), 2 * cb + rank, nz);
     return;
   }
   if (n_rows < kSegmentFrom) {   // every CTA sixteen columns
-    if (a.both) return;
     if (warp < kMcGate) {
       asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSgRegsChunks));
       mlstm_chunks<KS, 1>(a, raw, blockIdx.z);
@@ -702,14 +701,15 @@ __global__ void __launch_bounds__(kSgAll, 1) mlstm_segment_kernel(const MlstmArg
   __syncthreads();
 }
 
-// Chunks on their own, for steps whose portions take a kernel each: two CTAs share an SM where there are more of them than SMs.
-template <int KS, int CTAS>
-__global__ void __launch_bounds__(kMcThreads, CTAS) mlstm_chunk_kernel(const MlstmArgs a) {
+// Chunks on their own, two CTAs an SM, for steps of more CTAs than SMs; short portions are the pair's first CTA's, with both halves' columns, or the walk's kernel's.
+template <int KS>
+__global__ void __launch_bounds__(kMcThreads, 2) mlstm_chunk_kernel(const MlstmArgs a) {
   extern __shared__ __align__(16) unsigned char raw[];
   pdl_wait();
   pdl_launch_dependents();
   const int n_rows = a.seq_start[blockIdx.x + 1] - a.seq_start[blockIdx.x];
-  if (n_rows >= kChunkFrom && n_rows < kSegmentFrom) mlstm_chunks<KS, 0>(a, raw, blockIdx.z);
+  if (n_rows >= kChunkFrom) mlstm_chunks<KS, 0>(a, raw, blockIdx.z);
+  else if ((blockIdx.z & 1) == 0 && !a.both) mlstm_walk<__nv_bfloat16, KS / 4>(a, reinterpret_cast<float*>(raw), blockIdx.z >> 1, gridDim.z >> 1);
 }
 
 }  // namespace
@@ -719,28 +719,39 @@ bool mlstm_chunk_supported(const MlstmArgs& a) {
   return a.dim > 0 && a.dim <= 128 && a.dim % 8 == 0 && a.vd % 8 == 0 && a.ld % 8 == 0 && (a.q_off | a.k_off | a.v_off) % 8 == 0 &&
          reinterpret_cast<uintptr_t>(a.qkv) % 16 == 0;
 }
-// CTAs of a launch
-int64_t mlstm_chunk_ctas(const MlstmArgs& a, int S) { return (int64_t)S * a.heads * kSgCluster * ((a.vd + kSgCols - 1) / kSgCols); }
+// A launch's CTAs in segments, in chunks
+int64_t mlstm_segment_ctas(const MlstmArgs& a, int S) { return (int64_t)S * a.heads * kSgCluster * ((a.vd + kSgCols - 1) / kSgCols); }
+int64_t mlstm_chunk_ctas(const MlstmArgs& a, int S) { return (int64_t)S * a.heads * 2 * mlstm_col_blocks(a.vd); }
 
-int mlstm_chunk(MlstmArgs a, int S, cudaStream_t s) {
+int mlstm_segments(MlstmArgs a, int S, cudaStream_t s) {
   if (const int e = wait_status()) return e;
   a.vec_out = reinterpret_cast<uintptr_t>(a.out) % 16 == 0;
   const dim3 grid(S, a.heads, kSgCluster * ((a.vd + kSgCols - 1) / kSgCols)), block(kSgAll), cluster(1, 1, kSgCluster);
 #define SEGMENTS(K)                                                                                            \
   do {                                                                                                         \
-    static bool done[2][64] = {};                                                                              \
+    static bool done[64] = {};                                                                                 \
     constexpr size_t smem = std::max({(size_t)SgSmem<K>::bytes, sizeof(McSmem<K>), (size_t)ml_floats(K / 4) * 4});   \
-    if (a.both) {                                                                                              \
-      B200_CUDA(ensure_dynamic_smem(mlstm_chunk_kernel<K, 2>, (int)sizeof(McSmem<K>), done[1]));               \
-      B200_CUDA(launch_cluster(mlstm_chunk_kernel<K, 2>, dim3(S, a.heads, 2 * mlstm_col_blocks(a.vd)), dim3(kMcThreads), sizeof(McSmem<K>), s, dim3(1, 1, 2), a));   \
-    }                                                                                                          \
-    const PdlScope after_chunks(a.both);                                                                       \
-    B200_CUDA(ensure_dynamic_smem(mlstm_segment_kernel<K>, (int)smem, done[0]));                               \
+    B200_CUDA(ensure_dynamic_smem(mlstm_segment_kernel<K>, (int)smem, done));                                  \
     B200_CUDA(launch_cluster(mlstm_segment_kernel<K>, grid, block, smem, s, cluster, a, wait_status_word()));  \
   } while (0)
   if (a.dim <= 64) SEGMENTS(4);
   else SEGMENTS(8);
 #undef SEGMENTS
+  return B200_OK;
+}
+
+int mlstm_chunk(const MlstmArgs& a, int S, cudaStream_t s) {
+  const dim3 grid(S, a.heads, 2 * mlstm_col_blocks(a.vd)), block(kMcThreads), cluster(1, 1, 2);
+#define CHUNK(K)                                                                                               \
+  do {                                                                                                         \
+    static bool done[64] = {};                                                                                 \
+    constexpr size_t smem = std::max(sizeof(McSmem<K>), (size_t)ml_floats(K / 4) * 4);   /* chunks; walk */         \
+    B200_CUDA(ensure_dynamic_smem(mlstm_chunk_kernel<K>, (int)smem, done));                                    \
+    B200_CUDA(launch_cluster(mlstm_chunk_kernel<K>, grid, block, smem, s, cluster, a));                        \
+  } while (0)
+  if (a.dim <= 64) CHUNK(4);
+  else CHUNK(8);
+#undef CHUNK
   return B200_OK;
 }
 

@@ -20,13 +20,15 @@ struct MlstmArgs {
   int vec;        // rows of q and k can be read 16 bytes at a time
   int vec_state;  // state columns 8 bytes at a time
   int vec_out;    // outputs 16 bytes at a time
-  int both;       // the walk's, the chunks' and the segments' kernel are all launched, each for its portions
+  int both;       // the walk's and the chunks' kernel are both launched, each for its portions
 };
 
 // bf16 rows on the tensor cores (mlstm_chunk.cu)
 bool mlstm_chunk_supported(const MlstmArgs& a);
+int64_t mlstm_segment_ctas(const MlstmArgs& a, int S);
 int64_t mlstm_chunk_ctas(const MlstmArgs& a, int S);
-int mlstm_chunk(MlstmArgs a, int S, cudaStream_t s);
+int mlstm_segments(MlstmArgs a, int S, cudaStream_t s);
+int mlstm_chunk(const MlstmArgs& a, int S, cudaStream_t s);
 
 namespace {
 
