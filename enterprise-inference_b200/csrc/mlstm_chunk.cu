@@ -8,7 +8,8 @@
 // A cluster of four CTAs takes (sequence, head, 64 value columns), up to 1 024 rows at a time, each CTA a segment of up to 256:
 //   1. sums F and maxima M of its gates; D = K^T (w V) with w_s = exp(i_s - F_s - M_L), the segment's own part of the state (M: dimensions, N: columns);
 //   2. outputs as attention within the segment: scores Q K^T in blocks of 128 rows x 128 keys, weighted by the exponentials under the diagonal, times V;
-//   3. every CTA reads the earlier segments' D over the cluster's shared memory and adds up its S_0 (the last one the state after all): Q S_0.
+//   3. every CTA reads the earlier segments' D from the output rows where they left it (their own, not written yet; it stays in L2) and adds up its S_0 (the last one
+//      the state after all): Q S_0.
 // Nothing walks from chunk to chunk.  Everything that was fp32 in the walk stays so in effect: sums F are taken in 64 bits (differences of large
 // sums), an fp32 operand (weights, w V, S_0) enters the bf16 MMA as three bf16 terms (24 bits) against rows that are bf16 to begin with, the small
 // terms first, accumulators are fp32 and given up for a new one every 64 rows of D and 128 keys.
@@ -20,7 +21,7 @@
 // segments on mma.sync took 103 us, because m16n8k16 takes 16 cycles of a scheduler here (three terms of everything: 92 000 cycles).
 // What bounds it now: the instructions of a round (45 000 issue slots a scheduler for two rounds, a third of the stalls are instruction fetches,
 // hence loops that stay loops, one copy of each phase), and the phases' latency, one CTA an SM.  2 048 rows of 8 heads, 128 x 256: 142 -> 57 us; 1 024: 73 -> 31;
-// 512: 38 -> 21; two sequences together 2 048: 146 -> 102; 8 000 rows 545 -> 220; 64 x 128: 114 -> 54.
+// 512: 38 -> 21; 8 000 rows 545 -> 220; 64 x 128: 114 -> 54.
 // Error of the results against 64 bits, over 32 cases: 5.1e-7 (chunks 5.6e-7), of the state 6.8e-8 (7.8e-8); scores in one accumulator would
 // make it 6.0e-7 (eight truncated sums of 16 dimensions), weights by expf 6.4e-7.
 // Tried: eight warps instead of sixteen 68 us; D over the cluster's shared memory 12 000 cycles a round instead of 4 000; the MMAs issued by a warp with rows 65 us.
