@@ -215,8 +215,8 @@ int mlstm_scan(bool f32, const void* qkv, int64_t ld, int q_off, int k_off, int 
   MlstmArgs a = {qkv, gates, positions, seq_start, seq_slots, state, out, ld, slot_stride, q_off, k_off, v_off, heads, dim, vd, 1.0f / sqrtf((float)dim), -0.5 * log2((double)dim), 0, 0, 0, 0};
   mlstm_walk_widths(a, f32);
   // Steps of a few bf16 portions on the tensor cores where they are long.  While a launch in segments has no more CTAs than there are SMs, one launch takes all:
-  // segments from 193 rows on, chunks from 97, the walk below.  (Portions of 97 to 192 rows, whose length is known on the device only, 18.5 -> 19.7 us for it, of 69
-  // rows with keys of 64 15.3 -> 16.5; 2 048 rows of 8 heads, 128 x 256, 144 -> 59.)
+  // segments from 193 rows on, chunks from 97, the walk below.  (Portions of 97 to 192 rows, whose length is known on the device only, 18.5 -> 19.7 us for it; with
+  // keys of 64 portions of 60 to 256 rows 8 to 11 % more (215 rows 17.3 -> 18.6), 300 rows 20.8 -> 18.6; 2 048 rows of 8 heads, 128 x 256, 144 -> 59.)
   // Beyond that chunks for all long portions, two CTAs an SM, and while these fit at once the chunk kernel walks the short portions itself; else each kernel
   // takes its portions (64 rows of four sequences: 15.0 us, in one kernel 23.1: the idle half of each cluster holds up the next).  Segments there too were a
   // third launch, 5 us of host time for a call of 20 rows, and slower for portions of some hundred rows (three of 400 together, 4 heads, 29 -> 50 us); they won
