@@ -411,7 +411,7 @@ int paged_attn_mma(const float* q, const __nv_bfloat16* kc, const __nv_bfloat16*
                    const int32_t* row_to_seq, const int32_t* ctx_lens, __nv_bfloat16* out, const int32_t* runs, const int32_t* n_runs, int T,
                    int heads, int kv_heads, int dim, int vdim, int block_size, float scale, const float* sink, cudaStream_t s,
                    int n_splits = 1, float* part = nullptr, int window = 0, const AttnExtra& ex = AttnExtra(), bool one_row_each = false);
-// grouped-query attention for heads of at most 128 entries on tcgen05, two tiles of 128 (row, head) pairs a CTA (attn_rows_tc.cu)
+// grouped-query attention for heads of 64 or 128 entries on tcgen05, two tiles of 128 (row, head) pairs a CTA (attn_rows_tc.cu)
 struct RunShare;   // runs.cuh
 int attn_rows_tc_rows(int T, int heads, int kv_heads);
 bool attn_rows_tc_supported(int heads, int kv_heads, int dim, int vdim, int block_size);
