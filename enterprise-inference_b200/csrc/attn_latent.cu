@@ -53,7 +53,8 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // NG: 16-column output groups per warp (rank <= 128 NG).  EX: score cap, distance bias, per-head gate and kept first keys of AttnExtra.
 // MANY: launched beside a tcgen05 kernel for its share of the runs, as many CTAs as fit the device, each of which walks over items; otherwise one
 // item a CTA (with the loops in every launch 128 decode rows took 65.2 us, without 64.3).
-template <int NG, bool EX, bool MANY>
+// LO: weights of 16 bits, in two bf16 terms, for long steps whose heads attn_rows_tc.cu had taken with such weights.
+template <int NG, bool EX, bool MANY, bool LO>
 __global__ void __launch_bounds__(kLaThreads, NG == 1 ? 4 : NG == 2 ? 3 : 2)
 latent_attn_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __restrict__ kc, const __nv_bfloat16* __restrict__ vc,
                        int kv_heads, const int32_t* __restrict__ block_table,
@@ -94,6 +95,7 @@ latent_attn_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __restr
   float* lrow = mrow + kLaPairs;
   int* ctxp = reinterpret_cast<int*>(lrow + kLaPairs);
   int* lop = ctxp + kLaPairs;   // the first key a pair sees (0 without a window)
+  __nv_bfloat16* Pl = reinterpret_cast<__nv_bfloat16*>(lop + kLaPairs);   // LO: [16][72], what rounding took from the weights
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid < kLaPairs) {
     const int i = i0 + tid;
@@ -194,6 +196,10 @@ latent_attn_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __restr
       const float sum = warp_sum(p0 + p1);
       Ps[row * kPsStride + lane] = __float2bfloat16_rn(p0);
       Ps[row * kPsStride + lane + 32] = __float2bfloat16_rn(p1);
+      if constexpr (LO) {
+        Pl[row * kPsStride + lane] = __float2bfloat16_rn(p0 - round_bf16(p0));
+        Pl[row * kPsStride + lane + 32] = __float2bfloat16_rn(p1 - round_bf16(p1));
+      }
       __syncwarp();
       if (lane == 0) {
         mrow[row] = m_new;
@@ -214,8 +220,9 @@ latent_attn_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __restr
       const __nv_bfloat16* vp = Vs + ((lane & 7) + ((lane >> 3) & 1) * 8) * vs + (lane >> 4) * 8;
 #pragma unroll
       for (int kk = 0; kk < kLaKeys / 16; ++kk) {
-        uint32_t a[4];
+        uint32_t a[4], al[4];
         ldsm_x4(a, ap + kk * 16);
+        if constexpr (LO) ldsm_x4(al, ap + (Pl - Ps) + kk * 16);
 #pragma unroll
         for (int cg = 0; cg < NG; ++cg) {
           const int col0 = (warp + kLaWarps * cg) * 16;
@@ -224,6 +231,10 @@ latent_attn_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __restr
             ldsm_x4_t(b, vp + kk * 16 * vs + col0);
             mma_bf16(o[cg][0], o[cg][1], o[cg][2], o[cg][3], a, b[0], b[1]);
             mma_bf16(o[cg][4], o[cg][5], o[cg][6], o[cg][7], a, b[2], b[3]);
+            if constexpr (LO) {
+              mma_bf16(o[cg][0], o[cg][1], o[cg][2], o[cg][3], al, b[0], b[1]);
+              mma_bf16(o[cg][4], o[cg][5], o[cg][6], o[cg][7], al, b[2], b[3]);
+            }
           }
         }
       }
@@ -373,32 +384,33 @@ bool paged_attn_mma_supported(int heads, int kv_heads, int dim, int vdim) {
 static int attn_mma_launch(const float* q, const __nv_bfloat16* kc, const __nv_bfloat16* vc, int kv_heads, const int32_t* block_table,
                            int bt_stride, const int32_t* row_to_seq, const int32_t* ctx_lens, __nv_bfloat16* out, const int32_t* runs,
                            const int32_t* n_runs, int T, int heads, int krow, int rank, int block_size, float scale, const float* sink,
-                           cudaStream_t s, int n_splits, float* part, int window, const AttnExtra& ex, const RunShare* share = nullptr) {
+                           cudaStream_t s, int n_splits, float* part, int window, const AttnExtra& ex, const RunShare* share = nullptr, bool lo = false) {
   if (n_splits < 1 || part == nullptr) n_splits = 1;
   B200_REQUIRE(n_splits <= kLaMaxSplits, B200_ERR_INVALID, "attention: %d splits (at most %d)", n_splits, kLaMaxSplits);
   B200_REQUIRE(reinterpret_cast<uintptr_t>(kc) % 16 == 0 && reinterpret_cast<uintptr_t>(vc) % 16 == 0, B200_ERR_INVALID,
                "attention: cache not 16-byte aligned");
-  const size_t smem = la_smem(krow, rank, vc != nullptr);
+  const size_t smem = la_smem(krow, rank, vc != nullptr) + (lo ? kLaPairs * kPsStride * 2 : 0);
   // a run has at most 16 rows, so a kv head's group has at most 16 G pairs: G chunks of 16
   // (for a share of the runs: one wave of CTAs)
   const int64_t wave = (int64_t)kNumSMs * std::max(1, std::min(4, (int)(224 * 1024 / (smem + 1024))));
   const dim3 grid = share ? dim3((unsigned)std::min<int64_t>((int64_t)T * heads * n_splits, wave)) : dim3(T, heads, n_splits), block(kLaThreads);
-#define LA2(NGV, EXV, MV)                                                                                                             \
+#define LA2(NGV, EXV, MV, LOV)                                                                                                             \
   do {                                                                                                                              \
     static bool done[64] = {};                                                                                                      \
-    if (smem > 48 * 1024) B200_CUDA(ensure_dynamic_smem(latent_attn_mma_kernel<NGV, EXV, MV>, 200 * 1024, done));                       \
-    B200_CUDA(launch(latent_attn_mma_kernel<NGV, EXV, MV>, grid, block, smem, s, q, kc, vc, kv_heads, block_table, bt_stride, row_to_seq, \
+    if (smem > 48 * 1024) B200_CUDA(ensure_dynamic_smem(latent_attn_mma_kernel<NGV, EXV, MV, LOV>, 200 * 1024, done));                       \
+    B200_CUDA(launch(latent_attn_mma_kernel<NGV, EXV, MV, LOV>, grid, block, smem, s, q, kc, vc, kv_heads, block_table, bt_stride, row_to_seq, \
                      ctx_lens, out, runs, n_runs, heads, krow, rank, block_size, scale, sink, n_splits, part, window, ex, share ? *share : RunShare())); \
   } while (0)
-#define LA(NGV, MV)                     \
-  do {                                  \
-    if (ex.any()) LA2(NGV, true, MV);   \
-    else LA2(NGV, false, MV);           \
+#define LA(NGV, MV, LOV)                     \
+  do {                                       \
+    if (ex.any()) LA2(NGV, true, MV, LOV);   \
+    else LA2(NGV, false, MV, LOV);           \
   } while (0)
-  if (share) LA(1, true);   // (rank <= 128: attn_rows_tc.cu's shapes)
-  else if (rank <= 128) LA(1, false);
-  else if (rank <= 256) LA(2, false);
-  else LA(4, false);
+  if (share) LA(1, true, false);   // (rank <= 128: attn_rows_tc.cu's shapes)
+  else if (lo) LA(1, false, true);
+  else if (rank <= 128) LA(1, false, false);
+  else if (rank <= 256) LA(2, false, false);
+  else LA(4, false, false);
 #undef LA
 #undef LA2
   if (n_splits > 1)
@@ -510,8 +522,8 @@ int paged_attn_mma(const float* q, const __nv_bfloat16* kc, const __nv_bfloat16*
   // and so do scales that are not positive (masks and maxima of the other kernel are those of the unscaled scores) and decode rows, which fill
   // G of an item's 256 pairs there (256 rows at contexts 300..600, 16 heads over 4: 184 us against 80).  Short steps stay here
   // altogether; others launch both kernels, which share the step's runs (runs.cuh), unless every row is known to be a sequence of its own
-  if (T > 128 && row_to_seq && !one_row_each && scale > 0.f && attn_rows_tc_supported(heads, kv_heads, dim, vdim, block_size) && at(q) % 16 == 0 &&
-      at(out) % 16 == 0 && at(part) % 8 == 0) {
+  const bool runs_of_rows = T > 128 && row_to_seq && !one_row_each && scale > 0.f && at(q) % 16 == 0 && at(out) % 16 == 0 && at(part) % 8 == 0;
+  if (runs_of_rows && attn_rows_tc_supported(heads, kv_heads, dim, vdim, block_size)) {
     RunShare share;
     const int rc = attn_rows_tc_runs(q, kc, vc, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, kv_heads, dim, vdim,
                                      block_size, scale, sink, s, n_splits, part, window, ex, &share);
@@ -521,7 +533,7 @@ int paged_attn_mma(const float* q, const __nv_bfloat16* kc, const __nv_bfloat16*
                            scale, sink, s, n_splits, part, window, ex, &share);
   }
   return attn_mma_launch(q, kc, vc, kv_heads, block_table, bt_stride, row_to_seq, ctx_lens, out, runs, n_runs, T, heads, dim, vdim, block_size,
-                         scale, sink, s, n_splits, part, window, ex);
+                         scale, sink, s, n_splits, part, window, ex, nullptr, runs_of_rows && attn_rows_tc_declined(heads, kv_heads, dim, vdim, block_size));
 }
 
 }  // namespace b200

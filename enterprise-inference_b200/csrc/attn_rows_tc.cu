@@ -605,12 +605,18 @@ int attn_rows_tc_rows(int T, int heads, int kv_heads) {
   return (int64_t)T * kv_heads < (int64_t)tile * kNumSMs ? tile : 2 * tile;
 }
 
+static bool ar_form(int heads, int kv_heads, int dim, int vdim, int block_size) {
+  return heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && heads / kv_heads <= 16 && dim % 16 == 0 && dim >= 16 && dim <= 128 && vdim % 16 == 0 &&
+         vdim >= 16 && vdim <= 128 && block_size > 0 && block_size % 64 == 0;
+}
 // Rows of keys and values are whole boxes of 64 columns.  Two runs over narrower value rows (400 and 420 rows of one sequence, 6 heads over 2, keys of 64, values
-// of 32, of which a box takes 64) ended in an illegal address, each behind some hundred other tests; alone the same call passes, and reading has not shown which access it was.  Such
-// heads take the mma.sync kernel of attn_latent.cu, which reads their rows through pointers.
+// of 32, of which a box takes 64) ended in an illegal address, each behind some hundred other tests; alone the same call passes, and reading has not shown which access
+// it was.  Such heads take the mma.sync kernel of attn_latent.cu, which reads their rows through pointers, with weights of 16 bits as here.
 bool attn_rows_tc_supported(int heads, int kv_heads, int dim, int vdim, int block_size) {
-  return heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && heads / kv_heads <= 16 && (dim == 64 || dim == 128) && (vdim == 64 || vdim == 128) &&
-         block_size > 0 && block_size % 64 == 0;
+  return ar_form(heads, kv_heads, dim, vdim, block_size) && dim % 64 == 0 && vdim % 64 == 0;
+}
+bool attn_rows_tc_declined(int heads, int kv_heads, int dim, int vdim, int block_size) {
+  return ar_form(heads, kv_heads, dim, vdim, block_size) && !(dim % 64 == 0 && vdim % 64 == 0);
 }
 
 // bf16 queries in rows of ldq, weights of 16 bits; plan: attn_prefill.cu's items of at most attn_rows_tc_rows rows
@@ -692,7 +698,7 @@ int attn_rows_tc_runs(const float* q, const __nv_bfloat16* kc, const __nv_bfloat
 
 }  // namespace b200
 
-// debug helper (not in the public header): does the kernel take heads of this form?
+// debug helper (not in the public header): heads of this form in long steps: 1 on this kernel, 2 on the mma.sync one with weights of 16 bits
 extern "C" __attribute__((visibility("default"))) int b200_debug_attn_rows_tc(int32_t heads, int32_t kv_heads, int32_t dim, int32_t vdim, int32_t block_size) {
-  return b200::attn_rows_tc_supported(heads, kv_heads, dim, vdim, block_size) ? 1 : 0;
+  return b200::attn_rows_tc_supported(heads, kv_heads, dim, vdim, block_size) ? 1 : b200::attn_rows_tc_declined(heads, kv_heads, dim, vdim, block_size) ? 2 : 0;
 }

@@ -415,6 +415,7 @@ int paged_attn_mma(const float* q, const __nv_bfloat16* kc, const __nv_bfloat16*
 struct RunShare;   // runs.cuh
 int attn_rows_tc_rows(int T, int heads, int kv_heads);
 bool attn_rows_tc_supported(int heads, int kv_heads, int dim, int vdim, int block_size);
+bool attn_rows_tc_declined(int heads, int kv_heads, int dim, int vdim, int block_size);   // heads whose long steps take attn_latent.cu's kernel with the same weights
 int attn_rows_tc_plan(const __nv_bfloat16* q, int64_t ldq, const __nv_bfloat16* kc, const __nv_bfloat16* vc, const int32_t* block_table, int bt_stride,
                       const int32_t* ctx_lens, __nv_bfloat16* out, int64_t ldo, int T, int heads, int kv_heads, int dim, int block_size, float scale,
                       const void* plan, cudaStream_t s);
