@@ -73,7 +73,7 @@ __device__ __forceinline__ float sg_exp2(double x) {
 __device__ __forceinline__ unsigned char* sg_at(unsigned char* x, int row, int piece) {
   return x + (piece >> 3) * kSgPanel + row * 128 + (((piece ^ row) & 7) << 4);
 }
-// barriers.  By the MMA warp: scores of a block, D of a half's rows, weights of a block multiplied, the last ones, Q S_0
+// barriers (what an MMA reads from shared memory is behind one whose arrivals follow the writes, copies included, and a fence to the async proxy).  By the MMA warp: scores of a block, D of a half's rows, weights of a block multiplied, the last ones, Q S_0
 // (sixteen warps wait); by those: a half of w V is there, weights of a block are, S_0 is there
 enum { kScores, kD, kPv, kPvLast, kQs, kWeighed, kWeights, kTerms, kBars };
 constexpr double kLog2e = 1.4426950408889634;
@@ -496,9 +496,12 @@ __global__ void __launch_bounds__(kSgAll, 1) mlstm_segment_kernel(const MlstmArg
       }
       wait(kScores);
       weights(step ? 1 : 0, step >> 1, step > 0);
+      if (step == 0) {   // q's second tile too, whose scores are issued behind these weights (k's and v's: kWeighed of the second 128 rows)
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        fence_async_smem();
+      }
       if (step != 1) arrive(kWeights);
       if (step == 0) {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
         sync();   // all rows
         part_of_n();
       }

@@ -171,6 +171,33 @@ def test_mlstm_segments(rows, heads, dim, vdim, off):
     assert (state[0] == 7.5).all()
 
 
+# Two row tiles a segment (513 rows: of 144), whole rounds and two of them, while another stream copies memory: a row that the products do not wait for
+# would come late.  The same bits as alone, whose results the test above holds to the oracle.
+@pytest.mark.parametrize("rows", [513, 1024, 2048])
+@pytest.mark.parametrize("dim", [64, 128])
+def test_mlstm_segments_beside_copies(rows, dim):
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    heads, vdim = 8, 256
+    g = torch.Generator(device=DEV).manual_seed(rows + dim)
+    hd, hv = heads * dim, heads * vdim
+    floats, ld = int(lib.b200_mlstm_state_floats(heads, dim, vdim)), 2 * hd + hv
+    x, gates = torch.randn(rows, ld, generator=g, device=DEV).to(torch.bfloat16), torch.randn(rows, 2 * heads, generator=g, device=DEV)
+    gates[:, heads:] = torch.nn.functional.logsigmoid(gates[:, heads:] + 3)
+    state, out = torch.zeros(1, floats, device=DEV), torch.empty(rows, hv, device=DEV)
+    ptd, std, sld = _i32(list(range(rows))), _i32([0, rows]), _i32([0])
+    big, side, outs = torch.empty(2, 1 << 28, dtype=torch.uint8, device=DEV), torch.cuda.Stream(), []
+    torch.cuda.synchronize()
+    for run in range(40):
+        if run:
+            with torch.cuda.stream(side):
+                big[1].copy_(big[0])
+        check(lib.b200_mlstm_scan(0, x.data_ptr(), ld, 0, hd, 2 * hd, gates.data_ptr(), ptd.data_ptr(), std.data_ptr(), sld.data_ptr(), state.data_ptr(),
+                                  floats, out.data_ptr(), 1, heads, dim, vdim, torch.cuda.current_stream().cuda_stream))
+        outs.append((out.clone(), state.clone()))
+    torch.cuda.synchronize()
+    assert torch.isfinite(outs[0][0]).all() and all(torch.equal(a, b) for o in outs[1:] for a, b in zip(o, outs[0]))
+
+
 @pytest.mark.parametrize("what", ["value", "key", "forget gate", "input gate"])
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
 @pytest.mark.parametrize("row", [0, 127, 200, 540])
