@@ -75,7 +75,7 @@ __device__ __forceinline__ unsigned char* sg_at(unsigned char* x, int row, int p
 }
 // barriers (what an MMA reads from shared memory is behind one whose arrivals follow the writes, copies included, and a fence to the async proxy).  By the MMA warp: scores of a block, D of a half's rows, weights of a block multiplied, the last ones, Q S_0
 // (sixteen warps wait); by those: a half of w V is there, weights of a block are, S_0 is there
-enum { kScores, kD, kPv, kPvLast, kQs, kWeighed, kWeights, kTerms, kBars };
+enum { kScores, kD, kPv, kPvLast, kQs, kEnd, kWeighed, kWeights, kTerms, kBars };   // kEnd: after a wait that ran out, every MMA issued
 constexpr double kLog2e = 1.4426950408889634;
 struct SgSmall {
   double F[kSgRows], M[kSgRows], G[kSgRows];   // sums, running maxima of G, i - F (M and G times log2 e)
@@ -240,6 +240,10 @@ __global__ void __launch_bounds__(kSgAll, 1) mlstm_segment_kernel(const MlstmArg
       }
     }
     __syncthreads();
+    if (mbar_wait.stop()) {   // a wait ran out (all roles are at their ends): what is in flight finishes before tensor and shared memory are given up
+      commit(one, sm.bar + kEnd);
+      mbar_wait.drain(sm.bar + kEnd, 0);
+    }
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm), "r"(512u));
     return;
   }
