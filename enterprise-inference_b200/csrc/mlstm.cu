@@ -206,6 +206,21 @@ static int mlstm_scan_t(const MlstmArgs& a, int S, bool single_rows, cudaStream_
   return B200_OK;
 }
 
+// Steps of a few bf16 portions on the tensor cores where they are long.  While all clusters of a launch in segments run at a time, one launch takes all:
+// segments from 193 rows on, chunks from 97, the walk below.  (36 clusters, 9 heads of 256 columns: 160 rows 33.7 us, in chunks 16.6; 300 rows 36.2 and 25.2; 2 048
+// rows 109 and 142, but the length is known on the device only.)  (Portions of 97 to 192 rows 18.5 -> 19.7 us for it; with
+// keys of 64 portions of 60 to 256 rows 8 to 11 % more (215 rows 17.3 -> 18.6), 300 rows 20.8 -> 18.6; 2 048 rows of 8 heads, 128 x 256, 144 -> 59.)
+// Beyond that chunks for all long portions, two CTAs an SM, and while these fit at once the chunk kernel walks the short portions itself; else each kernel
+// takes its portions (64 rows of four sequences: 15.0 us, in one kernel 23.1: the idle half of each cluster holds up the next).  Segments there too were a
+// third launch, 5 us of host time for a call of 20 rows, and slower for portions of some hundred rows (three of 400 together, 4 heads, 29 -> 50 us); they won
+// from about 200 rows a portion on (four of 1 000, 8 heads, 111 -> 97), which the host does not know.
+// More sequences than four go to the walk alone (64 of one row 36 us; longer portions of many sequences on the tensor cores have not been measured).
+enum class MlstmRoute { kWalk, kChunks, kSegments };
+static MlstmRoute mlstm_route(const MlstmArgs& a, int S, bool f32, bool single_rows) {
+  if (f32 || single_rows || S > 4 || !mlstm_chunk_supported(a)) return MlstmRoute::kWalk;
+  return mlstm_segments_fit(a, S) ? MlstmRoute::kSegments : MlstmRoute::kChunks;
+}
+
 int mlstm_scan(bool f32, const void* qkv, int64_t ld, int q_off, int k_off, int v_off, const float* gates, const int32_t* positions,
                const int32_t* seq_start, const int32_t* seq_slots, float* state, int64_t slot_stride, float* out, int S, int heads,
                int dim, int vd, cudaStream_t s, bool single_rows) {
@@ -214,16 +229,9 @@ int mlstm_scan(bool f32, const void* qkv, int64_t ld, int q_off, int k_off, int 
   B200_REQUIRE(positions && seq_start && seq_slots && state, B200_ERR_INVALID, "mlstm_scan: null argument");
   MlstmArgs a = {qkv, gates, positions, seq_start, seq_slots, state, out, ld, slot_stride, q_off, k_off, v_off, heads, dim, vd, 1.0f / sqrtf((float)dim), -0.5 * log2((double)dim), 0, 0, 0, 0};
   mlstm_walk_widths(a, f32);
-  // Steps of a few bf16 portions on the tensor cores where they are long.  While a launch in segments has no more CTAs than there are SMs, one launch takes all:
-  // segments from 193 rows on, chunks from 97, the walk below.  (Portions of 97 to 192 rows, whose length is known on the device only, 18.5 -> 19.7 us for it; with
-  // keys of 64 portions of 60 to 256 rows 8 to 11 % more (215 rows 17.3 -> 18.6), 300 rows 20.8 -> 18.6; 2 048 rows of 8 heads, 128 x 256, 144 -> 59.)
-  // Beyond that chunks for all long portions, two CTAs an SM, and while these fit at once the chunk kernel walks the short portions itself; else each kernel
-  // takes its portions (64 rows of four sequences: 15.0 us, in one kernel 23.1: the idle half of each cluster holds up the next).  Segments there too were a
-  // third launch, 5 us of host time for a call of 20 rows, and slower for portions of some hundred rows (three of 400 together, 4 heads, 29 -> 50 us); they won
-  // from about 200 rows a portion on (four of 1 000, 8 heads, 111 -> 97), which the host does not know.
-  // More sequences than four go to the walk alone (64 of one row 36 us; longer portions of many sequences on the tensor cores have not been measured).
-  if (!f32 && !single_rows && S <= 4 && mlstm_chunk_supported(a)) {
-    if (mlstm_segment_ctas(a, S) <= kNumSMs) return mlstm_segments(a, S, s);
+  const MlstmRoute route = mlstm_route(a, S, f32, single_rows);
+  if (route == MlstmRoute::kSegments) return mlstm_segments(a, S, s);
+  if (route == MlstmRoute::kChunks) {
     a.both = mlstm_chunk_ctas(a, S) > 2 * kNumSMs;
     if (const int e = mlstm_chunk(a, S, s)) return e;
     if (!a.both) return B200_OK;
@@ -246,3 +254,12 @@ int head_norm_gate(bool f32, const float* o, const float* w, const void* gate, i
 }
 
 }  // namespace b200
+
+// debug helper (not in the public header): how a step of bf16 rows goes, with everything aligned (0 the walk alone, 1 chunks, 2 segments)
+extern "C" __attribute__((visibility("default"))) int b200_debug_mlstm_route(int32_t n_seqs, int32_t heads, int32_t dim, int32_t vdim) {
+  using namespace b200;
+  MlstmArgs a = {};
+  a.qkv = reinterpret_cast<const void*>(64);
+  a.heads = heads, a.dim = dim, a.vd = vdim;
+  return (int)mlstm_route(a, n_seqs, false, false);
+}

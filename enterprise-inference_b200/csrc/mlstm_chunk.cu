@@ -40,6 +40,7 @@ namespace {
 using namespace tc;
 
 constexpr int kSgCluster = 4, kSgRows = 256, kSgCols = 64;   // CTAs of a cluster; rows of a segment; value columns
+constexpr int kSgResident = 33;   // clusters of four CTAs, one an SM, that run at a time (cudaOccupancyMaxActiveClusters: 132 of the 148 SMs)
 constexpr int kSgThreads = 512, kSgAll = kSgThreads + 128;   // sixteen warps, and a group of four of which one issues the MMAs
 // registers a thread: 640 threads are launched with 96 each; four warps give what the sixteen others take (16 x 104 + 4 x 64 = 20 x 96)
 constexpr int kSgRegs = 104, kSgRegsMma = 64;
@@ -727,8 +728,8 @@ bool mlstm_chunk_supported(const MlstmArgs& a) {
   return a.dim > 0 && a.dim <= 128 && a.dim % 8 == 0 && a.vd % 8 == 0 && a.ld % 8 == 0 && (a.q_off | a.k_off | a.v_off) % 8 == 0 &&
          reinterpret_cast<uintptr_t>(a.qkv) % 16 == 0;
 }
-// A launch's CTAs in segments, in chunks
-int64_t mlstm_segment_ctas(const MlstmArgs& a, int S) { return (int64_t)S * a.heads * kSgCluster * ((a.vd + kSgCols - 1) / kSgCols); }
+// Are all clusters of a launch in segments on the device at a time?  A launch's CTAs in chunks
+bool mlstm_segments_fit(const MlstmArgs& a, int S) { return (int64_t)S * a.heads * ((a.vd + kSgCols - 1) / kSgCols) <= kSgResident; }
 int64_t mlstm_chunk_ctas(const MlstmArgs& a, int S) { return (int64_t)S * a.heads * 2 * mlstm_col_blocks(a.vd); }
 
 int mlstm_segments(MlstmArgs a, int S, cudaStream_t s) {

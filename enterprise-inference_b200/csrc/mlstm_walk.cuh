@@ -25,7 +25,7 @@ struct MlstmArgs {
 
 // bf16 rows on the tensor cores (mlstm_chunk.cu)
 bool mlstm_chunk_supported(const MlstmArgs& a);
-int64_t mlstm_segment_ctas(const MlstmArgs& a, int S);
+bool mlstm_segments_fit(const MlstmArgs& a, int S);
 int64_t mlstm_chunk_ctas(const MlstmArgs& a, int S);
 int mlstm_segments(MlstmArgs a, int S, cudaStream_t s);
 int mlstm_chunk(const MlstmArgs& a, int S, cudaStream_t s);
