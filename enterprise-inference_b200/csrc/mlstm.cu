@@ -210,7 +210,7 @@ static int mlstm_scan_t(const MlstmArgs& a, int S, bool single_rows, cudaStream_
 // segments from 193 rows on, chunks from 97, the walk below.  (36 clusters, 9 heads of 256 columns: 160 rows 33.7 us, in chunks 16.6; 300 rows 36.2 and 25.2; 2 048
 // rows 109 and 142, but the length is known on the device only.)  (Portions of 97 to 192 rows 18.5 -> 19.7 us for it; with
 // keys of 64 portions of 60 to 256 rows 8 to 11 % more (215 rows 17.3 -> 18.6), 300 rows 20.8 -> 18.6; 2 048 rows of 8 heads, 128 x 256, 144 -> 59.)
-// Beyond that chunks for all long portions, two CTAs an SM, and while these fit at once the chunk kernel walks the short portions itself; else each kernel
+// Beyond that chunks for all long portions, one or two CTAs an SM, and while these fit at once the chunk kernel walks the short portions itself; else each kernel
 // takes its portions (64 rows of four sequences: 15.0 us, in one kernel 23.1: the idle half of each cluster holds up the next).  Segments there too were a
 // third launch, 5 us of host time for a call of 20 rows, and slower for portions of some hundred rows (three of 400 together, 4 heads, 29 -> 50 us); they won
 // from about 200 rows a portion on (four of 1 000, 8 heads, 111 -> 97), which the host does not know.
