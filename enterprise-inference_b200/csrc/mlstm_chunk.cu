@@ -493,6 +493,10 @@ __global__ void __launch_bounds__(kSgAll, 1) mlstm_segment_kernel(const MlstmArg
     float* scratch = a.out + ((int64_t)(start + base) * heads + h) * vd + jb;   // of the round's first segment
     const int64_t segment = (int64_t)SL * heads * vd;
     auto place = [&](int j) { return (int64_t)(j * 32 + (tid >> 4)) * heads * vd + (tid & 15) * 4; };
+    auto place_of = [&](int j) {   // the same of `width` columns (a multiple of 8), whose 128 rows hold what 128 dimensions of them take
+      const int pieces = width >> 2, at = (part * 4 + j) * 128 + ml;
+      return (int64_t)(at / pieces) * heads * vd + at % pieces * 4;
+    };
 #pragma unroll 1
     for (int step = 0; step < (two ? 3 : 1); ++step) {
       if (step < 2) {
@@ -529,7 +533,8 @@ __global__ void __launch_bounds__(kSgAll, 1) mlstm_segment_kernel(const MlstmArg
             if (sm.odd_from[part * 16 + j] < kSgRows) D[j] = NAN;
         }
         // D: kept in shared memory and, for the segments behind, where this segment's first outputs will be (all 128 rows are there then; a cluster's
-        // shared memory is read at 8 bytes a cycle, L2 at 30).  A thread's four values side by side, or (fewer columns) where they would be as outputs
+        // shared memory is read at 8 bytes a cycle, L2 at 30).  Pieces of four values, a warp's side by side (each where its outputs would be: one portion of 300 rows, 8
+        // heads of 40 columns, 33.7 us one by one, 20.8 so); one by one where outputs do not start at 16-byte addresses
         if (rank == last) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) X[j * kSgThreads + tid] = make_float4(D[4 * j], D[4 * j + 1], D[4 * j + 2], D[4 * j + 3]);
@@ -537,6 +542,10 @@ __global__ void __launch_bounds__(kSgAll, 1) mlstm_segment_kernel(const MlstmArg
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             *reinterpret_cast<float4*>(scratch + rank * segment + place(j)) = make_float4(D[4 * j], D[4 * j + 1], D[4 * j + 2], D[4 * j + 3]);
+        } else if (a.vec_out) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (4 * j < cols) *reinterpret_cast<float4*>(scratch + rank * segment + place_of(j)) = make_float4(D[4 * j], D[4 * j + 1], D[4 * j + 2], D[4 * j + 3]);
         } else if (ml < dim) {
 #pragma unroll
           for (int j = 0; j < 16; ++j)
@@ -568,6 +577,10 @@ __global__ void __launch_bounds__(kSgAll, 1) mlstm_segment_kernel(const MlstmArg
         if (wide) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) x[j] = __ldcg(reinterpret_cast<const float4*>(scratch + i * segment + place(j)));
+        } else if (a.vec_out) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            x[j] = 4 * j < cols ? __ldcg(reinterpret_cast<const float4*>(scratch + i * segment + place_of(j))) : make_float4(0.f, 0.f, 0.f, 0.f);
         } else {
           float y[16];
 #pragma unroll
