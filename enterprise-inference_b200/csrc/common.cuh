@@ -480,7 +480,7 @@ int mlstm_col_blocks(int vd);
 int64_t mlstm_state_floats(int heads, int dim, int vd);
 int mlstm_scan(bool f32, const void* qkv, int64_t ld, int q_off, int k_off, int v_off, const float* gates, const int32_t* positions,
                const int32_t* seq_start, const int32_t* seq_slots, float* state, int64_t slot_stride, float* out, int S, int heads,
-               int dim, int vd, cudaStream_t s, bool single_rows = false);   // single_rows: every sequence of the step has one row
+               int dim, int vd, cudaStream_t s, int rows = 0);   // rows: of the step, where the caller knows them
 int head_norm_gate(bool f32, const float* o, const float* w, const void* gate, int64_t ldg, void* out, int T, int heads, int vd, float eps,
                    cudaStream_t s, bool gate_silu = false);   // gate_silu: times silu(gate) instead of sigmoid(gate)
 // post-norm layer form (postnorm.cu): layer norm with bias after the sum; attention whose values are its raw keys with per-head

@@ -208,28 +208,31 @@ static int mlstm_scan_t(const MlstmArgs& a, int S, bool single_rows, cudaStream_
 
 // Steps of a few bf16 portions on the tensor cores where they are long.  While all clusters of a launch in segments run at a time, one launch takes all:
 // segments from 193 rows on, chunks from 97, the walk below.  (36 clusters, 9 heads of 256 columns: 160 rows 33.7 us, in chunks 16.6; 300 rows 36.2 and 25.2; 2 048
-// rows 109 and 142, but the length is known on the device only.)  (Portions of 97 to 192 rows 18.5 -> 19.7 us for it; with
-// keys of 64 portions of 60 to 256 rows 8 to 11 % more (215 rows 17.3 -> 18.6), 300 rows 20.8 -> 18.6; 2 048 rows of 8 heads, 128 x 256, 144 -> 59.)
+// rows 109 and 142, but the length is known on the device only.)
+// Where the rows of the step are known to be too few for a long portion, chunks and walk are launched by themselves: in the segments' launch (us, in a graph, 8 heads)
+// 2 rows 5.3 instead of 5.0, 140 rows 17.8 and 16.5 (128 x 256); 2 rows 4.9 and 4.3, 69 rows 14.7 and 13.5, 215 rows 18.6 and 17.3 (64 x 128).  Segments pay from
+// 193 rows (215 rows 20.1, in chunks 20.8), with keys of 64 from 257 (300 rows 18.6 and 20.8); 2 048 rows of 128 x 256 58 and 142.
 // Beyond that chunks for all long portions, one or two CTAs an SM, and while these fit at once the chunk kernel walks the short portions itself; else each kernel
 // takes its portions (64 rows of four sequences: 15.0 us, in one kernel 23.1: the idle half of each cluster holds up the next).  Segments there too were a
 // third launch, 5 us of host time for a call of 20 rows, and slower for portions of some hundred rows (three of 400 together, 4 heads, 29 -> 50 us); they won
 // from about 200 rows a portion on (four of 1 000, 8 heads, 111 -> 97), which the host does not know.
 // More sequences than four go to the walk alone (64 of one row 36 us; longer portions of many sequences on the tensor cores have not been measured).
 enum class MlstmRoute { kWalk, kChunks, kSegments };
-static MlstmRoute mlstm_route(const MlstmArgs& a, int S, bool f32, bool single_rows) {
-  if (f32 || single_rows || S > 4 || !mlstm_chunk_supported(a)) return MlstmRoute::kWalk;
-  return mlstm_segments_fit(a, S) ? MlstmRoute::kSegments : MlstmRoute::kChunks;
+static MlstmRoute mlstm_route(const MlstmArgs& a, int S, bool f32, int rows) {   // rows 0: not known
+  if (f32 || rows == S || S > 4 || !mlstm_chunk_supported(a)) return MlstmRoute::kWalk;
+  const bool too_few = rows > 0 && rows - S + 1 < (a.dim <= 64 ? 257 : kSegmentFrom);
+  return mlstm_segments_fit(a, S) && !too_few ? MlstmRoute::kSegments : MlstmRoute::kChunks;
 }
 
 int mlstm_scan(bool f32, const void* qkv, int64_t ld, int q_off, int k_off, int v_off, const float* gates, const int32_t* positions,
                const int32_t* seq_start, const int32_t* seq_slots, float* state, int64_t slot_stride, float* out, int S, int heads,
-               int dim, int vd, cudaStream_t s, bool single_rows) {
+               int dim, int vd, cudaStream_t s, int rows) {
   if (S == 0) return B200_OK;
   B200_REQUIRE(dim > 0 && dim <= 256 && vd > 0, B200_ERR_UNSUPPORTED, "mlstm_scan: key size %d outside (0, 256]", dim);
   B200_REQUIRE(positions && seq_start && seq_slots && state, B200_ERR_INVALID, "mlstm_scan: null argument");
   MlstmArgs a = {qkv, gates, positions, seq_start, seq_slots, state, out, ld, slot_stride, q_off, k_off, v_off, heads, dim, vd, 1.0f / sqrtf((float)dim), -0.5 * log2((double)dim), 0, 0, 0, 0};
   mlstm_walk_widths(a, f32);
-  const MlstmRoute route = mlstm_route(a, S, f32, single_rows);
+  const MlstmRoute route = mlstm_route(a, S, f32, rows);
   if (route == MlstmRoute::kSegments) return mlstm_segments(a, S, s);
   if (route == MlstmRoute::kChunks) {
     a.both = mlstm_chunk_ctas(a, S) > 2 * kNumSMs;
@@ -238,7 +241,7 @@ int mlstm_scan(bool f32, const void* qkv, int64_t ld, int q_off, int k_off, int 
     const PdlScope after_chunks;
     return mlstm_scan_t<__nv_bfloat16>(a, S, false, s);
   }
-  return f32 ? mlstm_scan_t<float>(a, S, single_rows, s) : mlstm_scan_t<__nv_bfloat16>(a, S, single_rows, s);
+  return f32 ? mlstm_scan_t<float>(a, S, rows == S, s) : mlstm_scan_t<__nv_bfloat16>(a, S, rows == S, s);
 }
 
 int head_norm_gate(bool f32, const float* o, const float* w, const void* gate, int64_t ldg, void* out, int T, int heads, int vd, float eps,
@@ -255,11 +258,11 @@ int head_norm_gate(bool f32, const float* o, const float* w, const void* gate, i
 
 }  // namespace b200
 
-// debug helper (not in the public header): how a step of bf16 rows goes, with everything aligned (0 the walk alone, 1 chunks, 2 segments)
-extern "C" __attribute__((visibility("default"))) int b200_debug_mlstm_route(int32_t n_seqs, int32_t heads, int32_t dim, int32_t vdim) {
+// debug helper (not in the public header): how a step of bf16 rows (0: not known how many) goes, with everything aligned (0 the walk alone, 1 chunks, 2 segments)
+extern "C" __attribute__((visibility("default"))) int b200_debug_mlstm_route(int32_t n_seqs, int32_t heads, int32_t dim, int32_t vdim, int32_t rows) {
   using namespace b200;
   MlstmArgs a = {};
   a.qkv = reinterpret_cast<const void*>(64);
   a.heads = heads, a.dim = dim, a.vd = vdim;
-  return (int)mlstm_route(a, n_seqs, false, false);
+  return (int)mlstm_route(a, n_seqs, false, rows);
 }

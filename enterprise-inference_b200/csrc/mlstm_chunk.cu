@@ -533,8 +533,8 @@ __global__ void __launch_bounds__(kSgAll, 1) mlstm_segment_kernel(const MlstmArg
             if (sm.odd_from[part * 16 + j] < kSgRows) D[j] = NAN;
         }
         // D: kept in shared memory and, for the segments behind, where this segment's first outputs will be (all 128 rows are there then; a cluster's
-        // shared memory is read at 8 bytes a cycle, L2 at 30).  Pieces of four values, a warp's side by side (each where its outputs would be: one portion of 300 rows, 8
-        // heads of 40 columns, 33.7 us one by one, 20.8 so); one by one where outputs do not start at 16-byte addresses
+        // shared memory is read at 8 bytes a cycle, L2 at 30).  In pieces of four values, a warp's side by side (value by value, in rows far apart, one portion of 300
+        // rows, 8 heads of 40 columns, 33.7 us, so 20.8); value by value only where outputs do not start at 16-byte addresses
         if (rank == last) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) X[j * kSgThreads + tid] = make_float4(D[4 * j], D[4 * j + 1], D[4 * j + 2], D[4 * j + 3]);
