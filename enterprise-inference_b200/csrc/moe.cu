@@ -544,10 +544,12 @@ static int moe_experts_tc(const __nv_bfloat16* x, const __nv_bfloat16* w_gu, con
   B200_REQUIRE(smem_grp <= 200 * 1024, B200_ERR_UNSUPPORTED, "experts: %d experts exceed the grouping kernel", experts);
   static bool done_grp[64] = {};
   if (smem_grp > 40 * 1024) B200_CUDA(ensure_dynamic_smem(moe_group_gather_kernel, 200 * 1024, done_grp));
-  // about 16 rows a CTA, and no more CTAs than SMs: a second CTA on an SM counts the pairs once more and copies no faster.  The whole
-  // layer, against 64 rows and four CTAs per SM: 700 rows x 4 of 32 experts 112.7 -> 106.0 us, 600 x 2 of 16 40.3 -> 36.8, 500 x 8 of
-  // 64 264 -> 256, 2 048 x 4 of 32 alike; at three CTAs to two SMs the last takes 159 us instead of 154.
-  const int64_t per = std::max<int64_t>(1, std::min<int64_t>((int64_t)T * top / (16 * (int64_t)experts), kNumSMs / experts));
+  // About 16 rows a CTA while there are no more CTAs than SMs, beyond that (up to four per SM) 64: a second CTA on an SM counts the pairs once more, but an expert that
+  // most tokens choose is copied by its own CTAs alone.  The whole layer, against 64 rows throughout: 700 rows x 4 of 32 experts 112.7 -> 106.0 us, 600 x 2 of 16
+  // 40.3 -> 36.8, 500 x 8 of 64 264 -> 256.  Against no more CTAs than SMs throughout: 2 048 rows x 8 of 128 experts 217 -> 220 where the choices are even and 383 -> 294
+  // where every token chooses one of them, of 64 experts 169 -> 174 and 233 -> 199; three CTAs to two SMs for 2 048 x 4 of 32 took 159 instead of 154.
+  const int64_t pairs = (int64_t)T * top, sms = kNumSMs / experts, most = 4 * kNumSMs / experts;
+  const int64_t per = std::max<int64_t>(1, std::min(pairs / (16 * experts), std::max(sms, std::min(pairs / (64 * experts), most))));
   B200_CUDA(launch(moe_group_gather_kernel, dim3(experts, (unsigned)per), dim3(kGroupThreads), smem_grp, s, ids, T * top, experts, N, n_tiles, tile_expert,
                    pair_tile, row_pair, x, top, width, xg, form.weight_input ? wts : (const float*)nullptr, ones));
   const PdlScope after_grouping;

@@ -313,11 +313,11 @@ def _experts_rounded(x, ids, wts, gate, up, down):
 
 
 @pytest.mark.parametrize("T,W,ff,experts,top", [(1, 64, 64, 8, 2), (3, 136, 72, 5, 5), (40, 64, 200, 4, 2), (300, 256, 136, 6, 3),
-                                                (700, 128, 64, 3, 1), (3000, 64, 64, 4, 3), (100, 64, 128, 4, 1), (200, 72, 64, 4, 1)])
+                                                (700, 128, 64, 3, 1), (3000, 64, 64, 4, 3), (100, 64, 128, 4, 1), (200, 72, 64, 4, 1), (2100, 64, 64, 100, 8)])
 def test_experts_tensor_core_form(T, W, ff, experts, top):
     """Every token-tile size, runs that end inside a tile, experts nobody chose, slab rows past an expert's last row, ff
     that is and is not a multiple of 64 (activation in the epilogue or as a step of its own), more pairs than the grouping
-    kernel holds in shared memory at a time."""
+    kernel holds in shared memory at a time; many experts, one of which every token chooses."""
     g = torch.Generator().manual_seed(T + W)
     x = torch.randn(T, W, generator=g).to(torch.bfloat16)
     gate = [U.bf16_exact(torch.randn(ff, W, generator=g) * W ** -0.5) for _ in range(experts)]
@@ -326,6 +326,8 @@ def test_experts_tensor_core_form(T, W, ff, experts, top):
     ids = torch.stack([torch.randperm(experts, generator=g)[:top] for _ in range(T)]).to(torch.int32)
     if top == 1:
         ids[ids == experts - 1] = 0   # the last expert gets no token
+    if experts == 100:
+        ids = torch.cat([torch.full((T, 1), 99, dtype=torch.int32), torch.stack([torch.randperm(99, generator=g)[:top - 1] for _ in range(T)]).to(torch.int32)], 1)
     wts = torch.rand(T, top, generator=g)
     gu = torch.cat([torch.cat([gate[e], up[e]], 0) for e in range(experts)], 0)
     dn = torch.cat(down, 0)
