@@ -58,18 +58,17 @@ __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-// (a8, R5) bf16(silu(g)) for a bf16-valued g: accurate expf, the division as a correctly rounded reciprocal
-// times g (<= 1 fp32 ulp from g / d, i.e. the bf16 result differs once in ~2^15 elements; an IEEE division
-// costs three times as much and this sits in the gate_up epilogue).  One definition for the fused epilogue
-// and the stand-alone kernel: they stay bit-identical.
-// 1 / d by the hardware's estimate and one step of Newton's (fp32, its last bit at most off), without a branch: __frcp_rn has one for each value, which keeps
-// several of them from being worked out side by side (300 cycles a silu in an epilogue of 16 a thread, 60 so).
+// 1 / d by the hardware's estimate and one step of Newton's (fp32, its last bit at most off; from 1e38 on the estimate alone, since infinity times its reciprocal
+// would be NaN), without a branch: __frcp_rn has one for each value, which keeps several of them from being worked out side by side (300 cycles a silu in an epilogue
+// of 16 a thread, 60 so).
 __device__ __forceinline__ float rcp_newton(float d) {
   float r;
   asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
-  const float rest = d < 1e38f ? fmaf(-d, r, 1.0f) : 0.f;   // (up to infinity, whose reciprocal times it would be NaN)
+  const float rest = d < 1e38f ? fmaf(-d, r, 1.0f) : 0.f;
   return fmaf(r, rest, r);
 }
+// (a8, R5) bf16(silu(g)) for a bf16-valued g: expf, and the division as that reciprocal times g.  For every bf16 the same bits as with a correctly rounded reciprocal
+// (tests/test_kernels_gpu.py).  One definition for the fused epilogue and the stand-alone kernel: they stay bit-identical.
 __device__ __forceinline__ float silu_to_bf16(float g) { return round_bf16(g * rcp_newton(1.0f + expf(-g))); }
 
 // Warp max of floats in ONE instruction (redux.sync on an order-preserving integer image of the float)

@@ -393,6 +393,17 @@ def test_silu_mul(lib, abi, T, I):
     ulp_close(out, O.silu_mul(gu), max_ulp=1, max_frac=0.005)   # expf vs the host libm: rare 1-ulp flips
 
 
+def test_silu_of_every_bf16(lib, abi):
+    """The reciprocal inside is the hardware's estimate and one step of Newton's: the same bits as with IEEE's for every gate there is."""
+    g = torch.arange(-32768, 32768, dtype=torch.int32).to(torch.int16).view(torch.bfloat16).to("cuda")
+    out = torch.empty(1, 65536, dtype=torch.bfloat16, device="cuda")
+    sync_check(abi, lib.b200_silu_mul(torch.cat([g, torch.ones_like(g)]).data_ptr(), out.data_ptr(), 1, 65536, None))
+    x = g.float()
+    want = (x * torch.reciprocal(1.0 + torch.exp(-x))).to(torch.bfloat16)
+    nan = torch.isnan(want)
+    assert torch.equal(torch.isnan(out[0]), nan) and torch.equal(out[0][~nan], want[~nan])
+
+
 def test_argmax_exact_with_ties(lib, abi):
     V = 128256
     lg = torch.randn(6, V, generator=torch.Generator().manual_seed(9)).to(BF)
