@@ -11,7 +11,7 @@
 //    sequence's rows of the step in order (mlstm_walk.cuh; a decode row is a walk of one) with the state in registers; it is stored as
 //    [head][vdim][dim].  n and m are kept once per 32 columns (every CTA of a head needs them from the step before, so they cannot
 //    all share one copy that one of them overwrites).  A sequence whose first row is at position 0 starts from zeros.  Longer portions
-//    go through the tensor cores in chunks (mlstm_chunk.cuh) and segments (mlstm_chunk.cu).
+//    go through the tensor cores in chunks (mlstm_chunk.cuh) and segments (mlstm_segment.cu).
 //  * head_norm_gate: unit RMS per head, weight, sigmoid gate (or the gate's silu).
 #include "mlstm_walk.cuh"
 

@@ -1,4 +1,4 @@
-// The row-by-row walk of the matrix-memory recurrence (mlstm.cu), which the segments' kernel (mlstm_chunk.cu) can take for short portions too.
+// The row-by-row walk of the matrix-memory recurrence (mlstm.cu), which the segments' and the chunks' kernels (mlstm_segment.cu, mlstm_chunk.cu) can take for short portions too.
 #pragma once
 #include "common.cuh"
 #include "f32x2.cuh"
@@ -23,7 +23,7 @@ struct MlstmArgs {
   int both;       // the walk's and the chunks' kernel are both launched, each for its portions
 };
 
-// bf16 rows on the tensor cores (mlstm_chunk.cu)
+// bf16 rows on the tensor cores (mlstm_segment.cu, mlstm_chunk.cu)
 bool mlstm_chunk_supported(const MlstmArgs& a);
 bool mlstm_segments_fit(const MlstmArgs& a, int S);
 int64_t mlstm_chunk_ctas(const MlstmArgs& a, int S);
