@@ -460,6 +460,22 @@ def test_every_schedule_gives_the_oracles_logits_fp32(model_a):
     r.close()
 
 
+@pytest.mark.parametrize("dim", [128, 64])
+def test_delta_rule_of_many_prompts_in_one_step(dim):
+    """Nine prompts side by side (one row, a few, equal ones, both sides of the 64 and 128 rows from which a portion goes in blocks): more sequences than an entry
+    point without a row count takes in blocks, but the step's rows are known and many enough.  The second step goes on from the states of the first."""
+    cfg = F.make_cfg(width=64, layers=[F.delta(heads=2, kv_heads=2, dim=dim, vdim=64, conv=4)])
+    w = F.make_weights(cfg, 9)
+    first = dict(zip("abcdefghi", (70, 70, 1, 64, 33, 129, 130, 63, 5)))
+    then = dict(zip("abcdefghi", (3, 66, 128, 1, 70, 70, 2, 64, 150)))
+    prompts = {n: _prompt(cfg, first[n] + then[n], i + 1) for i, n in enumerate(first)}
+    r = F.make_runner(cfg, w, "float32", max_tokens=640, max_logit_rows=640, n_blocks=100, n_state_slots=10)
+    got = U.replay(U.make_engine(r, max_seqs=9), [list(first.items()), list(then.items())], prompts)
+    for n, p in prompts.items():
+        assert U.rel_rms(got[n], O.forward(F.public_cfg(cfg), w, p)[0].numpy()).max() < F32_TOL, n
+    r.close()
+
+
 def test_a_request_left_out_of_steps_goes_on_where_it_stopped(model_a):
     cfg, w = model_a
     prompts = {"a": _prompt(cfg, 40, 21), "b": _prompt(cfg, 40, 22)}

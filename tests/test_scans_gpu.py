@@ -93,12 +93,12 @@ def test_mlstm_scan_portions_and_hard_gates(f32, heads, dim, vdim, pad):
 @pytest.mark.parametrize("what", ["value", "key", "forget gate", "input gate"])
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
 @pytest.mark.parametrize("row", [0, 37, 100])
-def test_mlstm_chunks_are_causal_for_what_is_not_finite(what, bad, row, T=130):
+def test_mlstm_chunks_are_causal_for_what_is_not_finite(what, bad, row, T=130, heads=2):
     """An infinity or NaN of one row reaches that row and the later ones (a value's its own column, anything else's its head), and no earlier row."""
-    if "gate" in what and bad == float("inf"):
+    if what in ("forget gate", "input gate") and bad == float("inf"):   # ("gate of +inf" below: an input gate)
         bad = float("nan")
     lib, check = pkg("_abi").lib(), pkg("_abi").check
-    heads, dim, vdim, col = 2, 64, 64, 21
+    dim, vdim, col = 64, 64, 21
     g = torch.Generator().manual_seed(5)
     hd, hv = heads * dim, heads * vdim
     floats, ld = int(lib.b200_mlstm_state_floats(heads, dim, vdim)), 2 * hd + hv
@@ -206,16 +206,50 @@ def test_mlstm_segments_are_causal_for_what_is_not_finite(what, bad, row):
     test_mlstm_chunks_are_causal_for_what_is_not_finite(what, bad, row, T=600)
 
 
+# An input gate of +inf makes a head's later rows NaN, as the recurrence has it (the running maximum is infinite); gates of -inf are rows without weight, also where a
+# whole group of 32 rows, a segment's first rows or the sequence's have none: in chunks (130 rows), segments with one row tile and with two.
+@pytest.mark.parametrize("T", [130, 300, 600])
+def test_mlstm_infinite_input_gates(T):
+    test_mlstm_chunks_are_causal_for_what_is_not_finite("gate of +inf", float("inf"), T // 2, T=T)
+    lib, check = pkg("_abi").lib(), pkg("_abi").check
+    heads, dim, vdim = 2, 64, 64
+    g = torch.Generator().manual_seed(T)
+    hd, hv = heads * dim, heads * vdim
+    floats, ld = int(lib.b200_mlstm_state_floats(heads, dim, vdim)), 2 * hd + hv
+    x, gates = torch.randn(T, ld, generator=g).to(torch.bfloat16), torch.randn(T, 2 * heads, generator=g)
+    gates[:, heads:] = torch.nn.functional.logsigmoid(gates[:, heads:] + 3)
+    for lo, hi in ((0, 3), (32, 64), (77, 78), (T - 40, T)) + (((150, 330),) if T > 400 else ()):
+        gates[lo:hi, 1] = float("-inf")
+    zero = tuple(torch.zeros(s, dtype=torch.float64) for s in ((heads, vdim, dim), (heads, dim), (heads,)))
+    want, span, (S, _, m) = _mlstm(x.double(), gates.double(), zero, heads, dim, vdim)
+    state, out = torch.zeros(1, floats, device=DEV), torch.full((T, hv), float("nan"), device=DEV)
+    xd, gd, ptd, std, sld = x.to(DEV), gates.to(DEV), _i32(list(range(T))), _i32([0, T]), _i32([0])
+    check(lib.b200_mlstm_scan(0, xd.data_ptr(), ld, 0, hd, 2 * hd, gd.data_ptr(), ptd.data_ptr(), std.data_ptr(), sld.data_ptr(), state.data_ptr(), floats,
+                              out.data_ptr(), 1, heads, dim, vdim, None))
+    torch.cuda.synchronize()
+    assert ((out.double().cpu() - want).abs() <= 1e-5 * span + 1e-7 * want.abs()).all()     # (as above)
+    st = state[0].double().cpu()
+    assert (st[:hv * dim].reshape(heads, vdim, dim) - S).norm() < 1e-5 * S.norm() and (st[-heads * 2:].reshape(heads, 2) - m[:, None]).abs().max() < 1e-5
+
+
+# The chunks' own kernel, which takes launches of more than 33 clusters of segments: one CTA an SM (36 heads) and two (70)
+@pytest.mark.parametrize("what", ["value", "key", "forget gate", "input gate", "gate of +inf"])
+@pytest.mark.parametrize("heads,T", [(36, 130), (70, 260)])
+@pytest.mark.parametrize("row", [37, 100])
+def test_mlstm_chunk_kernel_is_causal_for_what_is_not_finite(what, heads, T, row):
+    test_mlstm_chunks_are_causal_for_what_is_not_finite(what, float("inf"), row, T=T, heads=heads)
+
+
 # Steps whose CTAs outnumber the SMs: two sequences of 8 heads of 256 columns (256 CTAs, two to an SM, short portions walked beside the chunks),
 # four (512 CTAs: chunks and walk in a launch each, whole portions on both sides of 97 rows), five (the walk alone); the second step
 # starts from the state the first one left.
 @pytest.mark.parametrize("dim", [64, 128])
 @pytest.mark.parametrize("steps", [([130, 30], [20, 97]), ([97, 96, 5, 161], [64, 1, 100, 98]), ([30, 1, 17, 100, 2], [1, 1, 1, 1, 1])])
-def test_mlstm_scan_of_many_ctas(dim, steps):
+def test_mlstm_scan_of_many_ctas(dim, steps, heads=8, vdim=256):
     lib, check = pkg("_abi").lib(), pkg("_abi").check
-    heads, vdim, S = 8, 256, len(steps[0])
+    S = len(steps[0])
     g = torch.Generator().manual_seed(dim + S)
-    hd, hv, nz = heads * dim, heads * vdim, vdim // 32
+    hd, hv, nz = heads * dim, heads * vdim, (vdim + 31) // 32
     floats, ld = int(lib.b200_mlstm_state_floats(heads, dim, vdim)), 2 * hd + hv
     state = torch.full((S + 1, floats), 7.5, device=DEV)
     slots, pos = [S - s for s in range(S)], [0] * S
@@ -245,6 +279,14 @@ def test_mlstm_scan_of_many_ctas(dim, steps):
             assert (st[hv * dim + heads * nz * dim:].reshape(heads, nz) - oracle[s][2][:, None]).abs().max() < 1e-5
             pos[s] += cuts[s]
     assert (state[0] == 7.5).all()
+
+
+# The chunks' own kernel over many chunks, which reuse its buffers, beside short portions: columns that leave a block ragged, one CTA an SM and two, and the walk in a
+# launch of its own (four sequences of 40 heads)
+@pytest.mark.parametrize("heads,dim,vdim,steps", [(20, 128, 72, [[300, 40], [5, 420]]), (36, 64, 64, [[420], [64], [230]]), (37, 40, 32, [[97], [300]]),
+                                                  (40, 64, 72, [[97, 1, 200, 40], [30, 130, 1, 96]])])
+def test_mlstm_chunk_kernel_over_many_chunks(heads, dim, vdim, steps):
+    test_mlstm_scan_of_many_ctas(dim, steps, heads, vdim)
 
 
 # channel decays / one per head, delta rule / plain, heads sharing keys, sizes that leave lanes and columns idle; strided decays (g_chan 2);
@@ -313,7 +355,7 @@ def _delta(q, k, v, beta, decay, S):
 @pytest.mark.parametrize("heads,kv,dim,vdim,steps", [
     (16, 16, 128, 128, [[300], [65]]), (2, 1, 128, 128, [[63], [64], [66], [72], [97]]), (3, 3, 100, 16, [[129], [80]]), (1, 1, 68, 40, [[200], [71]]),
     (16, 4, 128, 128, [[64, 90], [130, 7]]), (40, 8, 128, 48, [[70, 1], [67, 256]]),
-    (16, 16, 128, 128, [[128, 127, 20], [1, 140, 161]]), (8, 2, 64, 128, [[128], [145]]), (16, 4, 64, 128, [[160, 200], [5, 129]]), (4, 4, 36, 24, [[131], [250]]),
+    (16, 16, 128, 128, [[128, 127, 20], [1, 140, 161]]), (16, 16, 64, 128, [[128, 20, 200], [140, 129, 1]]), (8, 2, 64, 128, [[128], [145]]), (16, 4, 64, 128, [[160, 200], [5, 129]]), (4, 4, 36, 24, [[131], [250]]),
 ])
 def test_delta_blocks(heads, kv, dim, vdim, steps, chan):
     lib, check = pkg("_abi").lib(), pkg("_abi").check
@@ -350,10 +392,10 @@ def test_delta_blocks(heads, kv, dim, vdim, steps, chan):
 
 
 # Portions in the order of their length (equal ones, empty ones, the longest first and last), more CTAs than the device has places for, two and three of them
-# an SM, keys of 64 on CTAs of one and two an SM; the bound is that of the test above.
+# an SM, keys of 64 on CTAs of one and three an SM, and more CTAs than go in blocks (walked); the bound is that of the test above.
 @pytest.mark.parametrize("heads,kv,dim,vdim,steps", [
     (16, 16, 128, 128, [[70, 300, 1, 129], [129, 129, 64, 0]]), (16, 8, 128, 128, [[2, 200, 130, 128, 5, 31], [0, 64, 0, 90, 160, 64]]), (40, 40, 64, 128, [[5, 140, 131]]),
-    (8, 2, 64, 128, [[129, 260]]), (16, 16, 100, 48, [[128, 7, 300, 300, 66]]),
+    (16, 4, 64, 128, [[130, 7, 1, 256, 130, 64], [5, 0, 129, 0, 128, 64]]), (8, 2, 64, 128, [[129, 260]]), (16, 16, 100, 48, [[128, 7, 300, 300, 66]]),
 ])
 def test_delta_blocks_of_ordered_portions(heads, kv, dim, vdim, steps):
     test_delta_blocks(heads, kv, dim, vdim, steps, True)
