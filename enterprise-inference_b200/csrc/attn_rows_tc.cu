@@ -611,7 +611,8 @@ static bool ar_form(int heads, int kv_heads, int dim, int vdim, int block_size) 
 }
 // Rows of keys and values are whole boxes of 64 columns.  Two runs over narrower value rows (400 and 420 rows of one sequence, 6 heads over 2, keys of 64, values
 // of 32, of which a box takes 64) ended in an illegal address, each behind some hundred other tests; alone the same call passes, and reading has not shown which access
-// it was.  Such heads take the mma.sync kernel of attn_latent.cu, which reads their rows through pointers, with weights of 16 bits as here.
+// it was.  Such heads take the mma.sync kernel of attn_latent.cu, which reads their rows through pointers, with weights of 16 bits as here (1 900 rows of three
+// sequences, 16 heads of 96 over 4, window 1024: 272 us; heads of 128 here 74).
 bool attn_rows_tc_supported(int heads, int kv_heads, int dim, int vdim, int block_size) {
   return ar_form(heads, kv_heads, dim, vdim, block_size) && dim % 64 == 0 && vdim % 64 == 0;
 }

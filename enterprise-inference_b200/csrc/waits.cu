@@ -1,4 +1,4 @@
-// Waits of the tcgen05 attention kernels and pair linears that ran out (tc.cuh): the word they set in host memory, and the error that the next call makes of it.
+// Waits of the tcgen05 attention kernels, pair linears and matrix-memory segments that ran out (tc.cuh): the word they set in host memory, and the error that the next call makes of it.
 #include "tc.cuh"
 
 namespace b200 {

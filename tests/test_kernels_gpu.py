@@ -62,10 +62,10 @@ _fractions = []
 
 @pytest.fixture(scope="module", autouse=True)
 def _dump_fractions():
-    """Measured differing fractions of every ulp_close call, next to their bounds (gpurun_out/ulp_fractions.txt when
-    that directory exists): a regression inside a bound shows up in the file before it breaks a test."""
+    """Measured differing fractions of every ulp_close call, next to their bounds (ulp_fractions.txt in the folder that
+    B200_TEST_REPORTS names): a regression inside a bound shows up in the file before it breaks a test."""
     yield
-    d = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "gpurun_out")
+    d = os.environ.get("B200_TEST_REPORTS", "")
     if os.path.isdir(d) and _fractions:
         with open(os.path.join(d, "ulp_fractions.txt"), "w") as f:
             for name, frac, bound, mx in _fractions:

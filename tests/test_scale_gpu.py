@@ -26,7 +26,7 @@ MARGIN = 0.08
 
 def report(line: str):
     print(line)
-    d = os.path.join(ROOT, "gpurun_out")
+    d = os.environ.get("B200_TEST_REPORTS", "")
     if os.path.isdir(d):
         with open(os.path.join(d, "scale_report.txt"), "a") as f:
             f.write(line + "\n")
