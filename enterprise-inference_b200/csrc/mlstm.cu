@@ -210,7 +210,8 @@ static int mlstm_scan_t(const MlstmArgs& a, int S, bool single_rows, cudaStream_
 // segments from 193 rows on, chunks from 97, the walk below.  (36 clusters, 9 heads of 256 columns: 160 rows 33.7 us, in chunks 16.6; 300 rows 36.2 and 25.2; 2 048
 // rows 109 and 142, but the length is known on the device only.)
 // Where the rows of the step are known to be too few for a long portion, chunks and walk are launched by themselves: in the segments' launch (us, in a graph, 8 heads)
-// 2 rows 5.3 instead of 5.0, 140 rows 17.8 and 16.5 (128 x 256); 2 rows 4.9 and 4.3, 69 rows 14.7 and 13.5, 215 rows 18.6 and 17.3 (64 x 128).  Segments pay from
+// 2 rows 5.3 instead of 5.0, 140 rows 17.8 and 16.5 (128 x 256); 2 rows 4.9 and 4.3, 69 rows 14.7 and 13.5, 215 rows 18.6 and 17.3 (64 x 128).  (A kernel in which tensor memory is allocated at all
+// takes 0.3 us longer to start: the walk alone in that launch's shape 3.9 us for the 2 rows, with an allocation that it never comes to 4.2.)  Segments pay from
 // 193 rows (215 rows 20.1, in chunks 20.8), with keys of 64 from 257 (300 rows 18.6 and 20.8); 2 048 rows of 128 x 256 58 and 142.
 // Beyond that chunks for all long portions, one or two CTAs an SM, and while these fit at once the chunk kernel walks the short portions itself; else each kernel
 // takes its portions (64 rows of four sequences: 15.0 us, in one kernel 23.1: the idle half of each cluster holds up the next).  Segments there too were a
